@@ -184,95 +184,202 @@ __global__ void __launch_bounds__(256) mxfp8_slab_kernel(const __nv_bfloat16* __
 // ---------------------------------------------------------------------------
 // MXFP8 column mode, optionally with the row-quantised copy, for activations: the bandwidth-bound form.
 //
-// A CTA stages a slab of 32 rows x 512 columns as raw bf16 (16-byte loads, rows 1040 bytes apart so that
-// 16-byte reads of eight consecutive rows fall into different bank groups).  Block maxima are taken on the
-// bit patterns: |x| of a bf16 is its low 15 bits, their unsigned order is the order of the magnitudes, and
-// any pattern above 0x7f80 is a NaN, which makes the block non-finite exactly as the fp32 rule does
-// (bf16 -> fp32 is exact).  Two 16-bit lanes are compared per instruction.
-//   column pass: thread t owns columns 2t and 2t+1 (one 32-bit word per row);
-//   row pass   : lane r of a warp owns row r of one 32-column block (four 16-byte reads).
-// The column pass sweeps the slab twice (maxima, then conversion) instead of holding 32 rows in registers, which
-// lets six CTAs share an SM; it stores two bytes per lane, 64 contiguous bytes per warp and row.
+// Bound: HBM (reads of the source once, two E4M3 copies and their scales written once).  A tile is 128 rows x 128
+// columns: exactly one 512-byte scale atom of either orientation, so both atoms are assembled in shared memory and
+// leave as whole 128-byte lines (single scale bytes of a narrower tile are partial-sector writes: 2.3 M of them per
+// 73 728 x 4096 operand).  A warp owns 32 rows x 64 columns and a lane 8 rows x 8 columns of it, held in registers
+// as loaded (16 bytes per row and lane): row blocks are four neighbouring lanes, column blocks the four lanes of a
+// stride of eight, so both maxima are shuffles, nothing of the tile is staged and no barrier separates the loads from
+// the stores; every lane stores 8 bytes per row and copy (64 contiguous bytes per row of the warp's tile).
+// Block maxima are taken on the bit patterns: |x| of a bf16 is its low 15 bits, their unsigned order is the order of
+// the magnitudes, and any pattern above 0x7f80 is a NaN, which makes the block non-finite exactly as the fp32 rule
+// does (bf16 -> fp32 is exact).  Two 16-bit lanes are compared per instruction.
+// The grid is persistent, so that a launch whose predicate or row count leaves nothing to do ends at once.
+//
+// Measured against the form it replaces (32 x 512 slabs staged in shared memory, two-byte column stores), 73 728 rows,
+// one B200: W13 input gather 4096 wide 309 -> 207 us, gradient gather 329 -> 209 us, SwiGLU forward 1536 wide 216 -> 196 us,
+// SwiGLU backward 431 -> 316 us; a dense 32 768 x 4096 matrix 148 -> 98 us (5.6 TB/s of algorithmic bytes).  The SwiGLU
+// forms are bound by the sigmoid's arithmetic (69 % of the issue slots), the others by HBM.
 // ---------------------------------------------------------------------------
-constexpr int kSlabCols = 512;
-constexpr int kSlabRawStride = kSlabCols * 2 + 16;
+constexpr int kTileRows = 128;
+constexpr int kTileCols = 128;
 
-
-// Where a slab comes from: a dense [rows, C] matrix; rows named by a pointer table (a null pointer is a row of
+// Where a tile comes from: a dense [rows, C] matrix; rows named by a pointer table (a null pointer is a row of
 // zeros; pointers may address peer memory); or SwiGLU of a dense [rows, 2C] matrix [gate | up], rounded to
 // bf16 exactly as the standalone activation kernel rounds it.
-enum SlabSource : int { kSlabDense = 0, kSlabGather = 1, kSlabSwiglu = 2 };
+enum TileSource : int { kTileDense = 0, kTileGather = 1, kTileSwiglu = 2 };
 
-// Row pass, column pass and stores for one staged slab (see above).  `limit` bounds the columns this slab may
-// touch (the matrix width, or the end of the gate half when a CTA stages two slabs), `C` is the row pitch of the
-// outputs.  Called by every thread of the CTA after the slab has been written and a barrier has passed.
-__device__ __forceinline__ void slab_quantise(uint8_t* slab, int64_t rows, int64_t row0, int col0, int limit, int C,
-                                              int64_t max_rows, uint8_t* __restrict__ q_col, uint8_t* __restrict__ s_col,
-                                              int blocked, int col_atoms, uint8_t* __restrict__ q_row,
-                                              uint8_t* __restrict__ s_row, int row_atoms) {
-  const int t = threadIdx.x;
-  if (q_row != nullptr) {
+struct TileOut {
+  uint8_t* q_col;
+  uint8_t* s_col;
+  uint8_t* q_row;
+  uint8_t* s_row;
+  int64_t rows;
+  int64_t max_rows;
+  int C;  // row pitch of the outputs
+  int blocked, col_atoms, row_atoms;
+};
+
+struct TileLane {
+  int warp, lane, rg, cg, slab, half;  // rg: which 8 rows of the warp's 32; cg: which 8 columns of its 64
+  __device__ __forceinline__ TileLane() {
+    warp = threadIdx.x >> 5;
+    lane = threadIdx.x & 31;
+    rg = lane >> 3;
+    cg = lane & 7;
+    slab = warp >> 1;
+    half = warp & 1;
+  }
+  __device__ __forceinline__ int row() const { return slab * 32 + rg * 8; }   // first row inside the tile
+  __device__ __forceinline__ int col() const { return half * 64 + cg * 8; }   // first column inside the tile
+};
+
+// Scale byte and reciprocal of a block of bf16 values from the low 15 bits of its largest magnitude: the byte that
+// mxfp8_scale computes through fp32, in integers.  amax / 448 <= 2^(b - 127) holds for bf16 exactly when the
+// (exponent, mantissa) pair is <= (b + 8, 0x60), 448 being 1.75 * 2^8; bytes below 0 are 0, a non-finite block is 0xFF.
+__device__ __forceinline__ uint32_t mxfp8_scale_bits(uint32_t bits15, float& recip) {
+  const int b = static_cast<int>((bits15 + 0x1fu) >> 7) - 8;
+  const uint32_t byte = bits15 >= 0x7f80u ? 0xffu : static_cast<uint32_t>(b > 0 ? b : 0);
+  recip = byte == 0xffu ? __int_as_float(0x7fc00000) : __uint_as_float((254u - byte) << 23);
+  return byte;
+}
+
+// Products of two packed fp32 pairs (one instruction), as two E4M3 bytes.
+__device__ __forceinline__ uint32_t e4m3x2_scaled(float lo, float hi, float r_lo, float r_hi) {
+  float a, b;
+  asm("{\n\t"
+      ".reg .b64 x, y, z;\n\t"
+      "mov.b64 x, {%2, %3};\n\t"
+      "mov.b64 y, {%4, %5};\n\t"
+      "mul.rn.f32x2 z, x, y;\n\t"
+      "mov.b64 {%0, %1}, z;\n\t"
+      "}\n"
+      : "=f"(a), "=f"(b)
+      : "f"(lo), "f"(hi), "f"(r_lo), "f"(r_hi));
+  return __nv_cvt_float2_to_fp8x2(make_float2(a, b), __NV_SATFINITE, __NV_E4M3);
+}
+
+// Quantises the lane's 8 x 8 values (`w[r]` = row r, packed bf16, zeros outside the matrix) of the tile at
+// (row0, col0).  `limit` bounds the columns this tile may touch.  `atoms` is the CTA's 1 KiB of scale staging; called
+// by every thread of the CTA.
+__device__ __forceinline__ void tile_quantise(const uint4 (&w)[8], const TileLane& me, int64_t row0, int col0, int limit,
+                                              const TileOut& out, uint8_t* atoms) {
+  const int c = col0 + me.col();
+  const int64_t r0 = row0 + me.row();
+  uint8_t* row_atom = atoms;
+  uint8_t* col_atom = atoms + 512;
+  float rrow[8], rcol[8];
+  {
+    uint32_t m[4] = {0, 0, 0, 0};  // maxima of columns 2j (low) and 2j + 1 (high)
+    uint32_t n[4];                 // maxima of rows 2p (low) and 2p + 1 (high)
 #pragma unroll
-    for (int k = 0; k < 2; ++k) {
-      const int r = t & 31, b = (t >> 5) + 8 * k;
-      const int colb = col0 + b * 32;
-      if (row0 + r < rows && colb < limit) {
-        uint32_t w[16];
+    for (int p = 0; p < 4; ++p) {
+      uint32_t h[2];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const uint4 v = *reinterpret_cast<const uint4*>(slab + r * kSlabRawStride + b * 64 + j * 16);
-          w[4 * j] = v.x; w[4 * j + 1] = v.y; w[4 * j + 2] = v.z; w[4 * j + 3] = v.w;
-        }
-        uint32_t m = 0;
+      for (int q = 0; q < 2; ++q) {
+        const uint4 v = w[2 * p + q];
+        const uint32_t ax = v.x & 0x7fff7fffu, ay = v.y & 0x7fff7fffu, az = v.z & 0x7fff7fffu, aw = v.w & 0x7fff7fffu;
+        m[0] = __vmaxu2(m[0], ax);
+        m[1] = __vmaxu2(m[1], ay);
+        m[2] = __vmaxu2(m[2], az);
+        m[3] = __vmaxu2(m[3], aw);
+        h[q] = __vmaxu2(__vmaxu2(ax, ay), __vmaxu2(az, aw));
+      }
+      n[p] = __vmaxu2(__byte_perm(h[0], h[1], 0x5410), __byte_perm(h[0], h[1], 0x7632));
+      n[p] = __vmaxu2(n[p], __shfl_xor_sync(0xffffffffu, n[p], 1));
+      n[p] = __vmaxu2(n[p], __shfl_xor_sync(0xffffffffu, n[p], 2));
+    }
 #pragma unroll
-        for (int j = 0; j < 16; ++j) m = __vmaxu2(m, w[j] & 0x7fff7fffu);
-        const uint32_t top = (m >> 16) > (m & 0xffffu) ? (m >> 16) : (m & 0xffffu);
-        float recip;
-        const uint8_t byte = mxfp8_scale(amax_from_bf16_bits(top), recip);
-        uint32_t o[8];
+    for (int r = 0; r < 8; ++r) {
+      const uint32_t byte = mxfp8_scale_bits((r & 1) ? n[r >> 1] >> 16 : n[r >> 1] & 0xffffu, rrow[r]);
+      if ((me.lane & 3) == 0)
+        row_atom[(me.rg * 8 + r) * 16 + me.slab * 4 + me.half * 2 + (me.cg >> 2)] = static_cast<uint8_t>(byte);
+    }
 #pragma unroll
-        for (int j = 0; j < 8; ++j)
-          o[j] = e4m3x4(__uint_as_float(w[2 * j] << 16) * recip, __uint_as_float(w[2 * j] & 0xffff0000u) * recip,
-                        __uint_as_float(w[2 * j + 1] << 16) * recip, __uint_as_float(w[2 * j + 1] & 0xffff0000u) * recip);
-        uint4* dst = reinterpret_cast<uint4*>(q_row + (row0 + r) * C + colb);
-        dst[0] = make_uint4(o[0], o[1], o[2], o[3]);
-        dst[1] = make_uint4(o[4], o[5], o[6], o[7]);
-        s_row[blocked_offset(row0 + r, colb >> 5, row_atoms)] = byte;
+    for (int j = 0; j < 4; ++j) {
+      m[j] = __vmaxu2(m[j], __shfl_xor_sync(0xffffffffu, m[j], 8));
+      m[j] = __vmaxu2(m[j], __shfl_xor_sync(0xffffffffu, m[j], 16));
+      const uint32_t b0 = mxfp8_scale_bits(m[j] & 0xffffu, rcol[2 * j]);
+      const uint32_t b1 = mxfp8_scale_bits(m[j] >> 16, rcol[2 * j + 1]);
+      if (me.rg == j) {  // the four row groups share the eight columns' bytes between them
+        const int ct = me.col() + 2 * j;
+        col_atom[(ct & 31) * 16 + (ct >> 5) * 4 + me.slab] = static_cast<uint8_t>(b0);
+        col_atom[((ct & 31) + 1) * 16 + (ct >> 5) * 4 + me.slab] = static_cast<uint8_t>(b1);
       }
     }
   }
-  if (q_col == nullptr) return;  // uniform over the CTA
-
-  // column pass: 32 rows of two adjacent columns per thread, in two sweeps over the staged slab (maxima, then
-  // conversion) so that no row values are held in registers; a warp's 2-byte stores cover 64 contiguous bytes.
-  uint32_t m = 0;
+  const bool rowq = out.q_row != nullptr, colq = out.q_col != nullptr;
+  const bool col_wide = (reinterpret_cast<uintptr_t>(out.q_col) & 7) == 0;  // a caller's own buffer may be 2-byte aligned
+  const int64_t left = out.rows - r0;
+  const int live = c < limit ? (left < 8 ? static_cast<int>(left) : 8) : 0;
+  uint8_t* dr = out.q_row + r0 * out.C + c;
+  uint8_t* dc = out.q_col + r0 * out.C + c;
 #pragma unroll
-  for (int r = 0; r < 32; ++r)
-    m = __vmaxu2(m, *reinterpret_cast<const uint32_t*>(slab + r * kSlabRawStride + t * 4) & 0x7fff7fffu);
-  float recip0, recip1;
-  const uint8_t byte0 = mxfp8_scale(amax_from_bf16_bits(m & 0xffffu), recip0);
-  const uint8_t byte1 = mxfp8_scale(amax_from_bf16_bits(m >> 16), recip1);
-  const int c = col0 + 2 * t;
-  if (c >= limit) return;
-  const int64_t rb = row0 >> 5;
-  if (blocked) {
-    s_col[blocked_offset(c, static_cast<int>(rb), col_atoms)] = byte0;
-    s_col[blocked_offset(c + 1, static_cast<int>(rb), col_atoms)] = byte1;
+  for (int r = 0; r < 8; ++r) {
+    const uint4 v = w[r];
+    const float f0 = __uint_as_float(v.x << 16), f1 = __uint_as_float(v.x & 0xffff0000u);
+    const float f2 = __uint_as_float(v.y << 16), f3 = __uint_as_float(v.y & 0xffff0000u);
+    const float f4 = __uint_as_float(v.z << 16), f5 = __uint_as_float(v.z & 0xffff0000u);
+    const float f6 = __uint_as_float(v.w << 16), f7 = __uint_as_float(v.w & 0xffff0000u);
+    if (r < live) {
+      if (rowq)
+        *reinterpret_cast<uint2*>(dr) =
+            make_uint2(e4m3x2_scaled(f0, f1, rrow[r], rrow[r]) | (e4m3x2_scaled(f2, f3, rrow[r], rrow[r]) << 16),
+                       e4m3x2_scaled(f4, f5, rrow[r], rrow[r]) | (e4m3x2_scaled(f6, f7, rrow[r], rrow[r]) << 16));
+      if (colq) {
+        const uint32_t p0 = e4m3x2_scaled(f0, f1, rcol[0], rcol[1]), p1 = e4m3x2_scaled(f2, f3, rcol[2], rcol[3]);
+        const uint32_t p2 = e4m3x2_scaled(f4, f5, rcol[4], rcol[5]), p3 = e4m3x2_scaled(f6, f7, rcol[6], rcol[7]);
+        if (col_wide) {
+          *reinterpret_cast<uint2*>(dc) = make_uint2(p0 | (p1 << 16), p2 | (p3 << 16));
+        } else {
+          uint16_t* d2 = reinterpret_cast<uint16_t*>(dc);
+          d2[0] = static_cast<uint16_t>(p0);
+          d2[1] = static_cast<uint16_t>(p1);
+          d2[2] = static_cast<uint16_t>(p2);
+          d2[3] = static_cast<uint16_t>(p3);
+        }
+      }
+    }
+    dr += out.C;
+    dc += out.C;
+  }
+  __syncthreads();
+  // Scales.  A tile that lies wholly inside the matrix owns whole atoms; at the edges (or in a buffer that 16-byte
+  // stores cannot reach) only the bytes of real blocks are written, one by one: a caller may have zeroed the rest.
+  const int t = threadIdx.x;
+  const bool whole = out.blocked && row0 + kTileRows <= out.rows && col0 + kTileCols <= limit && (col0 & 127) == 0 &&
+                     ((reinterpret_cast<uintptr_t>(out.s_row) | reinterpret_cast<uintptr_t>(out.s_col)) & 15) == 0;
+  if (whole) {
+    if (t < 32) {
+      if (rowq)
+        reinterpret_cast<uint4*>(out.s_row + ((row0 >> 7) * out.row_atoms + (col0 >> 7)) * 512)[t] =
+            reinterpret_cast<const uint4*>(row_atom)[t];
+    } else if (t < 64) {
+      if (colq)
+        reinterpret_cast<uint4*>(out.s_col + (static_cast<int64_t>(col0 >> 7) * out.col_atoms + (row0 >> 7)) * 512)[t - 32] =
+            reinterpret_cast<const uint4*>(col_atom)[t - 32];
+    }
   } else {
-    const int64_t per_col = (max_rows + 31) / 32;
-    s_col[static_cast<int64_t>(c) * per_col + rb] = byte0;
-    s_col[static_cast<int64_t>(c + 1) * per_col + rb] = byte1;
+    for (int i = t; i < 512; i += 256) {
+      if (rowq) {
+        const int r = i >> 2, b = i & 3;  // row and 32-column block of the tile
+        if (row0 + r < out.rows && col0 + b * 32 < limit)
+          out.s_row[blocked_offset(row0 + r, (col0 >> 5) + b, out.row_atoms)] = row_atom[(r & 31) * 16 + (r >> 5) * 4 + b];
+      }
+      if (colq) {
+        const int ct = i >> 2, sl = i & 3;  // column and 32-row block of the tile
+        const int64_t rb = (row0 >> 5) + sl;
+        if (col0 + ct < limit && row0 + sl * 32 < out.rows) {
+          const uint8_t byte = col_atom[(ct & 31) * 16 + (ct >> 5) * 4 + sl];
+          if (out.blocked)
+            out.s_col[blocked_offset(col0 + ct, static_cast<int>(rb), out.col_atoms)] = byte;
+          else
+            out.s_col[static_cast<int64_t>(col0 + ct) * ((out.max_rows + 31) / 32) + rb] = byte;
+        }
+      }
+    }
   }
-  const int live = rows - row0 < 32 ? static_cast<int>(rows - row0) : 32;
-  uint8_t* dst = q_col + row0 * C + c;
-#pragma unroll 8
-  for (int r = 0; r < live; ++r) {
-    const uint32_t w = *reinterpret_cast<const uint32_t*>(slab + r * kSlabRawStride + t * 4);
-    const uint32_t pk = __nv_cvt_float2_to_fp8x2(
-        make_float2(__uint_as_float(w << 16) * recip0, __uint_as_float(w & 0xffff0000u) * recip1), __NV_SATFINITE,
-        __NV_E4M3);
-    *reinterpret_cast<uint16_t*>(dst + static_cast<int64_t>(r) * C) = static_cast<uint16_t>(pk);
-  }
+  __syncthreads();  // the staging bytes may be written again
 }
 
 // Placement chosen on the device: each pointer is an allocation base and the byte offset is read from device memory
@@ -296,107 +403,152 @@ __device__ __forceinline__ T* placed(T* base, const int64_t* off) {
   return reinterpret_cast<T*>(reinterpret_cast<uintptr_t>(base) + static_cast<uintptr_t>(*off));
 }
 
+// 16 bytes global -> shared without passing through registers; `bytes` 0 fills with zeros and reads nothing.
+__device__ __forceinline__ void cp_async16(void* smem_dst, const void* src, int bytes) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(smem_dst)), "l"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+// A lane's 8 rows of every input arrive in shared-memory slots of its own through asynchronous copies: the next tile's
+// rows are in flight while this tile is converted and stored, without holding registers, and the activation of the SwiGLU
+// forms runs in a rolled loop (the exponential and the IEEE reciprocal of 64 unrolled elements did not fit the
+// instruction cache: 265 against 196 us).  Slots are private to the thread, so no barrier is involved.
+constexpr int kTileSlot = 8 * 256;  // uint4 slots of one input
+
 template <int kSource>
-__global__ void __launch_bounds__(256) mxfp8_colrow_kernel(const uint4* __restrict__ x, const int64_t* __restrict__ row_ptrs,
-                                                           ActParams act, const int32_t* num_rows,
-                                                           int64_t max_rows, int C, uint8_t* __restrict__ q_col,
-                                                           uint8_t* __restrict__ s_col, int blocked, int col_atoms,
-                                                           uint8_t* __restrict__ q_row, uint8_t* __restrict__ s_row,
-                                                           int row_atoms, PlacedOffsets at) {
-  __shared__ __align__(16) uint8_t slab[32 * kSlabRawStride];
+__global__ void __launch_bounds__(256, 3) mxfp8_colrow_kernel(const uint4* __restrict__ x, const int64_t* __restrict__ row_ptrs,
+                                                              ActParams act, const int32_t* num_rows,
+                                                              int64_t max_rows, int C, uint8_t* __restrict__ q_col,
+                                                              uint8_t* __restrict__ s_col, int blocked, int col_atoms,
+                                                              uint8_t* __restrict__ q_row, uint8_t* __restrict__ s_row,
+                                                              int row_atoms, PlacedOffsets at) {
+  __shared__ __align__(16) uint8_t atoms[1024];
+  extern __shared__ uint4 slots[];
   if (at.cond != nullptr && *at.cond == 0) return;
   int64_t rows = num_rows ? *num_rows : max_rows;
   if (rows > max_rows) rows = max_rows;
   x = placed(x, at.x);
-  q_col = placed(q_col, at.q_col);
-  s_col = placed(s_col, at.s_col);
-  q_row = placed(q_row, at.q_row);
-  s_row = placed(s_row, at.s_row);
   if (at.compact_cols) col_atoms = static_cast<int>(((rows + 31) / 32 + 3) / 4);
-  const int64_t row0 = static_cast<int64_t>(blockIdx.y) * 32;
-  const int col0 = blockIdx.x * kSlabCols;
-  if (row0 >= rows) return;
-  const int t = threadIdx.x;
+  const TileOut out{placed(q_col, at.q_col), placed(s_col, at.s_col), placed(q_row, at.q_row), placed(s_row, at.s_row),
+                    rows, max_rows, C, blocked, col_atoms, row_atoms};
+  const TileLane me;
   const int vec_per_row = C >> 3;
+  const int col_tiles = (C + kTileCols - 1) / kTileCols;
+  const int64_t tiles = (rows + kTileRows - 1) / kTileRows * col_tiles;
+  uint4* slot = slots + threadIdx.x;
+  uint4* up = slot + kTileSlot;
+  auto fetch = [&](int64_t tile) {  // the lane's 8 rows of a tile on their way into its slots
+    const int64_t r0 = tile / col_tiles * kTileRows + me.row();
+    const int c = static_cast<int>(tile - tile / col_tiles * col_tiles) * kTileCols + me.col();
+    const int v = c >> 3;
+    const int64_t left = rows - r0;
+    const int live = c < C ? (left < 8 ? static_cast<int>(left) : 8) : 0;
 #pragma unroll
-  for (int k = 0; k < 8; ++k) {
-    const int i = t + 256 * k;
-    const int r = i >> 6, v = i & 63;
-    uint4 val = make_uint4(0, 0, 0, 0);
-    if (row0 + r < rows && col0 + v * 8 < C) {
-      if (kSource == kSlabDense) {
-        val = x[(row0 + r) * vec_per_row + (col0 >> 3) + v];
-      } else if (kSource == kSlabGather) {
-        const uint4* src = reinterpret_cast<const uint4*>(row_ptrs[row0 + r]);
-        if (src != nullptr) val = __ldcg(src + (col0 >> 3) + v);
+    for (int r = 0; r < 8; ++r) {
+      if (kSource == kTileSwiglu) {
+        const uint4* src = x + (r0 + r) * 2 * vec_per_row + v;
+        cp_async16(slot + 256 * r, r < live ? src : x, r < live ? 16 : 0);
+        cp_async16(up + 256 * r, r < live ? src + vec_per_row : x, r < live ? 16 : 0);
+      } else if (kSource == kTileDense) {
+        cp_async16(slot + 256 * r, r < live ? x + (r0 + r) * vec_per_row + v : x, r < live ? 16 : 0);
       } else {
-        const uint4 g4 = x[(row0 + r) * 2 * vec_per_row + (col0 >> 3) + v];
-        const uint4 u4 = x[(row0 + r) * 2 * vec_per_row + vec_per_row + (col0 >> 3) + v];
+        const uint4* src = r < live ? reinterpret_cast<const uint4*>(row_ptrs[r0 + r]) : nullptr;
+        cp_async16(slot + 256 * r, src != nullptr ? static_cast<const void*>(src + v) : row_ptrs, src != nullptr ? 16 : 0);
+      }
+    }
+  };
+  if (static_cast<int64_t>(blockIdx.x) < tiles) fetch(blockIdx.x);
+  for (int64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+    const int64_t row0 = tile / col_tiles * kTileRows;
+    const int col0 = static_cast<int>(tile - tile / col_tiles * col_tiles) * kTileCols;
+    cp_async_wait_all();
+    if (kSource == kTileSwiglu) {
+#pragma unroll 1
+      for (int r = 0; r < 8; ++r) {
         float g[8], u[8];
-        unpack8f(g4, g);
-        unpack8f(u4, u);
+        unpack8f(slot[256 * r], g);
+        unpack8f(up[256 * r], u);
         uint32_t z[4];
 #pragma unroll
         for (int j = 0; j < 4; ++j)
           z[j] = pack_bf16x2(swiglu_f32(g[2 * j], u[2 * j], act), swiglu_f32(g[2 * j + 1], u[2 * j + 1], act));
-        val = make_uint4(z[0], z[1], z[2], z[3]);
+        slot[256 * r] = make_uint4(z[0], z[1], z[2], z[3]);
       }
     }
-    *reinterpret_cast<uint4*>(slab + r * kSlabRawStride + v * 16) = val;
+    uint4 w[8];
+#pragma unroll
+    for (int r = 0; r < 8; ++r) w[r] = slot[256 * r];
+    if (tile + gridDim.x < tiles) fetch(tile + gridDim.x);  // in flight behind this tile's arithmetic and stores
+    tile_quantise(w, me, row0, col0, C, out, atoms);
   }
-  __syncthreads();
-  slab_quantise(slab, rows, row0, col0, C, C, max_rows, q_col, s_col, blocked, col_atoms, q_row, s_row, row_atoms);
 }
 
 // SwiGLU backward fused in: from h1 = [gate | up] ([rows, 2F]) and dz = dL/dh2 ([rows, F]) a CTA computes the
-// gate-gradient slab and the matching up-gradient slab of grad_h1 = [dgate | dup] (rounded to bf16 as the standalone
+// gate-gradient tile and the matching up-gradient tile of grad_h1 = [dgate | dup] (rounded to bf16 as the standalone
 // backward kernel rounds them) and quantises both; grad_h1 itself is never written.  Either copy may be left out.
-__global__ void __launch_bounds__(256) mxfp8_swiglu_bwd_colrow_kernel(const uint4* __restrict__ h1,
-                                                                      const uint4* __restrict__ dz, ActParams act,
-                                                                      const int32_t* num_rows, int64_t max_rows, int F,
-                                                                      uint8_t* __restrict__ q_col,
-                                                                      uint8_t* __restrict__ s_col, int col_atoms,
-                                                                      uint8_t* __restrict__ q_row,
-                                                                      uint8_t* __restrict__ s_row, int row_atoms,
-                                                                      PlacedOffsets at) {
-  extern __shared__ __align__(16) uint8_t slabs[];  // two slabs
-  uint8_t* slab_g = slabs;
-  uint8_t* slab_u = slabs + 32 * kSlabRawStride;
+__global__ void __launch_bounds__(256, 2) mxfp8_swiglu_bwd_colrow_kernel(const uint4* __restrict__ h1,
+                                                                         const uint4* __restrict__ dz, ActParams act,
+                                                                         const int32_t* num_rows, int64_t max_rows, int F,
+                                                                         uint8_t* __restrict__ q_col,
+                                                                         uint8_t* __restrict__ s_col, int col_atoms,
+                                                                         uint8_t* __restrict__ q_row,
+                                                                         uint8_t* __restrict__ s_row, int row_atoms,
+                                                                         PlacedOffsets at) {
+  __shared__ __align__(16) uint8_t atoms[1024];
+  extern __shared__ uint4 slots[];
   int64_t rows = num_rows ? *num_rows : max_rows;
   if (rows > max_rows) rows = max_rows;
   h1 = placed(h1, at.x);
   dz = placed(dz, at.x2);
-  q_col = placed(q_col, at.q_col);
-  s_col = placed(s_col, at.s_col);
-  q_row = placed(q_row, at.q_row);
-  s_row = placed(s_row, at.s_row);
   if (at.compact_cols) col_atoms = static_cast<int>(((rows + 31) / 32 + 3) / 4);
-  const int64_t row0 = static_cast<int64_t>(blockIdx.y) * 32;
-  const int col0 = blockIdx.x * kSlabCols;
-  if (row0 >= rows) return;
-  const int t = threadIdx.x;
+  const TileOut out{placed(q_col, at.q_col), placed(s_col, at.s_col), placed(q_row, at.q_row), placed(s_row, at.s_row),
+                    rows, max_rows, 2 * F, 1, col_atoms, row_atoms};
+  const TileLane me;
   const int vec_per_row = F >> 3;
+  const int col_tiles = (F + kTileCols - 1) / kTileCols;
+  const int64_t tiles = (rows + kTileRows - 1) / kTileRows * col_tiles;
+  uint4* gate = slots + threadIdx.x;
+  uint4* up = gate + kTileSlot;
+  uint4* grad = up + kTileSlot;
+  auto fetch = [&](int64_t tile) {
+    const int64_t r0 = tile / col_tiles * kTileRows + me.row();
+    const int c = static_cast<int>(tile - tile / col_tiles * col_tiles) * kTileCols + me.col();
+    const int v = c >> 3;
+    const int64_t left = rows - r0;
+    const int live = c < F ? (left < 8 ? static_cast<int>(left) : 8) : 0;
 #pragma unroll
-  for (int k = 0; k < 8; ++k) {
-    const int i = t + 256 * k;
-    const int r = i >> 6, v = i & 63;
-    uint4 dg4 = make_uint4(0, 0, 0, 0), du4 = make_uint4(0, 0, 0, 0);
-    if (row0 + r < rows && col0 + v * 8 < F) {
+    for (int r = 0; r < 8; ++r) {
+      const uint4* src = h1 + (r0 + r) * 2 * vec_per_row + v;
+      cp_async16(gate + 256 * r, r < live ? src : h1, r < live ? 16 : 0);
+      cp_async16(up + 256 * r, r < live ? src + vec_per_row : h1, r < live ? 16 : 0);
+      cp_async16(grad + 256 * r, r < live ? dz + (r0 + r) * vec_per_row + v : h1, r < live ? 16 : 0);
+    }
+  };
+  if (static_cast<int64_t>(blockIdx.x) < tiles) fetch(blockIdx.x);
+  for (int64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+    const int64_t row0 = tile / col_tiles * kTileRows;
+    const int col0 = static_cast<int>(tile - tile / col_tiles * col_tiles) * kTileCols;
+    cp_async_wait_all();
+#pragma unroll 1
+    for (int r = 0; r < 8; ++r) {
       float x[8], y[8], d[8], dx[8], dy[8];
-      unpack8f(h1[(row0 + r) * 2 * vec_per_row + (col0 >> 3) + v], x);
-      unpack8f(h1[(row0 + r) * 2 * vec_per_row + vec_per_row + (col0 >> 3) + v], y);
-      unpack8f(dz[(row0 + r) * vec_per_row + (col0 >> 3) + v], d);
+      unpack8f(gate[256 * r], x);
+      unpack8f(up[256 * r], y);
+      unpack8f(grad[256 * r], d);
 #pragma unroll
       for (int j = 0; j < 8; ++j) swiglu_bwd_f32(x[j], y[j], d[j], act, dx[j], dy[j]);
-      dg4 = make_uint4(pack_bf16x2(dx[0], dx[1]), pack_bf16x2(dx[2], dx[3]), pack_bf16x2(dx[4], dx[5]), pack_bf16x2(dx[6], dx[7]));
-      du4 = make_uint4(pack_bf16x2(dy[0], dy[1]), pack_bf16x2(dy[2], dy[3]), pack_bf16x2(dy[4], dy[5]), pack_bf16x2(dy[6], dy[7]));
+      gate[256 * r] = make_uint4(pack_bf16x2(dx[0], dx[1]), pack_bf16x2(dx[2], dx[3]), pack_bf16x2(dx[4], dx[5]), pack_bf16x2(dx[6], dx[7]));
+      up[256 * r] = make_uint4(pack_bf16x2(dy[0], dy[1]), pack_bf16x2(dy[2], dy[3]), pack_bf16x2(dy[4], dy[5]), pack_bf16x2(dy[6], dy[7]));
     }
-    *reinterpret_cast<uint4*>(slab_g + r * kSlabRawStride + v * 16) = dg4;
-    *reinterpret_cast<uint4*>(slab_u + r * kSlabRawStride + v * 16) = du4;
+#pragma unroll 1
+    for (int which = 0; which < 2; ++which) {
+      uint4 w[8];
+#pragma unroll
+      for (int r = 0; r < 8; ++r) w[r] = gate[which * kTileSlot + 256 * r];
+      if (which == 1 && tile + gridDim.x < tiles) fetch(tile + gridDim.x);
+      tile_quantise(w, me, row0, which * F + col0, (which + 1) * F, out, atoms);
+    }
   }
-  __syncthreads();
-  slab_quantise(slab_g, rows, row0, col0, F, 2 * F, max_rows, q_col, s_col, 1, col_atoms, q_row, s_row, row_atoms);
-  slab_quantise(slab_u, rows, row0, F + col0, 2 * F, 2 * F, max_rows, q_col, s_col, 1, col_atoms, q_row, s_row, row_atoms);
 }
 
 // ---------------------------------------------------------------------------
@@ -634,6 +786,13 @@ __global__ void __launch_bounds__(256) gather_packed_kernel(const int64_t* __res
   }
 }
 
+// Grid of the persistent 128 x 128 tile quantisers: `per_sm` resident CTAs per SM, never more than there are tiles.
+static int tile_grid(int64_t max_rows, int64_t C, int per_sm) {
+  const int64_t tiles = ceil_div64(max_rows, kTileRows) * ceil_div64(C, kTileCols);
+  const int64_t cap = grid_cap(per_sm);
+  return static_cast<int>(tiles < cap ? tiles : cap);
+}
+
 static int blocks_for(int64_t items, int threads, int cap) {
   int64_t b = (items + threads - 1) / threads;
   if (b > cap) b = cap;
@@ -666,8 +825,8 @@ extern "C" int dm_quant_mxfp8_col(const void* x, const int32_t* num_rows, int64_
   if (max_rows == 0) return kRcOk;
   const int atoms = static_cast<int>(((max_rows + 31) / 32 + 3) / 4);
   if ((C % 16) == 0 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(q)) % 16) == 0) {
-    const dim3 fast(static_cast<unsigned>((C + kSlabCols - 1) / kSlabCols), static_cast<unsigned>((max_rows + 31) / 32));
-    mxfp8_colrow_kernel<kSlabDense><<<fast, 256, 0, static_cast<cudaStream_t>(stream)>>>(
+    const int fast = tile_grid(max_rows, C, 3);
+    mxfp8_colrow_kernel<kTileDense><<<fast, 256, kTileSlot * 16, static_cast<cudaStream_t>(stream)>>>(
         static_cast<const uint4*>(x), nullptr, ActParams{0, 1.0f, 0.0f}, num_rows, max_rows, static_cast<int>(C),
         static_cast<uint8_t*>(q), static_cast<uint8_t*>(scales), blocked, atoms, nullptr, nullptr, 0, PlacedOffsets{});
     return static_cast<int>(cudaGetLastError());
@@ -684,10 +843,10 @@ extern "C" int dm_quant_mxfp8_rowcol(const void* x, const int32_t* num_rows, int
   if (!x || !q_row || !scales_row_blocked || !q_col || !scales_col_blocked || max_rows < 0 || C <= 0 || (C % 32) != 0)
     return kRcBadArg;
   if (max_rows == 0) return kRcOk;
-  const dim3 grid(static_cast<unsigned>((C + kSlabCols - 1) / kSlabCols), static_cast<unsigned>((max_rows + 31) / 32));
+  const int grid = tile_grid(max_rows, C, 3);
   const int col_atoms = static_cast<int>(((max_rows + 31) / 32 + 3) / 4);
   const int row_atoms = static_cast<int>((C / 32 + 3) / 4);
-  mxfp8_colrow_kernel<kSlabDense><<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(
+  mxfp8_colrow_kernel<kTileDense><<<grid, 256, kTileSlot * 16, static_cast<cudaStream_t>(stream)>>>(
       static_cast<const uint4*>(x), nullptr, ActParams{0, 1.0f, 0.0f}, num_rows, max_rows, static_cast<int>(C),
       static_cast<uint8_t*>(q_col), static_cast<uint8_t*>(scales_col_blocked), 1, col_atoms,
       static_cast<uint8_t*>(q_row), static_cast<uint8_t*>(scales_row_blocked), row_atoms, PlacedOffsets{});
@@ -700,10 +859,10 @@ static int launch_rowcol_gather(const int64_t* row_ptrs, const int32_t* num_rows
       (C % 32) != 0)
     return kRcBadArg;  // the column copy may be left out (a forward nothing will differentiate)
   if (max_rows == 0) return kRcOk;
-  const dim3 grid(static_cast<unsigned>((C + kSlabCols - 1) / kSlabCols), static_cast<unsigned>((max_rows + 31) / 32));
+  const int grid = tile_grid(max_rows, C, 3);
   const int col_atoms = static_cast<int>(((max_rows + 31) / 32 + 3) / 4);
   const int row_atoms = static_cast<int>((C / 32 + 3) / 4);
-  mxfp8_colrow_kernel<kSlabGather><<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(
+  mxfp8_colrow_kernel<kTileGather><<<grid, 256, kTileSlot * 16, static_cast<cudaStream_t>(stream)>>>(
       nullptr, row_ptrs, ActParams{0, 1.0f, 0.0f}, num_rows, max_rows, static_cast<int>(C), static_cast<uint8_t*>(q_col),
       static_cast<uint8_t*>(sf_col), 1, col_atoms, static_cast<uint8_t*>(q_row), static_cast<uint8_t*>(sf_row),
       row_atoms, at);
@@ -731,10 +890,17 @@ static int launch_swiglu_fwd_quant(const void* h1, const int32_t* num_rows, int6
   if (!h1 || !q_row || !sf_row || (q_col == nullptr) != (sf_col == nullptr) || max_rows < 0 || F <= 0 || (F % 32) != 0)
     return kRcBadArg;
   if (max_rows == 0) return kRcOk;
-  const dim3 grid(static_cast<unsigned>((F + kSlabCols - 1) / kSlabCols), static_cast<unsigned>((max_rows + 31) / 32));
+  constexpr int kSmem = 2 * kTileSlot * 16;
+  static PerDeviceOnce attr_set;
+  const int rc_attr = once_per_device(attr_set, [] {
+    return static_cast<int>(
+        cudaFuncSetAttribute(mxfp8_colrow_kernel<kTileSwiglu>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
+  });
+  if (rc_attr != 0) return rc_attr;
+  const int grid = tile_grid(max_rows, F, 3);
   const int col_atoms = static_cast<int>(((max_rows + 31) / 32 + 3) / 4);
   const int row_atoms = static_cast<int>((F / 32 + 3) / 4);
-  mxfp8_colrow_kernel<kSlabSwiglu><<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(
+  mxfp8_colrow_kernel<kTileSwiglu><<<grid, 256, kSmem, static_cast<cudaStream_t>(stream)>>>(
       static_cast<const uint4*>(h1), nullptr, ActParams{clamped, alpha, limit}, num_rows, max_rows, static_cast<int>(F),
       static_cast<uint8_t*>(q_col), static_cast<uint8_t*>(sf_col), 1, col_atoms, static_cast<uint8_t*>(q_row),
       static_cast<uint8_t*>(sf_row), row_atoms, at);
@@ -766,14 +932,14 @@ static int launch_swiglu_bwd_quant(const void* h1, const void* grad_h2, const in
       (q_row == nullptr && q_col == nullptr))
     return kRcBadArg;
   if (max_rows == 0) return kRcOk;
-  constexpr int kSmem = 2 * 32 * kSlabRawStride;
+  constexpr int kSmem = 3 * kTileSlot * 16;
   static PerDeviceOnce attr_set;
   const int rc_attr = once_per_device(attr_set, [] {
     return static_cast<int>(
         cudaFuncSetAttribute(mxfp8_swiglu_bwd_colrow_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
   });
   if (rc_attr != 0) return rc_attr;
-  const dim3 grid(static_cast<unsigned>((F + kSlabCols - 1) / kSlabCols), static_cast<unsigned>((max_rows + 31) / 32));
+  const int grid = tile_grid(max_rows, F, 2);
   const int col_atoms = static_cast<int>(((max_rows + 31) / 32 + 3) / 4);
   const int row_atoms = static_cast<int>((2 * F / 32 + 3) / 4);
   mxfp8_swiglu_bwd_colrow_kernel<<<grid, 256, kSmem, static_cast<cudaStream_t>(stream)>>>(

@@ -300,3 +300,52 @@ def test_nvfp4_token_live_rows_only(rows, cols):
         assert torch.equal(g[keep], w[keep])
     assert bool((got[0][~keep] == 0xAB).all()) and bool((got[1][~keep] == 0xAB).all())
     assert bool((got[2][~keep] == float(0xAB)).all())
+
+
+@pytest.mark.parametrize("rows,cols,gather,offset", [(1, 32, 0, 0), (127, 96, 1, 0), (128, 128, 0, 0), (129, 160, 1, 0),
+                                                     (261, 384, 0, 2), (300, 288, 1, 2), (384, 1056, 1, 0)])
+def test_mxfp8_rowcol_tile_edges_against_the_oracle(rows, cols, gather, offset):
+    """Both copies and both scale sets at the edges of the 128 x 128 tiles (partial rows, partial 32-row blocks, partial
+    column tiles), with blocks that are zero, infinite, NaN, subnormal or exactly 448 * 2^k, null row pointers, and
+    output buffers that are only 2-byte aligned.  Integer results: equal."""
+    nat = _nat()
+    x = _data(rows, cols, 7 * rows + cols)
+    x[:, 5] = 0
+    x[rows // 2, :] = 448.0 * 2.0 ** -6  # amax / 448 is a power of two: the scale must not round up
+    x[rows - 1, : min(32, cols)] = 2.0 ** -133  # subnormal bf16
+    cap = rows + 3
+    cnt = torch.tensor([rows], dtype=torch.int32, device=DEV)
+    ra, ca = (cols // 32 + 3) // 4, ((cap + 31) // 32 + 3) // 4
+    n_rs, n_cs = (cap + 127) // 128 * 128 * ra * 4, (cols + 127) // 128 * 128 * ca * 4
+    qr = torch.zeros(cap * cols, dtype=torch.uint8, device=DEV)
+    sr = torch.full((n_rs + 16,), 0xEE, dtype=torch.uint8, device=DEV)[offset: offset + n_rs]
+    qc = torch.zeros(cap * cols + 16, dtype=torch.uint8, device=DEV)[offset: offset + cap * cols]
+    sc = torch.full((n_cs + 16,), 0xEE, dtype=torch.uint8, device=DEV)[offset: offset + n_cs]
+    xd = x.to(DEV)
+    out = (qr.data_ptr(), sr.data_ptr(), qc.data_ptr(), sc.data_ptr())
+    if gather:
+        null = torch.arange(rows) % 5 == 2
+        ptrs = torch.where(null, 0, xd.data_ptr() + torch.arange(rows) * cols * 2).to(DEV)
+        x[null] = 0
+        nat.check(nat.lib.dm_quant_mxfp8_rowcol_gather(ptrs.data_ptr(), cnt.data_ptr(), cap, cols, *out, nat.stream_ptr()), "gather")
+    else:
+        nat.check(nat.lib.dm_quant_mxfp8_rowcol(xd.data_ptr(), cnt.data_ptr(), cap, cols, *out, nat.stream_ptr()), "rowcol")
+    torch.cuda.synchronize()
+
+    def same(got, want, scales):  # data of non-finite blocks is NaN of either sign
+        finite = scales != 255
+        np.testing.assert_array_equal(got[finite], want[finite])
+        assert ((got[~finite] & 0x7F) == 0x7F).all()
+
+    rq, rs = Q.mxfp8_row(x)
+    r, c = np.meshgrid(np.arange(rows), np.arange(cols // 32), indexing="ij")
+    np.testing.assert_array_equal(sr.cpu().numpy()[Q.blocked_scale_offset(r, c, ra)], rs)
+    same(qr.cpu().numpy().reshape(cap, cols)[:rows], rq, np.repeat(rs, 32, axis=1))
+    cq, cs = Q.mxfp8_col(x)
+    c, b = np.meshgrid(np.arange(cols), np.arange((rows + 31) // 32), indexing="ij")
+    np.testing.assert_array_equal(sc.cpu().numpy()[Q.blocked_scale_offset(c, b, ca)], cs)
+    same(qc.cpu().numpy().reshape(cap, cols)[:rows], cq, np.repeat(cs.T, 32, axis=0)[:rows])
+    # nothing outside the matrix was written
+    assert int(qr.view(cap, cols)[rows:].sum()) == 0 and int(qc.view(cap, cols)[rows:].sum()) == 0
+    assert int((sr.cpu() == 0xEE).sum()) >= n_rs - rs.size
+    assert int((sc.cpu() == 0xEE).sum()) >= n_cs - cs.size
