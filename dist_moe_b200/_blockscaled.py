@@ -399,8 +399,9 @@ def run_block_scaled(x, ids, scores, w13_weight, w2_weight, context: Any, option
                                                     buf.data_ptr() + lay.h_q, hq, buf.data_ptr() + lay.h_sf, 0, 1,
                                                     buf.data_ptr() + lay.h_inv, 4, st), "dm_quant_nvfp4_token_live(h2)")
     else:
-        nat.check(nat.lib.dm_quant_mxfp8_row(h2_ptr, recv.data_ptr(), max_rows, F, buf.data_ptr() + lay.h_q, 0,
-                                             buf.data_ptr() + lay.h_sf, 0, 1, st), "dm_quant_mxfp8_row(h2)")
+        nat.check(nat.lib.dm_quant_mxfp8_row_live(sct.data_ptr(), h2_ptr, recv.data_ptr(), max_rows, F,
+                                                  buf.data_ptr() + lay.h_q, 0, buf.data_ptr() + lay.h_sf, 0, 1, st),
+                  "dm_quant_mxfp8_row_live(h2)")
     # ---- W2 + scatter to the owners' combine buffers ---------------------------------------------
     if swapped:
         nat.check(nat.lib.dm_gemm_blockscaled_swapped(f, _view(buf, lay.h_q), _view(buf, lay.h_sf),

@@ -150,6 +150,7 @@ _SIGNATURES = {
         [_P, _P, c_int, _P, c_int, _P, _P, _P, c_float, c_int, c_int, _P, _P, c_int64, c_int, c_int64, _P],
     ),
     "dm_quant_mxfp8_row": (c_int, [_P, _P, c_int64, c_int64, _P, c_int64, _P, c_int64, c_int, _P]),
+    "dm_quant_mxfp8_row_live": (c_int, [_P, _P, _P, c_int64, c_int64, _P, c_int64, _P, c_int64, c_int, _P]),
     "dm_quant_mxfp8_col": (c_int, [_P, _P, c_int64, c_int64, _P, _P, c_int, _P]),
     "dm_quant_mxfp8_rowcol": (c_int, [_P, _P, c_int64, c_int64, _P, _P, _P, _P, _P]),
     "dm_quant_mxfp8_rowcol_gather": (c_int, [_P, _P, c_int64, c_int64, _P, _P, _P, _P, _P]),

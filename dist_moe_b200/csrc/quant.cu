@@ -18,48 +18,78 @@
 
 namespace dm {
 
+// Scale byte and reciprocal of a block of bf16 values from the low 15 bits of its largest magnitude: the byte that
+// mxfp8_scale computes through fp32, in integers.  amax / 448 <= 2^(b - 127) holds for bf16 exactly when the
+// (exponent, mantissa) pair is <= (b + 8, 0x60), 448 being 1.75 * 2^8; bytes below 0 are 0, a non-finite block is 0xFF.
+__device__ __forceinline__ uint32_t mxfp8_scale_bits(uint32_t bits15, float& recip) {
+  const int b = static_cast<int>((bits15 + 0x1fu) >> 7) - 8;
+  const uint32_t byte = bits15 >= 0x7f80u ? 0xffu : static_cast<uint32_t>(b > 0 ? b : 0);
+  recip = byte == 0xffu ? __int_as_float(0x7fc00000) : __uint_as_float((254u - byte) << 23);
+  return byte;
+}
+
+// Products of two packed fp32 pairs (one instruction), as two E4M3 bytes.
+__device__ __forceinline__ uint32_t e4m3x2_scaled(float lo, float hi, float r_lo, float r_hi) {
+  float a, b;
+  asm("{\n\t"
+      ".reg .b64 x, y, z;\n\t"
+      "mov.b64 x, {%2, %3};\n\t"
+      "mov.b64 y, {%4, %5};\n\t"
+      "mul.rn.f32x2 z, x, y;\n\t"
+      "mov.b64 {%0, %1}, z;\n\t"
+      "}\n"
+      : "=f"(a), "=f"(b)
+      : "f"(lo), "f"(hi), "f"(r_lo), "f"(r_hi));
+  return __nv_cvt_float2_to_fp8x2(make_float2(a, b), __NV_SATFINITE, __NV_E4M3);
+}
+
 // ---------------------------------------------------------------------------
-// MXFP8 row mode: 1x32 blocks along the contiguous dimension.  8 elements per
-// thread, 4 threads per block.
+// MXFP8 row mode: 1x32 blocks along the contiguous dimension.  HBM bound.  A warp takes 1024 elements of one row (four
+// 16-byte loads in flight per lane), four neighbouring lanes hold one block.  `live` (optional, one word per row) names
+// the padding rows by a zero: they are neither read nor written, which at decode sizes is nearly all of them (64 routes
+// on 42 experts padded to 5376 rows of 2816: 15.6 -> 5.4 us).  4096 x 2816: 11.7 -> 8.4 us.
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(256) mxfp8_row_kernel(const uint4* __restrict__ x, const int32_t* num_rows,
                                                         int64_t max_rows, int vec_per_row, uint8_t* __restrict__ q,
                                                         int64_t q_stride, uint8_t* __restrict__ scales,
-                                                        int64_t s_stride, int blocked, int n_col_atoms) {
+                                                        int64_t s_stride, int blocked, int n_col_atoms,
+                                                        const int64_t* __restrict__ live) {
   int64_t rows = num_rows ? *num_rows : max_rows;
   if (rows > max_rows) rows = max_rows;
-  const int64_t total = rows * vec_per_row;
-  const int64_t start = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
-  const int64_t step = static_cast<int64_t>(gridDim.x) * blockDim.x;
-  // The bound is rounded up to a whole warp so that every lane takes part in the shuffles.
-  for (int64_t i = start; i < (total + 31) / 32 * 32; i += step) {
-    const bool live = i < total;
-    float f[8];
-    if (live) {
-      unpack8f(x[i], f);
-    } else {
+  const int lane = threadIdx.x & 31;
+  const int segs = (vec_per_row + 127) >> 7;
+  const int64_t items = rows * segs;
+  const int64_t warps = static_cast<int64_t>(gridDim.x) * (blockDim.x >> 5);
+  for (int64_t i = static_cast<int64_t>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5); i < items; i += warps) {
+    const int64_t r = segs == 1 ? i : i / segs;
+    if (live != nullptr && live[r] == 0) continue;
+    const int v0 = static_cast<int>(i - r * segs) * 128 + lane;
+    const uint4* xr = x + r * vec_per_row;
+    uint4 w[4];
 #pragma unroll
-      for (int j = 0; j < 8; ++j) f[j] = 0.f;
-    }
-    float amax = 0.f;
+    for (int j = 0; j < 4; ++j) w[j] = v0 + 32 * j < vec_per_row ? xr[v0 + 32 * j] : make_uint4(0, 0, 0, 0);
 #pragma unroll
-    for (int j = 0; j < 8; ++j) amax = amax_nonfinite(amax, f[j]);
-    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
-    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
-    float recip;
-    const uint8_t byte = mxfp8_scale(amax, recip);
-    if (!live) continue;
-    const int64_t r = i / vec_per_row;
-    const int v = static_cast<int>(i - r * vec_per_row);
-    *reinterpret_cast<uint2*>(q + r * q_stride + v * 8) =
-        make_uint2(e4m3x4(f[0] * recip, f[1] * recip, f[2] * recip, f[3] * recip),
-                   e4m3x4(f[4] * recip, f[5] * recip, f[6] * recip, f[7] * recip));
-    if ((v & 3) == 0) {
-      const int blk = v >> 2;
-      if (blocked)
-        scales[blocked_offset(r, blk, n_col_atoms)] = byte;
-      else
-        scales[r * s_stride + blk] = byte;
+    for (int j = 0; j < 4; ++j) {
+      const int v = v0 + 32 * j;
+      uint32_t m = __vmaxu2(__vmaxu2(w[j].x & 0x7fff7fffu, w[j].y & 0x7fff7fffu),
+                            __vmaxu2(w[j].z & 0x7fff7fffu, w[j].w & 0x7fff7fffu));
+      m = __vmaxu2(m, __shfl_xor_sync(0xffffffffu, m, 1));
+      m = __vmaxu2(m, __shfl_xor_sync(0xffffffffu, m, 2));
+      float recip;
+      const uint32_t byte = mxfp8_scale_bits((m >> 16) > (m & 0xffffu) ? m >> 16 : m & 0xffffu, recip);
+      if (v >= vec_per_row) continue;
+      float f[8];
+      unpack8f(w[j], f);
+      *reinterpret_cast<uint2*>(q + r * q_stride + static_cast<int64_t>(v) * 8) =
+          make_uint2(e4m3x2_scaled(f[0], f[1], recip, recip) | (e4m3x2_scaled(f[2], f[3], recip, recip) << 16),
+                     e4m3x2_scaled(f[4], f[5], recip, recip) | (e4m3x2_scaled(f[6], f[7], recip, recip) << 16));
+      if ((v & 3) == 0) {
+        const int blk = v >> 2;
+        if (blocked)
+          scales[blocked_offset(r, blk, n_col_atoms)] = static_cast<uint8_t>(byte);
+        else
+          scales[r * s_stride + blk] = static_cast<uint8_t>(byte);
+      }
     }
   }
 }
@@ -233,31 +263,6 @@ struct TileLane {
   __device__ __forceinline__ int row() const { return slab * 32 + rg * 8; }   // first row inside the tile
   __device__ __forceinline__ int col() const { return half * 64 + cg * 8; }   // first column inside the tile
 };
-
-// Scale byte and reciprocal of a block of bf16 values from the low 15 bits of its largest magnitude: the byte that
-// mxfp8_scale computes through fp32, in integers.  amax / 448 <= 2^(b - 127) holds for bf16 exactly when the
-// (exponent, mantissa) pair is <= (b + 8, 0x60), 448 being 1.75 * 2^8; bytes below 0 are 0, a non-finite block is 0xFF.
-__device__ __forceinline__ uint32_t mxfp8_scale_bits(uint32_t bits15, float& recip) {
-  const int b = static_cast<int>((bits15 + 0x1fu) >> 7) - 8;
-  const uint32_t byte = bits15 >= 0x7f80u ? 0xffu : static_cast<uint32_t>(b > 0 ? b : 0);
-  recip = byte == 0xffu ? __int_as_float(0x7fc00000) : __uint_as_float((254u - byte) << 23);
-  return byte;
-}
-
-// Products of two packed fp32 pairs (one instruction), as two E4M3 bytes.
-__device__ __forceinline__ uint32_t e4m3x2_scaled(float lo, float hi, float r_lo, float r_hi) {
-  float a, b;
-  asm("{\n\t"
-      ".reg .b64 x, y, z;\n\t"
-      "mov.b64 x, {%2, %3};\n\t"
-      "mov.b64 y, {%4, %5};\n\t"
-      "mul.rn.f32x2 z, x, y;\n\t"
-      "mov.b64 {%0, %1}, z;\n\t"
-      "}\n"
-      : "=f"(a), "=f"(b)
-      : "f"(lo), "f"(hi), "f"(r_lo), "f"(r_hi));
-  return __nv_cvt_float2_to_fp8x2(make_float2(a, b), __NV_SATFINITE, __NV_E4M3);
-}
 
 // Quantises the lane's 8 x 8 values (`w[r]` = row r, packed bf16, zeros outside the matrix) of the tile at
 // (row0, col0).  `limit` bounds the columns this tile may touch.  `atoms` is the CTA's 1 KiB of scale staging; called
@@ -630,57 +635,90 @@ __global__ void __launch_bounds__(128) nvfp4_token_kernel(const uint4* __restric
   }
 }
 
-// Rows of up to 2048 elements: one warp per row, the row stays in registers between the row-maximum pass and
-// the quantising pass (no second read, no block-wide barriers).  Same arithmetic as the kernel above.
-template <int kVpl>
-__global__ void __launch_bounds__(256) nvfp4_token_warp_kernel(const uint4* __restrict__ x, const int32_t* num_rows,
-                                                               int64_t max_rows, int vec_per_row, uint8_t* q,
-                                                               int64_t q_stride, uint8_t* s, int64_t s_stride,
-                                                               uint8_t* inv, int64_t inv_stride, int blocked_atoms,
-                                                               const int64_t* __restrict__ live) {
+// The form for rows that fit the registers of their threads: `kThreads` threads (a warp, or a CTA of 256) hold a whole
+// row, `kBpt` 16-element blocks per thread, between the row-maximum pass and the quantising pass.  A thread owns whole
+// blocks, so the scale (a division and two conversions) is computed once per block, without exchange between lanes.
+// Same arithmetic as the kernel above: block maxima are taken on the bf16 bit patterns (their order is the order of the
+// magnitudes, a NaN makes the block non-finite); the row maximum ignores NaNs, so a block that holds one is gone through
+// again.  Bound: HBM for long inputs (read once, 0.56 bytes per element written).  One B200: 65 536 x 2048 with padding
+// rows skipped 68 us (eight elements per lane, the scale computed twice per block: 113 us); 8192 x 7168 into packed
+// rows 30 us (a CTA of 128 reading the row twice: 49 us).
+template <int kThreads, int kBpt>
+__global__ void __launch_bounds__(256) nvfp4_token_reg_kernel(const uint4* __restrict__ x, const int32_t* num_rows,
+                                                              int64_t max_rows, int blocks_per_row, uint8_t* q,
+                                                              int64_t q_stride, uint8_t* s, int64_t s_stride,
+                                                              uint8_t* inv, int64_t inv_stride, int blocked_atoms,
+                                                              const int64_t* __restrict__ live) {
+  __shared__ float red[2][8];
   int64_t rows = num_rows ? *num_rows : max_rows;
   if (rows > max_rows) rows = max_rows;
-  const int lane = threadIdx.x & 31;
-  const int64_t warps = static_cast<int64_t>(gridDim.x) * (blockDim.x >> 5);
-  for (int64_t r = static_cast<int64_t>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5); r < rows; r += warps) {
+  constexpr int kRowsPerCta = 256 / kThreads;
+  const int t = threadIdx.x & (kThreads - 1), lane = threadIdx.x & 31;
+  const int64_t step = static_cast<int64_t>(gridDim.x) * kRowsPerCta;
+  const bool wide = ((reinterpret_cast<uintptr_t>(q) | static_cast<uintptr_t>(q_stride)) & 7) == 0;
+  int parity = 0;
+  for (int64_t r = static_cast<int64_t>(blockIdx.x) * kRowsPerCta + threadIdx.x / kThreads; r < rows; r += step) {
     if (live != nullptr && live[r] == 0) continue;  // a padding row: nothing reads its quantised form
-    const uint4* xr = x + r * vec_per_row;
-    uint4 raw[kVpl];
+    const uint4* xr = x + r * blocks_per_row * 2;
+    uint4 w[2 * kBpt];
+#pragma unroll
+    for (int j = 0; j < kBpt; ++j) {
+      const int b = j * kThreads + t;
+      const bool in = b < blocks_per_row;
+      w[2 * j] = in ? xr[2 * b] : make_uint4(0, 0, 0, 0);
+      w[2 * j + 1] = in ? xr[2 * b + 1] : make_uint4(0, 0, 0, 0);
+    }
+    uint32_t top[kBpt];
     float amax = 0.f;
 #pragma unroll
-    for (int j = 0; j < kVpl; ++j) {
-      const int v = j * 32 + lane;
-      raw[j] = v < vec_per_row ? xr[v] : make_uint4(0, 0, 0, 0);
-      float f[8];
-      unpack8f(raw[j], f);
+    for (int j = 0; j < kBpt; ++j) {
+      const uint32_t v[8] = {w[2 * j].x, w[2 * j].y, w[2 * j].z, w[2 * j].w,
+                             w[2 * j + 1].x, w[2 * j + 1].y, w[2 * j + 1].z, w[2 * j + 1].w};
+      uint32_t m = 0;
 #pragma unroll
-      for (int i = 0; i < 8; ++i) amax = fmaxf(amax, fabsf(f[i]));
+      for (int i = 0; i < 8; ++i) m = __vmaxu2(m, v[i] & 0x7fff7fffu);
+      top[j] = (m >> 16) > (m & 0xffffu) ? m >> 16 : m & 0xffffu;
+      if (top[j] <= 0x7f80u) {
+        amax = fmaxf(amax, __uint_as_float(top[j] << 16));
+      } else {
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+          amax = fmaxf(amax, fmaxf(fabsf(__uint_as_float(v[i] << 16)), fabsf(__uint_as_float(v[i] & 0xffff0000u))));
+      }
     }
 #pragma unroll
     for (int d = 16; d > 0; d >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, d));
+    if (kThreads > 32) {
+      // two sets of partial maxima in turn: one barrier per row is enough
+      if (lane == 0) red[parity][threadIdx.x >> 5] = amax;
+      __syncthreads();
+#pragma unroll
+      for (int i = 0; i < 8; ++i) amax = fmaxf(amax, red[parity][i]);
+      parity ^= 1;
+    }
     const float row_scale = 2688.0f * __frcp_rn(fmaxf(amax, 1e-8f));
-    if (lane == 0 && inv != nullptr) *reinterpret_cast<float*>(inv + r * inv_stride) = __frcp_rn(row_scale);
+    if (t == 0 && inv != nullptr) *reinterpret_cast<float*>(inv + r * inv_stride) = __frcp_rn(row_scale);
 #pragma unroll
-    for (int j = 0; j < kVpl; ++j) {
-      const int v = j * 32 + lane;
-      float f[8];
-      unpack8f(raw[j], f);
-      float bmax = 0.f;
-#pragma unroll
-      for (int i = 0; i < 8; ++i) bmax = amax_nonfinite(bmax, f[i]);
-      const float other = __shfl_xor_sync(0xffffffffu, bmax, 1);
-      bmax = (other != other) ? other : fmaxf(bmax, other);
+    for (int j = 0; j < kBpt; ++j) {
+      const int b = j * kThreads + t;
+      if (b >= blocks_per_row) continue;
       float mult;
-      const uint8_t byte = nvfp4_block_scale(bmax, row_scale, mult);
-      if (v < vec_per_row) {
-        *reinterpret_cast<uint32_t*>(q + r * q_stride + v * 4) = e2m1x8(f, mult);
-        if ((v & 1) == 0) {
-          if (blocked_atoms > 0)
-            s[blocked_offset(r, v >> 1, blocked_atoms)] = byte;
-          else
-            s[r * s_stride + (v >> 1)] = byte;
-        }
+      const uint8_t byte = nvfp4_block_scale(amax_from_bf16_bits(top[j]), row_scale, mult);
+      float f[8], g[8];
+      unpack8f(w[2 * j], f);
+      unpack8f(w[2 * j + 1], g);
+      uint32_t* dst = reinterpret_cast<uint32_t*>(q + r * q_stride + b * 8);
+      const uint32_t lo = e2m1x8(f, mult), hi = e2m1x8(g, mult);
+      if (wide) {
+        *reinterpret_cast<uint2*>(dst) = make_uint2(lo, hi);
+      } else {
+        dst[0] = lo;
+        dst[1] = hi;
       }
+      if (blocked_atoms > 0)
+        s[blocked_offset(r, b, blocked_atoms)] = byte;
+      else
+        s[r * s_stride + b] = byte;
     }
   }
 }
@@ -739,6 +777,13 @@ __global__ void sf_swizzle_kernel(const uint8_t* __restrict__ src, uint8_t* __re
 // Packed dispatch rows [q | natural scales | fp32 inverse scale | pad] fetched through a pointer table
 // (sources may be peer memory) and unpacked into GEMM operand form: dense q rows, blocked scales,
 // per-row inverse scales.  A null pointer yields a zero row.
+//
+// Bound: HBM writes (the source rows of a rank fit L2).  A warp copies rows in pieces of 128 vectors.  The scales of a
+// 128-row block are written in whole 32-byte sectors: a lane reads one atom's word of the rows l, l + 32, l + 64, l + 96
+// and of their neighbours l + 1 ... (128 contiguous bytes of every row per warp, which is also what peer reads want) and
+// stores the atom's bytes of both.  A word per row and atom, each in a sector of its own, made 65 536 rows of 448 scales
+// take 101 us in all; 76 us now.  The last, partial block of a row count that is no multiple of 128 takes the
+// word-wise form.
 __global__ void __launch_bounds__(256) gather_packed_kernel(const int64_t* __restrict__ ptrs,
                                                             const int32_t* __restrict__ num_rows, int64_t max_rows,
                                                             int q_vecs, int scale_cols, int has_inv, uint8_t* q_base,
@@ -752,34 +797,55 @@ __global__ void __launch_bounds__(256) gather_packed_kernel(const int64_t* __res
   uint8_t* sf = sf_base + (sf_off ? *sf_off : 0);
   float* inv = has_inv ? reinterpret_cast<float*>(inv_base + (inv_off ? *inv_off : 0)) : nullptr;
   const int atoms = (scale_cols + 3) / 4;
-  const int lane = threadIdx.x & 31, wpb = blockDim.x >> 5;
-  for (int64_t r = blockIdx.x * static_cast<int64_t>(wpb) + (threadIdx.x >> 5); r < rows;
-       r += static_cast<int64_t>(gridDim.x) * wpb) {
-    const uint8_t* src = reinterpret_cast<const uint8_t*>(ptrs[r]);
-    for (int v0 = lane; v0 < q_vecs; v0 += 128) {  // four 16-byte loads in flight per lane
-      uint4 t[4];
+  const int lane = threadIdx.x & 31;
+  const int64_t first = static_cast<int64_t>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  const int64_t warps = static_cast<int64_t>(gridDim.x) * (blockDim.x >> 5);
+  const bool whole_atoms = (reinterpret_cast<uintptr_t>(sf) & 15) == 0;
+  // scale tasks first (eight rows of one 128-row block, 32 atoms), then row pieces
+  const int chunks = (atoms + 31) >> 5;
+  const int64_t blocks = whole_atoms ? rows >> 7 : 0;
+  for (int64_t i = first; i < blocks * 16 * chunks; i += warps) {
+    const int64_t pair = i / chunks;
+    const int c4 = static_cast<int>(i - pair * chunks) * 32 + lane;
+    const int64_t blk = pair >> 4;
+    const int l0 = static_cast<int>(pair & 15) * 2;
+    uint32_t w[2][4];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int v = v0 + 32 * j;
-        t[j] = (src && v < q_vecs) ? __ldcg(reinterpret_cast<const uint4*>(src) + v) : make_uint4(0, 0, 0, 0);
-      }
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int v = v0 + 32 * j;
-        if (v < q_vecs) q[r * q_vecs + v] = t[j];
-      }
+    for (int g = 0; g < 8; ++g) {
+      const int64_t src = ptrs[blk * 128 + 32 * (g >> 1) + l0 + (g & 1)];
+      w[g & 1][g >> 1] = (src != 0 && c4 < atoms)
+                             ? __ldcg(reinterpret_cast<const uint32_t*>(src + static_cast<int64_t>(q_vecs) * 16) + c4)
+                             : 0;
     }
+    if (c4 < atoms) {
+      uint4* dst = reinterpret_cast<uint4*>(sf + (blk * atoms + c4) * 512) + l0;
+      dst[0] = make_uint4(w[0][0], w[0][1], w[0][2], w[0][3]);
+      dst[1] = make_uint4(w[1][0], w[1][1], w[1][2], w[1][3]);
+    }
+  }
+  const int pieces = (q_vecs + 127) >> 7;
+  for (int64_t i = first; i < rows * pieces; i += warps) {
+    const int64_t r = pieces == 1 ? i : i / pieces;
+    const int piece = static_cast<int>(i - r * pieces);
+    const uint8_t* src = reinterpret_cast<const uint8_t*>(ptrs[r]);
+    const int v0 = piece * 128 + lane;
+    uint4 t[4];  // four 16-byte loads in flight per lane
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int v = v0 + 32 * j;
+      t[j] = (src && v < q_vecs) ? __ldcg(reinterpret_cast<const uint4*>(src) + v) : make_uint4(0, 0, 0, 0);
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int v = v0 + 32 * j;
+      if (v < q_vecs) q[r * q_vecs + v] = t[j];
+    }
+    if (piece != 0) continue;
     const uint8_t* ssrc = src ? src + static_cast<int64_t>(q_vecs) * 16 : nullptr;
-    for (int c4 = lane; c4 < atoms; c4 += 32) {
-      uint32_t w = 0;
-      if (ssrc) {
-        if (c4 * 4 + 4 <= scale_cols) {
-          w = __ldcg(reinterpret_cast<const uint32_t*>(ssrc) + c4);
-        } else {
-          for (int j = 0; c4 * 4 + j < scale_cols; ++j) w |= static_cast<uint32_t>(ssrc[c4 * 4 + j]) << (8 * j);
-        }
-      }
-      *reinterpret_cast<uint32_t*>(sf + blocked_offset(r, c4 * 4, atoms)) = w;
+    if ((r >> 7) >= blocks) {
+      for (int c4 = lane; c4 < atoms; c4 += 32)
+        *reinterpret_cast<uint32_t*>(sf + blocked_offset(r, c4 * 4, atoms)) =
+            ssrc ? __ldcg(reinterpret_cast<const uint32_t*>(ssrc) + c4) : 0;
     }
     if (inv != nullptr && lane == 0)
       inv[r] = src ? __ldcg(reinterpret_cast<const float*>(ssrc + scale_cols)) : 0.f;
@@ -803,9 +869,8 @@ static int blocks_for(int64_t items, int threads, int cap) {
 
 using namespace dm;
 
-extern "C" int dm_quant_mxfp8_row(const void* x, const int32_t* num_rows, int64_t max_rows, int64_t C, void* q,
-                                  int64_t q_row_stride, void* scales, int64_t scale_row_stride, int blocked,
-                                  void* stream) {
+static int mxfp8_row_impl(const int64_t* live, const void* x, const int32_t* num_rows, int64_t max_rows, int64_t C, void* q,
+                          int64_t q_row_stride, void* scales, int64_t scale_row_stride, int blocked, void* stream) {
   if (!x || !q || !scales || max_rows < 0 || C <= 0 || (C % 32) != 0) return kRcBadArg;
   if (q_row_stride == 0) q_row_stride = C;
   if (scale_row_stride == 0) scale_row_stride = C / 32;
@@ -813,10 +878,23 @@ extern "C" int dm_quant_mxfp8_row(const void* x, const int32_t* num_rows, int64_
   if (max_rows == 0) return kRcOk;
   const int vec = static_cast<int>(C / 8);
   const int atoms = static_cast<int>((C / 32 + 3) / 4);
-  mxfp8_row_kernel<<<blocks_for(max_rows * vec, 256, grid_cap(16)), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+  mxfp8_row_kernel<<<blocks_for(max_rows * ((vec + 127) / 128), 8, grid_cap(8)), 256, 0, static_cast<cudaStream_t>(stream)>>>(
       static_cast<const uint4*>(x), num_rows, max_rows, vec, static_cast<uint8_t*>(q), q_row_stride,
-      static_cast<uint8_t*>(scales), scale_row_stride, blocked, atoms);
+      static_cast<uint8_t*>(scales), scale_row_stride, blocked, atoms, live);
   return static_cast<int>(cudaGetLastError());
+}
+
+extern "C" int dm_quant_mxfp8_row(const void* x, const int32_t* num_rows, int64_t max_rows, int64_t C, void* q,
+                                  int64_t q_row_stride, void* scales, int64_t scale_row_stride, int blocked,
+                                  void* stream) {
+  return mxfp8_row_impl(nullptr, x, num_rows, max_rows, C, q, q_row_stride, scales, scale_row_stride, blocked, stream);
+}
+
+extern "C" int dm_quant_mxfp8_row_live(const int64_t* row_live, const void* x, const int32_t* num_rows, int64_t max_rows,
+                                       int64_t C, void* q, int64_t q_row_stride, void* scales, int64_t scale_row_stride,
+                                       int blocked, void* stream) {
+  if (!row_live) return kRcBadArg;
+  return mxfp8_row_impl(row_live, x, num_rows, max_rows, C, q, q_row_stride, scales, scale_row_stride, blocked, stream);
 }
 
 extern "C" int dm_quant_mxfp8_col(const void* x, const int32_t* num_rows, int64_t max_rows, int64_t C, void* q,
@@ -983,26 +1061,29 @@ static int nvfp4_token_impl(const int64_t* live, const void* x, const int32_t* n
   if (!x || !q || !scales || max_rows < 0 || C <= 0 || (C % 16) != 0 || (q_row_stride % 4) != 0) return kRcBadArg;
   if (scale_inv && (inv_row_stride % 4) != 0) return kRcBadArg;
   if (max_rows == 0) return kRcOk;
-  const int vec = static_cast<int>(C / 8);
-  if (vec <= 256) {
-    const int atoms = scales_blocked ? static_cast<int>((C / 16 + 3) / 4) : 0;
-    const int blocks = blocks_for(max_rows, 8, grid_cap(8));
-    cudaStream_t st = static_cast<cudaStream_t>(stream);
-#define DM_TOKEN_WARP(VPL)                                                                                            \
-    nvfp4_token_warp_kernel<VPL><<<blocks, 256, 0, st>>>(static_cast<const uint4*>(x), num_rows, max_rows, vec,         \
-                                                         static_cast<uint8_t*>(q), q_row_stride,                        \
-                                                         static_cast<uint8_t*>(scales), scale_row_stride,               \
-                                                         static_cast<uint8_t*>(scale_inv), inv_row_stride, atoms, live)
-    if (vec <= 64) {
-      DM_TOKEN_WARP(2);
-    } else if (vec <= 128) {
-      DM_TOKEN_WARP(4);
-    } else {
-      DM_TOKEN_WARP(8);
-    }
-#undef DM_TOKEN_WARP
+  // Up to 2048 elements a warp holds the row, up to 8192 a CTA does (launched with as many blocks per thread as the row
+  // needs); longer rows are read twice.
+  const int blocks = static_cast<int>(C / 16);
+  const int atoms = scales_blocked ? static_cast<int>((C / 16 + 3) / 4) : 0;
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+#define DM_TOKEN(THREADS, BPT)                                                                                       \
+  nvfp4_token_reg_kernel<THREADS, BPT><<<blocks_for(max_rows, 256 / THREADS, grid_cap(8)), 256, 0, st>>>(              \
+      static_cast<const uint4*>(x), num_rows, max_rows, blocks, static_cast<uint8_t*>(q), q_row_stride,                \
+      static_cast<uint8_t*>(scales), scale_row_stride, static_cast<uint8_t*>(scale_inv), inv_row_stride, atoms, live)
+  if (blocks <= 512) {
+    if (blocks <= 32)
+      DM_TOKEN(32, 1);
+    else if (blocks <= 64)
+      DM_TOKEN(32, 2);
+    else if (blocks <= 128)
+      DM_TOKEN(32, 4);
+    else if (blocks <= 256)
+      DM_TOKEN(256, 1);
+    else
+      DM_TOKEN(256, 2);
     return static_cast<int>(cudaGetLastError());
   }
+#undef DM_TOKEN
   nvfp4_token_kernel<<<blocks_for(max_rows, 1, grid_cap(16)), 128, 0, static_cast<cudaStream_t>(stream)>>>(
       static_cast<const uint4*>(x), num_rows, max_rows, static_cast<int>(C / 8), static_cast<uint8_t*>(q),
       q_row_stride, static_cast<uint8_t*>(scales), scale_row_stride, static_cast<uint8_t*>(scale_inv),
@@ -1054,7 +1135,7 @@ extern "C" int dm_gather_packed_rows(const int64_t* ptrs, const int32_t* num_row
     return kRcBadArg;
   if (has_inv && !scale_inv.base) return kRcBadArg;
   if (max_rows == 0) return kRcOk;
-  gather_packed_kernel<<<blocks_for(max_rows * 32, 256, grid_cap(8)), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+  gather_packed_kernel<<<blocks_for(max_rows * ((q_bytes / 16 + 127) / 128), 8, grid_cap(8)), 256, 0, static_cast<cudaStream_t>(stream)>>>(
       ptrs, num_rows, max_rows, static_cast<int>(q_bytes / 16), static_cast<int>(scale_cols), has_inv,
       static_cast<uint8_t*>(q.base), q.offset, static_cast<uint8_t*>(scales_blocked.base), scales_blocked.offset,
       static_cast<uint8_t*>(scale_inv.base), scale_inv.offset, cond);

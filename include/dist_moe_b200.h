@@ -429,6 +429,10 @@ int dm_rmsnorm_combine_bwd(const void* grad_out, const void* scores, int scores_
  * ------------------------------------------------------------------------- */
 int dm_quant_mxfp8_row(const void* x, const int32_t* num_rows, int64_t max_rows, int64_t C, void* q,
                        int64_t q_row_stride, void* scales, int64_t scale_row_stride, int blocked, void* stream);
+/* dm_quant_mxfp8_row restricted to the rows r with row_live[r] != 0, as dm_quant_nvfp4_token_live below. */
+int dm_quant_mxfp8_row_live(const int64_t* row_live, const void* x, const int32_t* num_rows, int64_t max_rows, int64_t C,
+                            void* q, int64_t q_row_stride, void* scales, int64_t scale_row_stride, int blocked,
+                            void* stream);
 int dm_quant_mxfp8_col(const void* x, const int32_t* num_rows, int64_t max_rows, int64_t C, void* q, void* scales,
                        int blocked, void* stream);
 /* Row- and column-quantised copies of one bf16 [rows, C] matrix in a single pass over the input (the pair the

@@ -349,3 +349,95 @@ def test_mxfp8_rowcol_tile_edges_against_the_oracle(rows, cols, gather, offset):
     assert int(qr.view(cap, cols)[rows:].sum()) == 0 and int(qc.view(cap, cols)[rows:].sum()) == 0
     assert int((sr.cpu() == 0xEE).sum()) >= n_rs - rs.size
     assert int((sc.cpu() == 0xEE).sum()) >= n_cs - cs.size
+
+
+@pytest.mark.parametrize("rows,cols", [(70, 16), (33, 512), (40, 528), (35, 1040), (21, 2064), (12, 4112), (9, 8192), (6, 8208)])
+def test_nvfp4_token_row_lengths_at_the_limits_of_the_register_forms(rows, cols):
+    """The warp-per-row (up to 2048 elements), CTA-per-row (8192) and two-pass forms, with an all-zero row and blocks that
+    hold infinities; packed bytes, block scales and inverse row scales equal the oracle's.  A NaN leaves the row's scale
+    to the other elements."""
+    nat = _nat()
+    x = _data(rows, cols, rows + cols, specials=False)
+    x[1] = 0
+    rp, rs, rinv = Q.nvfp4_token_rows(x)
+    xn = x.clone()
+    xn[2, cols - 1] = float("nan")
+    amax = torch.nan_to_num(xn[2].float(), nan=0.0).abs().max()
+
+    def run(t):
+        q = torch.zeros(rows, cols // 2, dtype=torch.uint8, device=DEV)
+        s = torch.zeros(rows, cols // 16, dtype=torch.uint8, device=DEV)
+        inv = torch.zeros(rows, dtype=torch.float32, device=DEV)
+        nat.check(nat.lib.dm_quant_nvfp4_token(t.to(DEV).data_ptr(), None, rows, cols, q.data_ptr(), cols // 2, s.data_ptr(),
+                                               cols // 16, 0, inv.data_ptr(), 4, nat.stream_ptr()), "nvfp4_token")
+        torch.cuda.synchronize()
+        return q.cpu().numpy(), s.cpu().numpy(), inv.cpu().numpy()
+
+    q, s, inv = run(x)
+    np.testing.assert_array_equal(inv.view(np.uint32), rinv.view(np.uint32))
+    np.testing.assert_array_equal(s, rs)
+    np.testing.assert_array_equal(q, rp)
+    q, s, inv = run(xn)
+    assert abs(inv[2] * 2688.0 / float(amax) - 1.0) < 1e-6
+    others = np.arange(rows) != 2
+    np.testing.assert_array_equal(q[others], rp[others])
+    np.testing.assert_array_equal(s[others], rs[others])
+
+
+@pytest.mark.parametrize("rows,q_bytes,scale_cols,has_inv", [(1, 16, 4, 0), (128, 2064, 132, 1), (200, 2816, 88, 0), (384, 3584, 448, 1)])
+def test_gather_packed_rows_unpacks_every_row_and_atom(rows, q_bytes, scale_cols, has_inv):
+    """Whole 128-row blocks (written sector by sector) and a partial last one, atom counts around a warp's 32, null
+    pointers as rows of zeros; plain copies of bytes: equal."""
+    nat = _nat()
+    stride = (q_bytes + scale_cols + 4 * has_inv + 15) // 16 * 16
+    g = torch.Generator().manual_seed(rows)
+    packed = torch.randint(0, 256, (rows, stride), dtype=torch.uint8, generator=g)
+    perm = torch.randperm(rows, generator=g)
+    null = torch.arange(rows) % 6 == 4
+    src = packed.to(DEV)
+    ptrs = torch.where(null, 0, src.data_ptr() + perm * stride).to(DEV)
+    cap = rows + 5
+    atoms = scale_cols // 4
+    q = torch.full((cap, q_bytes), 0xEE, dtype=torch.uint8, device=DEV)
+    sf = torch.full(((cap + 127) // 128 * 128 * scale_cols,), 0xEE, dtype=torch.uint8, device=DEV)
+    inv = torch.full((cap, 4), 0xEE, dtype=torch.uint8, device=DEV)
+    cnt = torch.tensor([rows], dtype=torch.int32, device=DEV)
+    op = lambda t: nat.Operand(t.data_ptr(), t.numel(), None)  # noqa: E731
+    ptrs_cap = torch.cat([ptrs, torch.zeros(5, dtype=torch.int64, device=DEV)])
+    nat.check(nat.lib.dm_gather_packed_rows(ptrs_cap.data_ptr(), cnt.data_ptr(), cap, q_bytes, scale_cols, has_inv, op(q), op(sf),
+                                            op(inv) if has_inv else nat.Operand(None, 0, None), None, nat.stream_ptr()), "gather")
+    torch.cuda.synchronize()
+    want = packed[perm].clone()
+    want[null] = 0
+    np.testing.assert_array_equal(q.cpu().numpy()[:rows], want[:, :q_bytes].numpy())
+    r, c = np.meshgrid(np.arange(rows), np.arange(scale_cols), indexing="ij")
+    got = sf.cpu().numpy()
+    np.testing.assert_array_equal(got[Q.blocked_scale_offset(r, c, atoms)], want[:, q_bytes: q_bytes + scale_cols].numpy())
+    if has_inv:
+        np.testing.assert_array_equal(inv.cpu().numpy()[:rows], want[:, q_bytes + scale_cols: q_bytes + scale_cols + 4].numpy())
+    assert bool((q[rows:] == 0xEE).all())
+    assert int((got == 0xEE).sum()) >= got.size - rows * scale_cols
+
+
+@pytest.mark.parametrize("rows,cols", [(4, 32), (37, 1056), (64, 2816)])
+def test_mxfp8_row_live_rows_only(rows, cols):
+    """dm_quant_mxfp8_row_live quantises the rows whose table entry is non-zero exactly as the plain call does and leaves
+    the others untouched; the plain call equals the oracle on the same rows."""
+    nat = _nat()
+    st = nat.stream_ptr()
+    x = _data(rows, cols, rows + 5)
+    xd = x.to(DEV)
+    live = torch.tensor([0 if r % 3 == 1 else 1000 + r for r in range(rows)], dtype=torch.int64, device=DEV)
+    want, got = ((torch.full((rows, cols), 0xAB, dtype=torch.uint8, device=DEV),
+                  torch.full((rows, cols // 32), 0xAB, dtype=torch.uint8, device=DEV)) for _ in range(2))
+    nat.check(nat.lib.dm_quant_mxfp8_row(xd.data_ptr(), None, rows, cols, want[0].data_ptr(), 0, want[1].data_ptr(), 0, 0, st), "plain")
+    nat.check(nat.lib.dm_quant_mxfp8_row_live(live.data_ptr(), xd.data_ptr(), None, rows, cols, got[0].data_ptr(), 0,
+                                              got[1].data_ptr(), 0, 0, st), "live")
+    torch.cuda.synchronize()
+    rq, rs = Q.mxfp8_row(x)
+    np.testing.assert_array_equal(want[1].cpu().numpy(), rs)
+    finite = np.repeat(rs != 255, 32, axis=1)
+    np.testing.assert_array_equal(want[0].cpu().numpy()[finite], rq[finite])
+    keep = live != 0
+    for g, w in zip(got, want):
+        assert torch.equal(g[keep], w[keep]) and bool((g[~keep] == 0xAB).all())

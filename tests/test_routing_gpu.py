@@ -148,3 +148,9 @@ def test_single_launch_decode_routing_equals_the_general_path_and_the_oracle(ep,
         np.testing.assert_array_equal(outs[1]["per_rank"], t.per_rank)
         np.testing.assert_array_equal(outs[1]["fwd"][:rows], t.fwd)
         np.testing.assert_array_equal(outs[1]["sct"][:rows], t.sct)
+
+
+@pytest.mark.parametrize("ep,T,K,E,m_mult", [(1, 70, 11, 37, 128), (1, 31, 9, 33, 0), (2, 33, 17, 66, 128)])
+def test_decode_routing_with_expert_and_id_counts_off_the_warp_and_load_steps(ep, T, K, E, m_mult):
+    """Local expert counts just above a scan step of 32 and ids per token that are no multiple of the eight loaded at once."""
+    test_single_launch_decode_routing_equals_the_general_path_and_the_oracle(ep, T, K, E, m_mult)
