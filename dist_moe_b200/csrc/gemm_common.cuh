@@ -46,6 +46,33 @@ __device__ __forceinline__ uint32_t mbar_poll(uint32_t bar_addr, uint32_t parity
       : "=r"(ok) : "r"(bar_addr), "r"(parity) : "memory");
   return ok;
 }
+// ---------------------------------------------------------------------------
+// Issuing warps.  tcgen05 and TMA instructions take their operands from uniform registers.  Code that only one lane runs
+// (`if (lane == 0)`) keeps everything in per-lane registers and moves each operand over for each instruction: 85 to 93
+// cycles per tcgen05.mma, measured.  The issuing warps here stay converged instead: all lanes walk the loop, values that
+// come from memory are made uniform with a shuffle, and only the instruction itself is behind the elected lane's
+// predicate: 39 cycles per tcgen05.mma of N <= 32 with its share of the loop, and N / 2 from N = 128 up (the pipe's rate).
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ uint32_t uniform(uint32_t v) { return __shfl_sync(0xffffffffu, v, 0); }
+__device__ __forceinline__ int uniform(int v) { return __shfl_sync(0xffffffffu, v, 0); }
+// Bounded wait of a whole converged warp; every lane has seen the phase complete when it returns true.
+__device__ __forceinline__ bool warp_mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag));
+}
+
+// One look at a barrier that never suspends the thread: asked for the next stage before this stage's MMAs are issued, its
+// latency hides behind them.
+__device__ __forceinline__ uint32_t mbar_test(uint32_t bar_addr, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t"
+      ".reg .pred p;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t"
+      "}\n"
+      : "=r"(ok) : "r"(bar_addr), "r"(parity) : "memory");
+  return ok;
+}
 // A bare polling loop (a million polls, tens of milliseconds), then the timed wait that can give up.
 __device__ __forceinline__ bool mbar_wait_lean(uint32_t bar_addr, uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
   for (uint32_t i = 0; i < (1u << 20); ++i)
@@ -68,6 +95,80 @@ __device__ __forceinline__ void umma_bf16_lo(uint32_t d_tmem, uint32_t a_lo, uin
 }
 __device__ __forceinline__ void tcgen05_commit_addr(uint32_t bar_addr) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar_addr) : "memory");
+}
+
+// ---------------------------------------------------------------------------
+// CTA pairs (clusters of two, tcgen05 cta_group::2).  The even CTA leads: it issues the MMAs of both, and its stage
+// barriers count the bytes that both CTAs load, each into its own shared memory.  No load is multicast.
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ uint32_t cluster_ctarank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+// Address of the same shared-memory location in CTA `rank` of the cluster.
+__device__ __forceinline__ uint32_t cluster_addr(uint32_t smem_addr, uint32_t rank) {
+  uint32_t a;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_addr), "r"(rank));
+  return a;
+}
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_bar) {
+  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
+}
+__device__ __forceinline__ void tmem_alloc_pair(uint32_t* smem_dst, uint32_t ncols) {
+  asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(smem_dst)), "r"(ncols)
+               : "memory");
+}
+__device__ __forceinline__ void tmem_relinquish_pair() {
+  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t ncols) {
+  asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
+}
+// Loads whose bytes count on the leader's barrier (`bar`: its shared::cluster address).
+__device__ __forceinline__ void tma_load_2d_pair(void* smem_dst, const void* tmap, int x, int y, uint32_t bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
+      ::"r"(smem_u32(smem_dst)), "l"(tmap), "r"(bar), "r"(x), "r"(y)
+      : "memory");
+}
+__device__ __forceinline__ void tma_load_3d_pair(void* smem_dst, const void* tmap, int x, int y, int z, uint32_t bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
+      ::"r"(smem_u32(smem_dst)), "l"(tmap), "r"(bar), "r"(x), "r"(y), "r"(z)
+      : "memory");
+}
+__device__ __forceinline__ void tma_load_5d_pair(void* smem_dst, const void* tmap, int c0, int c1, int c2, int c3, int c4,
+                                                 uint32_t bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.5d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6, "
+      "%7}], [%2];"
+      ::"r"(smem_u32(smem_dst)), "l"(tmap), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4)
+      : "memory");
+}
+__device__ __forceinline__ void umma_bf16_lo_pair(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t desc_hi,
+                                                  uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t"
+      ".reg .pred p;\n\t"
+      ".reg .b64 da, db;\n\t"
+      "setp.ne.b32 p, %5, 0;\n\t"
+      "mov.b64 da, {%1, %3};\n\t"
+      "mov.b64 db, {%2, %3};\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], da, db, %4, p;\n\t"
+      "}\n"
+      ::"r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(desc_hi), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+// Arrive on the barrier at this shared-memory offset in both CTAs of the pair once the MMAs issued so far are complete.
+__device__ __forceinline__ void tcgen05_commit_pair(uint32_t bar_addr) {
+  asm volatile(
+      "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar_addr),
+      "h"(static_cast<uint16_t>(3))
+      : "memory");
 }
 
 // Bulk tensor store and reduce-add of one staged box (shared memory -> global), issued by one thread.  The
@@ -107,6 +208,36 @@ static inline EncodeTiledFn get_encode() {
       fn = reinterpret_cast<EncodeTiledFn>(sym);
   }
   return fn;
+}
+
+// Grid of a persistent kernel of CTA pairs, one CTA per SM: the caller's wish, never more pairs than the device can hold
+// at once (CTAs wait on counters that other CTAs publish, so every one of them must be resident).
+template <class Kernel>
+static inline int pair_grid(Kernel kernel, int threads, size_t smem, int num_sms) {
+  static int resident[kMaxDevices] = {};  // per kernel signature; kernels that share one share their launch shape
+  const int slot = current_device_slot();
+  int clusters = slot >= 0 ? resident[slot] : 0;
+  if (clusters <= 0) {
+    cudaLaunchConfig_t cfg{};
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = 2;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cfg.gridDim = dim3(static_cast<unsigned>(sm_count() / 2 * 2));
+    cfg.blockDim = dim3(static_cast<unsigned>(threads));
+    cfg.dynamicSmemBytes = smem;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    if (cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) != cudaSuccess || clusters <= 0) {
+      cudaGetLastError();
+      clusters = sm_count() / 2;
+    }
+    if (clusters > sm_count() / 2) clusters = sm_count() / 2;
+    if (slot >= 0) resident[slot] = clusters;
+  }
+  const int wish = persistent_grid(num_sms) / 2;
+  const int n = wish < clusters ? wish : clusters;
+  return 2 * (n > 0 ? n : 1);
 }
 
 // bf16 matrix [rows][cols], cols contiguous; box = box_rows x 64 columns.

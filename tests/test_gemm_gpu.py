@@ -297,3 +297,19 @@ def test_fused_dispatch_gathers_rows_inside_the_gemm(mode):
             if hi > lo:
                 wt = w[ei].float().T if mode == "fprop" else w[ei].float()
                 _close(out[lo:hi], a_ref[lo:hi].float() @ wt, f"{mode} dispatch expert {ei}")
+
+
+@pytest.mark.parametrize("counts,kd,n", [
+    ([1, 31, 32, 33], 64, 64),           # one stage; tiles of 32 rows, a column block past the matrix in either CTA
+    ([255, 0, 256, 257], 192, 392),      # tiles of 256 and 160 rows; a width that is only a multiple of 8
+    ([513, 96, 5], 704, 1152),           # three tiles of 192, 192, 129 rows; more stages than the ring holds
+])
+def test_row_tiles_at_their_edges(counts, kd, n):
+    """Splits of an expert's rows into equal tiles of a multiple of 32 and output widths around the 256-column pair."""
+    test_fprop_matches_torch(counts, kd, n)
+    test_dgrad_matches_torch(counts, kd, n)
+
+
+@pytest.mark.parametrize("counts,kd,n", [([1, 32, 33, 257], 64, 256), ([300, 0, 191], 320, 768)])
+def test_fused_swiglu_row_tiles_at_their_edges(counts, kd, n):
+    test_fprop_fused_swiglu(counts, kd, n)
