@@ -115,8 +115,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1) wgrad_gemm_kernel(const __gri
   tcgen05_fence_before();
   __syncthreads();
   tcgen05_fence_after();
-  const uint32_t tmem_base = tmem_base_slot;
-  const int total_tiles = s_tile_start[p.e_local];
+  const uint32_t tmem_base = uniform(tmem_base_slot);
+  const int total_tiles = uniform(s_tile_start[p.e_local]);
 
   const int64_t a_off = p.a_off ? *p.a_off : 0;
   const int64_t b_off = p.b_off ? *p.b_off : 0;
@@ -127,36 +127,31 @@ __global__ void __launch_bounds__(kGemmThreads, 1) wgrad_gemm_kernel(const __gri
   const int wgrad_part = warp == 0 ? 0 : (warp == 10 ? 1 : (warp == 11 ? 2 : -1));
   if (warp == 0 || wgrad_part > 0) {
     // ======================= TMA producer =======================
+    const bool elected = elect_one();
     int stage = 0;
     uint32_t phase = 0;
     int e = 0;
-    const int a_line0 = static_cast<int>(a_off >> 7);
-    const int b_line0 = static_cast<int>(b_off >> 7);
+    const int a_line0 = uniform(static_cast<int>(a_off >> 7));
+    const int b_line0 = uniform(static_cast<int>(b_off >> 7));
     bool ok = true;
     for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
       const Tile t = decode_tile(tile, e, s_tile_start, s_off, n_tiles);
-      for (int kb = 0; kb < t.k_iters; ++kb) {
-        if (lane == 0) {
-          ok = mbar_wait(&empty_bar[stage], phase ^ 1u, &abort_flag);
-          if (ok) {
-            uint8_t* sa = smem + stage * kStageBytes;
-            uint8_t* sb = sa + kABytes;
-            if (wgrad_part == 0) mbar_arrive_expect_tx(&full_bar[stage], kStageBytes);
-            const int row = t.row0 + kb * kBK;
-            if (wgrad_part == 0) {
-#pragma unroll
-              for (int b = 0; b < kBM / 64; ++b)
-                tma_load_3d(sa + b * 8192, &p.tm_a, 0, a_line0 + t.m_blk * (kBM / 64) + b, row, &full_bar[stage]);
-            } else {
-              const int b0 = (wgrad_part - 1) * 2;
-#pragma unroll
-              for (int b = b0; b < b0 + 2; ++b)
-                tma_load_3d(sb + b * 8192, &p.tm_b, 0, b_line0 + t.n_blk * (kBN / 64) + b, row, &full_bar[stage]);
-            }
-          }
-        }
-        ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
+      const int k_iters = uniform(t.k_iters), row0 = uniform(t.row0);
+      const int line = wgrad_part == 0 ? a_line0 + uniform(t.m_blk) * (kBM / 64)
+                                       : b_line0 + uniform(t.n_blk) * (kBN / 64) + (wgrad_part - 1) * 2;
+      const uint32_t dst = wgrad_part == 0 ? 0u : kABytes + (wgrad_part - 1) * 16384u;
+      const CUtensorMap* map = wgrad_part == 0 ? &p.tm_a : &p.tm_b;
+#pragma unroll 1
+      for (int kb = 0; kb < k_iters; ++kb) {
+        ok = warp_mbar_wait(&empty_bar[stage], phase ^ 1u, &abort_flag);
         if (!ok) break;
+        uint8_t* box = smem + stage * kStageBytes + dst;
+        if (elected) {
+          if (wgrad_part == 0) mbar_arrive_expect_tx(&full_bar[stage], kStageBytes);
+          tma_load_3d(box, map, 0, line, row0 + kb * kBK, &full_bar[stage]);
+          tma_load_3d(box + 8192, map, 0, line + 1, row0 + kb * kBK, &full_bar[stage]);
+        }
+        __syncwarp();
         if (++stage == kStages) {
           stage = 0;
           phase ^= 1u;
@@ -165,47 +160,45 @@ __global__ void __launch_bounds__(kGemmThreads, 1) wgrad_gemm_kernel(const __gri
     }
   } else if (warp == 1) {
     // ======================= MMA issuer =======================
-    // One thread runs the whole issue loop: a poll of the stage barrier, the K = 16 MMAs with descriptor words
-    // derived by integer adds, one commit.  The other lanes join only where a weight-gradient tile ends in a
-    // ragged chunk whose tail rows must be zeroed in shared memory.  (Per-stage warp synchronisation in this
-    // loop costs about a quarter of the tensor time of a stage; tiles of the weight gradient are only a few
-    // stages long, so it mattered most there.)
+    // The warp stays converged around the elected lane's instructions (see "Issuing warps"); the next stage's barrier is
+    // looked at while this stage's MMAs are on their way.  All lanes zero the tail rows of a ragged last chunk.
     constexpr uint32_t idesc = umma_idesc_bf16(kBM, kBN, 1, 1);
     constexpr uint32_t kDescHi = (1024u >> 4) | (1u << 14) | (2u << 29);  // SBO 1024, version 1, 128-byte swizzle
     constexpr uint32_t kLboMN = (8192u >> 4) << 16;
-    constexpr uint32_t a_step = 2048u >> 4, b_step = 2048u >> 4;
-    const uint32_t a_lo0 = ((smem_u32(smem) & 0x3ffffu) >> 4) | kLboMN;
-    const uint32_t b_lo0 = (((smem_u32(smem) + kABytes) & 0x3ffffu) >> 4) | kLboMN;
-    const uint32_t empty0 = smem_u32(&empty_bar[0]), tfull0 = smem_u32(&tmem_full_bar[0]);
+    constexpr uint32_t k_step = 2048u >> 4;  // 16 rows of both operands
+    const bool elected = elect_one();
+    const uint32_t a_lo0 = uniform(((smem_u32(smem) & 0x3ffffu) >> 4) | kLboMN);
+    const uint32_t full0 = uniform(smem_u32(&full_bar[0])), empty0 = uniform(smem_u32(&empty_bar[0]));
+    const uint32_t tfull0 = uniform(smem_u32(&tmem_full_bar[0]));
     int stage = 0;
-    uint32_t phase = 0;
+    uint32_t phase = 0, ready = 0;  // ready: the current stage is known to be full
     int e = 0;
     int it = 0;
     bool ok = true;
-    for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x, ++it) {
+    for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x, ++it) {
       const Tile t = decode_tile(tile, e, s_tile_start, s_off, n_tiles);
+      const int k_iters = uniform(t.k_iters);
       const int buf = it & 1;
       const uint32_t acc_phase = (it >> 1) & 1u;
       const uint32_t d_tmem = tmem_base + buf * kBN;
-      // weight gradient: rows of the last chunk that belong to the expert, and whether its tail needs zeroing
-      const int valid_last = (t.row_end - t.row0) - (t.k_iters - 1) * kBK;
-      const bool ragged = t.k_iters > 0 && (valid_last & 15) != 0;
-      if (ragged && t.k_iters <= 16) {
-        // Short ragged tile: the lanes that must zero the tail stay in step with the issuing lane for the
-        // whole tile (re-joining lanes that waited through a single-thread loop costs about a microsecond,
-        // which only long tiles can afford).
-        if (lane == 0) ok = mbar_wait(&tmem_empty_bar[buf], acc_phase ^ 1u, &abort_flag);
-        ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
-        if (!ok) break;
-        tcgen05_fence_after();
-        for (int kb = 0; kb < t.k_iters; ++kb) {
-          if (lane == 0) ok = mbar_wait(&full_bar[stage], phase, &abort_flag);
-          ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
+      const int valid_last = uniform((t.row_end - t.row0) - (t.k_iters - 1) * kBK);  // rows of the last chunk
+      ok = warp_mbar_wait(&tmem_empty_bar[buf], acc_phase ^ 1u, &abort_flag);
+      if (!ok) break;
+      tcgen05_fence_after();
+      uint32_t acc = 0;
+#pragma unroll 1
+      for (int kb = 0; kb < k_iters; ++kb) {
+        if (!__all_sync(0xffffffffu, ready)) {
+          ok = warp_mbar_wait(&full_bar[stage], phase, &abort_flag);
           if (!ok) break;
-          int ksteps = kBK / 16;
-          if (kb == t.k_iters - 1) {
+        }
+        int ksteps = kBK / 16;
+        if (kb == k_iters - 1) {
+          // Only the K = 16 steps that hold rows of this expert are issued, and the rows between the expert's end and the
+          // end of its last step (at most 15) are zeroed.  Row r of every 64 x 64 box is one contiguous 128-byte line.
+          ksteps = (valid_last + 15) >> 4;
+          if ((valid_last & 15) != 0) {
             uint8_t* sa = smem + stage * kStageBytes;
-            ksteps = (valid_last + 15) >> 4;
             const int vec_per_box = (ksteps * 16 - valid_last) * 8;
             const int boxes = (kBM + kBN) / 64;
             for (int i = lane; i < boxes * vec_per_box; i += 32) {
@@ -215,88 +208,27 @@ __global__ void __launch_bounds__(kGemmThreads, 1) wgrad_gemm_kernel(const __gri
             fence_proxy_async_smem();
             __syncwarp();
           }
-          if (lane == 0) {
-            const uint32_t a_lo = a_lo0 + stage * (kStageBytes >> 4), b_lo = b_lo0 + stage * (kStageBytes >> 4);
-            umma_bf16_lo(d_tmem, a_lo, b_lo, kDescHi, idesc, kb > 0 ? 1u : 0u);
-            if (ksteps > 1) umma_bf16_lo(d_tmem, a_lo + a_step, b_lo + b_step, kDescHi, idesc, 1u);
-            if (ksteps > 2) umma_bf16_lo(d_tmem, a_lo + 2 * a_step, b_lo + 2 * b_step, kDescHi, idesc, 1u);
-            if (ksteps > 3) umma_bf16_lo(d_tmem, a_lo + 3 * a_step, b_lo + 3 * b_step, kDescHi, idesc, 1u);
-            tcgen05_commit_addr(empty0 + stage * 8);
-          }
-          __syncwarp();
-          if (++stage == kStages) {
-            stage = 0;
-            phase ^= 1u;
-          }
         }
-        if (!ok) break;
-        if (lane == 0) tcgen05_commit_addr(tfull0 + buf * 8);
-        __syncwarp();
-        continue;
-      }
-      const int solo = ragged ? t.k_iters - 1 : t.k_iters;  // stages lane 0 handles alone
-      if (lane == 0) {
-        ok = mbar_wait(&tmem_empty_bar[buf], acc_phase ^ 1u, &abort_flag);
-        tcgen05_fence_after();
-        int st = stage;
-        uint32_t ph = phase;
-        for (int kb = 0; kb < solo && ok; ++kb) {
-          ok = mbar_wait(&full_bar[st], ph, &abort_flag);
-          if (!ok) break;
-          const uint32_t a_lo = a_lo0 + st * (kStageBytes >> 4), b_lo = b_lo0 + st * (kStageBytes >> 4);
-          const int ksteps = kb == t.k_iters - 1 ? (valid_last + 15) >> 4 : kBK / 16;
-          umma_bf16_lo(d_tmem, a_lo, b_lo, kDescHi, idesc, kb > 0 ? 1u : 0u);
-          if (ksteps > 1) umma_bf16_lo(d_tmem, a_lo + a_step, b_lo + b_step, kDescHi, idesc, 1u);
-          if (ksteps > 2) umma_bf16_lo(d_tmem, a_lo + 2 * a_step, b_lo + 2 * b_step, kDescHi, idesc, 1u);
-          if (ksteps > 3) umma_bf16_lo(d_tmem, a_lo + 3 * a_step, b_lo + 3 * b_step, kDescHi, idesc, 1u);
-          tcgen05_commit_addr(empty0 + st * 8);
-          if (++st == kStages) {
-            st = 0;
-            ph ^= 1u;
-          }
-        }
-      }
-      {  // every lane tracks the ring position
-        const int adv = stage + solo;
-        phase ^= static_cast<uint32_t>(adv / kStages) & 1u;
-        stage = adv % kStages;
-      }
-      if (ragged) {
-        ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
-        if (ok && lane == 0) ok = mbar_wait(&full_bar[stage], phase, &abort_flag);
-        ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
-        if (ok) {
-          // Ragged last chunk: only the K = 16 steps that hold rows of this expert are issued, and the rows
-          // between the expert's end and the end of its last step (at most 15) are zeroed in shared memory.
-          // Row r of every 64 x 64 box is one contiguous 128-byte line.
-          uint8_t* sa = smem + stage * kStageBytes;
-          const int ksteps = (valid_last + 15) >> 4;
-          const int vec_per_box = (ksteps * 16 - valid_last) * 8;
-          const int boxes = (kBM + kBN) / 64;
-          for (int i = lane; i < boxes * vec_per_box; i += 32) {
-            const int box = i / vec_per_box, v = i - box * vec_per_box;
-            reinterpret_cast<uint4*>(sa + box * 8192 + valid_last * 128)[v] = make_uint4(0, 0, 0, 0);
-          }
-          fence_proxy_async_smem();
-          __syncwarp();
-          if (lane == 0) {
-            const uint32_t a_lo = a_lo0 + stage * (kStageBytes >> 4), b_lo = b_lo0 + stage * (kStageBytes >> 4);
-            umma_bf16_lo(d_tmem, a_lo, b_lo, kDescHi, idesc, t.k_iters > 1 ? 1u : 0u);
-            if (ksteps > 1) umma_bf16_lo(d_tmem, a_lo + a_step, b_lo + b_step, kDescHi, idesc, 1u);
-            if (ksteps > 2) umma_bf16_lo(d_tmem, a_lo + 2 * a_step, b_lo + 2 * b_step, kDescHi, idesc, 1u);
-            if (ksteps > 3) umma_bf16_lo(d_tmem, a_lo + 3 * a_step, b_lo + 3 * b_step, kDescHi, idesc, 1u);
-            tcgen05_commit_addr(empty0 + stage * 8);
-          }
-        }
+        const uint32_t a_lo = a_lo0 + stage * (kStageBytes >> 4), b_lo = a_lo + (kABytes >> 4);
+        const uint32_t empty = empty0 + stage * 8;
         if (++stage == kStages) {
           stage = 0;
           phase ^= 1u;
         }
+        ready = mbar_test(full0 + stage * 8, phase);
+        if (elected) {
+          umma_bf16_lo(d_tmem, a_lo, b_lo, kDescHi, idesc, acc);
+          if (ksteps > 1) umma_bf16_lo(d_tmem, a_lo + k_step, b_lo + k_step, kDescHi, idesc, 1u);
+          if (ksteps > 2) umma_bf16_lo(d_tmem, a_lo + 2 * k_step, b_lo + 2 * k_step, kDescHi, idesc, 1u);
+          if (ksteps > 3) umma_bf16_lo(d_tmem, a_lo + 3 * k_step, b_lo + 3 * k_step, kDescHi, idesc, 1u);
+          tcgen05_commit_addr(empty);
+        }
+        __syncwarp();
+        acc = 1;
       }
-      ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
       if (!ok) break;
-      if (lane == 0) {
-        if (t.k_iters > 0)
+      if (elected) {
+        if (k_iters > 0)
           tcgen05_commit_addr(tfull0 + buf * 8);
         else
           mbar_arrive(&tmem_full_bar[buf]);

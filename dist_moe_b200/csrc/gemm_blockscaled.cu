@@ -177,12 +177,14 @@ __global__ void __launch_bounds__(kWdThreads, 1) blockscaled_wide_kernel(const _
   tcgen05_fence_before();
   __syncthreads();
   tcgen05_fence_after();
-  const uint32_t tmem_base = tmem_base_slot;
-  const int total_tiles = s_tile_start[p.e_local];
+  const uint32_t tmem_base = uniform(tmem_base_slot);
+  const int total_tiles = uniform(s_tile_start[p.e_local]);
+  const uint32_t ring = uniform(smem_u32(smem));
 
   if (warp == 0) {
     // ======================= producer =======================
-    if (lane == 0) {
+    {
+      const bool elected = elect_one();
       int stage = 0;
       uint32_t phase = 0;
       int e = 0;
@@ -209,34 +211,39 @@ __global__ void __launch_bounds__(kWdThreads, 1) blockscaled_wide_kernel(const _
           sfb_row0 = p.sfb + t.e * p.sfb_group_bytes + static_cast<int64_t>(t.n_blk * 2) * b_col_atoms * 512;
         }
         const uint8_t* sfb_row1 = sfb_row0 + static_cast<int64_t>(b_col_atoms) * 512;
-        const bool second = t.n_blk * 2 + 1 < row_blocks;  // the tile's upper 128 columns exist
-        for (int kb = 0; kb < t.k_iters && ok; ++kb) {
-          ok = mbar_wait(&empty_bar[stage], phase ^ 1u, &abort_flag);
+        const bool second = uniform(t.n_blk * 2 + 1 < row_blocks ? 1 : 0) != 0;  // the tile's upper 128 columns exist
+        const int t_k = uniform(t.k_iters), t_e = uniform(t.e), t_m = uniform(t.m_blk), t_n = uniform(t.n_blk), t_row = uniform(t.row0);
+#pragma unroll 1
+        for (int kb = 0; kb < t_k; ++kb) {
+          ok = warp_mbar_wait(&empty_bar[stage], phase ^ 1u, &abort_flag);
           if (!ok) break;
           uint8_t* sa = smem + stage * stage_bytes;
           uint8_t* sb = sa + kBsABytes;
           uint8_t* ssa = sb + kWdBBytes;
           uint8_t* ssb = ssa + sf_bytes;
-          if (p.mode == 0) {
-            mbar_arrive_expect_tx(&full_bar[stage], kBsABytes + kWdBBytes + (second ? 3 : 2) * sf_bytes);
-            tma_load_3d(sa, &p.tm_a, 0, a_line0 + kb, t.row0, &full_bar[stage]);
-            tma_load_2d(sb, &p.tm_b, kb * 128, t.e * p.N + t.n_blk * kWdBN, &full_bar[stage]);
-          } else {
-            // B arrives as two 128-byte-wide boxes of 128 K rows (MN-major); the upper one only where it exists
-            mbar_arrive_expect_tx(&full_bar[stage], kBsABytes + (second ? kWdBBytes + 3 * sf_bytes : kWdBBytes / 2 + 2 * sf_bytes));
-            if (p.mode == 1) {
-              tma_load_3d(sa, &p.tm_a, 0, a_line0 + kb, t.row0, &full_bar[stage]);
-              tma_load_2d(sb, &p.tm_b, t.n_blk * kWdBN, t.e * p.Kw + kb * 128, &full_bar[stage]);
-              if (second) tma_load_2d(sb + kWdBBytes / 2, &p.tm_b, t.n_blk * kWdBN + 128, t.e * p.Kw + kb * 128, &full_bar[stage]);
+          if (elected) {
+            if (p.mode == 0) {
+              mbar_arrive_expect_tx(&full_bar[stage], kBsABytes + kWdBBytes + (second ? 3 : 2) * sf_bytes);
+              tma_load_3d(sa, &p.tm_a, 0, a_line0 + kb, t_row, &full_bar[stage]);
+              tma_load_2d(sb, &p.tm_b, kb * 128, t_e * p.N + t_n * kWdBN, &full_bar[stage]);
             } else {
-              tma_load_3d(sa, &p.tm_a, 0, a_line0 + t.m_blk, t.row0 + kb * 128, &full_bar[stage]);
-              tma_load_3d(sb, &p.tm_b, 0, b_line0 + t.n_blk * 2, t.row0 + kb * 128, &full_bar[stage]);
-              if (second) tma_load_3d(sb + kWdBBytes / 2, &p.tm_b, 0, b_line0 + t.n_blk * 2 + 1, t.row0 + kb * 128, &full_bar[stage]);
+              // B arrives as two 128-byte-wide boxes of 128 K rows (MN-major); the upper one only where it exists
+              mbar_arrive_expect_tx(&full_bar[stage], kBsABytes + (second ? kWdBBytes + 3 * sf_bytes : kWdBBytes / 2 + 2 * sf_bytes));
+              if (p.mode == 1) {
+                tma_load_3d(sa, &p.tm_a, 0, a_line0 + kb, t_row, &full_bar[stage]);
+                tma_load_2d(sb, &p.tm_b, t_n * kWdBN, t_e * p.Kw + kb * 128, &full_bar[stage]);
+                if (second) tma_load_2d(sb + kWdBBytes / 2, &p.tm_b, t_n * kWdBN + 128, t_e * p.Kw + kb * 128, &full_bar[stage]);
+              } else {
+                tma_load_3d(sa, &p.tm_a, 0, a_line0 + t_m, t_row + kb * 128, &full_bar[stage]);
+                tma_load_3d(sb, &p.tm_b, 0, b_line0 + t_n * 2, t_row + kb * 128, &full_bar[stage]);
+                if (second) tma_load_3d(sb + kWdBBytes / 2, &p.tm_b, 0, b_line0 + t_n * 2 + 1, t_row + kb * 128, &full_bar[stage]);
+              }
             }
+            bulk_load(ssa, sfa_row + static_cast<int64_t>(kb) * sf_bytes, sf_bytes, &full_bar[stage]);
+            bulk_load(ssb, sfb_row0 + static_cast<int64_t>(kb) * sf_bytes, sf_bytes, &full_bar[stage]);
+            if (second) bulk_load(ssb + sf_bytes, sfb_row1 + static_cast<int64_t>(kb) * sf_bytes, sf_bytes, &full_bar[stage]);
           }
-          bulk_load(ssa, sfa_row + static_cast<int64_t>(kb) * sf_bytes, sf_bytes, &full_bar[stage]);
-          bulk_load(ssb, sfb_row0 + static_cast<int64_t>(kb) * sf_bytes, sf_bytes, &full_bar[stage]);
-          if (second) bulk_load(ssb + sf_bytes, sfb_row1 + static_cast<int64_t>(kb) * sf_bytes, sf_bytes, &full_bar[stage]);
+          __syncwarp();
           if (++stage == stages) {
             stage = 0;
             phase ^= 1u;
@@ -247,51 +254,70 @@ __global__ void __launch_bounds__(kWdThreads, 1) blockscaled_wide_kernel(const _
     __syncwarp();
   } else if (warp == 1) {
     // ======================= MMA issuer =======================
-    if (lane == 0) {
-      int stage = 0;
-      uint32_t phase = 0;
-      int e = 0, it = 0;
-      bool ok = true;
+    {
+      const bool elected = elect_one();
+      constexpr uint32_t kDescHi = (1024u >> 4) | (1u << 14) | (2u << 29);  // SBO 1024, version 1, 128-byte swizzle
       const int a_mn = p.mode == 2, b_mn = p.mode != 0;
-      const uint32_t a_step = a_mn ? 4096u : 32u, b_step = b_mn ? 4096u : 32u;
-      const uint32_t b_lbo = b_mn ? kWdBBytes / 2 : 16u;  // MN-major: the two 128-byte-wide halves are 16 KiB apart
+      const uint32_t a_step = a_mn ? 4096u >> 4 : 32u >> 4, b_step = b_mn ? 4096u >> 4 : 32u >> 4;
+      const uint32_t a_lbo = (16u >> 4) << 16;
+      const uint32_t b_lbo = (b_mn ? (kWdBBytes / 2) >> 4 : 16u >> 4) << 16;  // MN-major: the 128-byte-wide halves are 16 KiB apart
       const uint32_t idesc4 = umma_idesc_blockscaled(kWdBN, 1, 0, 0);
       uint32_t idesc8[4];
 #pragma unroll
       for (int j = 0; j < 4; ++j) idesc8[j] = umma_idesc_blockscaled(kWdBN, 0, j, j, a_mn, b_mn);
-      for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x, ++it) {
+      const uint32_t full0 = uniform(smem_u32(&full_bar[0])), empty0 = uniform(smem_u32(&empty_bar[0]));
+      const uint32_t sf0 = uniform(smem_u32(&sf_bar[0])), tfull = uniform(smem_u32(&tmem_full_bar));
+      int stage = 0;
+      uint32_t phase = 0, ready = 0;  // ready: the current stage and its scales are known to be there
+      int e = 0, it = 0;
+      bool ok = true;
+      for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x, ++it) {
         const BsTile t = bs_decode(tile, e, s_tile_start, s_off, p.mode, n_tiles, p.k_iters);
-        ok = mbar_wait(&tmem_empty_bar, (it & 1u) ^ 1u, &abort_flag);  // the epilogue has drained the accumulator
+        const int k_iters = uniform(t.k_iters);
+        ok = warp_mbar_wait(&tmem_empty_bar, (it & 1u) ^ 1u, &abort_flag);  // the epilogue has drained the accumulator
         if (!ok) break;
         tcgen05_fence_after();
-        for (int kb = 0; kb < t.k_iters; ++kb) {
-          ok = mbar_wait(&full_bar[stage], phase, &abort_flag) && mbar_wait(&sf_bar[stage], phase, &abort_flag);
-          if (!ok) break;
+#pragma unroll 1
+        for (int kb = 0; kb < k_iters; ++kb) {
+          if (!__all_sync(0xffffffffu, ready)) {
+            ok = warp_mbar_wait(&full_bar[stage], phase, &abort_flag) && warp_mbar_wait(&sf_bar[stage], phase, &abort_flag);
+            if (!ok) break;
+          }
           tcgen05_fence_after();
-          const uint32_t a_addr = smem_u32(smem + stage * stage_bytes), b_addr = a_addr + kBsABytes;
+          const uint32_t a_addr = ring + stage * stage_bytes;
+          const uint32_t a_lo = ((a_addr & 0x3ffffu) >> 4) | a_lbo, b_lo = (((a_addr + kBsABytes) & 0x3ffffu) >> 4) | b_lbo;
           const uint32_t sfa_t = tmem_base + kWdSfTmemBase + stage * 64u;
           const uint32_t sfb_t = sfa_t + 16u;
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            const uint64_t da = umma_smem_desc(a_addr + j * a_step, 16, 1024);
-            const uint64_t db = umma_smem_desc(b_addr + j * b_step, b_lbo, 1024);
-            const uint32_t acc = (kb > 0 || j > 0) ? 1u : 0u;
-            if (p.fp4)
-              umma_nvf4(tmem_base, da, db, idesc4, sfa_t + 4 * j, sfb_t + 8 * j, acc);
-            else
-              umma_mxf8(tmem_base, da, db, idesc8[j], sfa_t, sfb_t, acc);
-          }
-          tcgen05_commit(&empty_bar[stage]);
+          const uint32_t empty = empty0 + stage * 8;
           if (++stage == stages) {
             stage = 0;
             phase ^= 1u;
           }
+          ready = mbar_test(full0 + stage * 8, phase) & mbar_test(sf0 + stage * 8, phase);
+          if (elected) {
+            if (p.fp4) {
+#pragma unroll
+              for (int j = 0; j < 4; ++j)
+                umma_nvf4_lo(tmem_base, a_lo + j * a_step, b_lo + j * b_step, kDescHi, idesc4, sfa_t + 4 * j, sfb_t + 8 * j,
+                             (kb > 0 || j > 0) ? 1u : 0u);
+            } else {
+#pragma unroll
+              for (int j = 0; j < 4; ++j)
+                umma_mxf8_lo(tmem_base, a_lo + j * a_step, b_lo + j * b_step, kDescHi, idesc8[j], sfa_t, sfb_t,
+                             (kb > 0 || j > 0) ? 1u : 0u);
+            }
+            tcgen05_commit_addr(empty);
+          }
+          __syncwarp();
         }
         if (!ok) break;
-        if (t.k_iters > 0)
-          tcgen05_commit(&tmem_full_bar);
-        else
-          mbar_arrive(&tmem_full_bar);
+        if (elected) {
+          if (k_iters > 0)
+            tcgen05_commit_addr(tfull);
+          else
+            mbar_arrive(&tmem_full_bar);
+        }
+        __syncwarp();
       }
     }
     __syncwarp();
@@ -308,6 +334,8 @@ __global__ void __launch_bounds__(kWdThreads, 1) blockscaled_wide_kernel(const _
     // Warp 10 then polls the accumulator-ready barrier for the epilogue warps and releases them through a hardware
     // named barrier; it arrives for every tile, also after a timeout, so that no epilogue warp is left blocked.
     const bool watcher = warp == 10;
+    const bool elected = elect_one();
+    const uint32_t sf0 = uniform(smem_u32(&sf_bar[0]));
     const int a_lo = watcher ? 2 : 0, a_hi = p.fp4 ? a_lo + 2 : (watcher ? 0 : 1);
     int stage = 0;
     uint32_t phase = 0;
@@ -315,20 +343,25 @@ __global__ void __launch_bounds__(kWdThreads, 1) blockscaled_wide_kernel(const _
     bool ok = true;
     const uint32_t sf_bytes = atoms * 512;
     for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x, ++it) {
-      if (lane == 0 && a_hi > a_lo && ok) {
+      if (a_hi > a_lo && ok) {
         const BsTile t = bs_decode(tile, e, s_tile_start, s_off, p.mode, n_tiles, p.k_iters);
-        for (int kb = 0; kb < t.k_iters; ++kb) {
-          ok = mbar_wait(&full_bar[stage], phase, &abort_flag);
+        const int k_iters = uniform(t.k_iters);
+#pragma unroll 1
+        for (int kb = 0; kb < k_iters; ++kb) {
+          ok = warp_mbar_wait(&full_bar[stage], phase, &abort_flag);
           if (!ok) break;
-          const uint32_t ssa = smem_u32(smem + stage * stage_bytes) + kBsABytes + kWdBBytes, ssb = ssa + sf_bytes;
+          const uint32_t ssa = ring + stage * stage_bytes + kBsABytes + kWdBBytes, ssb = ssa + sf_bytes;
           const uint32_t sfa_t = tmem_base + kWdSfTmemBase + stage * 64u;
           const uint32_t sfb_t = sfa_t + 16u;
-          for (int a = a_lo; a < a_hi; ++a) {
-            tmem_cp_sf_atom(sfa_t + 4 * a, sf_smem_desc(ssa + a * 512));
-            tmem_cp_sf_atom(sfb_t + 8 * a, sf_smem_desc(ssb + a * 512));
-            tmem_cp_sf_atom(sfb_t + 8 * a + 4, sf_smem_desc(ssb + sf_bytes + a * 512));
+          if (elected) {
+            for (int a = a_lo; a < a_hi; ++a) {
+              tmem_cp_sf_atom(sfa_t + 4 * a, sf_smem_desc(ssa + a * 512));
+              tmem_cp_sf_atom(sfb_t + 8 * a, sf_smem_desc(ssb + a * 512));
+              tmem_cp_sf_atom(sfb_t + 8 * a + 4, sf_smem_desc(ssb + sf_bytes + a * 512));
+            }
+            tcgen05_commit_addr(sf0 + stage * 8);
           }
-          tcgen05_commit(&sf_bar[stage]);
+          __syncwarp();
           if (++stage == stages) {
             stage = 0;
             phase ^= 1u;
