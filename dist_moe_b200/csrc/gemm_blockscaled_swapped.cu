@@ -149,121 +149,145 @@ __global__ void __launch_bounds__(kSwThreads, kSwCtasPerSm) blockscaled_swapped_
   tcgen05_fence_before();
   __syncthreads();
   tcgen05_fence_after();
-  const uint32_t tmem_base = tmem_base_slot;
-  const int total_tiles = s_tile_start[p.e_local];
+  const uint32_t tmem_base = uniform(tmem_base_slot);
+  const int total_tiles = uniform(s_tile_start[p.e_local]);
+  const uint32_t ring = uniform(smem_u32(smem));
 
   if (warp == 0) {
     // ======================= producer =======================
-    if (lane == 0) {
-      int stage = 0;
-      uint32_t phase = 0;
-      int e = 0;
-      const int x_line0 = static_cast<int>((p.x_off ? *p.x_off : 0) >> 7);
-      const uint8_t* sfx = p.sfx_base + (p.sfx_off ? *p.sfx_off : 0);
-      const uint32_t sf_bytes = atoms * 512;
-      bool ok = true;
-      for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
-        const SwTile t = sw_decode(tile, e, s_tile_start, s_off, s_cnt, m_tiles);
-        const int nq = (t.n_valid + 31) >> 5;
-        const uint8_t* sfw_row = p.sfw + t.e * p.sfw_group_bytes + static_cast<int64_t>(t.m_blk) * p.w_col_atoms * 512;
-        const uint8_t* sfx_row = sfx + static_cast<int64_t>(t.row0 >> 7) * p.x_col_atoms * 512;
-        for (int kb = 0; kb < p.k_iters && ok; ++kb) {
-          ok = mbar_wait(&empty_bar[stage], phase ^ 1u, &abort_flag);
-          if (!ok) break;
-          uint8_t* sw = smem + stage * kSwStageBytes;
-          uint8_t* sx = sw + kSwWBytes;
-          uint8_t* ssw = sx + kSwXBytes;
-          uint8_t* ssx = ssw + kSwSfBytes;
+    const bool elected = elect_one();
+    int stage = 0;
+    uint32_t phase = 0;
+    int e = 0;
+    const int x_line0 = uniform(static_cast<int>((p.x_off ? *p.x_off : 0) >> 7));
+    const uint8_t* sfx = p.sfx_base + (p.sfx_off ? *p.sfx_off : 0);
+    const uint32_t sf_bytes = atoms * 512;
+    bool ok = true;
+    for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
+      const SwTile t = sw_decode(tile, e, s_tile_start, s_off, s_cnt, m_tiles);
+      const int nq = uniform((t.n_valid + 31) >> 5), row0 = uniform(t.row0), w_row = uniform(t.e * p.N + t.m_blk * 128);
+      const uint8_t* sfw_row = p.sfw + t.e * p.sfw_group_bytes + static_cast<int64_t>(t.m_blk) * p.w_col_atoms * 512;
+      const uint8_t* sfx_row = sfx + static_cast<int64_t>(t.row0 >> 7) * p.x_col_atoms * 512;
+#pragma unroll 1
+      for (int kb = 0; kb < p.k_iters; ++kb) {
+        ok = warp_mbar_wait(&empty_bar[stage], phase ^ 1u, &abort_flag);
+        if (!ok) break;
+        uint8_t* sw = smem + stage * kSwStageBytes;
+        uint8_t* sx = sw + kSwWBytes;
+        uint8_t* ssw = sx + kSwXBytes;
+        uint8_t* ssx = ssw + kSwSfBytes;
+        if (elected) {
           mbar_arrive_expect_tx(&full_bar[stage], kSwWBytes + nq * 4096u + 2 * sf_bytes);
-          tma_load_2d(sw, &p.tm_w, kb * 128, t.e * p.N + t.m_blk * 128, &full_bar[stage]);
+          tma_load_2d(sw, &p.tm_w, kb * 128, w_row, &full_bar[stage]);
           for (int q = 0; q < nq; ++q)
-            tma_load_3d(sx + q * 4096, &p.tm_x, 0, x_line0 + kb, t.row0 + 32 * q, &full_bar[stage]);
+            tma_load_3d(sx + q * 4096, &p.tm_x, 0, x_line0 + kb, row0 + 32 * q, &full_bar[stage]);
           bulk_load(ssw, sfw_row + static_cast<int64_t>(kb) * sf_bytes, sf_bytes, &full_bar[stage]);
           bulk_load(ssx, sfx_row + static_cast<int64_t>(kb) * sf_bytes, sf_bytes, &full_bar[stage]);
-          if (++stage == kSwStages) {
-            stage = 0;
-            phase ^= 1u;
-          }
+        }
+        __syncwarp();
+        if (++stage == kSwStages) {
+          stage = 0;
+          phase ^= 1u;
         }
       }
     }
     __syncwarp();
   } else if (warp == 1) {
     // ======================= MMA issuer =======================
-    if (lane == 0) {
-      int stage = 0;
-      uint32_t phase = 0;
-      int e = 0, it = 0;
-      bool ok = true;
-      for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x, ++it) {
-        const SwTile t = sw_decode(tile, e, s_tile_start, s_off, s_cnt, m_tiles);
-        const int n_mma = ((t.n_valid + 31) >> 5) * 32;
-        const uint32_t col_off = static_cast<uint32_t>((t.row0 & 127) >> 5);  // the tile's 32-row group inside its atom
-        const uint32_t idesc4 = umma_idesc_blockscaled(n_mma, 1, 0, 0);
-        uint32_t idesc8[4];
+    const bool elected = elect_one();
+    constexpr uint32_t kDescHi = (1024u >> 4) | (1u << 14) | (2u << 29);  // SBO 1024, version 1, 128-byte swizzle
+    constexpr uint32_t kLbo = (16u >> 4) << 16;
+    const uint32_t full0 = uniform(smem_u32(&full_bar[0])), empty0 = uniform(smem_u32(&empty_bar[0]));
+    const uint32_t sf0 = uniform(smem_u32(&sf_bar[0])), tfull0 = uniform(smem_u32(&tmem_full_bar[0]));
+    int stage = 0;
+    uint32_t phase = 0, ready = 0;  // ready: the current stage and its scales are known to be there
+    int e = 0, it = 0;
+    bool ok = true;
+    for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x, ++it) {
+      const SwTile t = sw_decode(tile, e, s_tile_start, s_off, s_cnt, m_tiles);
+      const int n_mma = uniform(((t.n_valid + 31) >> 5) * 32);
+      const uint32_t col_off = uniform(static_cast<uint32_t>((t.row0 & 127) >> 5));  // the tile's 32-row group inside its atom
+      const uint32_t idesc4 = umma_idesc_blockscaled(n_mma, 1, 0, 0);
+      uint32_t idesc8[4];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) idesc8[j] = umma_idesc_blockscaled(n_mma, 0, j, j);
-        const int buf = it & 1;
-        const uint32_t acc_phase = (it >> 1) & 1u;
-        ok = mbar_wait(&tmem_empty_bar[buf], acc_phase ^ 1u, &abort_flag);
-        if (!ok) break;
-        tcgen05_fence_after();
-        const uint32_t d_tmem = tmem_base + buf * kSwTileRows;
-        for (int kb = 0; kb < p.k_iters; ++kb) {
-          ok = mbar_wait(&full_bar[stage], phase, &abort_flag) && mbar_wait(&sf_bar[stage], phase, &abort_flag);
+      for (int j = 0; j < 4; ++j) idesc8[j] = umma_idesc_blockscaled(n_mma, 0, j, j);
+      const int buf = it & 1;
+      const uint32_t acc_phase = (it >> 1) & 1u;
+      ok = warp_mbar_wait(&tmem_empty_bar[buf], acc_phase ^ 1u, &abort_flag);
+      if (!ok) break;
+      tcgen05_fence_after();
+      const uint32_t d_tmem = tmem_base + buf * kSwTileRows;
+#pragma unroll 1
+      for (int kb = 0; kb < p.k_iters; ++kb) {
+        if (!__all_sync(0xffffffffu, ready)) {
+          ok = warp_mbar_wait(&full_bar[stage], phase, &abort_flag) && warp_mbar_wait(&sf_bar[stage], phase, &abort_flag);
           if (!ok) break;
-          tcgen05_fence_after();
-          const uint32_t w_addr = smem_u32(smem + stage * kSwStageBytes), x_addr = w_addr + kSwWBytes;
-          const uint32_t sfw_t = tmem_base + kSwSfTmemBase + stage * 32u;
-          const uint32_t sfx_t = sfw_t + 16u;
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            const uint64_t dw = umma_smem_desc(w_addr + j * 32u, 16, 1024);
-            const uint64_t dx = umma_smem_desc(x_addr + j * 32u, 16, 1024);
-            const uint32_t acc = (kb > 0 || j > 0) ? 1u : 0u;
-            if (p.fp4)
-              umma_nvf4(d_tmem, dw, dx, idesc4, sfw_t + 4 * j, sfx_t + 4 * j + col_off, acc);
-            else
-              umma_mxf8(d_tmem, dw, dx, idesc8[j], sfw_t, sfx_t + col_off, acc);
-          }
-          tcgen05_commit(&empty_bar[stage]);
-          if (++stage == kSwStages) {
-            stage = 0;
-            phase ^= 1u;
-          }
         }
-        if (!ok) break;
+        tcgen05_fence_after();
+        const uint32_t w_addr = ring + stage * kSwStageBytes;
+        const uint32_t w_lo = ((w_addr & 0x3ffffu) >> 4) | kLbo, x_lo = (((w_addr + kSwWBytes) & 0x3ffffu) >> 4) | kLbo;
+        const uint32_t sfw_t = tmem_base + kSwSfTmemBase + stage * 32u;
+        const uint32_t sfx_t = sfw_t + 16u;
+        const uint32_t empty = empty0 + stage * 8;
+        if (++stage == kSwStages) {
+          stage = 0;
+          phase ^= 1u;
+        }
+        ready = mbar_test(full0 + stage * 8, phase) & mbar_test(sf0 + stage * 8, phase);
+        if (elected) {
+          if (p.fp4) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+              umma_nvf4_lo(d_tmem, w_lo + 2 * j, x_lo + 2 * j, kDescHi, idesc4, sfw_t + 4 * j, sfx_t + 4 * j + col_off,
+                           (kb > 0 || j > 0) ? 1u : 0u);
+          } else {
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+              umma_mxf8_lo(d_tmem, w_lo + 2 * j, x_lo + 2 * j, kDescHi, idesc8[j], sfw_t, sfx_t + col_off,
+                           (kb > 0 || j > 0) ? 1u : 0u);
+          }
+          tcgen05_commit_addr(empty);
+        }
+        __syncwarp();
+      }
+      if (!ok) break;
+      if (elected) {
         if (p.k_iters > 0)
-          tcgen05_commit(&tmem_full_bar[buf]);
+          tcgen05_commit_addr(tfull0 + buf * 8);
         else
           mbar_arrive(&tmem_full_bar[buf]);
       }
+      __syncwarp();
     }
     __syncwarp();
   } else if (warp == 7) {
     // ======================= scale copier =======================
     // Moves every stage's scale atoms from shared memory to the stage slot's TMEM columns.  The slot's previous
     // MMAs are complete by then: the producer refilled the stage only after their commit released it.
-    if (lane == 0) {
-      int stage = 0;
-      uint32_t phase = 0;
-      bool ok = true;
-      for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
-        for (int kb = 0; kb < p.k_iters; ++kb) {
-          ok = mbar_wait(&full_bar[stage], phase, &abort_flag);
-          if (!ok) break;
-          const uint32_t ssw = smem_u32(smem + stage * kSwStageBytes) + kSwWBytes + kSwXBytes, ssx = ssw + kSwSfBytes;
-          const uint32_t sfw_t = tmem_base + kSwSfTmemBase + stage * 32u;
-          const uint32_t sfx_t = sfw_t + 16u;
+    const bool elected = elect_one();
+    const uint32_t sf0 = uniform(smem_u32(&sf_bar[0]));
+    int stage = 0;
+    uint32_t phase = 0;
+    bool ok = true;
+    for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
+#pragma unroll 1
+      for (int kb = 0; kb < p.k_iters; ++kb) {
+        ok = warp_mbar_wait(&full_bar[stage], phase, &abort_flag);
+        if (!ok) break;
+        const uint32_t ssw = ring + stage * kSwStageBytes + kSwWBytes + kSwXBytes, ssx = ssw + kSwSfBytes;
+        const uint32_t sfw_t = tmem_base + kSwSfTmemBase + stage * 32u;
+        const uint32_t sfx_t = sfw_t + 16u;
+        if (elected) {
           for (int a = 0; a < atoms; ++a) {
             tmem_cp_sf_atom(sfw_t + 4 * a, sf_smem_desc(ssw + a * 512));
             tmem_cp_sf_atom(sfx_t + 4 * a, sf_smem_desc(ssx + a * 512));
           }
-          tcgen05_commit(&sf_bar[stage]);
-          if (++stage == kSwStages) {
-            stage = 0;
-            phase ^= 1u;
-          }
+          tcgen05_commit_addr(sf0 + stage * 8);
+        }
+        __syncwarp();
+        if (++stage == kSwStages) {
+          stage = 0;
+          phase ^= 1u;
         }
       }
     }
