@@ -68,7 +68,7 @@ def _dispatch_fprop(state, ptrs, a_op_off, w, c_op, h2_op, c, N, Kd, fuse, act, 
                              limit, condp, state.num_sms, status, st, what=what)
         return
     nat.check(nat.lib.dm_gather_rows(ptrs.data_ptr(), c.recv_rows.data_ptr(), state.arena.data_ptr(),
-                                     a_op_off.data_ptr(), Kd * 2, c.max_rows, condp, st), "dm_gather_rows")
+                                     a_op_off, Kd * 2, c.max_rows, condp, st), "dm_gather_rows")
     _gemm_fprop(_op(state, a_op_off), w.data_ptr(), c_op, h2_op, None, c.offsets.data_ptr(), state.e_local,
                 c.max_rows, N, Kd, int(fuse), clamped, alpha, limit, condp, state.num_sms, status, st, what=what)
 
@@ -80,8 +80,10 @@ class _Call:
                  "max_rows", "rstd", "callback_state")
 
 
-def _op(state, t: torch.Tensor | None) -> nat.Operand:
-    return state.arena_operand(t)
+# Planner offsets are named by the address of their int64 (base address of the offset tensor + 8 per entry): slicing the
+# tensor for every operand cost the host more than the launch it was for.
+def _op(state, offset_address: int) -> nat.Operand:
+    return state.arena_at(offset_address)
 
 
 def _none() -> nat.Operand:
@@ -147,8 +149,8 @@ def _expert_forward(state, c: _Call, w13, w2, xg_off, h1_off, h2_off, *, fuse: b
     _dispatch_fprop(state, c.fwd, xg_off, w13, _op(state, h1_off), _op(state, h2_off) if fuse else _none(), c, 2 * F, D,
                     fuse, (clamped, alpha, limit), condp, "gemm_fprop_dispatch(w13)")
     if not fuse:
-        nat.check(nat.lib.dm_swiglu_fwd(state.arena.data_ptr(), h1_off.data_ptr(), state.arena.data_ptr(),
-                                        h2_off.data_ptr(), c.recv_rows.data_ptr(), c.max_rows, F, clamped, alpha,
+        nat.check(nat.lib.dm_swiglu_fwd(state.arena.data_ptr(), h1_off, state.arena.data_ptr(),
+                                        h2_off, c.recv_rows.data_ptr(), c.max_rows, F, clamped, alpha,
                                         limit, nat.ptr(clip), float(clip_limit), None, st), "dm_swiglu_fwd")
     _gemm_fprop(_op(state, h2_off), w2.data_ptr(), _none(), _none(), c.sct.data_ptr(),
                                     c.offsets.data_ptr(), el, c.max_rows, D, F, 0, 0, 1.0, 0.0, condp, state.num_sms,
@@ -162,16 +164,16 @@ def forward_impl(state, x, ids, scores, w13, w2, options: ExecutionOptions, save
     scratch_only = (not save_for_backward) or cfg.inference or state.num_slots == 0
     with record_function("dist_moe_routing"):  # the reference's profiler range names (dist_moe/api.py:1979-2072)
         c = _route_and_plan(state, x, ids, scratch_only, options.validate_expert_ids)
-    fs = c.fwd_state
+    fs = c.fwd_state.data_ptr()
     if not scratch_only:
-        nat.check(nat.lib.dm_cond_copy(x.data_ptr(), None, state.arena.data_ptr(), fs[0:1].data_ptr(), T * D * 2,
+        nat.check(nat.lib.dm_cond_copy(x.data_ptr(), None, state.arena.data_ptr(), fs, T * D * 2,
                                        c.cond.data_ptr(), 1, st), "dm_cond_copy(save x)")
     clip = options.swiglu_clip_stats_out_3
     if clip is not None:
         clip.zero_()
     fuse = clip is None and F % 128 == 0
     with record_function("dist_moe_forward"):
-        _expert_forward(state, c, w13, w2, fs[1:2], fs[2:3], fs[3:4], fuse=fuse, cond=None, clip=clip,
+        _expert_forward(state, c, w13, w2, fs + 8, fs + 16, fs + 24, fuse=fuse, cond=None, clip=clip,
                         clip_limit=options.swiglu_clip_limit)
     state.barrier(state.combine)
     out = torch.empty(T, D, dtype=torch.bfloat16, device=x.device)
@@ -192,7 +194,7 @@ def forward_impl(state, x, ids, scores, w13, w2, options: ExecutionOptions, save
                                            int(scores.dtype == torch.bfloat16), ids.data_ptr(),
                                            int(ids.dtype == torch.int64), out.data_ptr(), T, K, D,
                                            None if scratch_only else state.arena.data_ptr(),
-                                           None if scratch_only else fs[4:5].data_ptr(),
+                                           None if scratch_only else fs + 32,
                                            None if scratch_only else c.cond.data_ptr(), 0, st), "dm_scale_and_sum")
     return out, c
 
@@ -247,7 +249,7 @@ def backward_impl(state, c: _Call, x_shape, ids, scores, w13, w2, w13_param, w2_
                                        c.need.data_ptr(), c.fwd_state.data_ptr(), bo.data_ptr(),
                                        state.moe_layer_id.data_ptr(), state.ep, cfg.max_num_local_input_tokens, K, D,
                                        F, state.slot_bytes, state.num_slots, status, st), "dm_plan_bwd_bf16")
-    fs, cond = c.fwd_state, c.cond
+    fs, bop, cond = c.fwd_state.data_ptr(), bo.data_ptr(), c.cond
     arena = state.arena.data_ptr()
     post = options.experts_output_postprocess
     is_norm = isinstance(post, RMSNormPostprocess)
@@ -255,23 +257,23 @@ def backward_impl(state, c: _Call, x_shape, ids, scores, w13, w2, w13_param, w2_
     # ---- recompute block (device-predicated on need_recompute) ----------------
     span = record_function("dist_moe_recompute")
     span.__enter__()
-    nat.check(nat.lib.dm_cond_copy(arena, fs[0:1].data_ptr(), state.dispatch.local().data_ptr(), None, T * D * 2,
+    nat.check(nat.lib.dm_cond_copy(arena, fs, state.dispatch.local().data_ptr(), None, T * D * 2,
                                    cond.data_ptr(), 1, st), "dm_cond_copy(republish x)")
     state.barrier(state.dispatch, cond)
-    _dispatch_fprop(state, c.fwd, bo[0:1], w13, _op(state, bo[1:2]), _none(), c, 2 * F, D, False,
+    _dispatch_fprop(state, c.fwd, bop, w13, _op(state, bop + 8), _none(), c, 2 * F, D, False,
                     (clamped, alpha, limit), cond.data_ptr(), "gemm_fprop_dispatch(w13 recompute)")
     # h2 is always rebuilt from h1: only x_gathered, h1 and h3 are ever saved.
-    nat.check(nat.lib.dm_swiglu_fwd(arena, bo[1:2].data_ptr(), arena, bo[2:3].data_ptr(), c.recv_rows.data_ptr(),
+    nat.check(nat.lib.dm_swiglu_fwd(arena, bop + 8, arena, bop + 16, c.recv_rows.data_ptr(),
                                     c.max_rows, F, clamped, alpha, limit, None, 0.0, None, st), "dm_swiglu_fwd(bwd)")
     need_h3 = (need_scores or is_norm) and not is_callback
     if need_h3:
-        _gemm_fprop(_op(state, bo[2:3]), w2.data_ptr(), _none(), _none(), c.sct.data_ptr(),
+        _gemm_fprop(_op(state, bop + 16), w2.data_ptr(), _none(), _none(), c.sct.data_ptr(),
                                         c.offsets.data_ptr(), el, c.max_rows, D, F, 0, 0, 1.0, 0.0, cond.data_ptr(),
                                         state.num_sms, status, st, what="gemm_fprop(w2 recompute)")
         # Saved path: the fused RMSNorm backward works on the expert outputs in place in the communication buffer,
         # so they are copied back there; the plain backward reads them where they were saved (selected on the device).
         if is_norm or not READ_SAVED_H3_IN_PLACE:
-            nat.check(nat.lib.dm_cond_copy(arena, fs[4:5].data_ptr(), state.combine.local().data_ptr(), None,
+            nat.check(nat.lib.dm_cond_copy(arena, fs + 32, state.combine.local().data_ptr(), None,
                                            T * K * D * 2, cond.data_ptr(), 0, st), "dm_cond_copy(load h3)")
         state.barrier(state.combine, cond)
     span.__exit__(None, None, None)
@@ -299,7 +301,7 @@ def backward_impl(state, c: _Call, x_shape, ids, scores, w13, w2, w13_param, w2_
         if need_scores and READ_SAVED_H3_IN_PLACE:
             nat.check(nat.lib.dm_broadcast_and_scale_select(grad_out.data_ptr(), scores.data_ptr(),
                                                             int(scores.dtype == torch.bfloat16), ids.data_ptr(),
-                                                            int(ids.dtype == torch.int64), arena, fs[4:5].data_ptr(),
+                                                            int(ids.dtype == torch.int64), arena, fs + 32,
                                                             combine, cond.data_ptr(), combine, nat.ptr(grad_scores), T,
                                                             K, D, st), "dm_broadcast_and_scale")
         else:
@@ -311,36 +313,36 @@ def backward_impl(state, c: _Call, x_shape, ids, scores, w13, w2, w13_param, w2_
     state.barrier(state.combine)
     # ---- W2: input gradient and weight gradient ----------------------------------
     if FUSED_DISPATCH:
-        _gemm_dgrad_dispatch(c.sct.data_ptr(), state.gather_flags.data_ptr(), _op(state, bo[4:5]), w2.data_ptr(),
-                             _op(state, bo[3:4]), c.offsets.data_ptr(), el, c.max_rows, F, D, None, state.num_sms,
+        _gemm_dgrad_dispatch(c.sct.data_ptr(), state.gather_flags.data_ptr(), _op(state, bop + 32), w2.data_ptr(),
+                             _op(state, bop + 24), c.offsets.data_ptr(), el, c.max_rows, F, D, None, state.num_sms,
                              status, st, what="gemm_dgrad_dispatch(w2)")
     else:
-        nat.check(nat.lib.dm_gather_rows(c.sct.data_ptr(), c.recv_rows.data_ptr(), arena, bo[4:5].data_ptr(), D * 2,
+        nat.check(nat.lib.dm_gather_rows(c.sct.data_ptr(), c.recv_rows.data_ptr(), arena, bop + 32, D * 2,
                                          c.max_rows, None, st), "dm_gather_rows(grad_h3)")
-        _gemm_dgrad(_op(state, bo[4:5]), w2.data_ptr(), _op(state, bo[3:4]), None, c.offsets.data_ptr(), el,
+        _gemm_dgrad(_op(state, bop + 32), w2.data_ptr(), _op(state, bop + 24), None, c.offsets.data_ptr(), el,
                     c.max_rows, F, D, None, state.num_sms, status, st, what="gemm_dgrad(w2)")
     grad_w13 = grad_w2 = None
     owners = options.wgrad_parameter_owners or (None, None)
     if need_w2:
         dst, acc, ret = _wgrad_destination(w2_param, (el, D, F), options, cfg, owners[1], wgrad_explicit[1], hooks, "w2")
-        _gemm_wgrad(_op(state, bo[4:5]), _op(state, bo[2:3]), dst.data_ptr(),
+        _gemm_wgrad(_op(state, bop + 32), _op(state, bop + 16), dst.data_ptr(),
                                         int(dst.dtype == torch.float32), acc, c.offsets.data_ptr(), el, c.max_rows,
                                         D, F, state.num_sms, status, st, what="gemm_wgrad(w2)")
         grad_w2 = dst.view(w2_param.shape) if ret else None
         if hooks is not None:
             grad_w2 = hooks.wgrad_postprocess("w2", grad_w2)
     # ---- SwiGLU backward, W13 input gradient (scattered to the owners) and weight gradient
-    nat.check(nat.lib.dm_swiglu_bwd(arena, bo[1:2].data_ptr(), arena, bo[3:4].data_ptr(), arena, bo[5:6].data_ptr(),
+    nat.check(nat.lib.dm_swiglu_bwd(arena, bop + 8, arena, bop + 24, arena, bop + 40,
                                     c.recv_rows.data_ptr(), c.max_rows, F, clamped, alpha, limit, st),
               "dm_swiglu_bwd")
     if need_x:
-        _gemm_dgrad(_op(state, bo[5:6]), w13.data_ptr(), _none(), c.bwd.data_ptr(),
+        _gemm_dgrad(_op(state, bop + 40), w13.data_ptr(), _none(), c.bwd.data_ptr(),
                                         c.offsets.data_ptr(), el, c.max_rows, D, 2 * F, None, state.num_sms, status,
                                         st, what="gemm_dgrad(w13)")
     if need_w13:
         dst, acc, ret = _wgrad_destination(w13_param, (el, 2 * F, D), options, cfg, owners[0], wgrad_explicit[0], hooks,
                                            "w13")
-        _gemm_wgrad(_op(state, bo[5:6]), _op(state, bo[0:1]), dst.data_ptr(),
+        _gemm_wgrad(_op(state, bop + 40), _op(state, bop), dst.data_ptr(),
                                         int(dst.dtype == torch.float32), acc, c.offsets.data_ptr(), el, c.max_rows,
                                         2 * F, D, state.num_sms, status, st, what="gemm_wgrad(w13)")
         grad_w13 = dst.view(w13_param.shape) if ret else None

@@ -149,7 +149,8 @@ def _quantize_weight(w: torch.Tensor, kind: str, inference: bool, out: PreparedW
             if t is None or tuple(t.shape) != tuple(shape) or t.dtype != dtype:
                 raise ValueError(f"out.{name} does not match the prepared layout")
             return t
-        return torch.zeros(shape, dtype=dtype, device=dev)
+        # every byte is written below: rows and scale columns fill their 128 x 4 atoms (checked above)
+        return torch.empty(shape, dtype=dtype, device=dev)
 
     fprop_data = storage("fprop_data", (E, N, qb), torch.uint8)
     fprop_scale = storage("fprop_scale", (E * grp,), torch.uint8)
@@ -571,12 +572,12 @@ def _mxfp8_forward_planned(state, x, ids, scores, p13, p2, options, need_h3: boo
         c.fwd_table.data_ptr(), state.slot_selector.data_ptr(), state.moe_layer_id.data_ptr(), ep,
         cfg.max_num_local_input_tokens, K, D, F, _storage_array(state), state.capacity_rows, state.slot_bytes,
         state.num_slots, state.num_layers_in_slot, 0, 0, 0, 0, 0, status, st), "dm_plan_fwd_blockscaled")
-    fs, ft = c.fwd_state, c.fwd_table
-    A = lambda table, group, entry: state.arena_operand(table[group * 9 + entry:group * 9 + entry + 1])  # noqa: E731
+    fs, ft = c.fwd_state.data_ptr(), c.fwd_table.data_ptr()
+    A = lambda table, group, entry: state.arena_at(table + 8 * (group * 9 + entry))  # noqa: E731
     none = nat.Operand(None, 0, None)
     arena = state.arena.data_ptr()
     # a layer that will be recomputed keeps only its dense input
-    nat.check(nat.lib.dm_cond_copy(x.data_ptr(), None, arena, fs[0:1].data_ptr(), T * D * 2, c.cond.data_ptr(), 1, st),
+    nat.check(nat.lib.dm_cond_copy(x.data_ptr(), None, arena, fs, T * D * 2, c.cond.data_ptr(), 1, st),
               "dm_cond_copy(save x)")
     # dispatch: the routed rows are pulled through the pointer table by the quantiser itself
     nat.check(nat.lib.dm_quant_mxfp8_rowcol_gather_at(c.fwd.data_ptr(), recv, R, D, A(ft, 0, _A_Q), A(ft, 0, _A_SF),
@@ -612,7 +613,7 @@ def _mxfp8_forward_planned(state, x, ids, scores, p13, p2, options, need_h3: boo
         nat.check(nat.lib.dm_scale_and_sum(state.combine.local().data_ptr(), scores.data_ptr(),
                                            int(scores.dtype == torch.bfloat16), ids.data_ptr(),
                                            int(ids.dtype == torch.int64), out.data_ptr(), T, K, D,
-                                           arena if need_h3 else None, fs[4:5].data_ptr() if need_h3 else None,
+                                           arena if need_h3 else None, fs + 32 if need_h3 else None,
                                            c.cond.data_ptr() if need_h3 else None, 0, st), "dm_scale_and_sum")
     state.last_recv = c.recv
     state.last_train_call = c
@@ -640,14 +641,15 @@ def _mxfp8_backward_planned(state, c: _TrainCall, x_shape, ids, scores, w13_para
         state.peak_min_free.data_ptr(), c.need.data_ptr(), c.fwd_state.data_ptr(), bo.data_ptr(), bt.data_ptr(),
         state.moe_layer_id.data_ptr(), ep, cfg.max_num_local_input_tokens, K, D, F, _storage_array(state),
         state.capacity_rows, state.slot_bytes, state.num_slots, 0, 0, status, st), "dm_plan_bwd_blockscaled")
-    A = lambda group, entry: state.arena_operand(bt[group * 9 + entry:group * 9 + entry + 1])  # noqa: E731
-    fs, cond = c.fwd_state, c.cond
+    btp = bt.data_ptr()
+    A = lambda group, entry: state.arena_at(btp + 8 * (group * 9 + entry))  # noqa: E731
+    fs, cond = c.fwd_state.data_ptr(), c.cond
     post = options.experts_output_postprocess
     is_norm = isinstance(post, RMSNormPostprocess)
     is_callback = post is not None and not is_norm  # the callable kept its own input and output (eager path)
     # ---- recompute block: every launch is a no-op unless the forward chose to recompute this layer ------------
     with record_function("dist_moe_recompute"):
-        nat.check(nat.lib.dm_cond_copy(arena, fs[0:1].data_ptr(), state.dispatch.local().data_ptr(), None, T * D * 2,
+        nat.check(nat.lib.dm_cond_copy(arena, fs, state.dispatch.local().data_ptr(), None, T * D * 2,
                                        cond.data_ptr(), 1, st), "dm_cond_copy(republish x)")
         state.barrier(state.dispatch, cond)
         nat.check(nat.lib.dm_quant_mxfp8_rowcol_gather_at(c.fwd.data_ptr(), recv, R, D, A(0, _A_Q), A(0, _A_SF),
@@ -668,7 +670,7 @@ def _mxfp8_backward_planned(state, c: _TrainCall, x_shape, ids, scores, w13_para
                                                   offs, el, R, D, F, 0, 0, 1.0, 0.0, cond.data_ptr(), state.num_sms,
                                                   status, st), "dm_gemm_blockscaled(w2 recompute)")
             if is_norm:  # the fused RMSNorm backward works on the expert outputs in place in the combine buffer
-                nat.check(nat.lib.dm_cond_copy(arena, fs[4:5].data_ptr(), combine, None, T * K * D * 2,
+                nat.check(nat.lib.dm_cond_copy(arena, fs + 32, combine, None, T * K * D * 2,
                                                cond.data_ptr(), 0, st), "dm_cond_copy(load h3)")
             state.barrier(state.combine, cond)
     # ---- gradient with respect to the expert outputs and the scores ------------------------------------------
@@ -682,7 +684,7 @@ def _mxfp8_backward_planned(state, c: _TrainCall, x_shape, ids, scores, w13_para
     elif need_scores:
         nat.check(nat.lib.dm_broadcast_and_scale_select(grad_out.data_ptr(), scores.data_ptr(),
                                                         int(scores.dtype == torch.bfloat16), ids.data_ptr(),
-                                                        int(ids.dtype == torch.int64), arena, fs[4:5].data_ptr(),
+                                                        int(ids.dtype == torch.int64), arena, fs + 32,
                                                         combine, cond.data_ptr(), combine, nat.ptr(grad_scores), T, K,
                                                         D, st), "dm_broadcast_and_scale")
     else:

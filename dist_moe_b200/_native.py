@@ -221,6 +221,7 @@ def operand(t, offset=None, nbytes: int | None = None) -> Operand:
 
 
 def stream_ptr() -> int:
+    """The current device's current stream."""
     import torch
 
-    return torch.cuda.current_stream().cuda_stream
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())

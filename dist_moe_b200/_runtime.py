@@ -239,6 +239,7 @@ class ContextState:
         nat.check(nat.lib.dm_barrier(buf.peer_pads.data_ptr(), self.rank, self.ep, 0, nat.ptr(cond),
                                      BARRIER_TIMEOUT_NS, self.status.data_ptr(), nat.stream_ptr()), "dm_barrier")
 
-    def arena_operand(self, offset_tensor: torch.Tensor | None) -> nat.Operand:
-        return nat.Operand(self.arena.data_ptr(), self.arena.numel(),
-                           None if offset_tensor is None else offset_tensor.data_ptr())
+    def arena_at(self, offset_address: int) -> nat.Operand:
+        """Operand whose byte offset inside the arena is the device int64 at ``offset_address``."""
+        arena = self.arena
+        return nat.Operand(arena.data_ptr(), arena.numel(), offset_address)
