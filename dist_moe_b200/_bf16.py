@@ -138,7 +138,8 @@ def _route_and_plan(state, x, ids, scratch_only: bool, validate: bool) -> _Call:
     return c
 
 
-def _expert_forward(state, c: _Call, w13, w2, xg_off, h1_off, h2_off, *, fuse: bool, cond, clip, clip_limit) -> None:
+def _expert_forward(state, c: _Call, w13, w2, xg_off, h1_off, h2_off, *, fuse: bool, cond, clip, clip_limit,
+                    keep_h1: bool = True) -> None:
     """gather -> W13 (+SwiGLU) -> W2 + scatter into the owners' combine buffers."""
     cfg = state.config
     D, F, el = cfg.hidden_dim, cfg.intermediate_dim, state.e_local
@@ -146,7 +147,9 @@ def _expert_forward(state, c: _Call, w13, w2, xg_off, h1_off, h2_off, *, fuse: b
     clamped, alpha, limit = _act(cfg)
     condp = nat.ptr(cond)
     # dispatch + W13: gather warps pull the routed rows (peer loads) while the tensor cores run
-    _dispatch_fprop(state, c.fwd, xg_off, w13, _op(state, h1_off), _op(state, h2_off) if fuse else _none(), c, 2 * F, D,
+    # (a forward without a backward has no reader of h1: the fused epilogue then writes h2 alone)
+    h1_op = _op(state, h1_off) if keep_h1 or not fuse else _none()
+    _dispatch_fprop(state, c.fwd, xg_off, w13, h1_op, _op(state, h2_off) if fuse else _none(), c, 2 * F, D,
                     fuse, (clamped, alpha, limit), condp, "gemm_fprop_dispatch(w13)")
     if not fuse:
         nat.check(nat.lib.dm_swiglu_fwd(state.arena.data_ptr(), h1_off, state.arena.data_ptr(),
@@ -174,7 +177,7 @@ def forward_impl(state, x, ids, scores, w13, w2, options: ExecutionOptions, save
     fuse = clip is None and F % 128 == 0
     with record_function("dist_moe_forward"):
         _expert_forward(state, c, w13, w2, fs + 8, fs + 16, fs + 24, fuse=fuse, cond=None, clip=clip,
-                        clip_limit=options.swiglu_clip_limit)
+                        clip_limit=options.swiglu_clip_limit, keep_h1=not scratch_only)
     state.barrier(state.combine)
     out = torch.empty(T, D, dtype=torch.bfloat16, device=x.device)
     post = options.experts_output_postprocess

@@ -68,7 +68,7 @@ struct RowsParams {
   const int64_t* a_off;        // device byte offsets (may be null = 0)
   const int64_t* c_off;
   const int64_t* h2_off;
-  uint8_t* c_base;
+  uint8_t* c_base;  // with the fused SwiGLU: h1, null where nothing reads it
   uint8_t* h2_base;
   const int64_t* scatter_ptrs;
   const int64_t* gather_ptrs;  // fused dispatch: row r of A is pulled from gather_ptrs[r] (may be peer memory)
@@ -448,6 +448,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kRwThreads, 1) rows_
         const int r = b * 32 + lane;
         if (r >= t.rows) return 0;
         if (!kSwiglu && p.scatter_ptrs != nullptr) return static_cast<uint64_t>(p.scatter_ptrs[t.row0 + r]);
+        if (kSwiglu && p.c_base == nullptr) return 0;
         return reinterpret_cast<uint64_t>(p.c_base) + c_off + static_cast<uint64_t>(t.row0 + r) * p.N * 2;
       };
       uint64_t my_row = b_begin < b_end ? row_ptr(b_begin) : 0;
@@ -485,11 +486,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kRwThreads, 1) rows_
                                swiglu_f32(__uint_as_float(gw & 0xffff0000u), __uint_as_float(uw & 0xffff0000u), p.act));
           }
           const int chunk = 2 * quad + (word >> 2);
+          if (p.c_base != nullptr) {
 #pragma unroll
-          for (int i = 0; i < 16; ++i) {
-            const int r = 2 * i + odd;
-            *reinterpret_cast<uint32_t*>(stg + r * 384 + up * 128 + ((chunk ^ (odd << 2) ^ (up << 1)) << 4) + (word & 3) * 4) =
-                rw_pair(w[i], odd);
+            for (int i = 0; i < 16; ++i) {
+              const int r = 2 * i + odd;
+              *reinterpret_cast<uint32_t*>(stg + r * 384 + up * 128 + ((chunk ^ (odd << 2) ^ (up << 1)) << 4) + (word & 3) * 4) =
+                  rw_pair(w[i], odd);
+            }
           }
 #pragma unroll
           for (int i = 0; i < 8; ++i) {
@@ -517,10 +520,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kRwThreads, 1) rows_
             if (b * 32 + r < t.rows && col + 8 <= F) {
               const uint8_t* src = stg + r * 384;
               const int sw = (r & 1) << 2;
-              *reinterpret_cast<uint4*>(h1 + static_cast<uint64_t>(col) * 2) =
-                  *reinterpret_cast<const uint4*>(src + ((c ^ sw) << 4));
-              *reinterpret_cast<uint4*>(h1 + static_cast<uint64_t>(F + col) * 2) =
-                  *reinterpret_cast<const uint4*>(src + 128 + ((c ^ sw ^ 2) << 4));
+              if (h1 != 0) {
+                *reinterpret_cast<uint4*>(h1 + static_cast<uint64_t>(col) * 2) =
+                    *reinterpret_cast<const uint4*>(src + ((c ^ sw) << 4));
+                *reinterpret_cast<uint4*>(h1 + static_cast<uint64_t>(F + col) * 2) =
+                    *reinterpret_cast<const uint4*>(src + 128 + ((c ^ sw ^ 2) << 4));
+              }
               *reinterpret_cast<uint4*>(p.h2_base + h2_off + (static_cast<int64_t>(t.row0 + b * 32 + r) * F + col) * 2) =
                   *reinterpret_cast<const uint4*>(src + 256 + ((c ^ sw ^ ((r >> 4) << 1)) << 4));
             }
@@ -626,10 +631,10 @@ static int fprop_impl(dm_operand a, const void* w, dm_operand c, dm_operand h2, 
                       int64_t max_rows, int64_t N, int64_t Kd, int fuse_swiglu, int clamped, float alpha, float limit,
                       const int* cond, int num_sms, int* status, void* stream) {
   if (!a.base || !w || !expert_offsets || e_local <= 0 || max_rows < 0 || N <= 0 || Kd <= 0) return kRcBadArg;
-  if (!c.base && !scatter_ptrs) return kRcBadArg;
+  if (!c.base && !scatter_ptrs && !fuse_swiglu) return kRcBadArg;  // the fused forward may leave h1 out
   if (e_local > kRwMaxGroups || max_rows > (1 << 30)) return kRcTooLarge;
   if ((Kd % 64) != 0 || (N % 8) != 0) return kRcUnsupportedShape;
-  if (fuse_swiglu && (((N / 2) % 128) != 0 || !h2.base || !c.base || scatter_ptrs)) return kRcUnsupportedShape;
+  if (fuse_swiglu && (((N / 2) % 128) != 0 || !h2.base || scatter_ptrs)) return kRcUnsupportedShape;
   if (max_rows == 0) return kRcOk;
   if (gather_ptrs != nullptr && gather_flags == nullptr) return kRcBadArg;
   RowsParams p{};

@@ -268,7 +268,8 @@ int dm_zero_padded_rows(void* routes_TKD, const void* ids, int ids_are_int64, in
  * use, what lies there.
  *
  *  dm_gemm_fprop:   C[r, :] = A[r, :] * W[e]^T           W = [e_local, N, Kd] (Kd contiguous)
- *     fuse_swiglu != 0: W = [e_local, 2, F, Kd]; writes h1 = C (2F wide) and h2 = SwiGLU(h1).
+ *     fuse_swiglu != 0: W = [e_local, 2, F, Kd]; writes h1 = C (2F wide; left out when c.base is null, for a forward
+ *     that nothing will differentiate) and h2 = SwiGLU(h1).
  *     scatter_ptrs != NULL: row r of C goes to scatter_ptrs[r] (peer memory) instead of C.
  *  dm_gemm_dgrad:   C[r, :] = A[r, :] * W[e]             W = [e_local, Kd, N] (N contiguous), A = [rows, Kd]
  *     scatter_ptrs as above.

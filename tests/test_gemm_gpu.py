@@ -313,3 +313,29 @@ def test_row_tiles_at_their_edges(counts, kd, n):
 @pytest.mark.parametrize("counts,kd,n", [([1, 32, 33, 257], 64, 256), ([300, 0, 191], 320, 768)])
 def test_fused_swiglu_row_tiles_at_their_edges(counts, kd, n):
     test_fprop_fused_swiglu(counts, kd, n)
+
+
+@pytest.mark.parametrize("counts,kd,f", [([1, 33], 64, 128), ([300, 0, 257], 192, 384)])
+def test_fused_swiglu_without_h1_writes_the_same_h2(counts, kd, f):
+    """A null C leaves h1 out and changes nothing else: h2 is equal bit for bit."""
+    nat = _native()
+    dev = torch.device("cuda", 0)
+    torch.manual_seed(9)
+    e = len(counts)
+    offs_t, off = _offsets(counts, dev)
+    rows = off[-1]
+    a = torch.zeros(rows + 300, kd, device=dev, dtype=torch.bfloat16)
+    a[:rows] = torch.randn(rows, kd, device=dev).bfloat16()
+    w = (torch.randn(e, 2 * f, kd, device=dev) * 0.1).bfloat16()
+    h1 = torch.zeros(rows + 300, 2 * f, device=dev, dtype=torch.bfloat16)
+    status = torch.zeros(8, dtype=torch.int32, device=dev)
+    op = lambda t: nat.Operand(t.data_ptr(), t.numel() * 2, None)  # noqa: E731
+    got = []
+    for c_op in (op(h1), nat.Operand(None, 0, None)):
+        h2 = torch.zeros(rows + 300, f, device=dev, dtype=torch.bfloat16)
+        nat.check(nat.lib.dm_gemm_fprop(op(a), w.data_ptr(), c_op, op(h2), None, offs_t.data_ptr(), e, rows, 2 * f, kd, 1, 0,
+                                        1.0, 0.0, None, 0, status.data_ptr(), nat.stream_ptr()), "dm_gemm_fprop")
+        got.append(h2)
+    torch.cuda.synchronize()
+    assert status[0].item() == 0
+    assert bool(h1[:rows].any()) and torch.equal(got[0], got[1])
