@@ -53,7 +53,7 @@ def kernel_source_digest() -> str:
     import hashlib
 
     h = hashlib.sha256()
-    for name in ("gemm_bf16.cu", "gemm_common.cuh", "common.cuh"):
+    for name in ("gemm_bf16.cu", "gemm_bf16_rows.cu", "gemm_common.cuh", "common.cuh"):
         h.update((ROOT / "dist_moe_b200" / "csrc" / name).read_bytes())
     return h.hexdigest()[:16]
 
@@ -787,7 +787,7 @@ def run_ours(args):
     peak_tf = pk.get("bf16_tflops_sustained") or pk["bf16_tflops"]
     achieved = flops_step * args.steps / (gemm_ms * 1e-3) / 1e12 if gemm_ms > 0 else None
     roofline = {
-        "kernel": "grouped_gemm_kernel<fprop|dgrad|wgrad> (tcgen05; 6 working launches per step, "
+        "kernel": "rows_gemm_kernel (forward, input gradient), wgrad_gemm_kernel (tcgen05; 6 working launches per step, "
                   "recompute launches are predicated off)",
         "bound": "tensor",
         "achieved": achieved,

@@ -13,6 +13,10 @@
 //               while the next tile's main loop already runs.
 //   warp 14     accumulator watcher.
 //
+// Bound: operand loads from L2 (48 KiB per 64-row stage and 128x256 tile) and, with few rows per expert, dW itself.  The
+// issuing warps stay converged (one lane in a divergent branch before): W13 8 experts x 3072 rows, D 2048, F 1408,
+// accumulated in place, 265 -> 215 us (1312 TFLOP/s); 64 x 384 359 -> 351 us.
+//
 // Groups are the local experts; their row ranges come from device memory
 // (expert_offsets), so the tile list is built by every CTA at kernel start and no
 // host read is needed.  Operands are addressed as (arena base, device

@@ -2,7 +2,7 @@
 //
 //   C[r, n] = sum_k  (A[r,k] * sfa[r, k/V]) * (W[e][n,k] * sfb[e][n, k/V])        V = 32 (MXFP8) or 16 (NVFP4)
 //
-// Same warp-specialised skeleton as the BF16 kernel (TMA producer warp, one MMA-issuing lane, eight
+// Same warp-specialised skeleton as the BF16 kernels (TMA producer warp, MMA-issuing warp, eight
 // epilogue warps, one 128 x 256 fp32 accumulator in TMEM).  Differences:
 //   * a pipeline stage is 128 bytes of K per row: 128 E4M3 or 256 packed E2M1 elements;
 //   * next to the A/B tiles the producer bulk-copies the stage's scale atoms.  Scales are
@@ -92,6 +92,10 @@ __device__ __forceinline__ BsTile bs_decode(int tile, int& e, const int* tile_st
 }
 
 // ---------------------------------------------------------------------------------------------------------
+// Measured when the issuing warps became converged (before: one lane each): NVFP4 65 536 rows W13 1010 -> 891 us, W2
+// 620 -> 588 us (four MMAs and twelve scale copies per stage share the tensor pipe: about 950 cycles); MXFP8 73 728 rows W13
+// 940 -> 869 us, input gradients 490 -> 452 and 923 -> 877 us (operand loads from L2, 12.8 TB/s), weight gradients
+// 804 -> 767 and 1655 -> 1563 us (dW read, added to and written: 4.1 TB/s of HBM).
 // 128 x 256 output tiles.  Per 128 bytes of K the tile moves 48 KiB of operands and needs, for NVFP4, twelve
 // scale-atom copies (about 47 cycles each, they serialise with the MMAs) per four 132-cycle MMAs; a 128 x 128
 // tile would spend more tensor-pipe time on its eight copies than on its four 69-cycle MMAs.  TMEM holds one
@@ -323,10 +327,9 @@ __global__ void __launch_bounds__(kWdThreads, 1) blockscaled_wide_kernel(const _
     __syncwarp();
   } else if (warp == 11 || warp == 10) {
     // ======================= scale copiers (the second one is also the accumulator watcher) =======================
-    // A thread issues a tcgen05 instruction every 50 to 100 cycles, and an NVFP4 stage needs twelve scale-atom
-    // copies next to its four MMAs; issued by one thread they cost more than the tensor pipe needs to run them.
-    // These two threads move every stage's atoms to the stage slot's TMEM columns and commit to a per-stage
-    // barrier the MMA thread waits on.  Columns: A atom a (K step a) at +4a; B atoms of the tile's lower and
+    // These two warps move every stage's atoms to the stage slot's TMEM columns and commit to a per-stage barrier the MMA
+    // warp waits on: an NVFP4 stage needs twelve copies next to its four MMAs, about 40 cycles of the tensor pipe each.
+    // Columns: A atom a (K step a) at +4a; B atoms of the tile's lower and
     // upper 128 columns side by side, 8 columns per K step.  The slot's previous MMAs are complete by then: the
     // producer refilled the stage only after their commit released it.  NVFP4 has four atoms per stage and
     // operand and each thread takes two; MXFP8 has one, taken by warp 11.

@@ -8,10 +8,10 @@
 // accumulator holds C transposed (TMEM lane = weight row, column = routed row).  A K stage then costs four MMAs of
 // N = 32 or 64 and eight scale-atom copies, and the weights stream through once.
 //
-//   * with MMAs this short the limit is how fast one thread can issue tcgen05 instructions (50 to 100 cycles
-//     each, measured; several issuing threads of one SM do not slow each other down).  So the scale-atom copies
-//     and the MMAs of a stage are issued by two different threads (the copier commits to a per-stage barrier the
-//     MMA thread waits on), and two CTAs share an SM, each with 256 TMEM columns and three stages;
+//   * with MMAs this short the issue of tcgen05 instructions counts.  The scale-atom copies and the MMAs of a stage are
+//     issued by two different warps (the copier commits to a per-stage barrier the MMA warp waits on), both converged around
+//     an elected lane (one lane in a divergent branch: W13 of 42 experts x 5632 x 2816 MXFP8 140.5 us, now 135 us; NVFP4
+//     32 x 4096 x 7168 116 us, now 112 us), and two CTAs share an SM, each with 256 TMEM columns and three stages;
 //   * a stage = 128 bytes of K: 16 KiB of weights (one TMA box), 4 or 8 KiB of routed rows (32-row boxes),
 //     and the stage's scale atoms of both;
 //   * the rows' scale atom covers 128 rows in four TMEM columns of 32 rows each, so a tile that starts at row

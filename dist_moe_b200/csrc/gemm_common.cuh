@@ -1,4 +1,4 @@
-// Helpers shared by the grouped GEMM kernels: epilogue staging tile, L2 reductions and the
+// Helpers shared by the grouped GEMM kernels: issue loops, epilogue staging tile, L2 reductions and the
 // host-side tensor-map encoding (through the driver entry point, no link-time libcuda).
 #pragma once
 
@@ -33,19 +33,10 @@ __device__ __forceinline__ uint4 pack8_bf16(const uint32_t* r) {
                     pack_bf16x2(__uint_as_float(r[6]), __uint_as_float(r[7])));
 }
 
-// Lean forms for the single-thread issue loops: barrier given by its shared-memory address, shared-memory
-// descriptors given by their lower word (address >> 4 | LBO >> 4 << 16) and a constant upper word.
-__device__ __forceinline__ uint32_t mbar_poll(uint32_t bar_addr, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t"
-      ".reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t"
-      "}\n"
-      : "=r"(ok) : "r"(bar_addr), "r"(parity) : "memory");
-  return ok;
-}
+// Forms for the issue loops: barriers given by their shared-memory address, shared-memory matrix descriptors by their
+// lower word (address >> 4 | LBO >> 4 << 16) and a constant upper word (SBO >> 4, version 1 in bit 14, 128-byte swizzle 2
+// in bits 29 to 31).  K-major operand: rows of 128 bytes, 8-row groups SBO = 1024 apart.  MN-major operand: lines of 128
+// bytes of M or N, one line per k, 8-k groups SBO = 1024 apart, the next 128 bytes of M or N LBO apart.
 // ---------------------------------------------------------------------------
 // Issuing warps.  tcgen05 and TMA instructions take their operands from uniform registers.  Code that only one lane runs
 // (`if (lane == 0)`) keeps everything in per-lane registers and moves each operand over for each instruction: 85 to 93
@@ -73,12 +64,6 @@ __device__ __forceinline__ uint32_t mbar_test(uint32_t bar_addr, uint32_t parity
       : "=r"(ok) : "r"(bar_addr), "r"(parity) : "memory");
   return ok;
 }
-// A bare polling loop (a million polls, tens of milliseconds), then the timed wait that can give up.
-__device__ __forceinline__ bool mbar_wait_lean(uint32_t bar_addr, uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
-  for (uint32_t i = 0; i < (1u << 20); ++i)
-    if (mbar_poll(bar_addr, parity)) return true;
-  return mbar_wait(bar, parity, abort_flag);
-}
 __device__ __forceinline__ void umma_bf16_lo(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t desc_hi,
                                              uint32_t idesc, uint32_t accumulate) {
   asm volatile(
@@ -93,7 +78,7 @@ __device__ __forceinline__ void umma_bf16_lo(uint32_t d_tmem, uint32_t a_lo, uin
       ::"r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(desc_hi), "r"(idesc), "r"(accumulate)
       : "memory");
 }
-// Block-scaled MMAs (see common.cuh) with descriptors given by their lower words.
+// Block-scaled MMAs: scale factors live in TMEM (copied there by tcgen05.cp from shared memory).
 __device__ __forceinline__ void umma_mxf8_lo(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t desc_hi, uint32_t idesc,
                                              uint32_t sfa_tmem, uint32_t sfb_tmem, uint32_t accumulate) {
   asm volatile(
