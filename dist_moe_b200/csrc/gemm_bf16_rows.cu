@@ -108,7 +108,8 @@ __device__ __forceinline__ RowsTile rw_decode(int tile, int& e, const int* tile_
   return t;
 }
 
-enum RowsMode : int { kRowsFprop = 0, kRowsDgrad = 1, kRowsSwiglu = 2 };  // kRowsSwiglu: W13 forward with SwiGLU
+// kRowsSwiglu: W13 forward with SwiGLU.  The values also name the kernel in a timeout status (2 is the weight gradient).
+enum RowsMode : int { kRowsFprop = 0, kRowsDgrad = 1, kRowsSwiglu = 3 };
 
 // Word of two neighbouring columns of one row from words of one column of two neighbouring rows: lanes 2p and 2p + 1
 // hold columns 2p and 2p + 1 of the rows (t, t + 1); the even lane receives row t, the odd lane row t + 1.
