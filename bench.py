@@ -53,7 +53,7 @@ def kernel_source_digest() -> str:
     import hashlib
 
     h = hashlib.sha256()
-    for name in ("gemm_bf16.cu", "gemm_bf16_rows.cu", "gemm_common.cuh", "common.cuh"):
+    for name in ("gemm_bf16.cu", "gemm_bf16_rows.cu", "row_tiles.cuh", "gemm_common.cuh", "common.cuh"):
         h.update((ROOT / "dist_moe_b200" / "csrc" / name).read_bytes())
     return h.hexdigest()[:16]
 

@@ -1,0 +1,66 @@
+// How the BF16 forward and input-gradient GEMMs split an expert's routed rows into tiles, and which gathered row blocks a
+// tile needs.  Plain arithmetic, for the kernel and for host code.
+#pragma once
+
+#include <stdint.h>
+
+#ifdef __CUDACC__
+#define DM_HOST_DEVICE __host__ __device__ __forceinline__
+#else
+#define DM_HOST_DEVICE inline
+#endif
+
+namespace dm {
+
+constexpr int kRwMaxN = 256;          // routed rows per tile (N side of the MMA)
+constexpr int kRwGatherBlock = 128;   // rows per readiness counter of the fused dispatch
+constexpr int kRwBoxes = 5;           // heights of the row boxes: the smallest one that covers half a tile is loaded
+
+// A CTA of the pair loads half of a tile's rows.
+DM_HOST_DEVICE constexpr int rw_box_rows(int i) { return i == 0 ? 16 : 32 * i; }
+DM_HOST_DEVICE constexpr int rw_box_index(int n) { return n <= 32 ? 0 : (n + 63) >> 6; }
+
+// Row tiles of an expert and the rows each of them takes (the last one what is left): equal tiles, multiples of 32.
+DM_HOST_DEVICE constexpr int rw_row_tiles(int rows) { return (rows + kRwMaxN - 1) / kRwMaxN; }
+DM_HOST_DEVICE constexpr int rw_rows_per_tile(int rows) {
+  return rows > 0 ? ((rows + rw_row_tiles(rows) - 1) / rw_row_tiles(rows) + 31) & ~31 : 32;
+}
+
+struct RowsTile {
+  int e, pair, row0, rows, n;  // rows: real rows of the tile, n: the MMA's N (rows rounded up to 32)
+};
+
+// `rows_per_tile[e]` rows per tile of an expert; consecutive tiles share the weight block (`pair` of column blocks).
+DM_HOST_DEVICE RowsTile rw_decode(int tile, int& e, const int* tile_start, const int* off, const uint16_t* rows_per_tile) {
+  while (tile >= tile_start[e + 1]) ++e;
+  const int local = tile - tile_start[e];
+  const int rows = off[e + 1] - off[e];
+  const int per = rows_per_tile[e];
+  const int nt = rw_row_tiles(rows);
+  RowsTile t;
+  t.e = e;
+  t.pair = local / nt;
+  const int first = (local - t.pair * nt) * per;
+  t.row0 = off[e] + first;
+  const int left = rows - first;
+  t.rows = left < per ? left : per;
+  if (t.rows < 0) t.rows = 0;
+  t.n = t.rows > 0 ? (t.rows + 31) & ~31 : 32;
+  return t;
+}
+
+// Row blocks [first, last] that hold the tile's rows.  Nothing about a tile's blocks follows from what an earlier tile of
+// the same CTA waited for: a CTA's next tile may lie in a later column block and start at an earlier row, and the blocks
+// between two tiles of one CTA are pulled for other CTAs.
+struct RowsBlocks {
+  int first, last;
+};
+DM_HOST_DEVICE RowsBlocks rw_tile_blocks(const RowsTile& t, int total_rows) {
+  const int end = t.row0 + t.n < total_rows ? t.row0 + t.n : total_rows;
+  RowsBlocks b;
+  b.first = t.row0 / kRwGatherBlock;
+  b.last = (end - 1) / kRwGatherBlock;
+  return b;
+}
+
+}  // namespace dm

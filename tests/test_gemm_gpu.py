@@ -299,6 +299,61 @@ def test_fused_dispatch_gathers_rows_inside_the_gemm(mode):
                 _close(out[lo:hi], a_ref[lo:hi].float() @ wt, f"{mode} dispatch expert {ei}")
 
 
+@pytest.mark.parametrize("mode", ["fprop", "swiglu", "dgrad"])
+@pytest.mark.parametrize("counts,kd,n,num_sms", [
+    ([2048], 256, 1024, 6),              # 32 tiles on three CTA pairs: each returns to earlier rows in later column blocks
+    ([1000, 0, 77, 600], 64, 768, 9),    # one stage per tile; an odd SM limit
+    ([2100, 513, 31], 256, 3072, 0),     # the whole device, more tiles than pairs
+])
+def test_fused_dispatch_with_several_tiles_per_cta_pair(counts, kd, n, num_sms, mode):
+    """The persistent form: pairs take several tiles, going back to earlier rows.  The operand that the rows are pulled into
+    holds NaNs before every launch, so a tile that is computed from rows which have not arrived shows."""
+    nat = _native()
+    dev = torch.device("cuda", 0)
+    torch.manual_seed(8)
+    e, f = len(counts), n // 2
+    offs_t, off = _offsets(counts, dev)
+    rows = off[-1]
+    src = torch.randn(3000, kd, device=dev).bfloat16()
+    idx = torch.randint(0, 3000, (rows,), device=dev)
+    ptrs = src.data_ptr() + idx.to(torch.int64) * kd * 2
+    ptrs[rows // 2] = 0
+    a_ref = src[idx].clone()
+    a_ref[rows // 2] = 0
+    w = (torch.randn(e, kd, n, device=dev) if mode == "dgrad" else torch.randn(e, n, kd, device=dev)).mul_(0.1).bfloat16()
+    a_buf = torch.empty((rows + 300) * kd, device=dev, dtype=torch.bfloat16)
+    out = torch.empty(rows, n, device=dev, dtype=torch.bfloat16)
+    h2 = torch.empty(rows, f, device=dev, dtype=torch.bfloat16)
+    flags = torch.full((rows // 128 + 2,), 77, dtype=torch.int32, device=dev)
+    status = torch.zeros(8, dtype=torch.int32, device=dev)
+    op = lambda t: nat.Operand(t.data_ptr(), t.numel() * 2, None)  # noqa: E731
+    none = nat.Operand(None, 0, None)
+    for _ in range(3):
+        for t in (a_buf, out, h2):
+            t.fill_(float("nan"))
+        if mode == "dgrad":
+            rc = nat.lib.dm_gemm_dgrad_dispatch(ptrs.data_ptr(), flags.data_ptr(), op(a_buf), w.data_ptr(), op(out),
+                                                offs_t.data_ptr(), e, rows, n, kd, None, num_sms, status.data_ptr(),
+                                                nat.stream_ptr())
+        else:
+            rc = nat.lib.dm_gemm_fprop_dispatch(ptrs.data_ptr(), flags.data_ptr(), op(a_buf), w.data_ptr(), op(out),
+                                                op(h2) if mode == "swiglu" else none, offs_t.data_ptr(), e, rows, n, kd,
+                                                int(mode == "swiglu"), 0, 1.0, 0.0, None, num_sms, status.data_ptr(),
+                                                nat.stream_ptr())
+        nat.check(rc, "dispatch gemm")
+        torch.cuda.synchronize()
+        assert status[0].item() == 0, status.tolist()
+        assert torch.equal(a_buf[: rows * kd].view(torch.int16), a_ref.view(torch.int16).reshape(-1)), "gathered rows differ"
+        for ei in range(e):
+            lo, hi = off[ei], off[ei + 1]
+            if hi > lo:
+                wt = w[ei].float() if mode == "dgrad" else w[ei].float().T
+                _close(out[lo:hi], a_ref[lo:hi].float() @ wt, f"{mode} dispatch expert {ei}")
+        if mode == "swiglu":
+            gate, up = out[:, :f].float(), out[:, f:].float()
+            _close(h2, gate * torch.sigmoid(gate) * up, "h2")
+
+
 @pytest.mark.parametrize("counts,kd,n", [
     ([1, 31, 32, 33], 64, 64),           # one stage; tiles of 32 rows, a column block past the matrix in either CTA
     ([255, 0, 256, 257], 192, 392),      # tiles of 256 and 160 rows; a width that is only a multiple of 8
