@@ -336,8 +336,8 @@ static inline int sm_count() {
   return n;
 }
 
-// Grid of a persistent one-CTA-per-SM kernel: the caller's wish, never more than the device has SMs.  The fused
-// dispatch launches make CTAs wait on counters that other CTAs publish, so every CTA must be resident.
+// Grid of a persistent one-CTA-per-SM kernel: the caller's wish, never more than the device has SMs.  No kernel needs all
+// of its CTAs to be resident at once.
 static inline int persistent_grid(int num_sms) {
   const int n = sm_count();
   return (num_sms > 0 && num_sms < n) ? num_sms : n;

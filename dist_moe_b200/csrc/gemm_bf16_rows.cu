@@ -68,6 +68,7 @@ struct RowsParams {
   const int64_t* scatter_ptrs;
   const int64_t* gather_ptrs;  // fused dispatch: row r of A is pulled from gather_ptrs[r] (may be peer memory)
   int* gather_flags;           // one counter per 128-row block of A, zero before the launch
+  int* gather_ticket;          // next unit to pull, zero before the launch
   uint8_t* a_base;             // where the pulled rows land (the A operand itself)
   const int32_t* expert_offsets;
   const int* cond;
@@ -115,6 +116,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kRwThreads, 1) rows_
   const int lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();
   const int first_tile = blockIdx.x >> 1, tile_step = gridDim.x >> 1;
+
+  // The first gather warp's unit, on its way while the tables are built; the other three draw only where there are more
+  // units than CTAs.  32 decoding tokens (24 units of 8 rows, 208 us in all) take 0.3 us longer than with units dealt out
+  // by CTA index, 0.8 us longer when all four warps draw, 1.4 us when a CTA draws four units at once.
+  int unit = 0;
+  if (warp == 10 && lane == 0 && p.gather_flags != nullptr) unit = atomicAdd(p.gather_ticket, 1);
 
   // ---- tile table -----------------------------------------------------------
   const int m_pairs = kSwiglu ? (p.N / 2) / 128 : (p.N + 2 * kRwBM - 1) / (2 * kRwBM);
@@ -342,19 +349,27 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kRwThreads, 1) rows_
     }
   } else if (warp >= 10) {
     // ======================= gather (fused dispatch) =======================
-    // Units of 8 rows are dealt round-robin over all gather warps of the grid in ascending row order, the order
-    // in which the tiles consume them.  Each warp pulls its unit with 16-byte loads (peer memory allowed), two rows
+    // Units of 8 rows go to the gather warps of the grid by ticket, in ascending row order, the order in which the tiles
+    // consume them.  Each warp pulls its unit with 16-byte loads (peer memory allowed), two rows
     // x eight loads in flight per lane, and then bumps the counter of the unit's 128-row block; the TMA producer of
-    // whichever CTA needs a block waits for sixteen reports.  Gather warps wait on nothing.  Small units matter at
-    // the start of the launch: a warp keeps 8 KiB in flight, so over NVLink a 32-row unit took about 30 us before
+    // whichever CTA needs a block waits for sixteen reports.  Gather warps wait on nothing, and a unit belongs only to a
+    // warp that is running: CTAs that come late, because kernels of other streams hold their SMs, delay no row that the
+    // CTAs already there are waiting for (dealt out by CTA index, such rows never came and the wait ran out).  Small units
+    // matter at the start of the launch: a warp keeps 8 KiB in flight, so over NVLink a 32-row unit took about 30 us before
     // the first tiles could begin, an 8-row unit a quarter of that, and later units are far ahead of the MMAs anyway.
     if (p.gather_flags != nullptr) {
-      const int gw = warp - 10;
       const int total_rows = s_off[p.e_local];
-      const int nblocks = (total_rows + kRwGatherBlock - 1) / kRwGatherBlock;
+      const int units = (total_rows + kRwGatherBlock - 1) / kRwGatherBlock * kRwGatherUnitsPerBlock;
+      if (warp != 10) {
+        unit = units;  // no more units than first warps: those are enough
+        if (units > static_cast<int>(gridDim.x) && lane == 0) unit = atomicAdd(p.gather_ticket, 1);
+      }
       const int vec_per_row = p.Kd / 8;
       uint4* dst_base = reinterpret_cast<uint4*>(p.a_base + a_off);
-      for (int u = gw * gridDim.x + blockIdx.x; u < nblocks * kRwGatherUnitsPerBlock; u += kRwGatherWarps * gridDim.x) {
+      int u = uniform(unit);
+      while (u < units) {
+        int next = 0;
+        if (lane == 0) next = atomicAdd(p.gather_ticket, 1);  // on its way while this unit is pulled
         const int blk = u / kRwGatherUnitsPerBlock;
         const int r_begin = blk * kRwGatherBlock + (u % kRwGatherUnitsPerBlock) * kRwGatherUnitRows;
         for (int rr = 0; rr < kRwGatherUnitRows; rr += 2) {
@@ -385,6 +400,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kRwThreads, 1) rows_
         __threadfence();
         __syncwarp();
         if (lane == 0) red_release_gpu_add(p.gather_flags + blk, 1);
+        u = uniform(next);
       }
     }
   } else {
@@ -538,7 +554,7 @@ static int rows_launch(const RowsParams& p, int num_sms, cudaStream_t st) {
                                                  static_cast<int>(kRwDynSmem)));
   });
   if (rc != 0) return rc;
-  const int grid = pair_grid(rows_gemm_kernel<kMode>, kRwThreads, kRwDynSmem, num_sms);
+  const int grid = pair_grid(num_sms);
   rows_gemm_kernel<kMode><<<grid, kRwThreads, kRwDynSmem, st>>>(p);
   return static_cast<int>(cudaGetLastError());
 }
@@ -563,6 +579,9 @@ static int encode_w13(CUtensorMap* tm, const void* w, int64_t experts, int64_t F
 
 using namespace dm;
 
+// gather_flags: a counter per 128-row block, then the ticket.
+static int64_t ticket_slot(int64_t max_rows) { return (max_rows + kRwGatherBlock - 1) / kRwGatherBlock; }
+
 // What the forward and the input gradient share: row maps, row destinations, dispatch counters.
 static int rows_setup(RowsParams& p, const dm_operand& a, const dm_operand& c, const int64_t* scatter_ptrs,
                       const int64_t* gather_ptrs, int32_t* gather_flags, const int32_t* expert_offsets, int e_local,
@@ -577,6 +596,7 @@ static int rows_setup(RowsParams& p, const dm_operand& a, const dm_operand& c, c
   p.scatter_ptrs = scatter_ptrs;
   p.gather_ptrs = gather_ptrs;
   p.gather_flags = gather_ptrs ? gather_flags : nullptr;
+  p.gather_ticket = gather_ptrs ? gather_flags + ticket_slot(max_rows) : nullptr;
   p.a_base = static_cast<uint8_t*>(a.base);
   p.expert_offsets = expert_offsets;
   p.cond = cond;
@@ -591,7 +611,7 @@ static int rows_setup(RowsParams& p, const dm_operand& a, const dm_operand& c, c
 static int clear_flags(const int64_t* gather_ptrs, int32_t* gather_flags, int64_t max_rows, cudaStream_t st) {
   if (gather_ptrs == nullptr) return kRcOk;
   return static_cast<int>(
-      cudaMemsetAsync(gather_flags, 0, sizeof(int32_t) * static_cast<size_t>((max_rows + 127) / 128 + 1), st));
+      cudaMemsetAsync(gather_flags, 0, sizeof(int32_t) * static_cast<size_t>(ticket_slot(max_rows) + 1), st));
 }
 
 static int fprop_impl(dm_operand a, const void* w, dm_operand c, dm_operand h2, const int64_t* scatter_ptrs,

@@ -224,34 +224,11 @@ static inline EncodeTiledFn get_encode() {
   return fn;
 }
 
-// Grid of a persistent kernel of CTA pairs, one CTA per SM: the caller's wish, never more pairs than the device can hold
-// at once (CTAs wait on counters that other CTAs publish, so every one of them must be resident).
-template <class Kernel>
-static inline int pair_grid(Kernel kernel, int threads, size_t smem, int num_sms) {
-  static int resident[kMaxDevices] = {};  // per kernel signature; kernels that share one share their launch shape
-  const int slot = current_device_slot();
-  int clusters = slot >= 0 ? resident[slot] : 0;
-  if (clusters <= 0) {
-    cudaLaunchConfig_t cfg{};
-    cudaLaunchAttribute attr{};
-    attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = 2;
-    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-    cfg.gridDim = dim3(static_cast<unsigned>(sm_count() / 2 * 2));
-    cfg.blockDim = dim3(static_cast<unsigned>(threads));
-    cfg.dynamicSmemBytes = smem;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
-    if (cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) != cudaSuccess || clusters <= 0) {
-      cudaGetLastError();
-      clusters = sm_count() / 2;
-    }
-    if (clusters > sm_count() / 2) clusters = sm_count() / 2;
-    if (slot >= 0) resident[slot] = clusters;
-  }
-  const int wish = persistent_grid(num_sms) / 2;
-  const int n = wish < clusters ? wish : clusters;
-  return 2 * (n > 0 ? n : 1);
+// Grid of a persistent kernel of CTA pairs, one CTA per SM: whole pairs within the caller's limit (one less for an odd
+// limit), at least one pair.
+static inline int pair_grid(int num_sms) {
+  const int pairs = persistent_grid(num_sms) / 2;
+  return 2 * (pairs > 0 ? pairs : 1);
 }
 
 // bf16 matrix [rows][cols], cols contiguous; box = box_rows x 64 columns.

@@ -273,6 +273,8 @@ int dm_zero_padded_rows(void* routes_TKD, const void* ids, int ids_are_int64, in
  *     scatter_ptrs != NULL: row r of C goes to scatter_ptrs[r] (peer memory) instead of C.
  *  dm_gemm_dgrad:   C[r, :] = A[r, :] * W[e]             W = [e_local, Kd, N] (N contiguous), A = [rows, Kd]
  *     scatter_ptrs as above.
+ *  num_sms (0 = the whole device) bounds the SMs a launch occupies.  dm_gemm_fprop and dm_gemm_dgrad run on pairs of
+ *  neighbouring SMs: an odd bound is used down to the next even number, 1 takes one pair.
  *  dm_gemm_wgrad:   dW[e] (+)= dY[e]^T * X[e]            dY = [rows, N], X = [rows, Kd], dW = [e_local, N, Kd]
  *     out_is_fp32 selects fp32 or bf16 dW; accumulate != 0 adds into dW (the fp32 accumulator is rounded to
  *     dW's type and added in L2 by bulk tensor reduce-adds, the reference's TMA reduce-add store).  dW must be
@@ -295,7 +297,9 @@ int dm_gemm_dgrad(dm_operand a, const void* w, dm_operand c, const int64_t* scat
  * allowed) by four extra warps of every CTA of the persistent kernel while the tensor cores already work
  * on the rows that have landed; `a` names where the pulled rows are kept (x_gathered / grad_h3_gathered,
  * needed again by the weight-gradient GEMMs).  gather_flags: int32[max_rows/128 + 2] scratch, cleared by
- * the call.  Replaces dist_grouped_gemm_fprop_dispatch / ..._dgrad_dispatch in one launch
+ * the call; it belongs to this launch until it has finished.  Rows are pulled only by CTAs that are running, so
+ * kernels of other streams that hold SMs delay the call but do not fail it.  Replaces
+ * dist_grouped_gemm_fprop_dispatch / ..._dgrad_dispatch in one launch
  * (dist_moe/kernels/dist_grouped_gemm.py:1148-1237, 1441-1489). */
 int dm_gemm_fprop_dispatch(const int64_t* gather_ptrs, int32_t* gather_flags, dm_operand a, const void* w,
                            dm_operand c, dm_operand h2, const int32_t* expert_offsets, int e_local, int64_t max_rows,

@@ -354,6 +354,44 @@ def test_fused_dispatch_with_several_tiles_per_cta_pair(counts, kd, n, num_sms, 
             _close(h2, gate * torch.sigmoid(gate) * up, "h2")
 
 
+def test_fused_dispatch_beside_kernels_that_hold_single_sms():
+    """Launches of another stream hold an odd number of SMs, so some CTA pairs of the dispatch come late: the rows reach the
+    tiles of the pairs that run, and the results are those of the same call alone."""
+    nat = _native()
+    dev = torch.device("cuda", 0)
+    torch.manual_seed(11)
+    kd, n, counts = 512, 1024, [900, 1300, 2000]
+    e = len(counts)
+    offs_t, off = _offsets(counts, dev)
+    rows = off[-1]
+    src = torch.randn(rows, kd, device=dev).bfloat16()
+    ptrs = src.data_ptr() + torch.randperm(rows, device=dev).to(torch.int64) * kd * 2
+    w = (torch.randn(e, n, kd, device=dev) * 0.1).bfloat16()
+    big = torch.randn(16384 + 300, 1024, device=dev).bfloat16()
+    big_offs, _ = _offsets([16384], dev)
+    dw = torch.empty(1024, 1024, device=dev, dtype=torch.float32)
+    status = torch.zeros(8, dtype=torch.int32, device=dev)
+    op = lambda t: nat.Operand(t.data_ptr(), t.numel() * 2, None)  # noqa: E731
+    side = torch.cuda.Stream()
+    got = []
+    for busy in (False, True):
+        a_buf = torch.full(((rows + 300) * kd,), float("nan"), device=dev, dtype=torch.bfloat16)
+        out = torch.full((rows, n), float("nan"), device=dev, dtype=torch.bfloat16)
+        flags = torch.zeros(rows // 128 + 2, dtype=torch.int32, device=dev)
+        torch.cuda.synchronize()
+        if busy:
+            for _ in range(10):
+                nat.check(nat.lib.dm_gemm_wgrad(op(big), op(big), dw.data_ptr(), 1, 0, big_offs.data_ptr(), 1, 16384, 1024, 1024,
+                                                31, status.data_ptr(), side.cuda_stream), "wgrad")
+        nat.check(nat.lib.dm_gemm_fprop_dispatch(ptrs.data_ptr(), flags.data_ptr(), op(a_buf), w.data_ptr(), op(out),
+                                                 nat.Operand(None, 0, None), offs_t.data_ptr(), e, rows, n, kd, 0, 0, 1.0, 0.0,
+                                                 None, 0, status.data_ptr(), nat.stream_ptr()), "dispatch")
+        torch.cuda.synchronize()
+        assert status[0].item() == 0, status.tolist()
+        got.append(out)
+    assert bool(torch.isfinite(got[0]).all()) and torch.equal(got[0], got[1])
+
+
 @pytest.mark.parametrize("counts,kd,n", [
     ([1, 31, 32, 33], 64, 64),           # one stage; tiles of 32 rows, a column block past the matrix in either CTA
     ([255, 0, 256, 257], 192, 392),      # tiles of 256 and 160 rows; a width that is only a multiple of 8
