@@ -81,6 +81,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) wgrad_gemm_kernel(const __gri
   __shared__ uint64_t tmem_empty_bar[2];
   __shared__ uint32_t tmem_base_slot;
   __shared__ int abort_flag;
+  __shared__ volatile int s_first_bad;  // first of this CTA's tiles whose accumulator never came
   __shared__ int s_off[kMaxGroups + 1];
   __shared__ int s_tile_start[kMaxGroups + 1];
 
@@ -96,6 +97,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) wgrad_gemm_kernel(const __gri
   }
   if (threadIdx.x == 0) {
     abort_flag = 0;
+    s_first_bad = kNoBadTile;
     for (int s = 0; s < kStages; ++s) {
       mbar_init(&full_bar[s], 1);
       mbar_init(&empty_bar[s], 1);
@@ -243,16 +245,15 @@ __global__ void __launch_bounds__(kGemmThreads, 1) wgrad_gemm_kernel(const __gri
     // ======================= accumulator watcher =======================
     // One warp polls the accumulator-ready barriers on behalf of the eight epilogue warps and releases them
     // through a hardware named barrier: the epilogue warps then sleep without taking issue slots from the
-    // MMA-issuing and TMA-issuing threads that share their schedulers.  The watcher arrives for every tile,
-    // also after a timeout, so that no epilogue warp is left blocked.
+    // MMA-issuing and TMA-issuing threads that share their schedulers.  After a timeout it releases them once more and stops.
     bool ok = true;
     int it = 0;
-    for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x, ++it) {
+    for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x, ++it) {
       const int buf = it & 1;
       const uint32_t acc_phase = (it >> 1) & 1u;
-      if (ok && lane == 0) ok = mbar_wait(&tmem_full_bar[buf], acc_phase, &abort_flag);
+      if (lane == 0) ok = handover_report(&s_first_bad, it, mbar_wait(&tmem_full_bar[buf], acc_phase, &abort_flag));
       ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
-      asm volatile("bar.arrive %0, %1;" ::"r"(1 + buf), "r"(8 * 32 + 32) : "memory");
+      asm volatile("bar.arrive %0, %1;" ::"r"(handover_barrier(it)), "r"(8 * 32 + 32) : "memory");
     }
   } else if (warp < 10) {
     // ======================= epilogue =======================
@@ -267,10 +268,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1) wgrad_gemm_kernel(const __gri
     for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x, ++it) {
       const Tile t = decode_tile(tile, e, s_tile_start, s_off, n_tiles);
       const int buf = it & 1;
-      const uint32_t acc_phase = (it >> 1) & 1u;
-      asm volatile("bar.sync %0, %1;" ::"r"(1 + buf), "r"(8 * 32 + 32) : "memory");  // released by the watcher
-      (void)acc_phase;
-      ok = abort_flag == 0;
+      asm volatile("bar.sync %0, %1;" ::"r"(handover_barrier(it)), "r"(8 * 32 + 32) : "memory");  // released by the watcher
+      ok = handover_good(&s_first_bad, it);  // the same for every epilogue warp
       if (!ok) break;
       tcgen05_fence_after();
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + buf * kBN;

@@ -131,7 +131,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kRwThreads, 1) rows_
   }
   if (threadIdx.x == 0) {
     abort_flag = 0;
-    s_first_bad = 0x7fffffff;
+    s_first_bad = kNoBadTile;
     for (int s = 0; s < kRwMaxStages; ++s) {
       mbar_init(&full_bar[s], 1);
       mbar_init(&empty_bar[s], 1);
@@ -332,20 +332,15 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kRwThreads, 1) rows_
     // ======================= accumulator watcher =======================
     // One warp polls the accumulator-ready barriers on behalf of the eight epilogue warps and releases them
     // through a hardware named barrier: the epilogue warps then sleep without taking issue slots from the
-    // MMA-issuing and TMA-issuing threads that share their schedulers.  The watcher arrives for every tile,
-    // also after a timeout, so that no epilogue warp is left blocked.
+    // MMA-issuing and TMA-issuing threads that share their schedulers.  After a timeout it releases them once more and stops.
     bool ok = true;
     int it = 0;
-    for (int tile = first_tile; tile < total_tiles; tile += tile_step, ++it) {
+    for (int tile = first_tile; tile < total_tiles && ok; tile += tile_step, ++it) {
       const int buf = it & 1;
       const uint32_t acc_phase = (it >> 1) & 1u;
-      if (ok && lane == 0) ok = mbar_wait(&tmem_full_bar[buf], acc_phase, &abort_flag);
-      if (!ok && lane == 0 && s_first_bad > it) {
-        s_first_bad = it;
-        __threadfence_block();
-      }
+      if (lane == 0) ok = handover_report(&s_first_bad, it, mbar_wait(&tmem_full_bar[buf], acc_phase, &abort_flag));
       ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
-      asm volatile("bar.arrive %0, %1;" ::"r"(1 + buf), "r"(8 * 32 + 32) : "memory");
+      asm volatile("bar.arrive %0, %1;" ::"r"(handover_barrier(it)), "r"(8 * 32 + 32) : "memory");
     }
   } else if (warp >= 10) {
     // ======================= gather (fused dispatch) =======================
@@ -413,7 +408,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kRwThreads, 1) rows_
     const int quad = warp & 3;  // TMEM lanes [32*quad, 32*quad+32)
     const int half = ew >> 2;
     uint8_t* stg = smem + kRing + half * kStaging;
-    const int bar_id = 3 + half;
+    const int bar_id = 1 + kHandoverBarriers + half;
     const uint32_t lead_empty = cluster_addr(smem_u32(&tmem_empty_bar[0]), 0);
     const int odd = lane & 1;
     int e = 0, it = 0;
@@ -436,9 +431,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kRwThreads, 1) rows_
         return reinterpret_cast<uint64_t>(p.c_base) + c_off + static_cast<uint64_t>(t.row0 + r) * p.N * 2;
       };
       uint64_t my_row = b_begin < b_end ? row_ptr(b_begin) : 0;
-      asm volatile("bar.sync %0, %1;" ::"r"(1 + buf), "r"(8 * 32 + 32) : "memory");  // released by the watcher
-      // Every warp of a group takes the same decision: the watcher records the first bad tile before it arrives for it.
-      ok = it < s_first_bad;
+      asm volatile("bar.sync %0, %1;" ::"r"(handover_barrier(it)), "r"(8 * 32 + 32) : "memory");  // released by the watcher
+      ok = handover_good(&s_first_bad, it);  // the same for every epilogue warp
       if (!ok) break;
       tcgen05_fence_after();
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + buf * kRwMaxN;

@@ -133,6 +133,7 @@ __global__ void __launch_bounds__(kWdThreads, 1) blockscaled_wide_kernel(const _
   __shared__ uint64_t tmem_empty_bar;
   __shared__ uint32_t tmem_base_slot;
   __shared__ int abort_flag;
+  __shared__ volatile int s_first_bad;  // first of this CTA's tiles whose accumulator never came
   __shared__ int s_off[kBsMaxGroups + 1];
   __shared__ int s_tile_start[kBsMaxGroups + 1];
 
@@ -150,6 +151,7 @@ __global__ void __launch_bounds__(kWdThreads, 1) blockscaled_wide_kernel(const _
   }
   if (threadIdx.x == 0) {
     abort_flag = 0;
+    s_first_bad = kNoBadTile;
     for (int s = 0; s < kWdMaxStages; ++s) {
       mbar_init(&full_bar[s], 1);
       mbar_init(&empty_bar[s], 1);
@@ -335,7 +337,7 @@ __global__ void __launch_bounds__(kWdThreads, 1) blockscaled_wide_kernel(const _
     // operand and each thread takes two; MXFP8 has one, taken by warp 11.
     //
     // Warp 10 then polls the accumulator-ready barrier for the epilogue warps and releases them through a hardware
-    // named barrier; it arrives for every tile, also after a timeout, so that no epilogue warp is left blocked.
+    // named barrier; after a timeout it releases them once more and stops.
     const bool watcher = warp == 10;
     const bool elected = elect_one();
     const uint32_t sf0 = uniform(smem_u32(&sf_bar[0]));
@@ -345,8 +347,8 @@ __global__ void __launch_bounds__(kWdThreads, 1) blockscaled_wide_kernel(const _
     int e = 0, it = 0;
     bool ok = true;
     const uint32_t sf_bytes = atoms * 512;
-    for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x, ++it) {
-      if (a_hi > a_lo && ok) {
+    for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x, ++it) {
+      if (a_hi > a_lo) {
         const BsTile t = bs_decode(tile, e, s_tile_start, s_off, p.mode, n_tiles, p.k_iters);
         const int k_iters = uniform(t.k_iters);
 #pragma unroll 1
@@ -372,9 +374,9 @@ __global__ void __launch_bounds__(kWdThreads, 1) blockscaled_wide_kernel(const _
         }
       }
       if (watcher) {
-        if (ok && lane == 0) ok = mbar_wait(&tmem_full_bar, it & 1u, &abort_flag);
+        if (lane == 0) ok = handover_report(&s_first_bad, it, ok && mbar_wait(&tmem_full_bar, it & 1u, &abort_flag));
         ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
-        asm volatile("bar.arrive %0, %1;" ::"r"(1 + (it & 1)), "r"(8 * 32 + 32) : "memory");
+        asm volatile("bar.arrive %0, %1;" ::"r"(handover_barrier(it)), "r"(8 * 32 + 32) : "memory");
       }
     }
     __syncwarp();
@@ -395,8 +397,8 @@ __global__ void __launch_bounds__(kWdThreads, 1) blockscaled_wide_kernel(const _
         p.row_inv_base ? reinterpret_cast<const float*>(p.row_inv_base + (p.row_inv_off ? *p.row_inv_off : 0)) : nullptr;
     for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x, ++it) {
       const BsTile t = bs_decode(tile, e, s_tile_start, s_off, p.mode, n_tiles, p.k_iters);
-      asm volatile("bar.sync %0, %1;" ::"r"(1 + (it & 1)), "r"(8 * 32 + 32) : "memory");  // released by the watcher
-      ok = abort_flag == 0;
+      asm volatile("bar.sync %0, %1;" ::"r"(handover_barrier(it)), "r"(8 * 32 + 32) : "memory");  // released by the watcher
+      ok = handover_good(&s_first_bad, it);  // the same for every epilogue warp
       if (!ok) break;
       tcgen05_fence_after();
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quad * 32) << 16);

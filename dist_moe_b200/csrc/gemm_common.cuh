@@ -5,6 +5,7 @@
 #include <cuda.h>
 
 #include "common.cuh"
+#include "tile_handover.cuh"
 #include "../../include/dist_moe_b200.h"
 
 namespace dm {
