@@ -80,6 +80,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) wgrad_gemm_kernel(const __gri
   __shared__ uint64_t tmem_full_bar[2];
   __shared__ uint64_t tmem_empty_bar[2];
   __shared__ uint32_t tmem_base_slot;
+  __shared__ uint32_t s_stop[4];  // where the three producers and the issuer stopped
   __shared__ int abort_flag;
   __shared__ volatile int s_first_bad;  // first of this CTA's tiles whose accumulator never came
   __shared__ int s_off[kMaxGroups + 1];
@@ -164,6 +165,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) wgrad_gemm_kernel(const __gri
         }
       }
     }
+    if (lane == 0) s_stop[wgrad_part] = ring_stop(stage, phase);
   } else if (warp == 1) {
     // ======================= MMA issuer =======================
     // The warp stays converged around the elected lane's instructions (see "Issuing warps"); the next stage's barrier is
@@ -241,6 +243,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) wgrad_gemm_kernel(const __gri
       }
       __syncwarp();
     }
+    if (lane == 0) s_stop[3] = ring_stop(stage, phase);
   } else if (warp == 14) {
     // ======================= accumulator watcher =======================
     // One warp polls the accumulator-ready barriers on behalf of the eight epilogue warps and releases them
@@ -332,7 +335,15 @@ __global__ void __launch_bounds__(kGemmThreads, 1) wgrad_gemm_kernel(const __gri
   // ---- teardown ---------------------------------------------------------------
   tcgen05_fence_before();
   __syncthreads();
-  if (abort_flag && threadIdx.x == 0) set_status(p.status, kPipelineTimeout, 2, blockIdx.x);
+  if (abort_flag) {
+    if (threadIdx.x == 0) {
+      set_status(p.status, kPipelineTimeout, 2, blockIdx.x);
+      const uint64_t deadline = globaltimer_ns() + kSettleNs;
+      settle_ring(empty_bar, kStages, s_stop[3], deadline);
+      for (int i = 0; i < 3; ++i) settle_ring(full_bar, kStages, s_stop[i], deadline);
+    }
+    __syncthreads();
+  }
   if (warp == 1) {
     tcgen05_fence_after();
     tmem_dealloc(tmem_base, kTmemCols);

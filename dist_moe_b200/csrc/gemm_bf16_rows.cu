@@ -104,6 +104,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kRwThreads, 1) rows_
   __shared__ uint32_t tmem_base_slot;
   __shared__ int abort_flag;
   __shared__ volatile int s_first_bad;  // first of this CTA's tiles whose accumulator never came
+  __shared__ uint32_t s_stop[3];  // where the weight producer, the row producer and the issuer stopped
   __shared__ int s_box;
   __shared__ int s_off[kRwMaxGroups + 1];
   __shared__ int s_tile_start[kRwMaxGroups + 1];
@@ -265,6 +266,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kRwThreads, 1) rows_
       }
       if (!ok) break;
     }
+    if (lane == 0) s_stop[rows_side ? 1 : 0] = ring_stop(stage, phase);
     __syncwarp();
   } else if (warp == 1) {
     // ======================= MMA issuer =======================
@@ -326,6 +328,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kRwThreads, 1) rows_
         if (elected) tcgen05_commit_pair(tfull0 + buf * 8);
         __syncwarp();
       }
+      if (lane == 0) s_stop[2] = ring_stop(static_cast<int>((full - full0) >> 3), phase);
     }
     __syncwarp();
   } else if (warp == 14) {
@@ -532,7 +535,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kRwThreads, 1) rows_
   // ---- teardown ---------------------------------------------------------------
   tcgen05_fence_before();
   __syncthreads();
-  cluster_sync();  // neither CTA leaves while the other may still signal its barriers
+  if (abort_flag && rank == 0 && threadIdx.x == 0) {  // the leader's barriers count both CTAs' loads and MMAs
+    const uint64_t deadline = globaltimer_ns() + kSettleNs;
+    settle_ring(empty_bar, stages, s_stop[2], deadline);
+    settle_ring(full_bar, stages, s_stop[0], deadline);
+    settle_ring(full_bar, stages, s_stop[1], deadline);
+  }
+  __syncwarp();
+  cluster_sync();  // neither CTA leaves while the other may still signal its barriers, or loads into either are in flight
   if (abort_flag && threadIdx.x == 0) set_status(p.status, kPipelineTimeout, kMode, blockIdx.x);
   if (warp == 1) {
     tcgen05_fence_after();

@@ -132,6 +132,7 @@ __global__ void __launch_bounds__(kWdThreads, 1) blockscaled_wide_kernel(const _
   __shared__ uint64_t tmem_full_bar;
   __shared__ uint64_t tmem_empty_bar;
   __shared__ uint32_t tmem_base_slot;
+  __shared__ uint32_t s_stop[4];  // where the producer, the issuer and the two scale copiers stopped
   __shared__ int abort_flag;
   __shared__ volatile int s_first_bad;  // first of this CTA's tiles whose accumulator never came
   __shared__ int s_off[kBsMaxGroups + 1];
@@ -256,6 +257,7 @@ __global__ void __launch_bounds__(kWdThreads, 1) blockscaled_wide_kernel(const _
           }
         }
       }
+      if (lane == 0) s_stop[0] = ring_stop(stage, phase);
     }
     __syncwarp();
   } else if (warp == 1) {
@@ -325,6 +327,7 @@ __global__ void __launch_bounds__(kWdThreads, 1) blockscaled_wide_kernel(const _
         }
         __syncwarp();
       }
+      if (lane == 0) s_stop[1] = ring_stop(stage, phase);
     }
     __syncwarp();
   } else if (warp == 11 || warp == 10) {
@@ -379,6 +382,7 @@ __global__ void __launch_bounds__(kWdThreads, 1) blockscaled_wide_kernel(const _
         asm volatile("bar.arrive %0, %1;" ::"r"(handover_barrier(it)), "r"(8 * 32 + 32) : "memory");
       }
     }
+    if (lane == 0) s_stop[watcher ? 3 : 2] = ring_stop(stage, phase);
     __syncwarp();
   } else {
     // ======================= epilogue =======================
@@ -630,7 +634,17 @@ __global__ void __launch_bounds__(kWdThreads, 1) blockscaled_wide_kernel(const _
 
   tcgen05_fence_before();
   __syncthreads();
-  if (abort_flag && threadIdx.x == 0) set_status(p.status, kPipelineTimeout, 4, blockIdx.x);
+  if (abort_flag) {
+    if (threadIdx.x == 0) {
+      set_status(p.status, kPipelineTimeout, 4, blockIdx.x);
+      const uint64_t deadline = globaltimer_ns() + kSettleNs;
+      settle_ring(empty_bar, stages, s_stop[1], deadline);
+      settle_ring(full_bar, stages, s_stop[0], deadline);
+      settle_ring(sf_bar, stages, s_stop[2], deadline);
+      if (p.fp4) settle_ring(sf_bar, stages, s_stop[3], deadline);
+    }
+    __syncthreads();
+  }
   if (warp == 1) {
     tcgen05_fence_after();
     tmem_dealloc(tmem_base, kBsTmemCols);

@@ -94,6 +94,7 @@ __global__ void __launch_bounds__(kSwThreads, kSwCtasPerSm) blockscaled_swapped_
   __shared__ uint64_t tmem_full_bar[2];
   __shared__ uint64_t tmem_empty_bar[2];
   __shared__ uint32_t tmem_base_slot;
+  __shared__ uint32_t s_stop[3];  // where the producer, the issuer and the scale copier stopped
   __shared__ int abort_flag;
   __shared__ volatile int s_first_bad;  // first of this CTA's tiles whose accumulator never came
   __shared__ int s_off[kSwMaxGroups + 1];
@@ -193,6 +194,7 @@ __global__ void __launch_bounds__(kSwThreads, kSwCtasPerSm) blockscaled_swapped_
         }
       }
     }
+    if (lane == 0) s_stop[0] = ring_stop(stage, phase);
     __syncwarp();
   } else if (warp == 1) {
     // ======================= MMA issuer =======================
@@ -261,6 +263,7 @@ __global__ void __launch_bounds__(kSwThreads, kSwCtasPerSm) blockscaled_swapped_
       }
       __syncwarp();
     }
+    if (lane == 0) s_stop[1] = ring_stop(stage, phase);
     __syncwarp();
   } else if (warp == 7) {
     // ======================= scale copier =======================
@@ -293,6 +296,7 @@ __global__ void __launch_bounds__(kSwThreads, kSwCtasPerSm) blockscaled_swapped_
         }
       }
     }
+    if (lane == 0) s_stop[2] = ring_stop(stage, phase);
     __syncwarp();
   } else if (warp == 6) {
     // ======================= accumulator watcher =======================
@@ -394,7 +398,16 @@ __global__ void __launch_bounds__(kSwThreads, kSwCtasPerSm) blockscaled_swapped_
 
   tcgen05_fence_before();
   __syncthreads();
-  if (abort_flag && threadIdx.x == 0) set_status(p.status, kPipelineTimeout, 4, blockIdx.x);
+  if (abort_flag) {
+    if (threadIdx.x == 0) {
+      set_status(p.status, kPipelineTimeout, 4, blockIdx.x);
+      const uint64_t deadline = globaltimer_ns() + kSettleNs;
+      settle_ring(empty_bar, kSwStages, s_stop[1], deadline);
+      settle_ring(full_bar, kSwStages, s_stop[0], deadline);
+      settle_ring(sf_bar, kSwStages, s_stop[2], deadline);
+    }
+    __syncthreads();
+  }
   if (warp == 1) {
     tcgen05_fence_after();
     tmem_dealloc(tmem_base, kSwTmemCols);

@@ -52,6 +52,16 @@ __device__ __forceinline__ bool warp_mbar_wait(uint64_t* bar, uint32_t parity, v
   return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag));
 }
 
+// After a wait ran out: a role's copies or MMAs that are still in flight have to end before the block gives its shared
+// memory and tensor memory back.  `bar` holds the barriers they complete, `stop` says where the role stopped.  Returns at
+// the deadline where a stage never completes (it was left half filled; what was issued for it has landed by then).
+__device__ __forceinline__ void settle_ring(uint64_t* bar, int stages, uint32_t stop, uint64_t deadline_ns) {
+  for (int s = 0; s < stages; ++s)
+    while (!mbar_try_wait(&bar[s], ring_last_parity(stop, s)))
+      if (globaltimer_ns() > deadline_ns) return;
+}
+constexpr uint64_t kSettleNs = 1000000;  // a millisecond; loads take microseconds
+
 // One look at a barrier that never suspends the thread: asked for the next stage before this stage's MMAs are issued, its
 // latency hides behind them.
 __device__ __forceinline__ uint32_t mbar_test(uint32_t bar_addr, uint32_t parity) {

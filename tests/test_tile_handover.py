@@ -6,6 +6,7 @@ the protocol around them is explored to the end, and every path has to end with 
 """
 
 import ctypes
+import random
 import subprocess
 from pathlib import Path
 
@@ -19,6 +20,7 @@ HARNESS = """
 extern "C" int barrier(int it) { return dm::handover_barrier(it) - 1; }
 extern "C" int none() { return dm::kNoBadTile; }
 extern "C" int report(int* first_bad, int it, int came) { return dm::handover_report(first_bad, it, came != 0); }
+extern "C" unsigned last_parity(int stage, unsigned phase, int s) { return dm::ring_last_parity(dm::ring_stop(stage, phase), s); }
 extern "C" int good(const int* first_bad, int it) { return dm::handover_good(first_bad, it); }
 """
 
@@ -134,3 +136,23 @@ def test_what_the_rule_is_for(lib):
     assert stuck_paths(Flag(lib)) > 0
     assert stuck_paths(Recorded(lib, keep_arriving=True)) > 0
     assert stuck_paths(Recorded(lib, barriers=2)) > 0
+
+
+def test_the_last_use_of_every_stage_is_what_is_waited_for(lib):
+    """An mbarrier reports the parity of the phase before its current one as complete.  With every use of a role complete, the
+    wait for its last use of each stage returns; with one use outstanding, the wait for that stage does not."""
+    complete = lambda phases, parity: (phases - 1) & 1 == parity  # noqa: E731  (a fresh barrier: parity 1)
+    rng = random.Random(5)
+    for _ in range(300):
+        stages, uses = rng.randint(1, 10), rng.randint(0, 45)
+        stage, phase, done = 0, 0, [0] * stages
+        for _ in range(uses):
+            done[stage] += 1
+            stage += 1
+            if stage == stages:
+                stage, phase = 0, phase ^ 1
+        parity = [lib.last_parity(stage, phase, s) for s in range(stages)]
+        assert all(complete(done[s], parity[s]) for s in range(stages))
+        for back in range(min(uses, stages)):  # the latest uses may still be in flight
+            s = (stage - 1 - back) % stages
+            assert not complete(done[s] - 1, parity[s])
