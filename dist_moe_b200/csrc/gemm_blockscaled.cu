@@ -630,6 +630,7 @@ __global__ void __launch_bounds__(kWdThreads, 1) blockscaled_wide_kernel(const _
         }
       }
     }
+    if (lane == 0) bulk_wait_all();  // weight gradient: staged boxes are out of shared memory and written
   }
 
   tcgen05_fence_before();
