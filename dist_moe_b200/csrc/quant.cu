@@ -442,6 +442,9 @@ __global__ void __launch_bounds__(256, 3) mxfp8_colrow_kernel(const uint4* __res
   const int64_t tiles = (rows + kTileRows - 1) / kTileRows * col_tiles;
   uint4* slot = slots + threadIdx.x;
   uint4* up = slot + kTileSlot;
+  // what a copy of zero bytes names as its source: nothing is read there, but the address has to be on 16 bytes as for any
+  // other copy of this width, which a table of 8-byte pointers need not be
+  const void* nowhere = reinterpret_cast<const void*>(reinterpret_cast<uintptr_t>(row_ptrs) & ~uintptr_t(15));
   auto fetch = [&](int64_t tile) {  // the lane's 8 rows of a tile on their way into its slots
     const int64_t r0 = tile / col_tiles * kTileRows + me.row();
     const int c = static_cast<int>(tile - tile / col_tiles * col_tiles) * kTileCols + me.col();
@@ -458,7 +461,7 @@ __global__ void __launch_bounds__(256, 3) mxfp8_colrow_kernel(const uint4* __res
         cp_async16(slot + 256 * r, r < live ? x + (r0 + r) * vec_per_row + v : x, r < live ? 16 : 0);
       } else {
         const uint4* src = r < live ? reinterpret_cast<const uint4*>(row_ptrs[r0 + r]) : nullptr;
-        cp_async16(slot + 256 * r, src != nullptr ? static_cast<const void*>(src + v) : row_ptrs, src != nullptr ? 16 : 0);
+        cp_async16(slot + 256 * r, src != nullptr ? static_cast<const void*>(src + v) : nowhere, src != nullptr ? 16 : 0);
       }
     }
   };

@@ -441,3 +441,25 @@ def test_mxfp8_row_live_rows_only(rows, cols):
     keep = live != 0
     for g, w in zip(got, want):
         assert torch.equal(g[keep], w[keep]) and bool((g[~keep] == 0xAB).all())
+
+
+@pytest.mark.parametrize("rows,cols", [(1, 32), (130, 160)])
+def test_mxfp8_gather_from_a_table_that_is_only_8_byte_aligned(rows, cols):
+    """A pointer table may start at any 8-byte address; null pointers, rows past the end and columns past the matrix read
+    nothing.  Same bytes as from a table on 16 bytes."""
+    nat = _nat()
+    x = _data(rows, cols, 3 * rows + cols, specials=False).to(DEV)
+    ptrs = torch.where(torch.arange(rows) % 4 == 3, 0, x.data_ptr() + torch.arange(rows) * cols * 2)
+    ra, ca = (cols // 32 + 3) // 4, ((rows + 31) // 32 + 3) // 4
+    got = []
+    for shift in (0, 1):
+        table = torch.zeros(rows + 2, dtype=torch.int64, device=DEV)
+        table[shift:shift + rows] = ptrs.to(DEV)
+        assert table[shift:].data_ptr() % 16 == 8 * shift
+        out = [torch.zeros(n, dtype=torch.uint8, device=DEV)
+               for n in (rows * cols, (rows + 127) // 128 * 128 * ra * 4, rows * cols, (cols + 127) // 128 * 128 * ca * 4)]
+        nat.check(nat.lib.dm_quant_mxfp8_rowcol_gather(table[shift:].data_ptr(), None, rows, cols, *[t.data_ptr() for t in out],
+                                                       nat.stream_ptr()), "gather")
+        torch.cuda.synchronize()
+        got.append(out)
+    assert all(torch.equal(a, b) for a, b in zip(*got)) and bool(got[0][0].any())
