@@ -255,7 +255,6 @@ __host__ __device__ constexpr uint32_t umma_idesc_bf16(int m, int n, int a_mn_ma
 // ----------------------------------------------------------------------------
 // Small numeric helpers
 // ----------------------------------------------------------------------------
-__device__ __forceinline__ float bf16_bits_to_f32(uint32_t bits16) { return __uint_as_float(bits16 << 16); }
 
 __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
   __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
@@ -347,6 +346,5 @@ static inline int persistent_grid(int num_sms) {
 static inline int grid_cap(int per_sm) { return sm_count() * per_sm; }
 
 __host__ __device__ constexpr int64_t ceil_div64(int64_t a, int64_t b) { return (a + b - 1) / b; }
-__host__ __device__ constexpr int64_t align_up64(int64_t a, int64_t b) { return (a + b - 1) / b * b; }
 
 }  // namespace dm

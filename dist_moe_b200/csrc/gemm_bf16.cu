@@ -7,8 +7,8 @@
 //   warps 0, 10, 11  TMA producers: fill a 4-stage shared-memory ring (dY 64 rows x 128, X 64 rows x 256, boxes of 64 x
 //               64, 128-byte swizzle) with cp.async.bulk.tensor loads, no multicast.
 //   warp 1      MMA issuer: owns the TMEM allocation (512 columns = two 128x256 fp32
-//               accumulators), issues tcgen05.mma (M128 N256 K16) from one lane and
-//               releases stages / publishes accumulators with tcgen05.commit.
+//               accumulators), stays converged around an elected lane's tcgen05.mma (M128 N256 K16)
+//               and releases stages / publishes accumulators with tcgen05.commit.
 //   warps 2..9  epilogue (two per TMEM lane quadrant): tcgen05.ld their 32 TMEM lanes, convert and store or add into dW
 //               while the next tile's main loop already runs.
 //   warp 14     accumulator watcher.

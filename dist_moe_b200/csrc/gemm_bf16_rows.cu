@@ -21,7 +21,7 @@
 //   warp 0       TMA producer of the weights: stages of 64 K elements, 16 KiB of weights and as many rows as the launch's
 //                largest tile needs (16 to 128 per CTA; small tiles leave room for up to ten stages, which keeps enough of
 //                the weight stream in flight when experts have few rows), no multicast.
-//   warp 1       MMA issuer (of the leading CTA): 512 TMEM columns = two accumulators of up to 256 rows; one lane issues
+//   warp 1       MMA issuer (of the leading CTA): 512 TMEM columns = two accumulators of up to 256 rows; the elected lane issues
 //                tcgen05.mma (M256, N = rows of the tile, K16) and publishes with tcgen05.commit.
 //   warps 2..9   epilogue (two per TMEM lane quadrant, each group of four owning half of the tile's rows): read 32 rows
 //                x 32 columns, exchange pairs of columns between neighbouring lanes, and collect 32 rows x 128 columns
@@ -44,7 +44,6 @@ constexpr int kRwBM = 128;    // output columns per CTA of a pair (weights, M si
 constexpr int kRwBK = 64;     // K of a stage (128 bytes per row)
 constexpr int kRwMaxStages = 10;
 constexpr int kRwThreads = 512;
-constexpr int kRwGatherWarps = 4;
 constexpr int kRwGatherUnitRows = 8;                                        // rows one gather warp pulls before it reports
 constexpr int kRwGatherUnitsPerBlock = kRwGatherBlock / kRwGatherUnitRows;  // reports that make a 128-row block ready
 constexpr int kRwMaxGroups = 256;

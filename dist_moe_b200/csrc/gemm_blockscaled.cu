@@ -97,10 +97,10 @@ __device__ __forceinline__ BsTile bs_decode(int tile, int& e, const int* tile_st
 // 940 -> 869 us, input gradients 490 -> 452 and 923 -> 877 us (operand loads from L2, 12.8 TB/s), weight gradients
 // 804 -> 767 and 1655 -> 1563 us (dW read, added to and written: 4.1 TB/s of HBM).
 // 128 x 256 output tiles.  Per 128 bytes of K the tile moves 48 KiB of operands and needs, for NVFP4, twelve
-// scale-atom copies (about 47 cycles each, they serialise with the MMAs) per four 132-cycle MMAs; a 128 x 128
-// tile would spend more tensor-pipe time on its eight copies than on its four 69-cycle MMAs.  TMEM holds one
-// 256-column accumulator plus two buffers of scale columns, so the epilogue (eight warps, a few thousand
-// cycles) does not overlap the next tile's MMAs; tiles here are tens of thousands of cycles long.  Experts
+// scale-atom copies (about 40 cycles of the tensor pipe each, they serialise with the MMAs) per four 128-cycle MMAs; a
+// 128 x 128 tile would spend more tensor-pipe time on its eight copies than on its four 64-cycle MMAs.  TMEM holds one
+// 256-column accumulator plus two buffers of scale columns: the epilogue warps read it into registers and hand it back
+// before they convert and store, so only that read stands between a tile's last MMA and the next tile's first.  Experts
 // with few rows take the swapped-operand kernel instead (gemm_blockscaled_swapped.cu).
 // ---------------------------------------------------------------------------------------------------------
 constexpr int kWdBN = 256;

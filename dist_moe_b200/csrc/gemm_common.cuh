@@ -10,15 +10,11 @@
 
 namespace dm {
 
-constexpr uint32_t kStagingBytes = 32 * 128;   // per epilogue warp: 32 rows x 128 bytes
-constexpr uint32_t kStaging64Bytes = 32 * 64;  // per epilogue warp: 32 rows x 64 bytes
+constexpr uint32_t kStaging64Bytes = 32 * 64;  // per epilogue warp: 32 rows x 64 bytes, or 16 rows x 128 bytes
 
-// Staging tile of one epilogue warp: row r is 128 bytes, its 16-byte chunk j sits at j ^ (r & 7).
+// Staging tile of one epilogue warp: row r is 128 bytes, its 16-byte chunk j sits at j ^ (r & 7) (the 128-byte swizzle).
 __device__ __forceinline__ void stage_put(uint8_t* stg, int row, int chunk, uint4 v) {
   reinterpret_cast<uint4*>(stg + row * 128)[chunk ^ (row & 7)] = v;
-}
-__device__ __forceinline__ uint4 stage_get(const uint8_t* stg, int row, int chunk) {
-  return reinterpret_cast<const uint4*>(stg + row * 128)[chunk ^ (row & 7)];
 }
 // 64-byte variant: row r is 64 bytes, its 16-byte chunk j sits at j ^ ((r >> 1) & 3).
 __device__ __forceinline__ void stage64_put(uint8_t* stg, int row, int chunk, uint4 v) {
@@ -34,10 +30,6 @@ __device__ __forceinline__ uint4 pack8_bf16(const uint32_t* r) {
                     pack_bf16x2(__uint_as_float(r[6]), __uint_as_float(r[7])));
 }
 
-// Forms for the issue loops: barriers given by their shared-memory address, shared-memory matrix descriptors by their
-// lower word (address >> 4 | LBO >> 4 << 16) and a constant upper word (SBO >> 4, version 1 in bit 14, 128-byte swizzle 2
-// in bits 29 to 31).  K-major operand: rows of 128 bytes, 8-row groups SBO = 1024 apart.  MN-major operand: lines of 128
-// bytes of M or N, one line per k, 8-k groups SBO = 1024 apart, the next 128 bytes of M or N LBO apart.
 // ---------------------------------------------------------------------------
 // Issuing warps.  tcgen05 and TMA instructions take their operands from uniform registers.  Code that only one lane runs
 // (`if (lane == 0)`) keeps everything in per-lane registers and moves each operand over for each instruction: 85 to 93
@@ -75,6 +67,11 @@ __device__ __forceinline__ uint32_t mbar_test(uint32_t bar_addr, uint32_t parity
       : "=r"(ok) : "r"(bar_addr), "r"(parity) : "memory");
   return ok;
 }
+
+// MMAs and commits for the issue loops: barriers given by their shared-memory address, shared-memory matrix descriptors by
+// their lower word (address >> 4 | LBO >> 4 << 16) and a constant upper word (SBO >> 4, version 1 in bit 14, 128-byte
+// swizzle 2 in bits 29 to 31).  K-major operand: rows of 128 bytes, 8-row groups SBO = 1024 apart.  MN-major operand: lines
+// of 128 bytes of M or N, one line per k, 8-k groups SBO = 1024 apart, the next 128 bytes of M or N LBO apart.
 __device__ __forceinline__ void umma_bf16_lo(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t desc_hi,
                                              uint32_t idesc, uint32_t accumulate) {
   asm volatile(
@@ -274,15 +271,14 @@ static inline int encode_arena(CUtensorMap* tm, const dm_operand& op, int64_t pi
   return r == CUDA_SUCCESS ? kRcOk : 1000 + static_cast<int>(r);
 }
 
-// Weight-gradient destination [groups][rows][cols] (bf16 or fp32), boxes of 32 rows x 64 bytes in the
-// 64-byte swizzle: the layout of an epilogue warp's staging tile.
+// Weight-gradient destination [groups][rows][cols] (bf16 or fp32), boxes of 16 rows x 128 bytes in the 128-byte swizzle:
+// the layout of an epilogue warp's staging tile, and whole 128-byte lines of dW per store or reduce-add.
 static inline int encode_out_3d(CUtensorMap* tm, void* base, int64_t groups, int64_t rows, int64_t cols, bool fp32) {
   EncodeTiledFn enc = get_encode();
   if (!enc) return kRcNoDriver;
   const cuuint64_t esz = fp32 ? 4 : 2;
   cuuint64_t dims[3] = {static_cast<cuuint64_t>(cols), static_cast<cuuint64_t>(rows), static_cast<cuuint64_t>(groups)};
   cuuint64_t strides[2] = {static_cast<cuuint64_t>(cols) * esz, static_cast<cuuint64_t>(cols) * rows * esz};
-  // boxes of 16 rows x 128 bytes: a reduce-add or store then moves whole 128-byte lines of dW
   cuuint32_t box[3] = {static_cast<cuuint32_t>(128 / esz), 16, 1};
   cuuint32_t estr[3] = {1, 1, 1};
   CUresult r = enc(tm, fp32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, base, dims, strides,
