@@ -48,13 +48,18 @@ def peaks():
 
 
 def kernel_source_digest() -> str:
-    """Digest of the grouped-GEMM sources; a recorded ncu traffic figure is only reported for the sources it was
-    captured on."""
+    """Digest of the BF16 grouped-GEMM sources and of the headers beside them that they include; a recorded ncu traffic
+    figure is only reported for the sources it was captured on."""
     import hashlib
+    import re
 
+    csrc = ROOT / "dist_moe_b200" / "csrc"
+    names = ["gemm_bf16.cu", "gemm_bf16_rows.cu"]
     h = hashlib.sha256()
-    for name in ("gemm_bf16.cu", "gemm_bf16_rows.cu", "row_tiles.cuh", "gemm_common.cuh", "common.cuh"):
-        h.update((ROOT / "dist_moe_b200" / "csrc" / name).read_bytes())
+    for name in names:  # grows while it is walked
+        text = (csrc / name).read_text()
+        h.update(text.encode())
+        names += [n for n in re.findall(r'#include "([\w.]+)"', text) if n not in names]
     return h.hexdigest()[:16]
 
 

@@ -43,3 +43,22 @@ def test_training_workloads_are_legal_configs():
     for cfg in (bf16, mxfp8):
         for ep in (1, 8):
             assert dm.plan_memory(cfg, ep).total_device_buffer_bytes > 0
+
+
+def test_a_recorded_traffic_figure_goes_stale_with_every_source_of_the_bf16_gemms(tmp_path, monkeypatch):
+    """The digest follows the includes of the two kernel files, headers of headers among them, and nothing else."""
+    import shutil
+
+    bench = _bench()
+    csrc = tmp_path / "dist_moe_b200" / "csrc"
+    shutil.copytree(bench.ROOT / "dist_moe_b200" / "csrc", csrc)
+    monkeypatch.setattr(bench, "ROOT", tmp_path)
+    now = bench.kernel_source_digest()
+    for name in ("gemm_bf16.cu", "gemm_bf16_rows.cu", "gemm_common.cuh", "common.cuh", "row_tiles.cuh", "tile_handover.cuh",
+                 "quant.cu"):
+        path = csrc / name
+        text = path.read_text()
+        path.write_text(text + "// changed\n")
+        assert (bench.kernel_source_digest() != now) == (name != "quant.cu"), name
+        path.write_text(text)
+    assert bench.kernel_source_digest() == now
