@@ -251,8 +251,11 @@ def _workspace(state):
 
 # Inference calls whose experts receive at most this many rows on average take the swapped-operand GEMMs (rows on
 # the MMA's N side in steps of 32); above it a 128-row tile is mostly real rows and the 128 x 256 kernel wins.
-# Measured crossovers (whole layer, one B200): NVFP4 wins at 32 rows per expert and loses at 64, MXFP8 wins at 16 and
-# loses at 32 (its MMAs move twice the bytes per row).  ``None`` keeps the per-format value.
+# Whole layer on one B200, swapped / 128 x 256, us.  NVFP4: 32 experts x 7168 x 2048 at 48 rows per expert 226 / 243, at 64
+# 237 / 247, at 96 274 / 255; 64 experts x 2048 x 2048 at 48 222 / 232, at 56 235 / 233, at 64 265 / 236.  MXFP8: 128
+# experts x 2816 x 2816 at 24 621 / 667, at 48 685 / 695, at 56 718 / 704; 32 experts x 4096 x 1536 at 24 186 / 196, at 48
+# 194 / 198, at 64 204 / 198.  So NVFP4 stops where its smaller layer stops winning; MXFP8 stops early, between 24 and 48 rows
+# the swapped form would be 1 to 6 % faster.  ``None`` keeps the per-format value.
 SWAPPED_MAX_ROWS_PER_EXPERT = None
 _SWAPPED_MAX_ROWS = {BlockScaledFormat.NVFP4: 48, BlockScaledFormat.MXFP8_E4M3: 24}
 
