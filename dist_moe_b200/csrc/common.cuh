@@ -197,20 +197,6 @@ __device__ __forceinline__ void tcgen05_fence_before() {
 __device__ __forceinline__ void tcgen05_fence_after() {
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 }
-// Copy one 128-row x 4-scale atom (32 rows x 16 bytes in shared memory) into 4 TMEM columns, replicated
-// over the four 32-lane sub-partitions.
-__device__ __forceinline__ void tmem_cp_sf_atom(uint32_t taddr, uint64_t smem_desc) {
-  asm volatile("tcgen05.cp.cta_group::1.32x128b.warpx4 [%0], %1;" ::"r"(taddr), "l"(smem_desc) : "memory");
-}
-// Shared-memory descriptor of a scale atom: no swizzle, rows 16 bytes apart, 8-row groups 128 bytes apart.
-__device__ __forceinline__ uint64_t sf_smem_desc(uint32_t smem_addr) {
-  uint64_t d = 0;
-  d |= static_cast<uint64_t>((smem_addr & 0x3ffff) >> 4);
-  d |= static_cast<uint64_t>(16 >> 4) << 16;
-  d |= static_cast<uint64_t>(128 >> 4) << 32;
-  d |= static_cast<uint64_t>(1) << 46;
-  return d;
-}
 // Instruction descriptor of the block-scaled kinds (M128, K-major operands).
 //   fp4 == 0: kind::mxf8f6f4, E4M3 data, UE8M0 scales, sf ids select the scale byte of the K=32 step.
 //   fp4 != 0: kind::mxf4nvf4, E2M1 data, UE4M3 scales (4 per K=64 step).

@@ -92,19 +92,17 @@ __device__ __forceinline__ BsTile bs_decode(int tile, int& e, const int* tile_st
 }
 
 // ---------------------------------------------------------------------------------------------------------
-// Measured when the issuing warps became converged (before: one lane each): NVFP4 65 536 rows W13 1010 -> 891 us, W2
-// 620 -> 588 us (four MMAs and twelve scale copies per stage share the tensor pipe: about 950 cycles); MXFP8 73 728 rows W13
-// 940 -> 869 us, input gradients 490 -> 452 and 923 -> 877 us (operand loads from L2, 12.8 TB/s), weight gradients
-// 804 -> 767 and 1655 -> 1563 us (dW read, added to and written: 4.1 TB/s of HBM).
+// Bound by operand loads from L2 (54 KiB a stage for NVFP4, 50 for MXFP8: 13 to 14 TB/s) and, for the weight gradients, by dW,
+// which is read, added to and written (4.1 TB/s of HBM).  Scale copies issued by the MMA warp instead of two warps of
+// their own: NVFP4 layer of 65 536 rows 2156 -> 2091 us, MXFP8 training layer of 73 728 rows 7390 -> 7198 us.
 // 128 x 256 output tiles.  Per 128 bytes of K the tile moves 48 KiB of operands and needs, for NVFP4, twelve
-// scale-atom copies (about 40 cycles of the tensor pipe each, they serialise with the MMAs) per four 128-cycle MMAs; a
-// 128 x 128 tile would spend more tensor-pipe time on its eight copies than on its four 64-cycle MMAs.  TMEM holds one
+// scale-atom copies (16 cycles each, hidden behind the MMAs) per four 128-cycle MMAs.  TMEM holds one
 // 256-column accumulator plus two buffers of scale columns: the epilogue warps read it into registers and hand it back
 // before they convert and store, so only that read stands between a tile's last MMA and the next tile's first.  Experts
 // with few rows take the swapped-operand kernel instead (gemm_blockscaled_swapped.cu).
 // ---------------------------------------------------------------------------------------------------------
 constexpr int kWdBN = 256;
-constexpr int kWdThreads = 384;  // TMA warp, MMA warp, eight epilogue warps, accumulator watcher, scale copier
+constexpr int kWdThreads = 352;  // TMA warp, MMA warp, eight epilogue warps, accumulator watcher
 constexpr uint32_t kWdBBytes = kWdBN * 128;                                   // 32 KiB
 constexpr uint32_t kWdStageFp4 = kBsABytes + kWdBBytes + 2048 + 4096;         // 54 KiB: 4 + 8 scale atoms
 constexpr uint32_t kWdStageFp8 = kBsABytes + kWdBBytes + 2048;                // 50 KiB: 1 + 2 scale atoms, padded
@@ -128,11 +126,10 @@ __global__ void __launch_bounds__(kWdThreads, 1) blockscaled_wide_kernel(const _
 
   __shared__ uint64_t full_bar[kWdMaxStages];
   __shared__ uint64_t empty_bar[kWdMaxStages];
-  __shared__ uint64_t sf_bar[kWdMaxStages];  // the stage's scale atoms are in TMEM
   __shared__ uint64_t tmem_full_bar;
   __shared__ uint64_t tmem_empty_bar;
   __shared__ uint32_t tmem_base_slot;
-  __shared__ uint32_t s_stop[4];  // where the producer, the issuer and the two scale copiers stopped
+  __shared__ uint32_t s_stop[2];  // where the producer and the issuer stopped
   __shared__ int abort_flag;
   __shared__ volatile int s_first_bad;  // first of this CTA's tiles whose accumulator never came
   __shared__ int s_off[kBsMaxGroups + 1];
@@ -156,7 +153,6 @@ __global__ void __launch_bounds__(kWdThreads, 1) blockscaled_wide_kernel(const _
     for (int s = 0; s < kWdMaxStages; ++s) {
       mbar_init(&full_bar[s], 1);
       mbar_init(&empty_bar[s], 1);
-      mbar_init(&sf_bar[s], p.fp4 ? 2 : 1);  // NVFP4: two copier threads share the stage's atoms
     }
     mbar_init(&tmem_full_bar, 1);
     mbar_init(&tmem_empty_bar, 8);
@@ -262,6 +258,12 @@ __global__ void __launch_bounds__(kWdThreads, 1) blockscaled_wide_kernel(const _
     __syncwarp();
   } else if (warp == 1) {
     // ======================= MMA issuer =======================
+    // The scale atoms of a stage are copied to the stage slot's TMEM columns by the warp that issues the MMAs, right before
+    // them: copies and MMAs of one thread execute in order, so no barrier stands between them, and the copies run while
+    // the MMAs issued before them occupy the pipe (twelve copies and four MMAs of N = 256: 512 cycles, as long as the
+    // MMAs alone; from other warps a copy took 54 cycles).  Columns: A atom a (K step a) at +4a; B atoms of the tile's lower
+    // and upper 128 columns side by side, 8 columns per K step.  The slot's previous MMAs are complete by then: the
+    // producer refilled the stage only after their commit released it.
     {
       const bool elected = elect_one();
       constexpr uint32_t kDescHi = (1024u >> 4) | (1u << 14) | (2u << 29);  // SBO 1024, version 1, 128-byte swizzle
@@ -274,9 +276,9 @@ __global__ void __launch_bounds__(kWdThreads, 1) blockscaled_wide_kernel(const _
 #pragma unroll
       for (int j = 0; j < 4; ++j) idesc8[j] = umma_idesc_blockscaled(kWdBN, 0, j, j, a_mn, b_mn);
       const uint32_t full0 = uniform(smem_u32(&full_bar[0])), empty0 = uniform(smem_u32(&empty_bar[0]));
-      const uint32_t sf0 = uniform(smem_u32(&sf_bar[0])), tfull = uniform(smem_u32(&tmem_full_bar));
+      const uint32_t tfull = uniform(smem_u32(&tmem_full_bar));
       int stage = 0;
-      uint32_t phase = 0, ready = 0;  // ready: the current stage and its scales are known to be there
+      uint32_t phase = 0, ready = 0;  // ready: the current stage is known to be there
       int e = 0, it = 0;
       bool ok = true;
       for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x, ++it) {
@@ -288,12 +290,13 @@ __global__ void __launch_bounds__(kWdThreads, 1) blockscaled_wide_kernel(const _
 #pragma unroll 1
         for (int kb = 0; kb < k_iters; ++kb) {
           if (!__all_sync(0xffffffffu, ready)) {
-            ok = warp_mbar_wait(&full_bar[stage], phase, &abort_flag) && warp_mbar_wait(&sf_bar[stage], phase, &abort_flag);
+            ok = warp_mbar_wait(&full_bar[stage], phase, &abort_flag);
             if (!ok) break;
           }
           tcgen05_fence_after();
           const uint32_t a_addr = ring + stage * stage_bytes;
           const uint32_t a_lo = ((a_addr & 0x3ffffu) >> 4) | a_lbo, b_lo = (((a_addr + kBsABytes) & 0x3ffffu) >> 4) | b_lbo;
+          const uint32_t sf_lo = sf_desc_lo(a_addr + kBsABytes + kWdBBytes);
           const uint32_t sfa_t = tmem_base + kWdSfTmemBase + stage * 64u;
           const uint32_t sfb_t = sfa_t + 16u;
           const uint32_t empty = empty0 + stage * 8;
@@ -301,14 +304,23 @@ __global__ void __launch_bounds__(kWdThreads, 1) blockscaled_wide_kernel(const _
             stage = 0;
             phase ^= 1u;
           }
-          ready = mbar_test(full0 + stage * 8, phase) & mbar_test(sf0 + stage * 8, phase);
+          ready = mbar_test(full0 + stage * 8, phase);
           if (elected) {
             if (p.fp4) {
+#pragma unroll
+              for (int j = 0; j < 4; ++j) {
+                tmem_cp_sf_lo(sfa_t + 4 * j, sf_lo + j * kSfAtomWords);
+                tmem_cp_sf_lo(sfb_t + 8 * j, sf_lo + (4 + j) * kSfAtomWords);
+                tmem_cp_sf_lo(sfb_t + 8 * j + 4, sf_lo + (8 + j) * kSfAtomWords);
+              }
 #pragma unroll
               for (int j = 0; j < 4; ++j)
                 umma_nvf4_lo(tmem_base, a_lo + j * a_step, b_lo + j * b_step, kDescHi, idesc4, sfa_t + 4 * j, sfb_t + 8 * j,
                              (kb > 0 || j > 0) ? 1u : 0u);
             } else {
+              tmem_cp_sf_lo(sfa_t, sf_lo);
+              tmem_cp_sf_lo(sfb_t, sf_lo + kSfAtomWords);
+              tmem_cp_sf_lo(sfb_t + 4, sf_lo + 2 * kSfAtomWords);
 #pragma unroll
               for (int j = 0; j < 4; ++j)
                 umma_mxf8_lo(tmem_base, a_lo + j * a_step, b_lo + j * b_step, kDescHi, idesc8[j], sfa_t, sfb_t,
@@ -330,60 +342,17 @@ __global__ void __launch_bounds__(kWdThreads, 1) blockscaled_wide_kernel(const _
       if (lane == 0) s_stop[1] = ring_stop(stage, phase);
     }
     __syncwarp();
-  } else if (warp == 11 || warp == 10) {
-    // ======================= scale copiers (the second one is also the accumulator watcher) =======================
-    // These two warps move every stage's atoms to the stage slot's TMEM columns and commit to a per-stage barrier the MMA
-    // warp waits on: an NVFP4 stage needs twelve copies next to its four MMAs, about 40 cycles of the tensor pipe each.
-    // Columns: A atom a (K step a) at +4a; B atoms of the tile's lower and
-    // upper 128 columns side by side, 8 columns per K step.  The slot's previous MMAs are complete by then: the
-    // producer refilled the stage only after their commit released it.  NVFP4 has four atoms per stage and
-    // operand and each thread takes two; MXFP8 has one, taken by warp 11.
-    //
-    // Warp 10 then polls the accumulator-ready barrier for the epilogue warps and releases them through a hardware
-    // named barrier; after a timeout it releases them once more and stops.
-    const bool watcher = warp == 10;
-    const bool elected = elect_one();
-    const uint32_t sf0 = uniform(smem_u32(&sf_bar[0]));
-    const int a_lo = watcher ? 2 : 0, a_hi = p.fp4 ? a_lo + 2 : (watcher ? 0 : 1);
-    int stage = 0;
-    uint32_t phase = 0;
-    int e = 0, it = 0;
+  } else if (warp == 10) {
+    // ======================= accumulator watcher =======================
+    // Polls the accumulator-ready barrier for the epilogue warps and releases them through a hardware named barrier;
+    // after a timeout it releases them once more and stops.
     bool ok = true;
-    const uint32_t sf_bytes = atoms * 512;
+    int it = 0;
     for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x, ++it) {
-      if (a_hi > a_lo) {
-        const BsTile t = bs_decode(tile, e, s_tile_start, s_off, p.mode, n_tiles, p.k_iters);
-        const int k_iters = uniform(t.k_iters);
-#pragma unroll 1
-        for (int kb = 0; kb < k_iters; ++kb) {
-          ok = warp_mbar_wait(&full_bar[stage], phase, &abort_flag);
-          if (!ok) break;
-          const uint32_t ssa = ring + stage * stage_bytes + kBsABytes + kWdBBytes, ssb = ssa + sf_bytes;
-          const uint32_t sfa_t = tmem_base + kWdSfTmemBase + stage * 64u;
-          const uint32_t sfb_t = sfa_t + 16u;
-          if (elected) {
-            for (int a = a_lo; a < a_hi; ++a) {
-              tmem_cp_sf_atom(sfa_t + 4 * a, sf_smem_desc(ssa + a * 512));
-              tmem_cp_sf_atom(sfb_t + 8 * a, sf_smem_desc(ssb + a * 512));
-              tmem_cp_sf_atom(sfb_t + 8 * a + 4, sf_smem_desc(ssb + sf_bytes + a * 512));
-            }
-            tcgen05_commit_addr(sf0 + stage * 8);
-          }
-          __syncwarp();
-          if (++stage == stages) {
-            stage = 0;
-            phase ^= 1u;
-          }
-        }
-      }
-      if (watcher) {
-        if (lane == 0) ok = handover_report(&s_first_bad, it, ok && mbar_wait(&tmem_full_bar, it & 1u, &abort_flag));
-        ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
-        asm volatile("bar.arrive %0, %1;" ::"r"(handover_barrier(it)), "r"(8 * 32 + 32) : "memory");
-      }
+      if (lane == 0) ok = handover_report(&s_first_bad, it, mbar_wait(&tmem_full_bar, it & 1u, &abort_flag));
+      ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
+      asm volatile("bar.arrive %0, %1;" ::"r"(handover_barrier(it)), "r"(8 * 32 + 32) : "memory");
     }
-    if (lane == 0) s_stop[watcher ? 3 : 2] = ring_stop(stage, phase);
-    __syncwarp();
   } else {
     // ======================= epilogue =======================
     // Eight warps: two per TMEM lane quadrant, each owning 128 of the tile's 256 columns.  A lane reads its own
@@ -641,8 +610,6 @@ __global__ void __launch_bounds__(kWdThreads, 1) blockscaled_wide_kernel(const _
       const uint64_t deadline = globaltimer_ns() + kSettleNs;
       settle_ring(empty_bar, stages, s_stop[1], deadline);
       settle_ring(full_bar, stages, s_stop[0], deadline);
-      settle_ring(sf_bar, stages, s_stop[2], deadline);
-      if (p.fp4) settle_ring(sf_bar, stages, s_stop[3], deadline);
     }
     __syncthreads();
   }

@@ -8,10 +8,11 @@
 // accumulator holds C transposed (TMEM lane = weight row, column = routed row).  A K stage then costs four MMAs of
 // N = 32 or 64 and eight scale-atom copies, and the weights stream through once.
 //
-//   * with MMAs this short the issue of tcgen05 instructions counts.  The scale-atom copies and the MMAs of a stage are
-//     issued by two different warps (the copier commits to a per-stage barrier the MMA warp waits on), both converged around
-//     an elected lane (one lane in a divergent branch: W13 of 42 experts x 5632 x 2816 MXFP8 140.5 us, now 135 us; NVFP4
-//     32 x 4096 x 7168 116 us, now 112 us), and two CTAs share an SM, each with 256 TMEM columns and three stages;
+//   * with MMAs this short the issue of tcgen05 instructions counts.  One warp, converged around an elected lane, copies a
+//     stage's scale atoms and issues its MMAs: eight copies and four MMAs of N = 32 take 224 cycles (162 without the copies),
+//     and no barrier stands between them.  With a copier warp of its own a layer took 245 us (MXFP8, 16 tokens, 128 experts x
+//     2816 x 2816) and 207 us (NVFP4, 128 tokens, 32 experts x 7168 x 2048), now 240 and 202.  Two CTAs share an SM, each
+//     with 256 TMEM columns and three stages;
 //   * a stage = 128 bytes of K: 16 KiB of weights (one TMA box), 4 or 8 KiB of routed rows (32-row boxes),
 //     and the stage's scale atoms of both;
 //   * the rows' scale atom covers 128 rows in four TMEM columns of 32 rows each, so a tile that starts at row
@@ -28,7 +29,7 @@ namespace dm {
 
 constexpr int kSwStages = 3;
 constexpr int kSwCtasPerSm = 2;
-constexpr int kSwThreads = 256;  // TMA warp, MMA warp, four epilogue warps, accumulator watcher, scale copier
+constexpr int kSwThreads = 224;  // TMA warp, MMA warp, four epilogue warps, accumulator watcher
 constexpr int kSwTileRows = 64;  // routed rows per tile (the MMA's N), in steps of 32
 constexpr uint32_t kSwWBytes = 128 * 128;            // 16 KiB of weights
 constexpr uint32_t kSwXBytes = kSwTileRows * 128;    // up to 8 KiB of routed rows
@@ -90,11 +91,10 @@ __global__ void __launch_bounds__(kSwThreads, kSwCtasPerSm) blockscaled_swapped_
 
   __shared__ uint64_t full_bar[kSwStages];
   __shared__ uint64_t empty_bar[kSwStages];
-  __shared__ uint64_t sf_bar[kSwStages];  // the stage's scale atoms are in TMEM
   __shared__ uint64_t tmem_full_bar[2];
   __shared__ uint64_t tmem_empty_bar[2];
   __shared__ uint32_t tmem_base_slot;
-  __shared__ uint32_t s_stop[3];  // where the producer, the issuer and the scale copier stopped
+  __shared__ uint32_t s_stop[2];  // where the producer and the issuer stopped
   __shared__ int abort_flag;
   __shared__ volatile int s_first_bad;  // first of this CTA's tiles whose accumulator never came
   __shared__ int s_off[kSwMaxGroups + 1];
@@ -116,7 +116,6 @@ __global__ void __launch_bounds__(kSwThreads, kSwCtasPerSm) blockscaled_swapped_
     for (int s = 0; s < kSwStages; ++s) {
       mbar_init(&full_bar[s], 1);
       mbar_init(&empty_bar[s], 1);
-      mbar_init(&sf_bar[s], 1);
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(&tmem_full_bar[b], 1);
@@ -202,9 +201,9 @@ __global__ void __launch_bounds__(kSwThreads, kSwCtasPerSm) blockscaled_swapped_
     constexpr uint32_t kDescHi = (1024u >> 4) | (1u << 14) | (2u << 29);  // SBO 1024, version 1, 128-byte swizzle
     constexpr uint32_t kLbo = (16u >> 4) << 16;
     const uint32_t full0 = uniform(smem_u32(&full_bar[0])), empty0 = uniform(smem_u32(&empty_bar[0]));
-    const uint32_t sf0 = uniform(smem_u32(&sf_bar[0])), tfull0 = uniform(smem_u32(&tmem_full_bar[0]));
+    const uint32_t tfull0 = uniform(smem_u32(&tmem_full_bar[0]));
     int stage = 0;
-    uint32_t phase = 0, ready = 0;  // ready: the current stage and its scales are known to be there
+    uint32_t phase = 0, ready = 0;  // ready: the current stage is known to be there
     int e = 0, it = 0;
     bool ok = true;
     for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x, ++it) {
@@ -224,12 +223,13 @@ __global__ void __launch_bounds__(kSwThreads, kSwCtasPerSm) blockscaled_swapped_
 #pragma unroll 1
       for (int kb = 0; kb < p.k_iters; ++kb) {
         if (!__all_sync(0xffffffffu, ready)) {
-          ok = warp_mbar_wait(&full_bar[stage], phase, &abort_flag) && warp_mbar_wait(&sf_bar[stage], phase, &abort_flag);
+          ok = warp_mbar_wait(&full_bar[stage], phase, &abort_flag);
           if (!ok) break;
         }
         tcgen05_fence_after();
         const uint32_t w_addr = ring + stage * kSwStageBytes;
         const uint32_t w_lo = ((w_addr & 0x3ffffu) >> 4) | kLbo, x_lo = (((w_addr + kSwWBytes) & 0x3ffffu) >> 4) | kLbo;
+        const uint32_t sfw_lo = sf_desc_lo(w_addr + kSwWBytes + kSwXBytes), sfx_lo = sfw_lo + (kSwSfBytes >> 4);
         const uint32_t sfw_t = tmem_base + kSwSfTmemBase + stage * 32u;
         const uint32_t sfx_t = sfw_t + 16u;
         const uint32_t empty = empty0 + stage * 8;
@@ -237,14 +237,21 @@ __global__ void __launch_bounds__(kSwThreads, kSwCtasPerSm) blockscaled_swapped_
           stage = 0;
           phase ^= 1u;
         }
-        ready = mbar_test(full0 + stage * 8, phase) & mbar_test(sf0 + stage * 8, phase);
+        ready = mbar_test(full0 + stage * 8, phase);
         if (elected) {
           if (p.fp4) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              tmem_cp_sf_lo(sfw_t + 4 * j, sfw_lo + j * kSfAtomWords);
+              tmem_cp_sf_lo(sfx_t + 4 * j, sfx_lo + j * kSfAtomWords);
+            }
 #pragma unroll
             for (int j = 0; j < 4; ++j)
               umma_nvf4_lo(d_tmem, w_lo + 2 * j, x_lo + 2 * j, kDescHi, idesc4, sfw_t + 4 * j, sfx_t + 4 * j + col_off,
                            (kb > 0 || j > 0) ? 1u : 0u);
           } else {
+            tmem_cp_sf_lo(sfw_t, sfw_lo);
+            tmem_cp_sf_lo(sfx_t, sfx_lo);
 #pragma unroll
             for (int j = 0; j < 4; ++j)
               umma_mxf8_lo(d_tmem, w_lo + 2 * j, x_lo + 2 * j, kDescHi, idesc8[j], sfw_t, sfx_t + col_off,
@@ -264,39 +271,6 @@ __global__ void __launch_bounds__(kSwThreads, kSwCtasPerSm) blockscaled_swapped_
       __syncwarp();
     }
     if (lane == 0) s_stop[1] = ring_stop(stage, phase);
-    __syncwarp();
-  } else if (warp == 7) {
-    // ======================= scale copier =======================
-    // Moves every stage's scale atoms from shared memory to the stage slot's TMEM columns.  The slot's previous
-    // MMAs are complete by then: the producer refilled the stage only after their commit released it.
-    const bool elected = elect_one();
-    const uint32_t sf0 = uniform(smem_u32(&sf_bar[0]));
-    int stage = 0;
-    uint32_t phase = 0;
-    bool ok = true;
-    for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
-#pragma unroll 1
-      for (int kb = 0; kb < p.k_iters; ++kb) {
-        ok = warp_mbar_wait(&full_bar[stage], phase, &abort_flag);
-        if (!ok) break;
-        const uint32_t ssw = ring + stage * kSwStageBytes + kSwWBytes + kSwXBytes, ssx = ssw + kSwSfBytes;
-        const uint32_t sfw_t = tmem_base + kSwSfTmemBase + stage * 32u;
-        const uint32_t sfx_t = sfw_t + 16u;
-        if (elected) {
-          for (int a = 0; a < atoms; ++a) {
-            tmem_cp_sf_atom(sfw_t + 4 * a, sf_smem_desc(ssw + a * 512));
-            tmem_cp_sf_atom(sfx_t + 4 * a, sf_smem_desc(ssx + a * 512));
-          }
-          tcgen05_commit_addr(sf0 + stage * 8);
-        }
-        __syncwarp();
-        if (++stage == kSwStages) {
-          stage = 0;
-          phase ^= 1u;
-        }
-      }
-    }
-    if (lane == 0) s_stop[2] = ring_stop(stage, phase);
     __syncwarp();
   } else if (warp == 6) {
     // ======================= accumulator watcher =======================
@@ -404,7 +378,6 @@ __global__ void __launch_bounds__(kSwThreads, kSwCtasPerSm) blockscaled_swapped_
       const uint64_t deadline = globaltimer_ns() + kSettleNs;
       settle_ring(empty_bar, kSwStages, s_stop[1], deadline);
       settle_ring(full_bar, kSwStages, s_stop[0], deadline);
-      settle_ring(sf_bar, kSwStages, s_stop[2], deadline);
     }
     __syncthreads();
   }

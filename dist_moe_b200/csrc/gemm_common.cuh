@@ -115,6 +115,20 @@ __device__ __forceinline__ void umma_nvf4_lo(uint32_t d_tmem, uint32_t a_lo, uin
       ::"r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(desc_hi), "r"(idesc), "r"(accumulate), "r"(sfa_tmem), "r"(sfb_tmem)
       : "memory");
 }
+// Scale atoms (512 bytes each) by the lower word of their no-swizzle descriptor: rows 16 bytes apart, 8-row groups 128.  An
+// atom (32 rows x 16 bytes in shared memory) goes to 4 TMEM columns, replicated over the four 32-lane sub-partitions.
+constexpr uint32_t kSfAtomWords = 512u >> 4;
+__device__ __forceinline__ uint32_t sf_desc_lo(uint32_t smem_addr) { return ((smem_addr & 0x3ffffu) >> 4) | ((16u >> 4) << 16); }
+__device__ __forceinline__ void tmem_cp_sf_lo(uint32_t taddr, uint32_t lo) {
+  asm volatile(
+      "{\n\t"
+      ".reg .b64 d;\n\t"
+      "mov.b64 d, {%1, %2};\n\t"
+      "tcgen05.cp.cta_group::1.32x128b.warpx4 [%0], d;\n\t"
+      "}\n"
+      ::"r"(taddr), "r"(lo), "n"((128 >> 4) | (1 << 14))
+      : "memory");
+}
 __device__ __forceinline__ void tcgen05_commit_addr(uint32_t bar_addr) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar_addr) : "memory");
 }
