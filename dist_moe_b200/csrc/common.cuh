@@ -247,42 +247,87 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
   return *reinterpret_cast<uint32_t*>(&v);
 }
 
-// sigmoid(x) = 1 / (1 + exp(-x)) with an IEEE round-to-nearest reciprocal.
-__device__ __forceinline__ float sigmoid_rn(float x) { return __frcp_rn(1.0f + expf(-x)); }
-
 struct ActParams {
   int clamped;   // 0 = plain SwiGLU, 1 = clamped
   float alpha;   // sigmoid multiplier (clamped only)
   float limit;   // clamp bound (clamped only)
 };
 
-// h2 = SwiGLU(gate, up) in fp32.
-__device__ __forceinline__ float swiglu_f32(float gate, float up, const ActParams& act) {
-  if (act.clamped) {
-    float g = fminf(gate, act.limit);
-    float u = fminf(fmaxf(up, -act.limit), act.limit);
-    return g * sigmoid_rn(act.alpha * g) * (u + 1.0f);
+// 1 / d rounded to nearest for 1 <= d <= 2^126 (or NaN): one Newton step in fused arithmetic from an approximation within one
+// ulp (P. Markstein, Computation of elementary functions on the IBM RISC System/6000 processor, 1990).  Equal to
+// __frcp_rn for every float of that range, compared one by one.  No branch: the IEEE reciprocal tests the range of each
+// operand, and the activation of eight elements then runs as eight dependent chains one after the other.
+// One B200: SwiGLU forward / backward of 24 576 x 1408 55 -> 47 / 72 -> 61 us, W13 with SwiGLU (64 experts x 384 rows, 2048 x
+// 2816) 280 -> 253 us, the MXFP8 quantisers behind it (73 728 x 1536) 213 -> 187 and 325 -> 281 us.
+__device__ __forceinline__ float rcp_newton(float d) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(d));
+  return fmaf(y, fmaf(-d, y, 1.0f), y);
+}
+
+// s = 1 / (1 + exp(-x)) with the reciprocal rounded to nearest.
+template <int N>
+__device__ __forceinline__ void sigmoid_rn(const float (&x)[N], float (&s)[N]) {
+  float d[N];
+  bool far = false;  // some reciprocal is subnormal or zero
+#pragma unroll
+  for (int j = 0; j < N; ++j) {
+    d[j] = 1.0f + expf(-x[j]);
+    s[j] = rcp_newton(d[j]);
+    far = far || d[j] > 0x1p126f;
   }
-  return gate * sigmoid_rn(gate) * up;
+  if (far) {
+#pragma unroll
+    for (int j = 0; j < N; ++j)
+      if (d[j] > 0x1p126f) s[j] = __frcp_rn(d[j]);
+  }
+}
+
+// h2 = SwiGLU(gate, up) in fp32.
+template <int N>
+__device__ __forceinline__ void swiglu_f32(const float (&gate)[N], const float (&up)[N], float (&z)[N], const ActParams& act) {
+  float x[N], s[N];
+  if (act.clamped) {
+#pragma unroll
+    for (int j = 0; j < N; ++j) x[j] = act.alpha * fminf(gate[j], act.limit);
+    sigmoid_rn(x, s);
+#pragma unroll
+    for (int j = 0; j < N; ++j)
+      z[j] = fminf(gate[j], act.limit) * s[j] * (fminf(fmaxf(up[j], -act.limit), act.limit) + 1.0f);
+  } else {
+    sigmoid_rn(gate, s);
+#pragma unroll
+    for (int j = 0; j < N; ++j) z[j] = gate[j] * s[j] * up[j];
+  }
 }
 
 // Gradients of h2 = SwiGLU(x, y) with respect to the gate x and the up value y, given dz = dL/dh2
 // (dist_moe/kernels/triton/swiglu.py:639-668: where a clamp saturates, that input's gradient is zero).
-__device__ __forceinline__ void swiglu_bwd_f32(float x, float y, float dz, const ActParams& act, float& dx, float& dy) {
+template <int N>
+__device__ __forceinline__ void swiglu_bwd_f32(const float (&x)[N], const float (&y)[N], const float (&dz)[N],
+                                               const ActParams& act, float (&dx)[N], float (&dy)[N]) {
+  float s[N];
   if (act.clamped) {
-    const float g = fminf(x, act.limit);
-    const float u = fminf(fmaxf(y, -act.limit), act.limit);
-    const float s = sigmoid_rn(act.alpha * g);
-    const float silu = g * s;
-    const float d_silu = s + act.alpha * g * s * (1.0f - s);
-    float a = dz * (u + 1.0f) * d_silu;
-    float b = dz * silu;
-    dx = x > act.limit ? 0.0f : a;
-    dy = (y > act.limit || y < -act.limit) ? 0.0f : b;
+    float t[N];
+#pragma unroll
+    for (int j = 0; j < N; ++j) t[j] = act.alpha * fminf(x[j], act.limit);
+    sigmoid_rn(t, s);
+#pragma unroll
+    for (int j = 0; j < N; ++j) {
+      const float g = fminf(x[j], act.limit);
+      const float u = fminf(fmaxf(y[j], -act.limit), act.limit);
+      const float silu = g * s[j];
+      const float d_silu = s[j] + act.alpha * g * s[j] * (1.0f - s[j]);
+      dx[j] = x[j] > act.limit ? 0.0f : dz[j] * (u + 1.0f) * d_silu;
+      dy[j] = (y[j] > act.limit || y[j] < -act.limit) ? 0.0f : dz[j] * silu;
+    }
   } else {
-    const float s = sigmoid_rn(x);
-    dx = dz * y * s * (1.0f + x - x * s);
-    dy = dz * x * s;
+    sigmoid_rn(x, s);
+#pragma unroll
+    for (int j = 0; j < N; ++j) {
+      dx[j] = dz[j] * y[j] * s[j] * (1.0f + x[j] - x[j] * s[j]);
+      dy[j] = dz[j] * x[j] * s[j];
+    }
   }
 }
 

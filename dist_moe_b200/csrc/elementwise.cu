@@ -44,15 +44,15 @@ __global__ void __launch_bounds__(256) swiglu_fwd_kernel(const uint8_t* h1_base,
     float g[8], u[8], z[8];
     unpack8(g4, g);
     unpack8(u4, u);
+    swiglu_f32(g, u, z, act);
+    if (kClip) {
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      z[j] = swiglu_f32(g[j], u[j], act);
-      if (kClip) {
+      for (int j = 0; j < 8; ++j) {
         n_gate += g[j] > clip_limit ? 1.f : 0.f;
         n_up += fabsf(u[j]) > clip_limit ? 1.f : 0.f;
       }
+      n_all += 8.f;
     }
-    if (kClip) n_all += 8.f;
     h2[r * vec_per_row + v] = pack8(z);
   }
   if (kClip) {
@@ -100,8 +100,7 @@ __global__ void __launch_bounds__(256) swiglu_bwd_kernel(const uint8_t* h1_base,
     unpack8(h1[r * 2 * vec_per_row + v], x);
     unpack8(h1[r * 2 * vec_per_row + vec_per_row + v], y);
     unpack8(gh2[r * vec_per_row + v], dz);
-#pragma unroll
-    for (int j = 0; j < 8; ++j) swiglu_bwd_f32(x[j], y[j], dz[j], act, dx[j], dy[j]);
+    swiglu_bwd_f32(x, y, dz, act, dx, dy);
     gh1[r * 2 * vec_per_row + v] = pack8(dx);
     gh1[r * 2 * vec_per_row + vec_per_row + v] = pack8(dy);
   }

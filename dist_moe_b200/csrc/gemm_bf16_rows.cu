@@ -460,10 +460,19 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kRwThreads, 1) rows_
 #pragma unroll
           for (int i = 0; i < 8; ++i) o[i] = __shfl_xor_sync(0xffffffffu, up ? w[i] : w[8 + i], 16);
 #pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            const uint32_t gw = up ? o[i] : w[i], uw = up ? w[8 + i] : o[i];
-            z[i] = pack_bf16x2(swiglu_f32(__uint_as_float(gw << 16), __uint_as_float(uw << 16), p.act),
-                               swiglu_f32(__uint_as_float(gw & 0xffff0000u), __uint_as_float(uw & 0xffff0000u), p.act));
+          for (int h = 0; h < 2; ++h) {
+            float gf[8], uf[8], zf[8];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              const uint32_t gw = up ? o[4 * h + i] : w[4 * h + i], uw = up ? w[8 + 4 * h + i] : o[4 * h + i];
+              gf[2 * i] = __uint_as_float(gw << 16);
+              gf[2 * i + 1] = __uint_as_float(gw & 0xffff0000u);
+              uf[2 * i] = __uint_as_float(uw << 16);
+              uf[2 * i + 1] = __uint_as_float(uw & 0xffff0000u);
+            }
+            swiglu_f32(gf, uf, zf, p.act);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) z[4 * h + i] = pack_bf16x2(zf[2 * i], zf[2 * i + 1]);
           }
           const int chunk = 2 * quad + (word >> 2);
           if (p.c_base != nullptr) {

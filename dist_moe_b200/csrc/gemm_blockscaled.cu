@@ -483,7 +483,8 @@ __global__ void __launch_bounds__(kWdThreads, 1) blockscaled_wide_kernel(const _
           uint4 zv[4], gv[4], uv[4];
 #pragma unroll
           for (int g = 0; g < 4; ++g) {
-            uint32_t gw[4], uw[4], zw[4];
+            uint32_t gw[4], uw[4];
+            float gf[8], uf[8], zf[8];
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
               const int b = 16 * (g & 1) + 2 * q;
@@ -495,12 +496,13 @@ __global__ void __launch_bounds__(kWdThreads, 1) blockscaled_wide_kernel(const _
               }
               gw[q] = pack_bf16x2(g0, g1);
               uw[q] = pack_bf16x2(u0, u1);
-              const float z0 = swiglu_f32(__uint_as_float(gw[q] << 16), __uint_as_float(uw[q] << 16), p.act);
-              const float z1 =
-                  swiglu_f32(__uint_as_float(gw[q] & 0xffff0000u), __uint_as_float(uw[q] & 0xffff0000u), p.act);
-              zw[q] = pack_bf16x2(z0, z1);
+              gf[2 * q] = __uint_as_float(gw[q] << 16);
+              gf[2 * q + 1] = __uint_as_float(gw[q] & 0xffff0000u);
+              uf[2 * q] = __uint_as_float(uw[q] << 16);
+              uf[2 * q + 1] = __uint_as_float(uw[q] & 0xffff0000u);
             }
-            zv[g] = make_uint4(zw[0], zw[1], zw[2], zw[3]);
+            swiglu_f32(gf, uf, zf, p.act);
+            zv[g] = make_uint4(pack_bf16x2(zf[0], zf[1]), pack_bf16x2(zf[2], zf[3]), pack_bf16x2(zf[4], zf[5]), pack_bf16x2(zf[6], zf[7]));
             gv[g] = make_uint4(gw[0], gw[1], gw[2], gw[3]);
             uv[g] = make_uint4(uw[0], uw[1], uw[2], uw[3]);
           }

@@ -329,12 +329,20 @@ __global__ void __launch_bounds__(kSwThreads, kSwCtasPerSm) blockscaled_swapped_
           const bool is_gate = (lane & 8) == 0;
           const int fl = (lane >> 4) * 8 + (lane & 7);
 #pragma unroll
-          for (int i = 0; i < 32; ++i) {
-            float v = __uint_as_float(r[i]);
-            if (scaled) v = (v * __shfl_sync(0xffffffffu, my_scale, i)) * escale;
-            const float vb = __uint_as_float(pack_bf16x2(0.0f, v) & 0xffff0000u);  // bf16-rounded, as h1 would hold it
-            const float other = __shfl_xor_sync(0xffffffffu, vb, 8);
-            if (is_gate) tp[i * 16 + fl] = static_cast<uint16_t>(pack_bf16x2(swiglu_f32(vb, other, p.act), 0.0f) & 0xffffu);
+          for (int i0 = 0; i0 < 32; i0 += 8) {
+            float vb[8], other[8], z[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+              float v = __uint_as_float(r[i0 + j]);
+              if (scaled) v = (v * __shfl_sync(0xffffffffu, my_scale, i0 + j)) * escale;
+              vb[j] = __uint_as_float(pack_bf16x2(0.0f, v) & 0xffff0000u);  // bf16-rounded, as h1 would hold it
+              other[j] = __shfl_xor_sync(0xffffffffu, vb[j], 8);
+            }
+            if (is_gate) {
+              swiglu_f32(vb, other, z, p.act);
+#pragma unroll
+              for (int j = 0; j < 8; ++j) tp[(i0 + j) * 16 + fl] = static_cast<uint16_t>(pack_bf16x2(z[j], 0.0f) & 0xffffu);
+            }
           }
           __syncwarp();
           const int f0 = col0 >> 1;

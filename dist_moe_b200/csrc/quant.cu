@@ -450,14 +450,11 @@ __global__ void __launch_bounds__(256, 3) mxfp8_colrow_kernel(const uint4* __res
     if (kSource == kTileSwiglu) {
 #pragma unroll 1
       for (int r = 0; r < 8; ++r) {
-        float g[8], u[8];
+        float g[8], u[8], z[8];
         unpack8f(slot[256 * r], g);
         unpack8f(up[256 * r], u);
-        uint32_t z[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-          z[j] = pack_bf16x2(swiglu_f32(g[2 * j], u[2 * j], act), swiglu_f32(g[2 * j + 1], u[2 * j + 1], act));
-        slot[256 * r] = make_uint4(z[0], z[1], z[2], z[3]);
+        swiglu_f32(g, u, z, act);
+        slot[256 * r] = make_uint4(pack_bf16x2(z[0], z[1]), pack_bf16x2(z[2], z[3]), pack_bf16x2(z[4], z[5]), pack_bf16x2(z[6], z[7]));
       }
     }
     uint4 w[8];
@@ -520,8 +517,7 @@ __global__ void __launch_bounds__(256, 2) mxfp8_swiglu_bwd_colrow_kernel(const u
       unpack8f(gate[256 * r], x);
       unpack8f(up[256 * r], y);
       unpack8f(grad[256 * r], d);
-#pragma unroll
-      for (int j = 0; j < 8; ++j) swiglu_bwd_f32(x[j], y[j], d[j], act, dx[j], dy[j]);
+      swiglu_bwd_f32(x, y, d, act, dx, dy);
       gate[256 * r] = make_uint4(pack_bf16x2(dx[0], dx[1]), pack_bf16x2(dx[2], dx[3]), pack_bf16x2(dx[4], dx[5]), pack_bf16x2(dx[6], dx[7]));
       up[256 * r] = make_uint4(pack_bf16x2(dy[0], dy[1]), pack_bf16x2(dy[2], dy[3]), pack_bf16x2(dy[4], dy[5]), pack_bf16x2(dy[6], dy[7]));
     }
