@@ -43,6 +43,12 @@ from ._execution import ExecutionOptions, PreparedWeight, RMSNormPostprocess
 from .formats import BlockScaledFormat, format_constants
 
 
+# Grouped GEMMs sized by the real rows of every expert (the routing step pads them to 128).
+_gemm = nat.lib.dm_gemm_blockscaled_counted
+_gemm_swiglu_mxfp8 = nat.lib.dm_gemm_blockscaled_swiglu_mxfp8_counted
+_gemm_dgrad = nat.lib.dm_gemm_blockscaled_dgrad_counted
+
+
 def _fmt_id(fmt: BlockScaledFormat) -> int:
     return 1 if fmt is BlockScaledFormat.NVFP4 else 0
 
@@ -250,14 +256,14 @@ def _workspace(state):
 
 
 # Inference calls whose experts receive at most this many rows on average take the swapped-operand GEMMs (rows on
-# the MMA's N side in steps of 32); above it a 128-row tile is mostly real rows and the 128 x 256 kernel wins.
-# Whole layer on one B200, swapped / 128 x 256, us.  NVFP4: 32 experts x 7168 x 2048 at 48 rows per expert 226 / 243, at 64
-# 237 / 247, at 96 274 / 255; 64 experts x 2048 x 2048 at 48 222 / 232, at 56 235 / 233, at 64 265 / 236.  MXFP8: 128
-# experts x 2816 x 2816 at 24 621 / 667, at 48 685 / 695, at 56 718 / 704; 32 experts x 4096 x 1536 at 24 186 / 196, at 48
-# 194 / 198, at 64 204 / 198.  So NVFP4 stops where its smaller layer stops winning; MXFP8 stops early, between 24 and 48 rows
-# the swapped form would be 1 to 6 % faster.  ``None`` keeps the per-format value.
+# the MMA's N side in steps of 32, two CTAs per SM); above it, for NVFP4, a 128-row tile is mostly real rows and the 128 x 256
+# kernel wins: whole layer on one B200, swapped / 128 x 256, us: 32 experts x 7168 x 2048 at 48 rows per expert 226 / 243, at
+# 64 237 / 247, at 96 274 / 255; 64 experts x 2048 x 2048 at 48 222 / 232, at 56 235 / 233, at 64 265 / 236.  MXFP8 has rows on
+# the N side of CTA pairs at every size, and quantises h2 on the way out: swapped / pairs, 128 experts x 2816 x 2816, 1 token
+# 99 / 82, 16 tokens (hot experts) 244 / 220, 256 tokens 580 / 561, 768 tokens 599 / 558; 32 x 4096 x 1536, 8 tokens 121.6 /
+# 120.8, 192 tokens 162 / 160.  ``None`` keeps the per-format value.
 SWAPPED_MAX_ROWS_PER_EXPERT = None
-_SWAPPED_MAX_ROWS = {BlockScaledFormat.NVFP4: 48, BlockScaledFormat.MXFP8_E4M3: 24}
+_SWAPPED_MAX_ROWS = {BlockScaledFormat.NVFP4: 48, BlockScaledFormat.MXFP8_E4M3: 0}
 
 
 def _view(buf: torch.Tensor, offset: int) -> nat.Operand:
@@ -370,26 +376,22 @@ def run_block_scaled(x, ids, scores, w13_weight, w2_weight, context: Any, option
         # MXFP8: the SwiGLU epilogue writes h2 already row-quantised, the operand of the W2 GEMM
         h2_dense = lay.dense
         h2_quantised = True
-        nat.check(nat.lib.dm_gemm_blockscaled_swiglu_mxfp8(_view(buf, lay.x_q), _view(buf, lay.x_sf),
-                                                           p13.fprop_data.data_ptr(), p13.fprop_scale.data_ptr(),
-                                                           _view(buf, lay.h_q), _view(buf, lay.h_sf),
-                                                           offsets.data_ptr(), el, max_rows, 2 * F, D, clamped, alpha,
-                                                           limit, None, state.num_sms, status, st),
-                  "dm_gemm_blockscaled_swiglu_mxfp8")
+        nat.check(_gemm_swiglu_mxfp8(_view(buf, lay.x_q), _view(buf, lay.x_sf), p13.fprop_data.data_ptr(),
+                                     p13.fprop_scale.data_ptr(), _view(buf, lay.h_q), _view(buf, lay.h_sf),
+                                     offsets.data_ptr(), real.data_ptr(), el, max_rows, 2 * F, D, clamped, alpha, limit,
+                                     None, state.num_sms, status, st), "dm_gemm_blockscaled_swiglu_mxfp8")
     elif fused:
         h2_dense = lay.dense
-        nat.check(nat.lib.dm_gemm_blockscaled(f, _view(buf, lay.x_q), _view(buf, lay.x_sf), p13.fprop_data.data_ptr(),
-                                              p13.fprop_scale.data_ptr(), none, _view(buf, h2_dense), None, row_inv,
-                                              nat.ptr(p13.global_scale_inv), offsets.data_ptr(), el, max_rows, 2 * F,
-                                              D, 1, clamped, alpha, limit, None, state.num_sms, status, st),
-                  "dm_gemm_blockscaled(w13+swiglu)")
+        nat.check(_gemm(f, _view(buf, lay.x_q), _view(buf, lay.x_sf), p13.fprop_data.data_ptr(),
+                        p13.fprop_scale.data_ptr(), none, _view(buf, h2_dense), None, row_inv,
+                        nat.ptr(p13.global_scale_inv), offsets.data_ptr(), real.data_ptr(), el, max_rows, 2 * F, D, 1,
+                        clamped, alpha, limit, None, state.num_sms, status, st), "dm_gemm_blockscaled(w13+swiglu)")
     else:
         h2_dense = lay.h2_dense
-        nat.check(nat.lib.dm_gemm_blockscaled(f, _view(buf, lay.x_q), _view(buf, lay.x_sf), p13.fprop_data.data_ptr(),
-                                              p13.fprop_scale.data_ptr(), _view(buf, lay.dense), none, None, row_inv,
-                                              nat.ptr(p13.global_scale_inv), offsets.data_ptr(), el, max_rows, 2 * F,
-                                              D, 0, 0, 1.0, 0.0, None, state.num_sms, status, st),
-                  "dm_gemm_blockscaled(w13)")
+        nat.check(_gemm(f, _view(buf, lay.x_q), _view(buf, lay.x_sf), p13.fprop_data.data_ptr(),
+                        p13.fprop_scale.data_ptr(), _view(buf, lay.dense), none, None, row_inv,
+                        nat.ptr(p13.global_scale_inv), offsets.data_ptr(), real.data_ptr(), el, max_rows, 2 * F, D, 0,
+                        0, 1.0, 0.0, None, state.num_sms, status, st), "dm_gemm_blockscaled(w13)")
         nat.check(nat.lib.dm_swiglu_fwd(buf.data_ptr() + lay.dense, None, buf.data_ptr() + h2_dense, None,
                                         recv.data_ptr(), max_rows, F, clamped, alpha, limit, None, 0.0, None, st),
                   "dm_swiglu_fwd")
@@ -415,11 +417,10 @@ def run_block_scaled(x, ids, scores, w13_weight, w2_weight, context: Any, option
                                                       real.data_ptr(), el, max_rows, D, F, 0, 0, 1.0, 0.0, None,
                                                       state.num_sms, status, st), "dm_gemm_blockscaled_swapped(w2)")
     else:
-        nat.check(nat.lib.dm_gemm_blockscaled(f, _view(buf, lay.h_q), _view(buf, lay.h_sf), p2.fprop_data.data_ptr(),
-                                              p2.fprop_scale.data_ptr(), none, none, sct.data_ptr(),
-                                              _view(buf, lay.h_inv) if lay.fp4 else none,
-                                              nat.ptr(p2.global_scale_inv), offsets.data_ptr(), el, max_rows, D, F, 0,
-                                              0, 1.0, 0.0, None, state.num_sms, status, st),
+        nat.check(_gemm(f, _view(buf, lay.h_q), _view(buf, lay.h_sf), p2.fprop_data.data_ptr(),
+                        p2.fprop_scale.data_ptr(), none, none, sct.data_ptr(),
+                        _view(buf, lay.h_inv) if lay.fp4 else none, nat.ptr(p2.global_scale_inv), offsets.data_ptr(),
+                        real.data_ptr(), el, max_rows, D, F, 0, 0, 1.0, 0.0, None, state.num_sms, status, st),
                   "dm_gemm_blockscaled(w2)")
     state.barrier(state.combine)
     out = torch.empty(T, D, dtype=torch.bfloat16, device=dev)
@@ -499,8 +500,8 @@ def _training_weights(w13_param, w2_param, p13, p2, cfg):
 
 
 class _TrainCall:
-    __slots__ = ("T", "R", "offsets", "recv", "fwd", "bwd", "sct", "h1", "x_col", "x_col_sf", "h2_col", "h2_col_sf",
-                 "h3", "p13", "p2", "rstd", "planned", "per_rank", "need", "cond", "fwd_state", "fwd_table",
+    __slots__ = ("T", "R", "offsets", "recv", "real", "fwd", "bwd", "sct", "h1", "x_col", "x_col_sf", "h2_col",
+                 "h2_col_sf", "h3", "p13", "p2", "rstd", "planned", "per_rank", "need", "cond", "fwd_state", "fwd_table",
                  "callback_state")
 
 
@@ -530,16 +531,17 @@ def _route_training(state, x, ids, options, c: "_TrainCall"):
     counts = torch.empty(el, dtype=torch.int32, device=dev)
     c.per_rank = torch.empty(ep, dtype=torch.int32, device=dev)
     c.offsets = torch.empty(el + 1, dtype=torch.int32, device=dev)
+    c.real = torch.empty(el, dtype=torch.int32, device=dev)  # rows per expert before the padding to 128
     c.fwd = torch.empty(size, dtype=torch.int64, device=dev)
     c.bwd = torch.empty(size, dtype=torch.int64, device=dev)
     c.sct = torch.empty(size, dtype=torch.int64, device=dev)
     stride = D * 2
-    nat.check(nat.lib.dm_route(state.routing.peer_ptrs.data_ptr(), state.dispatch.peer_ptrs.data_ptr(),
-                               state.combine.peer_ptrs.data_ptr(), state.rank, ep, T, K, E, stride, stride, stride, 128,
-                               state.capacity_rows, size, counts.data_ptr(), c.per_rank.data_ptr(),
-                               c.offsets.data_ptr(), c.fwd.data_ptr(), c.bwd.data_ptr(), c.sct.data_ptr(),
-                               state.route_workspace.data_ptr(), state.route_workspace_words, status, st),
-              nat.route_call_name(ep, T, el))
+    nat.check(nat.lib.dm_route_counted(state.routing.peer_ptrs.data_ptr(), state.dispatch.peer_ptrs.data_ptr(),
+                                       state.combine.peer_ptrs.data_ptr(), state.rank, ep, T, K, E, stride, stride,
+                                       stride, 128, state.capacity_rows, size, counts.data_ptr(), c.real.data_ptr(),
+                                       c.per_rank.data_ptr(), c.offsets.data_ptr(), c.fwd.data_ptr(), c.bwd.data_ptr(),
+                                       c.sct.data_ptr(), state.route_workspace.data_ptr(), state.route_workspace_words,
+                                       status, st), nat.route_call_name(ep, T, el))
     c.recv = c.offsets[el:]
 
 
@@ -564,7 +566,7 @@ def _mxfp8_forward_planned(state, x, ids, scores, p13, p2, options, need_h3: boo
     c.planned, c.p13, c.p2 = True, p13, p2
     c.h1 = c.x_col = c.x_col_sf = c.h2_col = c.h2_col_sf = c.h3 = c.callback_state = None
     _route_training(state, x, ids, options, c)
-    R, recv = c.R, c.recv.data_ptr()
+    R, recv, real = c.R, c.recv.data_ptr(), c.real.data_ptr()
     c.need = torch.empty(1, dtype=torch.uint8, device=dev)
     c.cond = torch.empty(1, dtype=torch.int32, device=dev)
     c.fwd_state = torch.empty(10, dtype=torch.int64, device=dev)  # [x, -, h1, -, h3, x_row, x_col, h2_row, h2_col, slot]
@@ -586,18 +588,16 @@ def _mxfp8_forward_planned(state, x, ids, scores, p13, p2, options, need_h3: boo
     nat.check(nat.lib.dm_quant_mxfp8_rowcol_gather_at(c.fwd.data_ptr(), recv, R, D, A(ft, 0, _A_Q), A(ft, 0, _A_SF),
                                                       A(ft, 0, _COL_Q), A(ft, 0, _COL_SF), None, st),
               "dm_quant_mxfp8_rowcol_gather_at(x)")
-    nat.check(nat.lib.dm_gemm_blockscaled(0, A(ft, 0, _A_Q), A(ft, 0, _A_SF), p13.fprop_data.data_ptr(),
-                                          p13.fprop_scale.data_ptr(), A(ft, 0, _C), none, None, none, None,
-                                          c.offsets.data_ptr(), el, R, 2 * F, D, 0, 0, 1.0, 0.0, None, state.num_sms,
-                                          status, st), "dm_gemm_blockscaled(w13)")
+    nat.check(_gemm(0, A(ft, 0, _A_Q), A(ft, 0, _A_SF), p13.fprop_data.data_ptr(), p13.fprop_scale.data_ptr(),
+                    A(ft, 0, _C), none, None, none, None, c.offsets.data_ptr(), real, el, R, 2 * F, D, 0, 0, 1.0, 0.0,
+                    None, state.num_sms, status, st), "dm_gemm_blockscaled(w13)")
     nat.check(nat.lib.dm_swiglu_fwd_quant_mxfp8_rowcol_at(A(ft, 1, _SRC_X), recv, R, F, clamped, alpha, limit,
                                                           A(ft, 1, _A_Q), A(ft, 1, _A_SF), A(ft, 1, _COL_Q),
                                                           A(ft, 1, _COL_SF), None, st),
               "dm_swiglu_fwd_quant_mxfp8_rowcol_at")
-    nat.check(nat.lib.dm_gemm_blockscaled(0, A(ft, 1, _A_Q), A(ft, 1, _A_SF), p2.fprop_data.data_ptr(),
-                                          p2.fprop_scale.data_ptr(), none, none, c.sct.data_ptr(), none, None,
-                                          c.offsets.data_ptr(), el, R, D, F, 0, 0, 1.0, 0.0, None, state.num_sms, status,
-                                          st), "dm_gemm_blockscaled(w2)")
+    nat.check(_gemm(0, A(ft, 1, _A_Q), A(ft, 1, _A_SF), p2.fprop_data.data_ptr(), p2.fprop_scale.data_ptr(), none, none,
+                    c.sct.data_ptr(), none, None, c.offsets.data_ptr(), real, el, R, D, F, 0, 0, 1.0, 0.0, None,
+                    state.num_sms, status, st), "dm_gemm_blockscaled(w2)")
     state.barrier(state.combine)
     out = torch.empty(T, D, dtype=torch.bfloat16, device=dev)
     post = options.experts_output_postprocess
@@ -634,7 +634,7 @@ def _mxfp8_backward_planned(state, c: _TrainCall, x_shape, ids, scores, w13_para
     clamped = 1 if cfg.activation == "swiglu_clamped" else 0
     alpha, limit = float(cfg.swiglu_alpha), float(cfg.swiglu_limit)
     need_x, need_scores, need_w13, need_w2 = needs
-    recv, offs = c.recv.data_ptr(), c.offsets.data_ptr()
+    recv, offs, real = c.recv.data_ptr(), c.offsets.data_ptr(), c.real.data_ptr()
     none = nat.Operand(None, 0, None)
     arena, combine = state.arena.data_ptr(), state.combine.local().data_ptr()
     bo = torch.empty(16, dtype=torch.int64, device=dev)
@@ -658,20 +658,18 @@ def _mxfp8_backward_planned(state, c: _TrainCall, x_shape, ids, scores, w13_para
         nat.check(nat.lib.dm_quant_mxfp8_rowcol_gather_at(c.fwd.data_ptr(), recv, R, D, A(0, _A_Q), A(0, _A_SF),
                                                           A(0, _COL_Q), A(0, _COL_SF), cond.data_ptr(), st),
                   "dm_quant_mxfp8_rowcol_gather_at(x recompute)")
-        nat.check(nat.lib.dm_gemm_blockscaled(0, A(0, _A_Q), A(0, _A_SF), c.p13.fprop_data.data_ptr(),
-                                              c.p13.fprop_scale.data_ptr(), A(0, _C), none, None, none, None, offs, el,
-                                              R, 2 * F, D, 0, 0, 1.0, 0.0, cond.data_ptr(), state.num_sms, status, st),
-                  "dm_gemm_blockscaled(w13 recompute)")
+        nat.check(_gemm(0, A(0, _A_Q), A(0, _A_SF), c.p13.fprop_data.data_ptr(), c.p13.fprop_scale.data_ptr(), A(0, _C),
+                        none, None, none, None, offs, real, el, R, 2 * F, D, 0, 0, 1.0, 0.0, cond.data_ptr(),
+                        state.num_sms, status, st), "dm_gemm_blockscaled(w13 recompute)")
         nat.check(nat.lib.dm_swiglu_fwd_quant_mxfp8_rowcol_at(A(1, _SRC_X), recv, R, F, clamped, alpha, limit,
                                                               A(1, _A_Q), A(1, _A_SF), A(1, _COL_Q), A(1, _COL_SF),
                                                               cond.data_ptr(), st),
                   "dm_swiglu_fwd_quant_mxfp8_rowcol_at(recompute)")
         if (need_scores or is_norm) and not is_callback:
             # the expert outputs again, scattered to their owners' combine buffers
-            nat.check(nat.lib.dm_gemm_blockscaled(0, A(1, _A_Q), A(1, _A_SF), c.p2.fprop_data.data_ptr(),
-                                                  c.p2.fprop_scale.data_ptr(), none, none, c.sct.data_ptr(), none, None,
-                                                  offs, el, R, D, F, 0, 0, 1.0, 0.0, cond.data_ptr(), state.num_sms,
-                                                  status, st), "dm_gemm_blockscaled(w2 recompute)")
+            nat.check(_gemm(0, A(1, _A_Q), A(1, _A_SF), c.p2.fprop_data.data_ptr(), c.p2.fprop_scale.data_ptr(), none,
+                            none, c.sct.data_ptr(), none, None, offs, real, el, R, D, F, 0, 0, 1.0, 0.0,
+                            cond.data_ptr(), state.num_sms, status, st), "dm_gemm_blockscaled(w2 recompute)")
             if is_norm:  # the fused RMSNorm backward works on the expert outputs in place in the combine buffer
                 nat.check(nat.lib.dm_cond_copy(arena, fs + 32, combine, None, T * K * D * 2,
                                                cond.data_ptr(), 0, st), "dm_cond_copy(load h3)")
@@ -701,9 +699,9 @@ def _mxfp8_backward_planned(state, c: _TrainCall, x_shape, ids, scores, w13_para
                                                       A(2, _COL_Q) if need_w2 else none,
                                                       A(2, _COL_SF) if need_w2 else none, None, st),
               "dm_quant_mxfp8_rowcol_gather_at(grad_h3)")
-    nat.check(nat.lib.dm_gemm_blockscaled_dgrad(A(2, _A_Q), A(2, _A_SF), c.p2.fprop_data.data_ptr(),
-                                                c.p2.dgrad_scale.data_ptr(), A(2, _C), None, offs, el, R, F, D, None,
-                                                state.num_sms, status, st), "dm_gemm_blockscaled_dgrad(w2)")
+    nat.check(_gemm_dgrad(A(2, _A_Q), A(2, _A_SF), c.p2.fprop_data.data_ptr(), c.p2.dgrad_scale.data_ptr(), A(2, _C),
+                          None, offs, real, el, R, F, D, None, state.num_sms, status, st),
+              "dm_gemm_blockscaled_dgrad(w2)")
     grad_w13 = grad_w2 = None
     owners = options.wgrad_parameter_owners or (None, None)
     if need_w2:
@@ -723,9 +721,8 @@ def _mxfp8_backward_planned(state, c: _TrainCall, x_shape, ids, scores, w13_para
                                                        A(4, _COL_SF) if need_w13 else none, st),
                   "dm_swiglu_bwd_quant_mxfp8_at")
     if need_x:
-        nat.check(nat.lib.dm_gemm_blockscaled_dgrad(A(4, _A_Q), A(4, _A_SF), c.p13.fprop_data.data_ptr(),
-                                                    c.p13.dgrad_scale.data_ptr(), none, c.bwd.data_ptr(), offs, el, R, D,
-                                                    2 * F, None, state.num_sms, status, st),
+        nat.check(_gemm_dgrad(A(4, _A_Q), A(4, _A_SF), c.p13.fprop_data.data_ptr(), c.p13.dgrad_scale.data_ptr(), none,
+                              c.bwd.data_ptr(), offs, real, el, R, D, 2 * F, None, state.num_sms, status, st),
                   "dm_gemm_blockscaled_dgrad(w13)")
     if need_w13:
         dst, acc, ret = _wgrad_destination(w13_param, (el, 2 * F, D), options, cfg, owners[0], wgrad_explicit[0], hooks,

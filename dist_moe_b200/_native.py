@@ -108,6 +108,11 @@ _SIGNATURES = {
         [c_int, Operand, Operand, _P, _P, Operand, Operand, _P, Operand, _P, _P, c_int, c_int64, c_int64, c_int64,
          c_int, c_int, c_float, c_float, _P, c_int, _P, _P],
     ),
+    "dm_gemm_blockscaled_counted": (
+        c_int,
+        [c_int, Operand, Operand, _P, _P, Operand, Operand, _P, Operand, _P, _P, _P, c_int, c_int64, c_int64, c_int64,
+         c_int, c_int, c_float, c_float, _P, c_int, _P, _P],
+    ),
     "dm_gemm_blockscaled_swapped": (
         c_int,
         [c_int, Operand, Operand, _P, _P, Operand, Operand, _P, Operand, _P, _P, _P, c_int, c_int64, c_int64, c_int64,
@@ -122,6 +127,15 @@ _SIGNATURES = {
         c_int,
         [Operand, Operand, _P, _P, Operand, Operand, _P, c_int, c_int64, c_int64, c_int64, c_int, c_float, c_float, _P,
          c_int, _P, _P],
+    ),
+    "dm_gemm_blockscaled_swiglu_mxfp8_counted": (
+        c_int,
+        [Operand, Operand, _P, _P, Operand, Operand, _P, _P, c_int, c_int64, c_int64, c_int64, c_int, c_float, c_float, _P,
+         c_int, _P, _P],
+    ),
+    "dm_gemm_blockscaled_dgrad_counted": (
+        c_int,
+        [Operand, Operand, _P, _P, Operand, _P, _P, _P, c_int, c_int64, c_int64, c_int64, _P, c_int, _P, _P],
     ),
     "dm_gemm_blockscaled_dgrad": (
         c_int,

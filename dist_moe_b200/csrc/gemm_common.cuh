@@ -30,6 +30,12 @@ __device__ __forceinline__ uint4 pack8_bf16(const uint32_t* r) {
                     pack_bf16x2(__uint_as_float(r[6]), __uint_as_float(r[7])));
 }
 
+// 16 bytes to global memory (a peer's included).  Through a generic pointer the store might alias the staging tile, and the
+// next read of the tile would wait for it.
+__device__ __forceinline__ void store_global16(uint64_t addr, uint4 v) {
+  asm volatile("st.global.v4.b32 [%0], {%1, %2, %3, %4};" ::"l"(addr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w));
+}
+
 // ---------------------------------------------------------------------------
 // Issuing warps.  tcgen05 and TMA instructions take their operands from uniform registers.  Code that only one lane runs
 // (`if (lane == 0)`) keeps everything in per-lane registers and moves each operand over for each instruction: 85 to 93
@@ -197,6 +203,31 @@ __device__ __forceinline__ void umma_bf16_lo_pair(uint32_t d_tmem, uint32_t a_lo
       "tcgen05.mma.cta_group::2.kind::f16 [%0], da, db, %4, p;\n\t"
       "}\n"
       ::"r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(desc_hi), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+__device__ __forceinline__ void umma_mxf8_lo_pair(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t desc_hi,
+                                                  uint32_t idesc, uint32_t sfa_tmem, uint32_t sfb_tmem, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t"
+      ".reg .pred p;\n\t"
+      ".reg .b64 da, db;\n\t"
+      "setp.ne.b32 p, %5, 0;\n\t"
+      "mov.b64 da, {%1, %3};\n\t"
+      "mov.b64 db, {%2, %3};\n\t"
+      "tcgen05.mma.cta_group::2.kind::mxf8f6f4.block_scale [%0], da, db, %4, [%6], [%7], p;\n\t"
+      "}\n"
+      ::"r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(desc_hi), "r"(idesc), "r"(accumulate), "r"(sfa_tmem), "r"(sfb_tmem)
+      : "memory");
+}
+// Both CTAs copy the atom at this offset of their own shared memory to these columns of their own TMEM.
+__device__ __forceinline__ void tmem_cp_sf_lo_pair(uint32_t taddr, uint32_t lo) {
+  asm volatile(
+      "{\n\t"
+      ".reg .b64 d;\n\t"
+      "mov.b64 d, {%1, %2};\n\t"
+      "tcgen05.cp.cta_group::2.32x128b.warpx4 [%0], d;\n\t"
+      "}\n"
+      ::"r"(taddr), "r"(lo), "n"((128 >> 4) | (1 << 14))
       : "memory");
 }
 // Arrive on the barrier at this shared-memory offset in both CTAs of the pair once the MMAs issued so far are complete.

@@ -334,6 +334,18 @@ int dm_gemm_blockscaled(int format, dm_operand a, dm_operand sfa, const void* w,
                         int64_t N, int64_t Kd, int swiglu_interleaved, int clamped, float alpha, float limit,
                         const int* cond, int num_sms, int* status, void* stream);
 
+/* dm_gemm_blockscaled given `expert_counts` (int32 [e_local], real rows inside each 128-padded group; NULL = the whole
+ * group).  MXFP8: the work is sized by real rows rounded up to 32.  Rows of a dense C past them are computed from A (up to
+ * the next multiple of 32) or set to zero, what the product gives for the zero rows that pad a group; h2 and scattered
+ * rows past the count are not written.  Runs on pairs of neighbouring SMs: an odd num_sms is used down to the next even
+ * number, 1 takes one pair.  Device offsets of `a` and `sfa` must be multiples of 128.  NVFP4: whole groups. */
+int dm_gemm_blockscaled_counted(int format, dm_operand a, dm_operand sfa, const void* w, const void* sfb, dm_operand c,
+                                dm_operand h2, const int64_t* scatter_ptrs, dm_operand row_scale_inv,
+                                const float* expert_scale_inv, const int32_t* expert_offsets,
+                                const int32_t* expert_counts, int e_local, int64_t max_rows, int64_t N, int64_t Kd,
+                                int swiglu_interleaved, int clamped, float alpha, float limit, const int* cond,
+                                int num_sms, int* status, void* stream);
+
 /* The same product for experts that received few rows (decode): weights on the 128-row side of the MMA, the
  * expert's rows on the N side in steps of 32, so that a K stage costs MMAs of N = 32 or 64 instead of a 128-row
  * tile and the layer is bound by streaming the weights once.  Replaces the reference's compact decode tiles
@@ -356,8 +368,12 @@ int dm_gemm_blockscaled_swiglu_mxfp8(dm_operand a, dm_operand sfa, const void* w
                                      dm_operand h2_sf, const int32_t* expert_offsets, int e_local, int64_t max_rows,
                                      int64_t N, int64_t Kd, int clamped, float alpha, float limit, const int* cond,
                                      int num_sms, int* status, void* stream);
-
- /* the current setting, without changing it */
+/* ... given the real rows of every group, as dm_gemm_blockscaled_counted: rows past them are not written */
+int dm_gemm_blockscaled_swiglu_mxfp8_counted(dm_operand a, dm_operand sfa, const void* w, const void* sfb, dm_operand h2_q,
+                                             dm_operand h2_sf, const int32_t* expert_offsets,
+                                             const int32_t* expert_counts, int e_local, int64_t max_rows, int64_t N,
+                                             int64_t Kd, int clamped, float alpha, float limit, const int* cond,
+                                             int num_sms, int* status, void* stream);
 
 /* MXFP8 training backward GEMMs (dist_moe/_blockscaled_ops.py: `dist_blockscaled_grouped_gemm_dgrad_dispatch`,
  * `..._dgrad_swiglu_bwd_combine`, `blockscaled_grouped_gemm_wgrad`; sequencing dist_moe/_blockscaled.py:2284-2512).
@@ -376,6 +392,11 @@ int dm_gemm_blockscaled_dgrad(dm_operand dy, dm_operand sf_dy, const void* w, co
                               const int64_t* scatter_ptrs, const int32_t* expert_offsets, int e_local,
                               int64_t max_rows, int64_t N, int64_t Kd, const int* cond, int num_sms, int* status,
                               void* stream);
+/* ... given the real rows of every group, as dm_gemm_blockscaled_counted */
+int dm_gemm_blockscaled_dgrad_counted(dm_operand dy, dm_operand sf_dy, const void* w, const void* sfb_dgrad, dm_operand c,
+                                      const int64_t* scatter_ptrs, const int32_t* expert_offsets,
+                                      const int32_t* expert_counts, int e_local, int64_t max_rows, int64_t N, int64_t Kd,
+                                      const int* cond, int num_sms, int* status, void* stream);
 int dm_gemm_blockscaled_wgrad(dm_operand dy_col, dm_operand sf_dy_col, dm_operand x_col, dm_operand sf_x_col, void* dw,
                               int dw_is_fp32, int accumulate, const int32_t* expert_offsets, int e_local,
                               int64_t max_rows, int64_t M, int64_t N, const int* cond, int num_sms, int* status,

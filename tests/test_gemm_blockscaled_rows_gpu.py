@@ -1,0 +1,124 @@
+"""MXFP8 GEMMs over routed rows (pairs of CTAs, rows on the MMA's N side) at the edges of their tiles: experts of no
+row, of one row, of one row more than a step of 32, an atom of 128 and a tile of 256, tiles that start inside a scale atom,
+and an odd number of 128-column blocks.  References and bounds as in test_gemm_blockscaled_gpu."""
+
+import pytest
+import torch
+
+from tests.test_gemm_blockscaled_gpu import _close, _nat, _quant_act, _tile32_weight
+from tests.test_gemm_blockscaled_swapped_gpu import _operands
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+COUNTS = [[1, 0, 33, 128, 129], [256, 257, 31], [300, 545, 0, 64], [1040]]
+
+
+def _op(nat, t):
+    return nat.Operand(t.data_ptr(), t.numel() * t.element_size(), None) if t is not None else nat.Operand(None, 0, None)
+
+
+@pytest.mark.parametrize("counts", COUNTS)
+@pytest.mark.parametrize("K,N", [(256, 384), (1280, 256)])
+def test_dense_and_scattered_rows(counts, K, N):
+    nat, fmt = _nat(), 0
+    E, off, real, R, (qa, sa, da, inv), (qw, sw, dw, einv), offs, cnts = _operands(nat, fmt, counts, K, N, 3 * fmt + K)
+    status = torch.zeros(8, dtype=torch.int32, device=DEV)
+    out = torch.full((R + 8, N), 5.0, device=DEV, dtype=torch.bfloat16)
+    sct = torch.full((R, N), 5.0, device=DEV, dtype=torch.bfloat16)
+    perm = torch.randperm(R, device=DEV)
+    ptrs = torch.zeros(R, dtype=torch.int64, device=DEV)
+    ptrs[real.to(DEV)] = sct.data_ptr() + perm[real.to(DEV)].to(torch.int64) * (N * 2)
+    for dst, table in ((out, None), (None, ptrs)):
+        rc = nat.lib.dm_gemm_blockscaled_counted(fmt, _op(nat, qa), _op(nat, sa), qw.data_ptr(), sw.data_ptr(), _op(nat, dst),
+                                                 _op(nat, None), nat.ptr(table), _op(nat, inv), nat.ptr(einv),
+                                                 offs.data_ptr(), cnts.data_ptr(), E, R, N, K, 0, 0, 1.0, 0.0, None, 0,
+                                                 status.data_ptr(), nat.stream_ptr())
+        nat.check(rc, "dm_gemm_blockscaled_counted")
+    torch.cuda.synchronize()
+    assert status[0].item() == 0, status.tolist()
+    got, touched = sct.cpu(), torch.zeros(R, dtype=torch.bool)
+    for e, n in enumerate(counts):
+        rows = torch.arange(off[e], off[e] + n)
+        if n:
+            _close(out.cpu()[rows], da[rows] @ dw[e].T, f"expert {e}")
+            touched[perm.cpu()[rows]] = True
+            assert torch.equal(got[perm.cpu()[rows]], out.cpu()[rows])
+        assert bool((out[off[e] + n:off[e + 1]] == 0).all()), "padding rows of a dense result are zero"
+    assert bool((out[off[-1]:] == 5.0).all()) and bool((got[~touched] == 5.0).all())
+
+
+@pytest.mark.parametrize("counts", COUNTS)
+def test_swiglu_rows(counts):
+    """h1, h2 and the quantised h2, at 2F = 384: the last pair of column blocks is half empty."""
+    nat, fmt = _nat(), 0
+    K, F = 512, 192
+    N = 2 * F
+    E, off, real, R, (qa, sa, da, inv), (qw, sw, dw, einv), offs, cnts = _operands(nat, fmt, counts, K, N, 17 + fmt, F)
+    status = torch.zeros(8, dtype=torch.int32, device=DEV)
+    h1 = torch.full((R, N), 5.0, device=DEV, dtype=torch.bfloat16)
+    h2 = torch.full((R, F), 5.0, device=DEV, dtype=torch.bfloat16)
+    st = nat.stream_ptr()
+    nat.check(nat.lib.dm_gemm_blockscaled_counted(fmt, _op(nat, qa), _op(nat, sa), qw.data_ptr(), sw.data_ptr(), _op(nat, h1),
+                                                  _op(nat, h2), None, _op(nat, inv), nat.ptr(einv), offs.data_ptr(),
+                                                  cnts.data_ptr(), E, R, N, K, 1, 0, 1.702, 7.0, None, 0,
+                                                  status.data_ptr(), st), "swiglu")
+    atoms = (F // 32 + 3) // 4
+    want_q, want_s = torch.zeros(R, F, dtype=torch.uint8, device=DEV), torch.zeros(R * atoms * 4, dtype=torch.uint8, device=DEV)
+    got_q, got_s = torch.zeros_like(want_q), torch.zeros_like(want_s)
+    live = torch.zeros(R, dtype=torch.int64, device=DEV)
+    live[real.to(DEV)] = 1
+    rows = torch.tensor([R], dtype=torch.int32, device=DEV)
+    nat.check(nat.lib.dm_quant_mxfp8_row_live(live.data_ptr(), h2.data_ptr(), rows.data_ptr(), R, F, want_q.data_ptr(), 0,
+                                              want_s.data_ptr(), 0, 1, st), "row")
+    nat.check(nat.lib.dm_gemm_blockscaled_swiglu_mxfp8_counted(_op(nat, qa), _op(nat, sa), qw.data_ptr(), sw.data_ptr(),
+                                                               _op(nat, got_q), _op(nat, got_s), offs.data_ptr(),
+                                                               cnts.data_ptr(), E, R, N, K, 0, 1.702, 7.0, None, 0,
+                                                               status.data_ptr(), st), "swiglu + quant")
+    torch.cuda.synchronize()
+    assert status[0].item() == 0, status.tolist()
+    idx = torch.stack([torch.arange(F).reshape(-1, 8), torch.arange(F).reshape(-1, 8) + F], dim=1).reshape(-1)
+    inv_idx = torch.empty_like(idx)
+    inv_idx[idx] = torch.arange(N)
+    pad = torch.ones(R, dtype=torch.bool)
+    pad[real] = False
+    h1c, h2c = h1.cpu(), h2.cpu()
+    for e, n in enumerate(counts):
+        rows = torch.arange(off[e], off[e] + n)
+        if n:
+            _close(h1c[rows], (da[rows] @ dw[e].T)[:, inv_idx], f"h1 expert {e}")
+            g, u = h1c[rows, :F].float(), h1c[rows, F:].float()
+            _close(h2c[rows], g * torch.sigmoid(g) * u, f"h2 expert {e}")
+    assert bool((h1c[pad] == 5.0).all()) and bool((h2c[pad] == 5.0).all())
+    assert torch.equal(got_q, want_q) and torch.equal(got_s, want_s)
+
+
+@pytest.mark.parametrize("counts", COUNTS)
+@pytest.mark.parametrize("K,N", [(256, 384), (640, 256)])
+def test_input_gradient_rows(counts, K, N):
+    nat = _nat()
+    off = [0]
+    for n in counts:
+        off.append(off[-1] + (n + 127) // 128 * 128)
+    E, R = len(counts), max(off[-1], 128)
+    torch.manual_seed(K + N)
+    dy = torch.zeros(R, K, device=DEV, dtype=torch.bfloat16)
+    for e, n in enumerate(counts):
+        dy[off[e]:off[e] + n] = torch.randn(n, K, device=DEV).bfloat16()
+    w = (torch.randn(E, K, N, device=DEV) * 0.05).bfloat16()
+    qa, sa, da, _ = _quant_act(nat, dy, 0)
+    qw, _, s_dgrad, dw = _tile32_weight(nat, w)
+    offs = torch.tensor(off, dtype=torch.int32, device=DEV)
+    cnts = torch.tensor(counts, dtype=torch.int32, device=DEV)
+    status = torch.zeros(8, dtype=torch.int32, device=DEV)
+    out = torch.full((R + 8, N), 5.0, device=DEV, dtype=torch.bfloat16)
+    nat.check(nat.lib.dm_gemm_blockscaled_dgrad_counted(_op(nat, qa), _op(nat, sa), qw.data_ptr(), s_dgrad.data_ptr(),
+                                                        _op(nat, out), None, offs.data_ptr(), cnts.data_ptr(), E, R, N, K,
+                                                        None, 0, status.data_ptr(), nat.stream_ptr()), "dgrad")
+    torch.cuda.synchronize()
+    assert status[0].item() == 0, status.tolist()
+    for e, n in enumerate(counts):
+        rows = torch.arange(off[e], off[e] + n)
+        if n:
+            _close(out.cpu()[rows], da[rows] @ dw[e], f"expert {e}")
+        assert bool((out[off[e] + n:off[e + 1]] == 0).all())
+    assert bool((out[off[-1]:] == 5.0).all())
