@@ -19,37 +19,15 @@ from __future__ import annotations
 from typing import Any
 
 import torch
-from torch.profiler import record_function
 
 from . import _native as nat
+from ._call import BWD, FWD, FWD_ALL, CallState, arguments, launch, observed, span
 from ._execution import ExecutionOptions, RMSNormPostprocess
 
 
 # When set to a list, every grouped-GEMM launch is bracketed by CUDA events on the launching
 # stream and (name, start, end) is appended; benchmarks use it to time the kernels in place.
 PROFILE: list | None = None
-
-
-def _profiled(fn):
-    def call(*args, what: str):
-        if PROFILE is None:
-            nat.check(fn(*args), what)
-            return
-        start, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-        start.record()
-        nat.check(fn(*args), what)
-        end.record()
-        PROFILE.append((what, start, end))
-
-    return call
-
-
-_gemm_fprop = _profiled(nat.lib.dm_gemm_fprop)
-_gemm_dgrad = _profiled(nat.lib.dm_gemm_dgrad)
-_gemm_fprop_dispatch = _profiled(nat.lib.dm_gemm_fprop_dispatch)
-_gemm_dgrad_dispatch = _profiled(nat.lib.dm_gemm_dgrad_dispatch)
-_gemm_wgrad = _profiled(nat.lib.dm_gemm_wgrad)
-
 
 # Fused dispatch pulls the routed rows inside the W13 / W2-dgrad GEMM launches (gather warps overlap the peer
 # transfer with the tensor cores).  With False the rows are gathered by a separate kernel first.
@@ -59,128 +37,64 @@ FUSED_DISPATCH = True
 READ_SAVED_H3_IN_PLACE = True
 
 
-def _dispatch_fprop(state, ptrs, a_op_off, w, c_op, h2_op, c, N, Kd, fuse, act, condp, what):
-    clamped, alpha, limit = act
-    st, status = nat.stream_ptr(), state.status.data_ptr()
-    if FUSED_DISPATCH:
-        _gemm_fprop_dispatch(ptrs.data_ptr(), state.gather_flags.data_ptr(), _op(state, a_op_off), w.data_ptr(), c_op,
-                             h2_op, c.offsets.data_ptr(), state.e_local, c.max_rows, N, Kd, int(fuse), clamped, alpha,
-                             limit, condp, state.num_sms, status, st, what=what)
-        return
-    nat.check(nat.lib.dm_gather_rows(ptrs.data_ptr(), c.recv_rows.data_ptr(), state.arena.data_ptr(),
-                                     a_op_off, Kd * 2, c.max_rows, condp, st), "dm_gather_rows")
-    _gemm_fprop(_op(state, a_op_off), w.data_ptr(), c_op, h2_op, None, c.offsets.data_ptr(), state.e_local,
-                c.max_rows, N, Kd, int(fuse), clamped, alpha, limit, condp, state.num_sms, status, st, what=what)
+class _Call(CallState):
+    """Device results of routing and planning of one BF16 call."""
+
+    def __init__(self, state=None, T: int = 0, with_bwd: bool = True):
+        fields = {}
+        if state is not None:
+            el, size = state.e_local, state.ep * state.e_local * T
+            i64, i32 = torch.int64, torch.int32
+            fields = {"fwd_state": (i64, 6), "need": (torch.uint8, 1), "cond": (i32, 1), "counts": (i32, el),
+                      "per_rank": (i32, state.ep), "offsets": (i32, el + 1), "fwd": (i64, size), "sct": (i64, size),
+                      "bwd": (i64, size if with_bwd else 0)}
+            self.T, self.size, self.max_rows = T, size, min(size, state.capacity_rows)
+        super().__init__(fields)
 
 
-class _Call:
-    """Per-call device tensors produced by routing and planning."""
-
-    __slots__ = ("T", "counts", "per_rank", "offsets", "recv_rows", "fwd", "bwd", "sct", "need", "cond", "fwd_state",
-                 "max_rows", "rstd", "callback_state")
-
-
-# Planner offsets are named by the address of their int64 (base address of the offset tensor + 8 per entry): slicing the
-# tensor for every operand cost the host more than the launch it was for.
-def _op(state, offset_address: int) -> nat.Operand:
-    return state.arena_at(offset_address)
+def _arguments(state, c: _Call, x, ids, scores, w13, w2, options: ExecutionOptions, scratch_only: bool):
+    k = arguments(state, c, x, ids, scores, options)
+    k.w13, k.w2 = w13.data_ptr(), w2.data_ptr()
+    k.scratch_only, k.separate_gather = scratch_only, not FUSED_DISPATCH
+    return k
 
 
-def _none() -> nat.Operand:
-    return nat.Operand(None, 0, None)
+def _forward(state, k, steps: int) -> None:
+    launch(nat.lib.dm_bf16_forward, FWD, state, k, steps)
 
 
-def _act(config) -> tuple[int, float, float]:
-    return (1 if config.activation == "swiglu_clamped" else 0, float(config.swiglu_alpha), float(config.swiglu_limit))
+def _backward(state, k, steps: int) -> None:
+    launch(nat.lib.dm_bf16_backward, BWD, state, k, steps)
 
 
-def _route_and_plan(state, x, ids, scratch_only: bool, validate: bool) -> _Call:
+def forward_impl(state, x, ids, scores, w13, w2, options: ExecutionOptions, save_for_backward: bool, hooks=None,
+                 separate: bool = False):
+    """``separate``: the call's device results as tensors of their own (registered operators return them)."""
     cfg = state.config
-    T, D, K, E = x.shape[0], cfg.hidden_dim, cfg.top_k, cfg.num_experts
-    dev, st = x.device, nat.stream_ptr()
-    el, ep = state.e_local, state.ep
-    with record_function("dist_moe_preprocess"):  # publish ids and rows, then the barrier every peer waits on
-        nat.check(nat.lib.dm_publish(x.data_ptr(), ids.data_ptr(), int(ids.dtype == torch.int64),
-                                     state.dispatch.local().data_ptr(), state.routing.local().data_ptr(), T, D, K, E,
-                                     int(validate), state.status.data_ptr(), st), "dm_publish")
-        state.barrier(state.dispatch)
-    c = _Call()
-    c.T = T
-    size = ep * el * T
-    c.counts = torch.empty(el, dtype=torch.int32, device=dev)
-    c.per_rank = torch.empty(ep, dtype=torch.int32, device=dev)
-    c.offsets = torch.empty(el + 1, dtype=torch.int32, device=dev)
-    c.fwd = torch.empty(size, dtype=torch.int64, device=dev)
-    c.bwd = None if scratch_only else torch.empty(size, dtype=torch.int64, device=dev)
-    c.sct = torch.empty(size, dtype=torch.int64, device=dev)
-    c.max_rows = min(size, state.capacity_rows)
-    stride = D * 2
-    nat.check(nat.lib.dm_route(state.routing.peer_ptrs.data_ptr(), state.dispatch.peer_ptrs.data_ptr(),
-                               state.combine.peer_ptrs.data_ptr(), state.rank, ep, T, K, E, stride, stride, stride, 0,
-                               state.capacity_rows, size, c.counts.data_ptr(), c.per_rank.data_ptr(),
-                               c.offsets.data_ptr(), c.fwd.data_ptr(), nat.ptr(c.bwd), c.sct.data_ptr(),
-                               state.route_workspace.data_ptr(), state.route_workspace_words,
-                               state.status.data_ptr(), st), nat.route_call_name(ep, T, el))
-    c.recv_rows = c.offsets[el:]
-    c.need = torch.empty(1, dtype=torch.uint8, device=dev)
-    c.cond = torch.empty(1, dtype=torch.int32, device=dev)
-    c.fwd_state = torch.empty(6, dtype=torch.int64, device=dev)
-    nat.check(nat.lib.dm_plan_fwd_bf16(c.recv_rows.data_ptr(), c.per_rank.data_ptr(), state.saved_bytes.data_ptr(),
-                                       state.buffer_offsets.data_ptr(), state.peak_min_free.data_ptr(),
-                                       c.need.data_ptr(), c.cond.data_ptr(), c.fwd_state.data_ptr(),
-                                       state.slot_selector.data_ptr(), state.moe_layer_id.data_ptr(), ep,
-                                       cfg.max_num_local_input_tokens, K, D, cfg.intermediate_dim,
-                                       state.slot_bytes, state.num_slots, state.num_layers_in_slot,
-                                       int(scratch_only), state.status.data_ptr(), st), "dm_plan_fwd_bf16")
-    c.rstd = None
-    c.callback_state = None
-    state.last_call = c
-    return c
-
-
-def _expert_forward(state, c: _Call, w13, w2, xg_off, h1_off, h2_off, *, fuse: bool, cond, clip, clip_limit,
-                    keep_h1: bool = True) -> None:
-    """gather -> W13 (+SwiGLU) -> W2 + scatter into the owners' combine buffers."""
-    cfg = state.config
-    D, F, el = cfg.hidden_dim, cfg.intermediate_dim, state.e_local
-    st, status = nat.stream_ptr(), state.status.data_ptr()
-    clamped, alpha, limit = _act(cfg)
-    condp = nat.ptr(cond)
-    # dispatch + W13: gather warps pull the routed rows (peer loads) while the tensor cores run
-    # (a forward without a backward has no reader of h1: the fused epilogue then writes h2 alone)
-    h1_op = _op(state, h1_off) if keep_h1 or not fuse else _none()
-    _dispatch_fprop(state, c.fwd, xg_off, w13, h1_op, _op(state, h2_off) if fuse else _none(), c, 2 * F, D,
-                    fuse, (clamped, alpha, limit), condp, "gemm_fprop_dispatch(w13)")
-    if not fuse:
-        nat.check(nat.lib.dm_swiglu_fwd(state.arena.data_ptr(), h1_off, state.arena.data_ptr(),
-                                        h2_off, c.recv_rows.data_ptr(), c.max_rows, F, clamped, alpha,
-                                        limit, nat.ptr(clip), float(clip_limit), None, st), "dm_swiglu_fwd")
-    _gemm_fprop(_op(state, h2_off), w2.data_ptr(), _none(), _none(), c.sct.data_ptr(),
-                                    c.offsets.data_ptr(), el, c.max_rows, D, F, 0, 0, 1.0, 0.0, condp, state.num_sms,
-                                    status, st, what="gemm_fprop(w2)")
-
-
-def forward_impl(state, x, ids, scores, w13, w2, options: ExecutionOptions, save_for_backward: bool, hooks=None):
-    cfg = state.config
-    T, D, K, F = x.shape[0], cfg.hidden_dim, cfg.top_k, cfg.intermediate_dim
-    st = nat.stream_ptr()
+    T, D, F = x.shape[0], cfg.hidden_dim, cfg.intermediate_dim
     scratch_only = (not save_for_backward) or cfg.inference or state.num_slots == 0
-    with record_function("dist_moe_routing"):  # the reference's profiler range names (dist_moe/api.py:1979-2072)
-        c = _route_and_plan(state, x, ids, scratch_only, options.validate_expert_ids)
-    fs = c.fwd_state.data_ptr()
-    if not scratch_only:
-        nat.check(nat.lib.dm_cond_copy(x.data_ptr(), None, state.arena.data_ptr(), fs, T * D * 2,
-                                       c.cond.data_ptr(), 1, st), "dm_cond_copy(save x)")
+    c = _Call(state, T, not scratch_only).allocate(x.device, separate)
+    out = torch.empty(T, D, dtype=torch.bfloat16, device=x.device)
+    k = _arguments(state, c, x, ids, scores, w13, w2, options, scratch_only)
+    k.out = out.data_ptr()
     clip = options.swiglu_clip_stats_out_3
     if clip is not None:
         clip.zero_()
-    fuse = clip is None and F % 128 == 0
-    with record_function("dist_moe_forward"):
-        _expert_forward(state, c, w13, w2, fs + 8, fs + 16, fs + 24, fuse=fuse, cond=None, clip=clip,
-                        clip_limit=options.swiglu_clip_limit, keep_h1=not scratch_only)
-    state.barrier(state.combine)
-    out = torch.empty(T, D, dtype=torch.bfloat16, device=x.device)
+        k.clip_stats, k.clip_limit = clip.data_ptr(), float(options.swiglu_clip_limit)
+    k.fuse_swiglu = clip is None and F % 128 == 0
     post = options.experts_output_postprocess
+    state.last_call = c
+    if not observed():
+        _forward(state, k, FWD_ALL if post is None else FWD_ALL - FWD["reduce"])
+    else:
+        with span("dist_moe_routing"):
+            with span("dist_moe_preprocess"):  # publish ids and rows, then the barrier every peer waits on
+                _forward(state, k, FWD["publish"])
+            _forward(state, k, FWD["route"])
+        _forward(state, k, FWD["save_x"])
+        with span("dist_moe_forward"):
+            _forward(state, k, FWD["w13"] | FWD["swiglu"] | FWD["w2"])
+        _forward(state, k, FWD["combine"] | (FWD["reduce"] if post is None else 0))
     if isinstance(post, RMSNormPostprocess):
         from ._postprocess import rmsnorm_combine_forward
 
@@ -192,13 +106,6 @@ def forward_impl(state, x, ids, scores, w13, w2, options: ExecutionOptions, save
         if hooks is None:
             raise RuntimeError("a callable expert-output post-process runs on the eager path only")
         hooks.postprocess_forward(state, c, post, scores, ids, out, save=not scratch_only)
-    else:
-        nat.check(nat.lib.dm_scale_and_sum(state.combine.local().data_ptr(), scores.data_ptr(),
-                                           int(scores.dtype == torch.bfloat16), ids.data_ptr(),
-                                           int(ids.dtype == torch.int64), out.data_ptr(), T, K, D,
-                                           None if scratch_only else state.arena.data_ptr(),
-                                           None if scratch_only else fs + 32,
-                                           None if scratch_only else c.cond.data_ptr(), 0, st), "dm_scale_and_sum")
     return out, c
 
 
@@ -243,126 +150,82 @@ def backward_impl(state, c: _Call, x_shape, ids, scores, w13, w2, w13_param, w2_
                   options: ExecutionOptions, needs, wgrad_explicit=(None, None), hooks=None):
     cfg = state.config
     T, D, K, F, el = c.T, cfg.hidden_dim, cfg.top_k, cfg.intermediate_dim, state.e_local
-    dev, st, status = grad_out.device, nat.stream_ptr(), state.status.data_ptr()
-    clamped, alpha, limit = _act(cfg)
+    dev = grad_out.device
     need_x, need_scores, need_w13, need_w2 = needs
     bo = torch.empty(6, dtype=torch.int64, device=dev)  # [xg, h1, h2, grad_h2, grad_h3_gathered, grad_h1]
-    nat.check(nat.lib.dm_plan_bwd_bf16(c.recv_rows.data_ptr(), c.per_rank.data_ptr(), state.saved_bytes.data_ptr(),
-                                       state.buffer_offsets.data_ptr(), state.peak_min_free.data_ptr(),
-                                       c.need.data_ptr(), c.fwd_state.data_ptr(), bo.data_ptr(),
-                                       state.moe_layer_id.data_ptr(), state.ep, cfg.max_num_local_input_tokens, K, D,
-                                       F, state.slot_bytes, state.num_slots, status, st), "dm_plan_bwd_bf16")
-    fs, bop, cond = c.fwd_state.data_ptr(), bo.data_ptr(), c.cond
-    arena = state.arena.data_ptr()
+    grad_scores = torch.empty(T, K, dtype=torch.float32, device=dev) if need_scores else None
     post = options.experts_output_postprocess
     is_norm = isinstance(post, RMSNormPostprocess)
     is_callback = post is not None and not is_norm  # the callable kept its own input and output (eager path)
-    # ---- recompute block (device-predicated on need_recompute) ----------------
-    span = record_function("dist_moe_recompute")
-    span.__enter__()
-    nat.check(nat.lib.dm_cond_copy(arena, fs, state.dispatch.local().data_ptr(), None, T * D * 2,
-                                   cond.data_ptr(), 1, st), "dm_cond_copy(republish x)")
-    state.barrier(state.dispatch, cond)
-    _dispatch_fprop(state, c.fwd, bop, w13, _op(state, bop + 8), _none(), c, 2 * F, D, False,
-                    (clamped, alpha, limit), cond.data_ptr(), "gemm_fprop_dispatch(w13 recompute)")
-    # h2 is always rebuilt from h1: only x_gathered, h1 and h3 are ever saved.
-    nat.check(nat.lib.dm_swiglu_fwd(arena, bop + 8, arena, bop + 16, c.recv_rows.data_ptr(),
-                                    c.max_rows, F, clamped, alpha, limit, None, 0.0, None, st), "dm_swiglu_fwd(bwd)")
-    need_h3 = (need_scores or is_norm) and not is_callback
-    if need_h3:
-        _gemm_fprop(_op(state, bop + 16), w2.data_ptr(), _none(), _none(), c.sct.data_ptr(),
-                                        c.offsets.data_ptr(), el, c.max_rows, D, F, 0, 0, 1.0, 0.0, cond.data_ptr(),
-                                        state.num_sms, status, st, what="gemm_fprop(w2 recompute)")
-        # Saved path: the fused RMSNorm backward works on the expert outputs in place in the communication buffer,
-        # so they are copied back there; the plain backward reads them where they were saved (selected on the device).
-        if is_norm or not READ_SAVED_H3_IN_PLACE:
-            nat.check(nat.lib.dm_cond_copy(arena, fs + 32, state.combine.local().data_ptr(), None,
-                                           T * K * D * 2, cond.data_ptr(), 0, st), "dm_cond_copy(load h3)")
-        state.barrier(state.combine, cond)
-    span.__exit__(None, None, None)
-    span = record_function("dist_moe_backward")
-    span.__enter__()
-    # ---- grad wrt expert outputs and scores ------------------------------------
-    grad_scores = torch.empty(T, K, dtype=torch.float32, device=dev) if need_scores else None
-    combine = state.combine.local().data_ptr()
-    if is_norm:
-        from ._postprocess import rmsnorm_combine_backward
+    k = _arguments(state, c, None, ids, scores, w13, w2, options, False)
+    k.bwd_offsets, k.grad_out, k.grad_scores = bo.data_ptr(), grad_out.data_ptr(), nat.ptr(grad_scores)
+    # Saved expert outputs: the fused RMSNorm backward works on them in place in the communication buffer, so they are
+    # copied back there; the plain backward reads them where they were saved (selected on the device).
+    load_h3 = is_norm or (need_scores and not is_callback and not READ_SAVED_H3_IN_PLACE)
+    k.h3_in_combine = load_h3
+    # recompute block: every launch is a no-op unless the forward chose to recompute this layer; h2 is always rebuilt
+    recompute = BWD["plan"] | BWD["republish"] | BWD["w13_again"] | BWD["swiglu_again"]
+    if (need_scores or is_norm) and not is_callback:
+        recompute |= BWD["w2_again"] | (BWD["load_h3"] if load_h3 else 0)
+    first = 0 if observed() or post is not None else recompute | BWD["grad_h3"] | BWD["combine"] | BWD["w2_dgrad"]
+    if first == 0:
+        with span("dist_moe_recompute"):
+            _backward(state, k, recompute)
+    with span("dist_moe_backward"):
+        # ---- grad wrt expert outputs and scores ------------------------------------
+        if is_norm:
+            from ._postprocess import rmsnorm_combine_backward
 
-        kept = None
-        if hooks is not None:
-            # the replay of a recomputed layer shows its expert outputs to the forward observer again; whether the
-            # layer was recomputed is a device-side decision, read here because observers run on the host anyway
-            if post.observe_expert_output_fn is not None and bool(c.need.item()):
-                hooks.observe_expert_output(state, post, ids, T)
-            kept = hooks.preserved_expert_output(state, post, ids, T)
-        rmsnorm_combine_backward(state, c, post, grad_out, scores, ids, grad_scores, h3=kept)
-        if kept is not None:
-            hooks.observe_expert_output_grad(state, post, kept, T)
-    elif is_callback:
-        hooks.postprocess_backward(state, c, grad_out, scores, ids, grad_scores)
-    else:
-        if need_scores and READ_SAVED_H3_IN_PLACE:
-            nat.check(nat.lib.dm_broadcast_and_scale_select(grad_out.data_ptr(), scores.data_ptr(),
-                                                            int(scores.dtype == torch.bfloat16), ids.data_ptr(),
-                                                            int(ids.dtype == torch.int64), arena, fs + 32,
-                                                            combine, cond.data_ptr(), combine, nat.ptr(grad_scores), T,
-                                                            K, D, st), "dm_broadcast_and_scale")
-        else:
-            nat.check(nat.lib.dm_broadcast_and_scale(grad_out.data_ptr(), scores.data_ptr(),
-                                                     int(scores.dtype == torch.bfloat16), ids.data_ptr(),
-                                                     int(ids.dtype == torch.int64), combine if need_scores else None,
-                                                     None, combine, nat.ptr(grad_scores), T, K, D, st),
-                      "dm_broadcast_and_scale")
-    state.barrier(state.combine)
-    # ---- W2: input gradient and weight gradient ----------------------------------
-    if FUSED_DISPATCH:
-        _gemm_dgrad_dispatch(c.sct.data_ptr(), state.gather_flags.data_ptr(), _op(state, bop + 32), w2.data_ptr(),
-                             _op(state, bop + 24), c.offsets.data_ptr(), el, c.max_rows, F, D, None, state.num_sms,
-                             status, st, what="gemm_dgrad_dispatch(w2)")
-    else:
-        nat.check(nat.lib.dm_gather_rows(c.sct.data_ptr(), c.recv_rows.data_ptr(), arena, bop + 32, D * 2,
-                                         c.max_rows, None, st), "dm_gather_rows(grad_h3)")
-        _gemm_dgrad(_op(state, bop + 32), w2.data_ptr(), _op(state, bop + 24), None, c.offsets.data_ptr(), el,
-                    c.max_rows, F, D, None, state.num_sms, status, st, what="gemm_dgrad(w2)")
-    grad_w13 = grad_w2 = None
-    owners = options.wgrad_parameter_owners or (None, None)
-    if need_w2:
-        dst, acc, ret = _wgrad_destination(w2_param, (el, D, F), options, cfg, owners[1], wgrad_explicit[1], hooks, "w2")
-        _gemm_wgrad(_op(state, bop + 32), _op(state, bop + 16), dst.data_ptr(),
-                                        int(dst.dtype == torch.float32), acc, c.offsets.data_ptr(), el, c.max_rows,
-                                        D, F, state.num_sms, status, st, what="gemm_wgrad(w2)")
-        grad_w2 = dst.view(w2_param.shape) if ret else None
-        if hooks is not None:
-            grad_w2 = hooks.wgrad_postprocess("w2", grad_w2)
-    # ---- SwiGLU backward, W13 input gradient (scattered to the owners) and weight gradient
-    nat.check(nat.lib.dm_swiglu_bwd(arena, bop + 8, arena, bop + 24, arena, bop + 40,
-                                    c.recv_rows.data_ptr(), c.max_rows, F, clamped, alpha, limit, st),
-              "dm_swiglu_bwd")
-    if need_x:
-        _gemm_dgrad(_op(state, bop + 40), w13.data_ptr(), _none(), c.bwd.data_ptr(),
-                                        c.offsets.data_ptr(), el, c.max_rows, D, 2 * F, None, state.num_sms, status,
-                                        st, what="gemm_dgrad(w13)")
-    if need_w13:
-        dst, acc, ret = _wgrad_destination(w13_param, (el, 2 * F, D), options, cfg, owners[0], wgrad_explicit[0], hooks,
-                                           "w13")
-        _gemm_wgrad(_op(state, bop + 40), _op(state, bop), dst.data_ptr(),
-                                        int(dst.dtype == torch.float32), acc, c.offsets.data_ptr(), el, c.max_rows,
-                                        2 * F, D, state.num_sms, status, st, what="gemm_wgrad(w13)")
-        grad_w13 = dst.view(w13_param.shape) if ret else None
-        if hooks is not None:
-            grad_w13 = hooks.wgrad_postprocess("w13", grad_w13)
-    grad_x = None
-    # The closing barrier is unconditional (dist_moe/api.py:2580): peers may still be pulling grad_h3 out of this
-    # rank's combine buffer, and the next call on this context overwrites it.
-    state.barrier(state.dispatch)
-    if need_x:
-        grad_x = torch.empty(x_shape, dtype=torch.bfloat16, device=dev)
-        nat.check(nat.lib.dm_scale_and_sum(state.dispatch.local().data_ptr(), None, 0, ids.data_ptr(),
-                                           int(ids.dtype == torch.int64), grad_x.data_ptr(), T, K, D, None, None,
-                                           None, 0, st), "dm_scale_and_sum(reduce_from_topk)")
-    if grad_scores is not None and scores.dtype != torch.float32:
-        grad_scores = grad_scores.to(scores.dtype)
-    span.__exit__(None, None, None)
+            kept = None
+            if hooks is not None:
+                # the replay of a recomputed layer shows its expert outputs to the forward observer again; whether the
+                # layer was recomputed is a device-side decision, read here because observers run on the host anyway
+                if post.observe_expert_output_fn is not None and bool(c.need.item()):
+                    hooks.observe_expert_output(state, post, ids, T)
+                kept = hooks.preserved_expert_output(state, post, ids, T)
+            rmsnorm_combine_backward(state, c, post, grad_out, scores, ids, grad_scores, h3=kept)
+            if kept is not None:
+                hooks.observe_expert_output_grad(state, post, kept, T)
+        elif is_callback:
+            hooks.postprocess_backward(state, c, grad_out, scores, ids, grad_scores)
+        rest = BWD["combine"] | BWD["w2_dgrad"] | (BWD["grad_h3"] if post is None else 0)
+        _backward(state, k, first if first else rest)
+        # ---- W2 weight gradient; SwiGLU backward, W13 input gradient (scattered to the owners) and weight gradient ----
+        grad_w13 = grad_w2 = grad_x = None
+        owners = options.wgrad_parameter_owners or (None, None)
+        steps = 0
+        if need_w2:
+            dst, k.dw2_accumulate, ret = _wgrad_destination(w2_param, (el, D, F), options, cfg, owners[1],
+                                                            wgrad_explicit[1], hooks, "w2")
+            k.dw2, k.dw2_is_fp32 = dst.data_ptr(), dst.dtype is torch.float32
+            grad_w2 = dst.view(w2_param.shape) if ret else None
+            steps = BWD["w2_wgrad"]
+            if hooks is not None:
+                _backward(state, k, steps)
+                grad_w2, steps = hooks.wgrad_postprocess("w2", grad_w2), 0
+        steps |= BWD["swiglu"]
+        if need_x:
+            steps |= BWD["w13_dgrad"]
+        if need_w13:
+            if hooks is not None:  # named destinations are asked for when the gradient is next
+                _backward(state, k, steps)
+                steps = 0
+            dst, k.dw13_accumulate, ret = _wgrad_destination(w13_param, (el, 2 * F, D), options, cfg, owners[0],
+                                                             wgrad_explicit[0], hooks, "w13")
+            k.dw13, k.dw13_is_fp32 = dst.data_ptr(), dst.dtype is torch.float32
+            grad_w13 = dst.view(w13_param.shape) if ret else None
+            steps |= BWD["w13_wgrad"]
+            if hooks is not None:
+                _backward(state, k, steps)
+                grad_w13, steps = hooks.wgrad_postprocess("w13", grad_w13), 0
+        steps |= BWD["close"]
+        if need_x:
+            grad_x = torch.empty(x_shape, dtype=torch.bfloat16, device=dev)
+            k.grad_x = grad_x.data_ptr()
+            steps |= BWD["reduce"]
+        _backward(state, k, steps)
+        if grad_scores is not None and scores.dtype != torch.float32:
+            grad_scores = grad_scores.to(scores.dtype)
     return grad_x, grad_scores, grad_w13, grad_w2
 
 
@@ -400,26 +263,47 @@ def _rmsnorm_args(post):
     return (None, False, 1e-6, torch.float32, torch.bfloat16, False, 0.0, False, False)
 
 
+def _plain_execution(*tensors) -> bool:
+    """Nothing acts on this call's operators: no tracing or fake tensors, no dispatch or function mode, no functorch
+    level.  The registered operators' bodies can then run without the dispatcher, which costs a small layer more than its
+    launches."""
+    return (torch._C._len_torch_dispatch_stack() == 0 and torch._C._len_torch_function_stack() == 0
+            and torch._ops._len_torch_dispatch_stack_pre_dispatch() == 0
+            and torch._C._functorch.peek_interpreter_stack() is None and torch._C._get_tracing_state() is None
+            and not torch.compiler.is_compiling()
+            and all(type(t) is torch.Tensor or type(t) is torch.nn.Parameter for t in tensors))
+
+
 class _RegisteredBf16Function(torch.autograd.Function):
     """Training call through the registered operators ``dist_moe::bf16_forward`` (``..._with_clip_stats``) and
     ``dist_moe::bf16_backward`` / ``bf16_backward_accumulate_`` (dist_moe/api.py:4027-4042 applies its
     ``_RegisteredBf16Autograd`` the same way), so that FakeTensor propagation, ``make_fx`` and ``torch.compile`` of
-    the caller's code see operator nodes with the reference's names and schemas."""
+    the caller's code see operator nodes with the reference's names and schemas.  Where nothing acts on operators
+    (``_plain_execution``) their bodies run directly, with the call's device results in one buffer."""
 
     @staticmethod
     def forward(ctx, x, ids, scores, w13_param, w2_param, context, options):
         state = context._state
+        clip = options.swiglu_clip_stats_out_3
+        ctx.context, ctx.options = context, options
+        ctx.direct = clip is None and _plain_execution(x, ids, scores, w13_param, w2_param)
+        if ctx.direct:
+            cfg = context.config
+            w13 = w13_param.detach().reshape(state.e_local, 2 * cfg.intermediate_dim, cfg.hidden_dim)
+            w2 = w2_param.detach().reshape(state.e_local, cfg.hidden_dim, cfg.intermediate_dim)
+            with span("dist_moe::bf16_forward"):
+                out, call = forward_impl(state, x.detach().contiguous(), ids, scores.detach(), w13, w2, options, True)
+            ctx.save_for_backward(ids, scores, w13_param, w2_param, call.buf, call.rstd)
+            return out
         rms = _rmsnorm_args(options.experts_output_postprocess)
         head = (x.detach().contiguous(), ids, scores.detach(), w13_param.detach(), w2_param.detach(), *rms,
                 state.slot_selector, state.num_layers_in_slot, bool(options.validate_expert_ids))
-        clip = options.swiglu_clip_stats_out_3
         if clip is None:
             out, st = torch.ops.dist_moe.bf16_forward(*head, context._context_id)
         else:
             out, st, counters = torch.ops.dist_moe.bf16_forward_with_clip_stats(*head, float(options.swiglu_clip_limit),
                                                                                   context._context_id)
             clip.copy_(counters)  # graph-visible copy into the caller's tensor
-        ctx.context, ctx.options, ctx.n_state = context, options, len(st)
         ctx.save_for_backward(ids, scores, w13_param, w2_param, *st)
         return out
 
@@ -429,27 +313,42 @@ class _RegisteredBf16Function(torch.autograd.Function):
 
         ids, scores, w13_param, w2_param, *st = ctx.saved_tensors
         context, options = ctx.context, ctx.options
-        cfg = context.config
+        cfg, state = context.config, context._state
+        needs = (ctx.needs_input_grad[0], ctx.needs_input_grad[2], ctx.needs_input_grad[3], ctx.needs_input_grad[4])
+        e_local, D, F = state.e_local, cfg.hidden_dim, cfg.intermediate_dim
+        destinations = (cfg.wgrad_dtype or w13_param.dtype,) * 2
+        if options.inplace_wgrad_accum:
+            owners = options.wgrad_parameter_owners or (None, None)
+            destinations = (_wgrad_destination(w13_param, (e_local, 2 * F, D), options, cfg, owners[0])[0],
+                            _wgrad_destination(w2_param, (e_local, D, F), options, cfg, owners[1])[0])
+        if ctx.direct:
+            call = _Call(state, ids.shape[0]).adopt(st[0])
+            call.rstd = st[1]
+            # a backward that is itself differentiated goes through the operators, which refuse it
+            if not torch.is_grad_enabled() and _plain_execution(grad_out, ids, scores, w13_param, w2_param, st[0]):
+                if context._closed:
+                    raise RuntimeError(f"distributed MoE context {context._context_id} is not live")
+                w13, w2 = w13_param.detach().reshape(e_local, 2 * F, D), w2_param.detach().reshape(e_local, D, F)
+                with torch.cuda.device(state.device), span("dist_moe::bf16_backward"):
+                    gx, gs, g13, g2 = backward_impl(state, call, grad_out.shape, ids, scores.detach(), w13, w2, w13_param,
+                                                    w2_param, grad_out.contiguous(), options, needs, destinations)
+                if options.inplace_wgrad_accum:
+                    torch.autograd.graph.increment_version(destinations)  # as the operator's mutated arguments
+                return gx, None, gs, g13, g2, None, None
+            st = _ops._pack_bf16_state(call, ids.device)
         rms = _rmsnorm_args(options.experts_output_postprocess)
         tail = (rms[1], rms[2], rms[3], rms[4], rms[5], rms[7], rms[8])
-        needs = (ctx.needs_input_grad[0], ctx.needs_input_grad[2], ctx.needs_input_grad[3], ctx.needs_input_grad[4])
-        e_local = context._state.e_local
-        D, F = cfg.hidden_dim, cfg.intermediate_dim
         _ops.NEEDS_HINT.append(needs)
         try:
             if options.inplace_wgrad_accum:
-                owners = options.wgrad_parameter_owners or (None, None)
-                acc13, _, _ = _wgrad_destination(w13_param, (e_local, 2 * F, D), options, cfg, owners[0])
-                acc2, _, _ = _wgrad_destination(w2_param, (e_local, D, F), options, cfg, owners[1])
                 gx, gs = torch.ops.dist_moe.bf16_backward_accumulate_(
-                    grad_out.contiguous(), w13_param.detach(), w2_param.detach(), acc13, acc2, ids, scores.detach(), st,
-                    *tail, acc13.dtype, context._context_id)
+                    grad_out.contiguous(), w13_param.detach(), w2_param.detach(), *destinations, ids, scores.detach(), st,
+                    *tail, destinations[0].dtype, context._context_id)
                 g13 = g2 = None
             else:
-                dtype = cfg.wgrad_dtype or w13_param.dtype
                 gx, gs, g13, g2 = torch.ops.dist_moe.bf16_backward(
-                    grad_out.contiguous(), w13_param.detach(), w2_param.detach(), ids, scores.detach(), st, *tail, dtype,
-                    context._context_id)
+                    grad_out.contiguous(), w13_param.detach(), w2_param.detach(), ids, scores.detach(), st, *tail,
+                    destinations[0], context._context_id)
         finally:
             _ops.NEEDS_HINT.clear()
         if gs is not None and needs[1] and gs.dtype != scores.dtype:

@@ -36,9 +36,9 @@ from __future__ import annotations
 from typing import Any
 
 import torch
-from torch.profiler import record_function
 
 from . import _native as nat
+from ._call import BWD, FWD, FWD_ALL, CallState, arguments, launch, observed, span
 from ._execution import ExecutionOptions, PreparedWeight, RMSNormPostprocess
 from .formats import BlockScaledFormat, format_constants
 
@@ -46,7 +46,6 @@ from .formats import BlockScaledFormat, format_constants
 # Grouped GEMMs sized by the real rows of every expert (the routing step pads them to 128).
 _gemm = nat.lib.dm_gemm_blockscaled_counted
 _gemm_swiglu_mxfp8 = nat.lib.dm_gemm_blockscaled_swiglu_mxfp8_counted
-_gemm_dgrad = nat.lib.dm_gemm_blockscaled_dgrad_counted
 
 
 def _fmt_id(fmt: BlockScaledFormat) -> int:
@@ -500,9 +499,8 @@ def _training_weights(w13_param, w2_param, p13, p2, cfg):
 
 
 class _TrainCall:
-    __slots__ = ("T", "R", "offsets", "recv", "real", "fwd", "bwd", "sct", "h1", "x_col", "x_col_sf", "h2_col",
-                 "h2_col_sf", "h3", "p13", "p2", "rstd", "planned", "per_rank", "need", "cond", "fwd_state", "fwd_table",
-                 "callback_state")
+    __slots__ = ("T", "R", "offsets", "recv", "fwd", "bwd", "sct", "h1", "x_col", "x_col_sf", "h2_col", "h2_col_sf", "h3",
+                 "p13", "p2", "rstd", "planned")
 
 
 # MXFP8 training keeps its activations in the context's arena, placed by the device planner (saved bundles in the
@@ -511,99 +509,43 @@ class _TrainCall:
 # ask for the SwiGLU clip counters (which need a dense h2 the plan has no room for) use per-call tensors instead.
 PLANNED_ARENA = True
 
-# groups of the planner's offset tables, nine entries each
-_A_Q, _B_Q, _C, _A_SF, _B_SF, _SRC_X, _SRC_Y, _COL_Q, _COL_SF = range(9)
+
+class _PlannedCall(CallState):
+    """Device results of routing and planning of one MXFP8 training call on the planner's placement."""
+
+    planned = True
+
+    def __init__(self, state, T: int, p13, p2):
+        K, el, ep = state.config.top_k, state.e_local, state.ep
+        size = max((ep * T * min(K, el) + el * 127 + 127) // 128 * 128, 128)
+        i64, i32 = torch.int64, torch.int32
+        # fwd_state: [x, -, h1, -, h3, x_row, x_col, h2_row, h2_col, slot]; real: rows per expert before the padding to 128
+        super().__init__({"fwd_state": (i64, 10), "fwd_table": (i64, 18), "need": (torch.uint8, 1), "cond": (i32, 1),
+                          "counts": (i32, el), "real": (i32, el), "per_rank": (i32, ep), "offsets": (i32, el + 1),
+                          "fwd": (i64, size), "bwd": (i64, size), "sct": (i64, size)})
+        self.T, self.size, self.max_rows = T, size, min(size, state.capacity_rows // 128 * 128)
+        self.p13, self.p2 = p13, p2
 
 
-def _route_training(state, x, ids, options, c: "_TrainCall"):
-    """publish -> barrier -> routing tables (rows of every expert padded to 128)."""
-    cfg = state.config
-    D, K, E = cfg.hidden_dim, cfg.top_k, cfg.num_experts
-    T, dev, el, ep = x.shape[0], x.device, state.e_local, state.ep
-    st, status = nat.stream_ptr(), state.status.data_ptr()
-    nat.check(nat.lib.dm_publish(x.data_ptr(), ids.data_ptr(), int(ids.dtype == torch.int64),
-                                 state.dispatch.local().data_ptr(), state.routing.local().data_ptr(), T, D, K, E,
-                                 int(options.validate_expert_ids), status, st), "dm_publish")
-    state.barrier(state.dispatch)
-    size = max((ep * T * min(K, el) + el * 127 + 127) // 128 * 128, 128)
-    c.T = T
-    c.R = min(size, state.capacity_rows // 128 * 128)
-    counts = torch.empty(el, dtype=torch.int32, device=dev)
-    c.per_rank = torch.empty(ep, dtype=torch.int32, device=dev)
-    c.offsets = torch.empty(el + 1, dtype=torch.int32, device=dev)
-    c.real = torch.empty(el, dtype=torch.int32, device=dev)  # rows per expert before the padding to 128
-    c.fwd = torch.empty(size, dtype=torch.int64, device=dev)
-    c.bwd = torch.empty(size, dtype=torch.int64, device=dev)
-    c.sct = torch.empty(size, dtype=torch.int64, device=dev)
-    stride = D * 2
-    nat.check(nat.lib.dm_route_counted(state.routing.peer_ptrs.data_ptr(), state.dispatch.peer_ptrs.data_ptr(),
-                                       state.combine.peer_ptrs.data_ptr(), state.rank, ep, T, K, E, stride, stride,
-                                       stride, 128, state.capacity_rows, size, counts.data_ptr(), c.real.data_ptr(),
-                                       c.per_rank.data_ptr(), c.offsets.data_ptr(), c.fwd.data_ptr(), c.bwd.data_ptr(),
-                                       c.sct.data_ptr(), state.route_workspace.data_ptr(), state.route_workspace_words,
-                                       status, st), nat.route_call_name(ep, T, el))
-    c.recv = c.offsets[el:]
-
-
-def _storage_array(state):
-    import ctypes
-
-    arr = getattr(state, "_planner_storage", None)
-    if arr is None:
-        arr = (ctypes.c_int * 6)(*planner_storage(state.config.block_scaled.format))
-        state._planner_storage = arr
-    return arr
+def _planned_arguments(state, c: _PlannedCall, x, ids, scores, options):
+    k = arguments(state, c, x, ids, scores, options)
+    k.real_counts, k.fwd_table = c.ptr("real"), c.ptr("fwd_table")
+    for name, p in (("w13", c.p13), ("w2", c.p2)):
+        setattr(k, name, p.fprop_data.data_ptr())
+        setattr(k, name + "_sf", p.fprop_scale.data_ptr())
+        setattr(k, name + "_dgrad_sf", p.dgrad_scale.data_ptr())
+    return k
 
 
 def _mxfp8_forward_planned(state, x, ids, scores, p13, p2, options, need_h3: bool, hooks=None):
-    cfg = state.config
-    D, F, K = cfg.hidden_dim, cfg.intermediate_dim, cfg.top_k
-    T, dev, el, ep = x.shape[0], x.device, state.e_local, state.ep
-    st, status = nat.stream_ptr(), state.status.data_ptr()
-    clamped = 1 if cfg.activation == "swiglu_clamped" else 0
-    alpha, limit = float(cfg.swiglu_alpha), float(cfg.swiglu_limit)
-    c = _TrainCall()
-    c.planned, c.p13, c.p2 = True, p13, p2
-    c.h1 = c.x_col = c.x_col_sf = c.h2_col = c.h2_col_sf = c.h3 = c.callback_state = None
-    _route_training(state, x, ids, options, c)
-    R, recv, real = c.R, c.recv.data_ptr(), c.real.data_ptr()
-    c.need = torch.empty(1, dtype=torch.uint8, device=dev)
-    c.cond = torch.empty(1, dtype=torch.int32, device=dev)
-    c.fwd_state = torch.empty(10, dtype=torch.int64, device=dev)  # [x, -, h1, -, h3, x_row, x_col, h2_row, h2_col, slot]
-    c.fwd_table = torch.empty(18, dtype=torch.int64, device=dev)
-    nat.check(nat.lib.dm_plan_fwd_blockscaled(
-        recv, c.per_rank.data_ptr(), None, state.saved_bytes.data_ptr(), state.buffer_offsets.data_ptr(),
-        state.peak_min_free.data_ptr(), c.need.data_ptr(), c.cond.data_ptr(), c.fwd_state.data_ptr(),
-        c.fwd_table.data_ptr(), state.slot_selector.data_ptr(), state.moe_layer_id.data_ptr(), ep,
-        cfg.max_num_local_input_tokens, K, D, F, _storage_array(state), state.capacity_rows, state.slot_bytes,
-        state.num_slots, state.num_layers_in_slot, 0, 0, 0, 0, 0, status, st), "dm_plan_fwd_blockscaled")
-    fs, ft = c.fwd_state.data_ptr(), c.fwd_table.data_ptr()
-    A = lambda table, group, entry: state.arena_at(table + 8 * (group * 9 + entry))  # noqa: E731
-    none = nat.Operand(None, 0, None)
-    arena = state.arena.data_ptr()
-    # a layer that will be recomputed keeps only its dense input
-    nat.check(nat.lib.dm_cond_copy(x.data_ptr(), None, arena, fs, T * D * 2, c.cond.data_ptr(), 1, st),
-              "dm_cond_copy(save x)")
-    # dispatch: the routed rows are pulled through the pointer table by the quantiser itself
-    nat.check(nat.lib.dm_quant_mxfp8_rowcol_gather_at(c.fwd.data_ptr(), recv, R, D, A(ft, 0, _A_Q), A(ft, 0, _A_SF),
-                                                      A(ft, 0, _COL_Q), A(ft, 0, _COL_SF), None, st),
-              "dm_quant_mxfp8_rowcol_gather_at(x)")
-    nat.check(_gemm(0, A(ft, 0, _A_Q), A(ft, 0, _A_SF), p13.fprop_data.data_ptr(), p13.fprop_scale.data_ptr(),
-                    A(ft, 0, _C), none, None, none, None, c.offsets.data_ptr(), real, el, R, 2 * F, D, 0, 0, 1.0, 0.0,
-                    None, state.num_sms, status, st), "dm_gemm_blockscaled(w13)")
-    nat.check(nat.lib.dm_swiglu_fwd_quant_mxfp8_rowcol_at(A(ft, 1, _SRC_X), recv, R, F, clamped, alpha, limit,
-                                                          A(ft, 1, _A_Q), A(ft, 1, _A_SF), A(ft, 1, _COL_Q),
-                                                          A(ft, 1, _COL_SF), None, st),
-              "dm_swiglu_fwd_quant_mxfp8_rowcol_at")
-    nat.check(_gemm(0, A(ft, 1, _A_Q), A(ft, 1, _A_SF), p2.fprop_data.data_ptr(), p2.fprop_scale.data_ptr(), none, none,
-                    c.sct.data_ptr(), none, None, c.offsets.data_ptr(), real, el, R, D, F, 0, 0, 1.0, 0.0, None,
-                    state.num_sms, status, st), "dm_gemm_blockscaled(w2)")
-    state.barrier(state.combine)
+    T, D, dev = x.shape[0], state.config.hidden_dim, x.device
+    c = _PlannedCall(state, T, p13, p2).allocate(dev)
     out = torch.empty(T, D, dtype=torch.bfloat16, device=dev)
+    k = _planned_arguments(state, c, x, ids, scores, options)
+    k.out, k.keep_h3 = out.data_ptr(), need_h3
     post = options.experts_output_postprocess
-    is_norm = isinstance(post, RMSNormPostprocess)
-    c.rstd = None
-    if is_norm:
+    launch(nat.lib.dm_mxfp8_forward, FWD, state, k, FWD_ALL if post is None else FWD_ALL - FWD["reduce"])
+    if isinstance(post, RMSNormPostprocess):
         from ._postprocess import rmsnorm_combine_forward
 
         c.rstd = rmsnorm_combine_forward(state, c, post, scores, ids, out, save=True)
@@ -611,137 +553,87 @@ def _mxfp8_forward_planned(state, x, ids, scores, p13, p2, options, need_h3: boo
         if hooks is None:
             raise RuntimeError("a callable expert-output post-process runs on the eager path only")
         hooks.postprocess_forward(state, c, post, scores, ids, out, save=True)  # keeps its own input and output
-    else:
-        # the expert outputs go to the slot (when the layer is saved) only if the score gradient will read them
-        nat.check(nat.lib.dm_scale_and_sum(state.combine.local().data_ptr(), scores.data_ptr(),
-                                           int(scores.dtype == torch.bfloat16), ids.data_ptr(),
-                                           int(ids.dtype == torch.int64), out.data_ptr(), T, K, D,
-                                           arena if need_h3 else None, fs + 32 if need_h3 else None,
-                                           c.cond.data_ptr() if need_h3 else None, 0, st), "dm_scale_and_sum")
-    state.last_recv = c.recv
+    state.last_recv = c.recv_rows
     state.last_train_call = c
     return out, c
 
 
-def _mxfp8_backward_planned(state, c: _TrainCall, x_shape, ids, scores, w13_param, w2_param, grad_out, options, needs,
+def _mxfp8_backward_planned(state, c: _PlannedCall, x_shape, ids, scores, w13_param, w2_param, grad_out, options, needs,
                             wgrad_explicit=(None, None), hooks=None):
     from ._bf16 import _wgrad_destination
 
     cfg = state.config
     D, F, K = cfg.hidden_dim, cfg.intermediate_dim, cfg.top_k
-    T, R, el, ep, dev = c.T, c.R, state.e_local, state.ep, grad_out.device
-    st, status = nat.stream_ptr(), state.status.data_ptr()
-    clamped = 1 if cfg.activation == "swiglu_clamped" else 0
-    alpha, limit = float(cfg.swiglu_alpha), float(cfg.swiglu_limit)
+    T, el, dev = c.T, state.e_local, grad_out.device
     need_x, need_scores, need_w13, need_w2 = needs
-    recv, offs, real = c.recv.data_ptr(), c.offsets.data_ptr(), c.real.data_ptr()
-    none = nat.Operand(None, 0, None)
-    arena, combine = state.arena.data_ptr(), state.combine.local().data_ptr()
-    bo = torch.empty(16, dtype=torch.int64, device=dev)
-    bt = torch.empty(54, dtype=torch.int64, device=dev)
-    nat.check(nat.lib.dm_plan_bwd_blockscaled(
-        recv, c.per_rank.data_ptr(), state.saved_bytes.data_ptr(), state.buffer_offsets.data_ptr(),
-        state.peak_min_free.data_ptr(), c.need.data_ptr(), c.fwd_state.data_ptr(), bo.data_ptr(), bt.data_ptr(),
-        state.moe_layer_id.data_ptr(), ep, cfg.max_num_local_input_tokens, K, D, F, _storage_array(state),
-        state.capacity_rows, state.slot_bytes, state.num_slots, 0, 0, status, st), "dm_plan_bwd_blockscaled")
-    btp = bt.data_ptr()
-    A = lambda group, entry: state.arena_at(btp + 8 * (group * 9 + entry))  # noqa: E731
-    fs, cond = c.fwd_state.data_ptr(), c.cond
+    plan = torch.empty(16 + 54, dtype=torch.int64, device=dev)  # the plan's offsets and its table of operands
+    grad_scores = torch.empty(T, K, dtype=torch.float32, device=dev) if need_scores else None
     post = options.experts_output_postprocess
     is_norm = isinstance(post, RMSNormPostprocess)
     is_callback = post is not None and not is_norm  # the callable kept its own input and output (eager path)
-    # ---- recompute block: every launch is a no-op unless the forward chose to recompute this layer ------------
-    with record_function("dist_moe_recompute"):
-        nat.check(nat.lib.dm_cond_copy(arena, fs, state.dispatch.local().data_ptr(), None, T * D * 2,
-                                       cond.data_ptr(), 1, st), "dm_cond_copy(republish x)")
-        state.barrier(state.dispatch, cond)
-        nat.check(nat.lib.dm_quant_mxfp8_rowcol_gather_at(c.fwd.data_ptr(), recv, R, D, A(0, _A_Q), A(0, _A_SF),
-                                                          A(0, _COL_Q), A(0, _COL_SF), cond.data_ptr(), st),
-                  "dm_quant_mxfp8_rowcol_gather_at(x recompute)")
-        nat.check(_gemm(0, A(0, _A_Q), A(0, _A_SF), c.p13.fprop_data.data_ptr(), c.p13.fprop_scale.data_ptr(), A(0, _C),
-                        none, None, none, None, offs, real, el, R, 2 * F, D, 0, 0, 1.0, 0.0, cond.data_ptr(),
-                        state.num_sms, status, st), "dm_gemm_blockscaled(w13 recompute)")
-        nat.check(nat.lib.dm_swiglu_fwd_quant_mxfp8_rowcol_at(A(1, _SRC_X), recv, R, F, clamped, alpha, limit,
-                                                              A(1, _A_Q), A(1, _A_SF), A(1, _COL_Q), A(1, _COL_SF),
-                                                              cond.data_ptr(), st),
-                  "dm_swiglu_fwd_quant_mxfp8_rowcol_at(recompute)")
-        if (need_scores or is_norm) and not is_callback:
-            # the expert outputs again, scattered to their owners' combine buffers
-            nat.check(_gemm(0, A(1, _A_Q), A(1, _A_SF), c.p2.fprop_data.data_ptr(), c.p2.fprop_scale.data_ptr(), none,
-                            none, c.sct.data_ptr(), none, None, offs, real, el, R, D, F, 0, 0, 1.0, 0.0,
-                            cond.data_ptr(), state.num_sms, status, st), "dm_gemm_blockscaled(w2 recompute)")
-            if is_norm:  # the fused RMSNorm backward works on the expert outputs in place in the combine buffer
-                nat.check(nat.lib.dm_cond_copy(arena, fs + 32, combine, None, T * K * D * 2,
-                                               cond.data_ptr(), 0, st), "dm_cond_copy(load h3)")
-            state.barrier(state.combine, cond)
-    # ---- gradient with respect to the expert outputs and the scores ------------------------------------------
-    grad_scores = torch.empty(T, K, dtype=torch.float32, device=dev) if need_scores else None
-    if is_norm:
-        from ._postprocess import rmsnorm_combine_backward
+    k = _planned_arguments(state, c, None, ids, scores, options)
+    k.bwd_offsets, k.bwd_table = plan.data_ptr(), plan.data_ptr() + 128
+    k.grad_out, k.grad_scores = grad_out.data_ptr(), nat.ptr(grad_scores)
+    k.want_x, k.want_w13, k.want_w2 = need_x, need_w13, need_w2
 
-        rmsnorm_combine_backward(state, c, post, grad_out, scores, ids, grad_scores)
-    elif is_callback:
-        hooks.postprocess_backward(state, c, grad_out, scores, ids, grad_scores)
-    elif need_scores:
-        nat.check(nat.lib.dm_broadcast_and_scale_select(grad_out.data_ptr(), scores.data_ptr(),
-                                                        int(scores.dtype == torch.bfloat16), ids.data_ptr(),
-                                                        int(ids.dtype == torch.int64), arena, fs + 32,
-                                                        combine, cond.data_ptr(), combine, nat.ptr(grad_scores), T, K,
-                                                        D, st), "dm_broadcast_and_scale")
+    def run(steps: int) -> None:
+        launch(nat.lib.dm_mxfp8_backward, BWD, state, k, steps)
+
+    # recompute block: every launch is a no-op unless the forward chose to recompute this layer
+    recompute = BWD["plan"] | BWD["republish"] | BWD["w13_again"] | BWD["swiglu_again"]
+    if (need_scores or is_norm) and not is_callback:
+        # the fused RMSNorm backward works on the expert outputs in place in the combine buffer
+        recompute |= BWD["w2_again"] | (BWD["load_h3"] if is_norm else 0)
+    steps = BWD["combine"] | BWD["w2_dgrad"]
+    if post is None and not observed():
+        steps |= recompute | BWD["grad_h3"]
     else:
-        nat.check(nat.lib.dm_broadcast_and_scale(grad_out.data_ptr(), scores.data_ptr(),
-                                                 int(scores.dtype == torch.bfloat16), ids.data_ptr(),
-                                                 int(ids.dtype == torch.int64), None, None, combine, None, T, K, D, st),
-                  "dm_broadcast_and_scale")
-    state.barrier(state.combine)
-    # ---- W2 ----------------------------------------------------------------------------------------------------
-    nat.check(nat.lib.dm_quant_mxfp8_rowcol_gather_at(c.sct.data_ptr(), recv, R, D, A(2, _A_Q), A(2, _A_SF),
-                                                      A(2, _COL_Q) if need_w2 else none,
-                                                      A(2, _COL_SF) if need_w2 else none, None, st),
-              "dm_quant_mxfp8_rowcol_gather_at(grad_h3)")
-    nat.check(_gemm_dgrad(A(2, _A_Q), A(2, _A_SF), c.p2.fprop_data.data_ptr(), c.p2.dgrad_scale.data_ptr(), A(2, _C),
-                          None, offs, real, el, R, F, D, None, state.num_sms, status, st),
-              "dm_gemm_blockscaled_dgrad(w2)")
-    grad_w13 = grad_w2 = None
+        with span("dist_moe_recompute"):
+            run(recompute)
+        if is_norm:
+            from ._postprocess import rmsnorm_combine_backward
+
+            rmsnorm_combine_backward(state, c, post, grad_out, scores, ids, grad_scores)
+        elif is_callback:
+            hooks.postprocess_backward(state, c, grad_out, scores, ids, grad_scores)
+        else:
+            steps |= BWD["grad_h3"]
+    run(steps)
+    # ---- W2 weight gradient; SwiGLU backward, W13 ------------------------------------------------------------------
+    grad_w13 = grad_w2 = grad_x = None
     owners = options.wgrad_parameter_owners or (None, None)
+    steps = 0
     if need_w2:
-        dst, acc, ret = _wgrad_destination(w2_param, (el, D, F), options, cfg, owners[1], wgrad_explicit[1], hooks, "w2")
-        nat.check(nat.lib.dm_gemm_blockscaled_wgrad_compact(A(3, _A_Q), A(3, _A_SF), A(3, _B_Q), A(3, _B_SF),
-                                                            dst.data_ptr(), int(dst.dtype == torch.float32), acc, offs,
-                                                            el, R, D, F, None, state.num_sms, status, st),
-                  "dm_gemm_blockscaled_wgrad(w2)")
+        dst, k.dw2_accumulate, ret = _wgrad_destination(w2_param, (el, D, F), options, cfg, owners[1], wgrad_explicit[1],
+                                                        hooks, "w2")
+        k.dw2, k.dw2_is_fp32 = dst.data_ptr(), dst.dtype is torch.float32
         grad_w2 = dst.view(w2_param.shape) if ret else None
+        steps = BWD["w2_wgrad"]
         if hooks is not None:
-            grad_w2 = hooks.wgrad_postprocess("w2", grad_w2)
-    # ---- SwiGLU backward, W13 ---------------------------------------------------------------------------------
+            run(steps)
+            grad_w2, steps = hooks.wgrad_postprocess("w2", grad_w2), 0
     if need_x or need_w13:
-        nat.check(nat.lib.dm_swiglu_bwd_quant_mxfp8_at(A(4, _SRC_Y), A(4, _SRC_X), recv, R, F, clamped, alpha, limit,
-                                                       A(4, _A_Q) if need_x else none, A(4, _A_SF) if need_x else none,
-                                                       A(4, _COL_Q) if need_w13 else none,
-                                                       A(4, _COL_SF) if need_w13 else none, st),
-                  "dm_swiglu_bwd_quant_mxfp8_at")
+        steps |= BWD["swiglu"]
     if need_x:
-        nat.check(_gemm_dgrad(A(4, _A_Q), A(4, _A_SF), c.p13.fprop_data.data_ptr(), c.p13.dgrad_scale.data_ptr(), none,
-                              c.bwd.data_ptr(), offs, real, el, R, D, 2 * F, None, state.num_sms, status, st),
-                  "dm_gemm_blockscaled_dgrad(w13)")
+        steps |= BWD["w13_dgrad"]
     if need_w13:
-        dst, acc, ret = _wgrad_destination(w13_param, (el, 2 * F, D), options, cfg, owners[0], wgrad_explicit[0], hooks,
-                                           "w13")
-        nat.check(nat.lib.dm_gemm_blockscaled_wgrad_compact(A(5, _A_Q), A(5, _A_SF), A(5, _B_Q), A(5, _B_SF),
-                                                            dst.data_ptr(), int(dst.dtype == torch.float32), acc, offs,
-                                                            el, R, 2 * F, D, None, state.num_sms, status, st),
-                  "dm_gemm_blockscaled_wgrad(w13)")
+        if hooks is not None:  # named destinations are asked for when the gradient is next
+            run(steps)
+            steps = 0
+        dst, k.dw13_accumulate, ret = _wgrad_destination(w13_param, (el, 2 * F, D), options, cfg, owners[0],
+                                                         wgrad_explicit[0], hooks, "w13")
+        k.dw13, k.dw13_is_fp32 = dst.data_ptr(), dst.dtype is torch.float32
         grad_w13 = dst.view(w13_param.shape) if ret else None
+        steps |= BWD["w13_wgrad"]
         if hooks is not None:
-            grad_w13 = hooks.wgrad_postprocess("w13", grad_w13)
-    grad_x = None
-    # unconditional, as in the reference (dist_moe/api.py:2580): peers may still be reading this rank's combine buffer
-    state.barrier(state.dispatch)
+            run(steps)
+            grad_w13, steps = hooks.wgrad_postprocess("w13", grad_w13), 0
+    steps |= BWD["close"]
     if need_x:
         grad_x = torch.empty(x_shape, dtype=torch.bfloat16, device=dev)
-        nat.check(nat.lib.dm_scale_and_sum(state.dispatch.local().data_ptr(), None, 0, ids.data_ptr(),
-                                           int(ids.dtype == torch.int64), grad_x.data_ptr(), T, K, D, None, None, None,
-                                           0, st), "dm_scale_and_sum(reduce_from_topk)")
+        k.grad_x = grad_x.data_ptr()
+        steps |= BWD["reduce"]
+    run(steps)
     if grad_scores is not None and scores.dtype != torch.float32:
         grad_scores = grad_scores.to(scores.dtype)
     return grad_x, grad_scores, grad_w13, grad_w2
@@ -924,7 +816,7 @@ class _Mxfp8Function(torch.autograd.Function):
     def forward(ctx, x, ids, scores, w13_param, w2_param, state, options, p13, p2):
         p13, p2 = _training_weights(w13_param, w2_param, p13, p2, state.config)
         planned = PLANNED_ARENA and state.num_slots > 0 and options.swiglu_clip_stats_out_3 is None
-        with record_function("dist_moe_forward"):
+        with span("dist_moe_forward"):
             forward = _mxfp8_forward_planned if planned else _mxfp8_forward
             out, call = forward(state, x.detach().contiguous(), ids, scores.detach(), p13, p2, options,
                                 need_h3=scores.requires_grad)
@@ -936,7 +828,7 @@ class _Mxfp8Function(torch.autograd.Function):
     def backward(ctx, grad_out):
         ids, scores, w13_param, w2_param = ctx.saved_tensors
         needs = (ctx.needs_input_grad[0], ctx.needs_input_grad[2], ctx.needs_input_grad[3], ctx.needs_input_grad[4])
-        with torch.cuda.device(ctx.state.device), record_function("dist_moe_backward"):
+        with torch.cuda.device(ctx.state.device), span("dist_moe_backward"):
             backward = _mxfp8_backward_planned if ctx.call.planned else _mxfp8_backward
             gx, gs, gw13, gw2 = backward(ctx.state, ctx.call, ctx.x_shape, ids, scores.detach(), w13_param, w2_param,
                                          grad_out.contiguous(), ctx.options, needs)
@@ -964,7 +856,7 @@ class _EagerMxfp8Function(torch.autograd.Function):
                              "with weights_preprocess_fn")
         hooks = CallbackHooks(options)
         _, _, p13, p2 = _EagerMxfp8Function._weights(options, w13_source, w2_source, state)
-        with record_function("dist_moe_forward"):
+        with span("dist_moe_forward"):
             out, call = _mxfp8_forward_planned(state, x.detach().contiguous(), ids, scores.detach(), p13, p2, options,
                                                need_h3=scores.requires_grad, hooks=hooks)
         call.p13 = call.p2 = None  # re-materialised before the backward, as the reference does
@@ -980,7 +872,7 @@ class _EagerMxfp8Function(torch.autograd.Function):
         # handed back in the sources' shapes
         w13, w2, call.p13, call.p2 = _EagerMxfp8Function._weights(options, w13_source, w2_source, state)
         needs = (ctx.needs_input_grad[0], ctx.needs_input_grad[2], ctx.needs_input_grad[3], ctx.needs_input_grad[4])
-        with torch.cuda.device(state.device), record_function("dist_moe_backward"):
+        with torch.cuda.device(state.device), span("dist_moe_backward"):
             gx, gs, g13, g2 = _mxfp8_backward_planned(state, call, ctx.x_shape, ids, scores.detach(), w13, w2,
                                                       grad_out.contiguous(), options, needs, hooks=ctx.hooks)
         if g13 is not None:

@@ -1,0 +1,148 @@
+"""What the BF16 and the MXFP8 training passes share on the host: the device results of a call, the argument structure of the
+native launch sequences, and running their steps.
+
+A pass is one or two native calls (``dm_bf16_forward`` and the like, csrc/sequence.cu); only observed passes (a profiler's
+ranges, GEMMs timed in place) and passes with Python callbacks between launches take more.  A foreign-function call per
+launch, a tensor per result and the dispatcher around the registered operators made small layers wait for the host: forward and
+backward of 16 tokens (D = F = 256, 8 experts) 656 -> 301 us, of 1531 tokens (D = 1088, F = 704, 24 experts, recomputed) 674 ->
+330 us, MXFP8 of 777 tokens with tensor weights 580 -> 397 us.
+"""
+
+from __future__ import annotations
+
+import ctypes
+
+import torch
+from torch.profiler import record_function
+
+from . import _native as nat
+
+# Steps of the forward and backward sequences (include/dist_moe_b200.h), in launch order.
+FWD = {name: 1 << i for i, name in enumerate(
+    ("publish", "route", "save_x", "w13", "swiglu", "w2", "combine", "reduce"))}
+BWD = {name: 1 << i for i, name in enumerate(
+    ("plan", "republish", "w13_again", "swiglu_again", "w2_again", "load_h3", "grad_h3", "combine", "w2_dgrad", "w2_wgrad",
+     "swiglu", "w13_dgrad", "w13_wgrad", "close", "reduce"))}
+FWD_ALL = 255
+_GEMM_NAMES = {
+    "dm_bf16_forward": {"w13": "gemm_fprop_dispatch(w13)", "w2": "gemm_fprop(w2)"},
+    "dm_bf16_backward": {
+        "w13_again": "gemm_fprop_dispatch(w13 recompute)", "w2_again": "gemm_fprop(w2 recompute)",
+        "w2_dgrad": "gemm_dgrad_dispatch(w2)", "w2_wgrad": "gemm_wgrad(w2)", "w13_dgrad": "gemm_dgrad(w13)",
+        "w13_wgrad": "gemm_wgrad(w13)"},
+}
+_REPORT = ctypes.c_int32 * 2
+
+
+def observed() -> bool:
+    """Someone wants to see the parts of a pass."""
+    from . import _bf16
+
+    return _bf16.PROFILE is not None or torch.autograd._profiler_enabled()
+
+
+class _NoSpan:
+    def __enter__(self):
+        return self
+
+    def __exit__(self, *exc):
+        return False
+
+
+def span(name: str):
+    """A profiler range with the reference's name (dist_moe/api.py:1979-2443), free where nothing records."""
+    return record_function(name) if torch.autograd._profiler_enabled() else _NoSpan()
+
+
+def launch(fn, names: dict, state, k, steps: int) -> None:
+    """Run the given steps of a sequence: one call, or one per step where the GEMMs are timed in place."""
+    from . import _bf16
+
+    context, st = state.native_layer(), nat.stream_ptr()
+
+    def run(bits: int) -> None:
+        report = _REPORT()
+        rc = fn(context, ctypes.byref(k), bits, report, st)
+        nat.LAUNCHES[0] += report[0]
+        if rc != 0:
+            failed = next((n for n, bit in names.items() if bit == report[1]), "arguments")
+            nat.check(rc, f"{fn.__name__}({failed})")
+
+    gemms = _GEMM_NAMES.get(fn.__name__)
+    if _bf16.PROFILE is None or gemms is None:
+        run(steps)
+        return
+    for name, bit in names.items():
+        if not steps & bit:
+            continue
+        if name not in gemms:
+            run(bit)
+            continue
+        start, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        start.record()
+        run(bit)
+        end.record()
+        _bf16.PROFILE.append((gemms[name], start, end))
+
+
+class CallState:
+    """Device results of routing and planning of one call: one buffer (``buf``) that the names of ``fields`` are views of, or
+    tensors of their own where a registered operator hands them out.  ``fields``: name -> (dtype, elements)."""
+
+    def __init__(self, fields: dict):
+        self.fields, self.buf, self.at = fields, None, {}
+        self.rstd = self.callback_state = None
+
+    def _place(self) -> int:
+        off = 0
+        for name, (dtype, n) in self.fields.items():
+            self.at[name] = off
+            off += (n * dtype.itemsize + 15) & ~15
+        return off
+
+    def allocate(self, device, separate: bool = False) -> "CallState":
+        if separate:
+            for name, (dtype, n) in self.fields.items():
+                setattr(self, name, torch.empty(n, dtype=dtype, device=device) if n else None)
+        else:
+            self.buf = torch.empty(self._place() // 8, dtype=torch.int64, device=device)
+        return self
+
+    def adopt(self, buf: torch.Tensor) -> "CallState":
+        """The results that an earlier call has left in ``buf``."""
+        self._place()
+        self.buf = buf
+        return self
+
+    def ptr(self, name: str) -> int | None:
+        if self.buf is None:
+            return nat.ptr(getattr(self, name))
+        return self.buf.data_ptr() + self.at[name] if self.fields[name][1] else None
+
+    def __getattr__(self, name: str):  # views of the buffer, made when asked for
+        if name == "recv_rows":
+            return self.offsets[self.offsets.numel() - 1:]
+        fields = self.__dict__.get("fields", {})
+        if name not in fields or self.__dict__.get("buf") is None:
+            raise AttributeError(name)
+        dtype, n = fields[name]
+        at = self.at[name]
+        view = self.buf.view(torch.uint8)[at:at + n * dtype.itemsize].view(dtype) if n else None
+        setattr(self, name, view)
+        return view
+
+
+def arguments(state, c: CallState, x, ids, scores, options) -> "nat.LayerCall":
+    """What the passes of a call have in common."""
+    k = nat.LayerCall()
+    if x is not None:
+        k.x = x.data_ptr()
+    k.ids, k.ids_are_int64 = ids.data_ptr(), ids.dtype is torch.int64
+    k.scores, k.scores_are_bf16 = scores.data_ptr(), scores.dtype is torch.bfloat16
+    ptr = c.ptr
+    k.counts, k.per_rank, k.expert_offsets = ptr("counts"), ptr("per_rank"), ptr("offsets")
+    k.fwd_ptrs, k.bwd_ptrs, k.sct_ptrs = ptr("fwd"), ptr("bwd"), ptr("sct")
+    k.need, k.cond, k.fwd_state = ptr("need"), ptr("cond"), ptr("fwd_state")
+    k.T, k.ptrs_size, k.max_rows = c.T, c.size, c.max_rows
+    k.num_layers, k.validate_ids = state.num_layers_in_slot, options.validate_expert_ids
+    return k

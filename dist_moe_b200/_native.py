@@ -31,6 +31,38 @@ class Operand(ctypes.Structure):
     _fields_ = [("base", c_void_p), ("bytes", c_int64), ("offset", c_void_p)]
 
 
+class LayerContext(ctypes.Structure):
+    """``dm_layer_context``: what a context keeps between calls."""
+
+    _fields_ = (
+        [("arena", c_void_p), ("arena_bytes", c_int64)]
+        + [(n, c_void_p) for n in ("dispatch", "combine", "routing", "dispatch_ptrs", "combine_ptrs", "routing_ptrs",
+                                   "dispatch_pads", "combine_pads", "saved_bytes", "buffer_offsets", "peak_min_free",
+                                   "slot_selector", "moe_layer_id", "route_workspace")]
+        + [("route_workspace_words", c_int64), ("gather_flags", c_void_p), ("status", c_void_p)]
+        + [(n, c_int64) for n in ("T_max", "D", "F", "slot_bytes", "capacity_rows")]
+        + [("barrier_timeout_ns", c_uint64)]
+        + [(n, c_int) for n in ("rank", "ep", "K", "E", "e_local", "num_slots", "num_sms", "clamped")]
+        + [("alpha", c_float), ("limit", c_float), ("storage", c_int * 6)]
+    )
+
+
+class LayerCall(ctypes.Structure):
+    """``dm_layer_call``: the tensors and options of one pass."""
+
+    _fields_ = (
+        [(n, c_void_p) for n in ("x", "ids", "scores", "w13", "w2", "w13_sf", "w13_dgrad_sf", "w2_sf", "w2_dgrad_sf", "out",
+                                 "counts", "real_counts", "per_rank", "expert_offsets", "fwd_ptrs", "bwd_ptrs", "sct_ptrs",
+                                 "need", "cond", "fwd_state", "fwd_table", "bwd_offsets", "bwd_table", "grad_out",
+                                 "grad_scores", "grad_x", "dw13", "dw2", "clip_stats")]
+        + [("clip_limit", c_float)]
+        + [(n, c_int64) for n in ("T", "ptrs_size", "max_rows")]
+        + [(n, c_int) for n in ("ids_are_int64", "scores_are_bf16", "scratch_only", "num_layers", "validate_ids",
+                                "fuse_swiglu", "separate_gather", "h3_in_combine", "dw13_is_fp32", "dw13_accumulate",
+                                "dw2_is_fp32", "dw2_accumulate", "keep_h3", "want_x", "want_w13", "want_w2")]
+    )
+
+
 class NativeError(RuntimeError):
     pass
 
@@ -187,6 +219,10 @@ _SIGNATURES = {
     ),
     "dm_gemm_dgrad_dispatch": (c_int, [_P, _P, Operand, _P, Operand, _P, c_int, c_int64, c_int64, c_int64, _P, c_int, _P, _P]),
     "dm_gemm_dgrad": (c_int, [Operand, _P, Operand, _P, _P, c_int, c_int64, c_int64, c_int64, _P, c_int, _P, _P]),
+    "dm_bf16_forward": (c_int, [_P, _P, ctypes.c_uint32, _P, _P]),
+    "dm_bf16_backward": (c_int, [_P, _P, ctypes.c_uint32, _P, _P]),
+    "dm_mxfp8_forward": (c_int, [_P, _P, ctypes.c_uint32, _P, _P]),
+    "dm_mxfp8_backward": (c_int, [_P, _P, ctypes.c_uint32, _P, _P]),
     "dm_gemm_wgrad": (c_int, [Operand, Operand, _P, c_int, c_int, _P, c_int, c_int64, c_int64, c_int64, c_int, _P, _P]),
 }
 

@@ -91,7 +91,8 @@ def _unpack_bf16_state(state, tensors, T: int):
     c.offsets[1:] = torch.cumsum(c.counts, 0)
     c.recv_rows = recv
     c.cond = c.need.to(torch.int32)
-    c.max_rows = min(c.fwd.numel(), state.capacity_rows)
+    c.size = c.fwd.numel()
+    c.max_rows = min(c.size, state.capacity_rows)
     c.rstd = rstd if rstd.numel() else None
     return c
 
@@ -106,7 +107,7 @@ def _bf16_forward_common(x, ids, scores, w13, w2, post, slot_id, num_layers, val
                                swiglu_clip_stats_out_3=clip, swiglu_clip_limit=clip_limit)
     w13 = w13.reshape(state.e_local, 2 * cfg.intermediate_dim, cfg.hidden_dim)
     w2 = w2.reshape(state.e_local, cfg.hidden_dim, cfg.intermediate_dim)
-    out, call = forward_impl(state, x.contiguous(), ids, scores, w13, w2, options, True)
+    out, call = forward_impl(state, x.contiguous(), ids, scores, w13, w2, options, True, separate=True)
     return out, _pack_bf16_state(call, x.device)
 
 

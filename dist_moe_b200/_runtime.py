@@ -14,6 +14,7 @@ rendezvous; all traffic is issued by this library's own kernels.
 
 from __future__ import annotations
 
+import ctypes
 import dataclasses
 import os
 from typing import Any
@@ -225,6 +226,7 @@ class ContextState:
 
     def close(self) -> None:
         torch.cuda.synchronize(self.device)
+        self._native_layer = None
         self._bs_workspace = None  # a view of the arena's scratch region (block-scaled forward-only calls)
         if getattr(self, "vmm_arena", None) is not None:
             self.arena = None
@@ -238,6 +240,34 @@ class ContextState:
             return
         nat.check(nat.lib.dm_barrier(buf.peer_pads.data_ptr(), self.rank, self.ep, 0, nat.ptr(cond),
                                      BARRIER_TIMEOUT_NS, self.status.data_ptr(), nat.stream_ptr()), "dm_barrier")
+
+    # ---- what the native call sequences read ----------------------------------
+    def native_layer(self):
+        """Reference to this context's ``dm_layer_context`` (everything it names lives as long as the context)."""
+        ref = getattr(self, "_native_layer", None)
+        if ref is None:
+            cfg, c = self.config, nat.LayerContext()
+            c.arena, c.arena_bytes = self.arena.data_ptr(), self.arena.numel()
+            for name in ("dispatch", "combine", "routing"):
+                buf = getattr(self, name)
+                setattr(c, name, buf.local().data_ptr())
+                setattr(c, name + "_ptrs", buf.peer_ptrs.data_ptr())
+            c.dispatch_pads, c.combine_pads = self.dispatch.peer_pads.data_ptr(), self.combine.peer_pads.data_ptr()
+            for name in ("saved_bytes", "buffer_offsets", "peak_min_free", "slot_selector", "moe_layer_id", "route_workspace",
+                         "gather_flags", "status"):
+                setattr(c, name, getattr(self, name).data_ptr())
+            c.route_workspace_words = self.route_workspace_words
+            c.T_max, c.D, c.F = cfg.max_num_local_input_tokens, cfg.hidden_dim, cfg.intermediate_dim
+            c.slot_bytes, c.capacity_rows, c.barrier_timeout_ns = self.slot_bytes, self.capacity_rows, BARRIER_TIMEOUT_NS
+            c.rank, c.ep, c.K, c.E, c.e_local = self.rank, self.ep, cfg.top_k, cfg.num_experts, self.e_local
+            c.num_slots, c.num_sms = self.num_slots, self.num_sms
+            c.clamped, c.alpha, c.limit = cfg.activation == "swiglu_clamped", cfg.swiglu_alpha, cfg.swiglu_limit
+            if cfg.block_scaled is not None:
+                from ._blockscaled import planner_storage
+
+                c.storage[:] = planner_storage(cfg.block_scaled.format)
+            ref = self._native_layer = ctypes.byref(c)
+        return ref
 
     def arena_at(self, offset_address: int) -> nat.Operand:
         """Operand whose byte offset inside the arena is the device int64 at ``offset_address``."""

@@ -531,6 +531,107 @@ int dm_vmm_create(int device, int num_sections, const int64_t* section_bytes, co
                   uint64_t* base_out, void** region_out);
 int dm_vmm_destroy(void* region);
 
+/* ---------------------------------------------------------------------------
+ * One pass as a sequence of the calls above (the reference's orchestration: BF16 dist_moe/api.py:1844-2188 and 2205-2609,
+ * MXFP8 training on the planner's placement dist_moe/_blockscaled.py:1309-1931 and 1951-2541), for hosts whose own call overhead exceeds the launches'.  `steps` selects launches; running a pass in
+ * several calls with disjoint steps, in the order of the bits, is the same as one call with all of them.  report[0]
+ * receives the launches made, report[1] the step that failed (0: none).  Barriers go with the step before them and are
+ * skipped where ep == 1.  Device pointers throughout, except report.
+ * ------------------------------------------------------------------------- */
+typedef struct { /* what a context keeps between calls */
+  void* arena;
+  int64_t arena_bytes;
+  void* dispatch; /* local symmetric buffers and the tables of all ranks' */
+  void* combine;
+  void* routing;
+  const uint64_t* dispatch_ptrs;
+  const uint64_t* combine_ptrs;
+  const uint64_t* routing_ptrs;
+  const uint64_t* dispatch_pads;
+  const uint64_t* combine_pads;
+  int64_t* saved_bytes; /* planner state */
+  int64_t* buffer_offsets;
+  int64_t* peak_min_free;
+  int64_t* slot_selector;
+  int64_t* moe_layer_id;
+  int32_t* route_workspace;
+  int64_t route_workspace_words;
+  int32_t* gather_flags;
+  int* status;
+  int64_t T_max, D, F, slot_bytes, capacity_rows;
+  uint64_t barrier_timeout_ns;
+  int rank, ep, K, E, e_local, num_slots, num_sms, clamped;
+  float alpha, limit;
+  int storage[6]; /* MXFP8: bundle geometry, as dm_plan_fwd_blockscaled takes it */
+} dm_layer_context;
+
+typedef struct {
+  const void* x; /* [T, D]; ids and scores [T, K] */
+  const void* ids;
+  const void* scores;
+  const void* w13; /* bf16, or E4M3 with forward and input-gradient scales */
+  const void* w2;
+  const void* w13_sf;
+  const void* w13_dgrad_sf;
+  const void* w2_sf;
+  const void* w2_dgrad_sf;
+  void* out;
+  int32_t* counts; /* routing tables and planner results of this call */
+  int32_t* real_counts; /* MXFP8: rows per expert before the padding to 128 */
+  int32_t* per_rank;
+  int32_t* expert_offsets;
+  int64_t* fwd_ptrs;
+  int64_t* bwd_ptrs; /* NULL where there is no backward */
+  int64_t* sct_ptrs;
+  uint8_t* need;
+  int32_t* cond;
+  int64_t* fwd_state;   /* int64[6], MXFP8 int64[10] */
+  int64_t* fwd_table;   /* MXFP8: int64[18] */
+  int64_t* bwd_offsets; /* int64[6], MXFP8 int64[16] */
+  int64_t* bwd_table;   /* MXFP8: int64[54] */
+  const void* grad_out;
+  float* grad_scores; /* NULL: not wanted */
+  void* grad_x;
+  void* dw13;
+  void* dw2;
+  float* clip_stats; /* unfused SwiGLU only */
+  float clip_limit;
+  int64_t T, ptrs_size, max_rows;
+  int ids_are_int64, scores_are_bf16, scratch_only, num_layers, validate_ids, fuse_swiglu, separate_gather, h3_in_combine;
+  int dw13_is_fp32, dw13_accumulate, dw2_is_fp32, dw2_accumulate;
+  int keep_h3, want_x, want_w13, want_w2; /* MXFP8 */
+} dm_layer_call;
+
+enum {
+  DM_FWD_PUBLISH = 1,
+  DM_FWD_ROUTE = 2, /* tables and plan */
+  DM_FWD_SAVE_X = 4,
+  DM_FWD_W13 = 8,
+  DM_FWD_SWIGLU = 16,
+  DM_FWD_W2 = 32,
+  DM_FWD_COMBINE = 64,
+  DM_FWD_REDUCE = 128,
+  DM_BWD_PLAN = 1,
+  DM_BWD_REPUBLISH = 2, /* to LOAD_H3: the recompute block, predicated on the plan */
+  DM_BWD_W13_AGAIN = 4,
+  DM_BWD_SWIGLU_AGAIN = 8,
+  DM_BWD_W2_AGAIN = 16,
+  DM_BWD_LOAD_H3 = 32, /* saved expert outputs back into the combine buffer */
+  DM_BWD_GRAD_H3 = 64,
+  DM_BWD_COMBINE = 128,
+  DM_BWD_W2_DGRAD = 256,
+  DM_BWD_W2_WGRAD = 512,
+  DM_BWD_SWIGLU = 1024,
+  DM_BWD_W13_DGRAD = 2048,
+  DM_BWD_W13_WGRAD = 4096,
+  DM_BWD_CLOSE = 8192,
+  DM_BWD_REDUCE = 16384
+};
+int dm_bf16_forward(const dm_layer_context* context, const dm_layer_call* call, uint32_t steps, int32_t* report, void* stream);
+int dm_bf16_backward(const dm_layer_context* context, const dm_layer_call* call, uint32_t steps, int32_t* report, void* stream);
+int dm_mxfp8_forward(const dm_layer_context* context, const dm_layer_call* call, uint32_t steps, int32_t* report, void* stream);
+int dm_mxfp8_backward(const dm_layer_context* context, const dm_layer_call* call, uint32_t steps, int32_t* report, void* stream);
+
 #ifdef __cplusplus
 }
 #endif
