@@ -364,6 +364,61 @@ __device__ __forceinline__ void tile_quantise(const uint4 (&w)[8], const TileLan
   __syncthreads();  // the staging bytes may be written again
 }
 
+// ---------------------------------------------------------------------------
+// 32x32 tile mode for weights whose sides are multiples of 128 (the general form is the slab kernel above): a CTA takes
+// 128 x 128, a warp 32 rows x 64 columns of it (two tiles), a lane 8 rows x 8 columns held in registers as loaded.  The tile
+// maximum is four shuffles, nothing of the matrix is staged.  The 4 x 4 scales of a CTA fill one 512-byte atom of either
+// orientation, 32 equal 16-byte rows each, which leave as whole lines (the slab form writes single bytes).
+// Bound: HBM.  Both weights of 16 experts x 1024 x 640 (63 MB) 95 us in slabs of 32 x 256, 21 us so.
+// ---------------------------------------------------------------------------
+__global__ void __launch_bounds__(256) mxfp8_tile32_kernel(const uint4* __restrict__ x, int64_t expert_rows, int C,
+                                                           uint8_t* __restrict__ q, uint8_t* __restrict__ s0,
+                                                           uint8_t* __restrict__ s1) {
+  __shared__ __align__(16) uint8_t sc[2][16];  // [row block][column block], and transposed
+  const TileLane me;
+  const int col_tiles = C >> 7;
+  const int64_t row_tile = blockIdx.x / col_tiles;
+  const int col_tile = static_cast<int>(blockIdx.x - row_tile * col_tiles);
+  const int64_t r0 = row_tile * kTileRows + me.row();
+  const int c = col_tile * kTileCols + me.col();
+  uint4 w[8];
+#pragma unroll
+  for (int r = 0; r < 8; ++r) w[r] = x[((r0 + r) * C + c) >> 3];
+  uint32_t m = 0;
+#pragma unroll
+  for (int r = 0; r < 8; ++r)
+    m = __vmaxu2(m, __vmaxu2(__vmaxu2(w[r].x & 0x7fff7fffu, w[r].y & 0x7fff7fffu), __vmaxu2(w[r].z & 0x7fff7fffu, w[r].w & 0x7fff7fffu)));
+  // the four column groups of a tile are neighbouring lanes, its four row groups eight lanes apart
+#pragma unroll
+  for (int d = 1; d <= 16; d <<= 1)
+    if (d != 4) m = __vmaxu2(m, __shfl_xor_sync(0xffffffffu, m, d));
+  float recip;
+  const uint32_t byte = mxfp8_scale_bits((m >> 16) > (m & 0xffffu) ? m >> 16 : m & 0xffffu, recip);
+  const int cb = me.half * 2 + (me.cg >> 2);
+  if ((me.lane & 0x1b) == 0) {  // one lane per tile
+    sc[0][me.slab * 4 + cb] = static_cast<uint8_t>(byte);
+    sc[1][cb * 4 + me.slab] = static_cast<uint8_t>(byte);
+  }
+#pragma unroll
+  for (int r = 0; r < 8; ++r) {
+    const uint4 v = w[r];
+    *reinterpret_cast<uint2*>(q + (r0 + r) * C + c) = make_uint2(
+        e4m3x2_scaled(__uint_as_float(v.x << 16), __uint_as_float(v.x & 0xffff0000u), recip, recip) |
+            (e4m3x2_scaled(__uint_as_float(v.y << 16), __uint_as_float(v.y & 0xffff0000u), recip, recip) << 16),
+        e4m3x2_scaled(__uint_as_float(v.z << 16), __uint_as_float(v.z & 0xffff0000u), recip, recip) |
+            (e4m3x2_scaled(__uint_as_float(v.w << 16), __uint_as_float(v.w & 0xffff0000u), recip, recip) << 16));
+  }
+  __syncthreads();
+  const int t = threadIdx.x;
+  if (t < 64) {
+    // atoms of either orientation: an expert's row blocks x column blocks, and the other way round
+    const int64_t row_blocks = expert_rows >> 7, e = row_tile / row_blocks, rb = row_tile - e * row_blocks;
+    const int64_t first = e * row_blocks * col_tiles;
+    const int64_t atom = t < 32 ? first + rb * col_tiles + col_tile : first + static_cast<int64_t>(col_tile) * row_blocks + rb;
+    reinterpret_cast<uint4*>((t < 32 ? s0 : s1) + atom * 512)[t & 31] = *reinterpret_cast<const uint4*>(sc[t >> 5]);
+  }
+}
+
 // Placement chosen on the device: each pointer is an allocation base and the byte offset is read from device memory
 // when the kernel starts (all null = the pointers are final).  `compact_cols` sizes the column-scale layout from the
 // device row count instead of max_rows, so that a column bundle occupies exactly dim * rows / 32 bytes; `cond`
@@ -1023,6 +1078,14 @@ extern "C" int dm_quant_mxfp8_tile32(const void* w, int64_t experts, int64_t N, 
                                      void* col_scales, int blocked, void* stream) {
   if (!w || !q || !row_scales || experts <= 0 || N <= 0 || K <= 0 || (N % 32) != 0 || (K % 32) != 0) return kRcBadArg;
   const int64_t rows = experts * N;
+  const uintptr_t all = reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(row_scales) |
+                        reinterpret_cast<uintptr_t>(col_scales);
+  if (blocked && col_scales && (N % 128) == 0 && (K % 128) == 0 && (all & 15) == 0 && (rows >> 7) * (K >> 7) < (1ll << 31)) {
+    mxfp8_tile32_kernel<<<static_cast<unsigned>((rows >> 7) * (K >> 7)), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+        static_cast<const uint4*>(w), N, static_cast<int>(K), static_cast<uint8_t*>(q), static_cast<uint8_t*>(row_scales),
+        static_cast<uint8_t*>(col_scales));
+    return static_cast<int>(cudaGetLastError());
+  }
   const dim3 grid(static_cast<unsigned>((K + 255) / 256), static_cast<unsigned>(rows / 32));
   mxfp8_slab_kernel<true><<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(
       static_cast<const __nv_bfloat16*>(w), nullptr, rows, static_cast<int>(K), static_cast<uint8_t*>(q),

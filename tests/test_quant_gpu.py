@@ -463,3 +463,31 @@ def test_mxfp8_gather_from_a_table_that_is_only_8_byte_aligned(rows, cols):
         torch.cuda.synchronize()
         got.append(out)
     assert all(torch.equal(a, b) for a, b in zip(*got)) and bool(got[0][0].any())
+
+
+@pytest.mark.parametrize("experts,n,k", [(1, 128, 128), (3, 256, 384), (2, 640, 128), (2, 128, 1152)])
+def test_mxfp8_tile32_forms_agree(experts, n, k):
+    """Aligned weights take the 128 x 128 form, the same weights two bytes further the slab form: equal bytes, with zero tiles,
+    infinities, NaNs and subnormals among the values."""
+    nat = _nat()
+    g = torch.Generator().manual_seed(n + k)
+    w = (torch.randn(experts, n, k, generator=g) * torch.exp2(torch.randint(-140, 120, (experts, n // 32, 1, k // 32, 1), generator=g)
+         .float()).expand(-1, -1, 32, -1, 32).reshape(experts, n, k)).bfloat16()
+    w[0, :32, :32] = 0
+    w[0, 5, 40] = float("inf")
+    w[-1, 100, 127] = float("nan")
+    flat = w.reshape(-1)
+    shifted = torch.zeros(flat.numel() + 1, dtype=torch.bfloat16, device=DEV)
+    shifted[1:] = flat.to(DEV)
+    aligned = flat.to(DEV)
+    out = []
+    for src in (aligned.data_ptr(), shifted.data_ptr() + 2):
+        q = torch.zeros(experts * n * k, dtype=torch.uint8, device=DEV)
+        s0 = torch.zeros(experts * n * (k // 32), dtype=torch.uint8, device=DEV)
+        s1 = torch.zeros(experts * k * (n // 32), dtype=torch.uint8, device=DEV)
+        nat.check(nat.lib.dm_quant_mxfp8_tile32(src, experts, n, k, q.data_ptr(), s0.data_ptr(), s1.data_ptr(), 1,
+                                                nat.stream_ptr()), "tile32")
+        out.append((q, s0, s1))
+    torch.cuda.synchronize()
+    for a, b in zip(*out):
+        assert torch.equal(a, b)
