@@ -1038,28 +1038,14 @@ def run_mxfp8_train(args, emit=True):
     if world > 1:
         dist.all_reduce(ms, op=dist.ReduceOp.MAX)
     ms = float(ms.item())
-    # per-call breakdown of one more step (rank 0)
-    events = []
-    names = [n for n in _native.EXPORTS if n.startswith("dm_") and n not in ("dm_version", "dm_route_workspace_words")]
-    saved = {n: getattr(_native.lib, n) for n in names}
+    # breakdown of one more step (rank 0)
+    from dist_moe_b200 import _bf16
 
-    def bracket(fn, n):
-        def call(*a):
-            a0, a1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-            a0.record()
-            r = fn(*a)
-            a1.record()
-            events.append((n, a0, a1))
-            return r
-        return call
-
-    for n in names:
-        setattr(_native.lib, n, bracket(saved[n], n))
+    _bf16.PROFILE = []
     step()
+    events, _bf16.PROFILE = _bf16.PROFILE, None
     torch.cuda.synchronize()
-    for n in names:
-        setattr(_native.lib, n, saved[n])
-    breakdown = [[n[3:], round(a0.elapsed_time(a1) * 1e3, 1)] for n, a0, a1 in events]
+    breakdown = [[n, round(a0.elapsed_time(a1) * 1e3, 1)] for n, a0, a1 in events]
     rows = int(padded) if world == 1 else None
     last = getattr(ctx._state, "last_train_call", None)  # what the device planner decided for the layer
     decision = None if last is None else ("recompute" if bool(last.need.item()) else "saved")

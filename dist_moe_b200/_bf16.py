@@ -25,8 +25,8 @@ from ._call import BWD, FWD, FWD_ALL, CallState, arguments, launch, observed, sp
 from ._execution import ExecutionOptions, RMSNormPostprocess
 
 
-# When set to a list, every grouped-GEMM launch is bracketed by CUDA events on the launching
-# stream and (name, start, end) is appended; benchmarks use it to time the kernels in place.
+# When set to a list, every grouped-GEMM launch of a BF16 pass and every step of an MXFP8 training pass is bracketed by
+# CUDA events on the launching stream and (name, start, end) is appended; benchmarks use it to time the kernels in place.
 PROFILE: list | None = None
 
 # Fused dispatch pulls the routed rows inside the W13 / W2-dgrad GEMM launches (gather warps overlap the peer
@@ -267,10 +267,11 @@ def _plain_execution(*tensors) -> bool:
     """Nothing acts on this call's operators: no tracing or fake tensors, no dispatch or function mode, no functorch
     level.  The registered operators' bodies can then run without the dispatcher, which costs a small layer more than its
     launches."""
+    if torch.compiler.is_compiling():  # first: a tracer of Python code must not meet the calls below
+        return False
     return (torch._C._len_torch_dispatch_stack() == 0 and torch._C._len_torch_function_stack() == 0
             and torch._ops._len_torch_dispatch_stack_pre_dispatch() == 0
             and torch._C._functorch.peek_interpreter_stack() is None and torch._C._get_tracing_state() is None
-            and not torch.compiler.is_compiling()
             and all(type(t) is torch.Tensor or type(t) is torch.nn.Parameter for t in tensors))
 
 

@@ -24,12 +24,14 @@ BWD = {name: 1 << i for i, name in enumerate(
     ("plan", "republish", "w13_again", "swiglu_again", "w2_again", "load_h3", "grad_h3", "combine", "w2_dgrad", "w2_wgrad",
      "swiglu", "w13_dgrad", "w13_wgrad", "close", "reduce"))}
 FWD_ALL = 255
-_GEMM_NAMES = {
+_TIMED = {
     "dm_bf16_forward": {"w13": "gemm_fprop_dispatch(w13)", "w2": "gemm_fprop(w2)"},
     "dm_bf16_backward": {
         "w13_again": "gemm_fprop_dispatch(w13 recompute)", "w2_again": "gemm_fprop(w2 recompute)",
         "w2_dgrad": "gemm_dgrad_dispatch(w2)", "w2_wgrad": "gemm_wgrad(w2)", "w13_dgrad": "gemm_dgrad(w13)",
         "w13_wgrad": "gemm_wgrad(w13)"},
+    "dm_mxfp8_forward": {name: f"forward.{name}" for name in FWD},
+    "dm_mxfp8_backward": {name: f"backward.{name}" for name in BWD},
 }
 _REPORT = ctypes.c_int32 * 2
 
@@ -55,7 +57,7 @@ def span(name: str):
 
 
 def launch(fn, names: dict, state, k, steps: int) -> None:
-    """Run the given steps of a sequence: one call, or one per step where the GEMMs are timed in place."""
+    """Run the given steps of a sequence: one call, or one per step where they are timed in place."""
     from . import _bf16
 
     context, st = state.native_layer(), nat.stream_ptr()
@@ -68,21 +70,21 @@ def launch(fn, names: dict, state, k, steps: int) -> None:
             failed = next((n for n, bit in names.items() if bit == report[1]), "arguments")
             nat.check(rc, f"{fn.__name__}({failed})")
 
-    gemms = _GEMM_NAMES.get(fn.__name__)
-    if _bf16.PROFILE is None or gemms is None:
+    timed = _TIMED[fn.__name__]
+    if _bf16.PROFILE is None:
         run(steps)
         return
     for name, bit in names.items():
         if not steps & bit:
             continue
-        if name not in gemms:
+        if name not in timed:
             run(bit)
             continue
         start, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
         start.record()
         run(bit)
         end.record()
-        _bf16.PROFILE.append((gemms[name], start, end))
+        _bf16.PROFILE.append((timed[name], start, end))
 
 
 class CallState:
