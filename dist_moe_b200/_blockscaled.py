@@ -26,8 +26,9 @@ MXFP8 training (autograd) follows the reference's staged sequence
             W2 dgrad (same qdata, transposed scales) -> W2 wgrad -> SwiGLU bwd -> quantise ->
             W13 dgrad scattered to the owners -> W13 wgrad -> barrier -> reduce over top-k
 
-Saved activations of the training path live in per-call torch allocations sized for the row capacity
-(h1 in bf16, x and h2 as column-quantised E4M3); the device planner of the BF16 path is not used here.
+Saved activations of the training path (h1 in bf16, x and h2 as column-quantised E4M3) lie where the device planner put
+them in the context's arena; the registered operators and calls with clip counters keep them in per-call allocations
+sized for the row capacity.  Each pass through the planner is one native call (``dm_mxfp8_forward`` / ``_backward``).
 NVFP4 has no backward (dist_moe/_blockscaled.py:245-321).
 """
 
