@@ -171,17 +171,16 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kBrThreads, 1)
       const int e = e0 + lane;
       int tiles = 0;
       if (e < p.e_local) {
-        const int room = s_off[e + 1] - s_off[e];
-        int rows = p.expert_counts ? p.expert_counts[e] : room;
-        rows = rows < room ? rows : room;
-        rows = rows > 0 ? rows : 0;
+        const int count = p.expert_counts ? p.expert_counts[e] : p.max_rows;
+        const int rows = bs_group_rows(s_off[e], s_off[e + 1], count);
         s_cnt[e] = rows;
+        if (count > 0 && s_off[e + 1] > s_off[e] && !bs_group_aligned(s_off[e]))
+          set_status(p.status, kCapacityExceeded, -1, e, s_off[e]);  // groups must be 128-padded
         const int nt = rw_row_tiles(rows);
         const int per = br_rows_per_tile(rows);
         s_per[e] = static_cast<uint16_t>(per);
         tiles = nt * m_pairs;
         if (nt > 0) box = max(box, rw_box_index(per));
-        if (rows > 0 && (s_off[e] & 127) != 0) set_status(p.status, kCapacityExceeded, -1, e, s_off[e]);  // rows must be 128-padded
       }
       int incl = tiles;
 #pragma unroll

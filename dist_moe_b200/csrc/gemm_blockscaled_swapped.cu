@@ -24,6 +24,7 @@
 // Forward only (inference has no backward); rows of every expert start at a multiple of 128 as the routing step
 // lays them out, and `expert_counts` tells how many of them are real.
 #include "gemm_common.cuh"
+#include "row_tiles.cuh"
 
 namespace dm {
 
@@ -125,17 +126,16 @@ __global__ void __launch_bounds__(kSwThreads, kSwCtasPerSm) blockscaled_swapped_
   }
   __syncthreads();
   for (int i = threadIdx.x; i < p.e_local; i += blockDim.x) {
-    const int room = s_off[i + 1] - s_off[i];
-    int c = p.expert_counts ? p.expert_counts[i] : room;
-    c = c < room ? c : room;
-    s_cnt[i] = c > 0 ? c : 0;
+    const int count = p.expert_counts ? p.expert_counts[i] : p.max_rows;
+    s_cnt[i] = bs_group_rows(s_off[i], s_off[i + 1], count);
+    if (count > 0 && s_off[i + 1] > s_off[i] && !bs_group_aligned(s_off[i]))
+      set_status(p.status, kCapacityExceeded, -1, i, s_off[i]);  // groups must be 128-padded
   }
   __syncthreads();
   if (threadIdx.x == 0) {
     int acc = 0;
     for (int e = 0; e < p.e_local; ++e) {
       s_tile_start[e] = acc;
-      if (s_cnt[e] > 0 && (s_off[e] & 127) != 0) set_status(p.status, kCapacityExceeded, -1, e, s_off[e]);
       acc += ((s_cnt[e] + kSwTileRows - 1) / kSwTileRows) * m_tiles;
     }
     s_tile_start[p.e_local] = acc;

@@ -1,5 +1,5 @@
-// How the BF16 forward and input-gradient GEMMs split an expert's routed rows into tiles, and which gathered row blocks a
-// tile needs.  Plain arithmetic, for the kernel and for host code.
+// How the forward and input-gradient GEMMs split an expert's routed rows into tiles, and which gathered row blocks a BF16
+// tile needs.  Plain arithmetic, for the kernels and for host code.
 #pragma once
 
 #include <stdint.h>
@@ -61,6 +61,15 @@ DM_HOST_DEVICE RowsBlocks rw_tile_blocks(const RowsTile& t, int total_rows) {
   b.first = t.row0 / kRwGatherBlock;
   b.last = (end - 1) / kRwGatherBlock;
   return b;
+}
+
+// Rows of the group [off, next) that a block-scaled GEMM works on, `count` of them real.  None where the group does not
+// start on a scale atom of 128 rows: the caller has broken the padding rule, and the MMA would take the rows' scales from an
+// odd TMEM column, which is a misaligned address.
+DM_HOST_DEVICE constexpr bool bs_group_aligned(int off) { return (off & 127) == 0; }
+DM_HOST_DEVICE int bs_group_rows(int off, int next, int count) {
+  const int room = next - off, rows = count < room ? count : room;
+  return rows > 0 && bs_group_aligned(off) ? rows : 0;
 }
 
 }  // namespace dm

@@ -326,7 +326,8 @@ int dm_gemm_wgrad(dm_operand dy, dm_operand x, void* dw, int out_is_fp32, int ac
  *   swiglu_interleaved != 0: W is W13 with rows interleaved in groups of 8 gate / 8 up rows
  *       (dist_moe/_blockscaled_weight.py:16-39); writes h2 = bf16(SwiGLU(bf16 gate, bf16 up)) [rows, N/2]
  *       and, when C is given, h1 = [gate | up] in the canonical (not interleaved) column order.
- * Every expert's row range must start on a multiple of 128 (routing with m_multiple_of = 128).
+ * Every expert's row range must start on a multiple of 128 (routing with m_multiple_of = 128).  Otherwise the status is
+ * set to DM_STATUS_CAPACITY_EXCEEDED and that expert's results are not defined; the MXFP8 and the swapped form leave it out.
  * ------------------------------------------------------------------------- */
 int dm_gemm_blockscaled(int format, dm_operand a, dm_operand sfa, const void* w, const void* sfb, dm_operand c,
                         dm_operand h2, const int64_t* scatter_ptrs, dm_operand row_scale_inv,

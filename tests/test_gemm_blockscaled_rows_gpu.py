@@ -122,3 +122,28 @@ def test_input_gradient_rows(counts, K, N):
             _close(out.cpu()[rows], da[rows] @ dw[e], f"expert {e}")
         assert bool((out[off[e] + n:off[e + 1]] == 0).all())
     assert bool((out[off[-1]:] == 5.0).all())
+
+
+@pytest.mark.parametrize("swapped,fmt", [(False, 0), (True, 0), (True, 1)])
+@pytest.mark.parametrize("counted", [True, False])
+def test_groups_that_are_not_padded_are_left_out(swapped, fmt, counted):
+    """Experts that do not start on 128 rows: a status, none of their rows written, the others as ever."""
+    nat = _nat()
+    K, N = 512, 256
+    E, off, real, R, (qa, sa, da, inv), (qw, sw, dw, einv), _, _ = _operands(nat, fmt, [128, 128, 128, 128], K, N, 23 + fmt)
+    off = [0, 128, 160, 384, 512]
+    offs = torch.tensor(off, dtype=torch.int32, device=DEV)
+    cnts = torch.tensor([100, 32, 200, 128], dtype=torch.int32, device=DEV)
+    status = torch.zeros(8, dtype=torch.int32, device=DEV)
+    out = torch.full((R, N), 5.0, device=DEV, dtype=torch.bfloat16)
+    fn = nat.lib.dm_gemm_blockscaled_swapped if swapped else nat.lib.dm_gemm_blockscaled_counted
+    nat.check(fn(fmt, _op(nat, qa), _op(nat, sa), qw.data_ptr(), sw.data_ptr(), _op(nat, out), _op(nat, None), None,
+                 _op(nat, inv), nat.ptr(einv), offs.data_ptr(), cnts.data_ptr() if counted else None, E, R, N, K, 0, 0, 1.0,
+                 0.0, None, 0, status.data_ptr(), nat.stream_ptr()), "unpadded group")
+    torch.cuda.synchronize()
+    assert status.tolist()[:4] == [2, -1, 2, 160]
+    got = out.cpu()
+    assert bool((got[160:384] == 5.0).all())
+    for e, rows in ((0, 100), (1, 32), (3, 128)):
+        at = torch.arange(off[e], off[e] + rows)
+        _close(got[at], da[at] @ dw[e].T, f"expert {e}")
