@@ -117,6 +117,7 @@ __global__ void __launch_bounds__(256) scale_and_sum_kernel(const uint4* __restr
                                                             const int* save_cond, int save_expect) {
   bool save = save_base != nullptr;
   if (save && save_cond != nullptr) save = ((*save_cond != 0) == (save_expect != 0));
+  if (save && save_offset != nullptr) save = *save_offset >= 0;
   uint4* save_dst = save ? reinterpret_cast<uint4*>(save_base + (save_offset ? *save_offset : 0)) : nullptr;
   const int64_t total = T * vec_per_row;
   for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < total;
@@ -174,7 +175,9 @@ __global__ void __launch_bounds__(256) broadcast_and_scale_kernel(const uint4* _
                                                                   float* grad_scores, int64_t T, int K,
                                                                   int vec_per_row) {
   const uint4* h3 = h3_base ? reinterpret_cast<const uint4*>(h3_base + (h3_offset ? *h3_offset : 0)) : nullptr;
-  if (h3_alt != nullptr && use_alt != nullptr && *use_alt != 0) h3 = reinterpret_cast<const uint4*>(h3_alt);
+  // (a negative offset: the planner gave the outputs no place in the slot)
+  if (h3_alt != nullptr && use_alt != nullptr && (*use_alt != 0 || (h3_offset != nullptr && *h3_offset < 0)))
+    h3 = reinterpret_cast<const uint4*>(h3_alt);
   const int lane = threadIdx.x & 31;
   const int warps_per_block = blockDim.x >> 5;
   const int64_t routes = T * K;

@@ -26,7 +26,7 @@ struct PlanFwdParams {
   int64_t* fwd_state;
   const int64_t* slot_selector;
   int64_t* moe_layer_id;
-  int ep, K, num_slots, num_layers, scratch_only;
+  int ep, K, num_slots, num_layers, scratch_only, bounded;
   int64_t T, D, F, slot_bytes;
   int* status;
 };
@@ -45,7 +45,7 @@ __global__ void plan_fwd_bf16_kernel(PlanFwdParams p) {
   const int64_t s_xg = s_h1 - xg_size;
   const int64_t selector = p.slot_selector[0];
 
-  bool need = true;
+  bool need = true, lost = false;
   int64_t x_off = 0, xg_off = s_xg, h1_off = s_h1, h2_off = s_h2, h3_off = 0;
   int64_t m = 0, new_free = 0, slot_end = 0, layer = 0;
   const int64_t x_mem = align128(p.T * p.D * es);
@@ -64,15 +64,18 @@ __global__ void plan_fwd_bf16_kernel(PlanFwdParams p) {
       worst = v > worst ? v : worst;
     }
     need = worst + layers_after * x_mem > p.slot_bytes;
+    new_free = free_start + (need ? x_mem : xg_size + h1_size + h3_mem);
+    // Calls that break the last-in-first-out order of a slot (forwards without a backward, backwards out of order) move
+    // its free pointer out of it, in the end out of the arena.  A save that is not inside the slot does not run.
+    lost = p.bounded && (new_free > slot_end || free_start < slot_end - p.slot_bytes);
     if (need) {
-      x_off = free_start;
-      new_free = x_off + x_mem;
+      x_off = lost ? -1 : free_start;
+    } else if (lost) {
+      h3_off = -1;
     } else {
       xg_off = free_start;
       h1_off = xg_off + xg_size;
       h3_off = h1_off + h1_size;
-      new_free = h3_off + h3_mem;
-      x_off = 0;
     }
   }
   p.need_recompute[0] = need ? 1 : 0;
@@ -84,14 +87,14 @@ __global__ void plan_fwd_bf16_kernel(PlanFwdParams p) {
   p.fwd_state[4] = h3_off;
   p.fwd_state[5] = selector;
 
-  const int64_t scratch_bottom = need ? xg_off : h2_off;
+  const int64_t scratch_bottom = need || lost ? xg_off : h2_off;
   const int64_t scratch_base = static_cast<int64_t>(N) * p.slot_bytes;
   if (scratch_bottom < scratch_base) set_status(p.status, kArenaOverflow, 0);
   const int64_t scratch_free = scratch_bottom - scratch_base;
   if (scratch_free < p.peak[N]) p.peak[N] = scratch_free;
 
   if (!p.scratch_only) {
-    if (new_free > slot_end) set_status(p.status, kArenaOverflow, 1, static_cast<int>(m));
+    if (new_free > slot_end || lost) set_status(p.status, kArenaOverflow, 1, static_cast<int>(m));
     const int64_t slot_free = slot_end - new_free;
     if (slot_free < p.peak[m]) p.peak[m] = slot_free;
     p.buffer_offsets[m] = new_free;
@@ -165,9 +168,12 @@ __global__ void plan_bwd_bf16_kernel(PlanBwdParams p) {
   p.bwd_offsets[4] = g_h3g;
   p.bwd_offsets[5] = g_h1;
 
-  p.buffer_offsets[m] = need ? fwd_x : fwd_xg;
   const int64_t x_mem = align128(p.T * p.D * es);
   const int64_t h3_mem = align128(p.T * p.K * p.D * es);
+  if ((need ? fwd_x : p.fwd_state[4]) < 0)  // the forward's save did not run: give back what it was counted with
+    p.buffer_offsets[m] = free_start - (need ? x_mem : xg_size + h1_size + h3_mem);
+  else
+    p.buffer_offsets[m] = need ? fwd_x : fwd_xg;
   for (int r = 0; r < p.ep; ++r) {
     const int64_t rr = p.per_rank[r];
     const int64_t full = align128(rr * p.D * es) + align128(rr * 2 * p.F * es) + h3_mem;
@@ -188,11 +194,13 @@ extern "C" int dm_plan_fwd_bf16(const int32_t* recv_rows, const int32_t* per_ran
                                 void* stream) {
   if (!recv_rows || !per_rank || !buffer_offsets || !peak_min_free || !need_recompute || !fwd_state || !slot_selector)
     return kRcBadArg;
+  const int bounded = scratch_only & DM_PLAN_BOUNDED;
+  scratch_only &= ~DM_PLAN_BOUNDED;
   if (!scratch_only && (!saved_bytes_per_rank || !moe_layer_id || num_slots <= 0)) return kRcBadArg;
   if (ep <= 0 || num_tokens <= 0 || K <= 0 || D <= 0 || F <= 0 || num_slots < 0) return kRcBadArg;
   PlanFwdParams p{recv_rows, per_rank, saved_bytes_per_rank, buffer_offsets, peak_min_free, need_recompute,
                   recompute_cond, fwd_state, slot_selector, moe_layer_id, ep, K, num_slots, num_moe_layers,
-                  scratch_only, num_tokens, D, F, slot_bytes, status};
+                  scratch_only, bounded, num_tokens, D, F, slot_bytes, status};
   plan_fwd_bf16_kernel<<<1, 32, 0, static_cast<cudaStream_t>(stream)>>>(p);
   return static_cast<int>(cudaGetLastError());
 }

@@ -94,7 +94,7 @@ struct BsPlanFwdParams {
   int64_t* fwd_offsets;   // [x, x_gathered, h1, h2, h3, x_row, x_col, h2_row, h2_col, slot selector]
   int64_t* fwd_table;     // 2 groups: dispatch (W13), combine (W2)
   const int64_t* slot_selector;
-  int num_layers, inference_mode, scratch_only, interleaved_fc13;
+  int num_layers, inference_mode, scratch_only, interleaved_fc13, bounded;
 };
 
 __global__ void plan_fwd_blockscaled_kernel(BsPlanFwdParams p) {
@@ -148,16 +148,20 @@ __global__ void plan_fwd_blockscaled_kernel(BsPlanFwdParams p) {
       worst = v > worst ? v : worst;
     }
     need = worst + layers_after * x_mem > c.slot_bytes;
-    int64_t new_free;
-    if (need && c.native_backward) {
-      x_off = free_start;  // the packed dispatch input
-      new_free = x_off + x_mem;
+    const int64_t saved_size = c.native_backward ? x_row.total() + h1_size + h2_row.total() + h3_mem
+                                                 : x_col.total() + h1_size + h2_col.total() + h3_mem;
+    const int64_t new_free = free_start + (need ? x_mem : saved_size);
+    // A save that is not inside the slot (calls that broke its last-in-first-out order) does not run: see planner.cu.
+    const bool lost = p.bounded && (new_free > slot_end || free_start < slot_end - c.slot_bytes);
+    if (need)
+      x_off = lost ? -1 : free_start;  // dense x, or the packed dispatch input
+    else if (lost)
+      h3_off = -1;
+    if ((need || lost) && c.native_backward) {
       h1_off = row_slot_off - h1_size;
       scratch_bottom = h1_off;
-    } else if (need) {
-      x_off = free_start;  // dense x; everything else is transient, descending below the row slot
-      new_free = x_off + x_mem;
-      x_col_off = row_slot_off - x_col.total();
+    } else if (need || lost) {
+      x_col_off = row_slot_off - x_col.total();  // transient, descending below the row slot
       h1_off = x_col_off - h1_size;
       h2_col_off = h1_off - h2_col.total();
       scratch_bottom = h2_col_off;
@@ -166,17 +170,15 @@ __global__ void plan_fwd_blockscaled_kernel(BsPlanFwdParams p) {
       h1_off = x_row_off + x_row.total();
       h2_row_off = h1_off + h1_size;
       h3_off = h2_row_off + h2_row.total();
-      new_free = h3_off + h3_mem;
       scratch_bottom = scratch_end;
     } else {
       x_col_off = free_start;  // saved, ascending: x_col, h1, h2_col, h3
       h1_off = x_col_off + x_col.total();
       h2_col_off = h1_off + h1_size;
       h3_off = h2_col_off + h2_col.total();
-      new_free = h3_off + h3_mem;
       scratch_bottom = row_slot_off;
     }
-    if (new_free > slot_end) set_status(c.status, kArenaOverflow, 1, static_cast<int>(m));
+    if (new_free > slot_end || lost) set_status(c.status, kArenaOverflow, 1, static_cast<int>(m));
     const int64_t slot_free = slot_end - new_free;
     if (slot_free < c.peak[m]) c.peak[m] = slot_free;
     c.buffer_offsets[m] = new_free;
@@ -372,9 +374,14 @@ __global__ void plan_bwd_blockscaled_kernel(BsPlanBwdParams p) {
 
   // rewind the slot to where the matching forward layer began, and undo its accounting
   const int64_t saved_base = c.native_backward ? fwd_x_row : x_col_off;
-  c.buffer_offsets[m] = need ? fwd_x : saved_base;
   const int64_t x_mem = c.native_backward ? packed_dispatch_size(c.T, c.D, g) : bs_align(c.T * c.D * g.element_size);
   const int64_t h3_mem = bs_align(c.T * c.K * c.D * g.element_size);
+  const int64_t saved_size = c.native_backward ? x_row.total() + h1_size + h2_row.total() + h3_mem
+                                               : x_col.total() + h1_size + h2_col.total() + h3_mem;
+  if ((need ? fwd_x : p.fwd_offsets[4]) < 0)  // the forward's save did not run: give back what it was counted with
+    c.buffer_offsets[m] = free_start - (need ? x_mem : saved_size);
+  else
+    c.buffer_offsets[m] = need ? fwd_x : saved_base;
   for (int r = 0; r < c.ep; ++r)
     c.saved[m * c.ep + r] -= need ? x_mem : no_recompute_alloc(c.per_rank[r], h3_mem, c.D, c.F, g, c.native_backward);
   c.moe_layer_id[m] -= 1;
@@ -401,6 +408,8 @@ extern "C" int dm_plan_fwd_blockscaled(const int32_t* recv_rows, const int32_t* 
   if (!recv_rows || !per_rank || !buffer_offsets || !peak_min_free || !need_recompute || !fwd_offsets ||
       !fwd_activation_offsets || !geometry_ok(storage))
     return kRcBadArg;
+  const int bounded = scratch_only & DM_PLAN_BOUNDED;
+  scratch_only &= ~DM_PLAN_BOUNDED;
   const bool uses_slots = !(inference_mode || scratch_only);
   if (uses_slots && (!saved_bytes_per_rank || !moe_layer_id || !slot_selector || num_slots <= 0)) return kRcBadArg;
   if (ep <= 0 || num_tokens <= 0 || K <= 0 || D <= 0 || F <= 0 || num_slots < 0 || capacity_rows < 0) return kRcBadArg;
@@ -419,6 +428,7 @@ extern "C" int dm_plan_fwd_blockscaled(const int32_t* recv_rows, const int32_t* 
   p.inference_mode = inference_mode;
   p.scratch_only = scratch_only;
   p.interleaved_fc13 = interleaved_fc13;
+  p.bounded = bounded;
   plan_fwd_blockscaled_kernel<<<1, 32, 0, static_cast<cudaStream_t>(stream)>>>(p);
   return static_cast<int>(cudaGetLastError());
 }

@@ -66,6 +66,7 @@ __global__ void __launch_bounds__(256) rmsnorm_combine_fwd_kernel(
   __shared__ float rs[kNormMaxK];
   bool save = save_base != nullptr;
   if (save && save_cond != nullptr) save = ((*save_cond != 0) == (save_expect != 0));
+  if (save && save_offset != nullptr) save = *save_offset >= 0;
   uint4* save_dst = save ? reinterpret_cast<uint4*>(save_base + (save_offset ? *save_offset : 0)) : nullptr;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const float inv_d = 1.0f / static_cast<float>(vec * 8);

@@ -412,8 +412,10 @@ __global__ void gather_rows_kernel(const int64_t* __restrict__ ptrs, const int32
 __global__ void cond_copy_kernel(const uint8_t* src_base, const int64_t* src_offset, uint8_t* dst_base,
                                  const int64_t* dst_offset, int64_t n_vec, const int* cond, int expect) {
   if (cond != nullptr && ((*cond != 0) != (expect != 0))) return;
-  const uint4* src = reinterpret_cast<const uint4*>(src_base + (src_offset ? *src_offset : 0));
-  uint4* dst = reinterpret_cast<uint4*>(dst_base + (dst_offset ? *dst_offset : 0));
+  const int64_t from = src_offset ? *src_offset : 0, to = dst_offset ? *dst_offset : 0;
+  if (from < 0 || to < 0) return;  // the planner gave this save no place
+  const uint4* src = reinterpret_cast<const uint4*>(src_base + from);
+  uint4* dst = reinterpret_cast<uint4*>(dst_base + to);
   for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < n_vec;
        i += static_cast<int64_t>(gridDim.x) * blockDim.x)
     dst[i] = src[i];

@@ -61,7 +61,7 @@ extern "C" int dm_bf16_forward(const dm_layer_context* ctx, const dm_layer_call*
   s.step(DM_FWD_ROUTE, 1, [&] {
     return dm_plan_fwd_bf16(recv, k.per_rank, c.saved_bytes, c.buffer_offsets, c.peak_min_free, k.need, k.cond, fs,
                             c.slot_selector, c.moe_layer_id, c.ep, c.T_max, c.K, c.D, c.F, c.slot_bytes, c.num_slots,
-                            k.num_layers, k.scratch_only, c.status, stream);
+                            k.num_layers, k.scratch_only | DM_PLAN_BOUNDED, c.status, stream);
   });
   if (!k.scratch_only)
     s.step(DM_FWD_SAVE_X, 1, [&] { return dm_cond_copy(k.x, nullptr, c.arena, fs, k.T * c.D * 2, k.cond, 1, stream); });
@@ -215,7 +215,8 @@ extern "C" int dm_mxfp8_forward(const dm_layer_context* ctx, const dm_layer_call
   s.step(DM_FWD_ROUTE, 1, [&] {
     return dm_plan_fwd_blockscaled(recv, k.per_rank, nullptr, c.saved_bytes, c.buffer_offsets, c.peak_min_free, k.need, k.cond,
                                    fs, ft, c.slot_selector, c.moe_layer_id, c.ep, c.T_max, c.K, c.D, c.F, c.storage,
-                                   c.capacity_rows, c.slot_bytes, c.num_slots, k.num_layers, 0, 0, 0, 0, 0, c.status, stream);
+                                   c.capacity_rows, c.slot_bytes, c.num_slots, k.num_layers, 0, 0, DM_PLAN_BOUNDED, 0, 0,
+                                   c.status, stream);
   });
   // a layer that will be recomputed keeps only its dense input
   s.step(DM_FWD_SAVE_X, 1, [&] { return dm_cond_copy(k.x, nullptr, c.arena, fs, k.T * c.D * 2, k.cond, 1, stream); });

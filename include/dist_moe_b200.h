@@ -146,7 +146,12 @@ int dm_route_decode_kernel_enabled(void); /* the current setting, without changi
  * reference does.  fwd_state = [x, x_gathered, h1, h2, h3, slot id],
  * bwd_offsets = [x_gathered, h1, h2, grad_h2, grad_h3_gathered, grad_h1].
  * need_recompute is one byte (bool).  Overflow sets DM_STATUS_ARENA_OVERFLOW.
+ * scratch_only: 0 or 1; | DM_PLAN_BOUNDED: a save that would not lie inside its slot (calls that broke the slot's
+ * last-in-first-out order) gets the offset -1 (x where the layer is recomputed, else h3), everything else of that call a
+ * place in scratch, so that no launch leaves the arena.  dm_cond_copy, dm_scale_and_sum and dm_rmsnorm_combine_fwd copy
+ * nothing to or from a negative offset; dm_broadcast_and_scale_select reads h3_alt then.
  * ------------------------------------------------------------------------- */
+enum { DM_PLAN_BOUNDED = 2 };
 int dm_plan_fwd_bf16(const int32_t* recv_rows, const int32_t* per_rank, int64_t* saved_bytes_per_rank,
                      int64_t* buffer_offsets, int64_t* peak_min_free, uint8_t* need_recompute,
                      int32_t* recompute_cond, int64_t* fwd_state, const int64_t* slot_selector,
@@ -176,6 +181,7 @@ int dm_plan_bwd_bf16(const int32_t* recv_rows, const int32_t* per_rank, int64_t*
  *                      grad_h3_row, grad_h3_col, dxy_row, dxy_col, x_row global scales, h2_row global scales};
  *   bwd_activation_offsets[6*9]: groups {recompute dispatch, recompute combine, W2 dgrad, W2 wgrad, W13 dgrad,
  *                      W13 wgrad}.
+ * scratch_only may carry DM_PLAN_BOUNDED, as above.
  * per_rank_snapshot (optional) receives a copy of per_rank.  Rows above capacity_rows set
  * DM_STATUS_CAPACITY_EXCEEDED, an overflowing slot or scratch region DM_STATUS_ARENA_OVERFLOW (the reference
  * asserts on the device).
@@ -206,7 +212,7 @@ int dm_gather_rows(const int64_t* ptrs, const int32_t* num_rows, void* dst_base,
 
 /* Device-predicated copy (dist_moe/kernels/triton/conditional_copy.py:482-630).
  * Copies `bytes` from src(+*src_offset) to dst(+*dst_offset) when cond is NULL
- * or (*cond != 0) == (expect != 0). */
+ * or (*cond != 0) == (expect != 0).  A negative offset: nothing is copied. */
 int dm_cond_copy(const void* src_base, const int64_t* src_offset, void* dst_base, const int64_t* dst_offset,
                  int64_t bytes, const int* cond, int expect, void* stream);
 
@@ -232,7 +238,7 @@ int dm_swiglu_bwd(const void* h1_base, const int64_t* h1_offset, const void* gra
  *   scale_and_sum:       out[t,:] = bf16( sum_k scores[t,k] * h3[t,k,:] ), routes with id < 0 skipped;
  *                        scores == NULL means weight 1 (reduce_from_topk).
  *                        save_base(+*save_offset) (may be NULL) receives a copy of h3 when save_cond is
- *                        NULL or (*save_cond != 0) == (save_expect != 0).
+ *                        NULL or (*save_cond != 0) == (save_expect != 0), and *save_offset is not negative.
  *   broadcast_and_scale: grad_h3[t,k,:] = bf16(scores[t,k] * grad_out[t,:]);
  *                        grad_scores[t,k] = sum_d h3[t,k,d] * grad_out[t,d]  (0 for id < 0).
  * scores are fp32 or bf16 (scores_are_bf16); ids int32 or int64.
@@ -244,8 +250,8 @@ int dm_broadcast_and_scale(const void* grad_out, const void* scores, int scores_
                            int ids_are_int64, const void* h3_base, const int64_t* h3_offset, void* grad_h3,
                            float* grad_scores, int64_t T, int K, int64_t D, void* stream);
 /* dm_broadcast_and_scale with the expert outputs read from `h3_alt` when *use_alt != 0 (recomputed into the
- * communication buffer), else from h3_base + *h3_offset (saved in the activation slot): the choice the planner
- * made on the device, without copying the saved outputs back first. */
+ * communication buffer) or *h3_offset is negative, else from h3_base + *h3_offset (saved in the activation slot): the
+ * choice the planner made on the device, without copying the saved outputs back first. */
 int dm_broadcast_and_scale_select(const void* grad_out, const void* scores, int scores_are_bf16, const void* ids,
                                   int ids_are_int64, const void* h3_base, const int64_t* h3_offset, const void* h3_alt,
                                   const int* use_alt, void* grad_h3, float* grad_scores, int64_t T, int K, int64_t D,

@@ -33,7 +33,12 @@ def _full(rr, D, F, h3_mem):
     return align(rr * D * 2) + align(rr * 2 * F * 2) + h3_mem
 
 
-def plan_forward(st: PlannerState, R, per_rank, selector, *, T, K, D, F, num_layers, scratch_only):
+def lost(st: PlannerState, m: int, free: int, new_free: int) -> bool:
+    """The bytes [free, new_free) are not all inside slot ``m`` (this library's bounded saves; not in the reference)."""
+    return free < m * st.slot_bytes or new_free > (m + 1) * st.slot_bytes
+
+
+def plan_forward(st: PlannerState, R, per_rank, selector, *, T, K, D, F, num_layers, scratch_only, bounded=False):
     es, N = 2, st.n
     xg, h1, h2 = align(R * D * es), align(R * 2 * F * es), align(R * F * es)
     end = st.buffer_offsets[N]
@@ -41,6 +46,7 @@ def plan_forward(st: PlannerState, R, per_rank, selector, *, T, K, D, F, num_lay
     s_h1 = s_h2 - h1
     s_xg = s_h1 - xg
     x_mem, h3_mem = align(T * D * es), align(T * K * D * es)
+    gone = False
     need, x_off, xg_off, h1_off, h2_off, h3_off = True, 0, s_xg, s_h1, s_h2, 0
     if not scratch_only:
         m = selector % N
@@ -49,13 +55,15 @@ def plan_forward(st: PlannerState, R, per_rank, selector, *, T, K, D, F, num_lay
         layer = st.layer[m]
         worst = max(st.saved[m * st.ep + r] + _full(per_rank[r], D, F, h3_mem) for r in range(st.ep))
         need = worst + (num_layers - 1 - layer) * x_mem > st.slot_bytes
+        new_free = free + (x_mem if need else xg + h1 + h3_mem)
+        gone = bounded and lost(st, m, free, new_free)
         if need:
-            x_off, new_free = free, free + x_mem
+            x_off = -1 if gone else free
+        elif gone:
+            h3_off = -1
         else:
-            xg_off, h1_off = free, free + xg
-            h3_off = h1_off + h1
-            new_free, x_off = h3_off + h3_mem, 0
-    bottom = xg_off if need else h2_off
+            xg_off, h1_off, h3_off = free, free + xg, free + xg + h1
+    bottom = xg_off if need or gone else h2_off
     st.peak[N] = min(st.peak[N], bottom - N * st.slot_bytes)
     if not scratch_only:
         st.peak[m] = min(st.peak[m], slot_end - new_free)
@@ -84,8 +92,11 @@ def plan_backward(st: PlannerState, R, per_rank, need, fwd_state, *, T, K, D, F)
         xg_off, h1_off, bottom = fwd_state[1], fwd_state[2], grad_bottom
     st.peak[m] = min(st.peak[m], slot_end - free)
     st.peak[N] = min(st.peak[N], bottom - N * st.slot_bytes)
-    st.buffer_offsets[m] = fwd_state[0] if need else fwd_state[1]
     x_mem, h3_mem = align(T * D * es), align(T * K * D * es)
+    if (fwd_state[0] if need else fwd_state[4]) < 0:
+        st.buffer_offsets[m] = free - (x_mem if need else xg + h1 + h3_mem)
+    else:
+        st.buffer_offsets[m] = fwd_state[0] if need else fwd_state[1]
     for r in range(st.ep):
         st.saved[m * st.ep + r] -= x_mem if need else _full(per_rank[r], D, F, h3_mem)
     st.layer[m] -= 1

@@ -12,7 +12,7 @@ from __future__ import annotations
 
 from dataclasses import dataclass
 
-from .planner import PlannerState, align
+from .planner import PlannerState, align, lost
 
 MISSING = -1
 
@@ -71,7 +71,7 @@ def _group(a_q=MISSING, b_q=MISSING, c=MISSING, a_scale=MISSING, b_scale=MISSING
 
 
 def plan_forward(st: PlannerState, rows, per_rank, selector, *, T, K, D, F, storage: Storage, num_layers,
-                 mega=False, inference=False, scratch_only=False, native=False, interleaved=False):
+                 mega=False, inference=False, scratch_only=False, native=False, interleaved=False, bounded=False):
     """Returns dict(need, offsets[10], table[18]); updates ``st`` in place."""
     s, N, es = storage, st.n, 2
     h1 = align(rows * 2 * F * es)
@@ -106,12 +106,17 @@ def plan_forward(st: PlannerState, rows, per_rank, selector, *, T, K, D, F, stor
         cost = [_saved_cost(per_rank[r], h3_mem, D, F, s, native) for r in range(st.ep)]
         worst = max(st.saved[m * st.ep + r] + cost[r] for r in range(st.ep))
         need = worst + (num_layers - 1 - layer) * x_mem > st.slot_bytes
-        if need and native:
-            x_off, new_free = free, free + x_mem
+        size = xr + h1 + hr + h3_mem if native else xc_q + xc_s + h1 + hc_q + hc_s + h3_mem
+        new_free = free + (x_mem if need else size)
+        gone = bounded and lost(st, m, free, new_free)
+        if need:
+            x_off = -1 if gone else free
+        elif gone:
+            h3_off = -1
+        if (need or gone) and native:
             h1_off = slot_off - h1
             bottom = h1_off
-        elif need:
-            x_off, new_free = free, free + x_mem
+        elif need or gone:
             x_col = slot_off - xc_q - xc_s
             h1_off = x_col - h1
             h2_col = h1_off - hc_q - hc_s
@@ -121,13 +126,13 @@ def plan_forward(st: PlannerState, rows, per_rank, selector, *, T, K, D, F, stor
             h1_off = x_row + xr
             h2_row = h1_off + h1
             h3_off = h2_row + hr
-            new_free, bottom = h3_off + h3_mem, end
+            bottom = end
         else:
             x_col = free
             h1_off = x_col + xc_q + xc_s
             h2_col = h1_off + h1
             h3_off = h2_col + hc_q + hc_s
-            new_free, bottom = h3_off + h3_mem, slot_off
+            bottom = slot_off
         st.peak[m] = min(st.peak[m], (m + 1) * st.slot_bytes - new_free)
         st.buffer_offsets[m] = new_free
         st.layer[m] = layer + 1
@@ -220,9 +225,13 @@ def plan_backward(st: PlannerState, rows, per_rank, need, fwd_offsets, *, T, K, 
         + _group(a_q=g3_col, b_q=h2_col, a_scale=g3cs, b_scale=hcs)
         + _group(a_q=dxy_row, a_scale=dxy_row + dr_q, source_x=g2_off, source_y=h1_off, col_q=dxy_col, col_scale=dcs)
         + _group(a_q=dxy_col, b_q=x_col, a_scale=dcs, b_scale=xcs))
-    st.buffer_offsets[m] = fwd_x if need else (fwd_x_row if native else x_col)
     x_mem = packed_dispatch_size(T, D, s) if native else align(T * D * es)
     h3_mem = align(T * K * D * es)
+    if (fwd_x if need else fwd_offsets[4]) < 0:
+        size = xr + h1 + hr + h3_mem if native else xc_q + xc_s + h1 + hc_q + hc_s + h3_mem
+        st.buffer_offsets[m] = free - (x_mem if need else size)
+    else:
+        st.buffer_offsets[m] = fwd_x if need else (fwd_x_row if native else x_col)
     for r in range(st.ep):
         st.saved[m * st.ep + r] -= x_mem if need else _saved_cost(per_rank[r], h3_mem, D, F, s, native)
     st.layer[m] -= 1
