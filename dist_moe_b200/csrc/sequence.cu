@@ -135,10 +135,10 @@ extern "C" int dm_bf16_backward(const dm_layer_context* ctx, const dm_layer_call
     return dm_gemm_fprop(s.arena(bo + 2), k.w2, kNone, kNone, k.sct_ptrs, k.expert_offsets, c.e_local, k.max_rows, c.D, c.F, 0,
                          0, 1.0f, 0.0f, k.cond, c.num_sms, c.status, stream);
   });
+  s.barrier(DM_BWD_W2_AGAIN, c.combine_pads, k.cond);
   s.step(DM_BWD_LOAD_H3, 1, [&] {
     return dm_cond_copy(c.arena, fs + 4, c.combine, nullptr, k.T * c.K * c.D * 2, k.cond, 0, stream);
   });
-  s.barrier(DM_BWD_W2_AGAIN, c.combine_pads, k.cond);
   // ---- gradient of the expert outputs and the scores: saved outputs are read where they were saved (chosen on the device)
   s.step(DM_BWD_GRAD_H3, 1, [&] {
     if (k.grad_scores != nullptr && !k.h3_in_combine)
@@ -290,10 +290,10 @@ extern "C" int dm_mxfp8_backward(const dm_layer_context* ctx, const dm_layer_cal
                                        k.expert_offsets, k.real_counts, c.e_local, k.max_rows, c.D, c.F, 0, 0, 1.0f, 0.0f,
                                        k.cond, c.num_sms, c.status, stream);
   });
+  s.barrier(DM_BWD_W2_AGAIN, c.combine_pads, k.cond);
   s.step(DM_BWD_LOAD_H3, 1, [&] {
     return dm_cond_copy(c.arena, fs + 4, c.combine, nullptr, k.T * c.K * c.D * 2, k.cond, 0, stream);
   });
-  s.barrier(DM_BWD_W2_AGAIN, c.combine_pads, k.cond);
   // ---- gradient of the expert outputs and the scores -------------------------------------------------------------
   s.step(DM_BWD_GRAD_H3, 1, [&] {
     if (k.grad_scores != nullptr)

@@ -21,13 +21,21 @@ def stub(tmp_path_factory):
     source = (ROOT / "dist_moe_b200" / "csrc" / "sequence.cu").read_text()
     called = sorted(set(re.findall(r"\b(dm_\w+)\(", source)) - {"dm_bf16_forward", "dm_bf16_backward", "dm_mxfp8_forward",
                                                                  "dm_mxfp8_backward"})
-    code = ['#include <string>', '#include "../../include/dist_moe_b200.h"', "static std::string calls, fail;",
+    # each call is recorded by name and, in a second log, with its barrier's pads and its predicate (pointers as numbers)
+    code = ['#include <string>', '#include "../../include/dist_moe_b200.h"', "static std::string calls, details, fail;",
             'extern "C" const char* stub_calls() { return calls.c_str(); }',
-            'extern "C" void stub_reset(const char* f) { calls.clear(); fail = f; }',
-            "static int note(const char* n) { calls += n; calls += ' '; return fail == n ? 7 : 0; }"]
+            'extern "C" const char* stub_details() { return details.c_str(); }',
+            'extern "C" void stub_reset(const char* f) { calls.clear(); details.clear(); fail = f; }',
+            "static int note(const char* n, const void* pads, const void* cond) {",
+            "  calls += n; calls += ' ';",
+            "  details += std::string(n) + ',' + std::to_string((unsigned long)pads) + ',' + std::to_string((unsigned long)cond) + ' ';",
+            "  return fail == n ? 7 : 0; }"]
     for name in called:
         text = re.search(r"^int " + name + r"\(.*?\);", HEADER, flags=re.M | re.S).group(0)[:-1]
-        answer = "return 1;" if name == "dm_route_decode_kernel_enabled" else f'return note("{name}");'
+        words = re.findall(r"\w+", text)
+        pads = "signal_pads" if "signal_pads" in words else "nullptr"
+        cond = next((w for w in ("cond", "save_cond", "use_alt") if w in words), "nullptr")
+        answer = "return 1;" if name == "dm_route_decode_kernel_enabled" else f'return note("{name}", {pads}, {cond});'
         code.append(f'extern "C" {text} {{ {answer} }}')
     src = work / "a" / "csrc"
     src.mkdir(parents=True)
@@ -39,14 +47,18 @@ def stub(tmp_path_factory):
     subprocess.run(["g++", "-std=c++17", "-shared", "-fPIC", "-o", str(out), str(src / "stub.cpp"), str(src / "sequence.cpp")],
                    check=True)
     lib = ctypes.CDLL(str(out))
-    lib.stub_calls.restype = ctypes.c_char_p
+    lib.stub_calls.restype = lib.stub_details.restype = ctypes.c_char_p
     return lib
+
+
+DISPATCH_PADS, COMBINE_PADS, COND = 0xD0, 0xC0, 0xCD
 
 
 def _run(lib, name, steps, fail="", ep=1, **fields):
     context, call, report = _native.LayerContext(), _native.LayerCall(), (ctypes.c_int32 * 2)()
     context.ep, context.e_local, context.T_max = ep, 4, 64
-    call.T = 64
+    context.dispatch_pads, context.combine_pads = DISPATCH_PADS, COMBINE_PADS
+    call.T, call.cond = 64, COND
     for key, value in fields.items():
         setattr(call, key, value)
     lib.stub_reset(fail.encode())
@@ -97,12 +109,51 @@ def test_order_parts_and_failures(stub, name, table, want):
     # barriers appear with several ranks only, and count as launches
     rc, calls, report = _run(stub, name, every, ep=2)
     assert [c for c in calls if c != "dm_barrier"] == want and calls.count("dm_barrier") >= 2 and report == [len(calls), 0]
+    assert sum([_run(stub, name, bit, ep=2)[1] for bit in table.values()], []) == calls
     # a failing call ends the sequence, and its step is named
     for i, fail in enumerate(want):
         if fail in want[:i]:
             continue
         rc, calls, report = _run(stub, name, every, fail=fail)
         assert rc == 7 and calls == want[:i + 1] and report[0] == i and report[1] in table.values()
+
+
+# Two ranks: every call with its predicate ("?": only where the planner's decision on this layer says so), and at which pads
+# the ranks meet.  Peers read what a barrier stands behind (published rows, expert outputs, their gradients), or have read it
+# before the next call overwrites it (the closing one); the two of the recompute block are predicated as it is.
+TWO_RANKS = {
+    "dm_bf16_forward": "publish barrier:dispatch route plan_fwd_bf16 cond_copy? gemm_fprop_dispatch swiglu_fwd gemm_fprop "
+                       "barrier:combine scale_and_sum?",
+    "dm_bf16_backward": "plan_bwd_bf16 cond_copy? barrier:dispatch? gemm_fprop_dispatch? swiglu_fwd gemm_fprop? "
+                        "barrier:combine? cond_copy? broadcast_and_scale_select? barrier:combine gemm_dgrad_dispatch gemm_wgrad "
+                        "swiglu_bwd gemm_dgrad gemm_wgrad barrier:dispatch scale_and_sum",
+    "dm_mxfp8_forward": "publish barrier:dispatch route_counted plan_fwd_blockscaled cond_copy? quant_mxfp8_rowcol_gather_at "
+                        "gemm_blockscaled_counted swiglu_fwd_quant_mxfp8_rowcol_at gemm_blockscaled_counted barrier:combine "
+                        "scale_and_sum?",
+    "dm_mxfp8_backward": "plan_bwd_blockscaled cond_copy? barrier:dispatch? quant_mxfp8_rowcol_gather_at? "
+                         "gemm_blockscaled_counted? swiglu_fwd_quant_mxfp8_rowcol_at? gemm_blockscaled_counted? "
+                         "barrier:combine? cond_copy? broadcast_and_scale_select? barrier:combine quant_mxfp8_rowcol_gather_at "
+                         "gemm_blockscaled_dgrad_counted gemm_blockscaled_wgrad_compact swiglu_bwd_quant_mxfp8_at "
+                         "gemm_blockscaled_dgrad_counted gemm_blockscaled_wgrad_compact barrier:dispatch scale_and_sum",
+}
+
+
+@pytest.mark.parametrize("name", sorted(TWO_RANKS))
+def test_barriers_and_predicates_with_two_ranks(stub, name):
+    table = _call.FWD if name.endswith("forward") else _call.BWD
+    score = ctypes.c_float()
+    options = dict(grad_scores=ctypes.addressof(score), keep_h3=1)
+
+    def shown(steps):
+        _run(stub, name, steps, ep=2, **options)
+        out = []
+        for call, pads, cond in (entry.split(",") for entry in stub.stub_details().decode().split()):
+            where = {0: "", DISPATCH_PADS: ":dispatch", COMBINE_PADS: ":combine"}[int(pads)]
+            out.append(call.removeprefix("dm_") + where + {0: "", COND: "?"}[int(cond)])
+        return out
+
+    assert shown(sum(table.values())) == TWO_RANKS[name].split()
+    assert sum([shown(bit) for bit in table.values()], []) == TWO_RANKS[name].split()
 
 
 def test_options_of_the_bf16_sequences(stub):
