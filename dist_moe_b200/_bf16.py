@@ -51,6 +51,35 @@ class _Call(CallState):
             self.T, self.size, self.max_rows = T, size, min(size, state.capacity_rows)
         super().__init__(fields)
 
+    def saved(self) -> list[torch.Tensor]:
+        """The state list of the registered operators, as views of the buffer."""
+        at, words, halves = self.at, self.buf, self.buf.view(torch.int32)
+
+        def piece(name: str, of: torch.Tensor, size: int, first: int = 0) -> torch.Tensor:
+            start = at[name] // size
+            return of[start + first:start + self.fields[name][1]]
+
+        rstd = self.rstd if self.rstd is not None else torch.empty(0, dtype=torch.float32, device=words.device)
+        return [piece("counts", halves, 4), piece("bwd", words, 8), piece("fwd", words, 8), piece("sct", words, 8),
+                piece("per_rank", halves, 4), piece("offsets", halves, 4, self.fields["counts"][1]),
+                words[at["need"] // 8:].view(torch.uint8)[:1], piece("fwd_state", words, 8), rstd]
+
+    @staticmethod
+    def from_saved(state, tensors: list[torch.Tensor], T: int):
+        """The call whose ``saved`` tensors these are, or None: they may be an operator's, or hooks have put them elsewhere."""
+        c = _Call(state, T)
+        total, storage = c._place() // 8, tensors[7].untyped_storage()
+        if storage.nbytes() != 8 * total:
+            return None
+        at, base = c.at, storage.data_ptr()
+        places = (at["counts"], at["bwd"], at["fwd"], at["sct"], at["per_rank"], at["offsets"] + 4 * state.e_local, at["need"],
+                  at["fwd_state"])
+        if any(t.data_ptr() != base + place for t, place in zip(tensors, places)):
+            return None
+        c.adopt(tensors[7].as_strided((total,), (1,), 0))
+        c.rstd = tensors[8] if tensors[8].numel() else None
+        return c
+
 
 def _arguments(state, c: _Call, x, ids, scores, w13, w2, options: ExecutionOptions, scratch_only: bool):
     k = arguments(state, c, x, ids, scores, options)
@@ -287,14 +316,16 @@ class _RegisteredBf16Function(torch.autograd.Function):
         state = context._state
         clip = options.swiglu_clip_stats_out_3
         ctx.context, ctx.options = context, options
-        ctx.direct = clip is None and _plain_execution(x, ids, scores, w13_param, w2_param)
-        if ctx.direct:
+        if clip is None and _plain_execution(x, ids, scores, w13_param, w2_param):
             cfg = context.config
             w13 = w13_param.detach().reshape(state.e_local, 2 * cfg.intermediate_dim, cfg.hidden_dim)
             w2 = w2_param.detach().reshape(state.e_local, cfg.hidden_dim, cfg.intermediate_dim)
             with span("dist_moe::bf16_forward"):
                 out, call = forward_impl(state, x.detach().contiguous(), ids, scores.detach(), w13, w2, options, True)
-            ctx.save_for_backward(ids, scores, w13_param, w2_param, call.buf, call.rstd)
+            # What a call saves must not depend on the way it goes where saved-tensor hooks look at it: activation
+            # checkpointing compares a forward with its repetition, which may run under other modes.
+            hooked = torch._C._autograd._top_saved_tensors_default_hooks(False) is not None
+            ctx.save_for_backward(ids, scores, w13_param, w2_param, *(call.saved() if hooked else (call.buf, call.rstd)))
             return out
         rms = _rmsnorm_args(options.experts_output_postprocess)
         head = (x.detach().contiguous(), ids, scores.detach(), w13_param.detach(), w2_param.detach(), *rms,
@@ -322,21 +353,24 @@ class _RegisteredBf16Function(torch.autograd.Function):
             owners = options.wgrad_parameter_owners or (None, None)
             destinations = (_wgrad_destination(w13_param, (e_local, 2 * F, D), options, cfg, owners[0])[0],
                             _wgrad_destination(w2_param, (e_local, D, F), options, cfg, owners[1])[0])
-        if ctx.direct:
-            call = _Call(state, ids.shape[0]).adopt(st[0])
-            call.rstd = st[1]
-            # a backward that is itself differentiated goes through the operators, which refuse it
-            if not torch.is_grad_enabled() and _plain_execution(grad_out, ids, scores, w13_param, w2_param, st[0]):
-                if context._closed:
-                    raise RuntimeError(f"distributed MoE context {context._context_id} is not live")
-                w13, w2 = w13_param.detach().reshape(e_local, 2 * F, D), w2_param.detach().reshape(e_local, D, F)
-                with torch.cuda.device(state.device), span("dist_moe::bf16_backward"):
-                    gx, gs, g13, g2 = backward_impl(state, call, grad_out.shape, ids, scores.detach(), w13, w2, w13_param,
-                                                    w2_param, grad_out.contiguous(), options, needs, destinations)
-                if options.inplace_wgrad_accum:
-                    torch.autograd.graph.increment_version(destinations)  # as the operator's mutated arguments
-                return gx, None, gs, g13, g2, None, None
-            st = _ops._pack_bf16_state(call, ids.device)
+        whole = None
+        if len(st) == 2:
+            whole = _Call(state, ids.shape[0]).adopt(st[0])
+            whole.rstd = st[1]
+        # a backward that is itself differentiated goes through the operators, which refuse it
+        if not torch.is_grad_enabled() and _plain_execution(grad_out, ids, scores, w13_param, w2_param, st[0]):
+            if context._closed:
+                raise RuntimeError(f"distributed MoE context {context._context_id} is not live")
+            call = whole or _ops._unpack_bf16_state(state, st, ids.shape[0])
+            w13, w2 = w13_param.detach().reshape(e_local, 2 * F, D), w2_param.detach().reshape(e_local, D, F)
+            with torch.cuda.device(state.device), span("dist_moe::bf16_backward"):
+                gx, gs, g13, g2 = backward_impl(state, call, grad_out.shape, ids, scores.detach(), w13, w2, w13_param,
+                                                w2_param, grad_out.contiguous(), options, needs, destinations)
+            if options.inplace_wgrad_accum:
+                torch.autograd.graph.increment_version(destinations)  # as the operator's mutated arguments
+            return gx, None, gs, g13, g2, None, None
+        if whole is not None:
+            st = whole.saved()
         rms = _rmsnorm_args(options.experts_output_postprocess)
         tail = (rms[1], rms[2], rms[3], rms[4], rms[5], rms[7], rms[8])
         _ops.NEEDS_HINT.append(needs)

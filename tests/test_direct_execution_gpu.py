@@ -26,7 +26,7 @@ class _Watch(TorchDispatchMode):
 
 
 def _run(mode, *, ids=torch.int64, scores=torch.float32, accumulate=False, grad=torch.bfloat16, slots=None, norm=False,
-         clamped=False, frozen=(), wrap=None):
+         clamped=False, frozen=(), wrap=None, two_layers=False):
     g = torch.Generator().manual_seed(3)
     rnd = lambda *s: torch.randn(*s, generator=g)  # noqa: E731
     x = rnd(T, D).bfloat16().to(DEV).requires_grad_("x" not in frozen)
@@ -39,7 +39,7 @@ def _run(mode, *, ids=torch.int64, scores=torch.float32, accumulate=False, grad=
     if slots:
         extra["activation_slot_capacity_factor"] = slots
     cfg = dm.Config(max_num_local_input_tokens=T, hidden_dim=D, intermediate_dim=F, top_k=K, num_experts=E,
-                    max_moe_layers_per_activation_slot=1, wgrad_dtype=grad, **extra)
+                    max_moe_layers_per_activation_slot=2 if two_layers else 1, wgrad_dtype=grad, **extra)
     post = dm.RMSNormPostprocess(eps=1e-6, norm_output_dtype=torch.float32, output_dtype=torch.bfloat16) if norm else None
     options = dm.ExecutionOptions(inplace_wgrad_accum=accumulate, experts_output_postprocess=post)
     if accumulate:
@@ -130,3 +130,26 @@ def test_a_differentiated_backward_is_refused():
             gx.float().sum().backward()
     finally:
         context.close()
+
+
+@pytest.mark.parametrize("form", [dict(), dict(slots=1.0), dict(norm=True)], ids=["plain", "saved", "norm"])
+@pytest.mark.parametrize("watched", ["forward", "backward", "both"])
+def test_checkpointing_under_modes(form, watched):
+    """Non-reentrant checkpointing compares the tensors that a forward and its repetition save, also where a mode covers only
+    one of them."""
+    from torch.utils.checkpoint import checkpoint
+
+    plain = _run(contextlib.nullcontext(), **form)
+    stack = contextlib.ExitStack()
+
+    def call_checkpointed(call, x, s):
+        with _Watch() if watched in ("forward", "both") else contextlib.nullcontext():
+            out = checkpoint(call, x, s, use_reentrant=False)
+        if watched in ("backward", "both"):
+            stack.enter_context(_Watch())
+        return out
+
+    with stack:
+        got = _run(contextlib.nullcontext(), wrap=call_checkpointed, two_layers=True, **form)
+    for a, b in zip(got, plain):
+        assert torch.equal(a, b)
