@@ -21,7 +21,7 @@ from typing import Any
 import torch
 
 from . import _native as nat
-from ._call import BWD, FWD, FWD_ALL, CallState, arguments, launch, observed, span
+from ._call import BWD, FWD, FWD_ALL, CallState, arguments, launch, observed, recorded, span
 from ._execution import ExecutionOptions, RMSNormPostprocess
 
 
@@ -294,11 +294,11 @@ def _rmsnorm_args(post):
 
 def _plain_execution(*tensors) -> bool:
     """Nothing acts on this call's operators: no tracing or fake tensors, no dispatch or function mode, no functorch
-    level.  The registered operators' bodies can then run without the dispatcher, which costs a small layer more than its
+    level, no recorder (profiler, execution trace).  The registered operators' bodies can then run without the dispatcher, which costs a small layer more than its
     launches."""
     if torch.compiler.is_compiling():  # first: a tracer of Python code must not meet the calls below
         return False
-    return (torch._C._len_torch_dispatch_stack() == 0 and torch._C._len_torch_function_stack() == 0
+    return (not recorded() and torch._C._len_torch_dispatch_stack() == 0 and torch._C._len_torch_function_stack() == 0
             and torch._ops._len_torch_dispatch_stack_pre_dispatch() == 0
             and torch._C._functorch.peek_interpreter_stack() is None and torch._C._get_tracing_state() is None
             and all(type(t) is torch.Tensor or type(t) is torch.nn.Parameter for t in tensors))
@@ -320,8 +320,7 @@ class _RegisteredBf16Function(torch.autograd.Function):
             cfg = context.config
             w13 = w13_param.detach().reshape(state.e_local, 2 * cfg.intermediate_dim, cfg.hidden_dim)
             w2 = w2_param.detach().reshape(state.e_local, cfg.hidden_dim, cfg.intermediate_dim)
-            with span("dist_moe::bf16_forward"):
-                out, call = forward_impl(state, x.detach().contiguous(), ids, scores.detach(), w13, w2, options, True)
+            out, call = forward_impl(state, x.detach().contiguous(), ids, scores.detach(), w13, w2, options, True)
             # What a call saves must not depend on the way it goes where saved-tensor hooks look at it: activation
             # checkpointing compares a forward with its repetition, which may run under other modes.
             hooked = torch._C._autograd._top_saved_tensors_default_hooks(False) is not None
@@ -363,7 +362,7 @@ class _RegisteredBf16Function(torch.autograd.Function):
                 raise RuntimeError(f"distributed MoE context {context._context_id} is not live")
             call = whole or _ops._unpack_bf16_state(state, st, ids.shape[0])
             w13, w2 = w13_param.detach().reshape(e_local, 2 * F, D), w2_param.detach().reshape(e_local, D, F)
-            with torch.cuda.device(state.device), span("dist_moe::bf16_backward"):
+            with torch.cuda.device(state.device):
                 gx, gs, g13, g2 = backward_impl(state, call, grad_out.shape, ids, scores.detach(), w13, w2, w13_param,
                                                 w2_param, grad_out.contiguous(), options, needs, destinations)
             if options.inplace_wgrad_accum:

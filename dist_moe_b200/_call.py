@@ -11,6 +11,7 @@ backward of 16 tokens (D = F = 256, 8 experts) 656 -> 301 us, of 1531 tokens (D 
 from __future__ import annotations
 
 import ctypes
+import os
 
 import torch
 from torch.profiler import record_function
@@ -36,11 +37,26 @@ _TIMED = {
 _REPORT = ctypes.c_int32 * 2
 
 
+def _recorder_query():
+    """``at::hasCallbacks()`` of ATen/record_function.h, which Python does not bind: whether anything records operators and
+    ranges on this thread.  That is the profiler, but also an ``ExecutionTraceObserver`` or NVTX emission, which
+    ``torch.autograd._profiler_enabled`` does not know of.  0.1 us a call; where the symbol is missing, always."""
+    try:
+        query = ctypes.PyDLL(os.path.join(os.path.dirname(torch.__file__), "lib", "libtorch_cpu.so"))._ZN2at12hasCallbacksEv
+    except (OSError, AttributeError):
+        return lambda: True
+    query.restype, query.argtypes = ctypes.c_bool, []
+    return query
+
+
+recorded = _recorder_query()
+
+
 def observed() -> bool:
     """Someone wants to see the parts of a pass."""
     from . import _bf16
 
-    return _bf16.PROFILE is not None or torch.autograd._profiler_enabled()
+    return _bf16.PROFILE is not None or recorded()
 
 
 class _NoSpan:
@@ -53,7 +69,7 @@ class _NoSpan:
 
 def span(name: str):
     """A profiler range with the reference's name (dist_moe/api.py:1979-2443), free where nothing records."""
-    return record_function(name) if torch.autograd._profiler_enabled() else _NoSpan()
+    return record_function(name) if recorded() else _NoSpan()
 
 
 def launch(fn, names: dict, state, k, steps: int) -> None:
