@@ -334,6 +334,8 @@ int dm_gemm_wgrad(dm_operand dy, dm_operand x, void* dw, int out_is_fp32, int ac
  *       and, when C is given, h1 = [gate | up] in the canonical (not interleaved) column order.
  * Every expert's row range must start on a multiple of 128 (routing with m_multiple_of = 128).  Otherwise the status is
  * set to DM_STATUS_CAPACITY_EXCEEDED and that expert's results are not defined; the MXFP8 and the swapped form leave it out.
+ * The device offset of `a` must be a multiple of 128, that of `sfa` a multiple of 16 (a multiple of 128 loads faster in the
+ * MXFP8 forms).  sfa.bytes smaller than the layout of max_rows counts as not told.
  * ------------------------------------------------------------------------- */
 int dm_gemm_blockscaled(int format, dm_operand a, dm_operand sfa, const void* w, const void* sfb, dm_operand c,
                         dm_operand h2, const int64_t* scatter_ptrs, dm_operand row_scale_inv,
@@ -345,7 +347,7 @@ int dm_gemm_blockscaled(int format, dm_operand a, dm_operand sfa, const void* w,
  * group).  MXFP8: the work is sized by real rows rounded up to 32.  Rows of a dense C past them are computed from A (up to
  * the next multiple of 32) or set to zero, what the product gives for the zero rows that pad a group; h2 and scattered
  * rows past the count are not written.  Runs on pairs of neighbouring SMs: an odd num_sms is used down to the next even
- * number, 1 takes one pair.  Device offsets of `a` and `sfa` must be multiples of 128.  NVFP4: whole groups. */
+ * number, 1 takes one pair.  NVFP4: whole groups. */
 int dm_gemm_blockscaled_counted(int format, dm_operand a, dm_operand sfa, const void* w, const void* sfb, dm_operand c,
                                 dm_operand h2, const int64_t* scatter_ptrs, dm_operand row_scale_inv,
                                 const float* expert_scale_inv, const int32_t* expert_offsets,

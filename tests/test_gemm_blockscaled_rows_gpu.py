@@ -147,3 +147,39 @@ def test_groups_that_are_not_padded_are_left_out(swapped, fmt, counted):
     for e, rows in ((0, 100), (1, 32), (3, 128)):
         at = torch.arange(off[e], off[e] + rows)
         _close(got[at], da[at] @ dw[e].T, f"expert {e}")
+
+
+@pytest.mark.parametrize("offset", [16, 112, 128, 656])
+@pytest.mark.parametrize("form", ["forward", "swiglu", "input gradient"])
+def test_scales_at_any_sixteen_bytes(form, offset):
+    """The rows' scales may start at any multiple of 16 bytes, and their extent need not be told: the entry points' older
+    kernel copied them by address.  Same bits as from the start of an allocation."""
+    nat = _nat()
+    counts, K, N = [300, 0, 33, 128], 1280, 256
+    E, off, real, R, (qa, sa, _, _), (qw, sw, _, _), offs, cnts = _operands(nat, 0, counts, K, N, 41)
+    if form == "input gradient":
+        w = (torch.randn(E, K, N, device=DEV) * 0.05).bfloat16()
+        qw, _, sw, _ = _tile32_weight(nat, w)
+    n = sa.numel()
+    wide = torch.full((n + 1024,), 0x55, dtype=torch.uint8, device=DEV)
+    wide[offset:offset + n] = sa.view(torch.uint8).reshape(-1)
+    at = torch.tensor([offset], dtype=torch.int64, device=DEV)
+    results = []
+    for scales in (_op(nat, sa), nat.Operand(wide.data_ptr(), wide.numel(), at.data_ptr()), nat.Operand(wide.data_ptr(), 0, at.data_ptr())):
+        status = torch.zeros(8, dtype=torch.int32, device=DEV)
+        out = torch.full((R, N // 2 if form == "swiglu" else N), 5.0, device=DEV, dtype=torch.bfloat16)
+        none, tail = _op(nat, None), (None, 0, status.data_ptr(), nat.stream_ptr())
+        if form == "input gradient":
+            rc = nat.lib.dm_gemm_blockscaled_dgrad(_op(nat, qa), scales, qw.data_ptr(), sw.data_ptr(), _op(nat, out), None,
+                                                   offs.data_ptr(), E, R, N, K, *tail)
+        else:
+            swiglu = form == "swiglu"
+            rc = nat.lib.dm_gemm_blockscaled(0, _op(nat, qa), scales, qw.data_ptr(), sw.data_ptr(), none if swiglu else _op(nat, out),
+                                             _op(nat, out) if swiglu else none, None, none, None, offs.data_ptr(), E, R, N, K,
+                                             int(swiglu), 0, 1.0, 0.0, *tail)
+        nat.check(rc, form)
+        torch.cuda.synchronize()
+        assert status[0].item() == 0, status.tolist()
+        results.append(out)
+    assert torch.equal(results[0], results[1]) and torch.equal(results[0], results[2])
+    assert bool((results[0][real.to(DEV)] != 5.0).any())
