@@ -244,8 +244,8 @@ class ContextState:
     # ---- what the native call sequences read ----------------------------------
     def native_layer(self):
         """Reference to this context's ``dm_layer_context`` (everything it names lives as long as the context)."""
-        ref = getattr(self, "_native_layer", None)
-        if ref is None:
+        c = getattr(self, "_native_layer", None)
+        if c is None:
             cfg, c = self.config, nat.LayerContext()
             c.arena, c.arena_bytes = self.arena.data_ptr(), self.arena.numel()
             for name in ("dispatch", "combine", "routing"):
@@ -258,7 +258,7 @@ class ContextState:
                 setattr(c, name, getattr(self, name).data_ptr())
             c.route_workspace_words = self.route_workspace_words
             c.T_max, c.D, c.F = cfg.max_num_local_input_tokens, cfg.hidden_dim, cfg.intermediate_dim
-            c.slot_bytes, c.capacity_rows, c.barrier_timeout_ns = self.slot_bytes, self.capacity_rows, BARRIER_TIMEOUT_NS
+            c.slot_bytes, c.capacity_rows = self.slot_bytes, self.capacity_rows
             c.rank, c.ep, c.K, c.E, c.e_local = self.rank, self.ep, cfg.top_k, cfg.num_experts, self.e_local
             c.num_slots, c.num_sms = self.num_slots, self.num_sms
             c.clamped, c.alpha, c.limit = cfg.activation == "swiglu_clamped", cfg.swiglu_alpha, cfg.swiglu_limit
@@ -266,8 +266,9 @@ class ContextState:
                 from ._blockscaled import planner_storage
 
                 c.storage[:] = planner_storage(cfg.block_scaled.format)
-            ref = self._native_layer = ctypes.byref(c)
-        return ref
+            self._native_layer = c
+        c.barrier_timeout_ns = BARRIER_TIMEOUT_NS  # as ``barrier``: the value of this call
+        return ctypes.byref(c)
 
     def arena_at(self, offset_address: int) -> nat.Operand:
         """Operand whose byte offset inside the arena is the device int64 at ``offset_address``."""
