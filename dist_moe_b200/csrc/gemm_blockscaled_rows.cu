@@ -16,7 +16,7 @@
 //   * a stage is 128 bytes of K per row;
 //   * scales are stored in 128-row x 4-column atoms of 512 bytes (row r, column c at (r%32)*16 + (r/32)*4 + c), the source
 //     shape of tcgen05.cp 32x128b.warpx4, which lands an atom in four TMEM columns of 32 rows each.  A CTA needs the atom of
-//     its own 128 weight columns and those of all rows of the tile (two; three where a tile starts inside an atom).
+//     its own 128 weight columns and those of all rows of the tile (at most two, see row_tiles.cuh).
 //     A tile that starts at row 32 q of an atom names column q (0 or 2) as its scale address;
 //   * the warp that issues the MMAs copies a stage's atoms right before them: copies and MMAs of one thread execute in order,
 //     and the copies hide behind the MMAs before them (512 cycles a stage with and without);
@@ -72,14 +72,6 @@ struct BrParams {
   int h_atoms;
   ActParams act;
 };
-
-// Row tiles of an expert: one of its rows rounded up to 32, or several nearly equal ones that start at multiples of 64 rows,
-// because the MMA takes its scale columns (32 rows each) from an even column on.
-__device__ __forceinline__ int br_rows_per_tile(int rows) {
-  if (rows <= kRwMaxN) return rw_rows_per_tile(rows);
-  const int nt = rw_row_tiles(rows);
-  return ((rows + nt - 1) / nt + 63) & ~63;
-}
 
 struct BrTile {
   int e, pair, row0, rows, n, last;  // rows: real rows of the tile, n: the MMA's N (rows rounded up to 32)
@@ -178,7 +170,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kBrThreads, 1)
         if (count > 0 && s_off[e + 1] > s_off[e] && !bs_group_aligned(s_off[e]))
           set_status(p.status, kCapacityExceeded, -1, e, s_off[e]);  // groups must be 128-padded
         const int nt = rw_row_tiles(rows);
-        const int per = br_rows_per_tile(rows);
+        const int per = bs_rows_per_tile(rows);
         s_per[e] = static_cast<uint16_t>(per);
         tiles = nt * m_pairs;
         if (nt > 0) box = max(box, rw_box_index(per));
@@ -205,10 +197,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kBrThreads, 1)
   tcgen05_fence_after();
   const uint32_t tmem_base = uniform(tmem_base_slot);
   const int total_tiles = uniform(s_tile_start[p.e_local]);
-  // Ring: stages as large as the launch's largest tile needs, as many as shared memory and the scale columns allow.  Tiles of
-  // at most 128 rows start with an atom (only experts of more than 256 rows have several tiles) and touch no second one.
+  // Ring: stages as large as the launch's largest tile needs, as many as shared memory and the scale columns allow.
   const int n_max = 2 * rw_box_rows(uniform(s_box));
-  const uint32_t x_groups = n_max <= 128 ? 1 : 3;  // most 128-row groups that a tile's rows touch
+  const uint32_t x_groups = bs_tile_atoms(n_max);
   const uint32_t slot_cols = (1 + x_groups) * 4;  // scale columns of a stage slot
   const uint32_t sf_at = kBrWBytes + static_cast<uint32_t>(n_max / 2) * 128;  // weight atoms, then the rows' atoms
   const uint32_t stage_bytes = sf_at + (((1 + x_groups) * kSfBytes + 1023) & ~1023u);
@@ -326,8 +317,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kBrThreads, 1)
           const uint32_t w_addr = ring + stage * stage_bytes;
           const uint32_t w_lo = ((w_addr & 0x3ffffu) >> 4) | kLbo, x_lo = w_lo + (kBrWBytes >> 4);
           const uint32_t sf_lo = sf_desc_lo(w_addr + sf_at);
-          const uint32_t sfw_t = sf_tmem + stage * slot_cols;
-          const uint32_t sfx_t = sfw_t + 4u;
+          // the weights' columns come last: a tile that starts at its atom's third column stays inside the slot
+          const uint32_t sfx_t = sf_tmem + stage * slot_cols;
+          const uint32_t sfw_t = sfx_t + 4u * x_groups;
           const uint32_t empty = empty0 + stage * 8;
           if (++stage == stages) {
             stage = 0;
@@ -338,7 +330,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kBrThreads, 1)
             tmem_cp_sf_lo_pair(sfw_t, sf_lo);
             tmem_cp_sf_lo_pair(sfx_t, sf_lo + kSfAtomWords);
             if (x_atoms > 1) tmem_cp_sf_lo_pair(sfx_t + 4, sf_lo + 2 * kSfAtomWords);
-            if (x_atoms > 2) tmem_cp_sf_lo_pair(sfx_t + 8, sf_lo + 3 * kSfAtomWords);
 #pragma unroll
             for (int j = 0; j < 4; ++j)
               umma_mxf8_lo_pair(d_tmem, w_lo + j * w_step, x_lo + j * x_step, kDescHi, idesc[j], sfw_t, sfx_t + q,

@@ -72,4 +72,14 @@ DM_HOST_DEVICE int bs_group_rows(int off, int next, int count) {
   return rows > 0 && bs_group_aligned(off) ? rows : 0;
 }
 
+// Row tiles of an expert in the MXFP8 pair kernel: one of its rows rounded up to 32, or several nearly equal ones that start
+// at multiples of 64 rows, because the MMA takes its scale columns (32 rows each) from an even column on.
+DM_HOST_DEVICE constexpr int bs_rows_per_tile(int rows) {
+  return rows <= kRwMaxN ? rw_rows_per_tile(rows) : ((rows + rw_row_tiles(rows) - 1) / rw_row_tiles(rows) + 63) & ~63;
+}
+
+// Scale atoms (128 rows) that the rows of a tile touch at most, in a launch whose largest tile has `n_max` rows: only experts
+// of more than 256 rows have several tiles, of 192 or 256 rows each, and those of 192 that start inside an atom end with one.
+DM_HOST_DEVICE constexpr int bs_tile_atoms(int n_max) { return n_max <= 128 ? 1 : 2; }
+
 }  // namespace dm
