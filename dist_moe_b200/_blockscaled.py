@@ -259,9 +259,10 @@ def _workspace(state):
 # the MMA's N side in steps of 32, two CTAs per SM); above it, for NVFP4, a 128-row tile is mostly real rows and the 128 x 256
 # kernel wins: whole layer on one B200, swapped / 128 x 256, us: 32 experts x 7168 x 2048 at 48 rows per expert 226 / 243, at
 # 64 237 / 247, at 96 274 / 255; 64 experts x 2048 x 2048 at 48 222 / 232, at 56 235 / 233, at 64 265 / 236.  MXFP8 has rows on
-# the N side of CTA pairs at every size, and quantises h2 on the way out: swapped / pairs, 128 experts x 2816 x 2816, 1 token
-# 99 / 82, 16 tokens (hot experts) 244 / 220, 256 tokens 580 / 561, 768 tokens 599 / 558; 32 x 4096 x 1536, 8 tokens 121.6 /
-# 120.8, 192 tokens 162 / 160.  ``None`` keeps the per-format value.
+# the N side of CTA pairs at every size, in this form too (which here only keeps h2's quantiser apart).  While it had a swapped
+# form on single CTAs, swapped / pairs: 128 experts x 2816 x 2816, 1 token 99 / 82, 16 tokens (hot experts) 244 / 220, 256 tokens
+# 580 / 561, 768 tokens 599 / 558; 32 x 4096 x 1536, 8 tokens 121.6 / 120.8, 192 tokens 162 / 160.  ``None`` keeps the
+# per-format value.
 SWAPPED_MAX_ROWS_PER_EXPERT = None
 _SWAPPED_MAX_ROWS = {BlockScaledFormat.NVFP4: 48, BlockScaledFormat.MXFP8_E4M3: 0}
 

@@ -269,8 +269,3 @@ class ContextState:
             self._native_layer = c
         c.barrier_timeout_ns = BARRIER_TIMEOUT_NS  # as ``barrier``: the value of this call
         return ctypes.byref(c)
-
-    def arena_at(self, offset_address: int) -> nat.Operand:
-        """Operand whose byte offset inside the arena is the device int64 at ``offset_address``."""
-        arena = self.arena
-        return nat.Operand(arena.data_ptr(), arena.numel(), offset_address)

@@ -64,6 +64,7 @@ struct BrParams {
   int* status;
   int64_t sfw_group_lines;
   int e_local, max_rows, N, Kw, k_iters, x_col_atoms, w_col_atoms;
+  int pad_rows;  // rows of a dense C past an expert's count are written too
   // SwiGLU epilogue that writes h2 as MXFP8 rows (E4M3 bytes + blocked E8M0 scales) instead of bf16
   uint8_t* hq_base;
   const int64_t* hq_off;
@@ -399,6 +400,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kBrThreads, 1)
         if (kSwiglu ? p.c_base == nullptr : false) return 0;
         if (!kSwiglu && p.scatter_ptrs != nullptr) return r < t.rows ? static_cast<uint64_t>(p.scatter_ptrs[t.row0 + r]) : 0;
         // dense rows up to the next multiple of 32 are computed (padding rows hold zeros)
+        if (!kSwiglu && !p.pad_rows && r >= t.rows) return 0;
         return reinterpret_cast<uint64_t>(p.c_base) + c_off + static_cast<uint64_t>(t.row0 + r) * p.N * 2;
       };
       auto row_scale = [&](int b) -> float { return row_inv != nullptr ? row_inv[t.row0 + b * 32 + lane] : 1.0f; };
@@ -556,7 +558,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kBrThreads, 1)
         scale_a = scale_n;
       }
       if (held) hand_back();
-      if (!kSwiglu && dense && t.last) {
+      if (!kSwiglu && dense && p.pad_rows && t.last) {
         // rows between the last multiple of 32 and the end of the padded group: zeros, as the product of their zero rows
         const int col = m_blk * kBrBM + (lane & 15) * 8;
         if (col + 8 <= p.N)
@@ -590,6 +592,11 @@ int nvfp4_forward(const dm_operand& a, const dm_operand& sfa, const void* w, con
                   const float* expert_scale_inv, const int32_t* expert_offsets, int e_local, int64_t max_rows, int64_t N,
                   int64_t Kd, int swiglu_interleaved, const ActParams& act, const int* cond, int num_sms, int* status,
                   cudaStream_t st);
+int mxfp8_forward(const dm_operand& a, const dm_operand& sfa, const void* w, const void* sfb, const dm_operand& c,
+                  const dm_operand& h2, const int64_t* scatter_ptrs, const dm_operand& row_scale_inv,
+                  const float* expert_scale_inv, const int32_t* expert_offsets, const int32_t* expert_counts, int e_local,
+                  int64_t max_rows, int64_t N, int64_t Kd, int swiglu_interleaved, const ActParams& act, bool pad_rows,
+                  const int* cond, int num_sms, int* status, cudaStream_t st);
 
 template <int kDgrad, bool kSwiglu>
 static int br_launch(const BrParams& p, int num_sms, cudaStream_t st) {
@@ -670,6 +677,30 @@ static int br_setup(BrParams& p, const dm_operand& x, const dm_operand& sfx, con
   return kRcOk;
 }
 
+// The MXFP8 forward of dm_gemm_blockscaled and of dm_gemm_blockscaled_swapped (arguments checked there).
+int dm::mxfp8_forward(const dm_operand& a, const dm_operand& sfa, const void* w, const void* sfb, const dm_operand& c,
+                      const dm_operand& h2, const int64_t* scatter_ptrs, const dm_operand& row_scale_inv,
+                      const float* expert_scale_inv, const int32_t* expert_offsets, const int32_t* expert_counts, int e_local,
+                      int64_t max_rows, int64_t N, int64_t Kd, int swiglu_interleaved, const ActParams& act, bool pad_rows,
+                      const int* cond, int num_sms, int* status, cudaStream_t st) {
+  BrParams p{};
+  int rc = br_setup(p, a, sfa, sfb, Kd, Kd / 32, expert_offsets, expert_counts, e_local, max_rows, N, cond, status);
+  if (rc != kRcOk) return rc;
+  rc = encode_2d_u8(&p.tm_w, w, static_cast<int64_t>(e_local) * N, Kd, kBrBM);
+  if (rc != kRcOk) return rc;
+  p.c_off = c.offset;
+  p.h2_off = h2.offset;
+  p.c_base = static_cast<uint8_t*>(c.base);
+  p.h2_base = static_cast<uint8_t*>(h2.base);
+  p.row_inv_base = static_cast<const uint8_t*>(row_scale_inv.base);
+  p.row_inv_off = row_scale_inv.offset;
+  p.expert_inv = expert_scale_inv;
+  p.scatter_ptrs = scatter_ptrs;
+  p.act = act;
+  p.pad_rows = pad_rows;
+  return swiglu_interleaved ? br_launch<0, true>(p, num_sms, st) : br_launch<0, false>(p, num_sms, st);
+}
+
 extern "C" int dm_gemm_blockscaled_counted(int format, dm_operand a, dm_operand sfa, const void* w, const void* sfb,
                                            dm_operand c, dm_operand h2, const int64_t* scatter_ptrs,
                                            dm_operand row_scale_inv, const float* expert_scale_inv,
@@ -691,21 +722,9 @@ extern "C" int dm_gemm_blockscaled_counted(int format, dm_operand a, dm_operand 
   if (fp4)
     return nvfp4_forward(a, sfa, w, sfb, c, h2, scatter_ptrs, row_scale_inv, expert_scale_inv, expert_offsets, e_local, max_rows,
                          N, Kd, swiglu_interleaved, ActParams{clamped, alpha, limit}, cond, num_sms, status, st);
-  BrParams p{};
-  int rc = br_setup(p, a, sfa, sfb, Kd, Kd / 32, expert_offsets, expert_counts, e_local, max_rows, N, cond, status);
-  if (rc != kRcOk) return rc;
-  rc = encode_2d_u8(&p.tm_w, w, static_cast<int64_t>(e_local) * N, Kd, kBrBM);
-  if (rc != kRcOk) return rc;
-  p.c_off = c.offset;
-  p.h2_off = h2.offset;
-  p.c_base = static_cast<uint8_t*>(c.base);
-  p.h2_base = static_cast<uint8_t*>(h2.base);
-  p.row_inv_base = static_cast<const uint8_t*>(row_scale_inv.base);
-  p.row_inv_off = row_scale_inv.offset;
-  p.expert_inv = expert_scale_inv;
-  p.scatter_ptrs = scatter_ptrs;
-  p.act = ActParams{clamped, alpha, limit};
-  return swiglu_interleaved ? br_launch<0, true>(p, num_sms, st) : br_launch<0, false>(p, num_sms, st);
+  return mxfp8_forward(a, sfa, w, sfb, c, h2, scatter_ptrs, row_scale_inv, expert_scale_inv, expert_offsets, expert_counts,
+                       e_local, max_rows, N, Kd, swiglu_interleaved, ActParams{clamped, alpha, limit}, true, cond, num_sms,
+                       status, st);
 }
 
 extern "C" int dm_gemm_blockscaled(int format, dm_operand a, dm_operand sfa, const void* w, const void* sfb,
@@ -774,6 +793,7 @@ extern "C" int dm_gemm_blockscaled_dgrad_counted(dm_operand dy, dm_operand sf_dy
   p.c_base = static_cast<uint8_t*>(c.base);
   p.scatter_ptrs = scatter_ptrs;
   p.Kw = static_cast<int>(Kd);
+  p.pad_rows = 1;
   p.act = ActParams{0, 1.0f, 0.0f};
   return br_launch<1, false>(p, num_sms, static_cast<cudaStream_t>(stream));
 }

@@ -1,6 +1,6 @@
-// Swapped-operand block-scaled grouped GEMM for experts that received few rows (decode).
+// Swapped-operand NVFP4 grouped GEMM for experts that received few rows (decode).
 //
-//   C[r, n] = sum_k  (X[r,k] * sfx[r, k/V]) * (W[e][n,k] * sfw[e][n, k/V])        V = 32 (MXFP8) or 16 (NVFP4)
+//   C[r, n] = sum_k  (X[r,k] * sfx[r, k/16]) * (W[e][n,k] * sfw[e][n, k/16])
 //
 // The 128 x 256 kernel puts an expert's rows on the 128-row M side of tcgen05.mma, so an expert that received 30
 // rows still pays for 128: at decode sizes the tensor pipe, not HBM, bounds the layer.  Here the roles are exchanged:
@@ -10,9 +10,8 @@
 //
 //   * with MMAs this short the issue of tcgen05 instructions counts.  One warp, converged around an elected lane, copies a
 //     stage's scale atoms and issues its MMAs: eight copies and four MMAs of N = 32 take 224 cycles (162 without the copies),
-//     and no barrier stands between them.  With a copier warp of its own a layer took 245 us (MXFP8, 16 tokens, 128 experts x
-//     2816 x 2816) and 207 us (NVFP4, 128 tokens, 32 experts x 7168 x 2048), now 240 and 202.  Two CTAs share an SM, each
-//     with 256 TMEM columns and three stages;
+//     and no barrier stands between them.  With a copier warp of its own a layer of 128 tokens, 32 experts x 7168 x 2048 took
+//     207 us, now 202.  Two CTAs share an SM, each with 256 TMEM columns and three stages;
 //   * a stage = 128 bytes of K: 16 KiB of weights (one TMA box), 4 or 8 KiB of routed rows (32-row boxes),
 //     and the stage's scale atoms of both;
 //   * the rows' scale atom covers 128 rows in four TMEM columns of 32 rows each, so a tile that starts at row
@@ -34,7 +33,7 @@ constexpr int kSwThreads = 224;  // TMA warp, MMA warp, four epilogue warps, acc
 constexpr int kSwTileRows = 64;  // routed rows per tile (the MMA's N), in steps of 32
 constexpr uint32_t kSwWBytes = 128 * 128;            // 16 KiB of weights
 constexpr uint32_t kSwXBytes = kSwTileRows * 128;    // up to 8 KiB of routed rows
-constexpr uint32_t kSwSfBytes = 2048;                // up to 4 atoms per operand
+constexpr uint32_t kSwSfBytes = 4 * 512;             // four scale atoms per operand
 constexpr uint32_t kSwStageBytes = kSwWBytes + kSwXBytes + 2 * kSwSfBytes;  // 28 KiB
 constexpr uint32_t kSwTransposeBytes = 32 * 32 * 2;  // per epilogue warp
 constexpr size_t kSwSmemBytes = kSwStages * kSwStageBytes + 4 * kSwTransposeBytes + 1024;
@@ -53,8 +52,8 @@ struct SwParams {
   const int64_t* row_inv_off;
   const uint8_t* sfx_base;
   const uint8_t* sfw;
-  const uint8_t* row_inv_base;  // fp32 per row (NVFP4 token scale inverse) or null
-  const float* expert_inv;      // fp32 per expert (NVFP4 weight global scale inverse) or null
+  const uint8_t* row_inv_base;  // fp32 per row (token scale inverse) or null
+  const float* expert_inv;      // fp32 per expert (weight global scale inverse) or null
   uint8_t* c_base;
   uint8_t* h2_base;
   const int64_t* scatter_ptrs;
@@ -63,7 +62,7 @@ struct SwParams {
   const int* cond;
   int* status;
   int64_t sfw_group_bytes;
-  int e_local, max_rows, N, k_iters, fp4, swiglu, x_col_atoms, w_col_atoms;
+  int e_local, max_rows, N, k_iters, swiglu, col_atoms;
   ActParams act;
 };
 
@@ -105,7 +104,6 @@ __global__ void __launch_bounds__(kSwThreads, kSwCtasPerSm) blockscaled_swapped_
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   const int m_tiles = p.N >> 7;
-  const int atoms = p.fp4 ? 4 : 1;  // scale atoms per stage and operand
 
   for (int i = threadIdx.x; i <= p.e_local; i += blockDim.x) {
     const int v = p.expert_offsets[i];
@@ -163,13 +161,12 @@ __global__ void __launch_bounds__(kSwThreads, kSwCtasPerSm) blockscaled_swapped_
     int e = 0;
     const int x_line0 = uniform(static_cast<int>((p.x_off ? *p.x_off : 0) >> 7));
     const uint8_t* sfx = p.sfx_base + (p.sfx_off ? *p.sfx_off : 0);
-    const uint32_t sf_bytes = atoms * 512;
     bool ok = true;
     for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
       const SwTile t = sw_decode(tile, e, s_tile_start, s_off, s_cnt, m_tiles);
       const int nq = uniform((t.n_valid + 31) >> 5), row0 = uniform(t.row0), w_row = uniform(t.e * p.N + t.m_blk * 128);
-      const uint8_t* sfw_row = p.sfw + t.e * p.sfw_group_bytes + static_cast<int64_t>(t.m_blk) * p.w_col_atoms * 512;
-      const uint8_t* sfx_row = sfx + static_cast<int64_t>(t.row0 >> 7) * p.x_col_atoms * 512;
+      const uint8_t* sfw_row = p.sfw + t.e * p.sfw_group_bytes + static_cast<int64_t>(t.m_blk) * p.col_atoms * 512;
+      const uint8_t* sfx_row = sfx + static_cast<int64_t>(t.row0 >> 7) * p.col_atoms * 512;
 #pragma unroll 1
       for (int kb = 0; kb < p.k_iters; ++kb) {
         ok = warp_mbar_wait(&empty_bar[stage], phase ^ 1u, &abort_flag);
@@ -179,12 +176,12 @@ __global__ void __launch_bounds__(kSwThreads, kSwCtasPerSm) blockscaled_swapped_
         uint8_t* ssw = sx + kSwXBytes;
         uint8_t* ssx = ssw + kSwSfBytes;
         if (elected) {
-          mbar_arrive_expect_tx(&full_bar[stage], kSwWBytes + nq * 4096u + 2 * sf_bytes);
+          mbar_arrive_expect_tx(&full_bar[stage], kSwWBytes + nq * 4096u + 2 * kSwSfBytes);
           tma_load_2d(sw, &p.tm_w, kb * 128, w_row, &full_bar[stage]);
           for (int q = 0; q < nq; ++q)
             tma_load_3d(sx + q * 4096, &p.tm_x, 0, x_line0 + kb, row0 + 32 * q, &full_bar[stage]);
-          bulk_load(ssw, sfw_row + static_cast<int64_t>(kb) * sf_bytes, sf_bytes, &full_bar[stage]);
-          bulk_load(ssx, sfx_row + static_cast<int64_t>(kb) * sf_bytes, sf_bytes, &full_bar[stage]);
+          bulk_load(ssw, sfw_row + static_cast<int64_t>(kb) * kSwSfBytes, kSwSfBytes, &full_bar[stage]);
+          bulk_load(ssx, sfx_row + static_cast<int64_t>(kb) * kSwSfBytes, kSwSfBytes, &full_bar[stage]);
         }
         __syncwarp();
         if (++stage == kSwStages) {
@@ -210,10 +207,7 @@ __global__ void __launch_bounds__(kSwThreads, kSwCtasPerSm) blockscaled_swapped_
       const SwTile t = sw_decode(tile, e, s_tile_start, s_off, s_cnt, m_tiles);
       const int n_mma = uniform(((t.n_valid + 31) >> 5) * 32);
       const uint32_t col_off = uniform(static_cast<uint32_t>((t.row0 & 127) >> 5));  // the tile's 32-row group inside its atom
-      const uint32_t idesc4 = umma_idesc_blockscaled(n_mma, 1, 0, 0);
-      uint32_t idesc8[4];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) idesc8[j] = umma_idesc_blockscaled(n_mma, 0, j, j);
+      const uint32_t idesc = umma_idesc_blockscaled(n_mma, 1, 0, 0);
       const int buf = it & 1;
       const uint32_t acc_phase = (it >> 1) & 1u;
       ok = warp_mbar_wait(&tmem_empty_bar[buf], acc_phase ^ 1u, &abort_flag);
@@ -239,24 +233,15 @@ __global__ void __launch_bounds__(kSwThreads, kSwCtasPerSm) blockscaled_swapped_
         }
         ready = mbar_test(full0 + stage * 8, phase);
         if (elected) {
-          if (p.fp4) {
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              tmem_cp_sf_lo(sfw_t + 4 * j, sfw_lo + j * kSfAtomWords);
-              tmem_cp_sf_lo(sfx_t + 4 * j, sfx_lo + j * kSfAtomWords);
-            }
-#pragma unroll
-            for (int j = 0; j < 4; ++j)
-              umma_nvf4_lo(d_tmem, w_lo + 2 * j, x_lo + 2 * j, kDescHi, idesc4, sfw_t + 4 * j, sfx_t + 4 * j + col_off,
-                           (kb > 0 || j > 0) ? 1u : 0u);
-          } else {
-            tmem_cp_sf_lo(sfw_t, sfw_lo);
-            tmem_cp_sf_lo(sfx_t, sfx_lo);
-#pragma unroll
-            for (int j = 0; j < 4; ++j)
-              umma_mxf8_lo(d_tmem, w_lo + 2 * j, x_lo + 2 * j, kDescHi, idesc8[j], sfw_t, sfx_t + col_off,
-                           (kb > 0 || j > 0) ? 1u : 0u);
+          for (int j = 0; j < 4; ++j) {
+            tmem_cp_sf_lo(sfw_t + 4 * j, sfw_lo + j * kSfAtomWords);
+            tmem_cp_sf_lo(sfx_t + 4 * j, sfx_lo + j * kSfAtomWords);
           }
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            umma_nvf4_lo(d_tmem, w_lo + 2 * j, x_lo + 2 * j, kDescHi, idesc, sfw_t + 4 * j, sfx_t + 4 * j + col_off,
+                         (kb > 0 || j > 0) ? 1u : 0u);
           tcgen05_commit_addr(empty);
         }
         __syncwarp();
@@ -395,13 +380,20 @@ __global__ void __launch_bounds__(kSwThreads, kSwCtasPerSm) blockscaled_swapped_
   }
 }
 
+// gemm_blockscaled_rows.cu
+int mxfp8_forward(const dm_operand& a, const dm_operand& sfa, const void* w, const void* sfb, const dm_operand& c,
+                  const dm_operand& h2, const int64_t* scatter_ptrs, const dm_operand& row_scale_inv,
+                  const float* expert_scale_inv, const int32_t* expert_offsets, const int32_t* expert_counts, int e_local,
+                  int64_t max_rows, int64_t N, int64_t Kd, int swiglu_interleaved, const ActParams& act, bool pad_rows,
+                  const int* cond, int num_sms, int* status, cudaStream_t st);
+
 }  // namespace dm
 
 using namespace dm;
 
 // Same contract as dm_gemm_blockscaled (forward, K-major weights) plus `expert_counts`, the real number of rows of
 // every expert inside its 128-padded group (null: the whole group).  Rows past the count are neither read into an
-// output nor written.
+// output nor written.  MXFP8 (format 0) runs on the pair kernel, which has rows on the N side at every size.
 extern "C" int dm_gemm_blockscaled_swapped(int format, dm_operand a, dm_operand sfa, const void* w, const void* sfb,
                                            dm_operand c, dm_operand h2, const int64_t* scatter_ptrs,
                                            dm_operand row_scale_inv, const float* expert_scale_inv,
@@ -419,6 +411,11 @@ extern "C" int dm_gemm_blockscaled_swapped(int format, dm_operand a, dm_operand 
   const int64_t row_bytes = fp4 ? Kd / 2 : Kd;
   if ((row_bytes % 128) != 0 || (N % 128) != 0 || (max_rows % 128) != 0) return kRcUnsupportedShape;
   if (max_rows == 0) return kRcOk;
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  const ActParams act{clamped, alpha, limit};
+  if (!fp4)
+    return mxfp8_forward(a, sfa, w, sfb, c, h2, scatter_ptrs, row_scale_inv, expert_scale_inv, expert_offsets, expert_counts,
+                         e_local, max_rows, N, Kd, swiglu_interleaved, act, false, cond, num_sms, status, st);
   static PerDeviceOnce attr_set;
   int rc = once_per_device(attr_set, [] {
     return static_cast<int>(cudaFuncSetAttribute(blockscaled_swapped_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -430,10 +427,8 @@ extern "C" int dm_gemm_blockscaled_swapped(int format, dm_operand a, dm_operand 
   if (rc != kRcOk) return rc;
   rc = encode_2d_u8(&p.tm_w, w, static_cast<int64_t>(e_local) * N, row_bytes, 128);
   if (rc != kRcOk) return rc;
-  const int64_t scale_cols = Kd / (fp4 ? 16 : 32);
-  p.x_col_atoms = static_cast<int>((scale_cols + 3) / 4);
-  p.w_col_atoms = p.x_col_atoms;
-  p.sfw_group_bytes = (N + 127) / 128 * 128 * static_cast<int64_t>(p.w_col_atoms) * 4;
+  p.col_atoms = static_cast<int>((Kd / 16 + 3) / 4);
+  p.sfw_group_bytes = (N + 127) / 128 * 128 * static_cast<int64_t>(p.col_atoms) * 4;
   p.x_off = a.offset;
   p.sfx_off = sfa.offset;
   p.sfx_base = static_cast<const uint8_t*>(sfa.base);
@@ -454,9 +449,8 @@ extern "C" int dm_gemm_blockscaled_swapped(int format, dm_operand a, dm_operand 
   p.max_rows = static_cast<int>(max_rows);
   p.N = static_cast<int>(N);
   p.k_iters = static_cast<int>(row_bytes / 128);
-  p.fp4 = fp4;
   p.swiglu = swiglu_interleaved ? 1 : 0;
-  p.act = ActParams{clamped, alpha, limit};
-  blockscaled_swapped_kernel<<<kSwCtasPerSm * persistent_grid(num_sms), kSwThreads, kSwSmemBytes, static_cast<cudaStream_t>(stream)>>>(p);
+  p.act = act;
+  blockscaled_swapped_kernel<<<kSwCtasPerSm * persistent_grid(num_sms), kSwThreads, kSwSmemBytes, st>>>(p);
   return static_cast<int>(cudaGetLastError());
 }

@@ -359,7 +359,8 @@ int dm_gemm_blockscaled_counted(int format, dm_operand a, dm_operand sfa, const 
  * expert's rows on the N side in steps of 32, so that a K stage costs MMAs of N = 32 or 64 instead of a 128-row
  * tile and the layer is bound by streaming the weights once.  Replaces the reference's compact decode tiles
  * (dist_moe/kernels/chunked_mega_blockscaled_policy.py:60-95, 32-row M tiles).  Arguments as dm_gemm_blockscaled
- * plus `expert_counts` (int32 [e_local], real rows inside each 128-padded group; NULL = the whole group).  With
+ * plus `expert_counts` (int32 [e_local], real rows inside each 128-padded group; NULL = the whole group); rows past the
+ * count are not written.  MXFP8 runs on the pair kernel of dm_gemm_blockscaled, which has rows on the N side anyway.  With
  * swiglu_interleaved only h2 is written (C must be NULL).  Forward only. */
 int dm_gemm_blockscaled_swapped(int format, dm_operand a, dm_operand sfa, const void* w, const void* sfb, dm_operand c,
                                 dm_operand h2, const int64_t* scatter_ptrs, dm_operand row_scale_inv,
