@@ -183,3 +183,86 @@ def test_scales_at_any_sixteen_bytes(form, offset):
         results.append(out)
     assert torch.equal(results[0], results[1]) and torch.equal(results[0], results[2])
     assert bool((results[0][real.to(DEV)] != 5.0).any())
+
+
+class _Launch:
+    """One launch of the pair kernel in any of its forms, its operands at device offsets inside wider buffers."""
+
+    FORMS = ("dense", "scattered", "swiglu", "swiglu quantised", "input gradient")
+
+    def __init__(self, form, counts, K, N, offset):
+        nat, self.form = _nat(), form
+        self.nat, self.K, self.N, self.F = nat, K, N, N // 2
+        self.E, self.off, self.real, self.R, (qa, sa, _, _), (qw, sw, _, _), self.offs, self.cnts = _operands(
+            nat, 0, counts, K, N, 57 + N, N // 2 if form.startswith("swiglu") else None)
+        if form == "input gradient":
+            qw, _, sw, _ = _tile32_weight(nat, (torch.randn(self.E, K, N, device=DEV) * 0.05).bfloat16())
+        self.qw, self.sw, self.offset = qw, sw, offset
+        self.at = torch.tensor([offset], dtype=torch.int64, device=DEV)
+        self.qa, self.sa = self._placed(qa.view(torch.uint8).reshape(-1)), self._placed(sa.view(torch.uint8).reshape(-1))
+        atoms = (self.F // 32 + 3) // 4
+        self.sizes = {"dense": [self.R * N * 2], "input gradient": [self.R * N * 2], "scattered": [self.R * N * 2],
+                      "swiglu": [self.R * N * 2, self.R * self.F * 2],
+                      "swiglu quantised": [self.R * self.F, self.R * atoms * 4]}[form]
+
+    def _placed(self, data):
+        wide = torch.full((data.numel() + 2 * self.offset + 1024,), 0x7F, dtype=torch.uint8, device=DEV)
+        wide[self.offset:self.offset + data.numel()] = data
+        return wide
+
+    def _at(self, t):
+        return self.nat.Operand(t.data_ptr(), t.numel(), self.at.data_ptr())
+
+    def run(self, num_sms, cond=None):
+        """The result bytes, poisoned before the launch, with those around them."""
+        nat, none = self.nat, self.nat.Operand(None, 0, None)
+        out = [torch.full((n + 2 * self.offset + 1024,), 0x7F, dtype=torch.uint8, device=DEV) for n in self.sizes]
+        status = torch.zeros(8, dtype=torch.int32, device=DEV)
+        tail = (nat.ptr(cond), num_sms, status.data_ptr(), nat.stream_ptr())
+        head = (self._at(self.qa), self._at(self.sa), self.qw.data_ptr(), self.sw.data_ptr())
+        shape = (self.offs.data_ptr(), self.cnts.data_ptr(), self.E, self.R, self.N, self.K)
+        if self.form == "input gradient":
+            rc = nat.lib.dm_gemm_blockscaled_dgrad_counted(*head, self._at(out[0]), None, *shape, *tail)
+        elif self.form == "swiglu quantised":
+            rc = nat.lib.dm_gemm_blockscaled_swiglu_mxfp8_counted(*head, self._at(out[0]), self._at(out[1]), *shape, 0, 1.0, 0.0,
+                                                                  *tail)
+        else:
+            swiglu, ptrs = self.form == "swiglu", None
+            if self.form == "scattered":
+                ptrs = torch.zeros(self.R, dtype=torch.int64, device=DEV)
+                rows = self.real.to(DEV)
+                ptrs[rows] = out[0].data_ptr() + self.offset + rows.flip(0) * (self.N * 2)
+            rc = nat.lib.dm_gemm_blockscaled_counted(0, *head, none if ptrs is not None else self._at(out[0]),
+                                                     self._at(out[1]) if swiglu else none, nat.ptr(ptrs), none, None, *shape,
+                                                     int(swiglu), 0, 1.0, 0.0, *tail)
+        nat.check(rc, self.form)
+        torch.cuda.synchronize()
+        assert status[0].item() == 0, status.tolist()
+        return out
+
+
+@pytest.mark.parametrize("form", _Launch.FORMS)
+@pytest.mark.parametrize("counts", [[256, 512, 100, 0, 257], [96, 33, 128, 64, 1, 120], [300, 545, 0, 64, 180]],
+                         ids=["shared columns", "one atom", "inside atoms"])
+@pytest.mark.parametrize("K", [256, 1152])
+def test_several_tiles_per_pair(form, counts, K):
+    """Pairs that take many tiles in turn: both accumulators, their shared columns, the ring running on from tile to tile.  The
+    bits of the launch that gives every tile a pair of its own, and nothing written beside the results."""
+    one_each = _Launch(form, counts, K, 768, 0).run(0)
+    several = _Launch(form, counts, K, 768, 0)
+    for num_sms in (1, 2, 5, 2):
+        for a, b in zip(one_each, several.run(num_sms)):
+            assert torch.equal(a, b), num_sms
+
+
+@pytest.mark.parametrize("form", _Launch.FORMS)
+def test_device_offsets_and_a_false_predicate(form):
+    """Operands and results that start inside an allocation, at an offset read on the device: the same bits there, none around
+    them.  Where the predicate is false nothing is written."""
+    plain, moved = (_Launch(form, [200, 0, 300, 31], 512, 384, offset) for offset in (0, 128 * 37))
+    yes, no = (torch.tensor([v], dtype=torch.int32, device=DEV) for v in (1, 0))
+    for size, a, b, c in zip(plain.sizes, plain.run(0), moved.run(0), moved.run(4, cond=yes)):
+        assert torch.equal(b[moved.offset:moved.offset + size], a[:size]) and torch.equal(b, c)
+        assert bool((b[:moved.offset] == 0x7F).all()) and bool((b[moved.offset + size:] == 0x7F).all())
+    for t in moved.run(0, cond=no):
+        assert bool((t == 0x7F).all())
