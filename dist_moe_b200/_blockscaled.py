@@ -28,7 +28,8 @@ MXFP8 training (autograd) follows the reference's staged sequence
 
 Saved activations of the training path (h1 in bf16, x and h2 as column-quantised E4M3) lie where the device planner put
 them in the context's arena; the registered operators and calls with clip counters keep them in per-call allocations
-sized for the row capacity.  Each pass through the planner is one native call (``dm_mxfp8_forward`` / ``_backward``).
+sized for the row capacity, and work on whole 128-row groups: the operators' state list (the reference's) does not hold the
+real rows of every expert.  Each pass through the planner is one native call (``dm_mxfp8_forward`` / ``_backward``).
 NVFP4 has no backward (dist_moe/_blockscaled.py:245-321).
 """
 

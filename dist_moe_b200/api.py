@@ -490,8 +490,9 @@ class Context:
     def check_status(self) -> None:
         """Synchronise and raise if a kernel reported a contract violation.
 
-        The reference traps the device in these cases; here the kernels record a code,
-        turn the rest of the call into no-ops and leave the CUDA context usable.
+        The reference traps the device in these cases; here the kernels record a code and leave the CUDA context usable.
+        A call that cannot be routed routes no rows; a slot that is full keeps nothing of the call (its output is right,
+        its gradients are not).
         """
         self._state.check_status()
 

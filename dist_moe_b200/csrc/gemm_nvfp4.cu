@@ -69,9 +69,9 @@ __device__ __forceinline__ N4Tile n4_decode(int tile, int& e, const int* tile_st
 // scale-atom copies (16 cycles each, hidden behind the MMAs) and four 128-cycle MMAs.  TMEM holds one 256-column accumulator
 // plus the scale columns of every stage slot: the epilogue warps read it into registers and hand it back before they
 // convert and store, so only that read stands between a tile's last MMA and the next tile's first.  Bound: operand loads from
-// L2, 14 TB/s.  32 experts, 65 536 rows, D = 7168, F = 2048: 2074 us a layer; the kernel that puts rows on the MMA's N side
-// over pairs of CTAs (gemm_blockscaled_rows.cu, MXFP8) loads a third less but took 2187 to 2233 us here, its epilogue of
-// 2 x 256 rows against eight stages of W2.  Experts with few rows take the swapped-operand kernel instead.
+// L2, 14 TB/s.  32 experts, 65 536 rows, D = 7168, F = 2048: 1976 us a layer; the kernel that puts rows on the MMA's N side
+// over pairs of CTAs (gemm_blockscaled_rows.cu, MXFP8) loads a third less but took 2187 to 2233 us where these tiles took
+// 2004, its epilogue of 2 x 256 rows against eight stages of W2.  Experts with few rows take the swapped-operand kernel instead.
 constexpr int kN4Threads = 352;  // TMA warp, MMA warp, eight epilogue warps, accumulator watcher
 constexpr uint32_t kN4Stage = kN4ABytes + kN4BBytes + 3 * kN4SfBytes;  // 54 KiB
 constexpr int kN4Stages = 3;

@@ -543,8 +543,9 @@ int dm_vmm_destroy(void* region);
 
 /* ---------------------------------------------------------------------------
  * One pass as a sequence of the calls above (the reference's orchestration: BF16 dist_moe/api.py:1844-2188 and 2205-2609,
- * MXFP8 training on the planner's placement dist_moe/_blockscaled.py:1309-1931 and 1951-2541), for hosts whose own call overhead exceeds the launches'.  `steps` selects launches; running a pass in
- * several calls with disjoint steps, in the order of the bits, is the same as one call with all of them.  report[0]
+ * MXFP8 training on the planner's placement dist_moe/_blockscaled.py:1309-1931 and 1951-2541), for hosts whose own call
+ * overhead exceeds the launches'.  `steps` selects launches; running a pass in several calls with disjoint steps, in the
+ * order of the bits, is the same as one call with all of them.  Plans are bounded (DM_PLAN_BOUNDED).  report[0]
  * receives the launches made, report[1] the step that failed (0: none).  Barriers go with the step before them and are
  * skipped where ep == 1.  Device pointers throughout, except report.
  * ------------------------------------------------------------------------- */
