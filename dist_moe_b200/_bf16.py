@@ -294,8 +294,8 @@ def _rmsnorm_args(post):
 
 def _plain_execution(*tensors) -> bool:
     """Nothing acts on this call's operators: no tracing or fake tensors, no dispatch or function mode, no functorch
-    level, no recorder (profiler, execution trace).  The registered operators' bodies can then run without the dispatcher, which costs a small layer more than its
-    launches."""
+    level, no recorder (profiler, execution trace).  The registered operators' bodies can then run without the dispatcher,
+    which costs a small layer more than its launches."""
     if torch.compiler.is_compiling():  # first: a tracer of Python code must not meet the calls below
         return False
     return (not recorded() and torch._C._len_torch_dispatch_stack() == 0 and torch._C._len_torch_function_stack() == 0

@@ -56,9 +56,9 @@ __device__ __forceinline__ BsTile bs_decode(int tile, int& e, const int* tile_st
 // 128 x 256 output tiles.  Per 128 rows of K the tile moves 48 KiB of operands for four MMAs of 128 cycles.  With few rows per
 // expert the epilogue bounds it: it takes 6900 cycles a tile and waits 25 of them for an accumulator; staging, proxy fences and
 // the copy engine's reads (2100 cycles) are its time, the adding into dW (4.3 to 4.7 TB/s of HBM) is behind them.  685 and
-// 1486 us for the W2 and W13 gradients of 128 experts, 73 728 rows, D = 4096, F = 1536.  TMEM holds one 256-column accumulator plus the scale
-// columns of the stage slots: the epilogue warps read it into registers and hand it back before they convert and store, so
-// only that read stands between a tile's last MMA and the next tile's first.
+// 1486 us for the W2 and W13 gradients of 128 experts, 73 728 rows, D = 4096, F = 1536.  TMEM holds one 256-column accumulator
+// plus the scale columns of the stage slots: the epilogue warps read it into registers and hand it back before they convert and
+// store, so only that read stands between a tile's last MMA and the next tile's first.
 constexpr int kWdBN = 256;
 constexpr int kWdThreads = 352;  // TMA warp, MMA warp, eight epilogue warps, accumulator watcher
 constexpr uint32_t kWdBBytes = kWdBN * 128;                            // 32 KiB

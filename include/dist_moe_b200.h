@@ -146,12 +146,12 @@ int dm_route_decode_kernel_enabled(void); /* the current setting, without changi
  * reference does.  fwd_state = [x, x_gathered, h1, h2, h3, slot id],
  * bwd_offsets = [x_gathered, h1, h2, grad_h2, grad_h3_gathered, grad_h1].
  * need_recompute is one byte (bool).  Overflow sets DM_STATUS_ARENA_OVERFLOW.
- * scratch_only: 0 or 1; | DM_PLAN_BOUNDED: a save that would not lie inside its slot (calls that broke the slot's
+ * scratch_only: zero or not; with DM_PLAN_BOUNDED added: a save that would not lie inside its slot (calls that broke the slot's
  * last-in-first-out order) gets the offset -1 (x where the layer is recomputed, else h3), everything else of that call a
  * place in scratch, so that no launch leaves the arena.  dm_cond_copy, dm_scale_and_sum and dm_rmsnorm_combine_fwd copy
  * nothing to or from a negative offset; dm_broadcast_and_scale_select reads h3_alt then.
  * ------------------------------------------------------------------------- */
-enum { DM_PLAN_BOUNDED = 2 };
+enum { DM_PLAN_BOUNDED = 1 << 16 };
 int dm_plan_fwd_bf16(const int32_t* recv_rows, const int32_t* per_rank, int64_t* saved_bytes_per_rank,
                      int64_t* buffer_offsets, int64_t* peak_min_free, uint8_t* need_recompute,
                      int32_t* recompute_cond, int64_t* fwd_state, const int64_t* slot_selector,
@@ -334,8 +334,8 @@ int dm_gemm_wgrad(dm_operand dy, dm_operand x, void* dw, int out_is_fp32, int ac
  *       and, when C is given, h1 = [gate | up] in the canonical (not interleaved) column order.
  * Every expert's row range must start on a multiple of 128 (routing with m_multiple_of = 128).  Otherwise the status is
  * set to DM_STATUS_CAPACITY_EXCEEDED and that expert's results are not defined; the MXFP8 and the swapped form leave it out.
- * The device offset of `a` must be a multiple of 128, that of `sfa` a multiple of 16 (a multiple of 128 loads faster in the
- * MXFP8 forms).  sfa.bytes smaller than the layout of max_rows counts as not told.
+ * The device offset of `a` must be a multiple of 128, that of `sfa` a multiple of 16.  sfa.bytes smaller than the layout of
+ * max_rows counts as not told.
  * ------------------------------------------------------------------------- */
 int dm_gemm_blockscaled(int format, dm_operand a, dm_operand sfa, const void* w, const void* sfb, dm_operand c,
                         dm_operand h2, const int64_t* scatter_ptrs, dm_operand row_scale_inv,

@@ -12,6 +12,7 @@ from oracle import planner_blockscaled as bs
 
 SLOTS, LAYERS, K, D, F, T = 2, 2, 2, 256, 384, 64
 ROWS = 256  # most rows of a call
+BOUNDED = 1 << 16  # DM_PLAN_BOUNDED
 
 
 def _sizes(kind, rows):
@@ -130,13 +131,13 @@ def test_planner_kernels_match_the_oracle(kind, seed):
             if kind == "bf16":
                 rc = nat.lib.dm_plan_fwd_bf16(rows.data_ptr(), rows.data_ptr(), saved.data_ptr(), offs.data_ptr(),
                                               peak.data_ptr(), need.data_ptr(), cond.data_ptr(), state.data_ptr(),
-                                              sel.data_ptr(), layer.data_ptr(), 1, T, K, D, F, slot_bytes, SLOTS, LAYERS, 2,
+                                              sel.data_ptr(), layer.data_ptr(), 1, T, K, D, F, slot_bytes, SLOTS, LAYERS, BOUNDED,
                                               status.data_ptr(), nat.stream_ptr())
             else:
                 rc = nat.lib.dm_plan_fwd_blockscaled(rows.data_ptr(), rows.data_ptr(), None, saved.data_ptr(), offs.data_ptr(),
                                                      peak.data_ptr(), need.data_ptr(), cond.data_ptr(), state.data_ptr(),
                                                      table.data_ptr(), sel.data_ptr(), layer.data_ptr(), 1, T, K, D, F,
-                                                     storage, 1 << 20, slot_bytes, SLOTS, LAYERS, 0, 0, 2, 0, 0,
+                                                     storage, 1 << 20, slot_bytes, SLOTS, LAYERS, 0, 0, BOUNDED, 0, 0,
                                                      status.data_ptr(), nat.stream_ptr())
             nat.check(rc, "plan forward")
             assert (bool(need.item()), state.tolist()) == (want[0], want[1]) and cond.item() == int(want[0])
