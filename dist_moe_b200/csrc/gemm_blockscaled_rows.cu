@@ -201,7 +201,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kBrThreads, 1)
   // Ring: stages as large as the launch's largest tile needs, as many as shared memory and the scale columns allow.
   const int n_max = 2 * rw_box_rows(uniform(s_box));
   const uint32_t x_groups = bs_tile_atoms(n_max);
-  const uint32_t slot_cols = (1 + x_groups) * 4;  // scale columns of a stage slot
+  // Scale columns of a stage slot: an atom of the weights and those of the rows, at a stride of 8 or 16.  Slots of twelve, all that
+  // two atoms of rows need, cost the plain forms 0.5 to 0.9 % (the four forward and input-gradient launches of a training layer).
+  const uint32_t slot_cols = x_groups == 1 ? 8 : 16;
   const uint32_t sf_at = kBrWBytes + static_cast<uint32_t>(n_max / 2) * 128;  // weight atoms, then the rows' atoms
   const uint32_t stage_bytes = sf_at + (((1 + x_groups) * kSfBytes + 1023) & ~1023u);
   const int fit = static_cast<int>(kRing / stage_bytes);
@@ -318,9 +320,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kBrThreads, 1)
           const uint32_t w_addr = ring + stage * stage_bytes;
           const uint32_t w_lo = ((w_addr & 0x3ffffu) >> 4) | kLbo, x_lo = w_lo + (kBrWBytes >> 4);
           const uint32_t sf_lo = sf_desc_lo(w_addr + sf_at);
-          // the weights' columns come last: a tile that starts at its atom's third column stays inside the slot
-          const uint32_t sfx_t = sf_tmem + stage * slot_cols;
-          const uint32_t sfw_t = sfx_t + 4u * x_groups;
+          const uint32_t sfw_t = sf_tmem + stage * slot_cols;
+          const uint32_t sfx_t = sfw_t + 4u;
           const uint32_t empty = empty0 + stage * 8;
           if (++stage == stages) {
             stage = 0;
