@@ -64,7 +64,6 @@ struct BrParams {
   int* status;
   int64_t sfw_group_lines;
   int e_local, max_rows, N, Kw, k_iters, x_col_atoms, w_col_atoms;
-  int pad_rows;  // rows of a dense C past an expert's count are written too
   // SwiGLU epilogue that writes h2 as MXFP8 rows (E4M3 bytes + blocked E8M0 scales) instead of bf16
   uint8_t* hq_base;
   const int64_t* hq_off;
@@ -101,7 +100,7 @@ __device__ __forceinline__ uint32_t br_pair(uint32_t w, int odd) {
   return __byte_perm(w, o, odd ? 0x3276 : 0x5410);
 }
 
-template <int kDgrad, bool kSwiglu>
+template <int kDgrad, bool kSwiglu, bool kPadRows>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kBrThreads, 1)
     blockscaled_rows_kernel(const __grid_constant__ BrParams p) {
   if (p.cond != nullptr && *p.cond == 0) return;
@@ -401,7 +400,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kBrThreads, 1)
         if (kSwiglu ? p.c_base == nullptr : false) return 0;
         if (!kSwiglu && p.scatter_ptrs != nullptr) return r < t.rows ? static_cast<uint64_t>(p.scatter_ptrs[t.row0 + r]) : 0;
         // dense rows up to the next multiple of 32 are computed (padding rows hold zeros)
-        if (!kSwiglu && !p.pad_rows && r >= t.rows) return 0;
+        if (!kSwiglu && !kPadRows && r >= t.rows) return 0;
         return reinterpret_cast<uint64_t>(p.c_base) + c_off + static_cast<uint64_t>(t.row0 + r) * p.N * 2;
       };
       auto row_scale = [&](int b) -> float { return row_inv != nullptr ? row_inv[t.row0 + b * 32 + lane] : 1.0f; };
@@ -559,7 +558,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kBrThreads, 1)
         scale_a = scale_n;
       }
       if (held) hand_back();
-      if (!kSwiglu && dense && p.pad_rows && t.last) {
+      if (!kSwiglu && kPadRows && dense && t.last) {
         // rows between the last multiple of 32 and the end of the padded group: zeros, as the product of their zero rows
         const int col = m_blk * kBrBM + (lane & 15) * 8;
         if (col + 8 <= p.N)
@@ -599,15 +598,16 @@ int mxfp8_forward(const dm_operand& a, const dm_operand& sfa, const void* w, con
                   int64_t max_rows, int64_t N, int64_t Kd, int swiglu_interleaved, const ActParams& act, bool pad_rows,
                   const int* cond, int num_sms, int* status, cudaStream_t st);
 
-template <int kDgrad, bool kSwiglu>
+// kPadRows: rows of a dense C past an expert's count are written too.
+template <int kDgrad, bool kSwiglu, bool kPadRows = true>
 static int br_launch(const BrParams& p, int num_sms, cudaStream_t st) {
   static PerDeviceOnce attr_set;
   const int rc = once_per_device(attr_set, [] {
-    return static_cast<int>(cudaFuncSetAttribute(blockscaled_rows_kernel<kDgrad, kSwiglu>,
+    return static_cast<int>(cudaFuncSetAttribute(blockscaled_rows_kernel<kDgrad, kSwiglu, kPadRows>,
                                                  cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kBrDynSmem)));
   });
   if (rc != 0) return rc;
-  blockscaled_rows_kernel<kDgrad, kSwiglu><<<pair_grid(num_sms), kBrThreads, kBrDynSmem, st>>>(p);
+  blockscaled_rows_kernel<kDgrad, kSwiglu, kPadRows><<<pair_grid(num_sms), kBrThreads, kBrDynSmem, st>>>(p);
   return static_cast<int>(cudaGetLastError());
 }
 
@@ -698,8 +698,8 @@ int dm::mxfp8_forward(const dm_operand& a, const dm_operand& sfa, const void* w,
   p.expert_inv = expert_scale_inv;
   p.scatter_ptrs = scatter_ptrs;
   p.act = act;
-  p.pad_rows = pad_rows;
-  return swiglu_interleaved ? br_launch<0, true>(p, num_sms, st) : br_launch<0, false>(p, num_sms, st);
+  if (swiglu_interleaved) return br_launch<0, true>(p, num_sms, st);
+  return pad_rows ? br_launch<0, false>(p, num_sms, st) : br_launch<0, false, false>(p, num_sms, st);
 }
 
 extern "C" int dm_gemm_blockscaled_counted(int format, dm_operand a, dm_operand sfa, const void* w, const void* sfb,
@@ -794,7 +794,6 @@ extern "C" int dm_gemm_blockscaled_dgrad_counted(dm_operand dy, dm_operand sf_dy
   p.c_base = static_cast<uint8_t*>(c.base);
   p.scatter_ptrs = scatter_ptrs;
   p.Kw = static_cast<int>(Kd);
-  p.pad_rows = 1;
   p.act = ActParams{0, 1.0f, 0.0f};
   return br_launch<1, false>(p, num_sms, static_cast<cudaStream_t>(stream));
 }
