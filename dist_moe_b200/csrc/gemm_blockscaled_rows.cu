@@ -46,8 +46,7 @@ struct BrParams {
   CUtensorMap tm_w;
   CUtensorMap tm_x[kRwBoxes];  // routed rows, boxes of rw_box_rows(i) rows x 128 bytes
   CUtensorMap tm_sfw;          // scales as lines of 128 bytes, boxes of one atom
-  CUtensorMap tm_sfx;
-  CUtensorMap tm_sfx16;        // the rows' scales as pieces of 16 bytes, for offsets that are not multiples of 128
+  CUtensorMap tm_sfx;          // the rows' scales as lines that overlap: they may start inside a line
   const int64_t* x_off;
   const int64_t* sfx_off;
   const int64_t* c_off;
@@ -223,7 +222,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kBrThreads, 1)
     const int64_t x_off = p.x_off ? *p.x_off : 0, sfx_off = p.sfx_off ? *p.sfx_off : 0;
     if (rows_side && lane == 0 && ((x_off & 127) | (sfx_off & 15)) != 0) set_status(p.status, kCapacityExceeded, -2, 0, 0);
     const int x_line0 = uniform(static_cast<int>(x_off >> 7)), sfx_line0 = uniform(static_cast<int>(sfx_off >> 7));
-    const int sfx_piece = uniform(static_cast<int>((sfx_off >> 4) & 7));  // 16-byte piece of its line that the scales start at
+    const int sfx_x = uniform(static_cast<int>((sfx_off >> 4) & 7) * 4);  // word of its line that the scales start at
     constexpr int kSfLines = kSfBytes / 128;
     bool ok = true;
     const uint32_t lead_full = uniform(cluster_addr(smem_u32(&full_bar[0]), 0));
@@ -249,13 +248,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kBrThreads, 1)
           if (rows_side) {
             tma_load_3d_pair(sw + kBrWBytes, tm_x, 0, x_line0 + kb, x_row, full);
             uint8_t* sf = sw + sf_at + kSfBytes;
-            for (int a = 0; a < x_atoms; ++a) {
-              const int line = sfx_line + a * p.x_col_atoms * 4 + kb * kSfLines;
-              if (sfx_piece == 0)
-                tma_load_2d_pair(sf + a * kSfBytes, &p.tm_sfx, 0, line, full);
-              else
-                tma_load_3d_pair(sf + a * kSfBytes, &p.tm_sfx16, 0, sfx_piece, line, full);
-            }
+            for (int a = 0; a < x_atoms; ++a)
+              tma_load_2d_pair(sf + a * kSfBytes, &p.tm_sfx, sfx_x, sfx_line + a * p.x_col_atoms * 4 + kb * kSfLines, full);
           } else {
             if (rank == 0) mbar_arrive_expect_tx(&full_bar[stage], tx);
             if (kDgrad)
@@ -611,31 +605,18 @@ static int br_launch(const BrParams& p, int num_sms, cudaStream_t st) {
   return static_cast<int>(cudaGetLastError());
 }
 
-// Scales as lines of 128 bytes, boxes of one atom; base 16-byte aligned.
-static int encode_sf(CUtensorMap* tm, const void* base, int64_t bytes) {
+// Scales as lines that start every 128 bytes, boxes of one atom (four lines of 128 bytes); base 16-byte aligned.  The rows' lines
+// are 256 bytes long and overlap: an atom that starts at word x < 32 of line l is the box at (x, l), contiguous as stored.
+// (Two maps, chosen in the kernel by the offset, cost 2 of 220 us: 16 tokens, 128 experts x 2816 x 2816.)
+static int encode_sf(CUtensorMap* tm, const void* base, int64_t bytes, bool overlap) {
   EncodeTiledFn enc = get_encode();
   if (!enc) return kRcNoDriver;
   if (bytes < 128) return kRcBadArg;
-  cuuint64_t dims[2] = {32, static_cast<cuuint64_t>(bytes / 128)};
+  cuuint64_t dims[2] = {overlap ? 64u : 32u, static_cast<cuuint64_t>(bytes / 128)};
   cuuint64_t strides[1] = {128};
   cuuint32_t box[2] = {32, 4};
   cuuint32_t estr[2] = {1, 1};
   CUresult r = enc(tm, CU_TENSOR_MAP_DATA_TYPE_UINT32, 2, const_cast<void*>(base), dims, strides, box, estr,
-                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  return r == CUDA_SUCCESS ? kRcOk : 1000 + static_cast<int>(r);
-}
-
-// The same bytes as lines that overlap: sixteen pieces of 16 bytes from every 128 bytes on, boxes of eight pieces by four
-// lines.  An atom that starts at piece p of line l is the box at (p, l), contiguous as stored.
-static int encode_sf16(CUtensorMap* tm, const void* base, int64_t bytes) {
-  EncodeTiledFn enc = get_encode();
-  if (!enc) return kRcNoDriver;
-  cuuint64_t dims[3] = {4, 16, static_cast<cuuint64_t>(bytes / 128)};
-  cuuint64_t strides[2] = {16, 128};
-  cuuint32_t box[3] = {4, 8, 4};
-  cuuint32_t estr[3] = {1, 1, 1};
-  CUresult r = enc(tm, CU_TENSOR_MAP_DATA_TYPE_UINT32, 3, const_cast<void*>(base), dims, strides, box, estr,
                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS ? kRcOk : 1000 + static_cast<int>(r);
@@ -659,11 +640,9 @@ static int br_setup(BrParams& p, const dm_operand& x, const dm_operand& sfx, con
   // it): the loads are then bounded by the rows alone, as they were.
   const int64_t layout_bytes = max_rows / 128 * static_cast<int64_t>(p.x_col_atoms) * 512;
   const int64_t sfx_bytes = sfx.bytes >= layout_bytes ? sfx.bytes : int64_t{1} << 37;
-  int rc = encode_sf(&p.tm_sfx, sfx.base, sfx_bytes);
+  int rc = encode_sf(&p.tm_sfx, sfx.base, sfx_bytes, true);
   if (rc != kRcOk) return rc;
-  rc = encode_sf16(&p.tm_sfx16, sfx.base, sfx_bytes);
-  if (rc != kRcOk) return rc;
-  rc = encode_sf(&p.tm_sfw, sfw, e_local * p.sfw_group_lines * 128);
+  rc = encode_sf(&p.tm_sfw, sfw, e_local * p.sfw_group_lines * 128, false);
   if (rc != kRcOk) return rc;
   p.x_off = x.offset;
   p.sfx_off = sfx.offset;
