@@ -199,8 +199,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kBrThreads, 1)
   // Ring: stages as large as the launch's largest tile needs, as many as shared memory and the scale columns allow.
   const int n_max = 2 * rw_box_rows(uniform(s_box));
   const uint32_t x_groups = bs_tile_atoms(n_max);
-  // Scale columns of a stage slot: an atom of the weights and those of the rows, at a stride of 8 or 16.  Slots of twelve, all that
-  // two atoms of rows need, cost the plain forms 0.5 to 0.9 % (the four forward and input-gradient launches of a training layer).
+  // Scale columns of a stage slot: an atom of the weights and those of the rows, at a stride of 8 or 16.  With slots of twelve, all
+  // that two atoms of rows need, the four forward and input-gradient launches of a training layer took 0.9 to 1.6 % longer.
   const uint32_t slot_cols = x_groups == 1 ? 8 : 16;
   const uint32_t sf_at = kBrWBytes + static_cast<uint32_t>(n_max / 2) * 128;  // weight atoms, then the rows' atoms
   const uint32_t stage_bytes = sf_at + (((1 + x_groups) * kSfBytes + 1023) & ~1023u);
