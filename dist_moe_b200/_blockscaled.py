@@ -267,6 +267,15 @@ def _workspace(state):
 SWAPPED_MAX_ROWS_PER_EXPERT = None
 _SWAPPED_MAX_ROWS = {BlockScaledFormat.NVFP4: 48, BlockScaledFormat.MXFP8_E4M3: 0}
 
+# NVFP4 calls whose experts receive at least this many rows on average run on CTA pairs (256 x 256 tiles): 32 experts x 7168 x
+# 2048, 128 x 256 tiles / pairs, us a layer under the power cap: 64 rows 223 / 243, 128 272 / 272, 256 370 / 377, 512 609 / 597,
+# 2048 1984 / 1907.
+_PAIR_MIN_ROWS = 512
+
+
+def _gemm_pairs(_format, *arguments):
+    return nat.lib.dm_gemm_nvfp4_pairs(*arguments)
+
 
 def _view(buf: torch.Tensor, offset: int) -> nat.Operand:
     return nat.Operand(buf.data_ptr() + offset, buf.numel() - offset, None)
@@ -365,6 +374,7 @@ def run_block_scaled(x, ids, scores, w13_weight, w2_weight, context: Any, option
     # few rows per expert (decode): weights on the MMA's M side, the rows on its N side
     limit_rows = _SWAPPED_MAX_ROWS[fmt] if SWAPPED_MAX_ROWS_PER_EXPERT is None else SWAPPED_MAX_ROWS_PER_EXPERT
     swapped = fused and ep * T * K <= limit_rows * E
+    gemm = _gemm_pairs if lay.fp4 and ep * T * K >= _PAIR_MIN_ROWS * E else _gemm
     if swapped:
         h2_dense = lay.dense
         nat.check(nat.lib.dm_gemm_blockscaled_swapped(f, _view(buf, lay.x_q), _view(buf, lay.x_sf),
@@ -384,16 +394,16 @@ def run_block_scaled(x, ids, scores, w13_weight, w2_weight, context: Any, option
                                      None, state.num_sms, status, st), "dm_gemm_blockscaled_swiglu_mxfp8")
     elif fused:
         h2_dense = lay.dense
-        nat.check(_gemm(f, _view(buf, lay.x_q), _view(buf, lay.x_sf), p13.fprop_data.data_ptr(),
-                        p13.fprop_scale.data_ptr(), none, _view(buf, h2_dense), None, row_inv,
-                        nat.ptr(p13.global_scale_inv), offsets.data_ptr(), real.data_ptr(), el, max_rows, 2 * F, D, 1,
-                        clamped, alpha, limit, None, state.num_sms, status, st), "dm_gemm_blockscaled(w13+swiglu)")
+        nat.check(gemm(f, _view(buf, lay.x_q), _view(buf, lay.x_sf), p13.fprop_data.data_ptr(),
+                       p13.fprop_scale.data_ptr(), none, _view(buf, h2_dense), None, row_inv,
+                       nat.ptr(p13.global_scale_inv), offsets.data_ptr(), real.data_ptr(), el, max_rows, 2 * F, D, 1,
+                       clamped, alpha, limit, None, state.num_sms, status, st), "dm_gemm_blockscaled(w13+swiglu)")
     else:
         h2_dense = lay.h2_dense
-        nat.check(_gemm(f, _view(buf, lay.x_q), _view(buf, lay.x_sf), p13.fprop_data.data_ptr(),
-                        p13.fprop_scale.data_ptr(), _view(buf, lay.dense), none, None, row_inv,
-                        nat.ptr(p13.global_scale_inv), offsets.data_ptr(), real.data_ptr(), el, max_rows, 2 * F, D, 0,
-                        0, 1.0, 0.0, None, state.num_sms, status, st), "dm_gemm_blockscaled(w13)")
+        nat.check(gemm(f, _view(buf, lay.x_q), _view(buf, lay.x_sf), p13.fprop_data.data_ptr(),
+                       p13.fprop_scale.data_ptr(), _view(buf, lay.dense), none, None, row_inv,
+                       nat.ptr(p13.global_scale_inv), offsets.data_ptr(), real.data_ptr(), el, max_rows, 2 * F, D, 0,
+                       0, 1.0, 0.0, None, state.num_sms, status, st), "dm_gemm_blockscaled(w13)")
         nat.check(nat.lib.dm_swiglu_fwd(buf.data_ptr() + lay.dense, None, buf.data_ptr() + h2_dense, None,
                                         recv.data_ptr(), max_rows, F, clamped, alpha, limit, None, 0.0, None, st),
                   "dm_swiglu_fwd")
@@ -419,10 +429,10 @@ def run_block_scaled(x, ids, scores, w13_weight, w2_weight, context: Any, option
                                                       real.data_ptr(), el, max_rows, D, F, 0, 0, 1.0, 0.0, None,
                                                       state.num_sms, status, st), "dm_gemm_blockscaled_swapped(w2)")
     else:
-        nat.check(_gemm(f, _view(buf, lay.h_q), _view(buf, lay.h_sf), p2.fprop_data.data_ptr(),
-                        p2.fprop_scale.data_ptr(), none, none, sct.data_ptr(),
-                        _view(buf, lay.h_inv) if lay.fp4 else none, nat.ptr(p2.global_scale_inv), offsets.data_ptr(),
-                        real.data_ptr(), el, max_rows, D, F, 0, 0, 1.0, 0.0, None, state.num_sms, status, st),
+        nat.check(gemm(f, _view(buf, lay.h_q), _view(buf, lay.h_sf), p2.fprop_data.data_ptr(),
+                       p2.fprop_scale.data_ptr(), none, none, sct.data_ptr(),
+                       _view(buf, lay.h_inv) if lay.fp4 else none, nat.ptr(p2.global_scale_inv), offsets.data_ptr(),
+                       real.data_ptr(), el, max_rows, D, F, 0, 0, 1.0, 0.0, None, state.num_sms, status, st),
                   "dm_gemm_blockscaled(w2)")
     state.barrier(state.combine)
     out = torch.empty(T, D, dtype=torch.bfloat16, device=dev)

@@ -145,6 +145,11 @@ _SIGNATURES = {
         [c_int, Operand, Operand, _P, _P, Operand, Operand, _P, Operand, _P, _P, _P, c_int, c_int64, c_int64, c_int64,
          c_int, c_int, c_float, c_float, _P, c_int, _P, _P],
     ),
+    "dm_gemm_nvfp4_pairs": (
+        c_int,
+        [Operand, Operand, _P, _P, Operand, Operand, _P, Operand, _P, _P, _P, c_int, c_int64, c_int64, c_int64, c_int, c_int,
+         c_float, c_float, _P, c_int, _P, _P],
+    ),
     "dm_gemm_blockscaled_swapped": (
         c_int,
         [c_int, Operand, Operand, _P, _P, Operand, Operand, _P, Operand, _P, _P, _P, c_int, c_int64, c_int64, c_int64,

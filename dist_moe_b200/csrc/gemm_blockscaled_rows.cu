@@ -605,23 +605,6 @@ static int br_launch(const BrParams& p, int num_sms, cudaStream_t st) {
   return static_cast<int>(cudaGetLastError());
 }
 
-// Scales as lines that start every 128 bytes, boxes of one atom (four lines of 128 bytes); base 16-byte aligned.  The rows' lines
-// are 256 bytes long and overlap: an atom that starts at word x < 32 of line l is the box at (x, l), contiguous as stored.
-// (Two maps, chosen in the kernel by the offset, cost 2 of 220 us: 16 tokens, 128 experts x 2816 x 2816.)
-static int encode_sf(CUtensorMap* tm, const void* base, int64_t bytes, bool overlap) {
-  EncodeTiledFn enc = get_encode();
-  if (!enc) return kRcNoDriver;
-  if (bytes < 128) return kRcBadArg;
-  cuuint64_t dims[2] = {overlap ? 64u : 32u, static_cast<cuuint64_t>(bytes / 128)};
-  cuuint64_t strides[1] = {128};
-  cuuint32_t box[2] = {32, 4};
-  cuuint32_t estr[2] = {1, 1};
-  CUresult r = enc(tm, CU_TENSOR_MAP_DATA_TYPE_UINT32, 2, const_cast<void*>(base), dims, strides, box, estr,
-                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  return r == CUDA_SUCCESS ? kRcOk : 1000 + static_cast<int>(r);
-}
-
 }  // namespace dm
 
 using namespace dm;

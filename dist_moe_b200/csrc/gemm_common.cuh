@@ -219,6 +219,20 @@ __device__ __forceinline__ void umma_mxf8_lo_pair(uint32_t d_tmem, uint32_t a_lo
       ::"r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(desc_hi), "r"(idesc), "r"(accumulate), "r"(sfa_tmem), "r"(sfb_tmem)
       : "memory");
 }
+__device__ __forceinline__ void umma_nvf4_lo_pair(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t desc_hi,
+                                                  uint32_t idesc, uint32_t sfa_tmem, uint32_t sfb_tmem, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t"
+      ".reg .pred p;\n\t"
+      ".reg .b64 da, db;\n\t"
+      "setp.ne.b32 p, %5, 0;\n\t"
+      "mov.b64 da, {%1, %3};\n\t"
+      "mov.b64 db, {%2, %3};\n\t"
+      "tcgen05.mma.cta_group::2.kind::mxf4nvf4.block_scale.scale_vec::4X [%0], da, db, %4, [%6], [%7], p;\n\t"
+      "}\n"
+      ::"r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(desc_hi), "r"(idesc), "r"(accumulate), "r"(sfa_tmem), "r"(sfb_tmem)
+      : "memory");
+}
 // Both CTAs copy the atom at this offset of their own shared memory to these columns of their own TMEM.
 __device__ __forceinline__ void tmem_cp_sf_lo_pair(uint32_t taddr, uint32_t lo) {
   asm volatile(
@@ -358,6 +372,23 @@ static inline int encode_arena_u8(CUtensorMap* tm, const dm_operand& op, int64_t
   cuuint32_t estr[3] = {1, 1, 1};
   CUresult r = enc(tm, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, op.base, dims, strides, box, estr,
                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? kRcOk : 1000 + static_cast<int>(r);
+}
+
+// Scales as lines that start every 128 bytes, boxes of `lines` lines (an atom has four); base 16-byte aligned.  The rows' lines
+// are 256 bytes long and overlap: an atom that starts at word x < 32 of line l is the box at (x, l), contiguous as stored.
+// (Two maps, chosen in the kernel by the offset, cost 2 of 220 us: 16 tokens, 128 experts x 2816 x 2816.)
+static inline int encode_sf(CUtensorMap* tm, const void* base, int64_t bytes, bool overlap, int lines = 4) {
+  EncodeTiledFn enc = get_encode();
+  if (!enc) return kRcNoDriver;
+  if (bytes < 128) return kRcBadArg;
+  cuuint64_t dims[2] = {overlap ? 64u : 32u, static_cast<cuuint64_t>(bytes / 128)};
+  cuuint64_t strides[1] = {128};
+  cuuint32_t box[2] = {32, static_cast<cuuint32_t>(lines)};
+  cuuint32_t estr[2] = {1, 1};
+  CUresult r = enc(tm, CU_TENSOR_MAP_DATA_TYPE_UINT32, 2, const_cast<void*>(base), dims, strides, box, estr,
+                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS ? kRcOk : 1000 + static_cast<int>(r);
 }

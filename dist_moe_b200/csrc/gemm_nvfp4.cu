@@ -14,6 +14,7 @@
 // per-row destinations), or SwiGLU over a W13 whose rows were interleaved in groups of 8 gate / 8 up rows at preparation
 // time, producing bf16 h2 (and h1).
 #include "gemm_common.cuh"
+#include "row_tiles.cuh"
 
 namespace dm {
 
@@ -28,6 +29,8 @@ constexpr int kN4MaxGroups = 256;
 struct N4Params {
   CUtensorMap tm_a;
   CUtensorMap tm_b;
+  CUtensorMap tm_sfa;  // scales as lines of 128 bytes, boxes of a stage's four atoms
+  CUtensorMap tm_sfb;
   const int64_t* a_off;
   const int64_t* sfa_off;
   const int64_t* c_off;
@@ -41,6 +44,7 @@ struct N4Params {
   uint8_t* h2_base;
   const int64_t* scatter_ptrs;
   const int32_t* expert_offsets;
+  const int32_t* expert_counts;  // real rows of every 128-padded group, or null: all of them
   const int* cond;
   int* status;
   int64_t sfb_group_bytes;
@@ -435,16 +439,384 @@ __global__ void __launch_bounds__(kN4Threads, 1) nvfp4_wide_kernel(const __grid_
   }
 }
 
-// The NVFP4 forward of dm_gemm_blockscaled (arguments checked there).
-int nvfp4_forward(const dm_operand& a, const dm_operand& sfa, const void* w, const void* sfb, const dm_operand& c,
-                  const dm_operand& h2, const int64_t* scatter_ptrs, const dm_operand& row_scale_inv,
-                  const float* expert_scale_inv, const int32_t* expert_offsets, int e_local, int64_t max_rows, int64_t N,
-                  int64_t Kd, int swiglu_interleaved, const ActParams& act, const int* cond, int num_sms, int* status,
-                  cudaStream_t st) {
-  N4Params p{};
+// 256 x 256 output tiles on CTA pairs (cta_group::2), for experts with hundreds of rows: each CTA has 128 rows on its M side
+// and loads half of the tile's 256 weight columns, 38 KiB per stage where the kernel above loads 54 for the same MMAs (scales:
+// its own rows' and all columns').  Five stages fit next to staging tiles for sixteen epilogue warps of 64 columns each:
+// with eight of 128 the latency of their arithmetic held the SwiGLU form back (8 stages of K: 13 us a tile, now 6).  Rows past
+// an expert's count are left out: a CTA without rows loads its peer's and stores nothing.
+// One B200, 32 experts x 7168 x 2048, 2048 rows each, W13 / W2: 804 / 567 -> 745 / 541 us, under the power cap 1984 -> 1907 us
+// a layer.  Bound: operand loads (without the epilogue 684 / 389 us, without the loads of A and B 596 / 388) and the hand-over of
+// the one accumulator, about 2000 cycles a tile; a second one does not fit next to the scales.  16 rows x 128 bytes per store
+// instead of 32 x 64 took W2 to 571.
+constexpr int kN4PairEpilogue = 16;   // epilogue warps
+constexpr int kN4PairThreads = (3 + kN4PairEpilogue) * 32;  // and TMA warp, MMA warp, accumulator watcher
+constexpr uint32_t kN4PairBBytes = 128 * 128;  // a CTA loads half of the tile's weight columns
+constexpr uint32_t kN4PairStage = kN4ABytes + kN4PairBBytes + 3 * kN4SfBytes;  // 38 KiB
+constexpr int kN4PairStages = 5;
+constexpr uint32_t kN4PairSfCols = 48;  // scale columns per stage slot after the accumulator: 16 of A, 32 of B
+constexpr size_t kN4PairSmem = kN4PairStages * kN4PairStage + kN4PairEpilogue * kStaging64Bytes + 1024;
+static_assert(kN4BN + kN4PairStages * kN4PairSfCols <= kN4TmemCols, "scale columns do not fit");
+
+__device__ __forceinline__ N4Tile n4_pair_decode(int tile, int& e, const int* tile_start, const int* off, const int* rows) {
+  while (tile >= tile_start[e + 1]) ++e;
+  const int local = tile - tile_start[e];
+  const int m_tiles = (rows[e] + 2 * kN4BM - 1) / (2 * kN4BM);
+  N4Tile t;
+  t.e = e;
+  t.n_blk = local / m_tiles;
+  t.row0 = off[e] + (local - t.n_blk * m_tiles) * 2 * kN4BM;
+  t.row_end = off[e] + rows[e];
+  return t;
+}
+
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kN4PairThreads, 1)
+    nvfp4_pair_kernel(const __grid_constant__ N4Params p) {
+  if (p.cond != nullptr && *p.cond == 0) return;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+
+  __shared__ uint64_t full_bar[kN4PairStages];
+  __shared__ uint64_t empty_bar[kN4PairStages];
+  __shared__ uint64_t tmem_full_bar;
+  __shared__ uint64_t tmem_empty_bar;
+  __shared__ uint32_t tmem_base_slot;
+  __shared__ uint32_t s_stop[2];  // where the producer and the issuer stopped
+  __shared__ int abort_flag;
+  __shared__ volatile int s_first_bad;  // first of this CTA's tiles whose accumulator never came
+  __shared__ int s_off[kN4MaxGroups + 1];
+  __shared__ int s_rows[kN4MaxGroups];  // rows of the group that are worked on
+  __shared__ int s_tile_start[kN4MaxGroups + 1];
+
+  const int warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31;
+  const int n_tiles = (p.N + kN4BN - 1) / kN4BN;
+  constexpr int stages = kN4PairStages;
+  const uint32_t rank = cluster_ctarank();
+  const int first_tile = blockIdx.x >> 1, tile_step = gridDim.x >> 1;
+
+  for (int i = threadIdx.x; i <= p.e_local; i += blockDim.x) {
+    const int v = p.expert_offsets[i];
+    s_off[i] = v < p.max_rows ? v : p.max_rows;
+  }
+  if (threadIdx.x == 0) {
+    abort_flag = 0;
+    s_first_bad = kNoBadTile;
+    for (int s = 0; s < kN4PairStages; ++s) {
+      mbar_init(&full_bar[s], 1);
+      mbar_init(&empty_bar[s], 1);
+    }
+    mbar_init(&tmem_full_bar, 1);
+    mbar_init(&tmem_empty_bar, 2 * kN4PairEpilogue);  // the leader's: the epilogue warps of both CTAs
+    mbar_fence_init();
+  }
+  __syncthreads();
+  if (warp == 0) {
+    int running = 0;
+    for (int e0 = 0; e0 < p.e_local; e0 += 32) {
+      const int e = e0 + lane;
+      int tiles = 0;
+      if (e < p.e_local) {
+        const int count = p.expert_counts ? p.expert_counts[e] : p.max_rows;
+        const int rows = bs_group_rows(s_off[e], s_off[e + 1], count);
+        s_rows[e] = rows;
+        if (count > 0 && s_off[e + 1] > s_off[e] && !bs_group_aligned(s_off[e]))
+          set_status(p.status, kCapacityExceeded, -1, e, s_off[e]);  // groups must be 128-padded
+        tiles = ((rows + 2 * kN4BM - 1) / (2 * kN4BM)) * n_tiles;
+      }
+      int incl = tiles;
+#pragma unroll
+      for (int d = 1; d < 32; d <<= 1) {
+        const int t = __shfl_up_sync(0xffffffffu, incl, d);
+        if (lane >= d) incl += t;
+      }
+      if (e < p.e_local) s_tile_start[e] = running + incl - tiles;
+      running += __shfl_sync(0xffffffffu, incl, 31);
+    }
+    if (lane == 0) s_tile_start[p.e_local] = running;
+  }
+  if (warp == 1) {
+    tmem_alloc_pair(&tmem_base_slot, kN4TmemCols);
+    tmem_relinquish_pair();
+  }
+  if (warp == 0 && lane == 0) {
+    tma_prefetch_desc(&p.tm_a);
+    tma_prefetch_desc(&p.tm_b);
+    tma_prefetch_desc(&p.tm_sfa);
+    tma_prefetch_desc(&p.tm_sfb);
+  }
+  tcgen05_fence_before();
+  __syncthreads();
+  cluster_sync();  // both CTAs' barriers exist before either is signalled from the other
+  tcgen05_fence_after();
+  const uint32_t tmem_base = uniform(tmem_base_slot);
+  const int total_tiles = uniform(s_tile_start[p.e_local]);
+  const uint32_t ring = uniform(smem_u32(smem));
+
+  if (warp == 0) {
+    // ======================= producer =======================
+    const bool elected = elect_one();
+    int stage = 0;
+    uint32_t phase = 0;
+    int e = 0;
+    const int64_t a_off = p.a_off ? *p.a_off : 0, sfa_off = p.sfa_off ? *p.sfa_off : 0;
+    const int a_line0 = uniform(static_cast<int>(a_off >> 7)), sfa_line0 = uniform(static_cast<int>(sfa_off >> 7));
+    const int sfa_x = uniform(static_cast<int>((sfa_off >> 4) & 7) * 4);  // word of its line that the scales start at
+    const int col_blocks = (p.N + 127) >> 7;  // 128-wide blocks of the B side
+    constexpr int kSfLines = kN4SfBytes / 128;
+    const uint32_t lead_full = uniform(cluster_addr(smem_u32(&full_bar[0]), 0));
+    bool ok = true;
+    for (int tile = first_tile; tile < total_tiles && ok; tile += tile_step) {
+      const N4Tile t = n4_pair_decode(tile, e, s_tile_start, s_off, s_rows);
+      const bool second = uniform(t.n_blk * 2 + 1 < col_blocks ? 1 : 0) != 0;  // the tile's upper 128 columns exist
+      // Groups end at multiples of 128: where the odd CTA has no rows it loads those of the even one.
+      const int row = uniform(t.row0 + kN4BM * static_cast<int>(rank) < t.row_end ? t.row0 + kN4BM * static_cast<int>(rank) : t.row0);
+      const int w_row = uniform(t.e * p.N + t.n_blk * kN4BN + 128 * static_cast<int>(rank));
+      const int sfa_line = uniform(sfa_line0 + (row >> 7) * p.col_atoms * 4);
+      const int sfb_line = uniform(static_cast<int>(t.e * (p.sfb_group_bytes >> 7)) + t.n_blk * 2 * p.col_atoms * 4);
+#pragma unroll 1
+      for (int kb = 0; kb < p.k_iters; ++kb) {
+        ok = warp_mbar_wait(&empty_bar[stage], phase ^ 1u, &abort_flag);
+        if (!ok) break;
+        uint8_t* sa = smem + stage * kN4PairStage;
+        uint8_t* sb = sa + kN4ABytes;
+        uint8_t* ssa = sb + kN4PairBBytes;
+        uint8_t* ssb = ssa + kN4SfBytes;
+        const uint32_t full = lead_full + stage * 8;
+        if (elected) {
+          if (rank == 0)
+            mbar_arrive_expect_tx(&full_bar[stage], 2 * (kN4ABytes + kN4PairBBytes + (second ? 3 : 2) * kN4SfBytes));
+          tma_load_3d_pair(sa, &p.tm_a, 0, a_line0 + kb, row, full);
+          tma_load_2d_pair(sb, &p.tm_b, kb * 128, w_row, full);
+          tma_load_2d_pair(ssa, &p.tm_sfa, sfa_x, sfa_line + kb * kSfLines, full);
+          tma_load_2d_pair(ssb, &p.tm_sfb, 0, sfb_line + kb * kSfLines, full);
+          if (second) tma_load_2d_pair(ssb + kN4SfBytes, &p.tm_sfb, 0, sfb_line + (p.col_atoms * 4 + kb * kSfLines), full);
+        }
+        __syncwarp();
+        if (++stage == stages) {
+          stage = 0;
+          phase ^= 1u;
+        }
+      }
+    }
+    if (lane == 0) s_stop[0] = ring_stop(stage, phase);
+    __syncwarp();
+  } else if (warp == 1) {
+    // ======================= MMA issuer =======================
+    // The warp that issues the MMAs copies a stage's scale atoms right before them, as in the kernel above.
+    if (rank == 0) {
+      const bool elected = elect_one();
+      constexpr uint32_t kDescHi = (1024u >> 4) | (1u << 14) | (2u << 29);  // SBO 1024, version 1, 128-byte swizzle
+      constexpr uint32_t kStep = 32u >> 4, kLbo = (16u >> 4) << 16;
+      constexpr uint32_t idesc = umma_idesc_blockscaled(kN4BN, 1, 0, 0, 0, 0, 2 * kN4BM);
+      const uint32_t full0 = uniform(smem_u32(&full_bar[0])), empty0 = uniform(smem_u32(&empty_bar[0]));
+      const uint32_t tfull = uniform(smem_u32(&tmem_full_bar));
+      int stage = 0;
+      uint32_t phase = 0, ready = 0;  // ready: the current stage is known to be there
+      int it = 0;
+      bool ok = true;
+      for (int tile = first_tile; tile < total_tiles; tile += tile_step, ++it) {
+        ok = warp_mbar_wait(&tmem_empty_bar, (it & 1u) ^ 1u, &abort_flag);  // the epilogue has drained the accumulator
+        if (!ok) break;
+        tcgen05_fence_after();
+#pragma unroll 1
+        for (int kb = 0; kb < p.k_iters; ++kb) {
+          if (!__all_sync(0xffffffffu, ready)) {
+            ok = warp_mbar_wait(&full_bar[stage], phase, &abort_flag);
+            if (!ok) break;
+          }
+          tcgen05_fence_after();
+          const uint32_t a_addr = ring + stage * kN4PairStage;
+          const uint32_t a_lo = ((a_addr & 0x3ffffu) >> 4) | kLbo, b_lo = (((a_addr + kN4ABytes) & 0x3ffffu) >> 4) | kLbo;
+          const uint32_t sf_lo = sf_desc_lo(a_addr + kN4ABytes + kN4PairBBytes);
+          const uint32_t sfa_t = tmem_base + kN4BN + stage * kN4PairSfCols;
+          const uint32_t sfb_t = sfa_t + 16u;
+          const uint32_t empty = empty0 + stage * 8;
+          if (++stage == stages) {
+            stage = 0;
+            phase ^= 1u;
+          }
+          ready = mbar_test(full0 + stage * 8, phase);
+          if (elected) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              tmem_cp_sf_lo_pair(sfa_t + 4 * j, sf_lo + j * kSfAtomWords);
+              tmem_cp_sf_lo_pair(sfb_t + 8 * j, sf_lo + (4 + j) * kSfAtomWords);
+              tmem_cp_sf_lo_pair(sfb_t + 8 * j + 4, sf_lo + (8 + j) * kSfAtomWords);
+            }
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+              umma_nvf4_lo_pair(tmem_base, a_lo + j * kStep, b_lo + j * kStep, kDescHi, idesc, sfa_t + 4 * j, sfb_t + 8 * j,
+                           (kb > 0 || j > 0) ? 1u : 0u);
+            tcgen05_commit_pair(empty);
+          }
+          __syncwarp();
+        }
+        if (!ok) break;
+        if (elected) tcgen05_commit_pair(tfull);
+        __syncwarp();
+      }
+      if (lane == 0) s_stop[1] = ring_stop(stage, phase);
+    }
+    __syncwarp();
+  } else if (warp == 2 + kN4PairEpilogue) {
+    // ======================= accumulator watcher =======================
+    // Polls the accumulator-ready barrier for the epilogue warps and releases them through a hardware named barrier;
+    // after a timeout it releases them once more and stops.
+    bool ok = true;
+    int it = 0;
+    for (int tile = first_tile; tile < total_tiles && ok; tile += tile_step, ++it) {
+      if (lane == 0) ok = handover_report(&s_first_bad, it, mbar_wait(&tmem_full_bar, it & 1u, &abort_flag));
+      ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
+      asm volatile("bar.arrive %0, %1;" ::"r"(handover_barrier(it)), "r"(kN4PairEpilogue * 32 + 32) : "memory");
+    }
+  } else {
+    // ======================= epilogue =======================
+    // Four warps per TMEM lane quadrant, each owning 64 of the tile's 256 columns.  A lane reads its own accumulator row, the
+    // warp hands the accumulator back at once, and 32 x 32 blocks are transposed through its staging tile and stored as
+    // 64-byte row segments while the next tile's MMAs run.
+    const int ew = warp - 2;
+    const int quad = warp & 3;
+    const int c0 = (ew >> 2) * 64;  // first of this warp's columns
+    const int row_in_tile = static_cast<int>(rank) * kN4BM + quad * 32 + lane;
+    const uint32_t lead_empty = cluster_addr(smem_u32(&tmem_empty_bar), 0);
+    const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + c0;
+    uint8_t* stg = smem + stages * kN4PairStage + ew * kStaging64Bytes;
+    int e = 0, it = 0;
+    bool ok = true;
+    const int64_t c_off = p.c_off ? *p.c_off : 0;
+    const int64_t h2_off = p.h2_off ? *p.h2_off : 0;
+    const float* row_inv =
+        p.row_inv_base ? reinterpret_cast<const float*>(p.row_inv_base + (p.row_inv_off ? *p.row_inv_off : 0)) : nullptr;
+    const bool scaled = row_inv != nullptr || p.expert_inv != nullptr;
+    for (int tile = first_tile; tile < total_tiles && ok; tile += tile_step, ++it) {
+      const N4Tile t = n4_pair_decode(tile, e, s_tile_start, s_off, s_rows);
+      const int row = t.row0 + row_in_tile;
+      const bool row_ok = row < t.row_end;
+      const float scale = row_inv != nullptr && row_ok ? row_inv[row] : 1.0f;
+      const float escale = p.expert_inv ? p.expert_inv[t.e] : 1.0f;
+      // where this lane's row goes: h2 (and h1) with SwiGLU, C or the scatter destination otherwise
+      uint64_t my_row = 0, my_h1 = 0;
+      const int F = p.N / 2;
+      if (row_ok) {
+        if (p.swiglu) {
+          my_row = reinterpret_cast<uint64_t>(p.h2_base) + h2_off + static_cast<uint64_t>(row) * F * 2;
+          if (p.c_base) my_h1 = reinterpret_cast<uint64_t>(p.c_base) + c_off + static_cast<uint64_t>(row) * p.N * 2;
+        } else if (p.scatter_ptrs != nullptr) {
+          my_row = static_cast<uint64_t>(p.scatter_ptrs[row]);
+        } else {
+          my_row = reinterpret_cast<uint64_t>(p.c_base) + c_off + static_cast<uint64_t>(row) * p.N * 2;
+        }
+      }
+      asm volatile("bar.sync %0, %1;" ::"r"(handover_barrier(it)), "r"(kN4PairEpilogue * 32 + 32) : "memory");  // released by the watcher
+      ok = handover_good(&s_first_bad, it);  // the same for every epilogue warp
+      if (!ok) break;
+      tcgen05_fence_after();
+      uint32_t ra[32], rb[32];
+      tmem_ld_32x32(taddr, ra);
+      tmem_ld_32x32(taddr + 32, rb);
+      tmem_ld_wait();
+      tcgen05_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive_cluster(lead_empty);
+      if (!__any_sync(0xffffffffu, row_ok)) continue;
+      if (!row_ok) {  // whatever pads the group: keep it off the slow path of the sigmoid
+#pragma unroll
+        for (int j = 0; j < 32; ++j) ra[j] = rb[j] = 0u;
+      }
+      // sends what the staging tile holds (32 rows x 64 bytes) to byte `at` of the rows `base` names, if the 8 columns from `col` on exist
+      auto store_block = [&](uint64_t base, int col, int limit, int64_t at) {
+        __syncwarp();
+        uint4 v[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) v[i] = stage64_get(stg, i * 8 + (lane >> 2), lane & 3);
+        __syncwarp();
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const uint64_t rp = __shfl_sync(0xffffffffu, base, i * 8 + (lane >> 2));
+          if (rp != 0 && col + 8 * (lane & 3) + 8 <= limit) store_global16(rp + at + 16 * (lane & 3), v[i]);
+        }
+      };
+      if (p.swiglu) {
+        // Columns come in groups of 16: 8 gate features then the matching 8 up features.
+        uint4 zv[4], gv[4], uv[4];
+#pragma unroll
+        for (int g = 0; g < 4; ++g) {
+          uint32_t gw[4], uw[4];
+          float gf[8], uf[8], zf[8];
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            const int b = 16 * (g & 1) + 2 * q;
+            float g0 = __uint_as_float(g < 2 ? ra[b] : rb[b]), g1 = __uint_as_float(g < 2 ? ra[b + 1] : rb[b + 1]);
+            float u0 = __uint_as_float(g < 2 ? ra[b + 8] : rb[b + 8]), u1 = __uint_as_float(g < 2 ? ra[b + 9] : rb[b + 9]);
+            if (scaled) {
+              g0 = (g0 * scale) * escale; g1 = (g1 * scale) * escale;
+              u0 = (u0 * scale) * escale; u1 = (u1 * scale) * escale;
+            }
+            gw[q] = pack_bf16x2(g0, g1);
+            uw[q] = pack_bf16x2(u0, u1);
+            gf[2 * q] = __uint_as_float(gw[q] << 16);
+            gf[2 * q + 1] = __uint_as_float(gw[q] & 0xffff0000u);
+            uf[2 * q] = __uint_as_float(uw[q] << 16);
+            uf[2 * q + 1] = __uint_as_float(uw[q] & 0xffff0000u);
+          }
+          swiglu_f32(gf, uf, zf, p.act);
+          zv[g] = make_uint4(pack_bf16x2(zf[0], zf[1]), pack_bf16x2(zf[2], zf[3]), pack_bf16x2(zf[4], zf[5]), pack_bf16x2(zf[6], zf[7]));
+          gv[g] = make_uint4(gw[0], gw[1], gw[2], gw[3]);
+          uv[g] = make_uint4(uw[0], uw[1], uw[2], uw[3]);
+        }
+        const int f0 = t.n_blk * (kN4BN / 2) + c0 / 2;  // first of this warp's 32 features
+#pragma unroll
+        for (int j = 0; j < 4; ++j) stage64_put(stg, lane, j, zv[j]);
+        store_block(my_row, f0, F, f0 * 2);
+        if (p.c_base != nullptr) {
+#pragma unroll
+          for (int j = 0; j < 4; ++j) stage64_put(stg, lane, j, gv[j]);
+          store_block(my_h1, f0, F, f0 * 2);
+#pragma unroll
+          for (int j = 0; j < 4; ++j) stage64_put(stg, lane, j, uv[j]);
+          store_block(my_h1, f0, F, (F + f0) * 2);
+        }
+      } else {
+#pragma unroll
+        for (int blk = 0; blk < 2; ++blk) {
+          uint32_t (&r)[32] = blk == 0 ? ra : rb;
+          if (scaled) {
+#pragma unroll
+            for (int j = 0; j < 32; ++j) r[j] = __float_as_uint((__uint_as_float(r[j]) * scale) * escale);
+          }
+#pragma unroll
+          for (int j = 0; j < 4; ++j) stage64_put(stg, lane, j, pack8_bf16(r + 8 * j));
+          const int col = t.n_blk * kN4BN + c0 + 32 * blk;
+          store_block(my_row, col, p.N, static_cast<int64_t>(col) * 2);
+        }
+      }
+    }
+  }
+
+  tcgen05_fence_before();
+  __syncthreads();
+  if (abort_flag && rank == 0 && threadIdx.x == 0) {  // the leader's barriers count both CTAs' loads and MMAs
+    const uint64_t deadline = globaltimer_ns() + kSettleNs;
+    settle_ring(empty_bar, stages, s_stop[1], deadline);
+    settle_ring(full_bar, stages, s_stop[0], deadline);
+  }
+  __syncwarp();
+  cluster_sync();  // neither CTA leaves while the other may still signal its barriers, or loads into either are in flight
+  if (abort_flag && threadIdx.x == 0) set_status(p.status, kPipelineTimeout, 4, blockIdx.x);
+  if (warp == 1) {
+    tcgen05_fence_after();
+    tmem_dealloc_pair(tmem_base, kN4TmemCols);
+  }
+}
+
+// What the two kernels share of the forward of dm_gemm_blockscaled (arguments checked by the entry points).
+static int n4_setup(N4Params& p, const dm_operand& a, const dm_operand& sfa, const void* w, const void* sfb, const dm_operand& c,
+                    const dm_operand& h2, const int64_t* scatter_ptrs, const dm_operand& row_scale_inv,
+                    const float* expert_scale_inv, const int32_t* expert_offsets, int e_local, int64_t max_rows, int64_t N,
+                    int64_t Kd, int swiglu_interleaved, const ActParams& act, const int* cond, int* status, int w_box_rows) {
   int rc = encode_arena_u8(&p.tm_a, a, Kd / 2, max_rows + 256, kN4BM);
   if (rc != kRcOk) return rc;
-  rc = encode_2d_u8(&p.tm_b, w, static_cast<int64_t>(e_local) * N, Kd / 2, kN4BN);
+  rc = encode_2d_u8(&p.tm_b, w, static_cast<int64_t>(e_local) * N, Kd / 2, w_box_rows);
   if (rc != kRcOk) return rc;
   p.col_atoms = static_cast<int>((Kd / 16 + 3) / 4);
   p.sfb_group_bytes = (N + 127) / 128 * 128 * static_cast<int64_t>(p.col_atoms) * 4;
@@ -468,8 +840,21 @@ int nvfp4_forward(const dm_operand& a, const dm_operand& sfa, const void* w, con
   p.N = static_cast<int>(N);
   p.k_iters = static_cast<int>(Kd / 256);
   p.swiglu = swiglu_interleaved ? 1 : 0;
-  p.direct_store = (swiglu_interleaved && !c.base) ? 1 : 0;
   p.act = act;
+  return kRcOk;
+}
+
+// The NVFP4 forward of dm_gemm_blockscaled (arguments checked there).
+int nvfp4_forward(const dm_operand& a, const dm_operand& sfa, const void* w, const void* sfb, const dm_operand& c,
+                  const dm_operand& h2, const int64_t* scatter_ptrs, const dm_operand& row_scale_inv,
+                  const float* expert_scale_inv, const int32_t* expert_offsets, int e_local, int64_t max_rows, int64_t N,
+                  int64_t Kd, int swiglu_interleaved, const ActParams& act, const int* cond, int num_sms, int* status,
+                  cudaStream_t st) {
+  N4Params p{};
+  int rc = n4_setup(p, a, sfa, w, sfb, c, h2, scatter_ptrs, row_scale_inv, expert_scale_inv, expert_offsets, e_local, max_rows,
+                    N, Kd, swiglu_interleaved, act, cond, status, kN4BN);
+  if (rc != kRcOk) return rc;
+  p.direct_store = (swiglu_interleaved && !c.base) ? 1 : 0;
   static PerDeviceOnce attr_set;
   rc = once_per_device(attr_set, [] {
     return static_cast<int>(cudaFuncSetAttribute(nvfp4_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -481,3 +866,39 @@ int nvfp4_forward(const dm_operand& a, const dm_operand& sfa, const void* w, con
 }
 
 }  // namespace dm
+
+using namespace dm;
+
+// dm_gemm_blockscaled_counted for NVFP4 experts that received many rows.
+extern "C" int dm_gemm_nvfp4_pairs(dm_operand a, dm_operand sfa, const void* w, const void* sfb, dm_operand c, dm_operand h2,
+                                   const int64_t* scatter_ptrs, dm_operand row_scale_inv, const float* expert_scale_inv,
+                                   const int32_t* expert_offsets, const int32_t* expert_counts, int e_local, int64_t max_rows,
+                                   int64_t N, int64_t Kd, int swiglu_interleaved, int clamped, float alpha, float limit,
+                                   const int* cond, int num_sms, int* status, void* stream) {
+  if (!a.base || !sfa.base || !w || !sfb || !expert_offsets || e_local <= 0 || max_rows < 0 || N <= 0 || Kd <= 0)
+    return kRcBadArg;
+  if (!swiglu_interleaved && !c.base && !scatter_ptrs) return kRcBadArg;
+  if (swiglu_interleaved && (!h2.base || scatter_ptrs)) return kRcBadArg;
+  if (e_local > kN4MaxGroups || max_rows > (1 << 30)) return kRcTooLarge;
+  if ((Kd % 256) != 0 || (N % 128) != 0 || (max_rows % 128) != 0) return kRcUnsupportedShape;
+  if (max_rows == 0) return kRcOk;
+  N4Params p{};
+  int rc = n4_setup(p, a, sfa, w, sfb, c, h2, scatter_ptrs, row_scale_inv, expert_scale_inv, expert_offsets, e_local, max_rows,
+                    N, Kd, swiglu_interleaved, ActParams{clamped, alpha, limit}, cond, status, 128);
+  if (rc != kRcOk) return rc;
+  p.expert_counts = scatter_ptrs || swiglu_interleaved ? expert_counts : nullptr;  // a dense C is written for whole groups
+  // an extent that does not hold the layout was never told in earnest: the rows alone bound the loads then
+  const int64_t layout_bytes = max_rows / 128 * static_cast<int64_t>(p.col_atoms) * 512;
+  rc = encode_sf(&p.tm_sfa, sfa.base, sfa.bytes >= layout_bytes ? sfa.bytes : int64_t{1} << 37, true, 16);
+  if (rc != kRcOk) return rc;
+  rc = encode_sf(&p.tm_sfb, sfb, e_local * p.sfb_group_bytes, false, 16);
+  if (rc != kRcOk) return rc;
+  static PerDeviceOnce attr_set;
+  rc = once_per_device(attr_set, [] {
+    return static_cast<int>(cudaFuncSetAttribute(nvfp4_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                 static_cast<int>(kN4PairSmem)));
+  });
+  if (rc != 0) return rc;
+  nvfp4_pair_kernel<<<pair_grid(num_sms), kN4PairThreads, kN4PairSmem, static_cast<cudaStream_t>(stream)>>>(p);
+  return static_cast<int>(cudaGetLastError());
+}

@@ -355,6 +355,15 @@ int dm_gemm_blockscaled_counted(int format, dm_operand a, dm_operand sfa, const 
                                 int swiglu_interleaved, int clamped, float alpha, float limit, const int* cond,
                                 int num_sms, int* status, void* stream);
 
+/* dm_gemm_blockscaled_counted for NVFP4 experts that received many rows: pairs of neighbouring SMs work on 256 x 256 tiles.
+ * Same arguments without the format.  With counts h2, an h1 next to it and scattered rows past them are not written; a dense C
+ * is written for whole groups.  An odd num_sms is used down to the next even number, 1 takes one pair. */
+int dm_gemm_nvfp4_pairs(dm_operand a, dm_operand sfa, const void* w, const void* sfb, dm_operand c, dm_operand h2,
+                        const int64_t* scatter_ptrs, dm_operand row_scale_inv, const float* expert_scale_inv,
+                        const int32_t* expert_offsets, const int32_t* expert_counts, int e_local, int64_t max_rows,
+                        int64_t N, int64_t Kd, int swiglu_interleaved, int clamped, float alpha, float limit,
+                        const int* cond, int num_sms, int* status, void* stream);
+
 /* The same product for experts that received few rows (decode): weights on the 128-row side of the MMA, the
  * expert's rows on the N side in steps of 32, so that a K stage costs MMAs of N = 32 or 64 instead of a 128-row
  * tile and the layer is bound by streaming the weights once.  Replaces the reference's compact decode tiles
