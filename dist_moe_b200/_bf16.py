@@ -21,7 +21,7 @@ from typing import Any
 import torch
 
 from . import _native as nat
-from ._call import BWD, FWD, FWD_ALL, CallState, arguments, launch, observed, recorded, span
+from ._call import BWD, FWD, FWD_ALL, CallState, Layout, arguments, launch, layout_of, observed, on_device, recorded, span
 from ._execution import ExecutionOptions, RMSNormPostprocess
 
 
@@ -41,15 +41,19 @@ class _Call(CallState):
     """Device results of routing and planning of one BF16 call."""
 
     def __init__(self, state=None, T: int = 0, with_bwd: bool = True):
-        fields = {}
-        if state is not None:
-            el, size = state.e_local, state.ep * state.e_local * T
+        if state is None:
+            super().__init__(Layout({}))
+            return
+        el, size = state.e_local, state.ep * state.e_local * T
+
+        def fields():
             i64, i32 = torch.int64, torch.int32
-            fields = {"fwd_state": (i64, 6), "need": (torch.uint8, 1), "cond": (i32, 1), "counts": (i32, el),
-                      "per_rank": (i32, state.ep), "offsets": (i32, el + 1), "fwd": (i64, size), "sct": (i64, size),
-                      "bwd": (i64, size if with_bwd else 0)}
-            self.T, self.size, self.max_rows = T, size, min(size, state.capacity_rows)
-        super().__init__(fields)
+            return {"fwd_state": (i64, 6), "need": (torch.uint8, 1), "cond": (i32, 1), "counts": (i32, el),
+                    "per_rank": (i32, state.ep), "offsets": (i32, el + 1), "fwd": (i64, size), "sct": (i64, size),
+                    "bwd": (i64, size if with_bwd else 0), "bwd_offsets": (i64, 6 if with_bwd else 0)}
+
+        super().__init__(layout_of(state, ("bf16", T, with_bwd), fields))
+        self.T, self.size, self.max_rows = T, size, min(size, state.capacity_rows)
 
     def saved(self) -> list[torch.Tensor]:
         """The state list of the registered operators, as views of the buffer."""
@@ -68,7 +72,7 @@ class _Call(CallState):
     def from_saved(state, tensors: list[torch.Tensor], T: int):
         """The call whose ``saved`` tensors these are, or None: they may be an operator's, or hooks have put them elsewhere."""
         c = _Call(state, T)
-        total, storage = c._place() // 8, tensors[7].untyped_storage()
+        total, storage = c.words, tensors[7].untyped_storage()
         if storage.nbytes() != 8 * total:
             return None
         at, base = c.at, storage.data_ptr()
@@ -100,10 +104,10 @@ def forward_impl(state, x, ids, scores, w13, w2, options: ExecutionOptions, save
                  separate: bool = False):
     """``separate``: the call's device results as tensors of their own (registered operators return them)."""
     cfg = state.config
-    T, D, F = x.shape[0], cfg.hidden_dim, cfg.intermediate_dim
+    T, F = x.shape[0], cfg.intermediate_dim
     scratch_only = (not save_for_backward) or cfg.inference or state.num_slots == 0
     c = _Call(state, T, not scratch_only).allocate(x.device, separate)
-    out = torch.empty(T, D, dtype=torch.bfloat16, device=x.device)
+    out = torch.empty(x.shape, dtype=torch.bfloat16, device=x.device)
     k = _arguments(state, c, x, ids, scores, w13, w2, options, scratch_only)
     k.out = out.data_ptr()
     clip = options.swiglu_clip_stats_out_3
@@ -157,7 +161,7 @@ def _wgrad_destination(param: torch.Tensor, shape, options: ExecutionOptions, cf
     if isinstance(explicit, torch.dtype):
         if explicit not in (torch.bfloat16, torch.float32):
             raise ValueError("wgrad_output_dtype must be torch.bfloat16 or torch.float32")
-        return torch.empty(shape, dtype=explicit, device=param.device), 0, True
+        return torch.empty(param.shape, dtype=explicit, device=param.device), 0, True
     if options.inplace_wgrad_accum:
         target = owner if owner is not None else param
         if target.grad is None:
@@ -172,7 +176,7 @@ def _wgrad_destination(param: torch.Tensor, shape, options: ExecutionOptions, cf
             raise ValueError("WGRAD owner gradient does not match the compute weight size")
         return grad, 1, False
     dtype = cfg.wgrad_dtype or param.dtype
-    return torch.empty(shape, dtype=dtype, device=param.device), 0, True
+    return torch.empty(param.shape, dtype=dtype, device=param.device), 0, True
 
 
 def backward_impl(state, c: _Call, x_shape, ids, scores, w13, w2, w13_param, w2_param, grad_out,
@@ -181,13 +185,14 @@ def backward_impl(state, c: _Call, x_shape, ids, scores, w13, w2, w13_param, w2_
     T, D, K, F, el = c.T, cfg.hidden_dim, cfg.top_k, cfg.intermediate_dim, state.e_local
     dev = grad_out.device
     need_x, need_scores, need_w13, need_w2 = needs
-    bo = torch.empty(6, dtype=torch.int64, device=dev)  # [xg, h1, h2, grad_h2, grad_h3_gathered, grad_h1]
+    # the plan's offsets: [xg, h1, h2, grad_h2, grad_h3_gathered, grad_h1]
+    bo = torch.empty(6, dtype=torch.int64, device=dev) if c.buf is None else None
     grad_scores = torch.empty(T, K, dtype=torch.float32, device=dev) if need_scores else None
     post = options.experts_output_postprocess
     is_norm = isinstance(post, RMSNormPostprocess)
     is_callback = post is not None and not is_norm  # the callable kept its own input and output (eager path)
     k = _arguments(state, c, None, ids, scores, w13, w2, options, False)
-    k.bwd_offsets, k.grad_out, k.grad_scores = bo.data_ptr(), grad_out.data_ptr(), nat.ptr(grad_scores)
+    k.bwd_offsets, k.grad_out, k.grad_scores = c.ptr("bwd_offsets") if bo is None else bo.data_ptr(), grad_out.data_ptr(), nat.ptr(grad_scores)
     # Saved expert outputs: the fused RMSNorm backward works on them in place in the communication buffer, so they are
     # copied back there; the plain backward reads them where they were saved (selected on the device).
     load_h3 = is_norm or (need_scores and not is_callback and not READ_SAVED_H3_IN_PLACE)
@@ -227,7 +232,7 @@ def backward_impl(state, c: _Call, x_shape, ids, scores, w13, w2, w13_param, w2_
             dst, k.dw2_accumulate, ret = _wgrad_destination(w2_param, (el, D, F), options, cfg, owners[1],
                                                             wgrad_explicit[1], hooks, "w2")
             k.dw2, k.dw2_is_fp32 = dst.data_ptr(), dst.dtype is torch.float32
-            grad_w2 = dst.view(w2_param.shape) if ret else None
+            grad_w2 = dst if ret else None
             steps = BWD["w2_wgrad"]
             if hooks is not None:
                 _backward(state, k, steps)
@@ -242,7 +247,7 @@ def backward_impl(state, c: _Call, x_shape, ids, scores, w13, w2, w13_param, w2_
             dst, k.dw13_accumulate, ret = _wgrad_destination(w13_param, (el, 2 * F, D), options, cfg, owners[0],
                                                              wgrad_explicit[0], hooks, "w13")
             k.dw13, k.dw13_is_fp32 = dst.data_ptr(), dst.dtype is torch.float32
-            grad_w13 = dst.view(w13_param.shape) if ret else None
+            grad_w13 = dst if ret else None
             steps |= BWD["w13_wgrad"]
             if hooks is not None:
                 _backward(state, k, steps)
@@ -298,10 +303,14 @@ def _plain_execution(*tensors) -> bool:
     which costs a small layer more than its launches."""
     if torch.compiler.is_compiling():  # first: a tracer of Python code must not meet the calls below
         return False
-    return (not recorded() and torch._C._len_torch_dispatch_stack() == 0 and torch._C._len_torch_function_stack() == 0
+    for t in tensors:
+        kind = type(t)
+        if kind is not torch.Tensor and kind is not torch.nn.Parameter:
+            return False
+    c = torch._C
+    return (not recorded() and c._len_torch_dispatch_stack() == 0 and c._len_torch_function_stack() == 0
             and torch._ops._len_torch_dispatch_stack_pre_dispatch() == 0
-            and torch._C._functorch.peek_interpreter_stack() is None and torch._C._get_tracing_state() is None
-            and all(type(t) is torch.Tensor or type(t) is torch.nn.Parameter for t in tensors))
+            and c._functorch.peek_interpreter_stack() is None and c._get_tracing_state() is None)
 
 
 class _RegisteredBf16Function(torch.autograd.Function):
@@ -317,10 +326,8 @@ class _RegisteredBf16Function(torch.autograd.Function):
         clip = options.swiglu_clip_stats_out_3
         ctx.context, ctx.options = context, options
         if clip is None and _plain_execution(x, ids, scores, w13_param, w2_param):
-            cfg = context.config
-            w13 = w13_param.detach().reshape(state.e_local, 2 * cfg.intermediate_dim, cfg.hidden_dim)
-            w2 = w2_param.detach().reshape(state.e_local, cfg.hidden_dim, cfg.intermediate_dim)
-            out, call = forward_impl(state, x.detach().contiguous(), ids, scores.detach(), w13, w2, options, True)
+            # gradients are off here, and of the weights only the address counts (sizes and layout have been checked)
+            out, call = forward_impl(state, x, ids, scores, w13_param, w2_param, options, True)
             # What a call saves must not depend on the way it goes where saved-tensor hooks look at it: activation
             # checkpointing compares a forward with its repetition, which may run under other modes.
             hooked = torch._C._autograd._top_saved_tensors_default_hooks(False) is not None
@@ -340,12 +347,11 @@ class _RegisteredBf16Function(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, grad_out):
-        from . import _ops
-
         ids, scores, w13_param, w2_param, *st = ctx.saved_tensors
         context, options = ctx.context, ctx.options
         cfg, state = context.config, context._state
-        needs = (ctx.needs_input_grad[0], ctx.needs_input_grad[2], ctx.needs_input_grad[3], ctx.needs_input_grad[4])
+        need = ctx.needs_input_grad
+        needs = (need[0], need[2], need[3], need[4])
         e_local, D, F = state.e_local, cfg.hidden_dim, cfg.intermediate_dim
         destinations = (cfg.wgrad_dtype or w13_param.dtype,) * 2
         if options.inplace_wgrad_accum:
@@ -360,14 +366,19 @@ class _RegisteredBf16Function(torch.autograd.Function):
         if not torch.is_grad_enabled() and _plain_execution(grad_out, ids, scores, w13_param, w2_param, st[0]):
             if context._closed:
                 raise RuntimeError(f"distributed MoE context {context._context_id} is not live")
-            call = whole or _ops._unpack_bf16_state(state, st, ids.shape[0])
-            w13, w2 = w13_param.detach().reshape(e_local, 2 * F, D), w2_param.detach().reshape(e_local, D, F)
-            with torch.cuda.device(state.device):
-                gx, gs, g13, g2 = backward_impl(state, call, grad_out.shape, ids, scores.detach(), w13, w2, w13_param,
+            call = whole
+            if call is None:
+                from . import _ops
+
+                call = _ops._unpack_bf16_state(state, st, ids.shape[0])
+            with on_device(state.device):
+                gx, gs, g13, g2 = backward_impl(state, call, grad_out.shape, ids, scores, w13_param, w2_param, w13_param,
                                                 w2_param, grad_out.contiguous(), options, needs, destinations)
             if options.inplace_wgrad_accum:
                 torch.autograd.graph.increment_version(destinations)  # as the operator's mutated arguments
             return gx, None, gs, g13, g2, None, None
+        from . import _ops
+
         if whole is not None:
             st = whole.saved()
         rms = _rmsnorm_args(options.experts_output_postprocess)

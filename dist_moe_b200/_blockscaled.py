@@ -40,7 +40,7 @@ from typing import Any
 import torch
 
 from . import _native as nat
-from ._call import BWD, FWD, FWD_ALL, CallState, arguments, launch, observed, span
+from ._call import BWD, FWD, FWD_ALL, CallState, arguments, launch, layout_of, observed, on_device, span
 from ._execution import ExecutionOptions, PreparedWeight, RMSNormPostprocess
 from .formats import BlockScaledFormat, format_constants
 
@@ -531,11 +531,15 @@ class _PlannedCall(CallState):
     def __init__(self, state, T: int, p13, p2):
         K, el, ep = state.config.top_k, state.e_local, state.ep
         size = max((ep * T * min(K, el) + el * 127 + 127) // 128 * 128, 128)
-        i64, i32 = torch.int64, torch.int32
-        # fwd_state: [x, -, h1, -, h3, x_row, x_col, h2_row, h2_col, slot]; real: rows per expert before the padding to 128
-        super().__init__({"fwd_state": (i64, 10), "fwd_table": (i64, 18), "need": (torch.uint8, 1), "cond": (i32, 1),
-                          "counts": (i32, el), "real": (i32, el), "per_rank": (i32, ep), "offsets": (i32, el + 1),
-                          "fwd": (i64, size), "bwd": (i64, size), "sct": (i64, size)})
+
+        def fields():
+            i64, i32 = torch.int64, torch.int32
+            # fwd_state: [x, -, h1, -, h3, x_row, x_col, h2_row, h2_col, slot]; real: rows per expert before the padding to 128
+            return {"fwd_state": (i64, 10), "fwd_table": (i64, 18), "need": (torch.uint8, 1), "cond": (i32, 1),
+                    "counts": (i32, el), "real": (i32, el), "per_rank": (i32, ep), "offsets": (i32, el + 1),
+                    "fwd": (i64, size), "bwd": (i64, size), "sct": (i64, size)}
+
+        super().__init__(layout_of(state, ("mxfp8", T), fields))
         self.T, self.size, self.max_rows = T, size, min(size, state.capacity_rows // 128 * 128)
         self.p13, self.p2 = p13, p2
 
@@ -620,7 +624,7 @@ def _mxfp8_backward_planned(state, c: _PlannedCall, x_shape, ids, scores, w13_pa
         dst, k.dw2_accumulate, ret = _wgrad_destination(w2_param, (el, D, F), options, cfg, owners[1], wgrad_explicit[1],
                                                         hooks, "w2")
         k.dw2, k.dw2_is_fp32 = dst.data_ptr(), dst.dtype is torch.float32
-        grad_w2 = dst.view(w2_param.shape) if ret else None
+        grad_w2 = dst if ret else None
         steps = BWD["w2_wgrad"]
         if hooks is not None:
             run(steps)
@@ -636,7 +640,7 @@ def _mxfp8_backward_planned(state, c: _PlannedCall, x_shape, ids, scores, w13_pa
         dst, k.dw13_accumulate, ret = _wgrad_destination(w13_param, (el, 2 * F, D), options, cfg, owners[0],
                                                          wgrad_explicit[0], hooks, "w13")
         k.dw13, k.dw13_is_fp32 = dst.data_ptr(), dst.dtype is torch.float32
-        grad_w13 = dst.view(w13_param.shape) if ret else None
+        grad_w13 = dst if ret else None
         steps |= BWD["w13_wgrad"]
         if hooks is not None:
             run(steps)
@@ -792,7 +796,7 @@ def _mxfp8_backward(state, c: _TrainCall, x_shape, ids, scores, w13_param, w2_pa
         nat.check(nat.lib.dm_gemm_blockscaled_wgrad(dyc, dycsf, full(c.h2_col), full(c.h2_col_sf), dst.data_ptr(),
                                                     int(dst.dtype == torch.float32), acc, offs, el, R, D, F, None,
                                                     state.num_sms, status, st), "dm_gemm_blockscaled_wgrad(w2)")
-        grad_w2 = dst.view(w2_param.shape) if ret else None
+        grad_w2 = dst if ret else None
     # ---- SwiGLU backward, W13 ---------------------------------------------------------------
     if need_x or need_w13:
         # grad_h1 goes straight from the SwiGLU backward arithmetic into its quantised copies
@@ -810,7 +814,7 @@ def _mxfp8_backward(state, c: _TrainCall, x_shape, ids, scores, w13_param, w2_pa
         nat.check(nat.lib.dm_gemm_blockscaled_wgrad(d1c, d1csf, full(c.x_col), full(c.x_col_sf), dst.data_ptr(),
                                                     int(dst.dtype == torch.float32), acc, offs, el, R, 2 * F, D, None,
                                                     state.num_sms, status, st), "dm_gemm_blockscaled_wgrad(w13)")
-        grad_w13 = dst.view(w13_param.shape) if ret else None
+        grad_w13 = dst if ret else None
     grad_x = None
     # unconditional, as in the reference (dist_moe/api.py:2580): peers may still be reading this rank's combine buffer
     state.barrier(state.dispatch)
@@ -831,8 +835,8 @@ class _Mxfp8Function(torch.autograd.Function):
         planned = PLANNED_ARENA and state.num_slots > 0 and options.swiglu_clip_stats_out_3 is None
         with span("dist_moe_forward"):
             forward = _mxfp8_forward_planned if planned else _mxfp8_forward
-            out, call = forward(state, x.detach().contiguous(), ids, scores.detach(), p13, p2, options,
-                                need_h3=scores.requires_grad)
+            # gradients are off here, x and the scores are contiguous (checked by the caller)
+            out, call = forward(state, x, ids, scores, p13, p2, options, need_h3=scores.requires_grad)
         ctx.state, ctx.call, ctx.options, ctx.x_shape = state, call, options, x.shape
         ctx.save_for_backward(ids, scores, w13_param, w2_param)
         return out
@@ -840,10 +844,11 @@ class _Mxfp8Function(torch.autograd.Function):
     @staticmethod
     def backward(ctx, grad_out):
         ids, scores, w13_param, w2_param = ctx.saved_tensors
-        needs = (ctx.needs_input_grad[0], ctx.needs_input_grad[2], ctx.needs_input_grad[3], ctx.needs_input_grad[4])
-        with torch.cuda.device(ctx.state.device), span("dist_moe_backward"):
+        need = ctx.needs_input_grad
+        needs = (need[0], need[2], need[3], need[4])
+        with on_device(ctx.state.device), span("dist_moe_backward"):
             backward = _mxfp8_backward_planned if ctx.call.planned else _mxfp8_backward
-            gx, gs, gw13, gw2 = backward(ctx.state, ctx.call, ctx.x_shape, ids, scores.detach(), w13_param, w2_param,
+            gx, gs, gw13, gw2 = backward(ctx.state, ctx.call, ctx.x_shape, ids, scores, w13_param, w2_param,
                                          grad_out.contiguous(), ctx.options, needs)
         return gx, None, gs, gw13, gw2, None, None, None, None
 
@@ -885,7 +890,7 @@ class _EagerMxfp8Function(torch.autograd.Function):
         # handed back in the sources' shapes
         w13, w2, call.p13, call.p2 = _EagerMxfp8Function._weights(options, w13_source, w2_source, state)
         needs = (ctx.needs_input_grad[0], ctx.needs_input_grad[2], ctx.needs_input_grad[3], ctx.needs_input_grad[4])
-        with torch.cuda.device(state.device), span("dist_moe_backward"):
+        with on_device(state.device), span("dist_moe_backward"):
             gx, gs, g13, g2 = _mxfp8_backward_planned(state, call, ctx.x_shape, ids, scores.detach(), w13, w2,
                                                       grad_out.contiguous(), options, needs, hooks=ctx.hooks)
         if g13 is not None:

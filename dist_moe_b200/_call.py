@@ -6,12 +6,16 @@ ranges, GEMMs timed in place) and passes with Python callbacks between launches 
 launch, a tensor per result and the dispatcher around the registered operators made small layers wait for the host: forward and
 backward of 16 tokens (D = F = 256, 8 experts) 656 -> 301 us, of 1531 tokens (D = 1088, F = 704, 24 experts, recomputed) 674 ->
 330 us, MXFP8 of 777 tokens with tensor weights 580 -> 397 us.
+What was left in Python (views and detached copies of tensors whose address alone was used, the layout of a call's results laid
+out twice per pass, device guards for the device that is current, imports inside functions) took 50 of 147 us of the first: 294 ->
+249 us; MXFP8 of 777 tokens 388 -> 351.
 """
 
 from __future__ import annotations
 
 import ctypes
 import os
+import sys
 
 import torch
 from torch.profiler import record_function
@@ -52,11 +56,18 @@ def _recorder_query():
 recorded = _recorder_query()
 
 
+def _profile() -> list | None:
+    """``_bf16.PROFILE`` of this moment (that module imports this one)."""
+    bf16 = sys.modules.get(_BF16)
+    return None if bf16 is None else bf16.PROFILE
+
+
+_BF16 = __package__ + "._bf16"
+
+
 def observed() -> bool:
     """Someone wants to see the parts of a pass."""
-    from . import _bf16
-
-    return _bf16.PROFILE is not None or recorded()
+    return _profile() is not None or recorded()
 
 
 class _NoSpan:
@@ -67,15 +78,21 @@ class _NoSpan:
         return False
 
 
+_NOTHING = _NoSpan()
+
+
 def span(name: str):
     """A profiler range with the reference's name (dist_moe/api.py:1979-2443), free where nothing records."""
-    return record_function(name) if recorded() else _NoSpan()
+    return record_function(name) if recorded() else _NOTHING
+
+
+def on_device(device: torch.device):
+    """``torch.cuda.device``, free where the device is the current one already."""
+    return _NOTHING if torch._C._cuda_getDevice() == device.index else torch.cuda.device(device)
 
 
 def launch(fn, names: dict, state, k, steps: int) -> None:
     """Run the given steps of a sequence: one call, or one per step where they are timed in place."""
-    from . import _bf16
-
     context, st = state.native_layer(), nat.stream_ptr()
 
     def run(bits: int) -> None:
@@ -86,10 +103,11 @@ def launch(fn, names: dict, state, k, steps: int) -> None:
             failed = next((n for n, bit in names.items() if bit == report[1]), "arguments")
             nat.check(rc, f"{fn.__name__}({failed})")
 
-    timed = _TIMED[fn.__name__]
-    if _bf16.PROFILE is None:
+    profile = _profile()
+    if profile is None:
         run(steps)
         return
+    timed = _TIMED[fn.__name__]
     for name, bit in names.items():
         if not steps & bit:
             continue
@@ -100,35 +118,46 @@ def launch(fn, names: dict, state, k, steps: int) -> None:
         start.record()
         run(bit)
         end.record()
-        _bf16.PROFILE.append((timed[name], start, end))
+        profile.append((timed[name], start, end))
+
+
+class Layout:
+    """Where the device results of a call lie in their buffer.  ``fields``: name -> (dtype, elements)."""
+
+    def __init__(self, fields: dict):
+        self.fields, self.at, off = fields, {}, 0
+        for name, (dtype, n) in fields.items():
+            self.at[name] = off
+            off += (n * dtype.itemsize + 15) & ~15
+        self.words = off // 8
+
+
+def layout_of(state, key: tuple, fields) -> Layout:
+    """The layout of this kind of call, built by ``fields()`` unless the context's last call was of the same kind."""
+    last = getattr(state, "_call_layout", None)
+    if last is None or last[0] != key:
+        last = state._call_layout = (key, Layout(fields()))  # one assignment: threads may call in turn
+    return last[1]
 
 
 class CallState:
-    """Device results of routing and planning of one call: one buffer (``buf``) that the names of ``fields`` are views of, or
-    tensors of their own where a registered operator hands them out.  ``fields``: name -> (dtype, elements)."""
+    """Device results of routing and planning of one call: one buffer (``buf``) that the names of the layout are views of, or
+    tensors of their own where a registered operator hands them out."""
 
-    def __init__(self, fields: dict):
-        self.fields, self.buf, self.at = fields, None, {}
+    def __init__(self, layout: Layout):
+        self.fields, self.at, self.words, self.buf = layout.fields, layout.at, layout.words, None
         self.rstd = self.callback_state = None
-
-    def _place(self) -> int:
-        off = 0
-        for name, (dtype, n) in self.fields.items():
-            self.at[name] = off
-            off += (n * dtype.itemsize + 15) & ~15
-        return off
 
     def allocate(self, device, separate: bool = False) -> "CallState":
         if separate:
             for name, (dtype, n) in self.fields.items():
                 setattr(self, name, torch.empty(n, dtype=dtype, device=device) if n else None)
         else:
-            self.buf = torch.empty(self._place() // 8, dtype=torch.int64, device=device)
+            self.buf = torch.empty(self.words, dtype=torch.int64, device=device)
         return self
 
     def adopt(self, buf: torch.Tensor) -> "CallState":
         """The results that an earlier call has left in ``buf``."""
-        self._place()
         self.buf = buf
         return self
 
@@ -157,10 +186,17 @@ def arguments(state, c: CallState, x, ids, scores, options) -> "nat.LayerCall":
         k.x = x.data_ptr()
     k.ids, k.ids_are_int64 = ids.data_ptr(), ids.dtype is torch.int64
     k.scores, k.scores_are_bf16 = scores.data_ptr(), scores.dtype is torch.bfloat16
-    ptr = c.ptr
-    k.counts, k.per_rank, k.expert_offsets = ptr("counts"), ptr("per_rank"), ptr("offsets")
-    k.fwd_ptrs, k.bwd_ptrs, k.sct_ptrs = ptr("fwd"), ptr("bwd"), ptr("sct")
-    k.need, k.cond, k.fwd_state = ptr("need"), ptr("cond"), ptr("fwd_state")
+    if c.buf is None:
+        ptr = c.ptr
+        k.counts, k.per_rank, k.expert_offsets = ptr("counts"), ptr("per_rank"), ptr("offsets")
+        k.fwd_ptrs, k.bwd_ptrs, k.sct_ptrs = ptr("fwd"), ptr("bwd"), ptr("sct")
+        k.need, k.cond, k.fwd_state = ptr("need"), ptr("cond"), ptr("fwd_state")
+    else:
+        base, at = c.buf.data_ptr(), c.at
+        k.counts, k.per_rank, k.expert_offsets = base + at["counts"], base + at["per_rank"], base + at["offsets"]
+        k.fwd_ptrs, k.sct_ptrs = base + at["fwd"], base + at["sct"]
+        k.bwd_ptrs = base + at["bwd"] if c.fields["bwd"][1] else None
+        k.need, k.cond, k.fwd_state = base + at["need"], base + at["cond"], base + at["fwd_state"]
     k.T, k.ptrs_size, k.max_rows = c.T, c.size, c.max_rows
     k.num_layers, k.validate_ids = state.num_layers_in_slot, options.validate_expert_ids
     return k

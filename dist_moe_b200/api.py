@@ -587,13 +587,16 @@ def _validate_inputs(x, ids, scores, w13, w2, context: Context, *, prepared: boo
     if not 1 <= T <= context.max_num_local_input_tokens:
         raise ValueError(
             f"x_TD has {T} tokens; the context accepts 1..{context.max_num_local_input_tokens} local tokens")
-    if tuple(ids.shape) != (T, context.top_k) or tuple(scores.shape) != (T, context.top_k):
+    if ids.shape != (T, context.top_k) or scores.shape != (T, context.top_k):
         raise ValueError(f"topk_expert_ids_TK and topk_scores_TK must have shape {(T, context.top_k)}")
     tensors = (x, ids, scores) if prepared else (x, ids, scores, w13, w2)
-    if any(t.device != x.device for t in tensors) or x.device.type != "cuda":
-        raise ValueError("all operation tensors must reside on the same CUDA device")
-    if any(not t.is_contiguous() for t in tensors):
-        raise ValueError("all operation tensors must be contiguous")
+    device = x.device
+    for t in tensors:
+        if t.device != device or device.type != "cuda":
+            raise ValueError("all operation tensors must reside on the same CUDA device")
+    for t in tensors:
+        if not t.is_contiguous():
+            raise ValueError("all operation tensors must be contiguous")
 
 
 def routed_experts(x_TD: torch.Tensor, topk_expert_ids_TK: torch.Tensor, topk_scores_TK: torch.Tensor,
@@ -635,8 +638,10 @@ def routed_experts(x_TD: torch.Tensor, topk_expert_ids_TK: torch.Tensor, topk_sc
     if context.config.inference and grads:
         raise RuntimeError("inference contexts do not support autograd")
     save_for_backward = torch.is_grad_enabled() and bool(grads)
+    from ._call import on_device
+
     # every launch below goes to the context's device and to that device's current stream
-    with torch.cuda.device(state.device):
+    with on_device(state.device):
         if context.config.block_scaled is not None:
             from ._blockscaled import run_block_scaled
 
