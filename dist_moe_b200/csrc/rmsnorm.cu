@@ -7,14 +7,18 @@
 // (dist_moe/kernels/norm/fused_rmsnorm_combine.py:427-466); the backward is its autograd:
 //   grad_s[t,k]    = <y[t,k,:], go[t,:]>
 //   grad_h3[t,k,:] = rstd * s * (go - y * <go, y> / D)
-// HBM bound: forward reads h3 once from DRAM (the second pass of a token's K rows hits L1),
-// backward reads h3 and go once and writes grad_h3 in place.
+// HBM bound: forward reads h3 once (a token's K rows stay in shared memory, or hit L1 in the second pass where they do not
+// fit), backward reads h3 and go once and writes grad_h3 in place.
+#include <type_traits>
+
 #include "common.cuh"
 #include "../../include/dist_moe_b200.h"
 
 namespace dm {
 
 constexpr int kNormMaxK = 32;
+constexpr int kNormBlocks = 4;                // resident blocks of the staged form, at most
+constexpr int64_t kNormStaged = 216 * 1024;  // rows in the shared memory of an SM
 
 __device__ __forceinline__ void up8(const uint4& v, float (&f)[8]) {
   const uint32_t w[4] = {v.x, v.y, v.z, v.w};
@@ -147,6 +151,151 @@ __global__ void __launch_bounds__(256) rmsnorm_combine_fwd_kernel(
   }
 }
 
+// The same sums in the same order with a token's K rows, which are contiguous, in shared memory: one bulk copy per token, the next
+// token's on its way while this one is worked on.  The kernel above has two loads of a thread in flight, reads every row twice and
+// looks at its options for every element (17 instructions each; issue-bound once the loads overlap: 41 us in the first example
+// below); here they are template parameters, and four rows are summed and reduced side by side.  One B200, us: T = 4096, K = 4, D =
+// 2816 61 -> 29; K = 8: D = 1024 53 -> 24, 4096 129 -> 62, 7168 235 -> 160 (one block per SM); T = 16, K = 4, D = 2816 8.4 -> 4.0.
+// Bound: HBM (92 MB in 29 us, 0.6 of the copy rate) and the three barriers of a token.
+template <typename IdT, bool kGamma, bool kNorm16, bool kKahan>
+__global__ void __launch_bounds__(256, kNormBlocks) rmsnorm_combine_fwd_staged_kernel(
+    const uint4* __restrict__ h3, const void* scores, int scores_bf16, const IdT* __restrict__ ids,
+    const uint4* __restrict__ gamma, float gain_center, float eps, int, uint4* __restrict__ out,
+    float* __restrict__ rstd_out, int64_t T, int K, int vec, uint8_t* save_base, const int64_t* save_offset,
+    const int* save_cond, int save_expect, int, int buffers) {
+  extern __shared__ __align__(128) uint8_t smem[];
+  __shared__ uint64_t full[2];
+  __shared__ int abort_flag;
+  __shared__ float part[kNormMaxK][8];
+  __shared__ float partc[kNormMaxK][8];
+  __shared__ float rs[kNormMaxK];
+  __shared__ float ws[kNormMaxK];
+  bool save = save_base != nullptr;
+  if (save && save_cond != nullptr) save = ((*save_cond != 0) == (save_expect != 0));
+  if (save && save_offset != nullptr) save = *save_offset >= 0;
+  uint4* save_dst = save ? reinterpret_cast<uint4*>(save_base + (save_offset ? *save_offset : 0)) : nullptr;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const float inv_d = 1.0f / static_cast<float>(vec * 8);
+  const int rows = K * vec;  // vectors of a token
+  const uint32_t bytes = static_cast<uint32_t>(rows) * 16;
+  auto fetch = [&](int64_t t, int b) {
+    mbar_arrive_expect_tx(&full[b], bytes);
+    bulk_load(smem + b * bytes, h3 + t * rows, bytes, &full[b]);
+  };
+  if (threadIdx.x == 0) {
+    abort_flag = 0;
+    mbar_init(&full[0], 1);
+    mbar_init(&full[1], 1);
+    mbar_fence_init();
+    fence_proxy_async_smem();
+    if (blockIdx.x < T) fetch(blockIdx.x, 0);
+  }
+  __syncthreads();
+  int b = 0, it = 0;
+  for (int64_t t = blockIdx.x; t < T; t += gridDim.x, ++it) {
+    const int64_t ahead = t + gridDim.x;
+    if (buffers == 2 && threadIdx.x == 0 && ahead < T) fetch(ahead, b ^ 1);  // every thread has left that buffer
+    if (threadIdx.x < K) {
+      const int64_t route = t * K + threadIdx.x;
+      ws[threadIdx.x] = scores_bf16 ? __bfloat162float(static_cast<const __nv_bfloat16*>(scores)[route])
+                                    : static_cast<const float*>(scores)[route];
+    }
+    const bool valid = threadIdx.x < K && ids[t * K + threadIdx.x] >= 0;
+    const uint32_t parity = buffers == 2 ? (it >> 1) & 1 : it & 1;
+    uint4* src = reinterpret_cast<uint4*>(smem + b * bytes);
+    if (!mbar_wait(&full[b], parity, &abort_flag))  // a copy that never came (none is known to): fetch the rows by hand
+      for (int v = threadIdx.x; v < rows; v += 256) src[v] = h3[t * rows + v];  // each thread reads what it has written alone
+    // four rows at a time: their loads, sums and reductions overlap
+    for (int k0 = 0; k0 < K; k0 += 4) {
+      float ss[4] = {0.f, 0.f, 0.f, 0.f}, cc[4] = {0.f, 0.f, 0.f, 0.f};
+      for (int v = threadIdx.x; v < vec; v += 256) {
+        uint4 raw[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) raw[q] = k0 + q < K ? src[(k0 + q) * vec + v] : make_uint4(0, 0, 0, 0);
+        float g[8];
+        if (kGamma) {
+          up8(gamma[v], g);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) g[j] += gain_center;
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          if (save && k0 + q < K) save_dst[t * rows + (k0 + q) * vec + v] = raw[q];
+          float h[8];
+          up8(raw[q], h);
+          if (kGamma) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) h[j] *= g[j];
+          }
+          if (kKahan) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) kahan_add(ss[q], cc[q], __fmul_rn(h[j], h[j]));
+          } else {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) ss[q] += h[j] * h[j];
+          }
+        }
+      }
+#pragma unroll
+      for (int q = 0; q < 4; ++q) warp_reduce_sumsq(ss[q], cc[q], kKahan);
+      if (lane == 0) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+          if (k0 + q < K) {
+            part[k0 + q][warp] = ss[q];
+            partc[k0 + q][warp] = cc[q];
+          }
+      }
+    }
+    __syncthreads();
+    if (threadIdx.x < K) {
+      float ss = 0.f;
+      if (kKahan) {
+        float cc = 0.f;
+#pragma unroll
+        for (int w = 0; w < 8; ++w) two_sum_merge(ss, cc, part[threadIdx.x][w], partc[threadIdx.x][w]);
+        ss = __fsub_rn(ss, cc);
+      } else {
+#pragma unroll
+        for (int w = 0; w < 8; ++w) ss += part[threadIdx.x][w];
+      }
+      const float r = valid ? rsqrtf(ss * inv_d + eps) : 0.f;
+      rs[threadIdx.x] = valid ? r : -1.0f;  // rsqrtf is never negative: a route that is left out
+      if (rstd_out != nullptr) rstd_out[t * K + threadIdx.x] = r;
+    }
+    __syncthreads();
+    for (int v = threadIdx.x; v < vec; v += 256) {
+      float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+      float g[8];
+      if (kGamma) {
+        up8(gamma[v], g);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) g[j] += gain_center;
+      }
+#pragma unroll 4
+      for (int k = 0; k < K; ++k) {
+        const float r = rs[k], w = ws[k];
+        if (r < 0.0f) continue;
+        float h[8];
+        up8(src[k * vec + v], h);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          float y = (kGamma ? h[j] * g[j] : h[j]) * r;
+          if (kNorm16) y = round_bf16(y);
+          acc[j] += y * w;
+        }
+      }
+      out[t * vec + v] = make_uint4(pack_bf16x2(acc[0], acc[1]), pack_bf16x2(acc[2], acc[3]),
+                                    pack_bf16x2(acc[4], acc[5]), pack_bf16x2(acc[6], acc[7]));
+    }
+    __syncthreads();
+    if (buffers == 2)
+      b ^= 1;
+    else if (threadIdx.x == 0 && ahead < T)
+      fetch(ahead, 0);
+  }
+}
+
 // One warp per route.  h3 may alias grad_h3 (each lane reads a chunk before it writes it).
 template <typename IdT>
 __global__ void __launch_bounds__(256) rmsnorm_combine_bwd_kernel(
@@ -237,19 +386,39 @@ extern "C" int dm_rmsnorm_combine_fwd(const void* h3, const void* scores, int sc
                                       int save_expect, void* stream) {
   if (!h3 || !scores || !ids || !out || T <= 0 || K <= 0 || K > kNormMaxK || D <= 0 || (D % 8) != 0) return kRcBadArg;
   const int vec = static_cast<int>(D / 8);
-  const int blocks = static_cast<int>(T < grid_cap(8) ? T : grid_cap(8));
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (ids_are_int64)
-    rmsnorm_combine_fwd_kernel<int64_t><<<blocks, 256, 0, st>>>(
-        static_cast<const uint4*>(h3), scores, scores_are_bf16, static_cast<const int64_t*>(ids),
-        static_cast<const uint4*>(gamma), gain_center, eps, norm_is_bf16, static_cast<uint4*>(out), rstd_out, T, K, vec,
-        static_cast<uint8_t*>(save_base), save_offset, save_cond, save_expect, use_kahan ? 1 : 0);
-  else
-    rmsnorm_combine_fwd_kernel<int32_t><<<blocks, 256, 0, st>>>(
-        static_cast<const uint4*>(h3), scores, scores_are_bf16, static_cast<const int32_t*>(ids),
-        static_cast<const uint4*>(gamma), gain_center, eps, norm_is_bf16, static_cast<uint4*>(out), rstd_out, T, K, vec,
-        static_cast<uint8_t*>(save_base), save_offset, save_cond, save_expect, use_kahan ? 1 : 0);
-  return static_cast<int>(cudaGetLastError());
+  auto run = [&](auto kernel, auto* typed_ids, int per_sm, size_t smem, auto... more) {
+    const int blocks = static_cast<int>(T < grid_cap(per_sm) ? T : grid_cap(per_sm));
+    kernel<<<blocks, 256, smem, st>>>(static_cast<const uint4*>(h3), scores, scores_are_bf16, typed_ids,
+                                      static_cast<const uint4*>(gamma), gain_center, eps, norm_is_bf16, static_cast<uint4*>(out),
+                                      rstd_out, T, K, vec, static_cast<uint8_t*>(save_base), save_offset, save_cond, save_expect,
+                                      use_kahan ? 1 : 0, more...);
+    return static_cast<int>(cudaGetLastError());
+  };
+  auto choose = [&](auto* typed_ids) {
+    using IdT = std::remove_const_t<std::remove_pointer_t<decltype(typed_ids)>>;
+    const int64_t bytes = K * D * 2;
+    if (bytes > kNormStaged) return run(rmsnorm_combine_fwd_kernel<IdT>, typed_ids, 8, 0);
+    const int buffers = 4 * bytes <= kNormStaged ? 2 : 1;  // two where two blocks of them fit on an SM
+    const int64_t fit = (kNormStaged + 4096) / (buffers * bytes + 4096);  // resident blocks; a block's tables take under 4 KiB
+    auto staged = [&](auto gamma_tag, auto norm_tag, auto kahan_tag) {
+      constexpr auto kernel =
+          rmsnorm_combine_fwd_staged_kernel<IdT, decltype(gamma_tag)::value, decltype(norm_tag)::value, decltype(kahan_tag)::value>;
+      static PerDeviceOnce attr_set;
+      const int rc = once_per_device(attr_set, [] {
+        return static_cast<int>(
+            cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kNormStaged)));
+      });
+      if (rc != 0) return rc;
+      return run(kernel, typed_ids, static_cast<int>(fit < kNormBlocks ? fit : kNormBlocks),
+                 static_cast<size_t>(buffers * bytes), buffers);
+    };
+    // The options are template parameters: looked at for every element they made the kernel issue-bound.
+    auto with_kahan = [&](auto g, auto n) { return use_kahan ? staged(g, n, std::true_type{}) : staged(g, n, std::false_type{}); };
+    auto with_norm = [&](auto g) { return norm_is_bf16 ? with_kahan(g, std::true_type{}) : with_kahan(g, std::false_type{}); };
+    return gamma ? with_norm(std::true_type{}) : with_norm(std::false_type{});
+  };
+  return ids_are_int64 ? choose(static_cast<const int64_t*>(ids)) : choose(static_cast<const int32_t*>(ids));
 }
 
 extern "C" int dm_rmsnorm_combine_bwd(const void* grad_out, const void* scores, int scores_are_bf16, const void* ids,
