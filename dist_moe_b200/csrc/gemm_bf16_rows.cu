@@ -44,8 +44,7 @@ constexpr int kRwBM = 128;    // output columns per CTA of a pair (weights, M si
 constexpr int kRwBK = 64;     // K of a stage (128 bytes per row)
 constexpr int kRwMaxStages = 10;
 constexpr int kRwThreads = 512;
-constexpr int kRwGatherUnitRows = 8;                                        // rows one gather warp pulls before it reports
-constexpr int kRwGatherUnitsPerBlock = kRwGatherBlock / kRwGatherUnitRows;  // reports that make a 128-row block ready
+constexpr int kRwGatherWarps = 4;
 constexpr int kRwMaxGroups = 256;
 constexpr uint32_t kRwWBytes = kRwBM * kRwBK * 2;  // 16 KiB
 constexpr uint32_t kRwTmemCols = 512;
@@ -89,6 +88,34 @@ __device__ __forceinline__ uint32_t rw_pair(uint32_t w, int odd) {
   return __byte_perm(w, o, odd ? 0x3276 : 0x5410);
 }
 
+// Pulls the `live` rows of a unit, kRows at a time (lane l holds row l's pointer, null: zeros), kLoads 16-byte pieces of each in
+// flight per lane.
+template <int kRows, int kLoads>
+__device__ __forceinline__ void rw_pull(uint64_t my_ptr, int live, uint4* dst, int vec_per_row, int lane) {
+  for (int rr = 0; rr < live; rr += kRows) {
+    const uint4* src[kRows];
+#pragma unroll
+    for (int i = 0; i < kRows; ++i) src[i] = reinterpret_cast<const uint4*>(__shfl_sync(0xffffffffu, my_ptr, (rr + i) & 31));
+    for (int v0 = 0; v0 < vec_per_row; v0 += 32 * kLoads) {
+      uint4 b[kRows][kLoads];
+#pragma unroll
+      for (int i = 0; i < kRows; ++i)
+#pragma unroll
+        for (int j = 0; j < kLoads; ++j) {
+          const int v = v0 + j * 32 + lane;
+          b[i][j] = (rr + i < live && src[i] != nullptr && v < vec_per_row) ? __ldcg(src[i] + v) : make_uint4(0, 0, 0, 0);
+        }
+#pragma unroll
+      for (int i = 0; i < kRows; ++i)
+#pragma unroll
+        for (int j = 0; j < kLoads; ++j) {
+          const int v = v0 + j * 32 + lane;
+          if (rr + i < live && v < vec_per_row) dst[static_cast<int64_t>(rr + i) * vec_per_row + v] = b[i][j];
+        }
+    }
+  }
+}
+
 template <int kMode>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kRwThreads, 1) rows_gemm_kernel(const __grid_constant__ RowsParams p) {
   if (p.cond != nullptr && *p.cond == 0) return;
@@ -105,11 +132,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kRwThreads, 1) rows_
   __shared__ volatile int s_first_bad;  // first of this CTA's tiles whose accumulator never came
   __shared__ uint32_t s_stop[3];  // where the weight producer, the row producer and the issuer stopped
   __shared__ int s_box;
+  __shared__ int s_unit;
   __shared__ int s_off[kRwMaxGroups + 1];
   __shared__ int s_tile_start[kRwMaxGroups + 1];
   __shared__ uint16_t s_per[kRwMaxGroups];
 
   constexpr bool kSwiglu = kMode == kRowsSwiglu;
+  constexpr int kTableBarrier = 1 + kHandoverBarriers + 2;  // after those of the hand-over and of the two epilogue groups
   constexpr uint32_t kRing = kSwiglu ? kRwRingFused : kRwRingPlain;
   constexpr uint32_t kStaging = kSwiglu ? kRwStageFused : kRwStagePlain;
   const int warp = threadIdx.x >> 5;
@@ -117,11 +146,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kRwThreads, 1) rows_
   const uint32_t rank = cluster_ctarank();
   const int first_tile = blockIdx.x >> 1, tile_step = gridDim.x >> 1;
 
-  // The first gather warp's unit, on its way while the tables are built; the other three draw only where there are more
-  // units than CTAs.  32 decoding tokens (24 units of 8 rows, 208 us in all) take 0.3 us longer than with units dealt out
-  // by CTA index, 0.8 us longer when all four warps draw, 1.4 us when a CTA draws four units at once.
-  int unit = 0;
-  if (warp == 10 && lane == 0 && p.gather_flags != nullptr) unit = atomicAdd(p.gather_ticket, 1);
+  // The gather warps' first units, four neighbouring ones per CTA, so that the rows of the first tiles come from the CTAs that
+  // started first.
+  if (warp == 10 && lane == 0 && p.gather_flags != nullptr) s_unit = atomicAdd(p.gather_ticket, kRwGatherWarps);
+  const int64_t a_off = p.a_off ? *p.a_off : 0;
 
   // ---- tile table -----------------------------------------------------------
   const int m_pairs = kSwiglu ? (p.N / 2) / 128 : (p.N + 2 * kRwBM - 1) / (2 * kRwBM);
@@ -147,10 +175,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kRwThreads, 1) rows_
     tmem_relinquish_pair();
   }
   __syncthreads();
+  cluster_arrive();  // this CTA's barriers exist
+  const bool gathers = warp >= 10 && warp < 10 + kRwGatherWarps && p.gather_flags != nullptr;
   if (warp == 0) {
     if (lane == 0) {
       tma_prefetch_desc(&p.tm_w);
-      tma_prefetch_desc(&p.tm_x[kRwBoxes - 1]);
     }
     int running = 0, box = 0;
     for (int e0 = 0; e0 < p.e_local; e0 += 32) {
@@ -181,8 +210,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kRwThreads, 1) rows_
     }
   }
   tcgen05_fence_before();
-  __syncthreads();
-  cluster_sync();  // both CTAs' barriers exist before either is signalled from the other
+  if (gathers) {
+    // The gather warps need none of it and start at once, before the weights fill the memory system.  A barrier of its own: at
+    // the one of __syncthreads they could arrive again, at the end of the kernel, before the tables are there.
+    asm volatile("bar.arrive %0, %1;" ::"n"(kTableBarrier), "n"(kRwThreads) : "memory");
+  } else {
+    asm volatile("bar.sync %0, %1;" ::"n"(kTableBarrier), "n"(kRwThreads) : "memory");
+    cluster_wait();  // both CTAs' barriers exist before either is signalled from the other
+  }
   tcgen05_fence_after();
   const uint32_t tmem_base = uniform(tmem_base_slot);
   const int total_tiles = uniform(s_tile_start[p.e_local]);
@@ -190,8 +225,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kRwThreads, 1) rows_
   const uint32_t stage_bytes = kRwWBytes + static_cast<uint32_t>(rw_box_rows(uniform(s_box))) * 128;
   const int fit = static_cast<int>(kRing / stage_bytes);
   const int stages = fit < kRwMaxStages ? fit : kRwMaxStages;
-
-  const int64_t a_off = p.a_off ? *p.a_off : 0;
 
   if (warp == 0 || warp == 15) {
     // ======================= TMA producers: warp 0 the weights, warp 15 the rows =======================
@@ -204,6 +237,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kRwThreads, 1) rows_
     bool ok = true;
     const int total_rows = s_off[p.e_local];
     const int k_iters = p.Kd / kRwBK;
+    const int ready = kRwGatherBlock / rw_gather_unit_rows(total_rows, static_cast<int>(gridDim.x) * kRwGatherWarps);
+    if (rows_side && elected) tma_prefetch_desc(&p.tm_x[s_box]);
     const uint32_t lead_full = uniform(cluster_addr(smem_u32(&full_bar[0]), 0));
     for (int tile = first_tile; tile < total_tiles; tile += tile_step) {
       const RowsTile t = rw_decode(tile, e, s_tile_start, s_off, s_per);
@@ -216,7 +251,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kRwThreads, 1) rows_
         if (b <= need.last) {
           const uint64_t t0 = globaltimer_ns();
           uint32_t spins = 0;
-          while (ld_acquire_gpu(p.gather_flags + b) < kRwGatherUnitsPerBlock) {
+          while (ld_acquire_gpu(p.gather_flags + b) < ready) {
             if ((++spins & 0xff) == 0 &&
                 (*const_cast<volatile int*>(&abort_flag) || globaltimer_ns() - t0 > 2000000000ull)) {
               abort_flag = 1;
@@ -228,7 +263,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kRwThreads, 1) rows_
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
         __syncwarp();             // what the polling lanes acquired is ordered before the elected lane's loads
-        fence_proxy_async_all();  // rows were written with ordinary stores, TMA reads them through the async proxy
+        fence_proxy_async_global();  // rows were written with ordinary stores, TMA reads them through the async proxy
       }
       const int box = uniform(rw_box_index(t.n));
       const CUtensorMap* tm_x = &p.tm_x[box];
@@ -346,59 +381,45 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kRwThreads, 1) rows_
     }
   } else if (warp >= 10) {
     // ======================= gather (fused dispatch) =======================
-    // Units of 8 rows go to the gather warps of the grid by ticket, in ascending row order, the order in which the tiles
-    // consume them.  Each warp pulls its unit with 16-byte loads (peer memory allowed), two rows
-    // x eight loads in flight per lane, and then bumps the counter of the unit's 128-row block; the TMA producer of
-    // whichever CTA needs a block waits for sixteen reports.  Gather warps wait on nothing, and a unit belongs only to a
-    // warp that is running: CTAs that come late, because kernels of other streams hold their SMs, delay no row that the
-    // CTAs already there are waiting for (dealt out by CTA index, such rows never came and the wait ran out).  Small units
-    // matter at the start of the launch: a warp keeps 8 KiB in flight, so over NVLink a 32-row unit took about 30 us before
-    // the first tiles could begin, an 8-row unit a quarter of that, and later units are far ahead of the MMAs anyway.
+    // Units of 1 to 8 rows go to the gather warps of the grid by ticket, in ascending row order, the order in which the tiles
+    // consume them.  Each warp pulls its unit with 16-byte loads (peer memory allowed), sixteen in flight per lane, and then bumps
+    // the counter of the unit's 128-row block; the TMA producer of whichever CTA needs a block waits for all of its units.
+    // Gather warps wait on nothing, and a unit belongs only to a warp that is running: CTAs that come late, because kernels
+    // of other streams hold their SMs, delay no row that the CTAs already there are waiting for (dealt out by CTA index,
+    // such rows never came and the wait ran out).
+    // The first tiles wait for the chain of one unit (pointer, rows, release, poll, proxy fence), so: units are as small as the
+    // number of gather warps allows, the pointers of a unit are loaded at once, the warps start before the tile table is there and
+    // with it before the weights fill the memory system, the CTAs that start first draw the first units, and the fence
+    // between the proxies names global memory alone (for all spaces it waits for the weights on their way, up to 5700 cycles).
+    // First row load after the start of the launch, cycles: 192 rows x 2048 22 900 -> 15 000, 4593 x 1088
+    // 20 000 -> 15 000, 32 x 256 12 800 -> 8800.  One B200, launches: W13 of 192 rows, 64 experts 120.5 -> 115.4 us, W13 / its
+    // repetition / W2 input gradient of 4593 rows 37.8 / 32.6 / 25.5 -> 30.1 / 28.6 / 18.2; layers 208.7 -> 204.9 and 330 -> 314.
+    // A warp keeps 8 KiB in flight: over NVLink a 32-row unit took about 30 us before the first tiles could begin, an 8-row
+    // unit a quarter of that.
     if (p.gather_flags != nullptr) {
       const int total_rows = s_off[p.e_local];
-      const int units = (total_rows + kRwGatherBlock - 1) / kRwGatherBlock * kRwGatherUnitsPerBlock;
-      if (warp != 10) {
-        unit = units;  // no more units than first warps: those are enough
-        if (units > static_cast<int>(gridDim.x) && lane == 0) unit = atomicAdd(p.gather_ticket, 1);
-      }
+      const int unit_rows = rw_gather_unit_rows(total_rows, static_cast<int>(gridDim.x) * kRwGatherWarps);
+      const int per_block = kRwGatherBlock / unit_rows;
+      const int units = (total_rows + kRwGatherBlock - 1) / kRwGatherBlock * per_block;
       const int vec_per_row = p.Kd / 8;
       uint4* dst_base = reinterpret_cast<uint4*>(p.a_base + a_off);
-      int u = uniform(unit);
+      int u = s_unit + warp - 10;
       while (u < units) {
         int next = 0;
         if (lane == 0) next = atomicAdd(p.gather_ticket, 1);  // on its way while this unit is pulled
-        const int blk = u / kRwGatherUnitsPerBlock;
-        const int r_begin = blk * kRwGatherBlock + (u % kRwGatherUnitsPerBlock) * kRwGatherUnitRows;
-        for (int rr = 0; rr < kRwGatherUnitRows; rr += 2) {
-          const int r0 = r_begin + rr, r1 = r0 + 1;
-          if (r0 >= total_rows) break;
-          const uint4* src0 = reinterpret_cast<const uint4*>(p.gather_ptrs[r0]);
-          const uint4* src1 = r1 < total_rows ? reinterpret_cast<const uint4*>(p.gather_ptrs[r1]) : nullptr;
-          uint4* dst0 = dst_base + static_cast<int64_t>(r0) * vec_per_row;
-          uint4* dst1 = dst_base + static_cast<int64_t>(r1) * vec_per_row;
-          for (int v0 = 0; v0 < vec_per_row; v0 += 256) {
-            uint4 b0[8], b1[8];
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-              const int v = v0 + j * 32 + lane;
-              b0[j] = (src0 != nullptr && v < vec_per_row) ? __ldcg(src0 + v) : make_uint4(0, 0, 0, 0);
-              b1[j] = (src1 != nullptr && v < vec_per_row) ? __ldcg(src1 + v) : make_uint4(0, 0, 0, 0);
-            }
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-              const int v = v0 + j * 32 + lane;
-              if (v < vec_per_row) {
-                dst0[v] = b0[j];
-                if (r1 < total_rows) dst1[v] = b1[j];
-              }
-            }
-          }
-        }
-        __threadfence();
-        __syncwarp();
-        if (lane == 0) red_release_gpu_add(p.gather_flags + blk, 1);
+        const int r_begin = u * unit_rows, left = total_rows - r_begin, live = left < unit_rows ? left : unit_rows;
+        const uint64_t ptr = lane < live ? static_cast<uint64_t>(p.gather_ptrs[r_begin + lane]) : 0;
+        uint4* dst = dst_base + static_cast<int64_t>(r_begin) * vec_per_row;
+        if (vec_per_row > 128)
+          rw_pull<2, 8>(ptr, live, dst, vec_per_row, lane);
+        else
+          rw_pull<4, 4>(ptr, live, dst, vec_per_row, lane);
+        __syncwarp();  // all lanes' rows are stored before the release below
+        if (lane == 0) red_release_gpu_add(p.gather_flags + u / per_block, 1);
         u = uniform(next);
       }
+      __syncwarp();
+      cluster_wait();  // the other half of the arrival above
     }
   } else {
     // ======================= epilogue =======================

@@ -127,6 +127,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kBrThreads, 1)
   const int lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();
   const int first_tile = blockIdx.x >> 1, tile_step = gridDim.x >> 1;
+  const int64_t x_off = p.x_off ? *p.x_off : 0, sfx_off = p.sfx_off ? *p.sfx_off : 0;  // on their way while the tables are built
 
   // ---- tile table ---------------------------------------------------------------------------------------------------
   const int m_pairs = (p.N + 2 * kBrBM - 1) / (2 * kBrBM);
@@ -152,6 +153,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kBrThreads, 1)
     tmem_relinquish_pair();
   }
   __syncthreads();
+  cluster_arrive();  // this CTA's barriers exist
   if (warp == 0) {
     if (lane == 0) {
       tma_prefetch_desc(&p.tm_w);
@@ -192,7 +194,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kBrThreads, 1)
   }
   tcgen05_fence_before();
   __syncthreads();
-  cluster_sync();  // both CTAs' barriers exist before either is signalled from the other
+  cluster_wait();  // both CTAs' barriers exist before either is signalled from the other
   tcgen05_fence_after();
   const uint32_t tmem_base = uniform(tmem_base_slot);
   const int total_tiles = uniform(s_tile_start[p.e_local]);
@@ -219,7 +221,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kBrThreads, 1)
     int stage = 0;
     uint32_t phase = 0;
     int e = 0;
-    const int64_t x_off = p.x_off ? *p.x_off : 0, sfx_off = p.sfx_off ? *p.sfx_off : 0;
     if (rows_side && lane == 0 && ((x_off & 127) | (sfx_off & 15)) != 0) set_status(p.status, kCapacityExceeded, -2, 0, 0);
     const int x_line0 = uniform(static_cast<int>(x_off >> 7)), sfx_line0 = uniform(static_cast<int>(sfx_off >> 7));
     const int sfx_x = uniform(static_cast<int>((sfx_off >> 4) & 7) * 4);  // word of its line that the scales start at

@@ -130,13 +130,21 @@ __global__ void __launch_bounds__(kSwThreads, kSwCtasPerSm) blockscaled_swapped_
       set_status(p.status, kCapacityExceeded, -1, i, s_off[i]);  // groups must be 128-padded
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    int acc = 0;
-    for (int e = 0; e < p.e_local; ++e) {
-      s_tile_start[e] = acc;
-      acc += ((s_cnt[e] + kSwTileRows - 1) / kSwTileRows) * m_tiles;
+  if (warp == 0) {
+    int running = 0;
+    for (int e0 = 0; e0 < p.e_local; e0 += 32) {
+      const int e = e0 + lane;
+      const int tiles = e < p.e_local ? ((s_cnt[e] + kSwTileRows - 1) / kSwTileRows) * m_tiles : 0;
+      int incl = tiles;
+#pragma unroll
+      for (int d = 1; d < 32; d <<= 1) {
+        const int t = __shfl_up_sync(0xffffffffu, incl, d);
+        if (lane >= d) incl += t;
+      }
+      if (e < p.e_local) s_tile_start[e] = running + incl - tiles;
+      running += __shfl_sync(0xffffffffu, incl, 31);
     }
-    s_tile_start[p.e_local] = acc;
+    if (lane == 0) s_tile_start[p.e_local] = running;
   }
   if (warp == 1) {
     tmem_alloc(&tmem_base_slot, kSwTmemCols);

@@ -493,6 +493,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kN4PairThreads, 1)
   constexpr int stages = kN4PairStages;
   const uint32_t rank = cluster_ctarank();
   const int first_tile = blockIdx.x >> 1, tile_step = gridDim.x >> 1;
+  const int64_t a_off = p.a_off ? *p.a_off : 0, sfa_off = p.sfa_off ? *p.sfa_off : 0;  // on their way while the tables are built
 
   for (int i = threadIdx.x; i <= p.e_local; i += blockDim.x) {
     const int v = p.expert_offsets[i];
@@ -510,6 +511,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kN4PairThreads, 1)
     mbar_fence_init();
   }
   __syncthreads();
+  cluster_arrive();  // this CTA's barriers exist
   if (warp == 0) {
     int running = 0;
     for (int e0 = 0; e0 < p.e_local; e0 += 32) {
@@ -546,7 +548,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kN4PairThreads, 1)
   }
   tcgen05_fence_before();
   __syncthreads();
-  cluster_sync();  // both CTAs' barriers exist before either is signalled from the other
+  cluster_wait();  // both CTAs' barriers exist before either is signalled from the other
   tcgen05_fence_after();
   const uint32_t tmem_base = uniform(tmem_base_slot);
   const int total_tiles = uniform(s_tile_start[p.e_local]);
@@ -558,7 +560,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kN4PairThreads, 1)
     int stage = 0;
     uint32_t phase = 0;
     int e = 0;
-    const int64_t a_off = p.a_off ? *p.a_off : 0, sfa_off = p.sfa_off ? *p.sfa_off : 0;
     const int a_line0 = uniform(static_cast<int>(a_off >> 7)), sfa_line0 = uniform(static_cast<int>(sfa_off >> 7));
     const int sfa_x = uniform(static_cast<int>((sfa_off >> 4) & 7) * 4);  // word of its line that the scales start at
     const int col_blocks = (p.N + 127) >> 7;  // 128-wide blocks of the B side

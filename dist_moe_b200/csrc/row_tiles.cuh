@@ -16,6 +16,11 @@ constexpr int kRwMaxN = 256;          // routed rows per tile (N side of the MMA
 constexpr int kRwGatherBlock = 128;   // rows per readiness counter of the fused dispatch
 constexpr int kRwBoxes = 5;           // heights of the row boxes: the smallest one that covers half a tile is loaded
 
+// Rows of a gather unit, 1 to 8: as few as leave no gather warp more than one unit of a launch, for at least that many rows.
+DM_HOST_DEVICE constexpr int rw_gather_unit_rows(int total_rows, int warps) {
+  return total_rows <= warps ? 1 : total_rows <= 2 * warps ? 2 : total_rows <= 4 * warps ? 4 : 8;
+}
+
 // A CTA of the pair loads half of a tile's rows.
 DM_HOST_DEVICE constexpr int rw_box_rows(int i) { return i == 0 ? 16 : 32 * i; }
 DM_HOST_DEVICE constexpr int rw_box_index(int n) { return n <= 32 ? 0 : (n + 63) >> 6; }
