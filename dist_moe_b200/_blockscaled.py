@@ -334,15 +334,9 @@ def run_block_scaled(x, ids, scores, w13_weight, w2_weight, context: Any, option
     stride = packed_row_stride(fmt, D)
     dispatch = state.dispatch.local().data_ptr()
     # ---- publish: quantise straight into the packed symmetric dispatch rows ----------------
-    if lay.fp4:
-        nat.check(nat.lib.dm_quant_nvfp4_token(x.data_ptr(), None, T, D, dispatch, stride, dispatch + xq, stride, 0,
-                                               dispatch + xq + xs, stride, st), "dm_quant_nvfp4_token")
-    else:
-        nat.check(nat.lib.dm_quant_mxfp8_row(x.data_ptr(), None, T, D, dispatch, stride, dispatch + xq, stride, 0, st),
-                  "dm_quant_mxfp8_row")
-    nat.check(nat.lib.dm_publish(None, ids.data_ptr(), int(ids.dtype == torch.int64), None,
-                                 state.routing.local().data_ptr(), T, 0, K, E, int(options.validate_expert_ids),
-                                 status, st), "dm_publish")
+    nat.check(nat.lib.dm_publish_quantised(f, x.data_ptr(), ids.data_ptr(), int(ids.dtype == torch.int64), dispatch, stride,
+                                           xq, xs, state.routing.local().data_ptr(), T, D, K, E,
+                                           int(options.validate_expert_ids), status, st), "dm_publish_quantised")
     state.barrier(state.dispatch)
     # ---- routing (rows of every expert padded to 128) -----------------------------------------
     size = (ep * T * min(K, el) + el * 127 + 127) // 128 * 128
@@ -361,20 +355,20 @@ def run_block_scaled(x, ids, scores, w13_weight, w2_weight, context: Any, option
                                        state.route_workspace.data_ptr(), state.route_workspace_words, status, st),
               nat.route_call_name(ep, T, el))
     recv = offsets[el:]
-    # ---- gather + unpack -----------------------------------------------------------------------
-    none = nat.Operand(None, 0, None)
-    nat.check(nat.lib.dm_gather_packed_rows(fwd.data_ptr(), recv.data_ptr(), max_rows, xq, xs, int(lay.fp4),
-                                            _view(buf, lay.x_q), _view(buf, lay.x_sf),
-                                            _view(buf, lay.x_inv) if lay.fp4 else none, None, st),
-              "dm_gather_packed_rows")
-    # ---- W13 (+SwiGLU) ---------------------------------------------------------------------------
     fused = bool(p13._interleaved_fc13)
-    row_inv = _view(buf, lay.x_inv) if lay.fp4 else none
-    h2_quantised = False
     # few rows per expert (decode): weights on the MMA's M side, the rows on its N side
     limit_rows = _SWAPPED_MAX_ROWS[fmt] if SWAPPED_MAX_ROWS_PER_EXPERT is None else SWAPPED_MAX_ROWS_PER_EXPERT
     swapped = fused and ep * T * K <= limit_rows * E
     gemm = _gemm_pairs if lay.fp4 and ep * T * K >= _PAIR_MIN_ROWS * E else _gemm
+    # ---- gather + unpack: rows that pad a group are left alone where the GEMMs know the real ones ------------------
+    none = nat.Operand(None, 0, None)
+    counted = swapped or gemm is _gemm_pairs or not lay.fp4
+    gather = nat.lib.dm_gather_packed_rows_live if counted and fused else nat.lib.dm_gather_packed_rows
+    nat.check(gather(fwd.data_ptr(), recv.data_ptr(), max_rows, xq, xs, int(lay.fp4), _view(buf, lay.x_q),
+                     _view(buf, lay.x_sf), _view(buf, lay.x_inv) if lay.fp4 else none, None, st), "dm_gather_packed_rows")
+    # ---- W13 (+SwiGLU) ---------------------------------------------------------------------------
+    row_inv = _view(buf, lay.x_inv) if lay.fp4 else none
+    h2_quantised = False
     if swapped:
         h2_dense = lay.dense
         nat.check(nat.lib.dm_gemm_blockscaled_swapped(f, _view(buf, lay.x_q), _view(buf, lay.x_sf),

@@ -211,6 +211,8 @@ _SIGNATURES = {
     "dm_quant_nvfp4_token": (c_int, [_P, _P, c_int64, c_int64, _P, c_int64, _P, c_int64, c_int, _P, c_int64, _P]),
     "dm_quant_nvfp4_token_live": (c_int, [_P, _P, _P, c_int64, c_int64, _P, c_int64, _P, c_int64, c_int, _P, c_int64, _P]),
     "dm_gather_packed_rows": (c_int, [_P, _P, c_int64, c_int64, c_int64, c_int, Operand, Operand, Operand, _P, _P]),
+    "dm_gather_packed_rows_live": (c_int, [_P, _P, c_int64, c_int64, c_int64, c_int, Operand, Operand, Operand, _P, _P]),
+    "dm_publish_quantised": (c_int, [c_int, _P, _P, c_int, _P, c_int64, c_int64, c_int64, _P, c_int64, c_int64, c_int, c_int, c_int, _P, _P]),
     "dm_quant_nvfp4_weight": (c_int, [_P, _P, c_int64, c_int64, c_int64, _P, _P, c_int, _P]),
     "dm_sf_swizzle": (c_int, [_P, _P, c_int64, c_int64, _P]),
     "dm_gemm_fprop": (

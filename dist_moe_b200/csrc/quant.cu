@@ -13,6 +13,7 @@
 //          in the low nibble.
 #include <cuda_fp4.h>
 
+#include "publish.cuh"
 #include "quant_common.cuh"
 #include "../../include/dist_moe_b200.h"
 
@@ -53,7 +54,8 @@ __global__ void __launch_bounds__(256) mxfp8_row_kernel(const uint4* __restrict_
                                                         int64_t max_rows, int vec_per_row, uint8_t* __restrict__ q,
                                                         int64_t q_stride, uint8_t* __restrict__ scales,
                                                         int64_t s_stride, int blocked, int n_col_atoms,
-                                                        const int64_t* __restrict__ live) {
+                                                        const int64_t* __restrict__ live, IdPublish ids) {
+  publish_ids(ids);
   int64_t rows = num_rows ? *num_rows : max_rows;
   if (rows > max_rows) rows = max_rows;
   const int lane = threadIdx.x & 31;
@@ -618,8 +620,9 @@ __global__ void __launch_bounds__(128) nvfp4_token_kernel(const uint4* __restric
                                                           int64_t max_rows, int vec_per_row, uint8_t* q,
                                                           int64_t q_stride, uint8_t* s, int64_t s_stride,
                                                           uint8_t* inv, int64_t inv_stride, int blocked_atoms,
-                                                          const int64_t* __restrict__ live) {
+                                                          const int64_t* __restrict__ live, IdPublish ids) {
   __shared__ float red[4];
+  publish_ids(ids);
   int64_t rows = num_rows ? *num_rows : max_rows;
   if (rows > max_rows) rows = max_rows;
   for (int64_t r = blockIdx.x; r < rows; r += gridDim.x) {
@@ -679,8 +682,9 @@ __global__ void __launch_bounds__(256) nvfp4_token_reg_kernel(const uint4* __res
                                                               int64_t max_rows, int blocks_per_row, uint8_t* q,
                                                               int64_t q_stride, uint8_t* s, int64_t s_stride,
                                                               uint8_t* inv, int64_t inv_stride, int blocked_atoms,
-                                                              const int64_t* __restrict__ live) {
+                                                              const int64_t* __restrict__ live, IdPublish ids) {
   __shared__ float red[2][8];
+  publish_ids(ids);
   int64_t rows = num_rows ? *num_rows : max_rows;
   if (rows > max_rows) rows = max_rows;
   constexpr int kRowsPerCta = 256 / kThreads;
@@ -820,7 +824,7 @@ __global__ void __launch_bounds__(256) gather_packed_kernel(const int64_t* __res
                                                             int q_vecs, int scale_cols, int has_inv, uint8_t* q_base,
                                                             const int64_t* q_off, uint8_t* sf_base,
                                                             const int64_t* sf_off, uint8_t* inv_base,
-                                                            const int64_t* inv_off, const int* cond) {
+                                                            const int64_t* inv_off, const int* cond, int live_only) {
   if (cond != nullptr && *cond == 0) return;
   int64_t rows = *num_rows;
   if (rows > max_rows) rows = max_rows;
@@ -841,9 +845,16 @@ __global__ void __launch_bounds__(256) gather_packed_kernel(const int64_t* __res
     const int64_t blk = pair >> 4;
     const int l0 = static_cast<int>(pair & 15) * 2;
     uint32_t w[2][4];
+    int64_t srcs[8], any = 0;
 #pragma unroll
     for (int g = 0; g < 8; ++g) {
-      const int64_t src = ptrs[blk * 128 + 32 * (g >> 1) + l0 + (g & 1)];
+      srcs[g] = ptrs[blk * 128 + 32 * (g >> 1) + l0 + (g & 1)];
+      any |= srcs[g];
+    }
+    if (live_only && any == 0) continue;
+#pragma unroll
+    for (int g = 0; g < 8; ++g) {
+      const int64_t src = srcs[g];
       w[g & 1][g >> 1] = (src != 0 && c4 < atoms)
                              ? __ldcg(reinterpret_cast<const uint32_t*>(src + static_cast<int64_t>(q_vecs) * 16) + c4)
                              : 0;
@@ -859,6 +870,7 @@ __global__ void __launch_bounds__(256) gather_packed_kernel(const int64_t* __res
     const int64_t r = pieces == 1 ? i : i / pieces;
     const int piece = static_cast<int>(i - r * pieces);
     const uint8_t* src = reinterpret_cast<const uint8_t*>(ptrs[r]);
+    if (live_only && src == nullptr) continue;
     const int v0 = piece * 128 + lane;
     uint4 t[4];  // four 16-byte loads in flight per lane
 #pragma unroll
@@ -900,7 +912,7 @@ static int blocks_for(int64_t items, int threads, int cap) {
 
 using namespace dm;
 
-static int mxfp8_row_impl(const int64_t* live, const void* x, const int32_t* num_rows, int64_t max_rows, int64_t C, void* q,
+static int mxfp8_row_impl(const IdPublish& ids, const int64_t* live, const void* x, const int32_t* num_rows, int64_t max_rows, int64_t C, void* q,
                           int64_t q_row_stride, void* scales, int64_t scale_row_stride, int blocked, void* stream) {
   if (!x || !q || !scales || max_rows < 0 || C <= 0 || (C % 32) != 0) return kRcBadArg;
   if (q_row_stride == 0) q_row_stride = C;
@@ -911,21 +923,21 @@ static int mxfp8_row_impl(const int64_t* live, const void* x, const int32_t* num
   const int atoms = static_cast<int>((C / 32 + 3) / 4);
   mxfp8_row_kernel<<<blocks_for(max_rows * ((vec + 127) / 128), 8, grid_cap(8)), 256, 0, static_cast<cudaStream_t>(stream)>>>(
       static_cast<const uint4*>(x), num_rows, max_rows, vec, static_cast<uint8_t*>(q), q_row_stride,
-      static_cast<uint8_t*>(scales), scale_row_stride, blocked, atoms, live);
+      static_cast<uint8_t*>(scales), scale_row_stride, blocked, atoms, live, ids);
   return static_cast<int>(cudaGetLastError());
 }
 
 extern "C" int dm_quant_mxfp8_row(const void* x, const int32_t* num_rows, int64_t max_rows, int64_t C, void* q,
                                   int64_t q_row_stride, void* scales, int64_t scale_row_stride, int blocked,
                                   void* stream) {
-  return mxfp8_row_impl(nullptr, x, num_rows, max_rows, C, q, q_row_stride, scales, scale_row_stride, blocked, stream);
+  return mxfp8_row_impl(IdPublish{}, nullptr, x, num_rows, max_rows, C, q, q_row_stride, scales, scale_row_stride, blocked, stream);
 }
 
 extern "C" int dm_quant_mxfp8_row_live(const int64_t* row_live, const void* x, const int32_t* num_rows, int64_t max_rows,
                                        int64_t C, void* q, int64_t q_row_stride, void* scales, int64_t scale_row_stride,
                                        int blocked, void* stream) {
   if (!row_live) return kRcBadArg;
-  return mxfp8_row_impl(row_live, x, num_rows, max_rows, C, q, q_row_stride, scales, scale_row_stride, blocked, stream);
+  return mxfp8_row_impl(IdPublish{}, row_live, x, num_rows, max_rows, C, q, q_row_stride, scales, scale_row_stride, blocked, stream);
 }
 
 extern "C" int dm_quant_mxfp8_col(const void* x, const int32_t* num_rows, int64_t max_rows, int64_t C, void* q,
@@ -1094,9 +1106,9 @@ extern "C" int dm_quant_mxfp8_tile32(const void* w, int64_t experts, int64_t N, 
   return static_cast<int>(cudaGetLastError());
 }
 
-static int nvfp4_token_impl(const int64_t* live, const void* x, const int32_t* num_rows, int64_t max_rows, int64_t C, void* q,
-                                    int64_t q_row_stride, void* scales, int64_t scale_row_stride, int scales_blocked,
-                                    void* scale_inv, int64_t inv_row_stride, void* stream) {
+static int nvfp4_token_impl(const IdPublish& ids, const int64_t* live, const void* x, const int32_t* num_rows, int64_t max_rows,
+                            int64_t C, void* q, int64_t q_row_stride, void* scales, int64_t scale_row_stride,
+                            int scales_blocked, void* scale_inv, int64_t inv_row_stride, void* stream) {
   if (!x || !q || !scales || max_rows < 0 || C <= 0 || (C % 16) != 0 || (q_row_stride % 4) != 0) return kRcBadArg;
   if (scale_inv && (inv_row_stride % 4) != 0) return kRcBadArg;
   if (max_rows == 0) return kRcOk;
@@ -1108,7 +1120,7 @@ static int nvfp4_token_impl(const int64_t* live, const void* x, const int32_t* n
 #define DM_TOKEN(THREADS, BPT)                                                                                       \
   nvfp4_token_reg_kernel<THREADS, BPT><<<blocks_for(max_rows, 256 / THREADS, grid_cap(8)), 256, 0, st>>>(              \
       static_cast<const uint4*>(x), num_rows, max_rows, blocks, static_cast<uint8_t*>(q), q_row_stride,                \
-      static_cast<uint8_t*>(scales), scale_row_stride, static_cast<uint8_t*>(scale_inv), inv_row_stride, atoms, live)
+      static_cast<uint8_t*>(scales), scale_row_stride, static_cast<uint8_t*>(scale_inv), inv_row_stride, atoms, live, ids)
   if (blocks <= 512) {
     if (blocks <= 32)
       DM_TOKEN(32, 1);
@@ -1126,14 +1138,14 @@ static int nvfp4_token_impl(const int64_t* live, const void* x, const int32_t* n
   nvfp4_token_kernel<<<blocks_for(max_rows, 1, grid_cap(16)), 128, 0, static_cast<cudaStream_t>(stream)>>>(
       static_cast<const uint4*>(x), num_rows, max_rows, static_cast<int>(C / 8), static_cast<uint8_t*>(q),
       q_row_stride, static_cast<uint8_t*>(scales), scale_row_stride, static_cast<uint8_t*>(scale_inv),
-      inv_row_stride, scales_blocked ? static_cast<int>((C / 16 + 3) / 4) : 0, live);
+      inv_row_stride, scales_blocked ? static_cast<int>((C / 16 + 3) / 4) : 0, live, ids);
   return static_cast<int>(cudaGetLastError());
 }
 
 extern "C" int dm_quant_nvfp4_token(const void* x, const int32_t* num_rows, int64_t max_rows, int64_t C, void* q,
                                     int64_t q_row_stride, void* scales, int64_t scale_row_stride, int scales_blocked,
                                     void* scale_inv, int64_t inv_row_stride, void* stream) {
-  return nvfp4_token_impl(nullptr, x, num_rows, max_rows, C, q, q_row_stride, scales, scale_row_stride, scales_blocked,
+  return nvfp4_token_impl(IdPublish{}, nullptr, x, num_rows, max_rows, C, q, q_row_stride, scales, scale_row_stride, scales_blocked,
                           scale_inv, inv_row_stride, stream);
 }
 
@@ -1142,7 +1154,7 @@ extern "C" int dm_quant_nvfp4_token_live(const int64_t* row_live, const void* x,
                                          int64_t scale_row_stride, int scales_blocked, void* scale_inv,
                                          int64_t inv_row_stride, void* stream) {
   if (!row_live) return kRcBadArg;
-  return nvfp4_token_impl(row_live, x, num_rows, max_rows, C, q, q_row_stride, scales, scale_row_stride, scales_blocked,
+  return nvfp4_token_impl(IdPublish{}, row_live, x, num_rows, max_rows, C, q, q_row_stride, scales, scale_row_stride, scales_blocked,
                           scale_inv, inv_row_stride, stream);
 }
 
@@ -1166,9 +1178,9 @@ extern "C" int dm_sf_swizzle(const void* natural, void* blocked_out, int64_t row
   return static_cast<int>(cudaGetLastError());
 }
 
-extern "C" int dm_gather_packed_rows(const int64_t* ptrs, const int32_t* num_rows, int64_t max_rows, int64_t q_bytes,
-                                     int64_t scale_cols, int has_inv, dm_operand q, dm_operand scales_blocked,
-                                     dm_operand scale_inv, const int* cond, void* stream) {
+static int gather_packed_impl(int live_only, const int64_t* ptrs, const int32_t* num_rows, int64_t max_rows, int64_t q_bytes,
+                              int64_t scale_cols, int has_inv, dm_operand q, dm_operand scales_blocked,
+                              dm_operand scale_inv, const int* cond, void* stream) {
   if (!ptrs || !num_rows || !q.base || !scales_blocked.base || q_bytes <= 0 || (q_bytes % 16) != 0 || scale_cols <= 0 ||
       (scale_cols % 4) != 0 || max_rows < 0)
     return kRcBadArg;
@@ -1177,6 +1189,34 @@ extern "C" int dm_gather_packed_rows(const int64_t* ptrs, const int32_t* num_row
   gather_packed_kernel<<<blocks_for(max_rows * ((q_bytes / 16 + 127) / 128), 8, grid_cap(8)), 256, 0, static_cast<cudaStream_t>(stream)>>>(
       ptrs, num_rows, max_rows, static_cast<int>(q_bytes / 16), static_cast<int>(scale_cols), has_inv,
       static_cast<uint8_t*>(q.base), q.offset, static_cast<uint8_t*>(scales_blocked.base), scales_blocked.offset,
-      static_cast<uint8_t*>(scale_inv.base), scale_inv.offset, cond);
+      static_cast<uint8_t*>(scale_inv.base), scale_inv.offset, cond, live_only);
   return static_cast<int>(cudaGetLastError());
+}
+
+extern "C" int dm_gather_packed_rows(const int64_t* ptrs, const int32_t* num_rows, int64_t max_rows, int64_t q_bytes,
+                                     int64_t scale_cols, int has_inv, dm_operand q, dm_operand scales_blocked,
+                                     dm_operand scale_inv, const int* cond, void* stream) {
+  return gather_packed_impl(0, ptrs, num_rows, max_rows, q_bytes, scale_cols, has_inv, q, scales_blocked, scale_inv, cond, stream);
+}
+
+extern "C" int dm_gather_packed_rows_live(const int64_t* ptrs, const int32_t* num_rows, int64_t max_rows, int64_t q_bytes,
+                                          int64_t scale_cols, int has_inv, dm_operand q, dm_operand scales_blocked,
+                                          dm_operand scale_inv, const int* cond, void* stream) {
+  return gather_packed_impl(1, ptrs, num_rows, max_rows, q_bytes, scale_cols, has_inv, q, scales_blocked, scale_inv, cond, stream);
+}
+
+// What an inference call publishes, in one launch: its tokens quantised into the packed dispatch rows [q | natural scales |
+// fp32 inverse scale (NVFP4)] and its expert ids.  The launch of the ids alone took 1.4 us and a gap.
+extern "C" int dm_publish_quantised(int format, const void* x, const void* ids, int ids_are_int64, void* dispatch_local,
+                                    int64_t row_stride, int64_t q_bytes, int64_t scale_bytes, void* routing_local, int64_t T,
+                                    int64_t D, int K, int E, int validate, int* status, void* stream) {
+  if (!x || !ids || !dispatch_local || !routing_local || T <= 0 || D <= 0 || K <= 0 || E <= 0 || E > 32767 ||
+      (format != 0 && format != 1))
+    return kRcBadArg;
+  const IdPublish publish{ids, static_cast<uint8_t*>(routing_local), T * K, ids_are_int64, static_cast<int>(T), E, validate, status};
+  uint8_t* rows = static_cast<uint8_t*>(dispatch_local);
+  if (format == 0)
+    return mxfp8_row_impl(publish, nullptr, x, nullptr, T, D, rows, row_stride, rows + q_bytes, row_stride, 0, stream);
+  return nvfp4_token_impl(publish, nullptr, x, nullptr, T, D, rows, row_stride, rows + q_bytes, row_stride, 0,
+                          rows + q_bytes + scale_bytes, row_stride, stream);
 }

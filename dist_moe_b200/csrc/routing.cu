@@ -12,6 +12,7 @@
 //                 checks capacity and writes counts / per-rank totals / offsets.
 //   route_fill  : same decomposition as route_count; a row's slot is
 //                 segment offset + popc(lower warps) + popc(lower lanes).
+#include "publish.cuh"
 #include "common.cuh"
 #include "../../include/dist_moe_b200.h"
 
@@ -24,21 +25,11 @@ constexpr int kMaxExpertsSmem = 2048;
 // ---------------------------------------------------------------------------
 // Publication
 // ---------------------------------------------------------------------------
-template <typename IdT>
-__global__ void publish_kernel(const uint4* __restrict__ x, const IdT* __restrict__ ids, uint4* __restrict__ dispatch,
-                               uint8_t* __restrict__ routing, int64_t n_vec, int64_t n_ids, int T, int E, int validate,
-                               int* status) {
-  const int64_t tid = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
-  const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
-  if (tid == 0) *reinterpret_cast<int32_t*>(routing) = T;
-  int16_t* ids_out = reinterpret_cast<int16_t*>(routing + DM_ROUTING_HEADER_BYTES);
-  for (int64_t i = tid; i < n_ids; i += stride) {
-    const int64_t v = static_cast<int64_t>(ids[i]);
-    if (validate && (v < -1 || v >= E)) set_status(status, kInvalidExpertId, static_cast<int>(i), static_cast<int>(v));
-    ids_out[i] = static_cast<int16_t>(v);
-  }
+__global__ void publish_kernel(const uint4* __restrict__ x, uint4* __restrict__ dispatch, int64_t n_vec, IdPublish ids) {
+  publish_ids(ids);
   if (x != nullptr) {
-    for (int64_t i = tid; i < n_vec; i += stride) dispatch[i] = x[i];
+    const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
+    for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < n_vec; i += stride) dispatch[i] = x[i];
   }
 }
 
@@ -438,17 +429,9 @@ extern "C" int dm_publish(const void* x_bf16, const void* ids, int ids_are_int64
   int blocks = static_cast<int>((work + 255) / 256);
   if (blocks > grid_cap(16)) blocks = grid_cap(16);
   if (blocks < 1) blocks = 1;
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (ids_are_int64)
-    publish_kernel<int64_t><<<blocks, 256, 0, st>>>(static_cast<const uint4*>(x_bf16), static_cast<const int64_t*>(ids),
-                                                    static_cast<uint4*>(dispatch_local),
-                                                    static_cast<uint8_t*>(routing_local), n_vec, n_ids,
-                                                    static_cast<int>(T), E, validate, status);
-  else
-    publish_kernel<int32_t><<<blocks, 256, 0, st>>>(static_cast<const uint4*>(x_bf16), static_cast<const int32_t*>(ids),
-                                                    static_cast<uint4*>(dispatch_local),
-                                                    static_cast<uint8_t*>(routing_local), n_vec, n_ids,
-                                                    static_cast<int>(T), E, validate, status);
+  publish_kernel<<<blocks, 256, 0, static_cast<cudaStream_t>(stream)>>>(
+      static_cast<const uint4*>(x_bf16), static_cast<uint4*>(dispatch_local), n_vec,
+      IdPublish{ids, static_cast<uint8_t*>(routing_local), n_ids, ids_are_int64, static_cast<int>(T), E, validate, status});
   return static_cast<int>(cudaGetLastError());
 }
 

@@ -534,6 +534,16 @@ int dm_sf_swizzle(const void* natural, void* blocked_out, int64_t rows, int64_t 
 int dm_gather_packed_rows(const int64_t* ptrs, const int32_t* num_rows, int64_t max_rows, int64_t q_bytes,
                           int64_t scale_cols, int has_inv, dm_operand q, dm_operand scales_blocked,
                           dm_operand scale_inv, const int* cond, void* stream);
+/* ... leaving out the rows with a null pointer: what the operands hold there stays.  For products that size their work by the
+ * real rows of a group (each output row depends on its own row alone). */
+int dm_gather_packed_rows_live(const int64_t* ptrs, const int32_t* num_rows, int64_t max_rows, int64_t q_bytes,
+                               int64_t scale_cols, int has_inv, dm_operand q, dm_operand scales_blocked,
+                               dm_operand scale_inv, const int* cond, void* stream);
+/* dm_quant_mxfp8_row (format 0) or dm_quant_nvfp4_token (1) of T tokens into packed rows [q_bytes | scale_bytes | fp32 inverse
+ * scale (NVFP4)] of `row_stride` bytes, and dm_publish of their expert ids, in one launch. */
+int dm_publish_quantised(int format, const void* x, const void* ids, int ids_are_int64, void* dispatch_local,
+                         int64_t row_stride, int64_t q_bytes, int64_t scale_bytes, void* routing_local, int64_t T,
+                         int64_t D, int K, int E, int validate, int* status, void* stream);
 
 /* ---------------------------------------------------------------------------
  * Host-backed overflow scratch (dist_moe/_vmm.py:149-427 `VMMRegion`): one contiguous virtual range whose
