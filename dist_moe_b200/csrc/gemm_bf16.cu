@@ -89,6 +89,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1) wgrad_gemm_kernel(const __gri
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
 
+  const int64_t a_off = p.a_off ? *p.a_off : 0, b_off = p.b_off ? *p.b_off : 0;  // on their way while the tables are built
+
   // ---- tile table -----------------------------------------------------------
   const int n_tiles = (p.Kd + kBN - 1) / kBN;
   const int m_tiles = (p.N + kBM - 1) / kBM;
@@ -109,7 +111,6 @@ __global__ void __launch_bounds__(kGemmThreads, 1) wgrad_gemm_kernel(const __gri
     }
     mbar_fence_init();
   }
-  __syncthreads();
   for (int e = threadIdx.x; e <= p.e_local; e += blockDim.x) s_tile_start[e] = e * m_tiles * n_tiles;
   if (warp == 1) {
     tmem_alloc(&tmem_base_slot, kTmemCols);
@@ -125,8 +126,6 @@ __global__ void __launch_bounds__(kGemmThreads, 1) wgrad_gemm_kernel(const __gri
   const uint32_t tmem_base = uniform(tmem_base_slot);
   const int total_tiles = uniform(s_tile_start[p.e_local]);
 
-  const int64_t a_off = p.a_off ? *p.a_off : 0;
-  const int64_t b_off = p.b_off ? *p.b_off : 0;
 
   // Weight gradient: a stage is six 64 x 64 boxes, and one thread cannot issue six TMA loads in the time the
   // tensor cores need for the stage, so the (otherwise idle) warps 10 and 11 issue the boxes of the second

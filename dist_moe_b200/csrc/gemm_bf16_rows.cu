@@ -132,7 +132,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kRwThreads, 1) rows_
   __shared__ volatile int s_first_bad;  // first of this CTA's tiles whose accumulator never came
   __shared__ uint32_t s_stop[3];  // where the weight producer, the row producer and the issuer stopped
   __shared__ int s_box;
-  __shared__ int s_unit;
   __shared__ int s_off[kRwMaxGroups + 1];
   __shared__ int s_tile_start[kRwMaxGroups + 1];
   __shared__ uint16_t s_per[kRwMaxGroups];
@@ -146,68 +145,47 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kRwThreads, 1) rows_
   const uint32_t rank = cluster_ctarank();
   const int first_tile = blockIdx.x >> 1, tile_step = gridDim.x >> 1;
 
-  // The gather warps' first units, four neighbouring ones per CTA, so that the rows of the first tiles come from the CTAs that
-  // started first.
-  if (warp == 10 && lane == 0 && p.gather_flags != nullptr) s_unit = atomicAdd(p.gather_ticket, kRwGatherWarps);
+  // The gather warps' first units: those of the first tiles go to the CTAs that start first.
+  const bool gathers = warp >= 10 && warp < 10 + kRwGatherWarps && p.gather_flags != nullptr;
+  int unit = 0;
+  if (gathers && lane == 0) unit = atomicAdd(p.gather_ticket, 1);
   const int64_t a_off = p.a_off ? *p.a_off : 0;
 
   // ---- tile table -----------------------------------------------------------
   const int m_pairs = kSwiglu ? (p.N / 2) / 128 : (p.N + 2 * kRwBM - 1) / (2 * kRwBM);
-  for (int i = threadIdx.x; i <= p.e_local; i += blockDim.x) {
-    const int v = p.expert_offsets[i];
-    s_off[i] = v < p.max_rows ? v : p.max_rows;
-  }
-  if (threadIdx.x == 0) {
-    abort_flag = 0;
-    s_first_bad = kNoBadTile;
-    for (int s = 0; s < kRwMaxStages; ++s) {
-      mbar_init(&full_bar[s], 1);
-      mbar_init(&empty_bar[s], 1);
+  if (warp == 2) {
+    if (lane < kRwMaxStages) {
+      mbar_init(&full_bar[lane], 1);
+      mbar_init(&empty_bar[lane], 1);
     }
-    for (int b = 0; b < 2; ++b) {
-      mbar_init(&tmem_full_bar[b], 1);
-      mbar_init(&tmem_empty_bar[b], 16);  // the leader's: eight epilogue warps of both CTAs
+    if (lane < 2) {
+      mbar_init(&tmem_full_bar[lane], 1);
+      mbar_init(&tmem_empty_bar[lane], 16);  // the leader's: eight epilogue warps of both CTAs
+    }
+    if (lane == 0) {
+      abort_flag = 0;
+      s_first_bad = kNoBadTile;
     }
     mbar_fence_init();
+    __syncwarp();
   }
+  cluster_arrive();  // this CTA's barriers exist
   if (warp == 1) {
     tmem_alloc_pair(&tmem_base_slot, kRwTmemCols);
     tmem_relinquish_pair();
   }
-  __syncthreads();
-  cluster_arrive();  // this CTA's barriers exist
-  const bool gathers = warp >= 10 && warp < 10 + kRwGatherWarps && p.gather_flags != nullptr;
   if (warp == 0) {
-    if (lane == 0) {
-      tma_prefetch_desc(&p.tm_w);
-    }
-    int running = 0, box = 0;
-    for (int e0 = 0; e0 < p.e_local; e0 += 32) {
-      const int e = e0 + lane;
-      int tiles = 0;
-      if (e < p.e_local) {
-        const int rows = s_off[e + 1] - s_off[e];
-        const int nt = rw_row_tiles(rows);
-        const int per = rw_rows_per_tile(rows);
-        s_per[e] = static_cast<uint16_t>(per);
-        tiles = nt * m_pairs;
-        if (nt > 0) box = max(box, rw_box_index(per));
-      }
-      int incl = tiles;
-#pragma unroll
-      for (int d = 1; d < 32; d <<= 1) {
-        const int t = __shfl_up_sync(0xffffffffu, incl, d);
-        if (lane >= d) incl += t;
-      }
-      if (e < p.e_local) s_tile_start[e] = running + incl - tiles;
-      running += __shfl_sync(0xffffffffu, incl, 31);
-    }
+    if (lane == 0) tma_prefetch_desc(&p.tm_w);
+    int box = 0;
+    tile_tables(p.expert_offsets, nullptr, p.e_local, p.max_rows, lane, s_off, s_tile_start, [&](int e, int lo, int hi, int) {
+      const int nt = rw_row_tiles(hi - lo), per = rw_rows_per_tile(hi - lo);
+      s_per[e] = static_cast<uint16_t>(per);
+      if (nt > 0) box = max(box, rw_box_index(per));
+      return nt * m_pairs;
+    });
 #pragma unroll
     for (int d = 16; d > 0; d >>= 1) box = max(box, __shfl_xor_sync(0xffffffffu, box, d));
-    if (lane == 0) {
-      s_tile_start[p.e_local] = running;
-      s_box = box;
-    }
+    if (lane == 0) s_box = box;
   }
   tcgen05_fence_before();
   if (gathers) {
@@ -397,13 +375,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kRwThreads, 1) rows_
     // A warp keeps 8 KiB in flight: over NVLink a 32-row unit took about 30 us before the first tiles could begin, an 8-row
     // unit a quarter of that.
     if (p.gather_flags != nullptr) {
-      const int total_rows = s_off[p.e_local];
+      const int total_rows = min(p.expert_offsets[p.e_local], p.max_rows);  // the tables may not be there yet
       const int unit_rows = rw_gather_unit_rows(total_rows, static_cast<int>(gridDim.x) * kRwGatherWarps);
       const int per_block = kRwGatherBlock / unit_rows;
       const int units = (total_rows + kRwGatherBlock - 1) / kRwGatherBlock * per_block;
       const int vec_per_row = p.Kd / 8;
       uint4* dst_base = reinterpret_cast<uint4*>(p.a_base + a_off);
-      int u = s_unit + warp - 10;
+      int u = uniform(unit);
       while (u < units) {
         int next = 0;
         if (lane == 0) next = atomicAdd(p.gather_ticket, 1);  // on its way while this unit is pulled

@@ -91,8 +91,9 @@ __global__ void __launch_bounds__(kWdThreads, 1) blockscaled_wide_kernel(const _
   const int m_tiles = (p.N + kBsBM - 1) / kBsBM;
 
   for (int i = threadIdx.x; i <= p.e_local; i += blockDim.x) {
-    const int v = p.expert_offsets[i];
-    s_off[i] = v < p.max_rows ? v : p.max_rows;
+    const int v = min(p.expert_offsets[i], p.max_rows);
+    s_off[i] = v;
+    if (i < p.e_local && (v & 127) != 0) set_status(p.status, kCapacityExceeded, -1, i, v);  // rows must be 128-padded
   }
   if (threadIdx.x == 0) {
     abort_flag = 0;
@@ -105,16 +106,7 @@ __global__ void __launch_bounds__(kWdThreads, 1) blockscaled_wide_kernel(const _
     mbar_init(&tmem_empty_bar, 8);
     mbar_fence_init();
   }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int acc = 0;
-    for (int e = 0; e < p.e_local; ++e) {
-      s_tile_start[e] = acc;
-      if ((s_off[e] & 127) != 0) set_status(p.status, kCapacityExceeded, -1, e, s_off[e]);  // rows must be 128-padded
-      acc += m_tiles * n_tiles;
-    }
-    s_tile_start[p.e_local] = acc;
-  }
+  for (int e = threadIdx.x; e <= p.e_local; e += blockDim.x) s_tile_start[e] = e * m_tiles * n_tiles;
   if (warp == 1) {
     tmem_alloc(&tmem_base_slot, kBsTmemCols);
     tmem_relinquish();

@@ -131,66 +131,48 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kBrThreads, 1)
 
   // ---- tile table ---------------------------------------------------------------------------------------------------
   const int m_pairs = (p.N + 2 * kBrBM - 1) / (2 * kBrBM);
-  for (int i = threadIdx.x; i <= p.e_local; i += blockDim.x) {
-    const int v = p.expert_offsets[i];
-    s_off[i] = v < p.max_rows ? v : p.max_rows;
-  }
-  if (threadIdx.x == 0) {
-    abort_flag = 0;
-    s_first_bad = kNoBadTile;
-    for (int s = 0; s < kBrMaxStages; ++s) {
-      mbar_init(&full_bar[s], 1);
-      mbar_init(&empty_bar[s], 1);
+  if (warp == 2) {
+    if (lane < kBrMaxStages) {
+      mbar_init(&full_bar[lane], 1);
+      mbar_init(&empty_bar[lane], 1);
     }
-    for (int b = 0; b < 2; ++b) {
-      mbar_init(&tmem_full_bar[b], 1);
-      mbar_init(&tmem_empty_bar[b], 16);  // the leader's: eight epilogue warps of both CTAs
+    if (lane < 2) {
+      mbar_init(&tmem_full_bar[lane], 1);
+      mbar_init(&tmem_empty_bar[lane], 16);  // the leader's: eight epilogue warps of both CTAs
+    }
+    if (lane == 0) {
+      abort_flag = 0;
+      s_first_bad = kNoBadTile;
     }
     mbar_fence_init();
+    __syncwarp();
   }
+  cluster_arrive();  // this CTA's barriers exist
   if (warp == 1) {
     tmem_alloc_pair(&tmem_base_slot, kBrTmemCols);
     tmem_relinquish_pair();
   }
-  __syncthreads();
-  cluster_arrive();  // this CTA's barriers exist
   if (warp == 0) {
     if (lane == 0) {
       tma_prefetch_desc(&p.tm_w);
       tma_prefetch_desc(&p.tm_sfw);
       tma_prefetch_desc(&p.tm_sfx);
     }
-    int running = 0, box = 0;
-    for (int e0 = 0; e0 < p.e_local; e0 += 32) {
-      const int e = e0 + lane;
-      int tiles = 0;
-      if (e < p.e_local) {
-        const int count = p.expert_counts ? p.expert_counts[e] : p.max_rows;
-        const int rows = bs_group_rows(s_off[e], s_off[e + 1], count);
-        s_cnt[e] = rows;
-        if (count > 0 && s_off[e + 1] > s_off[e] && !bs_group_aligned(s_off[e]))
-          set_status(p.status, kCapacityExceeded, -1, e, s_off[e]);  // groups must be 128-padded
-        const int nt = rw_row_tiles(rows);
-        const int per = bs_rows_per_tile(rows);
-        s_per[e] = static_cast<uint16_t>(per);
-        tiles = nt * m_pairs;
-        if (nt > 0) box = max(box, rw_box_index(per));
-      }
-      int incl = tiles;
-#pragma unroll
-      for (int d = 1; d < 32; d <<= 1) {
-        const int t = __shfl_up_sync(0xffffffffu, incl, d);
-        if (lane >= d) incl += t;
-      }
-      if (e < p.e_local) s_tile_start[e] = running + incl - tiles;
-      running += __shfl_sync(0xffffffffu, incl, 31);
-    }
+    int box = 0;
+    tile_tables(p.expert_offsets, p.expert_counts, p.e_local, p.max_rows, lane, s_off, s_tile_start,
+                [&](int e, int lo, int hi, int count) {
+      const int rows = bs_group_rows(lo, hi, count);
+      s_cnt[e] = rows;
+      if (count > 0 && hi > lo && !bs_group_aligned(lo))
+        set_status(p.status, kCapacityExceeded, -1, e, lo);  // groups must be 128-padded
+      const int nt = rw_row_tiles(rows), per = bs_rows_per_tile(rows);
+      s_per[e] = static_cast<uint16_t>(per);
+      if (nt > 0) box = max(box, rw_box_index(per));
+      return nt * m_pairs;
+    });
 #pragma unroll
     for (int d = 16; d > 0; d >>= 1) box = max(box, __shfl_xor_sync(0xffffffffu, box, d));
-    if (lane == 0) {
-      s_tile_start[p.e_local] = running;
-      s_box = box;
-    }
+    if (lane == 0) s_box = box;
   }
   tcgen05_fence_before();
   __syncthreads();

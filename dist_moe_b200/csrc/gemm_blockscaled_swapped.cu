@@ -105,54 +105,39 @@ __global__ void __launch_bounds__(kSwThreads, kSwCtasPerSm) blockscaled_swapped_
   const int lane = threadIdx.x & 31;
   const int m_tiles = p.N >> 7;
 
-  for (int i = threadIdx.x; i <= p.e_local; i += blockDim.x) {
-    const int v = p.expert_offsets[i];
-    s_off[i] = v < p.max_rows ? v : p.max_rows;
-  }
-  if (threadIdx.x == 0) {
-    abort_flag = 0;
-    s_first_bad = kNoBadTile;
-    for (int s = 0; s < kSwStages; ++s) {
-      mbar_init(&full_bar[s], 1);
-      mbar_init(&empty_bar[s], 1);
+  const int64_t x_off = p.x_off ? *p.x_off : 0, sfx_off = p.sfx_off ? *p.sfx_off : 0;  // on their way while the tables are built
+  if (warp == 2) {
+    if (lane < kSwStages) {
+      mbar_init(&full_bar[lane], 1);
+      mbar_init(&empty_bar[lane], 1);
     }
-    for (int b = 0; b < 2; ++b) {
-      mbar_init(&tmem_full_bar[b], 1);
-      mbar_init(&tmem_empty_bar[b], 4);
+    if (lane < 2) {
+      mbar_init(&tmem_full_bar[lane], 1);
+      mbar_init(&tmem_empty_bar[lane], 4);
+    }
+    if (lane == 0) {
+      abort_flag = 0;
+      s_first_bad = kNoBadTile;
     }
     mbar_fence_init();
-  }
-  __syncthreads();
-  for (int i = threadIdx.x; i < p.e_local; i += blockDim.x) {
-    const int count = p.expert_counts ? p.expert_counts[i] : p.max_rows;
-    s_cnt[i] = bs_group_rows(s_off[i], s_off[i + 1], count);
-    if (count > 0 && s_off[i + 1] > s_off[i] && !bs_group_aligned(s_off[i]))
-      set_status(p.status, kCapacityExceeded, -1, i, s_off[i]);  // groups must be 128-padded
-  }
-  __syncthreads();
-  if (warp == 0) {
-    int running = 0;
-    for (int e0 = 0; e0 < p.e_local; e0 += 32) {
-      const int e = e0 + lane;
-      const int tiles = e < p.e_local ? ((s_cnt[e] + kSwTileRows - 1) / kSwTileRows) * m_tiles : 0;
-      int incl = tiles;
-#pragma unroll
-      for (int d = 1; d < 32; d <<= 1) {
-        const int t = __shfl_up_sync(0xffffffffu, incl, d);
-        if (lane >= d) incl += t;
-      }
-      if (e < p.e_local) s_tile_start[e] = running + incl - tiles;
-      running += __shfl_sync(0xffffffffu, incl, 31);
-    }
-    if (lane == 0) s_tile_start[p.e_local] = running;
   }
   if (warp == 1) {
     tmem_alloc(&tmem_base_slot, kSwTmemCols);
     tmem_relinquish();
   }
-  if (warp == 0 && lane == 0) {
-    tma_prefetch_desc(&p.tm_x);
-    tma_prefetch_desc(&p.tm_w);
+  if (warp == 0) {
+    if (lane == 0) {
+      tma_prefetch_desc(&p.tm_x);
+      tma_prefetch_desc(&p.tm_w);
+    }
+    tile_tables(p.expert_offsets, p.expert_counts, p.e_local, p.max_rows, lane, s_off, s_tile_start,
+                [&](int e, int lo, int hi, int count) {
+      const int rows = bs_group_rows(lo, hi, count);
+      s_cnt[e] = rows;
+      if (count > 0 && hi > lo && !bs_group_aligned(lo))
+        set_status(p.status, kCapacityExceeded, -1, e, lo);  // groups must be 128-padded
+      return ((rows + kSwTileRows - 1) / kSwTileRows) * m_tiles;
+    });
   }
   tcgen05_fence_before();
   __syncthreads();
@@ -167,8 +152,8 @@ __global__ void __launch_bounds__(kSwThreads, kSwCtasPerSm) blockscaled_swapped_
     int stage = 0;
     uint32_t phase = 0;
     int e = 0;
-    const int x_line0 = uniform(static_cast<int>((p.x_off ? *p.x_off : 0) >> 7));
-    const uint8_t* sfx = p.sfx_base + (p.sfx_off ? *p.sfx_off : 0);
+    const int x_line0 = uniform(static_cast<int>(x_off >> 7));
+    const uint8_t* sfx = p.sfx_base + sfx_off;
     bool ok = true;
     for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
       const SwTile t = sw_decode(tile, e, s_tile_start, s_off, s_cnt, m_tiles);

@@ -50,6 +50,50 @@ __device__ __forceinline__ bool warp_mbar_wait(uint64_t* bar, uint32_t parity, v
   return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag));
 }
 
+// One warp builds a launch's tables: the groups' offsets (bounded by max_rows) and the first tile of every expert.  `tiles(e, lo, hi,
+// count)` tells how many tiles expert e's rows [lo, hi) make, `count` of them real (max_rows without counts).  All of its loads
+// are on their way before the first is used, and nothing waits for another warp.  With the offsets loaded by all threads and a block
+// barrier before the tables, a launch's first weight load came 4400 to 5200 cycles after its start (8 to 24 experts), so 3700 to
+// 4600; MXFP8 decode (128 experts, two launches) 213.6 -> 208.6 us.
+constexpr int kTableExperts = 256;
+template <class Tiles>
+__device__ __forceinline__ void tile_tables(const int32_t* offsets, const int32_t* counts, int e_local, int max_rows, int lane,
+                                            int* s_off, int* s_tile_start, Tiles&& tiles) {
+  int lo[kTableExperts / 32], hi[kTableExperts / 32], count[kTableExperts / 32];
+#pragma unroll
+  for (int c = 0; c < kTableExperts / 32; ++c) {
+    const int e = 32 * c + lane;
+    lo[c] = hi[c] = 0;
+    count[c] = max_rows;
+    if (e < e_local) {
+      lo[c] = offsets[e];
+      hi[c] = offsets[e + 1];
+      if (counts != nullptr) count[c] = counts[e];
+    }
+  }
+  int running = 0;
+#pragma unroll
+  for (int c = 0; c < kTableExperts / 32; ++c) {
+    if (32 * c >= e_local) break;
+    const int e = 32 * c + lane;
+    const int l = min(lo[c], max_rows), h = min(hi[c], max_rows);
+    const int own = e < e_local ? tiles(e, l, h, count[c]) : 0;
+    int incl = own;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const int t = __shfl_up_sync(0xffffffffu, incl, d);
+      if (lane >= d) incl += t;
+    }
+    if (e < e_local) {
+      s_off[e] = l;
+      s_tile_start[e] = running + incl - own;
+      if (e == e_local - 1) s_off[e_local] = h;
+    }
+    running += __shfl_sync(0xffffffffu, incl, 31);
+  }
+  if (lane == 0) s_tile_start[e_local] = running;
+}
+
 // After a wait ran out: a role's copies or MMAs that are still in flight have to end before the block gives its shared
 // memory and tensor memory back.  `bar` holds the barriers they complete, `stop` says where the role stopped.  Returns at
 // the deadline where a stage never completes (it was left half filled; what was issued for it has landed by then).

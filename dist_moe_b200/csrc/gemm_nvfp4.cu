@@ -495,56 +495,40 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kN4PairThreads, 1)
   const int first_tile = blockIdx.x >> 1, tile_step = gridDim.x >> 1;
   const int64_t a_off = p.a_off ? *p.a_off : 0, sfa_off = p.sfa_off ? *p.sfa_off : 0;  // on their way while the tables are built
 
-  for (int i = threadIdx.x; i <= p.e_local; i += blockDim.x) {
-    const int v = p.expert_offsets[i];
-    s_off[i] = v < p.max_rows ? v : p.max_rows;
-  }
-  if (threadIdx.x == 0) {
-    abort_flag = 0;
-    s_first_bad = kNoBadTile;
-    for (int s = 0; s < kN4PairStages; ++s) {
-      mbar_init(&full_bar[s], 1);
-      mbar_init(&empty_bar[s], 1);
+  if (warp == 2) {
+    if (lane < stages) {
+      mbar_init(&full_bar[lane], 1);
+      mbar_init(&empty_bar[lane], 1);
     }
-    mbar_init(&tmem_full_bar, 1);
-    mbar_init(&tmem_empty_bar, 2 * kN4PairEpilogue);  // the leader's: the epilogue warps of both CTAs
+    if (lane == 0) {
+      mbar_init(&tmem_full_bar, 1);
+      mbar_init(&tmem_empty_bar, 2 * kN4PairEpilogue);  // the leader's: the epilogue warps of both CTAs
+      abort_flag = 0;
+      s_first_bad = kNoBadTile;
+    }
     mbar_fence_init();
+    __syncwarp();
   }
-  __syncthreads();
   cluster_arrive();  // this CTA's barriers exist
-  if (warp == 0) {
-    int running = 0;
-    for (int e0 = 0; e0 < p.e_local; e0 += 32) {
-      const int e = e0 + lane;
-      int tiles = 0;
-      if (e < p.e_local) {
-        const int count = p.expert_counts ? p.expert_counts[e] : p.max_rows;
-        const int rows = bs_group_rows(s_off[e], s_off[e + 1], count);
-        s_rows[e] = rows;
-        if (count > 0 && s_off[e + 1] > s_off[e] && !bs_group_aligned(s_off[e]))
-          set_status(p.status, kCapacityExceeded, -1, e, s_off[e]);  // groups must be 128-padded
-        tiles = ((rows + 2 * kN4BM - 1) / (2 * kN4BM)) * n_tiles;
-      }
-      int incl = tiles;
-#pragma unroll
-      for (int d = 1; d < 32; d <<= 1) {
-        const int t = __shfl_up_sync(0xffffffffu, incl, d);
-        if (lane >= d) incl += t;
-      }
-      if (e < p.e_local) s_tile_start[e] = running + incl - tiles;
-      running += __shfl_sync(0xffffffffu, incl, 31);
-    }
-    if (lane == 0) s_tile_start[p.e_local] = running;
-  }
   if (warp == 1) {
     tmem_alloc_pair(&tmem_base_slot, kN4TmemCols);
     tmem_relinquish_pair();
   }
-  if (warp == 0 && lane == 0) {
-    tma_prefetch_desc(&p.tm_a);
-    tma_prefetch_desc(&p.tm_b);
-    tma_prefetch_desc(&p.tm_sfa);
-    tma_prefetch_desc(&p.tm_sfb);
+  if (warp == 0) {
+    if (lane == 0) {
+      tma_prefetch_desc(&p.tm_a);
+      tma_prefetch_desc(&p.tm_b);
+      tma_prefetch_desc(&p.tm_sfa);
+      tma_prefetch_desc(&p.tm_sfb);
+    }
+    tile_tables(p.expert_offsets, p.expert_counts, p.e_local, p.max_rows, lane, s_off, s_tile_start,
+                [&](int e, int lo, int hi, int count) {
+      const int rows = bs_group_rows(lo, hi, count);
+      s_rows[e] = rows;
+      if (count > 0 && hi > lo && !bs_group_aligned(lo))
+        set_status(p.status, kCapacityExceeded, -1, e, lo);  // groups must be 128-padded
+      return ((rows + 2 * kN4BM - 1) / (2 * kN4BM)) * n_tiles;
+    });
   }
   tcgen05_fence_before();
   __syncthreads();
