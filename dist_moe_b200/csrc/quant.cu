@@ -29,6 +29,15 @@ __device__ __forceinline__ uint32_t mxfp8_scale_bits(uint32_t bits15, float& rec
   return byte;
 }
 
+// The same of two maxima side by side, both finite: the scale bytes in 16 bits each, and the reciprocals (powers of two) as the two
+// bf16 of `recip2`.
+__device__ __forceinline__ uint32_t mxfp8_scale_bits2(uint32_t bits15x2, uint32_t& recip2) {
+  const uint32_t b = __vmaxu2(((bits15x2 + 0x001f001fu) >> 7) & 0x01ff01ffu, 0x00080008u) - 0x00080008u;
+  recip2 = (0x00fe00feu - b) << 7;
+  return b;
+}
+__device__ __forceinline__ bool any_nonfinite2(uint32_t bits15x2) { return __vmaxu2(bits15x2, 0x7f7f7f7fu) != 0x7f7f7f7fu; }
+
 // Products of two packed fp32 pairs (one instruction), as two E4M3 bytes.
 __device__ __forceinline__ uint32_t e4m3x2_scaled(float lo, float hi, float r_lo, float r_hi) {
   float a, b;
@@ -209,6 +218,8 @@ __global__ void __launch_bounds__(256) mxfp8_slab_kernel(const __nv_bfloat16* __
 // one B200: W13 input gather 4096 wide 309 -> 207 us, gradient gather 329 -> 209 us, SwiGLU forward 1536 wide 216 -> 196 us,
 // SwiGLU backward 431 -> 316 us; a dense 32 768 x 4096 matrix 148 -> 98 us (5.6 TB/s of algorithmic bytes).  The SwiGLU
 // forms are bound by the sigmoid's arithmetic (69 % of the issue slots), the others by HBM.
+// Two scales at a time and rows without a question each (see tile_quantise): 65 536 x 4096 gather 207 -> 175 us, from the combine
+// buffer 210 -> 209 (HBM), SwiGLU forward 1536 wide 186 -> 168, backward 246 -> 234.
 // ---------------------------------------------------------------------------
 constexpr int kTileRows = 128;
 constexpr int kTileCols = 128;
@@ -274,23 +285,46 @@ __device__ __forceinline__ void tile_quantise(const uint4 (&w)[8], const TileLan
       n[p] = __vmaxu2(n[p], __shfl_xor_sync(0xffffffffu, n[p], 2));
     }
 #pragma unroll
-    for (int r = 0; r < 8; ++r) {
-      const uint32_t byte = mxfp8_scale_bits((r & 1) ? n[r >> 1] >> 16 : n[r >> 1] & 0xffffu, rrow[r]);
-      if ((me.lane & 3) == 0)
-        row_atom[(me.rg * 8 + r) * 16 + me.slab * 4 + me.half * 2 + (me.cg >> 2)] = static_cast<uint8_t>(byte);
-    }
-#pragma unroll
     for (int j = 0; j < 4; ++j) {
       m[j] = __vmaxu2(m[j], __shfl_xor_sync(0xffffffffu, m[j], 8));
       m[j] = __vmaxu2(m[j], __shfl_xor_sync(0xffffffffu, m[j], 16));
-      const uint32_t b0 = mxfp8_scale_bits(m[j] & 0xffffu, rcol[2 * j]);
-      const uint32_t b1 = mxfp8_scale_bits(m[j] >> 16, rcol[2 * j + 1]);
-      if (me.rg == j) {  // the four row groups share the eight columns' bytes between them
-        const int ct = me.col() + 2 * j;
-        col_atom[(ct & 31) * 16 + (ct >> 5) * 4 + me.slab] = static_cast<uint8_t>(b0);
-        col_atom[((ct & 31) + 1) * 16 + (ct >> 5) * 4 + me.slab] = static_cast<uint8_t>(b1);
+    }
+    uint32_t nb[4], mb[4];  // scale bytes, 16 bits each
+    if (!any_nonfinite2(__vmaxu2(__vmaxu2(__vmaxu2(n[0], n[1]), __vmaxu2(n[2], n[3])),
+                                 __vmaxu2(__vmaxu2(m[0], m[1]), __vmaxu2(m[2], m[3]))))) {
+      // two scales at a time: one by one they were a sixth of the kernel's instructions
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        uint32_t r2;
+        nb[j] = mxfp8_scale_bits2(n[j], r2);
+        rrow[2 * j] = __uint_as_float(r2 << 16);
+        rrow[2 * j + 1] = __uint_as_float(r2 & 0xffff0000u);
+        mb[j] = mxfp8_scale_bits2(m[j], r2);
+        rcol[2 * j] = __uint_as_float(r2 << 16);
+        rcol[2 * j + 1] = __uint_as_float(r2 & 0xffff0000u);
+      }
+    } else {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        nb[j] = mxfp8_scale_bits(n[j] & 0xffffu, rrow[2 * j]);
+        nb[j] |= mxfp8_scale_bits(n[j] >> 16, rrow[2 * j + 1]) << 16;
+        mb[j] = mxfp8_scale_bits(m[j] & 0xffffu, rcol[2 * j]);
+        mb[j] |= mxfp8_scale_bits(m[j] >> 16, rcol[2 * j + 1]) << 16;
       }
     }
+    if ((me.lane & 3) == 0) {
+      uint8_t* to = row_atom + me.rg * 8 * 16 + me.slab * 4 + me.half * 2 + (me.cg >> 2);
+#pragma unroll
+      for (int r = 0; r < 8; ++r) to[r * 16] = static_cast<uint8_t>((r & 1) ? nb[r >> 1] >> 16 : nb[r >> 1]);
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (me.rg == j) {  // the four row groups share the eight columns' bytes between them
+        const int ct = me.col() + 2 * j;
+        uint8_t* to = col_atom + (ct & 31) * 16 + (ct >> 5) * 4 + me.slab;
+        to[0] = static_cast<uint8_t>(mb[j]);
+        to[16] = static_cast<uint8_t>(mb[j] >> 16);
+      }
   }
   const bool rowq = out.q_row != nullptr, colq = out.q_col != nullptr;
   const bool col_wide = (reinterpret_cast<uintptr_t>(out.q_col) & 7) == 0;  // a caller's own buffer may be 2-byte aligned
@@ -298,34 +332,45 @@ __device__ __forceinline__ void tile_quantise(const uint4 (&w)[8], const TileLan
   const int live = c < limit ? (left < 8 ? static_cast<int>(left) : 8) : 0;
   uint8_t* dr = out.q_row + r0 * out.C + c;
   uint8_t* dc = out.q_col + r0 * out.C + c;
+  auto row_bytes = [&](const float (&f)[8], int r) {
+    return make_uint2(e4m3x2_scaled(f[0], f[1], rrow[r], rrow[r]) | (e4m3x2_scaled(f[2], f[3], rrow[r], rrow[r]) << 16),
+                      e4m3x2_scaled(f[4], f[5], rrow[r], rrow[r]) | (e4m3x2_scaled(f[6], f[7], rrow[r], rrow[r]) << 16));
+  };
+  auto col_bytes = [&](const float (&f)[8]) {
+    return make_uint2(e4m3x2_scaled(f[0], f[1], rcol[0], rcol[1]) | (e4m3x2_scaled(f[2], f[3], rcol[2], rcol[3]) << 16),
+                      e4m3x2_scaled(f[4], f[5], rcol[4], rcol[5]) | (e4m3x2_scaled(f[6], f[7], rcol[6], rcol[7]) << 16));
+  };
+  if (rowq && colq && col_wide && live == 8) {  // both copies of whole rows: nothing to ask per row
 #pragma unroll
-  for (int r = 0; r < 8; ++r) {
-    const uint4 v = w[r];
-    const float f0 = __uint_as_float(v.x << 16), f1 = __uint_as_float(v.x & 0xffff0000u);
-    const float f2 = __uint_as_float(v.y << 16), f3 = __uint_as_float(v.y & 0xffff0000u);
-    const float f4 = __uint_as_float(v.z << 16), f5 = __uint_as_float(v.z & 0xffff0000u);
-    const float f6 = __uint_as_float(v.w << 16), f7 = __uint_as_float(v.w & 0xffff0000u);
-    if (r < live) {
-      if (rowq)
-        *reinterpret_cast<uint2*>(dr) =
-            make_uint2(e4m3x2_scaled(f0, f1, rrow[r], rrow[r]) | (e4m3x2_scaled(f2, f3, rrow[r], rrow[r]) << 16),
-                       e4m3x2_scaled(f4, f5, rrow[r], rrow[r]) | (e4m3x2_scaled(f6, f7, rrow[r], rrow[r]) << 16));
-      if (colq) {
-        const uint32_t p0 = e4m3x2_scaled(f0, f1, rcol[0], rcol[1]), p1 = e4m3x2_scaled(f2, f3, rcol[2], rcol[3]);
-        const uint32_t p2 = e4m3x2_scaled(f4, f5, rcol[4], rcol[5]), p3 = e4m3x2_scaled(f6, f7, rcol[6], rcol[7]);
-        if (col_wide) {
-          *reinterpret_cast<uint2*>(dc) = make_uint2(p0 | (p1 << 16), p2 | (p3 << 16));
-        } else {
-          uint16_t* d2 = reinterpret_cast<uint16_t*>(dc);
-          d2[0] = static_cast<uint16_t>(p0);
-          d2[1] = static_cast<uint16_t>(p1);
-          d2[2] = static_cast<uint16_t>(p2);
-          d2[3] = static_cast<uint16_t>(p3);
+    for (int r = 0; r < 8; ++r) {
+      float f[8];
+      unpack8f(w[r], f);
+      *reinterpret_cast<uint2*>(dr + static_cast<int64_t>(r) * out.C) = row_bytes(f, r);
+      *reinterpret_cast<uint2*>(dc + static_cast<int64_t>(r) * out.C) = col_bytes(f);
+    }
+  } else {
+#pragma unroll
+    for (int r = 0; r < 8; ++r) {
+      if (r < live) {
+        float f[8];
+        unpack8f(w[r], f);
+        if (rowq) *reinterpret_cast<uint2*>(dr) = row_bytes(f, r);
+        if (colq) {
+          const uint2 q = col_bytes(f);
+          if (col_wide) {
+            *reinterpret_cast<uint2*>(dc) = q;
+          } else {
+            uint16_t* d2 = reinterpret_cast<uint16_t*>(dc);
+            d2[0] = static_cast<uint16_t>(q.x);
+            d2[1] = static_cast<uint16_t>(q.x >> 16);
+            d2[2] = static_cast<uint16_t>(q.y);
+            d2[3] = static_cast<uint16_t>(q.y >> 16);
+          }
         }
       }
+      dr += out.C;
+      dc += out.C;
     }
-    dr += out.C;
-    dc += out.C;
   }
   __syncthreads();
   // Scales.  A tile that lies wholly inside the matrix owns whole atoms; at the edges (or in a buffer that 16-byte
