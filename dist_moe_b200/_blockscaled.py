@@ -353,7 +353,7 @@ def run_block_scaled(x, ids, scores, w13_weight, w2_weight, context: Any, option
                                        D * 2, 128, state.capacity_rows, size, counts.data_ptr(), real.data_ptr(),
                                        per_rank.data_ptr(), offsets.data_ptr(), fwd.data_ptr(), None, sct.data_ptr(),
                                        state.route_workspace.data_ptr(), state.route_workspace_words, status, st),
-              nat.route_call_name(ep, T, el))
+              nat.route_call_name(ep, T, el), nat.route_launches(ep, T, el))
     recv = offsets[el:]
     fused = bool(p13._interleaved_fc13)
     # few rows per expert (decode): weights on the MMA's M side, the rows on its N side
@@ -676,7 +676,8 @@ def _mxfp8_forward(state, x, ids, scores, p13, p2, options, need_h3: bool):
                                state.combine.peer_ptrs.data_ptr(), state.rank, ep, T, K, E, stride, stride, stride, 128,
                                state.capacity_rows, size, counts.data_ptr(), per_rank.data_ptr(), c.offsets.data_ptr(),
                                c.fwd.data_ptr(), c.bwd.data_ptr(), c.sct.data_ptr(), state.route_workspace.data_ptr(),
-                               state.route_workspace_words, status, st), nat.route_call_name(ep, T, el))
+                               state.route_workspace_words, status, st), nat.route_call_name(ep, T, el),
+              nat.route_launches(ep, T, el))
     c.recv = c.offsets[el:]
     recv = c.recv.data_ptr()
     ws = _Bump(_train_workspace(state, R))

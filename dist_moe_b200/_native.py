@@ -244,18 +244,28 @@ for _name, (_res, _args) in _SIGNATURES.items():
 # Kernel launches issued through this binding (benchmarks report the count).
 LAUNCHES = [0]
 _LAUNCHES_PER_CALL = {"dm_route": 3, "dm_route_counted": 3}
+_ROUTE_CHUNK_TOKENS, _ROUTE_TWO_LAUNCH_CHUNKS = 256, 1024  # include/dist_moe_b200.h
 
 
 def route_call_name(ep: int, tokens: int, e_local: int) -> str:
-    """Name under which a ``dm_route`` call is counted: the decode regime runs one launch instead of three."""
+    """Name under which a ``dm_route`` call is counted: the decode regime is one launch instead of several."""
     single = ep * tokens <= 1024 and e_local <= 512 and lib.dm_route_decode_kernel_enabled()
     return "dm_route(single launch)" if single else "dm_route"
 
 
-def check(rc: int, what: str) -> None:
+def route_launches(ep: int, tokens: int, e_local: int) -> int:
+    """Kernels that a ``dm_route`` call launches: one in the decode regime, two or three beyond."""
+    if e_local > 512:
+        return 3
+    if ep * tokens <= 1024 and lib.dm_route_decode_kernel_enabled():
+        return 1
+    return 2 if ep * -(-tokens // _ROUTE_CHUNK_TOKENS) <= _ROUTE_TWO_LAUNCH_CHUNKS else 3
+
+
+def check(rc: int, what: str, launches: int | None = None) -> None:
     """Raise on a non-zero return code of an entry point."""
     if rc == 0:
-        LAUNCHES[0] += _LAUNCHES_PER_CALL.get(what, 1)
+        LAUNCHES[0] += _LAUNCHES_PER_CALL.get(what, 1) if launches is None else launches
         return
     if rc < 0:
         raise NativeError(f"{what}: {RC_NAMES.get(rc, rc)}")

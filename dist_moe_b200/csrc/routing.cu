@@ -2,7 +2,7 @@
 //
 // Routing order contract (must equal the reference's general path): output rows
 // are sorted by (local expert ascending, source rank ascending, token ascending).
-// The three kernels below reach it without any sort:
+// The kernels below reach it without any sort:
 //   route_count : one CTA per (source rank, 256-token chunk) builds, per local
 //                 expert, a 32-bit lane mask per warp in shared memory and stores
 //                 the chunk's per-expert totals; a global histogram over all E
@@ -12,13 +12,14 @@
 //                 checks capacity and writes counts / per-rank totals / offsets.
 //   route_fill  : same decomposition as route_count; a row's slot is
 //                 segment offset + popc(lower warps) + popc(lower lanes).
+//   route_place : scan and fill in one, up to DM_ROUTE_TWO_LAUNCH_CHUNKS chunks.
 #include "publish.cuh"
 #include "common.cuh"
 #include "../../include/dist_moe_b200.h"
 
 namespace dm {
 
-constexpr int kChunkTokens = 256;  // tokens per CTA in route_count / route_fill
+constexpr int kChunkTokens = DM_ROUTE_CHUNK_TOKENS;  // tokens per CTA in route_count / route_fill / route_place
 constexpr int kChunkWarps = kChunkTokens / 32;
 constexpr int kMaxExpertsSmem = 2048;
 
@@ -94,6 +95,7 @@ struct RouteParams {
   int32_t* chunk_counts;   // [ep*chunks][e_local]
   int32_t* chunk_offsets;  // [ep*chunks][e_local], exclusive inside the expert segment
   int32_t* hist;           // [E]
+  int own_hist;            // one rank, two launches: chunk_offsets holds every chunk's routes per expert instead
   int* status;
 };
 
@@ -138,6 +140,11 @@ __global__ void __launch_bounds__(kChunkTokens) route_count_kernel(RouteParams p
 #pragma unroll
     for (int w = 0; w < kChunkWarps; ++w) n += __popc(mask[w * p.e_local + el]);
     out[el] = n;
+  }
+  if (p.own_hist) {
+    int32_t* own = p.chunk_offsets + static_cast<int64_t>(c) * p.E;
+    for (int e = threadIdx.x; e < p.E; e += blockDim.x) own[e] = hist_s[e];
+    return;
   }
   for (int e = threadIdx.x; e < p.E; e += blockDim.x) {
     const int n = hist_s[e];
@@ -233,24 +240,20 @@ __global__ void __launch_bounds__(1024) route_scan_kernel(RouteParams p) {
   }
 }
 
-__global__ void __launch_bounds__(kChunkTokens) route_fill_kernel(RouteParams p) {
-  extern __shared__ uint32_t smem_u[];
-  uint32_t* mask = smem_u;
-  const int s = blockIdx.y, c = blockIdx.x;
-  if (p.expert_offsets[p.e_local] == 0) return;  // nothing routed here, or capacity exceeded
-  build_masks(p, s, c, mask, nullptr, false);
+// Pointers of this chunk's routes: `base` where an expert's segment starts, `seg` its rows of lower chunks.
+__device__ __forceinline__ void route_fill(const RouteParams& p, int s, int c, const uint32_t* mask, const int32_t* base,
+                                           const int32_t* seg) {
   const int tok = c * kChunkTokens + threadIdx.x;
   if (tok >= p.T) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int16_t* ids = reinterpret_cast<const int16_t*>(p.routing_ptrs[s] + DM_ROUTING_HEADER_BYTES) +
                        static_cast<int64_t>(tok) * p.K;
-  const int32_t* seg = p.chunk_offsets + (static_cast<int64_t>(s) * p.chunks + c) * p.e_local;
   const int first = p.rank * p.e_local;
   const uint64_t dbase = p.dispatch_ptrs[s], cbase = p.combine_ptrs[s];
   for (int k = 0; k < p.K; ++k) {
     const int el = static_cast<int>(ids[k]) - first;
     if (ids[k] < 0 || ids[k] >= p.E || el < 0 || el >= p.e_local) continue;
-    int pos = p.expert_offsets[el] + seg[el];
+    int pos = base[el] + seg[el];
     for (int w = 0; w < warp; ++w) pos += __popc(mask[w * p.e_local + el]);
     pos += __popc(mask[warp * p.e_local + el] & ((1u << lane) - 1u));
     const int64_t route = static_cast<int64_t>(tok) * p.K + k;
@@ -258,6 +261,87 @@ __global__ void __launch_bounds__(kChunkTokens) route_fill_kernel(RouteParams p)
     p.sct[pos] = static_cast<int64_t>(cbase + static_cast<uint64_t>(route) * p.scatter_stride);
     if (p.bwd != nullptr) p.bwd[pos] = static_cast<int64_t>(dbase + static_cast<uint64_t>(route) * p.bwd_stride);
   }
+}
+
+__global__ void __launch_bounds__(kChunkTokens) route_fill_kernel(RouteParams p) {
+  extern __shared__ uint32_t smem_u[];
+  uint32_t* mask = smem_u;
+  const int s = blockIdx.y, c = blockIdx.x;
+  if (p.expert_offsets[p.e_local] == 0) return;  // nothing routed here, or capacity exceeded
+  build_masks(p, s, c, mask, nullptr, false);
+  route_fill(p, s, c, mask, p.expert_offsets, p.chunk_offsets + (static_cast<int64_t>(s) * p.chunks + c) * p.e_local);
+}
+
+// Scan and fill in one launch: every block sums the chunks' counts itself, for where the segments start and for its own
+// rows in them; block 0 writes the tables, and the padding rows are dealt out over the blocks.  Bound by latency, not bytes:
+// the scan was one block that walked all chunks and wrote all padding rows between two launches, and one rank's routes per
+// expert needed a memset and global atomics that block 0 now sums from the chunks.  One rank, padded to 128, the whole
+// routing step: 2,048 tokens x 8 of 32 experts 18.4 -> 10.3 us, 4,096 x 8 of 128 24.6 -> 12.5, 16,384 x 8 of 256
+// 47.9 -> 19.7; eight ranks, 2,048 x 6 of 64, unpadded, 14.6 -> 12.5 us.
+__global__ void __launch_bounds__(kChunkTokens) route_place_kernel(RouteParams p) {
+  extern __shared__ uint32_t smem_u[];
+  uint32_t* mask = smem_u;                                                    // [kChunkWarps][e_local]
+  int32_t* total = reinterpret_cast<int32_t*>(mask + kChunkWarps * p.e_local);  // [e_local] real rows
+  int32_t* below = total + p.e_local;                                         // [e_local] of them in lower chunks
+  int32_t* routes = below + p.e_local;                                        // [e_local] routes (one rank: of all experts)
+  int32_t* base = routes + p.e_local;                                         // [e_local + 1] padded exclusive prefix
+  __shared__ int overflow;
+  const int s = blockIdx.y, c = blockIdx.x, me = s * p.chunks + c, n = p.ep * p.chunks;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int el = threadIdx.x; el < p.e_local; el += blockDim.x) total[el] = below[el] = routes[el] = 0;
+  __syncthreads();
+  const int width = p.e_local < kChunkTokens ? p.e_local : kChunkTokens, groups = kChunkTokens / width;
+  const int g = threadIdx.x / width, l = threadIdx.x - g * width;
+  if (g < groups) {
+    for (int el = l; el < p.e_local; el += width) {
+      int sum = 0, lower = 0, listed = 0;
+#pragma unroll 4
+      for (int i = g; i < n; i += groups) {
+        const int v = p.chunk_counts[static_cast<int64_t>(i) * p.e_local + el];
+        sum += v;
+        if (i < me) lower += v;
+      }
+      if (p.own_hist && me == 0)
+        for (int i = g; i < n; i += groups) listed += p.chunk_offsets[static_cast<int64_t>(i) * p.e_local + el];
+      atomicAdd(&total[el], sum);
+      atomicAdd(&below[el], lower);
+      atomicAdd(&routes[el], listed);
+    }
+  }
+  build_masks(p, s, c, mask, nullptr, false);  // ends with a block barrier: the sums are there too
+  const int64_t acc = warp == 0 ? warp_padded_prefix(total, base, p.e_local, p.m_mult, lane) : 0;
+  if (threadIdx.x == 0) {
+    overflow = (acc > p.capacity_rows || acc > p.ptrs_size) ? 1 : 0;
+    if (overflow && me == 0) set_status(p.status, kCapacityExceeded, static_cast<int>(acc), static_cast<int>(p.capacity_rows));
+    // ranks that disagree on T cannot be routed: the call becomes a no-op (zero rows), like an overflow
+    if (p.status != nullptr && *reinterpret_cast<volatile int*>(p.status) == kTokenCountMismatch) overflow = 1;
+  }
+  __syncthreads();
+  const bool bad = overflow != 0;
+  if (me == 0) {
+    for (int el = threadIdx.x; el <= p.e_local; el += blockDim.x) {
+      p.expert_offsets[el] = bad ? 0 : base[el];
+      if (el < p.e_local) p.counts[el] = bad ? 0 : pad_rows(total[el], p.m_mult);
+      if (el < p.e_local && p.real_counts != nullptr) p.real_counts[el] = bad ? 0 : total[el];
+    }
+    for (int q = warp; q < p.ep; q += kChunkWarps) {
+      const int sum = warp_padded_sum(p.own_hist ? routes : p.hist + q * p.e_local, p.e_local, p.m_mult, lane);
+      if (lane == 0) p.per_rank[q] = sum;
+    }
+  }
+  if (bad) return;
+  if (p.m_mult > 0) {
+    // Padding rows of every expert segment hold a null pointer.
+    for (int el = me + n * warp; el < p.e_local; el += n * kChunkWarps) {
+      const int lo = base[el] + total[el], hi = base[el + 1];
+      for (int r = lo + lane; r < hi; r += 32) {
+        p.fwd[r] = 0;
+        p.sct[r] = 0;
+        if (p.bwd != nullptr) p.bwd[r] = 0;
+      }
+    }
+  }
+  route_fill(p, s, c, mask, base, below);
 }
 
 // ---------------------------------------------------------------------------
@@ -520,12 +604,24 @@ static int route_launch(const uint64_t* routing_ptrs, const uint64_t* dispatch_p
     route_decode_kernel<<<1, kDecodeThreads, smem, st>>>(p);
     return static_cast<int>(cudaGetLastError());
   }
-  cudaError_t err = cudaMemsetAsync(p.hist, 0, sizeof(int32_t) * E, st);
-  if (err != cudaSuccess) return static_cast<int>(err);
+  // The sums cost every block a read of all chunks' counts, so the work grows with the square of the chunks; the scan's one
+  // block grows linearly.  Measured on either side, us, three launches | two: 512 chunks x 64 experts 62 | 23, x 500 235 | 132;
+  // 1,024 x 64 111 | 49, x 256 372 | 167, x 500 445 | 335; 2,048 x 64 205 | 132, x 500 861 | 921, eight ranks of 32 experts
+  // 115 | 83; 4,096 x 64 394 | 458, x 256 1,418 | 1,737, eight ranks of 32 236 | 277.
+  const bool place = static_cast<int64_t>(ep) * p.chunks <= DM_ROUTE_TWO_LAUNCH_CHUNKS && p.e_local <= 512;
+  p.own_hist = place && ep == 1 ? 1 : 0;
+  if (!p.own_hist) {
+    const cudaError_t err = cudaMemsetAsync(p.hist, 0, sizeof(int32_t) * E, st);
+    if (err != cudaSuccess) return static_cast<int>(err);
+  }
   const dim3 grid(p.chunks, ep);
   const size_t smem_count = sizeof(uint32_t) * (kChunkWarps * p.e_local + E);
   const size_t smem_fill = sizeof(uint32_t) * (kChunkWarps * p.e_local);
   route_count_kernel<<<grid, kChunkTokens, smem_count, st>>>(p);
+  if (place) {
+    route_place_kernel<<<grid, kChunkTokens, smem_fill + sizeof(int32_t) * (4 * p.e_local + 1), st>>>(p);
+    return static_cast<int>(cudaGetLastError());
+  }
   route_scan_kernel<<<1, 1024, sizeof(int32_t) * (2 * p.e_local + 1), st>>>(p);
   route_fill_kernel<<<grid, kChunkTokens, smem_fill, st>>>(p);
   return static_cast<int>(cudaGetLastError());

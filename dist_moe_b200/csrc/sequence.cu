@@ -36,6 +36,12 @@ struct Sequence {
 
 const dm_operand kNone{nullptr, 0, nullptr};
 
+int launches_of_route(const dm_layer_context& c, const dm_layer_call& k) {
+  if (c.e_local > 512) return 3;
+  if (c.ep * k.T <= 1024 && dm_route_decode_kernel_enabled() != 0) return 1;
+  return c.ep * ((k.T + DM_ROUTE_CHUNK_TOKENS - 1) / DM_ROUTE_CHUNK_TOKENS) <= DM_ROUTE_TWO_LAUNCH_CHUNKS ? 2 : 3;
+}
+
 }  // namespace
 
 extern "C" int dm_bf16_forward(const dm_layer_context* ctx, const dm_layer_call* call, uint32_t steps, int32_t* report,
@@ -47,12 +53,12 @@ extern "C" int dm_bf16_forward(const dm_layer_context* ctx, const dm_layer_call*
   Sequence s{c, steps, report, stream};
   const int64_t stride = c.D * 2;
   int64_t* fs = k.fwd_state;
-  const bool single = c.ep * k.T <= 1024 && c.e_local <= 512 && dm_route_decode_kernel_enabled() != 0;
+  const int route_launches = launches_of_route(c, k);
   s.step(DM_FWD_PUBLISH, 1, [&] {
     return dm_publish(k.x, k.ids, k.ids_are_int64, c.dispatch, c.routing, k.T, c.D, c.K, c.E, k.validate_ids, c.status, stream);
   });
   s.barrier(DM_FWD_PUBLISH, c.dispatch_pads, nullptr);
-  s.step(DM_FWD_ROUTE, single ? 1 : 3, [&] {
+  s.step(DM_FWD_ROUTE, route_launches, [&] {
     return dm_route(c.routing_ptrs, c.dispatch_ptrs, c.combine_ptrs, c.rank, c.ep, k.T, c.K, c.E, stride, stride, stride, 0,
                     c.capacity_rows, k.ptrs_size, k.counts, k.per_rank, k.expert_offsets, k.fwd_ptrs, k.bwd_ptrs, k.sct_ptrs,
                     c.route_workspace, c.route_workspace_words, c.status, stream);
@@ -201,12 +207,12 @@ extern "C" int dm_mxfp8_forward(const dm_layer_context* ctx, const dm_layer_call
   Sequence s{c, steps, report, stream};
   const int64_t stride = c.D * 2;
   int64_t *fs = k.fwd_state, *ft = k.fwd_table;
-  const bool single = c.ep * k.T <= 1024 && c.e_local <= 512 && dm_route_decode_kernel_enabled() != 0;
+  const int route_launches = launches_of_route(c, k);
   s.step(DM_FWD_PUBLISH, 1, [&] {
     return dm_publish(k.x, k.ids, k.ids_are_int64, c.dispatch, c.routing, k.T, c.D, c.K, c.E, k.validate_ids, c.status, stream);
   });
   s.barrier(DM_FWD_PUBLISH, c.dispatch_pads, nullptr);
-  s.step(DM_FWD_ROUTE, single ? 1 : 3, [&] {
+  s.step(DM_FWD_ROUTE, route_launches, [&] {
     return dm_route_counted(c.routing_ptrs, c.dispatch_ptrs, c.combine_ptrs, c.rank, c.ep, k.T, c.K, c.E, stride, stride,
                             stride, 128, c.capacity_rows, k.ptrs_size, k.counts, k.real_counts, k.per_rank, k.expert_offsets,
                             k.fwd_ptrs, k.bwd_ptrs, k.sct_ptrs, c.route_workspace, c.route_workspace_words, c.status, stream);

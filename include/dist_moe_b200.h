@@ -39,6 +39,10 @@ extern "C" {
 /* Bytes of the routing-buffer header that precedes the int16 expert ids
  * (dist_moe/_buffers.py:33-35). Word 0 of the header is the int32 token count. */
 #define DM_ROUTING_HEADER_BYTES 128
+/* The general routing path works on chunks of this many tokens per source rank: two launches up to so many chunks over
+ * all ranks, three beyond. */
+#define DM_ROUTE_CHUNK_TOKENS 256
+#define DM_ROUTE_TWO_LAUNCH_CHUNKS 1024
 
 /* Library version / build probe; returns the compiled SM architecture (1000). */
 int dm_version(void);
@@ -133,7 +137,7 @@ int dm_route_static(const uint64_t* routing_ptrs, const uint64_t* dispatch_ptrs,
 
 /* Kernel selection for dm_route / dm_route_static: non-zero (default) lets calls with ep * T <= 1024 run the whole
  * routing step in one single-CTA launch (the decode regime; the reference's single-launch path,
- * dist_moe/_routing_metadata.py:265-300); zero keeps every call on the three general kernels.  Both produce the
+ * dist_moe/_routing_metadata.py:265-300); zero keeps every call on the general kernels.  Both produce the
  * same tables bit for bit (rows ordered by local expert, source rank, token).  Returns the previous setting. */
 int dm_set_route_decode_kernel(int enabled);
 int dm_route_decode_kernel_enabled(void); /* the current setting, without changing it */
