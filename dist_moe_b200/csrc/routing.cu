@@ -99,41 +99,88 @@ struct RouteParams {
   int* status;
 };
 
-// Build the per-warp lane masks of this chunk: mask[w][el] bit l = token (w*32+l)
-// routes to local expert el.  Returns through shared memory.
-__device__ __forceinline__ void build_masks(const RouteParams& p, int s, int c, uint32_t* mask, int32_t* hist_s,
-                                            bool do_hist) {
-  const int tok = c * kChunkTokens + threadIdx.x;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  for (int i = threadIdx.x; i < kChunkWarps * p.e_local; i += blockDim.x) mask[i] = 0u;
-  if (do_hist)
-    for (int i = threadIdx.x; i < p.E; i += blockDim.x) hist_s[i] = 0;
-  __syncthreads();
-  if (tok < p.T) {
-    const int16_t* ids = reinterpret_cast<const int16_t*>(p.routing_ptrs[s] + DM_ROUTING_HEADER_BYTES) +
-                         static_cast<int64_t>(tok) * p.K;
-    const int first = p.rank * p.e_local;
-    for (int k = 0; k < p.K; ++k) {
-      const int e = ids[k];
-      if (e < 0 || e >= p.E) continue;
-      if (do_hist) atomicAdd(&hist_s[e], 1);
-      const int el = e - first;
-      if (el >= 0 && el < p.e_local) atomicOr(&mask[warp * p.e_local + el], 1u << lane);
+// Eight ids on their way before the first shared-memory atomic (which the loads could not be moved across).
+__device__ __forceinline__ void load_ids(const int16_t* ids, int k0, int K, int (&e8)[8]) {
+#pragma unroll
+  for (int j = 0; j < 8; ++j) e8[j] = k0 + j < K ? static_cast<int>(ids[k0 + j]) : -1;
+}
+
+// Calls fn(k, e) for a token's valid ids; `first8` holds the first eight of them.  The ids past the eighth come one by one: they
+// are in L1 by then, and a second unrolled copy of `fn` cost the smallest calls 0.3 us of instruction fetches.
+template <class Fn>
+__device__ __forceinline__ void each_id(const RouteParams& p, const int16_t* ids, const int (&first8)[8], Fn&& fn) {
+#pragma unroll
+  for (int j = 0; j < 8; ++j)
+    if (first8[j] >= 0 && first8[j] < p.E) fn(j, first8[j]);
+#pragma unroll 1
+  for (int k0 = 8; k0 < p.K; ++k0) {
+    const int e = ids[k0];
+    if (e >= 0 && e < p.E) fn(k0, e);
+  }
+}
+
+__device__ __forceinline__ const int16_t* ids_of(const RouteParams& p, int s, int tok) {
+  return reinterpret_cast<const int16_t*>(p.routing_ptrs[s] + DM_ROUTING_HEADER_BYTES) + static_cast<int64_t>(tok) * p.K;
+}
+
+// Per-warp lane masks: bit l of mask_w[el] = token l of this warp routes to local expert el.  `hist_s`, if not null, counts
+// the routes of every expert.
+__device__ __forceinline__ void mark_ids(const RouteParams& p, const int16_t* ids, const int (&first8)[8], uint32_t* mask_w,
+                                         int32_t* hist_s) {
+  const int first = p.rank * p.e_local;
+  const uint32_t bit = 1u << (threadIdx.x & 31);
+  each_id(p, ids, first8, [&](int, int e) {
+    if (hist_s != nullptr) atomicAdd(&hist_s[e], 1);
+    const int el = e - first;
+    if (el >= 0 && el < p.e_local) atomicOr(&mask_w[el], bit);
+  });
+}
+
+// The pointers of one token's routes; `row` gives the row of a route to a local expert.
+template <class Fn>
+__device__ __forceinline__ void place_ids(const RouteParams& p, const int16_t* ids, const int (&first8)[8], int tok,
+                                          uint64_t dbase, uint64_t cbase, Fn&& row) {
+  const int first = p.rank * p.e_local;
+  each_id(p, ids, first8, [&](int k, int e) {
+    const int el = e - first;
+    if (el < 0 || el >= p.e_local) return;
+    const int pos = row(el);
+    const int64_t route = static_cast<int64_t>(tok) * p.K + k;
+    p.fwd[pos] = static_cast<int64_t>(dbase + static_cast<uint64_t>(tok) * p.gather_stride);
+    p.sct[pos] = static_cast<int64_t>(cbase + static_cast<uint64_t>(route) * p.scatter_stride);
+    if (p.bwd != nullptr) p.bwd[pos] = static_cast<int64_t>(dbase + static_cast<uint64_t>(route) * p.bwd_stride);
+  });
+}
+
+// Padding rows of the expert segments hold a null pointer: warp `w` of `warps` clears its share.
+__device__ __forceinline__ void clear_padding(const RouteParams& p, const int32_t* base, const int32_t* total, int w, int warps) {
+  if (p.m_mult <= 0) return;
+  const int lane = threadIdx.x & 31;
+  for (int el = w; el < p.e_local; el += warps) {
+    const int lo = base[el] + total[el], hi = base[el + 1];
+    for (int r = lo + lane; r < hi; r += 32) {
+      p.fwd[r] = 0;
+      p.sct[r] = 0;
+      if (p.bwd != nullptr) p.bwd[r] = 0;
     }
   }
-  __syncthreads();
 }
 
 __global__ void __launch_bounds__(kChunkTokens) route_count_kernel(RouteParams p) {
   extern __shared__ uint32_t smem_u[];
   uint32_t* mask = smem_u;
   int32_t* hist_s = reinterpret_cast<int32_t*>(smem_u + kChunkWarps * p.e_local);
-  const int s = blockIdx.y, c = blockIdx.x;
-  if (c == 0 && threadIdx.x == 0) {
-    const int peer_t = *reinterpret_cast<const int32_t*>(p.routing_ptrs[s]);
-    if (peer_t != p.T) set_status(p.status, kTokenCountMismatch, s, peer_t, p.T);
-  }
-  build_masks(p, s, c, mask, hist_s, true);
+  const int s = blockIdx.y, c = blockIdx.x, tok = c * kChunkTokens + threadIdx.x;
+  const int16_t* ids = ids_of(p, s, tok);
+  int first8[8];
+  const int peer_t = tok == 0 ? *reinterpret_cast<const int32_t*>(p.routing_ptrs[s]) : p.T;
+  load_ids(ids, 0, tok < p.T ? p.K : 0, first8);
+  for (int i = threadIdx.x; i < kChunkWarps * p.e_local; i += kChunkTokens) mask[i] = 0u;
+  for (int i = threadIdx.x; i < p.E; i += kChunkTokens) hist_s[i] = 0;
+  __syncthreads();
+  if (peer_t != p.T) set_status(p.status, kTokenCountMismatch, s, peer_t, p.T);
+  if (tok < p.T) mark_ids(p, ids, first8, mask + (threadIdx.x >> 5) * p.e_local, hist_s);
+  __syncthreads();
   int32_t* out = p.chunk_counts + (static_cast<int64_t>(s) * p.chunks + c) * p.e_local;
   for (int el = threadIdx.x; el < p.e_local; el += blockDim.x) {
     int n = 0;
@@ -154,26 +201,28 @@ __global__ void __launch_bounds__(kChunkTokens) route_count_kernel(RouteParams p
 
 __device__ __forceinline__ int pad_rows(int n, int m) { return m > 0 ? (n + m - 1) / m * m : n; }
 
-// Padded exclusive prefix of the experts' row counts, by one whole warp (32 experts per step); returns the total.
-// Latency bound: one thread walking the experts paid a dependent shared-memory load and add per expert, and the sum per
-// rank did so once more.  Single-launch kernel 18.4 -> 7.7 us at 128 experts and 16 tokens (8.3 -> 6.3 us at 64 experts
-// and 32 tokens); scan kernel of the general path 22 -> 9 us at 128 experts and 4096 tokens.
+// Padded exclusive prefix of the experts' row counts, by one whole warp: every lane sums neighbouring experts, one scan runs
+// over the lanes; returns the total.  Latency bound: one thread walking the experts paid a dependent shared-memory load and
+// add per expert (single-launch kernel 18.4 us at 128 experts and 16 tokens), a scan per 32 experts still paid its ten
+// shuffles each time (7.7 us).
 __device__ __forceinline__ int64_t warp_padded_prefix(const int32_t* total, int32_t* base, int n, int m_mult, int lane) {
-  int64_t running = 0;
-  for (int i0 = 0; i0 < n; i0 += 32) {
-    const int i = i0 + lane;
-    const int64_t v = i < n ? pad_rows(total[i], m_mult) : 0;
-    int64_t incl = v;
+  const int per = (n + 31) >> 5, lo = lane * per < n ? lane * per : n, hi = lo + per < n ? lo + per : n;
+  int64_t own = 0;
+  for (int i = lo; i < hi; ++i) own += pad_rows(total[i], m_mult);
+  int64_t incl = own;
 #pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-      const int64_t t = __shfl_up_sync(0xffffffffu, incl, d);
-      if (lane >= d) incl += t;
-    }
-    if (i < n) base[i] = static_cast<int32_t>(running + incl - v);
-    running += __shfl_sync(0xffffffffu, incl, 31);
+  for (int d = 1; d < 32; d <<= 1) {
+    const int64_t t = __shfl_up_sync(0xffffffffu, incl, d);
+    if (lane >= d) incl += t;
   }
-  if (lane == 0) base[n] = static_cast<int32_t>(running);
-  return running;
+  int64_t at = incl - own;
+  for (int i = lo; i < hi; ++i) {
+    base[i] = static_cast<int32_t>(at);
+    at += pad_rows(total[i], m_mult);
+  }
+  const int64_t all = __shfl_sync(0xffffffffu, incl, 31);
+  if (lane == 0) base[n] = static_cast<int32_t>(all);
+  return all;
 }
 
 // Padded rows that all experts of one rank receive, by one whole warp.
@@ -240,55 +289,52 @@ __global__ void __launch_bounds__(1024) route_scan_kernel(RouteParams p) {
   }
 }
 
-// Pointers of this chunk's routes: `base` where an expert's segment starts, `seg` its rows of lower chunks.
-__device__ __forceinline__ void route_fill(const RouteParams& p, int s, int c, const uint32_t* mask, const int32_t* base,
-                                           const int32_t* seg) {
-  const int tok = c * kChunkTokens + threadIdx.x;
-  if (tok >= p.T) return;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int16_t* ids = reinterpret_cast<const int16_t*>(p.routing_ptrs[s] + DM_ROUTING_HEADER_BYTES) +
-                       static_cast<int64_t>(tok) * p.K;
-  const int first = p.rank * p.e_local;
-  const uint64_t dbase = p.dispatch_ptrs[s], cbase = p.combine_ptrs[s];
-  for (int k = 0; k < p.K; ++k) {
-    const int el = static_cast<int>(ids[k]) - first;
-    if (ids[k] < 0 || ids[k] >= p.E || el < 0 || el >= p.e_local) continue;
-    int pos = base[el] + seg[el];
-    for (int w = 0; w < warp; ++w) pos += __popc(mask[w * p.e_local + el]);
-    pos += __popc(mask[warp * p.e_local + el] & ((1u << lane) - 1u));
-    const int64_t route = static_cast<int64_t>(tok) * p.K + k;
-    p.fwd[pos] = static_cast<int64_t>(dbase + static_cast<uint64_t>(tok) * p.gather_stride);
-    p.sct[pos] = static_cast<int64_t>(cbase + static_cast<uint64_t>(route) * p.scatter_stride);
-    if (p.bwd != nullptr) p.bwd[pos] = static_cast<int64_t>(dbase + static_cast<uint64_t>(route) * p.bwd_stride);
-  }
-}
-
 __global__ void __launch_bounds__(kChunkTokens) route_fill_kernel(RouteParams p) {
   extern __shared__ uint32_t smem_u[];
   uint32_t* mask = smem_u;
-  const int s = blockIdx.y, c = blockIdx.x;
+  const int s = blockIdx.y, c = blockIdx.x, tok = c * kChunkTokens + threadIdx.x;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (p.expert_offsets[p.e_local] == 0) return;  // nothing routed here, or capacity exceeded
-  build_masks(p, s, c, mask, nullptr, false);
-  route_fill(p, s, c, mask, p.expert_offsets, p.chunk_offsets + (static_cast<int64_t>(s) * p.chunks + c) * p.e_local);
+  const int16_t* ids = ids_of(p, s, tok);
+  int first8[8];
+  load_ids(ids, 0, tok < p.T ? p.K : 0, first8);
+  for (int i = threadIdx.x; i < kChunkWarps * p.e_local; i += kChunkTokens) mask[i] = 0u;
+  __syncthreads();
+  if (tok < p.T) mark_ids(p, ids, first8, mask + warp * p.e_local, nullptr);
+  __syncthreads();
+  if (tok >= p.T) return;
+  const int32_t* seg = p.chunk_offsets + (static_cast<int64_t>(s) * p.chunks + c) * p.e_local;
+  place_ids(p, ids, first8, tok, p.dispatch_ptrs[s], p.combine_ptrs[s], [&](int el) {
+    int pos = p.expert_offsets[el] + seg[el];
+    for (int w = 0; w < warp; ++w) pos += __popc(mask[w * p.e_local + el]);
+    return pos + __popc(mask[warp * p.e_local + el] & ((1u << lane) - 1u));
+  });
 }
 
 // Scan and fill in one launch: every block sums the chunks' counts itself, for where the segments start and for its own
 // rows in them; block 0 writes the tables, and the padding rows are dealt out over the blocks.  Bound by latency, not bytes:
 // the scan was one block that walked all chunks and wrote all padding rows between two launches, and one rank's routes per
-// expert needed a memset and global atomics that block 0 now sums from the chunks.  One rank, padded to 128, the whole
-// routing step: 2,048 tokens x 8 of 32 experts 18.4 -> 10.3 us, 4,096 x 8 of 128 24.6 -> 12.5, 16,384 x 8 of 256
-// 47.9 -> 19.7; eight ranks, 2,048 x 6 of 64, unpadded, 14.6 -> 12.5 us.
+// expert needed a memset and global atomics that block 0 now sums from the chunks.  A block's chain is pointer -> ids (kept
+// in registers for the fill) beside the counts, one prefix, the stores.  One rank, padded to 128, the whole
+// routing step: 2,048 tokens x 8 of 32 experts 18.4 -> 9.4 us, 4,096 x 8 of 128 24.6 -> 11.4, 16,384 x 8 of 256
+// 47.9 -> 19.1; eight ranks, 2,048 x 6 of 64, unpadded, 14.6 -> 11.4 us.
 __global__ void __launch_bounds__(kChunkTokens) route_place_kernel(RouteParams p) {
   extern __shared__ uint32_t smem_u[];
   uint32_t* mask = smem_u;                                                    // [kChunkWarps][e_local]
-  int32_t* total = reinterpret_cast<int32_t*>(mask + kChunkWarps * p.e_local);  // [e_local] real rows
+  uint32_t* wprefix = mask + kChunkWarps * p.e_local;                         // [kChunkWarps][e_local] routes of lower warps
+  int32_t* total = reinterpret_cast<int32_t*>(wprefix + kChunkWarps * p.e_local);  // [e_local] real rows
   int32_t* below = total + p.e_local;                                         // [e_local] of them in lower chunks
   int32_t* routes = below + p.e_local;                                        // [e_local] routes (one rank: of all experts)
   int32_t* base = routes + p.e_local;                                         // [e_local + 1] padded exclusive prefix
   __shared__ int overflow;
-  const int s = blockIdx.y, c = blockIdx.x, me = s * p.chunks + c, n = p.ep * p.chunks;
+  const int s = blockIdx.y, c = blockIdx.x, me = s * p.chunks + c, n = p.ep * p.chunks, tok = c * kChunkTokens + threadIdx.x;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  for (int el = threadIdx.x; el < p.e_local; el += blockDim.x) total[el] = below[el] = routes[el] = 0;
+  const int16_t* ids = ids_of(p, s, tok);
+  const uint64_t dbase = p.dispatch_ptrs[s], cbase = p.combine_ptrs[s];
+  for (int i = threadIdx.x; i < kChunkWarps * p.e_local; i += kChunkTokens) mask[i] = 0u;
+  for (int i = threadIdx.x; i < 3 * p.e_local; i += kChunkTokens) total[i] = 0;  // and below, routes
+  int first8[8];
+  load_ids(ids, 0, tok < p.T ? p.K : 0, first8);
   __syncthreads();
   const int width = p.e_local < kChunkTokens ? p.e_local : kChunkTokens, groups = kChunkTokens / width;
   const int g = threadIdx.x / width, l = threadIdx.x - g * width;
@@ -305,21 +351,33 @@ __global__ void __launch_bounds__(kChunkTokens) route_place_kernel(RouteParams p
         for (int i = g; i < n; i += groups) listed += p.chunk_offsets[static_cast<int64_t>(i) * p.e_local + el];
       atomicAdd(&total[el], sum);
       atomicAdd(&below[el], lower);
-      atomicAdd(&routes[el], listed);
+      if (listed) atomicAdd(&routes[el], listed);
     }
   }
-  build_masks(p, s, c, mask, nullptr, false);  // ends with a block barrier: the sums are there too
-  const int64_t acc = warp == 0 ? warp_padded_prefix(total, base, p.e_local, p.m_mult, lane) : 0;
-  if (threadIdx.x == 0) {
-    overflow = (acc > p.capacity_rows || acc > p.ptrs_size) ? 1 : 0;
-    if (overflow && me == 0) set_status(p.status, kCapacityExceeded, static_cast<int>(acc), static_cast<int>(p.capacity_rows));
-    // ranks that disagree on T cannot be routed: the call becomes a no-op (zero rows), like an overflow
-    if (p.status != nullptr && *reinterpret_cast<volatile int*>(p.status) == kTokenCountMismatch) overflow = 1;
+  if (tok < p.T) mark_ids(p, ids, first8, mask + warp * p.e_local, nullptr);
+  __syncthreads();
+  if (warp == 0) {
+    const int64_t acc = warp_padded_prefix(total, base, p.e_local, p.m_mult, lane);
+    if (lane == 0) {
+      overflow = (acc > p.capacity_rows || acc > p.ptrs_size) ? 1 : 0;
+      if (overflow && me == 0) set_status(p.status, kCapacityExceeded, static_cast<int>(acc), static_cast<int>(p.capacity_rows));
+      // ranks that disagree on T cannot be routed: the call becomes a no-op (zero rows), like an overflow
+      if (p.status != nullptr && *reinterpret_cast<volatile int*>(p.status) == kTokenCountMismatch) overflow = 1;
+    }
+  } else {
+    for (int el = threadIdx.x - 32; el < p.e_local; el += kChunkTokens - 32) {
+      int running = below[el];
+#pragma unroll
+      for (int w = 0; w < kChunkWarps; ++w) {
+        wprefix[w * p.e_local + el] = running;
+        running += __popc(mask[w * p.e_local + el]);
+      }
+    }
   }
   __syncthreads();
   const bool bad = overflow != 0;
   if (me == 0) {
-    for (int el = threadIdx.x; el <= p.e_local; el += blockDim.x) {
+    for (int el = threadIdx.x; el <= p.e_local; el += kChunkTokens) {
       p.expert_offsets[el] = bad ? 0 : base[el];
       if (el < p.e_local) p.counts[el] = bad ? 0 : pad_rows(total[el], p.m_mult);
       if (el < p.e_local && p.real_counts != nullptr) p.real_counts[el] = bad ? 0 : total[el];
@@ -330,22 +388,16 @@ __global__ void __launch_bounds__(kChunkTokens) route_place_kernel(RouteParams p
     }
   }
   if (bad) return;
-  if (p.m_mult > 0) {
-    // Padding rows of every expert segment hold a null pointer.
-    for (int el = me + n * warp; el < p.e_local; el += n * kChunkWarps) {
-      const int lo = base[el] + total[el], hi = base[el + 1];
-      for (int r = lo + lane; r < hi; r += 32) {
-        p.fwd[r] = 0;
-        p.sct[r] = 0;
-        if (p.bwd != nullptr) p.bwd[r] = 0;
-      }
-    }
-  }
-  route_fill(p, s, c, mask, base, below);
+  clear_padding(p, base, total, me + n * warp, n * kChunkWarps);
+  if (tok >= p.T) return;
+  place_ids(p, ids, first8, tok, dbase, cbase, [&](int el) {
+    return base[el] + static_cast<int>(wprefix[warp * p.e_local + el]) +
+           __popc(mask[warp * p.e_local + el] & ((1u << lane) - 1u));
+  });
 }
 
 // ---------------------------------------------------------------------------
-// Decode regime: the whole routing step in one CTA and one launch (the reference's single-launch path,
+// Decode regime: the whole routing step in one launch (the reference's single-launch path,
 // dist_moe/_routing_metadata.py:265-300 and kernels/triton/dist_dispatch_routing_kernel.py:120-260, which
 // orders rows inside an expert by an atomic counter; this kernel keeps the general path's deterministic order).
 //
@@ -353,9 +405,16 @@ __global__ void __launch_bounds__(kChunkTokens) route_place_kernel(RouteParams p
 // order of the output rows inside an expert: a row's position is its expert's base + the routes of lower warps
 // + the routes of lower lanes of its own warp, all from per-warp lane masks in shared memory.  No workspace,
 // no histogram in global memory, no memset.
+//
+// Latency bound.  The tables are cheap enough that every block of a small grid builds them all; block 0 writes them, the
+// pointers and the padding rows (up to 127 per expert, which one SM took 4 to 13 us to store) are dealt out over the blocks.
+// The ids are loaded once, beside the other addresses, and stay in registers.  One rank, padded to 128: 16 tokens x 8 of 128
+// experts 9.8 -> 5.7 us, 128 x 8 of 32 6.6 -> 5.6, 128 x 8 of 256 21.3 -> 6.9, 1,024 x 8 of 64 20.0 -> 7.8; unpadded,
+// 32 x 6 of 64 5.2 -> 5.1; eight ranks of 8 experts, 64 tokens each, 6.5 -> 6.8.
 // ---------------------------------------------------------------------------
 constexpr int kDecodeThreads = 1024;
 constexpr int kDecodeWarps = kDecodeThreads / 32;
+constexpr int kDecodeBlocks = 32, kDecodePadding = 512;  // at most so many blocks, one per so many padding rows
 
 __global__ void __launch_bounds__(kDecodeThreads) route_decode_kernel(RouteParams p) {
   extern __shared__ uint32_t smem_u[];
@@ -367,40 +426,32 @@ __global__ void __launch_bounds__(kDecodeThreads) route_decode_kernel(RouteParam
   __shared__ int overflow;
   __shared__ int mismatch;
   const int i = threadIdx.x, warp = i >> 5, lane = i & 31;
-  if (i == 0) mismatch = 0;
-  for (int j = i; j < kDecodeWarps * p.e_local; j += kDecodeThreads) mask[j] = 0u;
-  for (int j = i; j < p.E; j += kDecodeThreads) hist_s[j] = 0;
-  __syncthreads();
+  const bool writer = blockIdx.x == 0;
+  const int used = (p.ep * p.T + 31) >> 5;  // warps that hold tokens
   const int s = i / p.T, tok = i - s * p.T;
   const bool live = s < p.ep;
-  const int first = p.rank * p.e_local;
   const int16_t* ids = nullptr;
+  uint64_t dbase = 0, cbase = 0;
+  int first8[8], peer_t = p.T;
   if (live) {
-    if (tok == 0) {
-      const int peer_t = *reinterpret_cast<const int32_t*>(p.routing_ptrs[s]);
-      if (peer_t != p.T) {
-        set_status(p.status, kTokenCountMismatch, s, peer_t, p.T);
-        mismatch = 1;
-      }
+    ids = ids_of(p, s, tok);
+    if (tok == 0) peer_t = *reinterpret_cast<const int32_t*>(p.routing_ptrs[s]);
+    dbase = p.dispatch_ptrs[s];
+    cbase = p.combine_ptrs[s];
+    load_ids(ids, 0, p.K, first8);
+  }
+  if (i == 0) mismatch = 0;
+  for (int j = i; j < used * p.e_local; j += kDecodeThreads) mask[j] = 0u;
+  for (int j = i; j < p.E; j += kDecodeThreads) hist_s[j] = 0;
+  __syncthreads();
+  if (live) {
+    if (peer_t != p.T) {
+      if (writer) set_status(p.status, kTokenCountMismatch, s, peer_t, p.T);
+      mismatch = 1;
     }
-    ids = reinterpret_cast<const int16_t*>(p.routing_ptrs[s] + DM_ROUTING_HEADER_BYTES) + static_cast<int64_t>(tok) * p.K;
-    for (int k0 = 0; k0 < p.K; k0 += 8) {
-      // eight ids on their way before the first shared-memory atomic (which the loads could not be moved across)
-      int e8[8];
-#pragma unroll
-      for (int j = 0; j < 8; ++j) e8[j] = k0 + j < p.K ? static_cast<int>(ids[k0 + j]) : -1;
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const int e = e8[j];
-        if (e < 0 || e >= p.E) continue;
-        atomicAdd(&hist_s[e], 1);
-        const int el = e - first;
-        if (el >= 0 && el < p.e_local) atomicOr(&mask[warp * p.e_local + el], 1u << lane);
-      }
-    }
+    mark_ids(p, ids, first8, mask + warp * p.e_local, writer ? hist_s : nullptr);
   }
   __syncthreads();
-  const int used = (p.ep * p.T + 31) >> 5;  // warps that hold tokens
   for (int el = i; el < p.e_local; el += kDecodeThreads) {
     int running = 0;
     for (int w = 0; w < used; ++w) {
@@ -413,50 +464,30 @@ __global__ void __launch_bounds__(kDecodeThreads) route_decode_kernel(RouteParam
   const int64_t acc = warp == 0 ? warp_padded_prefix(total, base, p.e_local, p.m_mult, lane) : 0;
   if (i == 0) {
     overflow = (acc > p.capacity_rows || acc > p.ptrs_size) ? 1 : 0;
-    if (overflow) set_status(p.status, kCapacityExceeded, static_cast<int>(acc), static_cast<int>(p.capacity_rows));
+    if (overflow && writer) set_status(p.status, kCapacityExceeded, static_cast<int>(acc), static_cast<int>(p.capacity_rows));
     if (mismatch) overflow = 1;  // ranks that disagree on T: zero rows, the call becomes a no-op
   }
   __syncthreads();
   const bool bad = overflow != 0;
-  for (int el = i; el <= p.e_local; el += kDecodeThreads) {
-    p.expert_offsets[el] = bad ? 0 : base[el];
-    if (el < p.e_local) p.counts[el] = bad ? 0 : pad_rows(total[el], p.m_mult);
-    if (el < p.e_local && p.real_counts != nullptr) p.real_counts[el] = bad ? 0 : total[el];
-  }
-  for (int q = warp; q < p.ep; q += kDecodeWarps) {
-    const int sum = warp_padded_sum(hist_s + q * p.e_local, p.e_local, p.m_mult, lane);
-    if (lane == 0) p.per_rank[q] = sum;
+  if (writer) {
+    for (int el = i; el <= p.e_local; el += kDecodeThreads) {
+      p.expert_offsets[el] = bad ? 0 : base[el];
+      if (el < p.e_local) p.counts[el] = bad ? 0 : pad_rows(total[el], p.m_mult);
+      if (el < p.e_local && p.real_counts != nullptr) p.real_counts[el] = bad ? 0 : total[el];
+    }
+    for (int q = warp; q < p.ep; q += kDecodeWarps) {
+      const int sum = warp_padded_sum(hist_s + q * p.e_local, p.e_local, p.m_mult, lane);
+      if (lane == 0) p.per_rank[q] = sum;
+    }
   }
   if (bad) return;
-  if (p.m_mult > 0) {
-    // Padding rows of every expert segment hold a null pointer.
-    for (int el = warp; el < p.e_local; el += kDecodeWarps) {
-      const int lo = base[el] + total[el], hi = base[el + 1];
-      for (int r = lo + lane; r < hi; r += 32) {
-        p.fwd[r] = 0;
-        p.sct[r] = 0;
-        if (p.bwd != nullptr) p.bwd[r] = 0;
-      }
-    }
-  }
-  if (!live) return;
-  const uint64_t dbase = p.dispatch_ptrs[s], cbase = p.combine_ptrs[s];
-  for (int k0 = 0; k0 < p.K; k0 += 8) {
-    int e8[8];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) e8[j] = k0 + j < p.K ? static_cast<int>(ids[k0 + j]) : -1;
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const int el = e8[j] - first;
-      if (e8[j] < 0 || e8[j] >= p.E || el < 0 || el >= p.e_local) continue;
-      const int pos = base[el] + static_cast<int>(wprefix[warp * p.e_local + el]) +
-                      __popc(mask[warp * p.e_local + el] & ((1u << lane) - 1u));
-      const int64_t route = static_cast<int64_t>(tok) * p.K + k0 + j;
-      p.fwd[pos] = static_cast<int64_t>(dbase + static_cast<uint64_t>(tok) * p.gather_stride);
-      p.sct[pos] = static_cast<int64_t>(cbase + static_cast<uint64_t>(route) * p.scatter_stride);
-      if (p.bwd != nullptr) p.bwd[pos] = static_cast<int64_t>(dbase + static_cast<uint64_t>(route) * p.bwd_stride);
-    }
-  }
+  const int blocks = static_cast<int>(gridDim.x);
+  clear_padding(p, base, total, static_cast<int>(blockIdx.x) + blocks * warp, blocks * kDecodeWarps);
+  if (live && warp % blocks == static_cast<int>(blockIdx.x))
+    place_ids(p, ids, first8, tok, dbase, cbase, [&](int el) {
+      return base[el] + static_cast<int>(wprefix[warp * p.e_local + el]) +
+             __popc(mask[warp * p.e_local + el] & ((1u << lane) - 1u));
+    });
 }
 
 // ---------------------------------------------------------------------------
@@ -601,7 +632,9 @@ static int route_launch(const uint64_t* routing_ptrs, const uint64_t* dispatch_p
                                static_cast<int>(sizeof(uint32_t) * (2 * kDecodeWarps * 512 + kMaxExpertsSmem + 1025))));
     });
     if (rc_attr != 0) return rc_attr;
-    route_decode_kernel<<<1, kDecodeThreads, smem, st>>>(p);
+    const int64_t padding = static_cast<int64_t>(p.e_local) * (m_multiple_of > 0 ? m_multiple_of - 1 : 0);
+    const int64_t blocks = padding / kDecodePadding + 1;
+    route_decode_kernel<<<static_cast<int>(blocks < kDecodeBlocks ? blocks : kDecodeBlocks), kDecodeThreads, smem, st>>>(p);
     return static_cast<int>(cudaGetLastError());
   }
   // The sums cost every block a read of all chunks' counts, so the work grows with the square of the chunks; the scan's one
@@ -619,7 +652,7 @@ static int route_launch(const uint64_t* routing_ptrs, const uint64_t* dispatch_p
   const size_t smem_fill = sizeof(uint32_t) * (kChunkWarps * p.e_local);
   route_count_kernel<<<grid, kChunkTokens, smem_count, st>>>(p);
   if (place) {
-    route_place_kernel<<<grid, kChunkTokens, smem_fill + sizeof(int32_t) * (4 * p.e_local + 1), st>>>(p);
+    route_place_kernel<<<grid, kChunkTokens, 2 * smem_fill + sizeof(int32_t) * (4 * p.e_local + 1), st>>>(p);
     return static_cast<int>(cudaGetLastError());
   }
   route_scan_kernel<<<1, 1024, sizeof(int32_t) * (2 * p.e_local + 1), st>>>(p);

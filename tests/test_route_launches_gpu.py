@@ -1,4 +1,5 @@
-"""The general routing path up to 1,024 chunks of 256 tokens (two launches) and beyond (three) against the CPU oracle."""
+"""The routing launches at the sizes where they change, against the CPU oracle: the blocks of the single launch, two launches up
+to 1,024 chunks of 256 tokens, three beyond."""
 
 import numpy as np
 import pytest
@@ -42,6 +43,24 @@ def test_tables_are_the_oracles(ep, T, K, E, m_mult):
     ids[rng.random(ids.shape) < 0.05] = -1
     for rank in sorted({0, ep - 1}):
         check(ids, rank, E, m_mult)
+
+
+@pytest.mark.parametrize("ep,T,K,E,m_mult", [
+    (1, 5, 2, 4, 128),      # 508 padding rows: one block
+    (1, 5, 2, 5, 128),      # 635: two
+    (1, 1024, 9, 512, 128),  # the largest of everything: 32 blocks, an id past the eighth
+    (4, 33, 3, 64, 128),
+])
+def test_single_launch_over_several_blocks(ep, T, K, E, m_mult):
+    rng = np.random.default_rng(T + E)
+    ids = np.argsort(-rng.standard_normal((ep, T, E)), axis=-1)[..., :K].astype(np.int64)
+    ids[rng.random(ids.shape) < 0.05] = -1
+    for rank in sorted({0, ep - 1}):
+        rows = check(ids, rank, E, m_mult)
+    disp, comb = [(s + 1) << 40 for s in range(ep)], [(s + 1) << 41 for s in range(ep)]
+    out = run_route(ids, ep - 1, E, disp, comb, 1024, 1024, 1024, m_mult, capacity=rows - 1)
+    assert out["status"][0] == 2 and out["status"][1] == rows
+    assert not out["offsets"].any() and not out["counts"].any() and (out["fwd"] == -5).all()
 
 
 def test_every_token_on_one_expert_and_no_token_at_all():
