@@ -244,7 +244,8 @@ for _name, (_res, _args) in _SIGNATURES.items():
 # Kernel launches issued through this binding (benchmarks report the count).
 LAUNCHES = [0]
 _LAUNCHES_PER_CALL = {"dm_route": 3, "dm_route_counted": 3}
-_ROUTE_CHUNK_TOKENS, _ROUTE_TWO_LAUNCH_CHUNKS = 256, 1024  # include/dist_moe_b200.h
+GATHER_FLAGS_KEPT_CLEAR = 1 << 30  # include/dist_moe_b200.h, as the next two
+_ROUTE_CHUNK_TOKENS, _ROUTE_TWO_LAUNCH_CHUNKS = 256, 1024
 
 
 def route_call_name(ep: int, tokens: int, e_local: int) -> str:

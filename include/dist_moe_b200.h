@@ -307,10 +307,13 @@ int dm_gemm_dgrad(dm_operand a, const void* w, dm_operand c, const int64_t* scat
  * allowed) by four extra warps of every CTA of the persistent kernel while the tensor cores already work
  * on the rows that have landed; `a` names where the pulled rows are kept (x_gathered / grad_h3_gathered,
  * needed again by the weight-gradient GEMMs).  gather_flags: int32[max_rows/128 + 2] scratch, cleared by
- * the call; it belongs to this launch until it has finished.  Rows are pulled only by CTAs that are running, so
+ * the call; it belongs to this launch until it has finished.  With DM_GATHER_FLAGS_KEPT_CLEAR or'ed into num_sms (here, or
+ * in a dm_layer_context) the call finds int32[max_rows/128 + 3] cleared and leaves them cleared, without a launch for it:
+ * for a scratch that nothing else writes.  Rows are pulled only by CTAs that are running, so
  * kernels of other streams that hold SMs delay the call but do not fail it.  Replaces
  * dist_grouped_gemm_fprop_dispatch / ..._dgrad_dispatch in one launch
  * (dist_moe/kernels/dist_grouped_gemm.py:1148-1237, 1441-1489). */
+#define DM_GATHER_FLAGS_KEPT_CLEAR (1 << 30)
 int dm_gemm_fprop_dispatch(const int64_t* gather_ptrs, int32_t* gather_flags, dm_operand a, const void* w,
                            dm_operand c, dm_operand h2, const int32_t* expert_offsets, int e_local, int64_t max_rows,
                            int64_t N, int64_t Kd, int fuse_swiglu, int clamped, float alpha, float limit,
