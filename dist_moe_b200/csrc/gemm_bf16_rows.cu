@@ -166,7 +166,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kRwThreads, 1) rows_
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();
-  const int first_tile = blockIdx.x >> 1, tile_step = gridDim.x >> 1;
 
   // The gather warps' first units: those of the first tiles go to the CTAs that start first.
   const bool gathers = warp >= 10 && warp < 10 + kRwGatherWarps && p.gather_flags != nullptr;
@@ -223,6 +222,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kRwThreads, 1) rows_
   tcgen05_fence_after();
   const uint32_t tmem_base = uniform(tmem_base_slot);
   const int total_tiles = uniform(s_tile_start[p.e_local]);
+  // One B200, 64 experts x 2048 x 1408, W13 / W2, rows per expert on average: 3 117.7 / 61.7 -> 117.2 / 61.6 us, 48 128.7 / 67.4 ->
+  // 127.1 / 67.2, 64 131.1 / 66.1 -> 129.7 / 65.4, 96 136.6 / 68.4 -> 135.4 / 68.2; decode layer of 32 tokens 197.6 -> 195.3.  At
+  // 187 rows on average, tiles of up to 256, nothing changes (312.2 and 312.8 us a layer).
+  const int pair = blockIdx.x >> 1;
+  const int tile_step = balanced_pairs(total_tiles, gridDim.x >> 1, 2 * rw_box_rows(uniform(s_box)), 128);
+  const int first_tile = pair < tile_step ? pair : total_tiles;
   // ring: stages as large as the launch's largest tile needs
   const uint32_t stage_bytes = kRwWBytes + static_cast<uint32_t>(rw_box_rows(uniform(s_box))) * 128;
   const int fit = static_cast<int>(kRing / stage_bytes);
