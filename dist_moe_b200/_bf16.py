@@ -21,7 +21,8 @@ from typing import Any
 import torch
 
 from . import _native as nat
-from ._call import BWD, FWD, FWD_ALL, CallState, Layout, arguments, launch, layout_of, observed, on_device, recorded, span
+from ._call import (BWD, FWD, FWD_ALL, CallState, Layout, arguments, in_one_piece, launch, layout_of, observed, on_device,
+                    recorded, span)
 from ._execution import ExecutionOptions, RMSNormPostprocess
 
 
@@ -92,6 +93,11 @@ def _arguments(state, c: _Call, x, ids, scores, w13, w2, options: ExecutionOptio
     return k
 
 
+def _weights_in_one_piece(state, w13, w2):
+    n = state.e_local * state.config.intermediate_dim * state.config.hidden_dim
+    return in_one_piece(w13, 2 * n, "w13"), in_one_piece(w2, n, "w2")
+
+
 def _forward(state, k, steps: int) -> None:
     launch(nat.lib.dm_bf16_forward, FWD, state, k, steps)
 
@@ -105,6 +111,7 @@ def forward_impl(state, x, ids, scores, w13, w2, options: ExecutionOptions, save
     """``separate``: the call's device results as tensors of their own (registered operators return them)."""
     cfg = state.config
     T, F = x.shape[0], cfg.intermediate_dim
+    w13, w2 = _weights_in_one_piece(state, w13, w2)
     scratch_only = (not save_for_backward) or cfg.inference or state.num_slots == 0
     c = _Call(state, T, not scratch_only).allocate(x.device, separate)
     out = torch.empty(x.shape, dtype=torch.bfloat16, device=x.device)
@@ -185,6 +192,8 @@ def backward_impl(state, c: _Call, x_shape, ids, scores, w13, w2, w13_param, w2_
     T, D, K, F, el = c.T, cfg.hidden_dim, cfg.top_k, cfg.intermediate_dim, state.e_local
     dev = grad_out.device
     need_x, need_scores, need_w13, need_w2 = needs
+    w13, w2 = _weights_in_one_piece(state, w13, w2)
+    ids, scores = in_one_piece(ids, T * K, "topk_expert_ids_TK"), in_one_piece(scores, T * K, "topk_scores_TK")
     # the plan's offsets: [xg, h1, h2, grad_h2, grad_h3_gathered, grad_h1]
     bo = torch.empty(6, dtype=torch.int64, device=dev) if c.buf is None else None
     grad_scores = torch.empty(T, K, dtype=torch.float32, device=dev) if need_scores else None
@@ -326,7 +335,7 @@ class _RegisteredBf16Function(torch.autograd.Function):
         clip = options.swiglu_clip_stats_out_3
         ctx.context, ctx.options = context, options
         if clip is None and _plain_execution(x, ids, scores, w13_param, w2_param):
-            # gradients are off here, and of the weights only the address counts (sizes and layout have been checked)
+            # gradients are off here
             out, call = forward_impl(state, x, ids, scores, w13_param, w2_param, options, True)
             # What a call saves must not depend on the way it goes where saved-tensor hooks look at it: activation
             # checkpointing compares a forward with its repetition, which may run under other modes.

@@ -121,6 +121,16 @@ def launch(fn, names: dict, state, k, steps: int) -> None:
         profile.append((timed[name], start, end))
 
 
+def in_one_piece(t: torch.Tensor, numel: int, name: str) -> torch.Tensor:
+    """``t``, or a contiguous copy of it, for a pass that uses the address alone.  Checks at the entry point do not cover this: there
+    a weight's dimensions are merged first, which copies a (E, 2, F, D) view whose leading dimensions do not merge, and what a
+    backward unpacks is the leaf as it is at that moment (its ``.data`` may have been replaced) or what a saved-tensor hook made of
+    it.  The caller keeps the result alive until the pass is launched."""
+    if t.numel() != numel:
+        raise RuntimeError(f"{name} has {numel} elements in this call, not {t.numel()} (shape {tuple(t.shape)})")
+    return t if t.is_contiguous() else t.detach().contiguous()
+
+
 class Layout:
     """Where the device results of a call lie in their buffer.  ``fields``: name -> (dtype, elements)."""
 
