@@ -16,6 +16,7 @@ CUDA graph.  Bracketed steps are device-predicated on the planner's decision.
 
 from __future__ import annotations
 
+import math
 from typing import Any
 
 import torch
@@ -160,6 +161,8 @@ def _wgrad_destination(param: torch.Tensor, shape, options: ExecutionOptions, cf
         named = hooks.wgrad_destination(name, shape, cfg.wgrad_dtype or param.dtype, param.device)
         if named is not None:
             return named[0], int(named[1]), False
+    if param.numel() != math.prod(shape):  # the weight may be another one by now than in the forward; a GEMM writes all of ``shape``
+        raise RuntimeError(f"the gradient of a weight of shape {tuple(param.shape)} cannot hold one of shape {tuple(shape)}")
     if isinstance(explicit, torch.Tensor):
         if not explicit.is_contiguous() or explicit.dtype not in (torch.bfloat16, torch.float32) \
                 or explicit.numel() != param.numel():
