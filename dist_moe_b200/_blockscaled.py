@@ -435,11 +435,11 @@ def run_block_scaled(x, ids, scores, w13_weight, w2_weight, context: Any, option
         from ._postprocess import validate_rmsnorm
 
         validate_rmsnorm(post, config=cfg, training=False, x_dtype=out.dtype)
-        nat.check(nat.lib.dm_rmsnorm_combine_fwd(
+        nat.check(nat.lib.dm_rmsnorm_combine_fwd_status(
             state.combine.local().data_ptr(), scores.data_ptr(), int(scores.dtype == torch.bfloat16), ids.data_ptr(),
             int(ids.dtype == torch.int64), nat.ptr(post.weight), float(post.gain_center), float(post.eps),
             int(post.norm_output_dtype == torch.bfloat16), int(bool(post.use_kahan)), out.data_ptr(), None, T, K, D,
-            None, None, None, 0, st), "dm_rmsnorm_combine_fwd")
+            None, None, None, 0, status, st), "dm_rmsnorm_combine_fwd")
     else:
         nat.check(nat.lib.dm_scale_and_sum(state.combine.local().data_ptr(), scores.data_ptr(),
                                            int(scores.dtype == torch.bfloat16), ids.data_ptr(),

@@ -196,6 +196,11 @@ _SIGNATURES = {
         [_P, _P, c_int, _P, c_int, _P, c_float, c_float, c_int, c_int, _P, _P, c_int64, c_int, c_int64, _P, _P, _P, c_int,
          _P],
     ),
+    "dm_rmsnorm_combine_fwd_status": (
+        c_int,
+        [_P, _P, c_int, _P, c_int, _P, c_float, c_float, c_int, c_int, _P, _P, c_int64, c_int, c_int64, _P, _P, _P, c_int,
+         _P, _P],
+    ),
     "dm_rmsnorm_combine_bwd": (
         c_int,
         [_P, _P, c_int, _P, c_int, _P, _P, _P, c_float, c_int, c_int, _P, _P, c_int64, c_int, c_int64, _P],

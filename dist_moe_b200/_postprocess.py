@@ -1,6 +1,6 @@
 """Typed post-expert processing: fused RMSNorm + score-weighted top-k reduction.
 
-Host-side validation and launch of ``dm_rmsnorm_combine_fwd/bwd``; mirrors the contract of the
+Host-side validation and launch of ``dm_rmsnorm_combine_fwd_status`` and ``dm_rmsnorm_combine_bwd``; mirrors the contract of the
 reference's ``RMSNormPostprocess`` path (dist_moe/_postprocess.py:648-719 validation,
 dist_moe/kernels/norm/fused_rmsnorm_combine.py:326-348 tensor contract).
 """
@@ -54,11 +54,11 @@ def rmsnorm_combine_forward(state, call, post: RMSNormPostprocess, scores, ids, 
         base, offset, cond = state.arena.data_ptr(), call.fwd_state[4:5].data_ptr(), call.cond.data_ptr()
     else:
         base = offset = cond = None
-    nat.check(nat.lib.dm_rmsnorm_combine_fwd(
+    nat.check(nat.lib.dm_rmsnorm_combine_fwd_status(
         state.combine.local().data_ptr(), scores.data_ptr(), int(scores.dtype == torch.bfloat16), ids.data_ptr(),
         int(ids.dtype == torch.int64), nat.ptr(post.weight), float(post.gain_center), float(post.eps),
         int(post.norm_output_dtype == torch.bfloat16), int(bool(post.use_kahan)), out.data_ptr(), nat.ptr(rstd), T, K,
-        D, base, offset, cond, 0, nat.stream_ptr()), "dm_rmsnorm_combine_fwd")
+        D, base, offset, cond, 0, state.status.data_ptr(), nat.stream_ptr()), "dm_rmsnorm_combine_fwd")
     return rstd
 
 

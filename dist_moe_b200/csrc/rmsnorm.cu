@@ -59,22 +59,16 @@ __device__ __forceinline__ void warp_reduce_sumsq(float& ss, float& cc, int kaha
   }
 }
 
+// A block's tokens from `first` on, their rows read from memory.
 template <typename IdT>
-__global__ void __launch_bounds__(256) rmsnorm_combine_fwd_kernel(
-    const uint4* __restrict__ h3, const void* scores, int scores_bf16, const IdT* __restrict__ ids,
-    const uint4* __restrict__ gamma, float gain_center, float eps, int norm_bf16, uint4* __restrict__ out,
-    float* __restrict__ rstd_out, int64_t T, int K, int vec, uint8_t* save_base, const int64_t* save_offset,
-    const int* save_cond, int save_expect, int kahan) {
-  __shared__ float part[kNormMaxK][8];
-  __shared__ float partc[kNormMaxK][8];
-  __shared__ float rs[kNormMaxK];
-  bool save = save_base != nullptr;
-  if (save && save_cond != nullptr) save = ((*save_cond != 0) == (save_expect != 0));
-  if (save && save_offset != nullptr) save = *save_offset >= 0;
-  uint4* save_dst = save ? reinterpret_cast<uint4*>(save_base + (save_offset ? *save_offset : 0)) : nullptr;
+__device__ __forceinline__ void norm_tokens(int64_t first, const uint4* __restrict__ h3, const void* scores, int scores_bf16,
+                                            const IdT* __restrict__ ids, const uint4* __restrict__ gamma, float gain_center, float eps,
+                                            int norm_bf16, uint4* __restrict__ out, float* __restrict__ rstd_out, int64_t T, int K,
+                                            int vec, uint4* save_dst, int kahan, float (*part)[8], float (*partc)[8], float* rs) {
+  const bool save = save_dst != nullptr;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const float inv_d = 1.0f / static_cast<float>(vec * 8);
-  for (int64_t t = blockIdx.x; t < T; t += gridDim.x) {
+  for (int64_t t = first; t < T; t += gridDim.x) {
     for (int k = 0; k < K; ++k) {
       const int64_t route = t * K + k;
       float ss = 0.f, cc = 0.f;
@@ -150,19 +144,47 @@ __global__ void __launch_bounds__(256) rmsnorm_combine_fwd_kernel(
     __syncthreads();
   }
 }
+// The same out of line: what the staged form below falls back on costs its registers and its code nothing.
+template <typename IdT>
+__device__ __noinline__ void norm_tokens_late(int64_t first, const uint4* h3, const void* scores, int scores_bf16, const IdT* ids,
+                                              const uint4* gamma, float gain_center, float eps, int norm_bf16, uint4* out,
+                                              float* rstd_out, int64_t T, int K, int vec, uint4* save_dst, int kahan,
+                                              float (*part)[8], float (*partc)[8], float* rs) {
+  norm_tokens<IdT>(first, h3, scores, scores_bf16, ids, gamma, gain_center, eps, norm_bf16, out, rstd_out, T, K, vec, save_dst, kahan,
+                   part, partc, rs);
+}
+
+template <typename IdT>
+__global__ void __launch_bounds__(256) rmsnorm_combine_fwd_kernel(
+    const uint4* __restrict__ h3, const void* scores, int scores_bf16, const IdT* __restrict__ ids,
+    const uint4* __restrict__ gamma, float gain_center, float eps, int norm_bf16, uint4* __restrict__ out,
+    float* __restrict__ rstd_out, int64_t T, int K, int vec, uint8_t* save_base, const int64_t* save_offset,
+    const int* save_cond, int save_expect, int kahan, int*) {
+  __shared__ float part[kNormMaxK][8];
+  __shared__ float partc[kNormMaxK][8];
+  __shared__ float rs[kNormMaxK];
+  bool save = save_base != nullptr;
+  if (save && save_cond != nullptr) save = ((*save_cond != 0) == (save_expect != 0));
+  if (save && save_offset != nullptr) save = *save_offset >= 0;
+  uint4* save_dst = save ? reinterpret_cast<uint4*>(save_base + (save_offset ? *save_offset : 0)) : nullptr;
+  norm_tokens<IdT>(blockIdx.x, h3, scores, scores_bf16, ids, gamma, gain_center, eps, norm_bf16, out, rstd_out, T, K, vec, save_dst,
+                   kahan, part, partc, rs);
+}
 
 // The same sums in the same order with a token's K rows, which are contiguous, in shared memory: one bulk copy per token, the next
 // token's on its way while this one is worked on.  The kernel above has two loads of a thread in flight, reads every row twice and
 // looks at its options for every element (17 instructions each; issue-bound once the loads overlap: 41 us in the first example
 // below); here they are template parameters, and four rows are summed and reduced side by side.  One B200, us: T = 4096, K = 4, D =
 // 2816 61 -> 29; K = 8: D = 1024 53 -> 24, 4096 129 -> 62, 7168 235 -> 160 (one block per SM); T = 16, K = 4, D = 2816 8.4 -> 4.0.
-// Bound: HBM (92 MB in 29 us, 0.6 of the copy rate) and the three barriers of a token.
+// Bound: HBM (92 MB in 29 us, 0.6 of the copy rate) and the three barriers of a token.  What the loop keeps for a copy that does not
+// come in time costs 0.3 us of the first example and under 0.1 at T = 16; asking all threads at a barrier (__syncthreads_or) cost
+// 2.0, copies by the threads that read them (cp.async), which need no such thing, 5.7.
 template <typename IdT, bool kGamma, bool kNorm16, bool kKahan>
 __global__ void __launch_bounds__(256, kNormBlocks) rmsnorm_combine_fwd_staged_kernel(
     const uint4* __restrict__ h3, const void* scores, int scores_bf16, const IdT* __restrict__ ids,
     const uint4* __restrict__ gamma, float gain_center, float eps, int, uint4* __restrict__ out,
     float* __restrict__ rstd_out, int64_t T, int K, int vec, uint8_t* save_base, const int64_t* save_offset,
-    const int* save_cond, int save_expect, int, int buffers) {
+    const int* save_cond, int save_expect, int, int* status, int buffers) {
   extern __shared__ __align__(128) uint8_t smem[];
   __shared__ uint64_t full[2];
   __shared__ int abort_flag;
@@ -178,7 +200,9 @@ __global__ void __launch_bounds__(256, kNormBlocks) rmsnorm_combine_fwd_staged_k
   const float inv_d = 1.0f / static_cast<float>(vec * 8);
   const int rows = K * vec;  // vectors of a token
   const uint32_t bytes = static_cast<uint32_t>(rows) * 16;
+  int issued = 0;  // copies that thread 0 has started
   auto fetch = [&](int64_t t, int b) {
+    ++issued;
     mbar_arrive_expect_tx(&full[b], bytes);
     bulk_load(smem + b * bytes, h3 + t * rows, bytes, &full[b]);
   };
@@ -203,8 +227,11 @@ __global__ void __launch_bounds__(256, kNormBlocks) rmsnorm_combine_fwd_staged_k
     const bool valid = threadIdx.x < K && ids[t * K + threadIdx.x] >= 0;
     const uint32_t parity = buffers == 2 ? (it >> 1) & 1 : it & 1;
     uint4* src = reinterpret_cast<uint4*>(smem + b * bytes);
-    if (!mbar_wait(&full[b], parity, &abort_flag))  // a copy that never came (none is known to): fetch the rows by hand
-      for (int v = threadIdx.x; v < rows; v += 256) src[v] = h3[t * rows + v];  // each thread reads what it has written alone
+    // A copy that did not come in time (none is known): a thread fetches the rows' pieces that it reads itself.  The copy may still
+    // land, with the same bytes; the block leaves this loop before anything else takes their place.
+    if (!mbar_wait(&full[b], parity, &abort_flag))
+      for (int k = 0; k < K; ++k)
+        for (int v = threadIdx.x; v < vec; v += 256) src[k * vec + v] = h3[t * rows + k * vec + v];
     // four rows at a time: their loads, sums and reductions overlap
     for (int k0 = 0; k0 < K; k0 += 4) {
       float ss[4] = {0.f, 0.f, 0.f, 0.f}, cc[4] = {0.f, 0.f, 0.f, 0.f};
@@ -264,6 +291,8 @@ __global__ void __launch_bounds__(256, kNormBlocks) rmsnorm_combine_fwd_staged_k
       if (rstd_out != nullptr) rstd_out[t * K + threadIdx.x] = r;
     }
     __syncthreads();
+    // raised before the barriers above, or by a wait for the next token: the same for all threads
+    const bool stop = *const_cast<volatile int*>(&abort_flag) != 0;
     for (int v = threadIdx.x; v < vec; v += 256) {
       float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
       float g[8];
@@ -289,6 +318,19 @@ __global__ void __launch_bounds__(256, kNormBlocks) rmsnorm_combine_fwd_staged_k
                                     pack_bf16x2(acc[4], acc[5]), pack_bf16x2(acc[6], acc[7]));
     }
     __syncthreads();
+    if (stop) {  // no further copies; the rest of the block's tokens with their rows in memory, and the copies under way to their end
+      norm_tokens_late<IdT>(ahead, h3, scores, scores_bf16, ids, gamma, gain_center, eps, kNorm16, out, rstd_out, T, K, vec, save_dst,
+                            kKahan, part, partc, rs);
+      if (threadIdx.x == 0) {
+        set_status(status, kPipelineTimeout, 5, blockIdx.x);
+        const uint64_t t0 = globaltimer_ns();
+        for (; it < issued; ++it)
+          while (!mbar_try_wait(&full[buffers == 2 ? it & 1 : 0], buffers == 2 ? (it >> 1) & 1 : it & 1) &&
+                 globaltimer_ns() - t0 < 1000000000ull) {
+          }
+      }
+      return;
+    }
     if (buffers == 2)
       b ^= 1;
     else if (threadIdx.x == 0 && ahead < T)
@@ -379,11 +421,11 @@ __global__ void __launch_bounds__(256) rmsnorm_combine_bwd_kernel(
 
 using namespace dm;
 
-extern "C" int dm_rmsnorm_combine_fwd(const void* h3, const void* scores, int scores_are_bf16, const void* ids,
-                                      int ids_are_int64, const void* gamma, float gain_center, float eps,
-                                      int norm_is_bf16, int use_kahan, void* out, float* rstd_out, int64_t T, int K,
-                                      int64_t D, void* save_base, const int64_t* save_offset, const int* save_cond,
-                                      int save_expect, void* stream) {
+extern "C" int dm_rmsnorm_combine_fwd_status(const void* h3, const void* scores, int scores_are_bf16, const void* ids,
+                                             int ids_are_int64, const void* gamma, float gain_center, float eps,
+                                             int norm_is_bf16, int use_kahan, void* out, float* rstd_out, int64_t T, int K,
+                                             int64_t D, void* save_base, const int64_t* save_offset, const int* save_cond,
+                                             int save_expect, int* status, void* stream) {
   if (!h3 || !scores || !ids || !out || T <= 0 || K <= 0 || K > kNormMaxK || D <= 0 || (D % 8) != 0) return kRcBadArg;
   const int vec = static_cast<int>(D / 8);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
@@ -392,7 +434,7 @@ extern "C" int dm_rmsnorm_combine_fwd(const void* h3, const void* scores, int sc
     kernel<<<blocks, 256, smem, st>>>(static_cast<const uint4*>(h3), scores, scores_are_bf16, typed_ids,
                                       static_cast<const uint4*>(gamma), gain_center, eps, norm_is_bf16, static_cast<uint4*>(out),
                                       rstd_out, T, K, vec, static_cast<uint8_t*>(save_base), save_offset, save_cond, save_expect,
-                                      use_kahan ? 1 : 0, more...);
+                                      use_kahan ? 1 : 0, status, more...);
     return static_cast<int>(cudaGetLastError());
   };
   auto choose = [&](auto* typed_ids) {
@@ -419,6 +461,16 @@ extern "C" int dm_rmsnorm_combine_fwd(const void* h3, const void* scores, int sc
     return gamma ? with_norm(std::true_type{}) : with_norm(std::false_type{});
   };
   return ids_are_int64 ? choose(static_cast<const int64_t*>(ids)) : choose(static_cast<const int32_t*>(ids));
+}
+
+extern "C" int dm_rmsnorm_combine_fwd(const void* h3, const void* scores, int scores_are_bf16, const void* ids,
+                                      int ids_are_int64, const void* gamma, float gain_center, float eps,
+                                      int norm_is_bf16, int use_kahan, void* out, float* rstd_out, int64_t T, int K,
+                                      int64_t D, void* save_base, const int64_t* save_offset, const int* save_cond,
+                                      int save_expect, void* stream) {
+  return dm_rmsnorm_combine_fwd_status(h3, scores, scores_are_bf16, ids, ids_are_int64, gamma, gain_center, eps, norm_is_bf16,
+                                       use_kahan, out, rstd_out, T, K, D, save_base, save_offset, save_cond, save_expect, nullptr,
+                                       stream);
 }
 
 extern "C" int dm_rmsnorm_combine_bwd(const void* grad_out, const void* scores, int scores_are_bf16, const void* ids,

@@ -449,6 +449,11 @@ int dm_rmsnorm_combine_fwd(const void* h3, const void* scores, int scores_are_bf
                            int ids_are_int64, const void* gamma, float gain_center, float eps, int norm_is_bf16,
                            int use_kahan, void* out, float* rstd_out, int64_t T, int K, int64_t D, void* save_base,
                            const int64_t* save_offset, const int* save_cond, int save_expect, void* stream);
+/* The same; a wait for rows on their way to shared memory that ran out (the result does not suffer) is recorded in `status`. */
+int dm_rmsnorm_combine_fwd_status(const void* h3, const void* scores, int scores_are_bf16, const void* ids, int ids_are_int64,
+                                  const void* gamma, float gain_center, float eps, int norm_is_bf16, int use_kahan, void* out,
+                                  float* rstd_out, int64_t T, int K, int64_t D, void* save_base, const int64_t* save_offset,
+                                  const int* save_cond, int save_expect, int* status, void* stream);
 int dm_rmsnorm_combine_bwd(const void* grad_out, const void* scores, int scores_are_bf16, const void* ids,
                            int ids_are_int64, const void* h3_base, const int64_t* h3_offset, const float* rstd,
                            float eps, int norm_is_bf16, int use_kahan, void* grad_h3, float* grad_scores, int64_t T,

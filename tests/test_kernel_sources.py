@@ -36,3 +36,30 @@ def test_bulk_stores_are_waited_for_before_the_block_ends(name):
 
 def test_the_kernels_were_found():
     assert {"wgrad_gemm_kernel", "blockscaled_wide_kernel", "rows_gemm_kernel", "blockscaled_swapped_kernel"} <= set(KERNELS)
+
+
+@pytest.mark.parametrize("name", sorted(n for n, body in KERNELS.items() if "mbar_wait(" in body))
+def test_a_wait_that_runs_out_is_recorded(name):
+    """A kernel that may give up waiting says so."""
+    assert "set_status(" in KERNELS[name]
+
+
+def test_rows_fetched_by_hand_are_those_the_thread_reads():
+    """Where a bulk copy of a token's rows does not come in time, nothing lies between a thread's own fetch and its reads: the pieces
+    that it fetches, walked over as the kernel does, have to be the ones that it reads."""
+    body = KERNELS["rmsnorm_combine_fwd_staged_kernel"]
+    fetch = re.search(r"if \(!mbar_wait\([^\n]*\n(.*?)src\[(.*?)\] = ", body, re.S)
+    loops, index = re.findall(r"for \(int (\w+) = ([\w.]+); \w+ < (\w+); (?:\+\+\w+|\w+ \+= (\d+))\)", fetch[1]), fetch[2]
+    assert loops and index
+
+    def walk(todo, names):
+        if not todo:
+            return {eval(index, {}, names)}
+        (name, first, end, step), rest = todo[0], todo[1:]
+        first = names["thread"] if first == "threadIdx.x" else int(first)
+        return set().union(*(walk(rest, {**names, name: i}) for i in range(first, names[end], int(step or 1))))
+
+    for K, vec in [(1, 32), (4, 352), (3, 256), (8, 896), (5, 1)]:
+        for thread in (0, 1, 31, 255):
+            reads = {k * vec + v for k in range(K) for v in range(thread, vec, 256)}
+            assert walk(loops, {"K": K, "vec": vec, "rows": K * vec, "thread": thread}) == reads, (K, vec, thread)
