@@ -441,8 +441,12 @@ extern "C" int dm_rmsnorm_combine_fwd_status(const void* h3, const void* scores,
     using IdT = std::remove_const_t<std::remove_pointer_t<decltype(typed_ids)>>;
     const int64_t bytes = K * D * 2;
     if (bytes > kNormStaged) return run(rmsnorm_combine_fwd_kernel<IdT>, typed_ids, 8, 0);
-    const int buffers = 4 * bytes <= kNormStaged ? 2 : 1;  // two where two blocks of them fit on an SM
-    const int64_t fit = (kNormStaged + 4096) / (buffers * bytes + 4096);  // resident blocks; a block's tables take under 4 KiB
+    // Resident blocks with so many buffers each; a block's tables take under 4 KiB.  Two buffers only where two blocks of them fit: with
+    // one such block an SM (K x D from 27,137 to 27,648) 4,096 tokens of K = 4, D = 6912 took 85 us, with three blocks of one
+    // buffer 56; K = 6, D = 4608 101 | 63, K = 8, D = 3456 90 | 58.
+    auto resident = [&](int buffers) { return (kNormStaged + 4096) / (buffers * bytes + 4096); };
+    const int buffers = resident(2) >= 2 ? 2 : 1;
+    const int64_t fit = resident(buffers);
     auto staged = [&](auto gamma_tag, auto norm_tag, auto kahan_tag) {
       constexpr auto kernel =
           rmsnorm_combine_fwd_staged_kernel<IdT, decltype(gamma_tag)::value, decltype(norm_tag)::value, decltype(kahan_tag)::value>;

@@ -63,3 +63,25 @@ def test_rows_fetched_by_hand_are_those_the_thread_reads():
         for thread in (0, 1, 31, 255):
             reads = {k * vec + v for k in range(K) for v in range(thread, vec, 256)}
             assert walk(loops, {"K": K, "vec": vec, "rows": K * vec, "thread": thread}) == reads, (K, vec, thread)
+
+
+def test_two_buffers_only_where_two_blocks_of_them_fit():
+    """The rule of dm_rmsnorm_combine_fwd, evaluated from its own expressions for every K x D: a block per SM with two buffers leaves
+    the SM to a single block where three with one buffer would fit."""
+    text = (CSRC / "rmsnorm.cu").read_text()
+    text = text[text.index("auto choose ="):]
+
+    def python(source):
+        return re.sub(r"(.*) \? (\S+) : (\S+)", r"(\2 if \1 else \3)", source.replace("kNormStaged", "216 * 1024").replace(" / ", " // "))
+
+    buffers_rule = python(re.search(r"const int buffers = (.*?);", text)[1])
+    fit_rule = python(re.search(r"const int64_t fit = (.*?);", text)[1])
+    helper = re.search(r"auto resident = .*? return (.*?); \};", text)
+    for elements in range(8, 216 * 1024 // 2 + 1, 8):
+        names = {"bytes": 2 * elements}
+        if helper:
+            names["resident"] = lambda buffers: eval(python(helper[1]), {}, {"bytes": 2 * elements, "buffers": buffers})
+        names["buffers"] = eval(buffers_rule, {}, names)
+        fit = eval(fit_rule, {}, names)
+        assert fit >= names["buffers"], (elements, names["buffers"], fit)
+        assert fit * (names["buffers"] * 2 * elements + 4096) <= 227 * 1024 - 1024 + 4096 * (fit == 1)

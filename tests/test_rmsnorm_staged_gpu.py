@@ -63,3 +63,8 @@ def test_smallest_rows():
     want = (x * r[..., None] * scores.double()[..., None]).sum(1)
     assert torch.allclose(rstd.cpu().double(), r, rtol=1e-5)  # fp32 sum of eight squares and rsqrtf
     assert bool(((got.cpu().double() - want).abs() <= want.abs() * 2 ** -8 + 1e-5).all())  # one bf16 rounding of an fp32 sum
+
+
+@pytest.mark.parametrize("K,D", [(4, 6784), (4, 6792), (4, 6912), (4, 6920), (8, 3456)])
+def test_where_the_number_of_buffers_changes(K, D):
+    test_staged_rows_match_rows_in_memory(1500, K, D, torch.int64, torch.float32, False, False, False)
