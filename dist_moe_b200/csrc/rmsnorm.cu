@@ -175,8 +175,8 @@ __global__ void __launch_bounds__(256) rmsnorm_combine_fwd_kernel(
 // token's on its way while this one is worked on.  The kernel above has two loads of a thread in flight, reads every row twice and
 // looks at its options for every element (17 instructions each; issue-bound once the loads overlap: 41 us in the first example
 // below); here they are template parameters, and four rows are summed and reduced side by side.  One B200, us: T = 4096, K = 4, D =
-// 2816 61 -> 29; K = 8: D = 1024 53 -> 24, 4096 129 -> 62, 7168 235 -> 160 (one block per SM); T = 16, K = 4, D = 2816 8.4 -> 4.0.
-// Bound: HBM (92 MB in 29 us, 0.6 of the copy rate) and the three barriers of a token.  What the loop keeps for a copy that does not
+// 2816 59 -> 27; K = 8: D = 1024 57 -> 25, 3456 116 -> 54, 7168 229 -> 157 (one block per SM); T = 16, K = 4, D = 2816 5.5 -> 3.1.
+// Bound: HBM (92 MB in 27 us, 0.6 of the copy rate) and the three barriers of a token.  What the loop keeps for a copy that does not
 // come in time costs 0.3 us of the first example and under 0.1 at T = 16; asking all threads at a barrier (__syncthreads_or) cost
 // 2.0, copies by the threads that read them (cp.async), which need no such thing, 5.7.
 template <typename IdT, bool kGamma, bool kNorm16, bool kKahan>
@@ -440,10 +440,12 @@ extern "C" int dm_rmsnorm_combine_fwd_status(const void* h3, const void* scores,
   auto choose = [&](auto* typed_ids) {
     using IdT = std::remove_const_t<std::remove_pointer_t<decltype(typed_ids)>>;
     const int64_t bytes = K * D * 2;
-    if (bytes > kNormStaged) return run(rmsnorm_combine_fwd_kernel<IdT>, typed_ids, 8, 0);
+    // One short row has nothing to overlap with: 4,096 tokens of K = 1, rows in memory | staged, D = 256 9.9 | 12.0 us, 1024 11.0 | 13.4,
+    // 2048 15.3 | 16.4, 2816 20.8 | 18.9, 7168 39.1 | 31.1.  Two rows: D = 128 13.7 | 12.5, 1024 19.0 | 14.8.
+    if (bytes > kNormStaged || (K == 1 && D <= 2048)) return run(rmsnorm_combine_fwd_kernel<IdT>, typed_ids, 8, 0);
     // Resident blocks with so many buffers each; a block's tables take under 4 KiB.  Two buffers only where two blocks of them fit: with
     // one such block an SM (K x D from 27,137 to 27,648) 4,096 tokens of K = 4, D = 6912 took 85 us, with three blocks of one
-    // buffer 56; K = 6, D = 4608 101 | 63, K = 8, D = 3456 90 | 58.
+    // buffer 52; K = 6, D = 4608 101 | 59, K = 8, D = 3456 90 | 54.
     auto resident = [&](int buffers) { return (kNormStaged + 4096) / (buffers * bytes + 4096); };
     const int buffers = resident(2) >= 2 ? 2 : 1;
     const int64_t fit = resident(buffers);

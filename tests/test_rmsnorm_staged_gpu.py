@@ -68,3 +68,18 @@ def test_smallest_rows():
 @pytest.mark.parametrize("K,D", [(4, 6784), (4, 6792), (4, 6912), (4, 6920), (7, 3944)])
 def test_where_the_number_of_buffers_changes(K, D):
     test_staged_rows_match_rows_in_memory(1500, K, D, torch.int64, torch.float32, False, False, False)
+
+
+@pytest.mark.parametrize("T", [1, 2500])
+@pytest.mark.parametrize("D", [8, 2048, 2056])
+def test_a_single_row(T, D):
+    """One row: read from memory up to D = 2048, staged beyond; 32 of them, all but one left out, are staged."""
+    g = torch.Generator().manual_seed(T + D)
+    wide, scores = torch.randn(T, 32, D, generator=g).bfloat16().to(DEV), torch.rand(T, 32, generator=g).to(DEV)
+    ids = torch.full((T, 32), -1, dtype=torch.int64, device=DEV)
+    ids[1:, 0] = 0
+    want, want_rstd, _ = _run(wide, scores, ids, None, False, False, False)
+    own = [t[:, :1].contiguous() for t in (wide, scores, ids)]
+    got, got_rstd, kept = _run(*own, None, False, False, True)
+    assert torch.equal(got.view(torch.int16), want.view(torch.int16))
+    assert torch.equal(got_rstd, want_rstd[:, :1]) and torch.equal(kept, own[0])
