@@ -152,6 +152,12 @@ class ContextState:
         peak = [self.slot_bytes] * n + [self.arena_bytes - n * self.slot_bytes - self.reserved_scratch_bytes]
         self.peak_min_free.copy_(torch.tensor(peak, dtype=torch.int64))
         self.moe_layer_id.zero_()
+        self.clear_gather_flags()
+
+    def clear_gather_flags(self) -> None:
+        """The fused dispatch finds its counters clear and leaves them clear.  Launches that ran at the same time (calls on one
+        context have to be ordered) may have left some of them behind, and later ones would take rows for gathered that are not."""
+        self.gather_flags.zero_()
 
     def select_slot(self, slot: int, num_layers: int) -> None:
         if self.num_slots == 0:
@@ -176,6 +182,7 @@ class ContextState:
         words = self.status.tolist()
         if words[0] != 0:
             self.status.zero_()
+            self.clear_gather_flags()
             raise RuntimeError(
                 f"dist_moe_b200 device contract violation: {nat.STATUS_NAMES.get(words[0], words[0])} "
                 f"(details {words[1:4]})")
