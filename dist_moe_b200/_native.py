@@ -43,7 +43,7 @@ class LayerContext(ctypes.Structure):
         + [(n, c_int64) for n in ("T_max", "D", "F", "slot_bytes", "capacity_rows")]
         + [("barrier_timeout_ns", c_uint64)]
         + [(n, c_int) for n in ("rank", "ep", "K", "E", "e_local", "num_slots", "num_sms", "clamped")]
-        + [("alpha", c_float), ("limit", c_float), ("storage", c_int * 6)]
+        + [("alpha", c_float), ("limit", c_float), ("storage", c_int * 6), ("gather_flags_kept_clear", c_int)]
     )
 
 

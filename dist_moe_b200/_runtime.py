@@ -267,7 +267,7 @@ class ContextState:
             c.T_max, c.D, c.F = cfg.max_num_local_input_tokens, cfg.hidden_dim, cfg.intermediate_dim
             c.slot_bytes, c.capacity_rows = self.slot_bytes, self.capacity_rows
             c.rank, c.ep, c.K, c.E, c.e_local = self.rank, self.ep, cfg.top_k, cfg.num_experts, self.e_local
-            c.num_slots, c.num_sms = self.num_slots, self.num_sms | nat.GATHER_FLAGS_KEPT_CLEAR
+            c.num_slots, c.num_sms, c.gather_flags_kept_clear = self.num_slots, self.num_sms, 1
             c.clamped, c.alpha, c.limit = cfg.activation == "swiglu_clamped", cfg.swiglu_alpha, cfg.swiglu_limit
             if cfg.block_scaled is not None:
                 from ._blockscaled import planner_storage

@@ -653,8 +653,9 @@ static int rows_setup(RowsParams& p, const dm_operand& a, const dm_operand& c, c
 // Takes DM_GATHER_FLAGS_KEPT_CLEAR out of num_sms; without it the flags are cleared in front of the launch.
 static int clear_flags(RowsParams& p, int64_t max_rows, int& num_sms, cudaStream_t st) {
   if (p.gather_flags == nullptr) return kRcOk;
-  if (num_sms > 0 && (num_sms & DM_GATHER_FLAGS_KEPT_CLEAR) != 0) {
-    num_sms &= ~DM_GATHER_FLAGS_KEPT_CLEAR;
+  static_assert(DM_GATHER_FLAGS_KEPT_CLEAR == kRwKeptClear, "the header's mark");
+  if (rw_flags_kept_clear(num_sms)) {
+    num_sms &= 0xffff;
     p.gather_done = p.gather_ticket + 1;
     return kRcOk;
   }

@@ -21,6 +21,11 @@ DM_HOST_DEVICE constexpr int rw_gather_unit_rows(int total_rows, int warps) {
   return total_rows <= warps ? 1 : total_rows <= 2 * warps ? 2 : total_rows <= 4 * warps ? 4 : 8;
 }
 
+// Whether a dispatch GEMM's `num_sms` says that its flags are kept clear: the mark with a bound on the SMs of up to 16 bits, zero for
+// none.  Larger numbers are bounds and nothing else, as they are to the other GEMMs (all of the device).
+constexpr int kRwKeptClear = 1 << 30;
+DM_HOST_DEVICE constexpr bool rw_flags_kept_clear(int num_sms) { return (num_sms & ~0xffff) == kRwKeptClear; }
+
 // A CTA of the pair loads half of a tile's rows.
 DM_HOST_DEVICE constexpr int rw_box_rows(int i) { return i == 0 ? 16 : 32 * i; }
 DM_HOST_DEVICE constexpr int rw_box_index(int n) { return n <= 32 ? 0 : (n + 63) >> 6; }

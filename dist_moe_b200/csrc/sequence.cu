@@ -31,7 +31,11 @@ struct Sequence {
     if (c.ep > 1)
       step(bit, 1, [&] { return dm_barrier(pads, c.rank, c.ep, 0, cond, c.barrier_timeout_ns, c.status, stream); });
   }
-  int sms() const { return c.num_sms > 0 ? c.num_sms & ~DM_GATHER_FLAGS_KEPT_CLEAR : c.num_sms; }
+  // num_sms of a dispatch GEMM
+  int dispatch_sms() const {
+    if (!c.gather_flags_kept_clear) return c.num_sms;
+    return DM_GATHER_FLAGS_KEPT_CLEAR | (c.num_sms < 0 ? 0 : c.num_sms > 0xffff ? 0xffff : c.num_sms);
+  }
   dm_operand arena(const int64_t* offset) const { return dm_operand{c.arena, c.arena_bytes, offset}; }
 };
 
@@ -79,12 +83,12 @@ extern "C" int dm_bf16_forward(const dm_layer_context* ctx, const dm_layer_call*
     const dm_operand h2 = k.fuse_swiglu ? s.arena(fs + 3) : kNone;
     if (!k.separate_gather)
       return dm_gemm_fprop_dispatch(k.fwd_ptrs, c.gather_flags, xg, k.w13, h1, h2, k.expert_offsets, c.e_local, k.max_rows,
-                                    2 * c.F, c.D, k.fuse_swiglu, c.clamped, c.alpha, c.limit, nullptr, c.num_sms, c.status,
+                                    2 * c.F, c.D, k.fuse_swiglu, c.clamped, c.alpha, c.limit, nullptr, s.dispatch_sms(), c.status,
                                     stream);
     const int rc = dm_gather_rows(k.fwd_ptrs, recv, c.arena, fs + 1, stride, k.max_rows, nullptr, stream);
     if (rc != 0) return rc;
     return dm_gemm_fprop(xg, k.w13, h1, h2, nullptr, k.expert_offsets, c.e_local, k.max_rows, 2 * c.F, c.D, k.fuse_swiglu,
-                         c.clamped, c.alpha, c.limit, nullptr, s.sms(), c.status, stream);
+                         c.clamped, c.alpha, c.limit, nullptr, c.num_sms, c.status, stream);
   });
   if (!k.fuse_swiglu)
     s.step(DM_FWD_SWIGLU, 1, [&] {
@@ -93,7 +97,7 @@ extern "C" int dm_bf16_forward(const dm_layer_context* ctx, const dm_layer_call*
     });
   s.step(DM_FWD_W2, 1, [&] {
     return dm_gemm_fprop(s.arena(fs + 3), k.w2, kNone, kNone, k.sct_ptrs, k.expert_offsets, c.e_local, k.max_rows, c.D, c.F, 0,
-                         0, 1.0f, 0.0f, nullptr, s.sms(), c.status, stream);
+                         0, 1.0f, 0.0f, nullptr, c.num_sms, c.status, stream);
   });
   s.barrier(DM_FWD_COMBINE, c.combine_pads, nullptr);
   s.step(DM_FWD_REDUCE, 1, [&] {
@@ -126,12 +130,12 @@ extern "C" int dm_bf16_backward(const dm_layer_context* ctx, const dm_layer_call
   s.step(DM_BWD_W13_AGAIN, k.separate_gather ? 2 : 1, [&] {
     if (!k.separate_gather)
       return dm_gemm_fprop_dispatch(k.fwd_ptrs, c.gather_flags, s.arena(bo), k.w13, s.arena(bo + 1), kNone, k.expert_offsets,
-                                    c.e_local, k.max_rows, 2 * c.F, c.D, 0, c.clamped, c.alpha, c.limit, k.cond, c.num_sms,
+                                    c.e_local, k.max_rows, 2 * c.F, c.D, 0, c.clamped, c.alpha, c.limit, k.cond, s.dispatch_sms(),
                                     c.status, stream);
     const int rc = dm_gather_rows(k.fwd_ptrs, recv, c.arena, bo, stride, k.max_rows, k.cond, stream);
     if (rc != 0) return rc;
     return dm_gemm_fprop(s.arena(bo), k.w13, s.arena(bo + 1), kNone, nullptr, k.expert_offsets, c.e_local, k.max_rows, 2 * c.F,
-                         c.D, 0, c.clamped, c.alpha, c.limit, k.cond, s.sms(), c.status, stream);
+                         c.D, 0, c.clamped, c.alpha, c.limit, k.cond, c.num_sms, c.status, stream);
   });
   // h2 is always rebuilt from h1: only x_gathered, h1 and h3 are ever saved
   s.step(DM_BWD_SWIGLU_AGAIN, 1, [&] {
@@ -140,7 +144,7 @@ extern "C" int dm_bf16_backward(const dm_layer_context* ctx, const dm_layer_call
   });
   s.step(DM_BWD_W2_AGAIN, 1, [&] {
     return dm_gemm_fprop(s.arena(bo + 2), k.w2, kNone, kNone, k.sct_ptrs, k.expert_offsets, c.e_local, k.max_rows, c.D, c.F, 0,
-                         0, 1.0f, 0.0f, k.cond, s.sms(), c.status, stream);
+                         0, 1.0f, 0.0f, k.cond, c.num_sms, c.status, stream);
   });
   s.barrier(DM_BWD_W2_AGAIN, c.combine_pads, k.cond);
   s.step(DM_BWD_LOAD_H3, 1, [&] {
@@ -160,15 +164,15 @@ extern "C" int dm_bf16_backward(const dm_layer_context* ctx, const dm_layer_call
   s.step(DM_BWD_W2_DGRAD, k.separate_gather ? 2 : 1, [&] {
     if (!k.separate_gather)
       return dm_gemm_dgrad_dispatch(k.sct_ptrs, c.gather_flags, s.arena(bo + 4), k.w2, s.arena(bo + 3), k.expert_offsets,
-                                    c.e_local, k.max_rows, c.F, c.D, nullptr, c.num_sms, c.status, stream);
+                                    c.e_local, k.max_rows, c.F, c.D, nullptr, s.dispatch_sms(), c.status, stream);
     const int rc = dm_gather_rows(k.sct_ptrs, recv, c.arena, bo + 4, stride, k.max_rows, nullptr, stream);
     if (rc != 0) return rc;
     return dm_gemm_dgrad(s.arena(bo + 4), k.w2, s.arena(bo + 3), nullptr, k.expert_offsets, c.e_local, k.max_rows, c.F, c.D,
-                         nullptr, s.sms(), c.status, stream);
+                         nullptr, c.num_sms, c.status, stream);
   });
   s.step(DM_BWD_W2_WGRAD, 1, [&] {
     return dm_gemm_wgrad(s.arena(bo + 4), s.arena(bo + 2), k.dw2, k.dw2_is_fp32, k.dw2_accumulate, k.expert_offsets, c.e_local,
-                         k.max_rows, c.D, c.F, s.sms(), c.status, stream);
+                         k.max_rows, c.D, c.F, c.num_sms, c.status, stream);
   });
   // ---- SwiGLU backward, W13 input gradient (scattered to the owners) and weight gradient -----------------------------
   s.step(DM_BWD_SWIGLU, 1, [&] {
@@ -177,11 +181,11 @@ extern "C" int dm_bf16_backward(const dm_layer_context* ctx, const dm_layer_call
   });
   s.step(DM_BWD_W13_DGRAD, 1, [&] {
     return dm_gemm_dgrad(s.arena(bo + 5), k.w13, kNone, k.bwd_ptrs, k.expert_offsets, c.e_local, k.max_rows, c.D, 2 * c.F,
-                         nullptr, s.sms(), c.status, stream);
+                         nullptr, c.num_sms, c.status, stream);
   });
   s.step(DM_BWD_W13_WGRAD, 1, [&] {
     return dm_gemm_wgrad(s.arena(bo + 5), s.arena(bo), k.dw13, k.dw13_is_fp32, k.dw13_accumulate, k.expert_offsets, c.e_local,
-                         k.max_rows, 2 * c.F, c.D, s.sms(), c.status, stream);
+                         k.max_rows, 2 * c.F, c.D, c.num_sms, c.status, stream);
   });
   // The closing barrier is unconditional (dist_moe/api.py:2580): peers may still be pulling grad_h3 out of this rank's
   // combine buffer, and the next call on this context overwrites it.
@@ -235,7 +239,7 @@ extern "C" int dm_mxfp8_forward(const dm_layer_context* ctx, const dm_layer_call
   s.step(DM_FWD_W13, 1, [&] {
     return dm_gemm_blockscaled_counted(0, s.arena(at(ft, 0, kAQ)), s.arena(at(ft, 0, kASf)), k.w13, k.w13_sf,
                                        s.arena(at(ft, 0, kC)), kNone, nullptr, kNone, nullptr, k.expert_offsets, k.real_counts,
-                                       c.e_local, k.max_rows, 2 * c.F, c.D, 0, 0, 1.0f, 0.0f, nullptr, s.sms(), c.status,
+                                       c.e_local, k.max_rows, 2 * c.F, c.D, 0, 0, 1.0f, 0.0f, nullptr, c.num_sms, c.status,
                                        stream);
   });
   s.step(DM_FWD_SWIGLU, 1, [&] {
@@ -246,7 +250,7 @@ extern "C" int dm_mxfp8_forward(const dm_layer_context* ctx, const dm_layer_call
   s.step(DM_FWD_W2, 1, [&] {
     return dm_gemm_blockscaled_counted(0, s.arena(at(ft, 1, kAQ)), s.arena(at(ft, 1, kASf)), k.w2, k.w2_sf, kNone, kNone,
                                        k.sct_ptrs, kNone, nullptr, k.expert_offsets, k.real_counts, c.e_local, k.max_rows, c.D,
-                                       c.F, 0, 0, 1.0f, 0.0f, nullptr, s.sms(), c.status, stream);
+                                       c.F, 0, 0, 1.0f, 0.0f, nullptr, c.num_sms, c.status, stream);
   });
   s.barrier(DM_FWD_COMBINE, c.combine_pads, nullptr);
   // the expert outputs go to the slot (when the layer is saved) only if the score gradient will read them
@@ -286,7 +290,7 @@ extern "C" int dm_mxfp8_backward(const dm_layer_context* ctx, const dm_layer_cal
   s.step(DM_BWD_W13_AGAIN, 1, [&] {
     return dm_gemm_blockscaled_counted(0, A(0, kAQ), A(0, kASf), k.w13, k.w13_sf, A(0, kC), kNone, nullptr, kNone, nullptr,
                                        k.expert_offsets, k.real_counts, c.e_local, k.max_rows, 2 * c.F, c.D, 0, 0, 1.0f, 0.0f,
-                                       k.cond, s.sms(), c.status, stream);
+                                       k.cond, c.num_sms, c.status, stream);
   });
   s.step(DM_BWD_SWIGLU_AGAIN, 1, [&] {
     return dm_swiglu_fwd_quant_mxfp8_rowcol_at(A(1, kSrcX), recv, k.max_rows, c.F, c.clamped, c.alpha, c.limit, A(1, kAQ),
@@ -295,7 +299,7 @@ extern "C" int dm_mxfp8_backward(const dm_layer_context* ctx, const dm_layer_cal
   s.step(DM_BWD_W2_AGAIN, 1, [&] {  // the expert outputs again, scattered to their owners' combine buffers
     return dm_gemm_blockscaled_counted(0, A(1, kAQ), A(1, kASf), k.w2, k.w2_sf, kNone, kNone, k.sct_ptrs, kNone, nullptr,
                                        k.expert_offsets, k.real_counts, c.e_local, k.max_rows, c.D, c.F, 0, 0, 1.0f, 0.0f,
-                                       k.cond, s.sms(), c.status, stream);
+                                       k.cond, c.num_sms, c.status, stream);
   });
   s.barrier(DM_BWD_W2_AGAIN, c.combine_pads, k.cond);
   s.step(DM_BWD_LOAD_H3, 1, [&] {
@@ -317,13 +321,13 @@ extern "C" int dm_mxfp8_backward(const dm_layer_context* ctx, const dm_layer_cal
   });
   s.step(DM_BWD_W2_DGRAD, 1, [&] {
     return dm_gemm_blockscaled_dgrad_counted(A(2, kAQ), A(2, kASf), k.w2, k.w2_dgrad_sf, A(2, kC), nullptr, k.expert_offsets,
-                                             k.real_counts, c.e_local, k.max_rows, c.F, c.D, nullptr, s.sms(), c.status,
+                                             k.real_counts, c.e_local, k.max_rows, c.F, c.D, nullptr, c.num_sms, c.status,
                                              stream);
   });
   s.step(DM_BWD_W2_WGRAD, 1, [&] {
     return dm_gemm_blockscaled_wgrad_compact(A(3, kAQ), A(3, kASf), A(3, kBQ), A(3, kBSf), k.dw2, k.dw2_is_fp32,
                                              k.dw2_accumulate, k.expert_offsets, c.e_local, k.max_rows, c.D, c.F, nullptr,
-                                             s.sms(), c.status, stream);
+                                             c.num_sms, c.status, stream);
   });
   // ---- SwiGLU backward, W13 -----------------------------------------------------------------------------------------
   s.step(DM_BWD_SWIGLU, 1, [&] {
@@ -333,13 +337,13 @@ extern "C" int dm_mxfp8_backward(const dm_layer_context* ctx, const dm_layer_cal
   });
   s.step(DM_BWD_W13_DGRAD, 1, [&] {
     return dm_gemm_blockscaled_dgrad_counted(A(4, kAQ), A(4, kASf), k.w13, k.w13_dgrad_sf, kNone, k.bwd_ptrs, k.expert_offsets,
-                                             k.real_counts, c.e_local, k.max_rows, c.D, 2 * c.F, nullptr, s.sms(), c.status,
+                                             k.real_counts, c.e_local, k.max_rows, c.D, 2 * c.F, nullptr, c.num_sms, c.status,
                                              stream);
   });
   s.step(DM_BWD_W13_WGRAD, 1, [&] {
     return dm_gemm_blockscaled_wgrad_compact(A(5, kAQ), A(5, kASf), A(5, kBQ), A(5, kBSf), k.dw13, k.dw13_is_fp32,
                                              k.dw13_accumulate, k.expert_offsets, c.e_local, k.max_rows, 2 * c.F, c.D, nullptr,
-                                             s.sms(), c.status, stream);
+                                             c.num_sms, c.status, stream);
   });
   // unconditional, as in the reference (dist_moe/api.py:2580): peers may still be reading this rank's combine buffer
   s.barrier(DM_BWD_CLOSE, c.dispatch_pads, nullptr);

@@ -307,9 +307,9 @@ int dm_gemm_dgrad(dm_operand a, const void* w, dm_operand c, const int64_t* scat
  * allowed) by four extra warps of every CTA of the persistent kernel while the tensor cores already work
  * on the rows that have landed; `a` names where the pulled rows are kept (x_gathered / grad_h3_gathered,
  * needed again by the weight-gradient GEMMs).  gather_flags: int32[max_rows/128 + 2] scratch, cleared by
- * the call; it belongs to this launch until it has finished.  With DM_GATHER_FLAGS_KEPT_CLEAR or'ed into num_sms (here, or
- * in a dm_layer_context) the call finds int32[max_rows/128 + 3] cleared and leaves them cleared, without a launch for it:
- * for a scratch that nothing else writes.  Rows are pulled only by CTAs that are running, so
+ * the call; it belongs to this launch until it has finished.  With DM_GATHER_FLAGS_KEPT_CLEAR or'ed into a num_sms
+ * of 0 to 65,535 the call finds int32[max_rows/128 + 3] cleared and leaves them cleared, without a launch for it: for a
+ * scratch that nothing else writes, by launches that run one after another.  Any other num_sms is a bound only.  Rows are pulled only by CTAs that are running, so
  * kernels of other streams that hold SMs delay the call but do not fail it.  Replaces
  * dist_grouped_gemm_fprop_dispatch / ..._dgrad_dispatch in one launch
  * (dist_moe/kernels/dist_grouped_gemm.py:1148-1237, 1441-1489). */
@@ -605,6 +605,7 @@ typedef struct { /* what a context keeps between calls */
   int rank, ep, K, E, e_local, num_slots, num_sms, clamped;
   float alpha, limit;
   int storage[6]; /* MXFP8: bundle geometry, as dm_plan_fwd_blockscaled takes it */
+  int gather_flags_kept_clear; /* nothing but these calls, one after another, writes gather_flags, which were clear at first */
 } dm_layer_context;
 
 typedef struct {
