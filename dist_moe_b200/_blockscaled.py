@@ -35,6 +35,7 @@ NVFP4 has no backward (dist_moe/_blockscaled.py:245-321).
 
 from __future__ import annotations
 
+import math
 from typing import Any
 
 import torch
@@ -267,10 +268,28 @@ def _workspace(state):
 SWAPPED_MAX_ROWS_PER_EXPERT = None
 _SWAPPED_MAX_ROWS = {BlockScaledFormat.NVFP4: 48, BlockScaledFormat.MXFP8_E4M3: 0}
 
-# NVFP4 calls whose experts receive at least this many rows on average run on CTA pairs (256 x 256 tiles): 32 experts x 7168 x
-# 2048, 128 x 256 tiles / pairs, us a layer under the power cap: 64 rows 223 / 243, 128 272 / 272, 256 370 / 377, 512 609 / 597,
-# 2048 1984 / 1907.
+# NVFP4 products with at least this many rows per expert on average may run on CTA pairs (256 x 256 tiles, `_on_pairs`).
 _PAIR_MIN_ROWS = 512
+
+
+def _on_pairs(routes: int, experts: int, n: int, kd: int, swiglu: bool, num_sms: int) -> bool:
+    """Whether a NVFP4 product of ``routes`` rows with ``experts`` weights of ``n`` x ``kd`` runs on CTA pairs.
+
+    A pair's tile is two of the other kernel's and takes 0.85 of the time of one of those on either CTA, but a group's rows fill tiles
+    of 256 less well than of 128, and its rounds count: the estimate below compares them (a group is taken to fill all but 0.45 of its
+    last tile).  Without SwiGLU the hand-over of the one accumulator, 2000 cycles, wants more than eight stages of K (2048).
+    One B200, us, 128 x 256 tiles | pairs, rows per expert on average.  SwiGLU: 32 experts x 7168 x 2048, 512 239 | 231, 2048 807 | 745;
+    32 x 2048 x 768, 512 61 | 55, 2048 174 | 146; 8 x 7168 x 1024, 512 (two rounds | three) 41 | 48, 768 53 | 49, 2048 115 | 103; 16 x
+    7168 x 768, 512 (3 | 4) 57 | 61, 768 83 | 73; 8 x 2048 x 768, 512 (2 | 2) 22 | 20.  Without: K = 768 to 7168 wide, 2048 rows, 170 |
+    240; 1024 112 | 147; 1536 273 | 305; 2048 565 | 569 and 164 | 170; 2304 103 | 94; 4096 78 | 66; 7168 444 | 368."""
+    if routes < _PAIR_MIN_ROWS * experts or not (swiglu or kd > 2048):
+        return False
+    rows, columns, ctas = routes / experts, -(-n // 256), min(num_sms or 148, 148)
+
+    def rounds(tile_rows: int, workers: int) -> int:
+        return math.ceil(experts * (rows / tile_rows + 0.45) * columns / workers)
+
+    return 0.85 * rounds(256, max(1, ctas // 2)) <= rounds(128, ctas)
 
 
 def _gemm_pairs(_format, *arguments):
@@ -359,10 +378,11 @@ def run_block_scaled(x, ids, scores, w13_weight, w2_weight, context: Any, option
     # few rows per expert (decode): weights on the MMA's M side, the rows on its N side
     limit_rows = _SWAPPED_MAX_ROWS[fmt] if SWAPPED_MAX_ROWS_PER_EXPERT is None else SWAPPED_MAX_ROWS_PER_EXPERT
     swapped = fused and ep * T * K <= limit_rows * E
-    gemm = _gemm_pairs if lay.fp4 and ep * T * K >= _PAIR_MIN_ROWS * E else _gemm
+    gemm13, gemm2 = (_gemm_pairs if lay.fp4 and _on_pairs(T * K, el, n, kd, swiglu, state.num_sms) else _gemm
+                     for n, kd, swiglu in ((2 * F, D, fused), (D, F, False)))
     # ---- gather + unpack: rows that pad a group are left alone where the GEMMs know the real ones ------------------
     none = nat.Operand(None, 0, None)
-    counted = swapped or gemm is _gemm_pairs or not lay.fp4
+    counted = swapped or gemm13 is _gemm_pairs or not lay.fp4
     gather = nat.lib.dm_gather_packed_rows_live if counted and fused else nat.lib.dm_gather_packed_rows
     nat.check(gather(fwd.data_ptr(), recv.data_ptr(), max_rows, xq, xs, int(lay.fp4), _view(buf, lay.x_q),
                      _view(buf, lay.x_sf), _view(buf, lay.x_inv) if lay.fp4 else none, None, st), "dm_gather_packed_rows")
@@ -388,16 +408,16 @@ def run_block_scaled(x, ids, scores, w13_weight, w2_weight, context: Any, option
                                      None, state.num_sms, status, st), "dm_gemm_blockscaled_swiglu_mxfp8")
     elif fused:
         h2_dense = lay.dense
-        nat.check(gemm(f, _view(buf, lay.x_q), _view(buf, lay.x_sf), p13.fprop_data.data_ptr(),
-                       p13.fprop_scale.data_ptr(), none, _view(buf, h2_dense), None, row_inv,
-                       nat.ptr(p13.global_scale_inv), offsets.data_ptr(), real.data_ptr(), el, max_rows, 2 * F, D, 1,
-                       clamped, alpha, limit, None, state.num_sms, status, st), "dm_gemm_blockscaled(w13+swiglu)")
+        nat.check(gemm13(f, _view(buf, lay.x_q), _view(buf, lay.x_sf), p13.fprop_data.data_ptr(),
+                         p13.fprop_scale.data_ptr(), none, _view(buf, h2_dense), None, row_inv,
+                         nat.ptr(p13.global_scale_inv), offsets.data_ptr(), real.data_ptr(), el, max_rows, 2 * F, D, 1,
+                         clamped, alpha, limit, None, state.num_sms, status, st), "dm_gemm_blockscaled(w13+swiglu)")
     else:
         h2_dense = lay.h2_dense
-        nat.check(gemm(f, _view(buf, lay.x_q), _view(buf, lay.x_sf), p13.fprop_data.data_ptr(),
-                       p13.fprop_scale.data_ptr(), _view(buf, lay.dense), none, None, row_inv,
-                       nat.ptr(p13.global_scale_inv), offsets.data_ptr(), real.data_ptr(), el, max_rows, 2 * F, D, 0,
-                       0, 1.0, 0.0, None, state.num_sms, status, st), "dm_gemm_blockscaled(w13)")
+        nat.check(gemm13(f, _view(buf, lay.x_q), _view(buf, lay.x_sf), p13.fprop_data.data_ptr(),
+                         p13.fprop_scale.data_ptr(), _view(buf, lay.dense), none, None, row_inv,
+                         nat.ptr(p13.global_scale_inv), offsets.data_ptr(), real.data_ptr(), el, max_rows, 2 * F, D, 0,
+                         0, 1.0, 0.0, None, state.num_sms, status, st), "dm_gemm_blockscaled(w13)")
         nat.check(nat.lib.dm_swiglu_fwd(buf.data_ptr() + lay.dense, None, buf.data_ptr() + h2_dense, None,
                                         recv.data_ptr(), max_rows, F, clamped, alpha, limit, None, 0.0, None, st),
                   "dm_swiglu_fwd")
@@ -423,10 +443,10 @@ def run_block_scaled(x, ids, scores, w13_weight, w2_weight, context: Any, option
                                                       real.data_ptr(), el, max_rows, D, F, 0, 0, 1.0, 0.0, None,
                                                       state.num_sms, status, st), "dm_gemm_blockscaled_swapped(w2)")
     else:
-        nat.check(gemm(f, _view(buf, lay.h_q), _view(buf, lay.h_sf), p2.fprop_data.data_ptr(),
-                       p2.fprop_scale.data_ptr(), none, none, sct.data_ptr(),
-                       _view(buf, lay.h_inv) if lay.fp4 else none, nat.ptr(p2.global_scale_inv), offsets.data_ptr(),
-                       real.data_ptr(), el, max_rows, D, F, 0, 0, 1.0, 0.0, None, state.num_sms, status, st),
+        nat.check(gemm2(f, _view(buf, lay.h_q), _view(buf, lay.h_sf), p2.fprop_data.data_ptr(),
+                        p2.fprop_scale.data_ptr(), none, none, sct.data_ptr(),
+                        _view(buf, lay.h_inv) if lay.fp4 else none, nat.ptr(p2.global_scale_inv), offsets.data_ptr(),
+                        real.data_ptr(), el, max_rows, D, F, 0, 0, 1.0, 0.0, None, state.num_sms, status, st),
                   "dm_gemm_blockscaled(w2)")
     state.barrier(state.combine)
     out = torch.empty(T, D, dtype=torch.bfloat16, device=dev)

@@ -444,10 +444,10 @@ __global__ void __launch_bounds__(kN4Threads, 1) nvfp4_wide_kernel(const __grid_
 // its own rows' and all columns').  Five stages fit next to staging tiles for sixteen epilogue warps of 64 columns each:
 // with eight of 128 the latency of their arithmetic held the SwiGLU form back (8 stages of K: 13 us a tile, now 6).  Rows past
 // an expert's count are left out: a CTA without rows loads its peer's and stores nothing.
-// One B200, 32 experts x 7168 x 2048, 2048 rows each, W13 / W2: 804 / 567 -> 745 / 541 us, under the power cap 1984 -> 1907 us
-// a layer.  Bound: operand loads (without the epilogue 684 / 389 us, without the loads of A and B 596 / 388) and the hand-over of
-// the one accumulator, about 2000 cycles a tile; a second one does not fit next to the scales.  16 rows x 128 bytes per store
-// instead of 32 x 64 took W2 to 571.
+// One B200, 32 experts x 7168 x 2048, 2048 rows each: W13 with SwiGLU 807 -> 745 us; the plain form takes 569 us for W2 (K = 2048)
+// where the kernel above takes 565, and wins from there on (K = 4096, 8 experts: 78 -> 66).  Bound: operand loads (W13 without the
+// epilogue 684 us, without the loads of A and B 596) and the hand-over of the one accumulator, about 2000 cycles a tile; a second
+// one does not fit next to the scales.  16 rows x 128 bytes per store instead of 32 x 64 cost W2 another 30 us.
 constexpr int kN4PairEpilogue = 16;   // epilogue warps
 constexpr int kN4PairThreads = (3 + kN4PairEpilogue) * 32;  // and TMA warp, MMA warp, accumulator watcher
 constexpr uint32_t kN4PairBBytes = 128 * 128;  // a CTA loads half of the tile's weight columns
