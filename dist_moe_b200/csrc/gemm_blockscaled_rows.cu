@@ -182,11 +182,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kBrThreads, 1)
   // Ring: stages as large as the launch's largest tile needs, as many as shared memory and the scale columns allow.
   const int n_max = 2 * rw_box_rows(uniform(s_box));
   const uint32_t x_groups = bs_tile_atoms(n_max);
-  // One B200, 128 experts x 2816, W13 with SwiGLU / W2, us: 16 tokens on few experts 113.6 / 63.4 -> 115.0 / 60.1 (layer 205.8 -> 201.6),
-  // 4 rows per expert on average 323.2 / 169.2 -> 312.4 / 170.2, 16 324.6 / 176.0 -> 324.0 / 176.6.  From tiles of 64 rows up the
-  // epilogues want all pairs: 32 rows on average 343 / 171 -> 346 / 172, 64 361 / 175 -> 371 / 174, 96 388 / 181 -> 397 / 178.
+  // One B200, 2816 x 2816, all pairs | even rounds, us.  W13 with SwiGLU: 16 tokens on 47 of 128 experts 118.5 | 115.7, 4 rows per
+  // expert on average 326.5 | 325.8, 16 327.5 | 327.9; 154 tiles (three rounds, the last with 6) 33.1 | 32.0, 242 43.0 | 40.3, but 132 (two,
+  // the last with 58 of 74) 27.7 | 29.0, 198 34.8 | 36.0, 144 of 2048 x 768 25.5 | 26.4.  W2: 62.2 | 59.7, 169.5 | 166.5, 175.6 | 174.0; 66 to
+  // 418 tiles 0.5 to 12 % less, 132 24.4 | 24.0, 198 32.2 | 30.9.  From tiles of 64 rows up the epilogues want all pairs: 32 rows on
+  // average 343 / 171 | 346 / 172, 64 361 / 175 | 371 / 174, 96 388 / 181 | 397 / 178.
   const int pair = blockIdx.x >> 1;
-  const int tile_step = balanced_pairs(total_tiles, gridDim.x >> 1, n_max, 32);
+  const int tile_step = balanced_pairs(total_tiles, gridDim.x >> 1, n_max, 32, kSwiglu);
   const int first_tile = pair < tile_step ? pair : total_tiles;
   // Scale columns of a stage slot: an atom of the weights and those of the rows, at a stride of 8 or 16.  With slots of twelve, all
   // that two atoms of rows need, the four forward and input-gradient launches of a training layer took 0.9 to 1.6 % longer.

@@ -299,14 +299,6 @@ __device__ __forceinline__ void tcgen05_commit_pair(uint32_t bar_addr) {
       : "memory");
 }
 
-// Pairs that take tiles where tiles are short of rows and the launch streams weights: as few as need the rounds that all of them
-// would need.  A last round with a part of the pairs has too few loads in flight for HBM; with these all rounds are alike, and the
-// pairs that are left out were not missed.  `rows` is the launch's largest tile, `limit` the kernel's line, `workers` all pairs.
-__device__ __forceinline__ int balanced_pairs(int tiles, int workers, int rows, int limit) {
-  const int rounds = (tiles + workers - 1) / workers;
-  return rows <= limit && rounds > 1 ? (tiles + rounds - 1) / rounds : workers;
-}
-
 // Bulk tensor store and reduce-add of one staged box (shared memory -> global), issued by one thread.  The
 // staged bytes must have been made visible to the async proxy (fence_proxy_async_smem by every writer, then
 // a barrier) and stay untouched until bulk_wait_read has returned.

@@ -73,6 +73,18 @@ DM_HOST_DEVICE RowsBlocks rw_tile_blocks(const RowsTile& t, int total_rows) {
   return b;
 }
 
+// Pairs that take tiles where tiles are short of rows and the launch streams weights: as few as need the rounds that all of them
+// would need.  A last round with a part of the pairs has too few loads in flight for HBM; with these all rounds are alike, and the
+// pairs that are left out were not missed.  `rows` is the launch's largest tile, `limit` the kernel's line, `workers` all pairs.
+// `heavy`: where the epilogue counts (SwiGLU and quantisation), two or three rounds stay as they are if the last one has more
+// than half of the pairs.
+DM_HOST_DEVICE constexpr int balanced_pairs(int tiles, int workers, int rows, int limit, bool heavy = false) {
+  const int rounds = (tiles + workers - 1) / workers;
+  if (rows > limit || rounds <= 1) return workers;
+  if (heavy && rounds <= 3 && 2 * (tiles - (rounds - 1) * workers) > workers) return workers;
+  return (tiles + rounds - 1) / rounds;
+}
+
 // Rows of the group [off, next) that a block-scaled GEMM works on, `count` of them real.  None where the group does not
 // start on a scale atom of 128 rows: the caller has broken the padding rule, and the MMA would take the rows' scales from an
 // odd TMEM column, which is a misaligned address.

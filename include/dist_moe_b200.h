@@ -362,8 +362,8 @@ int dm_gemm_blockscaled_counted(int format, dm_operand a, dm_operand sfa, const 
                                 int swiglu_interleaved, int clamped, float alpha, float limit, const int* cond,
                                 int num_sms, int* status, void* stream);
 
-/* dm_gemm_blockscaled_counted for NVFP4 experts that received many rows (without SwiGLU: and Kd beyond 2048): pairs of neighbouring SMs work on 256 x 256 tiles.
- * Same arguments without the format.  With counts h2, an h1 next to it and scattered rows past them are not written; a dense C
+/* dm_gemm_blockscaled_counted for NVFP4 experts that received many rows (without SwiGLU: and Kd beyond 2048): pairs of
+ * neighbouring SMs work on 256 x 256 tiles.  Same arguments without the format.  With counts h2, an h1 next to it and scattered rows past them are not written; a dense C
  * is written for whole groups.  An odd num_sms is used down to the next even number, 1 takes one pair. */
 int dm_gemm_nvfp4_pairs(dm_operand a, dm_operand sfa, const void* w, const void* sfb, dm_operand c, dm_operand h2,
                         const int64_t* scatter_ptrs, dm_operand row_scale_inv, const float* expert_scale_inv,

@@ -101,3 +101,25 @@ def test_a_high_water_mark_would_leave_blocks_unchecked(walk, counts, n):
                 mark = last + 1
             skipped += len(set(range(first, last + 1)) - checked)
     assert skipped > 0
+
+
+def test_pairs_that_take_tiles(tmp_path):
+    """Even rounds: no more rounds than with all pairs, every pair with tiles in all of them but the last; all pairs where rounds
+    do not matter (one round, large tiles), and, where the epilogue counts, where two or three rounds fill more than half of the last."""
+    (tmp_path / "p.cpp").write_text('#include "row_tiles.cuh"\nextern "C" int pairs(int t, int w, int r, int l, bool h) '
+                                    '{ return dm::balanced_pairs(t, w, r, l, h); }\n')
+    subprocess.run(["g++", "-std=c++17", "-shared", "-fPIC", f"-I{CSRC}", "-o", str(tmp_path / "p.so"), str(tmp_path / "p.cpp")],
+                   check=True)
+    pairs = ctypes.CDLL(str(tmp_path / "p.so")).pairs
+    pairs.argtypes = [ctypes.c_int] * 4 + [ctypes.c_bool]
+    for workers in (1, 3, 74):
+        for tiles in range(0, 12 * workers + 2):
+            rounds = -(-tiles // workers)
+            assert pairs(tiles, workers, 65, 64, False) == workers
+            even = pairs(tiles, workers, 64, 64, False)
+            assert even == workers if rounds <= 1 else even <= workers and (rounds - 1) * even < tiles <= rounds * even
+            heavy = pairs(tiles, workers, 64, 64, True)
+            last = tiles - (rounds - 1) * workers
+            assert heavy == (workers if 2 <= rounds <= 3 and 2 * last > workers else even)
+    # measured: 132 tiles (58 in the second round) and 198 (50 in the third) lose by even rounds, 154 (6), 242 and 264 gain
+    assert [pairs(t, 74, 32, 32, True) for t in (132, 198, 154, 242, 264)] == [74, 74, 52, 61, 66]
