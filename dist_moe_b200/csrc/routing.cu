@@ -204,21 +204,30 @@ __device__ __forceinline__ int pad_rows(int n, int m) { return m > 0 ? (n + m - 
 // Padded exclusive prefix of the experts' row counts, by one whole warp: every lane sums neighbouring experts, one scan runs
 // over the lanes; returns the total.  Latency bound: one thread walking the experts paid a dependent shared-memory load and
 // add per expert (single-launch kernel 18.4 us at 128 experts and 16 tokens), a scan per 32 experts still paid its ten
-// shuffles each time (7.7 us).
+// shuffles each time (7.7 us).  The padding divides once per expert, and up to 32 experts take no loop: with a second division
+// and loops of one step 8 experts took 0.3 us longer.
 __device__ __forceinline__ int64_t warp_padded_prefix(const int32_t* total, int32_t* base, int n, int m_mult, int lane) {
   const int per = (n + 31) >> 5, lo = lane * per < n ? lane * per : n, hi = lo + per < n ? lo + per : n;
   int64_t own = 0;
-  for (int i = lo; i < hi; ++i) own += pad_rows(total[i], m_mult);
+  if (n <= 32) {  // an expert per lane, without the loops' latency
+    own = lane < n ? pad_rows(total[lane], m_mult) : 0;
+  } else {
+    for (int i = lo; i < hi; ++i) {
+      base[i] = static_cast<int32_t>(own);
+      own += pad_rows(total[i], m_mult);
+    }
+  }
   int64_t incl = own;
 #pragma unroll
   for (int d = 1; d < 32; d <<= 1) {
     const int64_t t = __shfl_up_sync(0xffffffffu, incl, d);
     if (lane >= d) incl += t;
   }
-  int64_t at = incl - own;
-  for (int i = lo; i < hi; ++i) {
-    base[i] = static_cast<int32_t>(at);
-    at += pad_rows(total[i], m_mult);
+  const int32_t at = static_cast<int32_t>(incl - own);
+  if (n <= 32) {
+    if (lane < n) base[lane] = at;
+  } else {
+    for (int i = lo; i < hi; ++i) base[i] += at;
   }
   const int64_t all = __shfl_sync(0xffffffffu, incl, 31);
   if (lane == 0) base[n] = static_cast<int32_t>(all);
@@ -410,12 +419,15 @@ __global__ void __launch_bounds__(kChunkTokens) route_place_kernel(RouteParams p
 // pointers and the padding rows (up to 127 per expert, which one SM took 4 to 13 us to store) are dealt out over the blocks.
 // The ids are loaded once, beside the other addresses, and stay in registers.  One rank, padded to 128: 16 tokens x 8 of 128
 // experts 9.8 -> 5.7 us, 128 x 8 of 32 6.6 -> 5.6, 128 x 8 of 256 21.3 -> 6.9, 1,024 x 8 of 64 20.0 -> 7.8; unpadded,
-// 32 x 6 of 64 5.2 -> 5.1; eight ranks of 8 experts, 64 tokens each, 6.5 -> 6.8.
+// eight ranks of 8 experts, 64 tokens each, 6.9 both; unpadded (a form of its own: no division, no second block), 32 x 6 of 64
+// 5.4 -> 4.7, 16 x 2 of 8 4.6 -> 4.0, eight ranks of 8 experts, 64 x 6, 5.7 -> 5.5.
 // ---------------------------------------------------------------------------
 constexpr int kDecodeThreads = 1024;
 constexpr int kDecodeWarps = kDecodeThreads / 32;
-constexpr int kDecodeBlocks = 32, kDecodePadding = 512;  // at most so many blocks, one per so many padding rows
+// At most so many blocks, one per so many padding rows (1,024 tokens x 8 of 32 experts: 512 8.0 us, 1,024 9.0, 2,048 12.0).
+constexpr int kDecodeBlocks = 32, kDecodePadding = 512;
 
+template <bool kPad>
 __global__ void __launch_bounds__(kDecodeThreads) route_decode_kernel(RouteParams p) {
   extern __shared__ uint32_t smem_u[];
   uint32_t* mask = smem_u;                                                // [32][e_local] lane masks
@@ -426,7 +438,8 @@ __global__ void __launch_bounds__(kDecodeThreads) route_decode_kernel(RouteParam
   __shared__ int overflow;
   __shared__ int mismatch;
   const int i = threadIdx.x, warp = i >> 5, lane = i & 31;
-  const bool writer = blockIdx.x == 0;
+  const bool writer = !kPad || blockIdx.x == 0;
+  const int mult = kPad ? p.m_mult : 0;
   const int used = (p.ep * p.T + 31) >> 5;  // warps that hold tokens
   const int s = i / p.T, tok = i - s * p.T;
   const bool live = s < p.ep;
@@ -461,7 +474,7 @@ __global__ void __launch_bounds__(kDecodeThreads) route_decode_kernel(RouteParam
     total[el] = running;
   }
   __syncthreads();
-  const int64_t acc = warp == 0 ? warp_padded_prefix(total, base, p.e_local, p.m_mult, lane) : 0;
+  const int64_t acc = warp == 0 ? warp_padded_prefix(total, base, p.e_local, mult, lane) : 0;
   if (i == 0) {
     overflow = (acc > p.capacity_rows || acc > p.ptrs_size) ? 1 : 0;
     if (overflow && writer) set_status(p.status, kCapacityExceeded, static_cast<int>(acc), static_cast<int>(p.capacity_rows));
@@ -472,18 +485,18 @@ __global__ void __launch_bounds__(kDecodeThreads) route_decode_kernel(RouteParam
   if (writer) {
     for (int el = i; el <= p.e_local; el += kDecodeThreads) {
       p.expert_offsets[el] = bad ? 0 : base[el];
-      if (el < p.e_local) p.counts[el] = bad ? 0 : pad_rows(total[el], p.m_mult);
+      if (el < p.e_local) p.counts[el] = bad ? 0 : pad_rows(total[el], mult);
       if (el < p.e_local && p.real_counts != nullptr) p.real_counts[el] = bad ? 0 : total[el];
     }
     for (int q = warp; q < p.ep; q += kDecodeWarps) {
-      const int sum = warp_padded_sum(hist_s + q * p.e_local, p.e_local, p.m_mult, lane);
+      const int sum = warp_padded_sum(hist_s + q * p.e_local, p.e_local, mult, lane);
       if (lane == 0) p.per_rank[q] = sum;
     }
   }
   if (bad) return;
   const int blocks = static_cast<int>(gridDim.x);
-  clear_padding(p, base, total, static_cast<int>(blockIdx.x) + blocks * warp, blocks * kDecodeWarps);
-  if (live && warp % blocks == static_cast<int>(blockIdx.x))
+  if (kPad) clear_padding(p, base, total, static_cast<int>(blockIdx.x) + blocks * warp, blocks * kDecodeWarps);
+  if (live && (!kPad || warp % blocks == static_cast<int>(blockIdx.x)))
     place_ids(p, ids, first8, tok, dbase, cbase, [&](int el) {
       return base[el] + static_cast<int>(wprefix[warp * p.e_local + el]) +
              __popc(mask[warp * p.e_local + el] & ((1u << lane) - 1u));
@@ -625,16 +638,20 @@ static int route_launch(const uint64_t* routing_ptrs, const uint64_t* dispatch_p
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (g_route_decode && static_cast<int64_t>(ep) * T <= kDecodeThreads && p.e_local <= 512) {
     const size_t smem = sizeof(uint32_t) * (2 * kDecodeWarps * p.e_local + E + 2 * p.e_local + 1);
+    constexpr int kMost = static_cast<int>(sizeof(uint32_t) * (2 * kDecodeWarps * 512 + kMaxExpertsSmem + 1025));
     static PerDeviceOnce attr_set;
     const int rc_attr = once_per_device(attr_set, [] {
-      return static_cast<int>(
-          cudaFuncSetAttribute(route_decode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               static_cast<int>(sizeof(uint32_t) * (2 * kDecodeWarps * 512 + kMaxExpertsSmem + 1025))));
+      const auto most = cudaFuncAttributeMaxDynamicSharedMemorySize;
+      const cudaError_t err = cudaFuncSetAttribute(route_decode_kernel<true>, most, kMost);
+      return static_cast<int>(err != cudaSuccess ? err : cudaFuncSetAttribute(route_decode_kernel<false>, most, kMost));
     });
     if (rc_attr != 0) return rc_attr;
-    const int64_t padding = static_cast<int64_t>(p.e_local) * (m_multiple_of > 0 ? m_multiple_of - 1 : 0);
-    const int64_t blocks = padding / kDecodePadding + 1;
-    route_decode_kernel<<<static_cast<int>(blocks < kDecodeBlocks ? blocks : kDecodeBlocks), kDecodeThreads, smem, st>>>(p);
+    if (m_multiple_of > 0) {
+      const int64_t blocks = static_cast<int64_t>(p.e_local) * (m_multiple_of - 1) / kDecodePadding + 1;
+      route_decode_kernel<true><<<static_cast<int>(blocks < kDecodeBlocks ? blocks : kDecodeBlocks), kDecodeThreads, smem, st>>>(p);
+    } else {
+      route_decode_kernel<false><<<1, kDecodeThreads, smem, st>>>(p);
+    }
     return static_cast<int>(cudaGetLastError());
   }
   // The sums cost every block a read of all chunks' counts, so the work grows with the square of the chunks; the scan's one
