@@ -159,6 +159,7 @@ _SIGNATURES = {
     "dm_vmm_create": (c_int, [c_int, c_int, _P, _P, _P, _P]),
     "dm_vmm_destroy": (c_int, [_P]),
     "dm_set_route_decode_kernel": (c_int, [c_int]),
+    "dm_route_launches": (c_int, [c_int, c_int64, c_int]),
     "dm_route_decode_kernel_enabled": (c_int, []),
     "dm_gemm_blockscaled_swiglu_mxfp8": (
         c_int,
@@ -249,23 +250,17 @@ for _name, (_res, _args) in _SIGNATURES.items():
 # Kernel launches issued through this binding (benchmarks report the count).
 LAUNCHES = [0]
 _LAUNCHES_PER_CALL = {"dm_route": 3, "dm_route_counted": 3}
-GATHER_FLAGS_KEPT_CLEAR = 1 << 30  # include/dist_moe_b200.h, as the next two
-_ROUTE_CHUNK_TOKENS, _ROUTE_TWO_LAUNCH_CHUNKS = 256, 1024
-
-
-def route_call_name(ep: int, tokens: int, e_local: int) -> str:
-    """Name under which a ``dm_route`` call is counted: the decode regime is one launch instead of several."""
-    single = ep * tokens <= 1024 and e_local <= 512 and lib.dm_route_decode_kernel_enabled()
-    return "dm_route(single launch)" if single else "dm_route"
+GATHER_FLAGS_KEPT_CLEAR = 1 << 30  # include/dist_moe_b200.h
 
 
 def route_launches(ep: int, tokens: int, e_local: int) -> int:
     """Kernels that a ``dm_route`` call launches: one in the decode regime, two or three beyond."""
-    if e_local > 512:
-        return 3
-    if ep * tokens <= 1024 and lib.dm_route_decode_kernel_enabled():
-        return 1
-    return 2 if ep * -(-tokens // _ROUTE_CHUNK_TOKENS) <= _ROUTE_TWO_LAUNCH_CHUNKS else 3
+    return lib.dm_route_launches(ep, tokens, e_local)
+
+
+def route_call_name(ep: int, tokens: int, e_local: int) -> str:
+    """Name under which a ``dm_route`` call is counted: the decode regime is one launch instead of several."""
+    return "dm_route(single launch)" if route_launches(ep, tokens, e_local) == 1 else "dm_route"
 
 
 def check(rc: int, what: str, launches: int | None = None) -> None:

@@ -591,6 +591,8 @@ extern "C" int dm_set_route_decode_kernel(int enabled) {
 
 extern "C" int dm_route_decode_kernel_enabled(void) { return g_route_decode; }
 
+extern "C" int dm_route_launches(int ep, int64_t T, int e_local) { return DM_ROUTE_LAUNCHES(ep, T, e_local, g_route_decode); }
+
 static int route_launch(const uint64_t* routing_ptrs, const uint64_t* dispatch_ptrs, const uint64_t* combine_ptrs,
                         int rank, int ep, int64_t T, int K, int E, int64_t gather_stride_bytes,
                         int64_t bwd_gather_stride_bytes, int64_t scatter_stride_bytes, int m_multiple_of,
@@ -636,7 +638,9 @@ static int route_launch(const uint64_t* routing_ptrs, const uint64_t* dispatch_p
   p.hist = workspace + 2 * n;
   p.status = status;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (g_route_decode && static_cast<int64_t>(ep) * T <= kDecodeThreads && p.e_local <= 512) {
+  const int launches = DM_ROUTE_LAUNCHES(ep, T, p.e_local, g_route_decode);
+  static_assert(DM_ROUTE_LAUNCHES(1, kDecodeThreads, 1, 1) == 1 && DM_ROUTE_LAUNCHES(1, kDecodeThreads + 1, 1, 1) == 2, "");
+  if (launches == 1) {
     const size_t smem = sizeof(uint32_t) * (2 * kDecodeWarps * p.e_local + E + 2 * p.e_local + 1);
     constexpr int kMost = static_cast<int>(sizeof(uint32_t) * (2 * kDecodeWarps * 512 + kMaxExpertsSmem + 1025));
     static PerDeviceOnce attr_set;
@@ -658,7 +662,7 @@ static int route_launch(const uint64_t* routing_ptrs, const uint64_t* dispatch_p
   // block grows linearly.  Measured on either side, us, three launches | two: 512 chunks x 64 experts 62 | 23, x 500 235 | 132;
   // 1,024 x 64 111 | 49, x 256 372 | 167, x 500 445 | 335; 2,048 x 64 205 | 132, x 500 861 | 921, eight ranks of 32 experts
   // 115 | 83; 4,096 x 64 394 | 458, x 256 1,418 | 1,737, eight ranks of 32 236 | 277.
-  const bool place = static_cast<int64_t>(ep) * p.chunks <= DM_ROUTE_TWO_LAUNCH_CHUNKS && p.e_local <= 512;
+  const bool place = launches == 2;
   p.own_hist = place && ep == 1 ? 1 : 0;
   if (!p.own_hist) {
     const cudaError_t err = cudaMemsetAsync(p.hist, 0, sizeof(int32_t) * E, st);

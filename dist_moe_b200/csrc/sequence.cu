@@ -41,12 +41,6 @@ struct Sequence {
 
 const dm_operand kNone{nullptr, 0, nullptr};
 
-int launches_of_route(const dm_layer_context& c, const dm_layer_call& k) {
-  if (c.e_local > 512) return 3;
-  if (c.ep * k.T <= 1024 && dm_route_decode_kernel_enabled() != 0) return 1;
-  return c.ep * ((k.T + DM_ROUTE_CHUNK_TOKENS - 1) / DM_ROUTE_CHUNK_TOKENS) <= DM_ROUTE_TWO_LAUNCH_CHUNKS ? 2 : 3;
-}
-
 }  // namespace
 
 extern "C" int dm_bf16_forward(const dm_layer_context* ctx, const dm_layer_call* call, uint32_t steps, int32_t* report,
@@ -58,7 +52,7 @@ extern "C" int dm_bf16_forward(const dm_layer_context* ctx, const dm_layer_call*
   Sequence s{c, steps, report, stream};
   const int64_t stride = c.D * 2;
   int64_t* fs = k.fwd_state;
-  const int route_launches = launches_of_route(c, k);
+  const int route_launches = DM_ROUTE_LAUNCHES(c.ep, k.T, c.e_local, dm_route_decode_kernel_enabled());
   s.step(DM_FWD_PUBLISH, 1, [&] {
     return dm_publish(k.x, k.ids, k.ids_are_int64, c.dispatch, c.routing, k.T, c.D, c.K, c.E, k.validate_ids, c.status, stream);
   });
@@ -212,7 +206,7 @@ extern "C" int dm_mxfp8_forward(const dm_layer_context* ctx, const dm_layer_call
   Sequence s{c, steps, report, stream};
   const int64_t stride = c.D * 2;
   int64_t *fs = k.fwd_state, *ft = k.fwd_table;
-  const int route_launches = launches_of_route(c, k);
+  const int route_launches = DM_ROUTE_LAUNCHES(c.ep, k.T, c.e_local, dm_route_decode_kernel_enabled());
   s.step(DM_FWD_PUBLISH, 1, [&] {
     return dm_publish(k.x, k.ids, k.ids_are_int64, c.dispatch, c.routing, k.T, c.D, c.K, c.E, k.validate_ids, c.status, stream);
   });

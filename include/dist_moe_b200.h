@@ -43,6 +43,12 @@ extern "C" {
  * all ranks, three beyond. */
 #define DM_ROUTE_CHUNK_TOKENS 256
 #define DM_ROUTE_TWO_LAUNCH_CHUNKS 1024
+/* Kernels that a routing call launches (`decode`: dm_route_decode_kernel_enabled()): one in the decode regime, two or three
+ * beyond. */
+#define DM_ROUTE_LAUNCHES(ep, T, e_local, decode)                                                                       \
+  ((e_local) > 512                        ? 3                                                                            \
+   : (decode) && (int64_t)(ep) * (T) <= 1024 ? 1                                                                         \
+   : (int64_t)(ep) * (((T) + DM_ROUTE_CHUNK_TOKENS - 1) / DM_ROUTE_CHUNK_TOKENS) <= DM_ROUTE_TWO_LAUNCH_CHUNKS ? 2 : 3)
 
 /* Library version / build probe; returns the compiled SM architecture (1000). */
 int dm_version(void);
@@ -141,6 +147,7 @@ int dm_route_static(const uint64_t* routing_ptrs, const uint64_t* dispatch_ptrs,
  * same tables bit for bit (rows ordered by local expert, source rank, token).  Returns the previous setting. */
 int dm_set_route_decode_kernel(int enabled);
 int dm_route_decode_kernel_enabled(void); /* the current setting, without changing it */
+int dm_route_launches(int ep, int64_t T, int e_local); /* DM_ROUTE_LAUNCHES under the current setting */
 
 /* ---------------------------------------------------------------------------
  * Activation-arena planner, BF16
