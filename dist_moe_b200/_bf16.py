@@ -16,14 +16,13 @@ CUDA graph.  Bracketed steps are device-predicated on the planner's decision.
 
 from __future__ import annotations
 
-import math
 from typing import Any
 
 import torch
 
 from . import _native as nat
 from ._call import (BWD, FWD, FWD_ALL, CallState, Layout, arguments, in_one_piece, launch, layout_of, observed, on_device,
-                    recorded, span)
+                    recorded, routes_in_one_piece, span)
 from ._execution import ExecutionOptions, RMSNormPostprocess
 
 
@@ -95,7 +94,10 @@ def _arguments(state, c: _Call, x, ids, scores, w13, w2, options: ExecutionOptio
 
 
 def _weights_in_one_piece(state, w13, w2):
-    n = state.e_local * state.config.intermediate_dim * state.config.hidden_dim
+    cfg = state.config
+    n = state.e_local * cfg.intermediate_dim * cfg.hidden_dim
+    if w2.numel() == n and w13.numel() == 2 * n and w2.is_contiguous() and w13.is_contiguous():
+        return w13, w2
     return in_one_piece(w13, 2 * n, "w13"), in_one_piece(w2, n, "w2")
 
 
@@ -161,7 +163,7 @@ def _wgrad_destination(param: torch.Tensor, shape, options: ExecutionOptions, cf
         named = hooks.wgrad_destination(name, shape, cfg.wgrad_dtype or param.dtype, param.device)
         if named is not None:
             return named[0], int(named[1]), False
-    if param.numel() != math.prod(shape):  # the weight may be another one by now than in the forward; a GEMM writes all of ``shape``
+    if param.numel() != shape[0] * shape[1] * shape[2]:  # the weight may be another one by now than in the forward; a GEMM writes all of ``shape``
         raise RuntimeError(f"the gradient of a weight of shape {tuple(param.shape)} cannot hold one of shape {tuple(shape)}")
     if isinstance(explicit, torch.Tensor):
         if not explicit.is_contiguous() or explicit.dtype not in (torch.bfloat16, torch.float32) \
@@ -196,7 +198,7 @@ def backward_impl(state, c: _Call, x_shape, ids, scores, w13, w2, w13_param, w2_
     dev = grad_out.device
     need_x, need_scores, need_w13, need_w2 = needs
     w13, w2 = _weights_in_one_piece(state, w13, w2)
-    ids, scores = in_one_piece(ids, T * K, "topk_expert_ids_TK"), in_one_piece(scores, T * K, "topk_scores_TK")
+    ids, scores = routes_in_one_piece(ids, scores, T * K)
     # the plan's offsets: [xg, h1, h2, grad_h2, grad_h3_gathered, grad_h1]
     bo = torch.empty(6, dtype=torch.int64, device=dev) if c.buf is None else None
     grad_scores = torch.empty(T, K, dtype=torch.float32, device=dev) if need_scores else None

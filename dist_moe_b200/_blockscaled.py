@@ -41,7 +41,8 @@ from typing import Any
 import torch
 
 from . import _native as nat
-from ._call import BWD, FWD, FWD_ALL, CallState, arguments, in_one_piece, launch, layout_of, observed, on_device, span
+from ._call import (BWD, FWD, FWD_ALL, CallState, arguments, launch, layout_of, observed, on_device, routes_in_one_piece,
+                    span)
 from ._execution import ExecutionOptions, PreparedWeight, RMSNormPostprocess
 from .formats import BlockScaledFormat, format_constants
 
@@ -597,7 +598,7 @@ def _mxfp8_backward_planned(state, c: _PlannedCall, x_shape, ids, scores, w13_pa
     D, F, K = cfg.hidden_dim, cfg.intermediate_dim, cfg.top_k
     T, el, dev = c.T, state.e_local, grad_out.device
     need_x, need_scores, need_w13, need_w2 = needs
-    ids, scores = in_one_piece(ids, T * K, "topk_expert_ids_TK"), in_one_piece(scores, T * K, "topk_scores_TK")
+    ids, scores = routes_in_one_piece(ids, scores, T * K)
     plan = torch.empty(16 + 54, dtype=torch.int64, device=dev)  # the plan's offsets and its table of operands
     grad_scores = torch.empty(T, K, dtype=torch.float32, device=dev) if need_scores else None
     post = options.experts_output_postprocess
@@ -768,7 +769,7 @@ def _mxfp8_backward(state, c: _TrainCall, x_shape, ids, scores, w13_param, w2_pa
     clamped = 1 if cfg.activation == "swiglu_clamped" else 0
     alpha, limit = float(cfg.swiglu_alpha), float(cfg.swiglu_limit)
     need_x, need_scores, need_w13, need_w2 = needs
-    ids, scores = in_one_piece(ids, T * K, "topk_expert_ids_TK"), in_one_piece(scores, T * K, "topk_scores_TK")
+    ids, scores = routes_in_one_piece(ids, scores, T * K)
     recv, offs = c.recv.data_ptr(), c.offsets.data_ptr()
     none = nat.Operand(None, 0, None)
     full = lambda t: nat.Operand(t.data_ptr(), t.numel() * t.element_size(), None)  # noqa: E731

@@ -131,6 +131,12 @@ def in_one_piece(t: torch.Tensor, numel: int, name: str) -> torch.Tensor:
     return t if t.is_contiguous() else t.detach().contiguous()
 
 
+def routes_in_one_piece(ids: torch.Tensor, scores: torch.Tensor, routes: int) -> tuple[torch.Tensor, torch.Tensor]:
+    if ids.numel() == routes == scores.numel() and ids.is_contiguous() and scores.is_contiguous():
+        return ids, scores
+    return in_one_piece(ids, routes, "topk_expert_ids_TK"), in_one_piece(scores, routes, "topk_scores_TK")
+
+
 class Layout:
     """Where the device results of a call lie in their buffer.  ``fields``: name -> (dtype, elements)."""
 
